@@ -7,6 +7,7 @@ import os
 
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG_DIR, "libcdssm_b200.so")
+HOST_PATH = os.path.join(_PKG_DIR, "_cdssm_host.so")
 
 OK = 0
 ERRORS = {
@@ -61,10 +62,28 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class CdssmError(RuntimeError):
     pass
+
+
+def host():
+    """Load the native host path (csrc/host) once; raise if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise CdssmError(f"{HOST_PATH} not found: build it with `python __graft_entry__.py`")
+        import importlib.util
+        import torch  # noqa: F401  (the extension links against its libraries)
+        spec = importlib.util.spec_from_file_location("_cdssm_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_error_type(CdssmError)
+        _host = mod
+    return _host
 
 
 def lib():

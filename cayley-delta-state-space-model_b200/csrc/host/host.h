@@ -1,0 +1,155 @@
+// Native host path of the operator and model API: argument checks, output allocation and the launches of one call in
+// C++, so that a call costs a few microseconds of host time instead of tens (a ctypes call with thirty arguments and
+// its Python-side checks took 29 us around a 4 us kernel).  The kernels stay behind the C ABI of libcdssm_b200.so.
+#pragma once
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
+
+#include "../../../include/cdssm_b200.h"
+
+namespace cdssm_host {
+
+using at::Tensor;
+
+// Raised as the package's CdssmError.
+struct Error : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+
+void check(int rc, const char* what);   // throws Error unless rc is CDSSM_OK
+
+inline int dtype_code(const Tensor& t) {
+    if (t.scalar_type() == at::kBFloat16) return CDSSM_BF16;
+    if (t.scalar_type() == at::kFloat) return CDSSM_F32;
+    throw Error(std::string("unsupported dtype ") + c10::toString(t.scalar_type()) +
+                ": use bfloat16 (the reference's type) or float32");
+}
+
+inline void need_cuda(const Tensor& t, const char* name) {
+    if (!t.is_cuda()) throw Error(std::string(name) + " must be a CUDA tensor (no CPU fallback exists)");
+}
+
+// A dense CUDA tensor of the wanted type, or an error (the reference launchers check neither).
+inline Tensor dense(const Tensor& t, at::ScalarType dt, const char* name) {
+    need_cuda(t, name);
+    if (t.scalar_type() != dt)
+        throw Error(std::string(name) + " has dtype " + c10::toString(t.scalar_type()) + ", expected " + c10::toString(dt));
+    return t.is_contiguous() ? t : t.contiguous();
+}
+
+// Per-head float32 vectors; a bf16 buffer (a model cast with .bfloat16()) is converted.
+inline Tensor f32_vector(const Tensor& t, const char* name) {
+    need_cuda(t, name);
+    if (t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
+    return t.detach().to(at::kFloat).contiguous();
+}
+
+inline const void* cptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
+inline void* mptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline const float* fptr(const Tensor& t) { return t.defined() ? static_cast<const float*>(t.const_data_ptr()) : nullptr; }
+inline float* fmut(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+
+inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+inline Tensor empty_like_dims(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options()); }
+inline Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) {
+    return at::empty(sizes, like.options().dtype(at::kFloat));
+}
+
+struct Dyn {   // the five scalars of the dynamics
+    float c[5];
+};
+
+// The grow-only scratch buffer of a (device, current stream): 256-byte aligned start and usable bytes.
+struct Workspace {
+    void* ptr;
+    size_t bytes;
+};
+Workspace workspace(const Tensor& on, size_t bytes);
+void* workspace_if_any(int device);   // start of the buffer of (device, its current stream), or nullptr
+
+// ---- operators (ops.cpp)
+struct ScanOut {
+    Tensor y, final_state, tail;
+};
+ScanOut scan_fused(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gate, const Tensor& lds,
+                   const Tensor& rope, const Dyn& dyn, int64_t H, int64_t N, int64_t C, const Tensor& h0, double shortcut,
+                   int64_t pos0, bool want_tail, int64_t flags, const Tensor& out, int64_t segs);
+Tensor decode_step(const Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gate,
+                   const Tensor& lds, const Tensor& rope, const Dyn& dyn, int64_t H, int64_t N, int64_t pos,
+                   const Tensor& pos_dev, double shortcut, const Tensor& out, const Tensor& v_first, const Tensor& mix);
+Tensor rms_norm(const Tensor& x, const Tensor& w, double eps);
+Tensor groupnorm_gate(const Tensor& y, const Tensor& gw, const Tensor& gb, const Tensor& z, const Tensor& skip,
+                      const Tensor& x_conv, int64_t groups, double eps, bool per_token);
+Tensor conv1d_silu(const Tensor& x, const Tensor& w, const Tensor& b);
+Tensor conv1d_silu_step(const Tensor& x, const Tensor& hist, const Tensor& w, const Tensor& b);
+
+// ---- Python side helpers
+struct Args {   // positional arguments of a METH_FASTCALL function
+    PyObject* const* a;
+    Py_ssize_t n, at = 0;
+    PyObject* next() {
+        if (at >= n) throw Error("too few arguments");
+        return a[at++];
+    }
+    Tensor tensor(const char* name) {
+        PyObject* o = next();
+        if (!THPVariable_Check(o)) throw Error(std::string(name) + " must be a tensor");
+        return THPVariable_Unpack(o);
+    }
+    Tensor tensor_or_none(const char* name) {
+        PyObject* o = next();
+        if (o == Py_None) return Tensor();
+        if (!THPVariable_Check(o)) throw Error(std::string(name) + " must be a tensor or None");
+        return THPVariable_Unpack(o);
+    }
+    double number() {
+        const double v = PyFloat_AsDouble(next());
+        if (v == -1.0 && PyErr_Occurred()) throw std::invalid_argument("number");
+        return v;
+    }
+    int64_t integer() {
+        PyObject* o = next();
+        PyObject* i = PyLong_Check(o) ? (Py_INCREF(o), o) : PyNumber_Long(o);
+        if (!i) throw std::invalid_argument("integer");
+        const int64_t v = PyLong_AsLongLong(i);
+        Py_DECREF(i);
+        if (v == -1 && PyErr_Occurred()) throw std::invalid_argument("integer");
+        return v;
+    }
+    bool flag() { return PyObject_IsTrue(next()) == 1; }
+    Dyn dyn() {
+        Dyn d;
+        for (float& x : d.c) x = (float)number();
+        return d;
+    }
+};
+
+extern PyObject* g_error_type;
+// Runs fn and turns C++ exceptions into Python ones.
+template <typename F>
+PyObject* guarded(F&& fn) {
+    try {
+        return fn();
+    } catch (const Error& e) {
+        PyErr_SetString(g_error_type ? g_error_type : PyExc_RuntimeError, e.what());
+    } catch (const c10::OutOfMemoryError& e) {
+        PyObject* t = PyObject_GetAttrString(PyImport_AddModule("torch"), "OutOfMemoryError");
+        PyErr_SetString(t ? t : PyExc_RuntimeError, e.what_without_backtrace());
+        Py_XDECREF(t);
+    } catch (const c10::Error& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    } catch (const std::exception& e) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+    }
+    return nullptr;
+}
+inline PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
+
+PyMethodDef* model_methods();   // lm.cpp
+
+}  // namespace cdssm_host

@@ -2,9 +2,8 @@
 
 This is the caller side of the hot path (the reference's cdssm/models/{model,block}.py), written
 from the behaviour of the reference so that benchmark configurations 1 (prefill) and 3 (batched
-recurrent decode) can run on random-initialised weights.  Projections, norms and the LM head are
-ordinary torch library calls (plumbing); the scan path itself is ``ops.scan_fused`` /
-``ops.decode_step`` and the depthwise conv is ``ops.CUDAConv1dSiLUOp``.
+recurrent decode) can run on random-initialised weights.  The passes themselves are native (csrc/host/lm.cpp):
+large projections and the LM head are ordinary library products (plumbing), everything else this library's kernels.
 
 Layer structure restated from cdssm/models/block.py:140-229, constants from
 cdssm/config/model.py:38-109, initialisation from cdssm/models/init.py:13-126 and
@@ -14,7 +13,6 @@ import math
 from dataclasses import dataclass
 
 import torch
-import torch.nn.functional as F
 
 from . import ops
 
@@ -50,13 +48,6 @@ class CdssmConfig:
     @property
     def dyn_consts(self):
         return (self.gating_c, self.omega_thresh, self.adt_delta, self.adt_smoothness, self.adt_eps)
-
-
-def _rms_norm(x, weight, eps):
-    if x.shape[-1] % 8 == 0:
-        return ops.rms_norm(x, weight, eps)           # one kernel
-    xf = x.float()
-    return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)).to(x.dtype) * weight
 
 
 class CdssmBlockParams:
@@ -119,15 +110,17 @@ class CdssmBlockParams:
         self.b_qg = torch.cat([torch.zeros(di, device=self.b_gate.device, dtype=self.b_gate.dtype), self.b_gate])
         self.w_q, self.w_gate = self.w_qg[:di], self.w_qg[di:]
 
-    def residual_mix(self, dtype):
-        """sigmoid(v_residual_gate) in the activation dtype (block.py:167-171), computed once per value of the
-        parameter instead of two small kernels per layer and token."""
-        g = self.v_residual_gate
-        key = (g.data_ptr(), g._version, dtype)
-        if getattr(self, "_mix_key", None) != key:
-            self._mix = torch.sigmoid(g).to(dtype)[None, None, :, None]
-            self._mix_key = key
-        return self._mix
+    # Every assignment to an attribute counts: the model lays its weights out for the native path once per state.
+    version = 0
+
+    def __setattr__(self, name, value):
+        self.__dict__[name] = value
+        self.__dict__["version"] = self.version + 1
+
+    def native(self):
+        return (self.norm_w, self.w_in, self.b_in, self.conv_w, self.conv_b, self.w_gate, self.b_gate, self.log_dt_scale,
+                self.rope_freqs, self.w_q, self.w_readout, self.w_out, self.gn_w, self.gn_b, self.D, self.v_residual_gate,
+                self.w_qg, self.b_qg, float(self.shortcut_scale))
 
     def load_reference(self, sd, prefix, device, dtype):
         """Take this block's weights from a reference state dict (parameter names of
@@ -179,117 +172,45 @@ class CdssmLM:
         self.blocks = [CdssmBlockParams(cfg, i, gen, device, dtype) for i in range(cfg.n_layers)]
         self.final_norm_w = torch.ones(cfg.d_model, device=device, dtype=dtype)
         self.per_token_group_norm = False   # False = the reference's sequence-wide GroupNorm statistics
+        self._plan = None
 
-    # ------------------------------------------------------------------ one block
-    def _block(self, p: CdssmBlockParams, x, v_first, pos0, cache, scan_flags):
-        cfg = self.cfg
-        B, L, _ = x.shape
-        H, N, di = cfg.n_heads, cfg.state_dim, cfg.d_inner
-        xn = _rms_norm(x, p.norm_w, cfg.eps_norm)
-        if L > 1:
-            # One product per consumer (row blocks of the in_proj weight are contiguous views): each output is
-            # dense, so neither the conv nor the scan has to copy a column slice of a wide projection first.
-            z, x_gate, K, V = (F.linear(xn, p.w_in[a:b], p.b_in[a:b]) for a, b in
-                               ((0, di), (di, 2 * di), (2 * di, 3 * di), (3 * di, 3 * di + H * N)))
-        else:
-            z, x_gate, K, V = F.linear(xn, p.w_in, p.b_in).split([di, di, di, H * N], dim=-1)
-        K = K.reshape(B, L, H, cfg.head_dim)
-        V = V.reshape(B, L, H, N)
-        decoding = cache is not None and "state" in cache     # a populated cache: one-token step
-        mix = None
-        if v_first is None:
-            v_first = V.contiguous() if decoding else V     # one small copy per step; the kernels read it densely
-        elif decoding:                          # the decode kernel applies the value residual itself
-            mix = p.residual_mix(V.dtype)
-        else:                                   # value residual across layers (block.py:167-171)
-            V = torch.lerp(v_first, V, p.residual_mix(V.dtype))
-        if not decoding:
-            x_conv = ops.CUDAConv1dSiLUOp.apply(x_gate, p.conv_w, p.conv_b)
-            if cache is not None:               # last three inputs of the causal 4-tap conv
-                hist = torch.zeros(B, 3, di, device=x.device, dtype=x.dtype)
-                n = min(3, L)
-                hist[:, 3 - n:] = x_gate[:, L - n:]
-                cache["conv"] = hist
-        else:                                   # decode: one output from the cached history, shifted in place
-            x_conv = ops.conv1d_silu_step(x_gate[:, 0], cache["conv"], p.conv_w, p.conv_b).unsqueeze(1)
-        if decoding:                            # one product for Q and the gates; the step kernel reads the slices
-            qg = F.linear(x_conv, p.w_qg, p.b_qg)
-            Q, gates = qg[..., :di].unflatten(-1, (H, cfg.head_dim)), qg[..., di:]
-        else:
-            gates = F.linear(x_conv, p.w_gate, p.b_gate)
-            Q = F.linear(x_conv, p.w_q).reshape(B, L, H, cfg.head_dim)
-        if decoding:
-            y = ops.decode_step(cache["state"], Q[:, 0], K[:, 0], V[:, 0], gates[:, 0], p.log_dt_scale,
-                                p.rope_freqs, *cfg.dyn_consts, H, N, pos0, shortcut_scale=p.shortcut_scale,
-                                v_first=None if mix is None else v_first[:, 0], mix=mix).unsqueeze(1)
-        elif cache is not None:
-            y, _, tail = ops.scan_fused(Q, K, V, gates, p.log_dt_scale, p.rope_freqs, *cfg.dyn_consts, H, N,
-                                        cfg.chunk_size, shortcut_scale=p.shortcut_scale, pos0=pos0,
-                                        return_tail_state=True)
-            cache["state"] = tail
-        else:
-            y, _ = ops.scan_fused(Q, K, V, gates, p.log_dt_scale, p.rope_freqs, *cfg.dyn_consts, H, N,
-                                  cfg.chunk_size, shortcut_scale=p.shortcut_scale, pos0=pos0, flags=scan_flags)
-        y = F.linear(y.reshape(B, L, H * N), p.w_readout)
-        # The reference normalises over (channels of the group) x (ALL positions of the sequence)
-        # (block.py:216-222: group_norm on (B, d_inner, L)), which makes its forward non-causal.  A
-        # cached decode cannot reproduce that, so the prefill/decode path - and forward() when
-        # per_token_group_norm is set - takes the statistics per token instead.
-        per_token = cache is not None or self.per_token_group_norm
-        if (di // cfg.ssm_norm_groups) % 8 == 0 and di <= 8192:
-            y = ops.groupnorm_gate(y, p.gn_w, p.gn_b, z, p.D, x_conv, cfg.ssm_norm_groups, 1e-5, per_token=per_token)
-        else:
-            if per_token:
-                y = F.group_norm(y.float().reshape(B * L, di, 1), cfg.ssm_norm_groups, p.gn_w.float(),
-                                 p.gn_b.float(), 1e-5).to(x.dtype).reshape(B, L, di)
-            else:
-                y = F.group_norm(y.float().transpose(1, 2), cfg.ssm_norm_groups, p.gn_w.float(), p.gn_b.float(),
-                                 1e-5).to(x.dtype).transpose(1, 2)
-            y = y * F.silu(z) + p.D * x_conv
-        # the residual add rides in the product's epilogue
-        return torch.addmm(x.reshape(B * L, -1), y.reshape(B * L, di), p.w_out.t()).reshape(B, L, -1), v_first
+    def _native(self):
+        """The model as the native path holds it (csrc/host/lm.cpp: the blocks' layers, one call per pass).  Rebuilt when a
+        weight tensor was replaced; writes into the tensors themselves are seen anyway."""
+        key = (id(self.embedding), id(self.final_norm_w), *[(id(p), p.version) for p in self.blocks])
+        if self._plan is None or self._plan[0] != key:
+            c = self.cfg
+            plan = ops._lib.host().lm_plan(c.d_model, c.d_inner, c.n_heads, c.state_dim, c.chunk_size, c.ssm_norm_groups,
+                                           c.eps_norm, *c.dyn_consts, self.embedding, self.final_norm_w,
+                                           [p.native() for p in self.blocks])
+            self._plan = (key, plan, self.embedding, self.final_norm_w, list(self.blocks))   # ids stay taken
+        return self._plan[1]
 
     # ------------------------------------------------------------------ public API
     @torch.no_grad()
     def forward(self, input_ids, scan_flags=0):
         """Prefill: (B,L) token ids -> (B,L,vocab) logits (cdssm/models/model.py:37-51)."""
-        x = self.embedding[input_ids]
-        v_first = None
-        for p in self.blocks:
-            x, v_first = self._block(p, x, v_first, 0, None, scan_flags)
-        return F.linear(_rms_norm(x, self.final_norm_w, 2.0 ** -14), self.embedding)
+        return ops._lib.host().lm_forward(self._native(), input_ids, self.per_token_group_norm, scan_flags)
 
     @torch.no_grad()
     def prefill(self, input_ids, last_only=True):
         """Prefill that also returns the decode cache: per layer the recurrent state after the last
         token (B,H,N,D) fp32 and the last three conv inputs; plus the position counter."""
-        x = self.embedding[input_ids]
-        caches, v_first = [], None
-        for p in self.blocks:
-            c = {}
-            x, v_first = self._block(p, x, v_first, 0, c, 0)
-            caches.append(c)
-        if last_only:
-            x = x[:, -1:]
-        logits = F.linear(_rms_norm(x, self.final_norm_w, 2.0 ** -14), self.embedding)
-        return logits, {"layers": caches, "pos": input_ids.shape[1]}
+        logits, flat = ops._lib.host().lm_prefill(self._native(), input_ids, last_only)
+        layers = [{"state": flat[i], "conv": flat[i + 1]} for i in range(0, len(flat), 2)]
+        return logits, {"layers": layers, "pos": input_ids.shape[1]}
 
     @torch.no_grad()
     def decode(self, token_ids, cache):
         """One token per sequence: (B,) ids -> (B,vocab) logits; the cache is updated in place.
         The reference instead re-runs the whole window per token (cdssm/inference/predict.py:53-67)."""
-        x = self.embedding[token_ids].unsqueeze(1)
-        v_first = None
         # one position counter: the host integer, or - once a decode graph exists - the device int32 that
         # makes the step graph-replayable (see position())
-        pos = cache["pos_dev"] if "pos_dev" in cache else cache["pos"]
-        for p, c in zip(self.blocks, cache["layers"]):
-            x, v_first = self._block(p, x, v_first, pos, c, 0)
-        if "pos_dev" in cache:
-            cache["pos_dev"] += 1
-        else:
-            cache["pos"] += 1
-        return F.linear(_rms_norm(x[:, 0], self.final_norm_w, 2.0 ** -14), self.embedding)
+        name = "pos_dev" if "pos_dev" in cache else "pos"
+        flat = [c[n] for c in cache["layers"] for n in ("state", "conv")]
+        logits = ops._lib.host().lm_decode(self._native(), token_ids, flat, cache[name])
+        cache[name] += 1
+        return logits
 
     @staticmethod
     def position(cache):

@@ -302,22 +302,14 @@ TEST_WITHHOLD = 2048   # self-test of the bounded waits: see include/cdssm_b200.
 FP32_DECAY = 4096      # keep the transition A_bar in float32 (NOT the reference's arithmetic): the reference's
 #                        bfloat16 A_bar lets its carry grow without bound over some 1e5 tokens, see the header
 
-_workspaces = {}
-
-
 def scan_fused_workspace_bytes(B, L, H, D, N, C) -> int:
     return int(_lib.lib().cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C))
 
 
-def _workspace(device, nbytes):
-    """One grow-only scratch buffer per (device, stream); the library itself allocates nothing."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(nbytes + 256, dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    off = (-buf.data_ptr()) % 256
-    return buf.data_ptr() + off, buf.numel() - off
+def _workspace(on: Tensor, nbytes):
+    """(address, bytes) of the grow-only scratch buffer of the tensor's device and its current stream; the library
+    itself allocates nothing."""
+    return _lib.host().workspace(on, nbytes)
 
 
 def scan_fused(q: Tensor, k: Tensor, v: Tensor, gate_raw: Tensor, log_dt_scale: Tensor,
@@ -346,55 +338,19 @@ def scan_fused(q: Tensor, k: Tensor, v: Tensor, gate_raw: Tensor, log_dt_scale: 
     tensor-core kernels ran out (the outputs are undefined then); without it the call stays asynchronous
     and :func:`scan_fused_status` reports the same word on demand.
     """
-    if semantics not in ("reference", "exact"):
-        raise CdssmError("semantics must be 'reference' (the reference's chunked scan, bug for bug) or "
-                         "'exact' (the sequential recurrence)")
-    if semantics == "exact":
+    if semantics != "reference":
+        if semantics != "exact":
+            raise CdssmError("semantics must be 'reference' (the reference's chunked scan, bug for bug) or "
+                             "'exact' (the sequential recurrence)")
         flags = int(flags) | EXACT
-    q = _prep(q, name="q")
-    k = _prep(k, dtype=q.dtype, name="k")
-    v = _prep(v, dtype=q.dtype, name="v")
-    g = _prep(gate_raw, dtype=q.dtype, name="gate_raw")
-    B, L, H, D = q.shape
-    N, C = int(state_dim), int(chunk_size)
-    if H != int(n_heads) or k.shape != q.shape or tuple(v.shape) != (B, L, H, N) or \
-            tuple(g.shape) != (B, L, (N + 5) * H):
-        raise CdssmError("scan_fused: inconsistent shapes")
-    lds, rf = _f32(log_dt_scale, "log_dt_scale"), _f32(rope_freqs, "rope_freqs")
-    if h0 is not None:
-        h0 = _prep(h0, dtype=torch.float32, name="h0")
-        if tuple(h0.shape) != (B, H, N, D):
-            raise CdssmError("h0 must be (B,H,N,D)")
-    dev = q.device
-    y = out if out is not None else torch.empty(B, L, H, N, dtype=q.dtype, device=dev)
-    if out is not None and (tuple(out.shape) != (B, L, H, N) or out.dtype != q.dtype or not out.is_contiguous()):
-        raise CdssmError("out must be a contiguous (B,L,H,N) tensor of the input dtype")
-    final = torch.empty(B, H, N, D, dtype=torch.float32, device=dev)
-    tail = torch.empty(B, H, N, D, dtype=torch.float32, device=dev) if return_tail_state else None
-    if B * L == 0:   # nothing to scan: the carry passes through
-        final.zero_() if h0 is None else final.copy_(h0)
-        if tail is not None:
-            tail.copy_(final)
-        return (y, final, tail) if return_tail_state else (y, final)
-    with torch.cuda.device(dev):
-        ws_ptr, ws_bytes = _workspace(dev, scan_fused_workspace_bytes(B, L, H, D, N, C))
-        if segs == 1:
-            check(_lib.lib().cdssm_b200_scan_fused_fwd(
-                _p(q), _p(k), _p(v), _p(g), _p(lds), _p(rf), _p(h0), _p(y), _p(final), _p(tail), ws_ptr,
-                ws_bytes, gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps, shortcut_scale,
-                B, L, H, D, N, C, int(pos0), _dtype_code(q), int(flags), _stream()), "scan_fused_fwd")
-        else:
-            if return_tail_state:
-                raise CdssmError("tail_state is not available for segmented batches")
-            check(_lib.lib().cdssm_b200_scan_fused_segmented_fwd(
-                _p(q), _p(k), _p(v), _p(g), _p(lds), _p(rf), _p(h0), _p(y), _p(final), ws_ptr, ws_bytes,
-                gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps, shortcut_scale, B, L, H, D, N,
-                C, int(pos0), int(segs), _dtype_code(q), int(flags), _stream()), "scan_fused_segmented_fwd")
+    res = _lib.host().scan_fused(q, k, v, gate_raw, log_dt_scale, rope_freqs, gating_c, omega_thresh, adt_delta,
+                                 adt_smoothness, adt_eps, n_heads, state_dim, chunk_size, h0, shortcut_scale, pos0,
+                                 return_tail_state, flags, out, segs)
     if strict:
-        code = scan_fused_status(dev)
+        code = scan_fused_status(q.device)
         if code != 0:
             raise CdssmError(f"scan_fused: a device-side wait ran out (status {code}); the outputs are undefined")
-    return (y, final, tail) if return_tail_state else (y, final)
+    return res
 
 
 def decode_step(state: Tensor, q: Tensor, k: Tensor, v: Tensor, gate_raw: Tensor,
@@ -412,49 +368,8 @@ def decode_step(state: Tensor, q: Tensor, k: Tensor, v: Tensor, gate_raw: Tensor
     for every new token); the update is one iteration of intra_chunk_scan.cu:117-167 with the
     gates of dynamics_fused.cu:64-139 at position ``pos``.
     """
-    if not q.is_cuda:
-        raise CdssmError("q must be a CUDA tensor (no CPU fallback exists)")
-    B, H, D = q.shape
-    N = int(state_dim)
-    dt = q.dtype
-
-    def rows(t, shape, name):
-        """Rows dense inside; only the batch stride may be larger (a column slice of a projection)."""
-        ok = t.is_cuda and t.dtype == dt and tuple(t.shape) == tuple(shape)
-        inner = 1
-        for i in range(len(shape) - 1, 0, -1):
-            ok = ok and t.stride(i) == inner
-            inner *= shape[i]
-        ok = ok and t.stride(0) >= inner and (t.stride(0) * t.element_size()) % 16 == 0 and t.data_ptr() % 16 == 0
-        return t if ok else _prep(t, dtype=dt, name=name)       # anything else: a dense copy (as before)
-
-    q = rows(q, (B, H, D), "q")
-    k, v = rows(k, (B, H, D), "k"), rows(v, (B, H, N), "v")
-    g = rows(gate_raw, (B, (N + 5) * H), "gate_raw")
-    if not state.is_cuda or state.dtype != torch.float32 or not state.is_contiguous():
-        raise CdssmError("state must be a contiguous float32 CUDA tensor (B,H,N,D)")
-    if H != int(n_heads) or tuple(state.shape) != (B, H, N, D) or tuple(k.shape) != (B, H, D) or \
-            tuple(v.shape) != (B, H, N) or tuple(g.shape) != (B, (N + 5) * H):
-        raise CdssmError("decode_step: inconsistent shapes")
-    if (v_first is None) != (mix is None):
-        raise CdssmError("decode_step: v_first and mix go together")
-    if v_first is not None:
-        v_first = _prep(v_first, dtype=q.dtype, name="v_first")
-        mix = _prep(mix.reshape(-1), dtype=q.dtype, name="mix")
-        if tuple(v_first.shape) != (B, H, N) or mix.numel() != H:
-            raise CdssmError("decode_step: v_first must be (B,H,N) and mix (H)")
-    lds, rf = _f32(log_dt_scale, "log_dt_scale"), _f32(rope_freqs, "rope_freqs")
-    y = out if out is not None else torch.empty(B, H, N, dtype=q.dtype, device=q.device)
-    pos_dev, pos_i = (pos, 0) if isinstance(pos, Tensor) else (None, int(pos))
-    if pos_dev is not None and (pos_dev.dtype != torch.int32 or not pos_dev.is_cuda):
-        raise CdssmError("a tensor position must be an int32 CUDA tensor")   # device memory: graph-replayable
-    with torch.cuda.device(q.device):
-        check(_lib.lib().cdssm_b200_decode_step_strided(
-            _p(state), _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(v_first), _p(mix), _p(g),
-            g.stride(0), _p(lds), _p(rf),
-            _p(y), gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps, shortcut_scale, B, H, D, N, pos_i,
-            _p(pos_dev), _dtype_code(q), _stream()), "decode_step")
-    return y
+    return _lib.host().decode_step(state, q, k, v, gate_raw, log_dt_scale, rope_freqs, gating_c, omega_thresh, adt_delta,
+                                   adt_smoothness, adt_eps, n_heads, state_dim, pos, shortcut_scale, out, v_first, mix)
 
 
 def reference_decode_state(carry: Tensor, dtype=torch.bfloat16):
@@ -509,15 +424,14 @@ def scan_fused_status(device=None) -> int:
     0 means every bounded device-side wait of the tensor-core kernel completed; anything else is
     the code of the wait that ran out, and that call's outputs are undefined."""
     import ctypes
-    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    buf = _workspaces.get(key)
-    if buf is None:
+    device = torch.device("cuda" if device is None else device)
+    index = torch.cuda.current_device() if device.index is None else device.index
+    ptr = _lib.host().workspace_address(index)
+    if ptr == 0:
         return 0
     out = ctypes.c_int(0)
-    ptr = buf.data_ptr() + ((-buf.data_ptr()) % 256)
-    with torch.cuda.device(device):
-        rc = _lib.lib().cdssm_b200_scan_fused_status(ptr, ctypes.addressof(out), key[1])
+    with torch.cuda.device(index):
+        rc = _lib.lib().cdssm_b200_scan_fused_status(ptr, ctypes.addressof(out), _stream())
     if rc not in (0, -5):
         check(rc, "scan_fused_status")
     return out.value
@@ -525,14 +439,7 @@ def scan_fused_status(device=None) -> int:
 
 def rms_norm(x: Tensor, weight: Tensor, eps: float) -> Tensor:
     """RMSNorm over the last dimension in one kernel (cdssm/models/modules.py:50-53)."""
-    x = _prep(x, name="x")
-    w = _prep(weight, dtype=x.dtype, name="weight")
-    d = x.shape[-1]
-    out = torch.empty_like(x)
-    with torch.cuda.device(x.device):
-        check(_lib.lib().cdssm_b200_rmsnorm_fwd(_p(x), _p(w), _p(out), x.numel() // d, d, float(eps),
-                                                _dtype_code(x), _stream()), "rmsnorm_fwd")
-    return out
+    return _lib.host().rms_norm(x, weight, eps)
 
 
 def groupnorm_gate(y: Tensor, gn_weight: Tensor, gn_bias: Tensor, z: Tensor, skip: Tensor, x_conv: Tensor,
@@ -541,45 +448,13 @@ def groupnorm_gate(y: Tensor, gn_weight: Tensor, gn_bias: Tensor, z: Tensor, ski
     (statistics over channels x all positions, as the reference takes them) or, with per_token=True, in one
     (statistics per token: the causal form used with a decode cache).  z may be a column slice of a wider
     projection (rows strided)."""
-    y = _prep(y, name="y")
-    xc = _prep(x_conv, dtype=y.dtype, name="x_conv")
-    B, L, di = y.shape
-    if not z.is_cuda or z.dtype != y.dtype or tuple(z.shape) != (B, L, di) or z.stride(-1) != 1 or \
-            (L > 1 and z.stride(0) != L * z.stride(1)):
-        z = z.contiguous()
-    zs = z.stride(1) if L > 1 else (z.stride(0) if B > 1 else di)
-    if (zs * z.element_size()) % 16 or z.data_ptr() % 16:      # the kernel reads 16-byte pieces
-        z, zs = z.contiguous(), di
-    gw, gb, sk = (_prep(t, dtype=y.dtype, name="groupnorm parameter") for t in (gn_weight, gn_bias, skip))
-    out = torch.empty_like(y)
-    with torch.cuda.device(y.device):
-        stats = None
-        if not per_token:
-            n_stats = int(_lib.lib().cdssm_b200_groupnorm_stats_floats(B, L, int(groups)))
-            stats = torch.empty(n_stats, dtype=torch.float32, device=y.device)   # results first, then scratch
-            check(_lib.lib().cdssm_b200_groupnorm_stats(_p(y), _p(stats), B, L, di, int(groups), float(eps),
-                                                        _dtype_code(y), _stream()), "groupnorm_stats")
-        check(_lib.lib().cdssm_b200_groupnorm_gate_fwd(_p(y), _p(stats), _p(gw), _p(gb), _p(z), zs, _p(sk), _p(xc),
-                                                       _p(out), B, L, di, int(groups), float(eps), _dtype_code(y),
-                                                       _stream()), "groupnorm_gate_fwd")
-    return out
+    return _lib.host().groupnorm_gate(y, gn_weight, gn_bias, z, skip, x_conv, groups, eps, per_token)
 
 
 def conv1d_silu_step(x: Tensor, hist: Tensor, weight: Tensor, bias: Tensor) -> Tensor:
     """One position of the causal depthwise conv + SiLU: x (B,Dm) (rows may be strided), hist (B,3,Dm) the last
     three inputs, shifted in place.  Returns (B,Dm)."""
-    if not x.is_cuda or x.stride(-1) != 1:
-        x = x.contiguous()
-    B, Dm = x.shape
-    if hist.dtype != x.dtype or not hist.is_contiguous() or tuple(hist.shape) != (B, 3, Dm):
-        raise CdssmError("conv1d_silu_step: hist must be a contiguous (B,3,Dm) tensor of the input dtype")
-    w = _prep(weight, dtype=x.dtype, name="weight")
-    b = _prep(bias, dtype=x.dtype, name="bias")
-    out = torch.empty(B, Dm, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        check(_lib.lib().cdssm_b200_conv1d_silu_step(_p(x), x.stride(0) if B > 1 else Dm, _p(hist), _p(w), _p(b),
-                                                     _p(out), B, Dm, _dtype_code(x), _stream()), "conv1d_silu_step")
-    return out
+    return _lib.host().conv1d_silu_step(x, hist, weight, bias)
 
 
 def set_wait_limit_ns(limit_ns: int) -> int:
@@ -619,7 +494,7 @@ def scan_summary(k: Tensor, v: Tensor, gate_raw: Tensor, log_dt_scale: Tensor, r
     if B * L == 0:
         return (carry if h0 is None else h0.clone()), decay
     with torch.cuda.device(k.device):
-        ws_ptr, ws_bytes = _workspace(k.device, scan_fused_workspace_bytes(B, L, H, D, N, C))
+        ws_ptr, ws_bytes = _workspace(k, scan_fused_workspace_bytes(B, L, H, D, N, C))
         check(_lib.lib().cdssm_b200_scan_summary_fwd(
             _p(k), _p(v), _p(g), _p(lds), _p(rf), _p(h0), _p(carry), _p(decay), ws_ptr, ws_bytes, gating_c,
             omega_thresh, adt_delta, adt_smoothness, adt_eps, B, L, H, D, N, C, int(pos0), int(segs),
