@@ -1,0 +1,215 @@
+// One decode step of one (sequence, head, complex pair) by eight lanes: dynamics, normalised q and k, one delta-rule step
+// on the float32 state in place, read-out.  Shared by the stand-alone step kernel (scan_simt.cu) and the whole-model step
+// (lm_decode.cu).
+#pragma once
+#include "cdssm_common.cuh"
+
+namespace cdssm {
+
+constexpr int kLanesPerUnit = 8;
+
+template <int kLanes = 8>
+__device__ __forceinline__ float group_sum(float v) {   // sum over the kLanes (8 or 16) lanes of a unit
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    if (kLanes == 16) v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v;
+}
+
+// Raw (storage-typed) slice of one row: kCols contiguous columns starting at g*kCols.
+template <typename T, int kCols> struct RowSlice;
+template <int kCols> struct RowSlice<__nv_bfloat16, kCols> {
+    uint4 v[kCols / 8];
+    __device__ __forceinline__ void load(const __nv_bfloat16* row, int g, int D, bool vec) {
+        if (vec) {
+            const uint4* p = reinterpret_cast<const uint4*>(row + g * kCols);
+#pragma unroll
+            for (int i = 0; i < kCols / 8; i++) v[i] = __ldg(p + i);
+        } else {
+            unsigned short* s = reinterpret_cast<unsigned short*>(v);
+#pragma unroll
+            for (int i = 0; i < kCols; i++) {
+                const int d = g * kCols + i;
+                s[i] = d < D ? __ldg(reinterpret_cast<const unsigned short*>(row) + d) : (unsigned short)0;
+            }
+        }
+    }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < kCols / 8; i++) v[i] = make_uint4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ void get(float* f) const {
+#pragma unroll
+        for (int i = 0; i < kCols / 8; i++) unpack8(v[i], f + 8 * i);
+    }
+};
+template <int kCols> struct RowSlice<float, kCols> {
+    float4 v[kCols / 4];
+    __device__ __forceinline__ void load(const float* row, int g, int D, bool vec) {
+        if (vec) {
+            const float4* p = reinterpret_cast<const float4*>(row + g * kCols);
+#pragma unroll
+            for (int i = 0; i < kCols / 4; i++) v[i] = __ldg(p + i);
+        } else {
+            float* s = reinterpret_cast<float*>(v);
+#pragma unroll
+            for (int i = 0; i < kCols; i++) {
+                const int d = g * kCols + i;
+                s[i] = d < D ? __ldg(row + d) : 0.f;
+            }
+        }
+    }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < kCols / 4; i++) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __device__ __forceinline__ void get(float* f) const {
+        const float* s = reinterpret_cast<const float*>(v);
+#pragma unroll
+        for (int i = 0; i < kCols; i++) f[i] = s[i];
+    }
+};
+
+// x * rsqrt(sum x^2 + 1e-6) over the unit's row, rounded like the reference's K_norm/Q_norm
+// store (normalize_kq.cu:72-79).
+template <typename T, int kCols>
+__device__ __forceinline__ void normalise(float* f) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kCols; i++) ss += f[i] * f[i];
+    const float inv = rsqrtf(group_sum(ss) + kEps);
+#pragma unroll
+    for (int i = 0; i < kCols; i++) f[i] = IO<T>::rnd(f[i] * inv);
+}
+
+// One-token decode step: one pass over the state (read + write), everything else is a few hundred bytes per head.
+struct DecodeUnitArgs {
+    float* state;                  // (B,H,N,D)
+    const void *q, *k, *v, *gate;  // rows with their own strides (column slices of a wider projection), in elements
+    long long q_stride, k_stride, v_stride, gate_stride;
+    const void *v_first, *mix;     // or NULL: v <- lerp(v_first, v, mix[head]) (value residual)
+    long long v_first_stride;
+    const float *log_dt_scale, *rope_freqs;
+    void* y;                       // (B,H,N)
+    DynConsts dc;
+    float shortcut_scale;
+    int H, D, N, pos;
+    long long units;               // B*H*N/2
+};
+
+// Unit u of this thread's group of eight lanes; the whole warp calls together (units past the end take part in the
+// shuffles and write nothing).
+template <typename T, int kCols>
+__device__ __forceinline__ void decode_unit(const DecodeUnitArgs& a, long long u) {
+    const int g = threadIdx.x % kLanesPerUnit;
+    const bool active = u < a.units;
+    if (!active) u = a.units - 1;
+    const int NH = a.N >> 1, D = a.D, H = a.H;
+    const int j = (int)(u % NH);
+    const int hd = (int)((u / NH) % H);
+    const long long b = u / ((long long)NH * H);
+    const bool vec = (D == kCols * kLanesPerUnit);
+    const long long bh = b * H + hd;
+
+    RowSlice<T, kCols> kraw, qraw;
+    kraw.load(static_cast<const T*>(a.k) + b * a.k_stride + (long long)hd * D, g, D, vec);
+    qraw.load(static_cast<const T*>(a.q) + b * a.q_stride + (long long)hd * D, g, D, vec);
+    float* st = a.state + (bh * a.N + 2 * j) * D;
+    float zr[kCols], zi[kCols];
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < kCols / 4; i++) {
+            const float4 x = *reinterpret_cast<const float4*>(st + g * kCols + 4 * i);
+            const float4 w = *reinterpret_cast<const float4*>(st + D + g * kCols + 4 * i);
+            zr[4 * i] = x.x; zr[4 * i + 1] = x.y; zr[4 * i + 2] = x.z; zr[4 * i + 3] = x.w;
+            zi[4 * i] = w.x; zi[4 * i + 1] = w.y; zi[4 * i + 2] = w.z; zi[4 * i + 3] = w.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kCols; i++) {
+            const int d = g * kCols + i;
+            zr[i] = d < D ? st[d] : 0.f;
+            zi[i] = d < D ? st[D + d] : 0.f;
+        }
+    }
+    // dynamics (every lane of the unit computes the same scalars; dynamics_fused.cu:64-139)
+    const T* gr = static_cast<const T*>(a.gate) + b * a.gate_stride;
+    const T* s5 = gr + a.N * H;
+    const float freq = a.rope_freqs[hd], pos = (float)a.pos;
+    DynShared ds = dyn_shared<IO<T>::kBf16>(IO<T>::ld(gr + hd), IO<T>::ld(gr + NH * H + hd), IO<T>::ld(s5 + hd),
+                              IO<T>::ld(s5 + H + hd), IO<T>::ld(s5 + 2 * H + hd),
+                              IO<T>::ld(s5 + 3 * H + hd), IO<T>::ld(s5 + 4 * H + hd),
+                              a.log_dt_scale[hd], freq, pos, a.dc);
+    float a_re, a_im, vp;
+    dyn_pair<IO<T>::kBf16>(IO<T>::ld(gr + j * H + hd), IO<T>::ld(gr + (NH + j) * H + hd), freq, pos, ds, a_re, a_im, vp);
+    a_re = IO<T>::rnd(a_re);
+    a_im = IO<T>::rnd(a_im);
+    vp = IO<T>::rnd(vp);
+    const float be = IO<T>::rnd(ds.beta), sc = IO<T>::rnd(ds.sel_c);
+    const T* vrow = static_cast<const T*>(a.v) + b * a.v_stride + (long long)hd * a.N + 2 * j;
+    float v0 = IO<T>::ld(vrow), v1 = IO<T>::ld(vrow + 1);
+    if (a.v_first) {   // value residual across layers (block.py:167-171), rounded like the eager lerp's output
+        const T* f = static_cast<const T*>(a.v_first) + b * a.v_first_stride + (long long)hd * a.N + 2 * j;
+        const float w = IO<T>::ld(static_cast<const T*>(a.mix) + hd), f0 = IO<T>::ld(f), f1 = IO<T>::ld(f + 1);
+        const float d0 = v0 - f0, d1 = v1 - f1;
+        v0 = IO<T>::rnd(fabsf(w) < 0.5f ? f0 + w * d0 : v0 - d0 * (1.f - w));
+        v1 = IO<T>::rnd(fabsf(w) < 0.5f ? f1 + w * d1 : v1 - d1 * (1.f - w));
+    }
+    const float vr = IO<T>::rnd(v0 * vp), vi = IO<T>::rnd(v1 * vp);
+
+    float kk[kCols], qq[kCols];
+    kraw.get(kk);
+    qraw.get(qq);
+    normalise<T, kCols>(kk);
+    normalise<T, kCols>(qq);
+    float ur = 0.f, ui = 0.f;
+#pragma unroll
+    for (int i = 0; i < kCols; i++) { ur += zr[i] * kk[i]; ui += zi[i] * kk[i]; }
+    ur = be * group_sum(ur);
+    ui = be * group_sum(ui);
+    const float ivr = be * vr, ivi = be * vi;
+    float yr = 0.f, yi = 0.f;
+#pragma unroll
+    for (int i = 0; i < kCols; i++) {
+        const float er = zr[i] - ur * kk[i], ei = zi[i] - ui * kk[i];
+        zr[i] = a_re * er - a_im * ei + ivr * kk[i];
+        zi[i] = a_re * ei + a_im * er + ivi * kk[i];
+        yr += zr[i] * qq[i];
+        yi += zi[i] * qq[i];
+    }
+    yr = group_sum(yr);
+    yi = group_sum(yi);
+    if (a.shortcut_scale != 0.f) {
+        float qk = 0.f;
+#pragma unroll
+        for (int i = 0; i < kCols; i++) qk += qq[i] * kk[i];
+        qk = group_sum(qk);
+        const float f = a.shortcut_scale * qk * qk;
+        yr += f * vr;
+        yi += f * vi;
+    }
+    if (!active) return;
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < kCols / 4; i++) {
+            *reinterpret_cast<float4*>(st + g * kCols + 4 * i) =
+                make_float4(zr[4 * i], zr[4 * i + 1], zr[4 * i + 2], zr[4 * i + 3]);
+            *reinterpret_cast<float4*>(st + D + g * kCols + 4 * i) =
+                make_float4(zi[4 * i], zi[4 * i + 1], zi[4 * i + 2], zi[4 * i + 3]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kCols; i++) {
+            const int d = g * kCols + i;
+            if (d < D) { st[d] = zr[i]; st[D + d] = zi[i]; }
+        }
+    }
+    if (g == 0) {
+        T* o = static_cast<T*>(a.y) + bh * a.N + 2 * j;
+        IO<T>::st(o, IO<T>::rnd(yr) * sc);
+        IO<T>::st(o + 1, IO<T>::rnd(yi) * sc);
+    }
+}
+
+}  // namespace cdssm

@@ -4,6 +4,7 @@
 #include "host.h"
 
 #include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 
 namespace cdssm_host {
 namespace {
@@ -33,11 +34,13 @@ struct Plan {
     Dyn dyn;
     Tensor embedding, final_norm_w;
     std::vector<Block> blocks;
+    bool small_batch_ok = false;   // bf16, dense and 16-byte aligned: what the fused decode kernels read
 };
 
 constexpr double kFinalEps = 1.0 / 16384;   // 2^-14
 constexpr double kGroupEps = 1e-5;
 constexpr int64_t kHeadDim = 64;
+constexpr int64_t kGraphBatch = 32;
 
 const char* kCapsule = "cdssm_lm_plan";
 Plan& plan_of(PyObject* o) {
@@ -120,6 +123,39 @@ void block_step(Plan& p, Block& b, const Tensor& x, Tensor& v_first, const Tenso
     x.view({B, p.d_model}).addmm_(o.view({B, di}), b.w_out_t);
 }
 
+bool aligned_dense(const Tensor& t, at::ScalarType dt) {
+    return t.is_cuda() && t.scalar_type() == dt && t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0;
+}
+
+// The whole step by the small-batch kernels (csrc/lm_decode.cu); false where they do not apply.
+bool decode_small_batch(Plan& p, const Tensor& x, const std::vector<Cache>& caches, const Tensor& logits, int64_t pos,
+                        const Tensor& pos_dev) {
+    const int64_t B = x.size(0), V = p.embedding.size(0);
+    if (!p.small_batch_ok) return false;
+    // replayed from a graph, the library's products are not held up by their launches: see lm_decode_takes()
+    if (B > kGraphBatch && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return false;
+    const size_t bytes = cdssm_b200_lm_decode_workspace_bytes((int)B, (int)p.d_model, (int)p.N, (int)p.groups, (int)V, CDSSM_BF16);
+    if (bytes == 0) return false;
+    std::vector<cdssm_lm_layer> layers(p.blocks.size());
+    for (size_t i = 0; i < layers.size(); i++) {
+        const Cache& c = caches[i];
+        if (!aligned_dense(c.state, at::kFloat) || !aligned_dense(c.conv, at::kBFloat16) ||
+            c.state.sizes() != at::IntArrayRef({B, p.heads, p.N, kHeadDim}) || c.conv.sizes() != at::IntArrayRef({B, 3, p.d_inner}))
+            return false;
+        Block& b = p.blocks[i];
+        layers[i] = {cptr(b.norm_w), cptr(b.w_in), cptr(b.b_in), cptr(b.conv_w), cptr(b.conv_b), cptr(b.w_qg), cptr(b.b_qg),
+                     fptr(b.lds), fptr(b.rope), cptr(b.residual_mix(at::kBFloat16)), cptr(b.w_readout), cptr(b.gn_w),
+                     cptr(b.gn_b), cptr(b.D), cptr(b.w_out), (float)b.shortcut, mptr(c.state), mptr(c.conv)};
+    }
+    const Tensor ws = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
+    check(cdssm_b200_lm_decode(layers.data(), (int)layers.size(), mptr(x), cptr(p.final_norm_w), cptr(p.embedding), mptr(logits),
+                               mptr(ws), bytes, (float)p.eps_norm, (float)kGroupEps, (float)kFinalEps, p.dyn.c[0], p.dyn.c[1],
+                               p.dyn.c[2], p.dyn.c[3], p.dyn.c[4], (int)B, (int)p.d_model, (int)p.N, (int)p.groups, (int)V,
+                               (int)pos, static_cast<const int*>(cptr(pos_dev)), CDSSM_BF16, stream_of(x)),
+          "lm_decode");
+    return true;
+}
+
 Tensor embed(const Plan& p, const Tensor& ids) { return at::index(p.embedding, {std::optional<Tensor>(ids)}); }
 Tensor head(const Plan& p, const Tensor& x) { return at::linear(rms_norm(x, p.final_norm_w, kFinalEps), p.embedding); }
 
@@ -156,8 +192,15 @@ PyObject* py_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
             b.w_k = rows(b.w_in, 2 * di, 3 * di); b.b_k = rows(b.b_in, 2 * di, 3 * di);
             b.w_v = rows(b.w_in, 3 * di, b.w_in.size(0)); b.b_v = rows(b.b_in, 3 * di, b.b_in.size(0));
             b.w_out_t = b.w_out.t();
+            bool ok = aligned_dense(b.lds, at::kFloat) && aligned_dense(b.rope, at::kFloat);
+            for (const Tensor* w : {&b.norm_w, &b.w_in, &b.b_in, &b.conv_w, &b.conv_b, &b.w_qg, &b.b_qg, &b.w_readout, &b.w_out,
+                                    &b.gn_w, &b.gn_b, &b.D})
+                ok = ok && aligned_dense(*w, at::kBFloat16);
+            p->small_batch_ok = (i == 0 || p->small_batch_ok) && ok;
             p->blocks.push_back(std::move(b));
         }
+        p->small_batch_ok = p->small_batch_ok && aligned_dense(p->embedding, at::kBFloat16) &&
+                            aligned_dense(p->final_norm_w, at::kBFloat16);
         return PyCapsule_New(p.release(), kCapsule, [](PyObject* o) {
             delete static_cast<Plan*>(PyCapsule_GetPointer(o, kCapsule));
         });
@@ -223,7 +266,14 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const NoGrad ng;
         const c10::cuda::CUDAGuard guard(p.embedding.device());
         const int64_t B = ids.size(0);
-        Tensor x = embed(p, ids).view({B, 1, p.d_model}), v_first;
+        if (pos_dev.defined() && (pos_dev.scalar_type() != at::kInt || !pos_dev.is_cuda()))
+            throw Error("a tensor position must be an int32 CUDA tensor");
+        Tensor x = embed(p, ids).view({B, p.d_model}), v_first;
+        if (p.small_batch_ok) {
+            const Tensor logits = at::empty({B, p.embedding.size(0)}, x.options());
+            if (decode_small_batch(p, x, caches, logits, pos, pos_dev)) return wrap(logits);
+        }
+        x = x.view({B, 1, p.d_model});
         for (size_t i = 0; i < layers; i++) block_step(p, p.blocks[i], x, v_first, caches[i].state, caches[i].conv, pos, pos_dev);
         return wrap(head(p, x.view({B, p.d_model})));
     });

@@ -340,6 +340,13 @@ __device__ __forceinline__ bool elect_one_sync() {
     return e != 0;
 }
 
+// ---- asynchronous 16-byte copies global -> shared (zero fill where `on` is false; the address must still be valid)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---- warp-level matrix instructions (the skinny products with the running state) ---------------
 // Four 8x8 bf16 matrices from shared memory; lane l supplies the address of row (l & 7) of matrix (l >> 3).
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {

@@ -360,6 +360,36 @@ CDSSM_API int cdssm_b200_decode_step_strided(float* state, const void* q, int64_
                                              float shortcut_scale, int B, int H, int D, int N, int pos,
                                              const int* pos_dev, int dtype, void* stream);
 
+/* One decode step of the whole language model for a small batch (bf16 weights and activations, float32 states): per
+ * layer RMSNorm -> in-projection -> one-token conv + SiLU -> Q and gates -> recurrent step -> read-out -> GroupNorm per
+ * token, silu(z) gate, D * x_conv -> out-projection with the residual; then the final RMSNorm and the logits.
+ * layers: HOST array of n_layers; every pointer in it is a device pointer, rows of the weight matrices and all vectors
+ * 16-byte aligned.  x (B,d_model): the embedded tokens, overwritten (the residual stream); head_w (vocab,d_model);
+ * logits (B,vocab).  state and conv of every layer are updated in place, pos as in cdssm_b200_decode_step_strided.
+ * head_dim is 64, d_inner 2 * d_model, heads d_inner / 64 (cdssm/config/model.py:59-62).
+ * cdssm_b200_lm_decode_workspace_bytes is 0 where the sizes are outside what these kernels take.
+ * The reference has no decode step (see cdssm_b200_decode_step); layer structure cdssm/models/block.py:140-229. */
+typedef struct cdssm_lm_layer {
+    const void *norm_w, *w_in, *b_in;      /* (d), (3 di + H N, d), (3 di + H N): rows z | conv input | k | v */
+    const void *conv_w, *conv_b;           /* (di,1,4), (di) */
+    const void *w_qg, *b_qg;               /* (di + (N+5) H, di), (di + (N+5) H): rows q | gates */
+    const float *log_dt_scale, *rope_freqs;/* (H) */
+    const void* mix;                       /* (H): sigmoid(v_residual_gate); unused in layer 0 */
+    const void* w_readout;                 /* (di, H N) */
+    const void *gn_w, *gn_b, *skip;        /* (di) */
+    const void* w_out;                     /* (d, di) */
+    float shortcut_scale;
+    void* state;                           /* (B,H,N,64) float32 */
+    void* conv;                            /* (B,3,di) */
+} cdssm_lm_layer;
+CDSSM_API size_t cdssm_b200_lm_decode_workspace_bytes(int B, int d_model, int state_dim, int groups, int vocab, int dtype);
+CDSSM_API int cdssm_b200_lm_decode(const cdssm_lm_layer* layers, int n_layers, void* x, const void* final_norm_w,
+                                   const void* head_w, void* logits, void* workspace, size_t workspace_bytes,
+                                   float eps_norm, float eps_group, float eps_final, float gating_c, float omega_thresh,
+                                   float adt_delta, float adt_smoothness, float adt_eps, int B, int d_model,
+                                   int state_dim, int groups, int vocab, int pos, const int* pos_dev, int dtype,
+                                   void* stream);
+
 /* One-token decode step that reproduces the reference's CHUNKED scan (whose outputs beyond the first chunk are
  * not those of the plain recurrence): the state per (batch, head) is the local state (zero at every chunk
  * start), the correction (starts from the bf16-rounded carry; erased and rotated, never injected; read BEFORE
