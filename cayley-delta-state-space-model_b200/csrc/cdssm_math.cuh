@@ -105,6 +105,15 @@ __device__ __forceinline__ void dyn_pair(float alpha_raw, float omega_raw, float
     vp = fminf(sqrtf(fmaxf(1.0f - eff, kEps)), 1.0f);
 }
 
+// s <- gamma s + l, real and imaginary part.  A fixed operation order: the carry pass and the kernel that hands the carry on
+// itself give the same bits, so results do not depend on which of them a length happens to take.
+__device__ __forceinline__ float carry_re(float gr, float gi, float sr, float si, float l) {
+    return __fmaf_rn(gr, sr, __fmaf_rn(-gi, si, l));
+}
+__device__ __forceinline__ float carry_im(float gr, float gi, float sr, float si, float l) {
+    return __fmaf_rn(gr, si, __fmaf_rn(gi, sr, l));
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

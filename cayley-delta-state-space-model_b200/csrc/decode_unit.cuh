@@ -17,7 +17,8 @@ __device__ __forceinline__ float group_sum(float v) {   // sum over the kLanes (
     return v;
 }
 
-// Raw (storage-typed) slice of one row: kCols contiguous columns starting at g*kCols.
+// Raw (storage-typed) slice of one row: kCols contiguous columns starting at g*kCols.  (Plain loads: kernels that start
+// before their predecessor has finished must not move them above the wait, which __ldg would allow.)
 template <typename T, int kCols> struct RowSlice;
 template <int kCols> struct RowSlice<__nv_bfloat16, kCols> {
     uint4 v[kCols / 8];
@@ -25,13 +26,13 @@ template <int kCols> struct RowSlice<__nv_bfloat16, kCols> {
         if (vec) {
             const uint4* p = reinterpret_cast<const uint4*>(row + g * kCols);
 #pragma unroll
-            for (int i = 0; i < kCols / 8; i++) v[i] = __ldg(p + i);
+            for (int i = 0; i < kCols / 8; i++) v[i] = p[i];
         } else {
             unsigned short* s = reinterpret_cast<unsigned short*>(v);
 #pragma unroll
             for (int i = 0; i < kCols; i++) {
                 const int d = g * kCols + i;
-                s[i] = d < D ? __ldg(reinterpret_cast<const unsigned short*>(row) + d) : (unsigned short)0;
+                s[i] = d < D ? reinterpret_cast<const unsigned short*>(row)[d] : (unsigned short)0;
             }
         }
     }
@@ -50,13 +51,13 @@ template <int kCols> struct RowSlice<float, kCols> {
         if (vec) {
             const float4* p = reinterpret_cast<const float4*>(row + g * kCols);
 #pragma unroll
-            for (int i = 0; i < kCols / 4; i++) v[i] = __ldg(p + i);
+            for (int i = 0; i < kCols / 4; i++) v[i] = p[i];
         } else {
             float* s = reinterpret_cast<float*>(v);
 #pragma unroll
             for (int i = 0; i < kCols; i++) {
                 const int d = g * kCols + i;
-                s[i] = d < D ? __ldg(row + d) : 0.f;
+                s[i] = d < D ? row[d] : 0.f;
             }
         }
     }

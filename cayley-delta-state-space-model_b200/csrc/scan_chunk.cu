@@ -1,0 +1,1145 @@
+// The scan on tensor cores: bf16 storage, head_dim D = chunk C in {64, 128}, any even state_dim N <= 16, any head count.
+//
+// One thread block owns one chunk of one head, warp w its 32-token block w.  With g_t the coefficient that the step at
+// token t adds along k_t (raw keys; n_t = 1/|k_t|, c_t = beta_t n_t^2, W_t = a_0 ... a_t),
+//     local state     z_t = W_t sum_{i<=t} (g_i / W_i) k_i,   g_t = beta_t n_t v_t - c_t W_t sum_{i<t} (g_i / W_i) G[t,i]
+//     correction      r_t = W_t (r_0 - sum_{i<=t} h_i k_i),   h_t = c_t (k_t.r_0) - c_t sum_{i<t} h_i G[t,i]
+//     read-out        y_t ~ W_t sum_{i<=t} (g_i / W_i) P[t,i]  +  W_{t-1} (q_t.r_0 - sum_{i<t} h_i P[t,i])
+// with G = K K^T, P = Q K^T.  In the scaled unknowns g_i / W_i and h_i both systems have the same REAL unit lower
+// triangular matrix I + M, M[t,i] = c_t G[t,i], for every complex pair of the head: the pairs are right-hand sides.  So
+//   - G and P are products of the chunk's tiles (mma.sync on ldmatrix fragments of the swizzled TMA tiles, lower triangle
+//     only), computed once per head and chunk whatever N is;
+//   - the two 16 x 16 diagonal blocks of a warp are inverted by substitution, a row per lane, all rows at once and
+//     independent of any state;
+//   - what is left of the serial chain is three 16-wide products per 32 tokens, passed from warp to warp;
+//   - everything with a right-hand side (cross-block terms, read-outs, K^T g, K r_0, Q r_0) is a product with n = 8
+//     columns {pair 2q: re hi, re lo, im hi, im lo, pair 2q+1: ...}; fp32 values enter as bf16 hi + lo (16 bits), on the
+//     matrix side too, accumulation is fp32.
+// The division by W_i only spans a 32-token block, relative to its middle (|W ratio| of 16 tokens >= 1e-30); values cross
+// blocks relative to the block ends, where all factors are plain products.  A (block, pair) that decays further is walked
+// step by step (slow_walk).
+//
+// The reference's carry s_{c+1} = gamma_c s_c + z_{C-1} (inter_chunk_scan.cu:73-83) is handed from block to block inside
+// the kernel: blocks take (chunk, batch, head) work in chunk-major order from a ticket counter, so the chunk a block waits
+// for is held by a block that started before it.  kLocal / kOutput are the two halves with the carry pass of scan_simt.cu
+// between them (summaries, and shapes whose chain of chunks is longer than their work: one_kernel_pays() there).
+//
+// Reference semantics (intra_chunk_scan.cu:100-195, exact_correction.cu:89-150): z starts at zero at the chunk start, r
+// from the bf16-rounded carry, the correction is read before its step.
+#include "cdssm_common.cuh"
+#include "sm100_ptx.cuh"
+#include "tile_map.cuh"
+
+namespace cdssm {
+using namespace sm100;
+
+namespace chunk {
+
+enum Mode { kLocal, kOutput, kFused };
+
+struct Args {
+    const float2* rec_a;         // (B,NC,H,NP,C): transition a_t
+    const uint32_t* rec_v;       // (B,NC,H,NP,C): vp-scaled v_t, bf16 pair
+    const uint32_t* rec_g;       // (B,NC,H,C): beta_t, sel_C, bf16 pair
+    const float* h0;
+    __nv_bfloat16* y;
+    float *final_state, *tail_state;
+    float* ws_gamma;             // (B,NC,H,NP,2): chunk decays (kLocal); kFused: first word of a unit = "carry is there"
+    float* ws_state;             // (B,NC,H,NP,2,D): z_{C-1} (kLocal), carry into the chunk (kOutput: rounded, kFused: not)
+    int *status, *ticket;
+    unsigned long long wait_ns;  // limit of every device-side wait
+    int withhold;                // test hook: nothing is loaded, so the first wait runs out
+    float shortcut_scale;
+    int B, L, H, N, NC;
+};
+
+struct cplx { float r, i; };
+__device__ __forceinline__ cplx cmul(cplx a, cplx b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
+__device__ __forceinline__ cplx cshfl(cplx v, int src) {
+    return {__shfl_sync(0xffffffffu, v.r, src), __shfl_sync(0xffffffffu, v.i, src)};
+}
+__device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+// x = hi + lo, hi = x truncated to bf16 and lo the (exact) rest truncated to bf16: 16 significant bits, integer and FMA
+// pipes only.  pair_hi / pair_lo: the two parts of two values; hi_lo: both parts of one value.
+__device__ __forceinline__ uint32_t pair_hi(float x0, float x1) { return __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632); }
+__device__ __forceinline__ float rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t pair_lo(float x0, float x1) { return pair_hi(rest(x0), rest(x1)); }
+__device__ __forceinline__ uint32_t hi_lo(float x) { return pair_hi(x, rest(x)); }
+__device__ __forceinline__ uint32_t movmatrix(uint32_t x) {   // 8 x 8 bf16 matrix, one row a quad, transposed
+    uint32_t y;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+__device__ __forceinline__ float bits_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+__device__ __forceinline__ float bits_lo(uint32_t w) { return __uint_as_float(w << 16); }
+
+template <int kD, int kPairs_>
+struct Geo {
+    static constexpr int kPairs = kPairs_;               // complex pairs held (>= N / 2)
+    static constexpr int kTiles = (kPairs + 1) / 2;      // column tiles of two pairs
+    static constexpr int kBlocks = kD / 32;              // warps: one per 32-token block
+    static constexpr int kThreads = 32 * kBlocks;
+    static constexpr int kSlabs = kD / 64, kKs = kD / 16;
+    static constexpr uint32_t kSlab = kD * 128;          // bytes of kD rows x 64 bf16 columns
+    static constexpr uint32_t kTile = kSlabs * kSlab;
+    // right-hand-side fragments of a 32-token block, published for others: g for every later block (rotated to its
+    // start) and for the chunk end, h for every later block and itself
+    static constexpr int kCross = kBlocks * (kBlocks - 1) / 2;
+    static constexpr int kSlots = kCross + 2 * kBlocks;
+    static __device__ __forceinline__ int slot_g(int from, int to) { return to * (to - 1) / 2 + from; }
+    static __device__ __forceinline__ int slot_end(int from) { return kCross + from; }
+    static __device__ __forceinline__ int slot_h(int from) { return kCross + kBlocks + from; }
+};
+
+struct BlockPair {   // of one 32-token block and pair
+    cplx A, R, D31;  // product of a over the block; product of its first half (the scaling's reference); D of the last token
+    int slow, pad;
+};
+
+union Scratch {   // of one warp, until the Q tile arrives in its place
+    float mt[2][16][20];                                 // the diagonal blocks of M, transposed
+    unsigned char t[32][80];                             // rows of the inverses, bf16 hi (32 B) | lo (32 B)
+};
+
+// (head_dim 128 with one pair: 74.2 KB, three blocks per SM)
+template <int kD, int kPairs, Mode kMode>
+struct __align__(1024) Smem {
+    using G = Geo<kD, kPairs>;
+    static constexpr int kLanes = kPairs == 1 ? 16 : 32; // a single pair fills half of the columns
+    uint8_t k[G::kTile];                                 // swizzled rows = tokens
+    union {
+        uint8_t q[kMode == kLocal ? 1024 : G::kTile];
+        Scratch scr[G::kBlocks];
+    };
+    uint2 frag[G::kSlots][G::kTiles][2][kLanes];         // [slot][tile][16-token half][lane]
+    float2 viw[kPairs][kD], dd[kPairs][kD];              // v / D, D
+    float beta[kD], sel[kD];
+    BlockPair bp[kPairs][G::kBlocks];
+    float s_in[2 * kPairs][kD];                          // carry into the chunk
+    __nv_bfloat16 r0[2 * kPairs][kD + 8];                // the same rounded (padded rows: fragment loads hit distinct banks)
+    float4 walk[G::kBlocks][32];                         // slow_walk results
+    __nv_bfloat16 y_[kPairs == 1 ? 1 : G::kBlocks][kPairs == 1 ? 1 : 32][2 * kPairs + 2];
+    // outputs of a warp on their way to one row a lane (with one pair: in place of its walk results)
+    __device__ __forceinline__ __nv_bfloat16* y(int block, int row) {
+        if constexpr (kPairs == 1) return reinterpret_cast<__nv_bfloat16*>(walk[block]) + row * 4;
+        else return y_[block][row];
+    }
+    uint64_t full_k, full_q;
+    int abort_flag, item, stop;
+    __device__ __forceinline__ void put(int slot, int tile, int half, int lane, uint2 f) {
+        if (kLanes == 32 || lane < 16) frag[slot][tile][half][lane & (kLanes - 1)] = f;
+    }
+    __device__ __forceinline__ uint2 get(int slot, int tile, int half, int lane) const {
+        const uint2 f = frag[slot][tile][half][lane & (kLanes - 1)];
+        return kLanes == 32 || lane < 16 ? f : make_uint2(0u, 0u);
+    }
+};
+
+// ---- dynamics ------------------------------------------------------------------------------------------------
+// dynamics_fused.cu:64-139 and the vp scale of block.py:194-195, every result rounded to bf16 like the reference's stores
+// (the transition optionally not).  The gates lie heads-fastest, the scan wants a head's tokens side by side: a block takes
+// 32 tokens of up to 32 heads, lane = head, and turns its results around in shared memory, so that both sides move whole
+// sectors.  Read where they are used, by the block of one head, each 2-byte gate costs a sector and a slot of the L1 miss
+// queue of its own (seven per token and head): the local pass at B 8, L 2048, H 24, D 64 took 52 us, of which this was 2/3.
+struct DynArgs {
+    const __nv_bfloat16 *v, *gate_raw;
+    const float *log_dt_scale, *rope_freqs;
+    float2* rec_a;
+    uint32_t *rec_v, *rec_g;
+    DynConsts dc;
+    int B, L, H, N, C, NC, pos0, segs, fp32_decay;
+};
+constexpr int kDynTokens = 32, kDynWarps = 8;
+__global__ void __launch_bounds__(32 * kDynWarps) dynamics_kernel(const DynArgs a) {
+    using T = __nv_bfloat16;
+    __shared__ float2 sa[32][kDynTokens + 1];
+    __shared__ uint32_t sv[32][kDynTokens + 1];
+    grid_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, H = a.H, N = a.N, NP = N >> 1;
+    const int head0 = blockIdx.y * 32, hd = head0 + lane, heads = min(32, H - head0);
+    const int tiles = (a.NC * a.C) / kDynTokens, b = blockIdx.x / tiles, l0 = (blockIdx.x % tiles) * kDynTokens;
+    const int c = l0 / a.C, in_chunk = l0 % a.C;
+    constexpr int kPer = kDynTokens / kDynWarps;
+    const bool on = lane < heads;
+    const float lds = on ? a.log_dt_scale[hd] : 0.f, freq = on ? a.rope_freqs[hd] : 0.f;
+    DynShared ds[kPer];
+    float g0[kPer], g1[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+        const int l = l0 + warp * kPer + i;
+        float x[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        g0[i] = g1[i] = 0.f;
+        if (on && l < a.L) {
+            const T* gr = a.gate_raw + ((size_t)b * a.L + l) * (size_t)((N + 5) * H) + hd;
+            g0[i] = IO<T>::ld(gr);
+            g1[i] = IO<T>::ld(gr + NP * H);
+#pragma unroll
+            for (int s = 0; s < 5; s++) x[s] = IO<T>::ld(gr + (N + s) * H);
+        }
+        const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
+        ds[i] = dyn_shared<true>(g0[i], g1[i], x[0], x[1], x[2], x[3], x[4], lds, freq, pos, a.dc);
+        // behind the sequence end a = 1, beta = v = 0: the state stands still
+        sv[lane][warp * kPer + i] = on && l < a.L ? pack2(ds[i].beta, ds[i].sel_c) : 0u;
+    }
+    const size_t unit0 = ((size_t)b * a.NC + c) * H + head0;
+    __syncthreads();
+    for (int h = warp; h < heads; h += kDynWarps) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sv[h][lane];
+    for (int p = 0; p < NP; p++) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            const int t = warp * kPer + i, l = l0 + t;
+            float2 at = make_float2(1.f, 0.f);
+            uint32_t vg = 0u;
+            if (on && l < a.L) {
+                const T* gr = a.gate_raw + ((size_t)b * a.L + l) * (size_t)((N + 5) * H) + hd;
+                const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
+                const float ga = p == 0 ? g0[i] : IO<T>::ld(gr + p * H), gw = p == 0 ? g1[i] : IO<T>::ld(gr + (NP + p) * H);
+                const uint32_t vv = *reinterpret_cast<const uint32_t*>(a.v + (((size_t)b * a.L + l) * H + hd) * N + 2 * p);
+                float ar, ai, vp;
+                dyn_pair<true>(ga, gw, freq, pos, ds[i], ar, ai, vp);
+                if (!a.fp32_decay) { ar = bfr(ar); ai = bfr(ai); }
+                vp = bfr(vp);
+                at = make_float2(ar, ai);
+                vg = pack2(bits_lo(vv) * vp, bits_hi(vv) * vp);
+            }
+            sa[lane][t] = at;
+            sv[lane][t] = vg;
+        }
+        __syncthreads();
+        for (int h = warp; h < heads; h += kDynWarps) {
+            const size_t o = ((unit0 + h) * NP + p) * a.C + in_chunk + lane;
+            a.rec_a[o] = sa[h][lane];
+            a.rec_v[o] = sv[h][lane];
+        }
+    }
+}
+
+// ---- fragments ------------------------------------------------------------------------------------------------
+// A (16 tokens x 16 columns, row-major) or, with registers {0,2} / {1,3}, two B fragments (8 tokens each)
+template <uint32_t kSlab>
+__device__ __forceinline__ uint32_t row_frag(uint32_t tile, int row0, int ks, int lane) {
+    const int row = row0 + (lane & 7) + ((lane >> 3) & 1) * 8, piece = (ks & 3) * 2 + (lane >> 4);
+    return tile + (uint32_t)(ks >> 2) * kSlab + (uint32_t)row * 128u + (uint32_t)((piece ^ (row & 7)) << 4);
+}
+// A fragment of the transposed tile: 16 columns x 16 tokens (for ldmatrix.trans)
+template <uint32_t kSlab>
+__device__ __forceinline__ uint32_t col_frag(uint32_t tile, int tok0, int col0, int lane) {
+    const int row = tok0 + (lane & 7) + ((lane >> 4) & 1) * 8, piece = ((col0 & 63) >> 3) + ((lane >> 3) & 1);
+    return tile + (uint32_t)(col0 >> 6) * kSlab + (uint32_t)row * 128u + (uint32_t)((piece ^ (row & 7)) << 4);
+}
+
+// acc[mt][nt] = rows row_a + 16 mt .. of tile A against rows row_b + 8 nt .. of tile B, 32 x 32
+template <int kD, int kPairs, bool kSame>
+__device__ __forceinline__ void gram_block(float (&acc)[2][4][4], uint32_t ta, int row_a, uint32_t tb, int row_b, int lane,
+                                           bool diagonal) {
+    using G = Geo<kD, kPairs>;
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[m][n][e] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < G::kKs; ks++) {
+        uint32_t a[2][4], b[2][4];
+        ldsm_x4(row_frag<G::kSlab>(ta, row_a, ks, lane), a[0]);
+        ldsm_x4(row_frag<G::kSlab>(ta, row_a + 16, ks, lane), a[1]);
+        if (!kSame) {
+            ldsm_x4(row_frag<G::kSlab>(tb, row_b, ks, lane), b[0]);
+            ldsm_x4(row_frag<G::kSlab>(tb, row_b + 16, ks, lane), b[1]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t(&bb)[4] = kSame ? a[h] : b[h];
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                if (m == 0 && h == 1 && diagonal) continue;   // above the diagonal
+                mma_bf16_m16n8k16(acc[m][2 * h], a[m], bb[0], bb[2]);
+                mma_bf16_m16n8k16(acc[m][2 * h + 1], a[m], bb[1], bb[3]);
+            }
+        }
+    }
+}
+
+// Diagonal elements of a 16 x 16 block held as two 16 x 8 accumulators: rows g and g + 8, handed to the whole quad.
+__device__ __forceinline__ void diagonal_of(const float (&n0)[4], const float (&n1)[4], int lane, float& d0, float& d1) {
+    const int g = lane >> 2, src = (lane & ~3) | (g >> 1);
+    const float x0 = (g & 1) ? n0[1] : n0[0], x1 = (g & 1) ? n1[3] : n1[2];
+    d0 = __shfl_sync(0xffffffffu, x0, src);
+    d1 = __shfl_sync(0xffffffffu, x1, src);
+}
+
+struct Split { uint32_t hi[4], lo[4]; };   // a 16 x 16 A fragment, bf16 hi + lo
+__device__ __forceinline__ Split split(const float (&n0)[4], const float (&n1)[4]) {
+    Split s;
+    s.hi[0] = pair_hi(n0[0], n0[1]); s.lo[0] = pair_lo(n0[0], n0[1]);
+    s.hi[1] = pair_hi(n0[2], n0[3]); s.lo[1] = pair_lo(n0[2], n0[3]);
+    s.hi[2] = pair_hi(n1[0], n1[1]); s.lo[2] = pair_lo(n1[0], n1[1]);
+    s.hi[3] = pair_hi(n1[2], n1[3]); s.lo[3] = pair_lo(n1[2], n1[3]);
+    return s;
+}
+__device__ __forceinline__ void mma_split(float (&d)[4], const Split& a, uint2 b) {
+    mma_bf16_m16n8k16(d, a.hi, b.x, b.y);
+    mma_bf16_m16n8k16(d, a.lo, b.x, b.y);
+}
+// values of rows g, g + 8 (this lane's complex component) as the B fragment of 16 tokens
+__device__ __forceinline__ uint2 rhs_frag(float x0, float x1) { return make_uint2(movmatrix(hi_lo(x0)), movmatrix(hi_lo(x1))); }
+
+// ---- decay scalings of a 32-token block and pair (lane = token) ---------------------------------------------------
+// The scaled unknowns need ratios of the prefix products W_t = a_0 ... a_t only, taken relative to the middle of the
+// block, D_t = W_t / W_15: lanes 0-15 hold the suffix product a_{t+1} ... a_15 = 1 / D_t, lanes 16-31 the prefix product
+// a_16 ... a_t = D_t, and neither half leaves the float range unless one half alone decays by more than 1e-30.
+__device__ __forceinline__ void scalings(cplx at, cplx vg, int tl, cplx& viw, cplx& D, BlockPair& bp) {
+    const bool lo = tl < 16;
+    cplx X = at;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const cplx other = cshfl(X, lo ? tl + o : tl - o);
+        if (lo ? (tl + o < 16) : (tl - o >= 16)) X = cmul(X, other);
+    }
+    const cplx R = cshfl(X, 0);                  // a_0 ... a_15
+    cplx E = cshfl(X, tl + 1);                   // first half: exclusive suffix = inclusive suffix of lane t + 1
+    if (tl == 15) E = {1.f, 0.f};
+    if (!lo) E = X;
+    const float m = fmaxf(fabsf(E.r), fabsf(E.i));
+    const bool in_range = m >= 1e-30f && m <= 1e30f;
+    const float sc1 = __fdividef(1.f, m);
+    const cplx En = {E.r * sc1, E.i * sc1};
+    const float q = __fdividef(sc1, En.r * En.r + En.i * En.i);
+    const cplx Einv = {En.r * q, -En.i * q};
+    D = lo ? Einv : E;
+    viw = cmul(vg, lo ? E : Einv);
+    const cplx D31 = cshfl(D, 31);
+    const float mr = fmaxf(fabsf(R.r), fabsf(R.i));
+    const bool fast = __all_sync(0xffffffffu, in_range && mr >= 1e-30f && mr <= 1e30f);
+    bp.A = cmul(D31, R);                         // both factors are plain products of a: valid for any a
+    bp.R = R;
+    bp.D31 = D31;
+    bp.slow = fast ? 0 : 1;
+    if (!fast) {   // the walk reads a and v themselves
+        viw = vg;
+        D = at;
+        bp.R = bp.D31 = {1.f, 0.f};
+    }
+}
+
+// Step-by-step walk of pair p over this warp's block, for decays the scaled form cannot hold: state columns over the
+// lanes.  kReadout: walk[t] = {q_t.z_t, W_{t-1} from the block start}, else {g_t carried to the block end}.  The incoming state is rebuilt from
+// the fragments the earlier blocks published for this one.
+template <int kD, int kPairs, Mode kMode, bool kReadout>
+__device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I, int tl) {
+    using G = Geo<kD, kPairs>;
+    constexpr int kCols = kD / 32;
+    auto column = [&](const uint8_t* tile, int row, int c) {
+        const int piece = (c & 63) >> 3;
+        const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(tile + (c >> 6) * G::kSlab + row * 128 + ((piece ^ (row & 7)) << 4));
+        return __bfloat162float(x[c & 7]);
+    };
+    float zr[kCols], zi[kCols];
+#pragma unroll
+    for (int i = 0; i < kCols; i++) zr[i] = zi[i] = 0.f;
+    for (int J = 0; J < I; J++)
+        for (int t = 0; t < 32; t++) {
+            const int half = t >> 4, r = t & 15, q = (r & 7) >> 1;
+            auto value = [&](int col) {
+                const uint2 f = sm.get(G::slot_g(J, I), p >> 1, half, col * 4 + q);
+                const uint32_t w = r >= 8 ? f.y : f.x;
+                return (r & 1) ? bits_hi(w) : bits_lo(w);
+            };
+            const int c0 = 4 * (p & 1);
+            const float wr = value(c0) + value(c0 + 1), wi = value(c0 + 2) + value(c0 + 3);
+#pragma unroll
+            for (int i = 0; i < kCols; i++) {
+                const float k = column(sm.k, 32 * J + t, tl + 32 * i);
+                zr[i] += wr * k;
+                zi[i] += wi * k;
+            }
+        }
+    cplx own = {0.f, 0.f};
+    for (int t = 0; t < 32; t++) {
+        const int row = 32 * I + t;
+        const float2 a = sm.dd[p][row], vg = sm.viw[p][row];
+        const float be = sm.beta[row];
+        float k[kCols], kk = 0.f, ur = 0.f, ui = 0.f;
+#pragma unroll
+        for (int i = 0; i < kCols; i++) {
+            k[i] = column(sm.k, row, tl + 32 * i);
+            kk += k[i] * k[i];
+            ur += zr[i] * k[i];
+            ui += zi[i] * k[i];
+        }
+        kk = warp_sum(kk); ur = warp_sum(ur); ui = warp_sum(ui);
+        const float n = rsqrtf(kk + kEps);
+        const cplx au = cmul({a.x, a.y}, {n * ur, n * ui});
+        const cplx gt = {be * n * (vg.x - au.r), be * n * (vg.y - au.i)};
+#pragma unroll
+        for (int i = 0; i < kCols; i++) {
+            const cplx z = cmul({a.x, a.y}, {zr[i], zi[i]});
+            zr[i] = z.r + gt.r * k[i];
+            zi[i] = z.i + gt.i * k[i];
+        }
+        if (kReadout) {
+            float yr = 0.f, yi = 0.f;
+#pragma unroll
+            for (int i = 0; i < kCols; i++) {
+                const float q = column(sm.q, row, tl + 32 * i);
+                yr += zr[i] * q;
+                yi += zi[i] * q;
+            }
+            yr = warp_sum(yr); yi = warp_sum(yi);
+            if (tl == t) own = {yr, yi};
+        } else if (tl == t) {
+            own = gt;
+        }
+    }
+    // g carried to the block end: times a_{t+1} ... a_31; W_{t-1} = a_0 ... a_{t-1}
+    const float2 a = sm.dd[p][32 * I + tl];
+    cplx S = {a.x, a.y};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int from = kReadout ? tl - o : tl + o;
+        const cplx other = cshfl(S, from);
+        if (from >= 0 && from < 32) S = cmul(S, other);
+    }
+    cplx V = cshfl(S, kReadout ? tl - 1 : tl + 1);
+    if (tl == (kReadout ? 0 : 31)) V = {1.f, 0.f};
+    if (!kReadout) own = cmul(V, own);
+    __syncwarp();
+    sm.walk[I][tl] = make_float4(own.r, own.i, V.r, V.i);
+    __syncwarp();
+}
+
+// resident blocks per SM the registers are cut for (more blocks spill: N 16, head_dim 64, 5 / 7 / 8 blocks: 279 / 308 / 328 us)
+template <int kD, int kPairs>
+constexpr int kMinBlocks = kD == 128 ? (kPairs == 1 ? 3 : 2) : (kPairs <= 2 ? 6 : 5);
+
+template <int kD, int kPairs, Mode kMode>
+__global__ void __launch_bounds__(Geo<kD, kPairs>::kThreads, kMinBlocks<kD, kPairs>)
+scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const Args a) {
+    using G = Geo<kD, kPairs>;
+    constexpr int kBlocks = G::kBlocks, kTiles = G::kTiles, kKs = G::kKs;
+    constexpr bool kOut = kMode != kLocal, kNeedEnd = kMode != kOutput;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    Smem<kD, kPairs, kMode>& sm = *reinterpret_cast<Smem<kD, kPairs, kMode>*>(smem_raw);
+    const int tid = threadIdx.x, I = tid >> 5, tl = tid & 31, g = tl >> 2, t4 = tl & 3;
+    const int H = a.H, N = a.N, NP = N >> 1, L = a.L;
+
+    if (tid == 0) {
+        mbar_init(&sm.full_k, 1);
+        mbar_init(&sm.full_q, 1);
+        sm.abort_flag = 0;
+        fence_barrier_init();
+        sm.item = kMode == kFused ? atomicAdd(a.ticket, 1) : (int)blockIdx.x;
+        sm.stop = *reinterpret_cast<volatile int*>(a.status);
+    }
+    __syncthreads();
+    if ((smem_u32(smem_raw) & 1023u) != 0) {   // the swizzled tiles need 1024-byte alignment
+        if (tid == 0) atomicCAS(a.status, 0, 399);
+        return;
+    }
+    if (sm.stop) return;   // an earlier block gave up
+    // chunk-major: every block that a block may wait for has an earlier ticket
+    const int item = sm.item, hd = item % H, b = (item / H) % a.B, c = item / (H * a.B);
+    const size_t unit = ((size_t)b * a.NC + c) * H + hd;       // workspace slot
+    const int Lc = min(kD, L - c * kD);
+    if (tid == 0 && !a.withhold) {
+        mbar_arrive_expect_tx(&sm.full_k, G::kTile);
+#pragma unroll
+        for (int s = 0; s < G::kSlabs; s++) tma_load_4d(sm.k + s * G::kSlab, &tmK, &sm.full_k, 64 * s, hd, c * kD, b);
+    }
+
+    // ---- carry into the chunk: this warp's 32 columns of every state row.  Already there (previous pass), or early if
+    // its producer is done; else polled for behind the products that do not need it.
+    const float* carry_src = a.ws_state + unit * (size_t)N * kD;
+    int* carry_flag = reinterpret_cast<int*>(a.ws_gamma + unit * (size_t)N);   // a bit per warp
+    auto flag_set = [&]() {
+        int v;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(carry_flag) : "memory");
+        return ((v >> I) & 1) != 0;
+    };
+    auto load_carry = [&](const float* src) {
+        const int col = 32 * I + 4 * (tl & 7);
+#pragma unroll
+        for (int n0 = 0; n0 < 2 * kPairs; n0 += 4) {
+            const int n = n0 + (tl >> 3);
+            if (n < 2 * kPairs) {
+                const bool on = src != nullptr && n < N;
+                cp_async16(&sm.s_in[n][col], on ? src + (size_t)n * kD + col : a.ws_state, on);
+            }
+        }
+        cp_async_commit();
+    };
+    bool have_carry = true;
+    if (kMode == kOutput) {
+        load_carry(carry_src);
+    } else if (kMode == kFused) {
+        if (c == 0) load_carry(a.h0 ? a.h0 + ((size_t)b * H + hd) * N * kD : nullptr);
+        else if ((have_carry = __all_sync(0xffffffffu, flag_set()))) load_carry(carry_src);
+    }
+    const bool k_here = mbar_wait_suspend(&sm.full_k, 0, &sm.abort_flag, a.wait_ns);
+    if (!__syncthreads_and(k_here)) {
+        if (tid == 0) atomicCAS(a.status, 0, 201);
+        cp_async_wait_all();
+        return;
+    }
+    const uint32_t kt = smem_u32(sm.k), qt = smem_u32(sm.q);
+
+    // ---- G: diagonal block, |k|^-1, inverses
+    float cc[4], bn[4], nrm[4];               // c_t, beta_t n_t, n_t of rows g, g + 8, g + 16, g + 24
+    Split T11, T22, M21;
+    Split M[kBlocks > 1 ? kBlocks - 1 : 1][2][2];
+    {
+        float acc[2][4][4];
+        gram_block<kD, kPairs, true>(acc, kt, 32 * I, kt, 32 * I, tl, true);
+        float kk[4];
+        diagonal_of(acc[0][0], acc[0][1], tl, kk[0], kk[1]);
+        diagonal_of(acc[1][2], acc[1][3], tl, kk[2], kk[3]);
+        // the token's dynamics, from the kernel before this one (its launch let this one start early; no __ldg here: loads
+        // that claim the data constant may be moved above the wait)
+        grid_dependency_wait();
+        {
+            const uint32_t gg = __ldcg(a.rec_g + unit * kD + tid);
+            const float2* ra = a.rec_a + unit * (size_t)NP * kD + tid;
+            const uint32_t* rv = a.rec_v + unit * (size_t)NP * kD + tid;
+            float2 at[kPairs];
+            uint32_t vg[kPairs];
+#pragma unroll
+            for (int p = 0; p < kPairs; p++) {
+                at[p] = p < NP ? __ldcg(ra + p * kD) : make_float2(1.f, 0.f);
+                vg[p] = p < NP ? __ldcg(rv + p * kD) : 0u;
+            }
+            sm.beta[tid] = bits_lo(gg);
+            sm.sel[tid] = bits_hi(gg);
+#pragma unroll
+            for (int p = 0; p < kPairs; p++) {   // parked where the results will go
+                sm.dd[p][tid] = at[p];
+                sm.viw[p][tid] = make_float2(bits_lo(vg[p]), bits_hi(vg[p]));
+            }
+#pragma unroll 1
+            for (int p = 0; p < kPairs; p++) {
+                const float2 x = sm.dd[p][tid], y = sm.viw[p][tid];
+                cplx viw, D;
+                BlockPair bp;
+                scalings({x.x, x.y}, {y.x, y.y}, tl, viw, D, bp);
+                sm.viw[p][tid] = make_float2(viw.r, viw.i);
+                sm.dd[p][tid] = make_float2(D.r, D.i);
+                if (tl == 0) sm.bp[p][I] = bp;
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const float be = sm.beta[32 * I + 8 * r + g];
+            nrm[r] = rsqrtf(kk[r] + kEps);
+            bn[r] = be * nrm[r];
+            cc[r] = bn[r] * nrm[r];
+        }
+        // strictly lower part of the two diagonal 16 x 16 blocks of M, transposed: mt[block][column][row]
+        auto& mt = sm.scr[I].mt;
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int row = g + 8 * (e >> 1), col = 8 * n + 2 * t4 + (e & 1);
+                    mt[m][col][row] = row > col ? cc[2 * m + (e >> 1)] * acc[m][2 * m + n][e] : 0.f;
+                }
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[1][n][e] *= cc[2 + (e >> 1)];
+        M21 = split(acc[1][0], acc[1][1]);
+        __syncwarp();
+        // row r of the inverse of I + M (lanes 0-15: first block, 16-31: second): T[r][j] = - sum_{i>j} T[r][i] M[i][j]
+        const int r = tl & 15, blk = tl >> 4;
+        float2 T2[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) T2[j] = make_float2(2 * j == r ? 1.f : 0.f, 2 * j + 1 == r ? 1.f : 0.f);
+#pragma unroll
+        for (int j = 14; j >= 0; j--) {
+            float2 s = make_float2(0.f, 0.f), s2 = s;
+#pragma unroll
+            for (int i4 = (j + 1) / 4; i4 < 4; i4++) {
+                const float4 mm = *reinterpret_cast<const float4*>(&mt[blk][j][4 * i4]);
+                s = __ffma2_rn(T2[2 * i4], make_float2(mm.x, mm.y), s);
+                s2 = __ffma2_rn(T2[2 * i4 + 1], make_float2(mm.z, mm.w), s2);
+            }
+            const float sum = (s.x + s.y) + (s2.x + s2.y);
+            if (j & 1) T2[j >> 1].y -= sum;
+            else T2[j >> 1].x -= sum;
+        }
+        __syncwarp();
+        uint32_t* row = reinterpret_cast<uint32_t*>(sm.scr[I].t[tl]);
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+            *reinterpret_cast<uint4*>(row + j) = make_uint4(pair_hi(T2[j].x, T2[j].y), pair_hi(T2[j + 1].x, T2[j + 1].y),
+                                                            pair_hi(T2[j + 2].x, T2[j + 2].y), pair_hi(T2[j + 3].x, T2[j + 3].y));
+            *reinterpret_cast<uint4*>(row + 8 + j) = make_uint4(pair_lo(T2[j].x, T2[j].y), pair_lo(T2[j + 1].x, T2[j + 1].y),
+                                                                pair_lo(T2[j + 2].x, T2[j + 2].y), pair_lo(T2[j + 3].x, T2[j + 3].y));
+        }
+        __syncwarp();
+        const uint32_t ts = smem_u32(sm.scr[I].t) + (uint32_t)((tl & 7) + ((tl >> 3) & 1) * 8) * 80u + (uint32_t)(tl >> 4) * 16u;
+        ldsm_x4(ts, T11.hi);
+        ldsm_x4(ts + 32, T11.lo);
+        ldsm_x4(ts + 16 * 80, T22.hi);
+        ldsm_x4(ts + 16 * 80 + 32, T22.lo);
+    }
+    // (block decays of all warps are in shared memory; the scratch has been read: the Q tile comes in its place)
+    fence_proxy_async();
+    __syncthreads();
+    if (kOut) {
+        if (tid == 0) {
+            mbar_arrive_expect_tx(&sm.full_q, G::kTile);
+#pragma unroll
+            for (int s = 0; s < G::kSlabs; s++) tma_load_4d(sm.q + s * G::kSlab, &tmQ, &sm.full_q, 64 * s, hd, c * kD, b);
+        }
+    }
+    // ---- M against the earlier blocks
+#pragma unroll
+    for (int J = 0; J < kBlocks - 1; J++)
+        if (J < I) {
+            float acc[2][4][4];
+            gram_block<kD, kPairs, false>(acc, kt, 32 * I, kt, 32 * J, tl, false);
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+#pragma unroll
+                for (int n = 0; n < 4; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[m][n][e] *= cc[2 * m + (e >> 1)];
+                M[J][m][0] = split(acc[m][0], acc[m][1]);
+                M[J][m][1] = split(acc[m][2], acc[m][3]);
+            }
+        }
+    // x <- (I + M_own)^-1 rhs for one column tile; f: the solution as B fragments of the two 16-token halves
+    auto solve = [&](float (&x)[4], uint2 (&f)[2]) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_split(d, T11, rhs_frag(x[0], x[1]));
+        x[0] = d[0] + d[1];
+        x[1] = d[2] + d[3];
+        f[0] = rhs_frag(x[0], x[1]);
+        float e[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_split(e, M21, f[0]);
+        x[2] -= e[0] + e[1];
+        x[3] -= e[2] + e[3];
+        float h[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_split(h, T22, rhs_frag(x[2], x[3]));
+        x[2] = h[0] + h[1];
+        x[3] = h[2] + h[3];
+        f[1] = rhs_frag(x[2], x[3]);
+    };
+    // sum over the earlier blocks of M times their published fragments, subtracted from the right-hand sides
+    auto subtract_earlier = [&](int J, int slot, float (&x)[kTiles][4]) {
+#pragma unroll
+        for (int q = 0; q < kTiles; q++) {
+            float d[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) d[m][e] = 0.f;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint2 f = sm.get(slot, q, h, tl);
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+#pragma unroll
+                    for (int JJ = 0; JJ < kBlocks - 1; JJ++)
+                        if (JJ == J) mma_split(d[m], M[JJ][m][h], f);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                x[q][2 * m] -= d[m][0] + d[m][1];
+                x[q][2 * m + 1] -= d[m][2] + d[m][3];
+            }
+        }
+    };
+    const int comp = t4 & 1;
+    // pair of the lane's component / of the fragment column in tile q (with one pair, the second half repeats it unused)
+    auto pair_of = [&](int q) { return kPairs == 1 ? 0 : 2 * q + (t4 >> 1); };
+    auto column_pair = [&](int q) { return kPairs == 1 ? 0 : 2 * q + (g >> 2); };
+    constexpr int kPerTile = kPairs == 1 ? 1 : 2;
+    // complex factor times the lane's component; `other` is the other component of the same value
+    auto rotate = [&](cplx f, float own, float other) { return f.r * own + (comp ? f.i : -f.i) * other; };
+
+    // ---- g: the chain over the blocks of the chunk
+    uint2 gf[kTiles][2];                       // own block's g / D
+    float gx[kTiles][4];
+    {
+#pragma unroll
+        for (int q = 0; q < kTiles; q++)
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float2 e = sm.viw[pair_of(q)][32 * I + 8 * r + g];
+                gx[q][r] = kPairs == 1 && t4 >= 2 ? 0.f : bn[r] * (comp ? e.y : e.x);
+            }
+#pragma unroll
+        for (int J = 0; J < kBlocks - 1; J++)
+            if (J < I) {
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + J), "r"(32 * (kBlocks - J)) : "memory");
+                subtract_earlier(J, G::slot_g(J, I), gx);
+            }
+#pragma unroll
+        for (int q = 0; q < kTiles; q++) solve(gx[q], gf[q]);
+#pragma unroll
+        for (int q = 0; q < kTiles; q++) {
+            const int p = pair_of(q);
+            float w[4];                        // g carried to the block end
+            const cplx d31 = sm.bp[p][I].D31;
+#pragma unroll
+            for (int r = 0; r < 4; r++) w[r] = rotate(d31, gx[q][r], __shfl_xor_sync(0xffffffffu, gx[q][r], 1));
+#pragma unroll 1
+            for (int s = 0; s < kPerTile; s++)   // decays beyond the scaled form: step by step
+                if (sm.bp[2 * q + s][I].slow) {
+                    slow_walk<kD, kPairs, kMode, false>(sm, 2 * q + s, I, tl);
+                    if (kPairs == 1 || (t4 >> 1) == s) {
+#pragma unroll
+                        for (int r = 0; r < 4; r++) {
+                            const float4 x = sm.walk[I][8 * r + g];
+                            w[r] = comp ? x.y : x.x;
+                        }
+                    }
+                    __syncwarp();
+                }
+            float wo[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) wo[r] = __shfl_xor_sync(0xffffffffu, w[r], 1);
+            // to every later block's start (times its reference product), and to the chunk end
+            cplx f = {1.f, 0.f};
+#pragma unroll
+            for (int to = 1; to <= kBlocks; to++) {
+                const bool end = to == kBlocks;
+                if (to > I) {
+                    if (!end || kNeedEnd || a.tail_state) {
+                        const cplx ff = end ? f : cmul(f, sm.bp[p][to < kBlocks ? to : 0].R);
+                        const int slot = end ? G::slot_end(I) : G::slot_g(I, to);
+                        sm.put(slot, q, 0, tl, rhs_frag(rotate(ff, w[0], wo[0]), rotate(ff, w[1], wo[1])));
+                        sm.put(slot, q, 1, tl, rhs_frag(rotate(ff, w[2], wo[2]), rotate(ff, w[3], wo[3])));
+                    }
+                    if (!end) f = cmul(f, sm.bp[p][to < kBlocks ? to : 0].A);
+                }
+            }
+        }
+        if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + I), "r"(32 * (kBlocks - I)) : "memory");
+        // (a slow pair takes no part in the scaled read-out)
+#pragma unroll
+        for (int q = 0; q < kTiles; q++)
+            if (sm.bp[2 * q][I].slow | sm.bp[2 * q + kPerTile - 1][I].slow) {
+                const bool mine = sm.bp[pair_of(q)][I].slow;                   // rows: this lane's pair
+                const bool col = sm.bp[column_pair(q)][I].slow;                // fragment: this lane's column
+#pragma unroll
+                for (int r = 0; r < 4; r++) gx[q][r] = mine ? 0.f : gx[q][r];
+                if (col) gf[q][0] = gf[q][1] = make_uint2(0u, 0u);
+            }
+    }
+    __syncthreads();
+
+    // product of K^T (this warp's 32 columns) with the fragments `slot0 + block` of all blocks, one column tile
+    auto k_transposed = [&](int slot0, int q, float (&d)[2][4]) {
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) d[m][e] = 0.f;
+#pragma unroll
+        for (int J = 0; J < kBlocks; J++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint2 f = sm.get(slot0 + J, q, h, tl);
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    uint32_t ka[4];
+                    ldsm_x4_trans(col_frag<G::kSlab>(kt, 32 * J + 16 * h, 32 * I + 16 * m, tl), ka);
+                    mma_bf16_m16n8k16(d[m], ka, f.x, f.y);
+                }
+            }
+    };
+    auto chunk_decay = [&](int p) {
+        cplx w = sm.bp[p][0].A;
+#pragma unroll
+        for (int J = 1; J < kBlocks; J++) w = cmul(w, sm.bp[p][J].A);
+        return w;
+    };
+
+    // ---- z at the chunk end; the carry
+    if (kNeedEnd) {
+        float z[kTiles][2][4];
+#pragma unroll
+        for (int q = 0; q < kTiles; q++) k_transposed(G::slot_end(0), q, z[q]);
+        if (kMode == kFused) {
+            if (!have_carry) {
+                const unsigned long long t0 = global_ns();
+                while (!(have_carry = __all_sync(0xffffffffu, flag_set()))) {
+                    __nanosleep(20);
+                    if (*reinterpret_cast<volatile int*>(a.status) != 0 || global_ns() - t0 > a.wait_ns) break;
+                }
+                have_carry = __all_sync(0xffffffffu, have_carry);
+                if (have_carry) load_carry(carry_src);
+            }
+            cp_async_wait_all();
+            __syncwarp();
+        }
+        const bool whole = Lc == kD;           // the reference's zero padding wipes state and decay (ssd.py:60-67)
+#pragma unroll
+        for (int q = 0; q < kTiles; q++) {
+            const int p = pair_of(q);
+            if (p < NP && (kPairs > 1 || t4 < 2)) {
+                cplx gam = chunk_decay(p);
+                gam = whole ? cplx{bfr(gam.r), bfr(gam.i)} : cplx{0.f, 0.f};
+                if (kMode == kLocal && I == 0 && g == 0)
+                    a.ws_gamma[unit * N + 2 * p + comp] = comp ? gam.i : gam.r;
+                const int n = 2 * p + comp;
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const int d = 32 * I + 16 * m + 8 * e + g;
+                        const float l = whole ? bfr(z[q][m][2 * e] + z[q][m][2 * e + 1]) : 0.f;
+                        if (kMode == kLocal) {
+                            a.ws_state[(unit * N + n) * kD + d] = l;
+                        } else {
+                            const float sr = sm.s_in[2 * p][d], si = sm.s_in[2 * p + 1][d];
+                            const float s = comp ? carry_im(gam.r, gam.i, sr, si, l) : carry_re(gam.r, gam.i, sr, si, l);
+                            if (c + 1 < a.NC) a.ws_state[((unit + H) * N + n) * kD + d] = s;
+                            else if (a.final_state) a.final_state[(((size_t)b * H + hd) * N + n) * kD + d] = s;
+                        }
+                    }
+            }
+        }
+        if (kMode == kLocal) return;
+        if (c + 1 < a.NC && have_carry) {      // release this warp's columns to the next chunk
+            __syncwarp();
+            int* next = reinterpret_cast<int*>(a.ws_gamma + (unit + H) * (size_t)N);
+            if (tl == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(next), "r"(1 << I) : "memory");
+        }
+    } else {
+        cp_async_wait_all();
+        __syncwarp();
+    }
+    // r_0: the carry rounded to bf16
+#pragma unroll
+    for (int n = 0; n < 2 * kPairs; n++) sm.r0[n][32 * I + tl] = __float2bfloat16_rn(sm.s_in[n][32 * I + tl]);
+    const bool q_here = mbar_wait_suspend(&sm.full_q, 0, &sm.abort_flag, a.wait_ns);
+    if (!__syncthreads_and(q_here && have_carry)) {
+        if (tid == 0) atomicCAS(a.status, 0, 202);
+        return;
+    }
+
+    // B fragment of r_0^T: columns in the tiles' order, the lo columns empty (r_0 is bf16)
+    auto r0_frag = [&](int q, int ks) {
+        const int n = 2 * column_pair(q) + ((g >> 1) & 1);
+        const uint32_t* s = reinterpret_cast<const uint32_t*>(&sm.r0[n][16 * ks + 2 * t4]);
+        return (g & 1) || (kPairs == 1 && g >= 4) ? make_uint2(0u, 0u) : make_uint2(s[0], s[4]);
+    };
+    // ---- h: right-hand sides c_t k_t.r_0, the same chain
+    float hx[kTiles][4];
+    {
+        float d[kTiles][2][4];
+#pragma unroll
+        for (int q = 0; q < kTiles; q++)
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) d[q][m][e] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < kKs; ks++) {
+            uint32_t ka[2][4];
+            ldsm_x4(row_frag<G::kSlab>(kt, 32 * I, ks, tl), ka[0]);
+            ldsm_x4(row_frag<G::kSlab>(kt, 32 * I + 16, ks, tl), ka[1]);
+#pragma unroll
+            for (int q = 0; q < kTiles; q++) {
+                const uint2 f = r0_frag(q, ks);
+                mma_bf16_m16n8k16(d[q][0], ka[0], f.x, f.y);
+                mma_bf16_m16n8k16(d[q][1], ka[1], f.x, f.y);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kTiles; q++)
+#pragma unroll
+            for (int r = 0; r < 4; r++) hx[q][r] = cc[r] * d[q][r >> 1][2 * (r & 1)];
+#pragma unroll
+        for (int J = 0; J < kBlocks - 1; J++)
+            if (J < I) {
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + J), "r"(32 * (kBlocks - J)) : "memory");
+                subtract_earlier(J, G::slot_h(J), hx);
+            }
+#pragma unroll
+        for (int q = 0; q < kTiles; q++) {
+            uint2 f[2];
+            solve(hx[q], f);
+            sm.put(G::slot_h(I), q, 0, tl, f[0]);
+            sm.put(G::slot_h(I), q, 1, tl, f[1]);
+        }
+        if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + I), "r"(32 * (kBlocks - I)) : "memory");
+        __syncwarp();
+    }
+
+    // ---- |q|^-1 and q.r_0
+    float mq[4], rho[kTiles][4];
+    {
+        float qd[2][2][4], d[kTiles][2][4];
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) qd[m][0][e] = qd[m][1][e] = 0.f;
+#pragma unroll
+        for (int q = 0; q < kTiles; q++)
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) d[q][m][e] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < kKs; ks++) {
+            uint32_t qa[2][4];
+            ldsm_x4(row_frag<G::kSlab>(qt, 32 * I, ks, tl), qa[0]);
+            ldsm_x4(row_frag<G::kSlab>(qt, 32 * I + 16, ks, tl), qa[1]);
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                mma_bf16_m16n8k16(qd[m][0], qa[m], qa[m][0], qa[m][2]);
+                mma_bf16_m16n8k16(qd[m][1], qa[m], qa[m][1], qa[m][3]);
+            }
+#pragma unroll
+            for (int q = 0; q < kTiles; q++) {
+                const uint2 f = r0_frag(q, ks);
+                mma_bf16_m16n8k16(d[q][0], qa[0], f.x, f.y);
+                mma_bf16_m16n8k16(d[q][1], qa[1], f.x, f.y);
+            }
+        }
+        diagonal_of(qd[0][0], qd[0][1], tl, mq[0], mq[1]);
+        diagonal_of(qd[1][0], qd[1][1], tl, mq[2], mq[3]);
+#pragma unroll
+        for (int r = 0; r < 4; r++) mq[r] = rsqrtf(mq[r] + kEps);
+#pragma unroll
+        for (int q = 0; q < kTiles; q++)
+#pragma unroll
+            for (int r = 0; r < 4; r++) rho[q][r] = d[q][r >> 1][2 * (r & 1)];
+    }
+    // ---- read-out: P against the block itself and the earlier ones
+    float oz[kTiles][4], pd[4];
+#pragma unroll
+    for (int q = 0; q < kTiles; q++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) oz[q][r] = 0.f;
+#pragma unroll 1
+    for (int J = I; J >= 0; J--) {
+        const bool diag = J == I;
+        float acc[2][4][4];
+        gram_block<kD, kPairs, false>(acc, qt, 32 * I, kt, 32 * J, tl, diag);
+        if (diag) {
+            diagonal_of(acc[0][0], acc[0][1], tl, pd[0], pd[1]);
+            diagonal_of(acc[1][2], acc[1][3], tl, pd[2], pd[3]);
+#pragma unroll
+            for (int m = 0; m < 2; m++)        // strictly lower (the diagonal enters with g itself below)
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (g + 8 * (e >> 1) <= 8 * n + 2 * t4 + (e & 1)) acc[m][2 * m + n][e] = 0.f;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const Split p0 = split(acc[0][2 * h], acc[0][2 * h + 1]), p1 = split(acc[1][2 * h], acc[1][2 * h + 1]);
+#pragma unroll
+            for (int q = 0; q < kTiles; q++) {
+                const uint2 fg = diag ? gf[q][h] : sm.get(G::slot_g(J, I), q, h, tl);
+                const uint2 fh = sm.get(G::slot_h(J), q, h, tl);
+                float dz[2][4], dh[2][4];
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) dz[m][e] = dh[m][e] = 0.f;
+                if (!(diag && h == 1)) {
+                    mma_split(dz[0], p0, fg);
+                    mma_split(dh[0], p0, fh);
+                }
+                mma_split(dz[1], p1, fg);
+                mma_split(dh[1], p1, fh);
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    oz[q][r] += dz[r >> 1][2 * (r & 1)] + dz[r >> 1][2 * (r & 1) + 1];
+                    rho[q][r] -= dh[r >> 1][2 * (r & 1)] + dh[r >> 1][2 * (r & 1) + 1];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kTiles; q++) {
+        const int p = pair_of(q);
+        // W_{t-1} = D_{t-1} F, F = (decay up to the block) R; the first token of a block takes the decay itself
+        cplx pre = {1.f, 0.f};
+#pragma unroll
+        for (int J = 0; J < kBlocks - 1; J++)
+            if (J < I) pre = cmul(pre, sm.bp[p][J].A);
+        const cplx F = cmul(pre, sm.bp[p][I].R);
+        float y[4], ho[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int row = 32 * I + 8 * r + g;
+            const float x = oz[q][r] + pd[r] * gx[q][r], xo = __shfl_xor_sync(0xffffffffu, x, 1);
+            ho[r] = __shfl_xor_sync(0xffffffffu, rho[q][r], 1);
+            const float2 D = sm.dd[p][row], D0 = sm.dd[p][row > 0 ? row - 1 : 0];
+            const bool first = r == 0 && g == 0;
+            const cplx w0 = first ? pre : cmul({D0.x, D0.y}, F);
+            y[r] = rotate({D.x, D.y}, x, xo) + rotate(w0, rho[q][r], ho[r]);
+        }
+#pragma unroll 1
+        for (int s = 0; s < kPerTile; s++)
+            if (sm.bp[2 * q + s][I].slow) {
+                slow_walk<kD, kPairs, kMode, true>(sm, 2 * q + s, I, tl);
+                if (kPairs == 1 || (t4 >> 1) == s) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const float4 x = sm.walk[I][8 * r + g];
+                        y[r] = (comp ? x.y : x.x) + rotate(cmul(pre, {x.z, x.w}), rho[q][r], ho[r]);
+                    }
+                }
+                __syncwarp();
+            }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int row = 32 * I + 8 * r + g;
+            float yy = mq[r] * y[r];
+            if (a.shortcut_scale != 0.f) {   // block.py:202-208; v after the vp scale
+                const float qk = mq[r] * nrm[r] * pd[r];
+                const float2 e = sm.viw[p][row], D = sm.dd[p][row];
+                const cplx vg = sm.bp[p][I].slow ? cplx{e.x, e.y} : cmul({e.x, e.y}, {D.x, D.y});
+                yy += a.shortcut_scale * qk * qk * bfr(comp ? vg.i : vg.r);
+            }
+            if (kPairs > 1 || t4 < 2) sm.y(I, 8 * r + g)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * sm.sel[row]);
+        }
+    }
+    __syncwarp();
+    if (32 * I + tl < Lc) {   // lane = token: its row of N values
+        __nv_bfloat16* yo = a.y + (((size_t)b * L + c * kD + 32 * I + tl) * H + hd) * N;
+        const uint32_t* ys = reinterpret_cast<const uint32_t*>(sm.y(I, tl));
+        if (kPairs >= 4 && N == 2 * kPairs && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < kPairs; i += 4)
+                *reinterpret_cast<uint4*>(yo + 2 * i) = make_uint4(ys[i], ys[i + 1], ys[i + 2], ys[i + 3]);
+        } else {
+            for (int i = 0; i < NP; i++) reinterpret_cast<uint32_t*>(yo)[i] = ys[i];
+        }
+    }
+    // ---- the recurrent state after the last token
+    if (a.tail_state && c == a.NC - 1) {
+        __syncthreads();   // every block's h is published
+#pragma unroll 1
+        for (int q = 0; q < kTiles; q++) {
+            float z[2][4], h[2][4];
+            k_transposed(G::slot_end(0), q, z);
+            k_transposed(G::slot_h(0), q, h);
+            const int p = pair_of(q);
+            const cplx w = chunk_decay(p);
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int d = 32 * I + 16 * m + 8 * e + g, n = 2 * p + comp;
+                    const float r = __bfloat162float(sm.r0[n][d]) - (h[m][2 * e] + h[m][2 * e + 1]);
+                    const float o = __shfl_xor_sync(0xffffffffu, r, 1);
+                    if (p < NP && (kPairs > 1 || t4 < 2))
+                        a.tail_state[(((size_t)b * H + hd) * N + n) * kD + d] = z[m][2 * e] + z[m][2 * e + 1] + rotate(w, r, o);
+                }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// Host side
+// ------------------------------------------------------------------------------------------
+template <int kD, int kPairs, Mode kMode> struct KernelTag {};
+
+template <int kD, int kPairs, Mode kMode>
+static int launch_one(const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, cudaStream_t st) {
+    const size_t smem = sizeof(Smem<kD, kPairs, kMode>);
+    static_assert(sizeof(Smem<kD, kPairs, kMode>) <= 227 * 1024, "shared memory");
+    if (int rc = allow_smem<KernelTag<kD, kPairs, kMode>>((const void*)scan_chunk_kernel<kD, kPairs, kMode>, smem)) return rc;
+    const long long units = (long long)a.B * a.NC * a.H;
+    return launch_overlapped(scan_chunk_kernel<kD, kPairs, kMode>, dim3((unsigned)units), dim3(Geo<kD, kPairs>::kThreads), smem, st,
+                             tmK, tmQ, a);
+}
+template <int kD, int kPairs>
+static int launch_mode(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, cudaStream_t st) {
+    if (m == kLocal) return launch_one<kD, kPairs, kLocal>(tmK, tmQ, a, st);
+    if (m == kOutput) return launch_one<kD, kPairs, kOutput>(tmK, tmQ, a, st);
+    return launch_one<kD, kPairs, kFused>(tmK, tmQ, a, st);
+}
+template <int kD>
+static int launch_tiles(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, cudaStream_t st) {
+    if (a.N <= 2) return launch_mode<kD, 1>(m, tmK, tmQ, a, st);
+    if (a.N <= 4) return launch_mode<kD, 2>(m, tmK, tmQ, a, st);
+    if (a.N <= 8) return launch_mode<kD, 4>(m, tmK, tmQ, a, st);
+    return launch_mode<kD, 8>(m, tmK, tmQ, a, st);
+}
+
+}  // namespace chunk
+
+bool scan_chunk_supported(int D, int N, int C, int dtype) {
+    return dtype == CDSSM_BF16 && D == C && (D == 64 || D == 128) && N <= 16;
+}
+
+// Bytes of the per-token records: transition and scaled v per pair, beta and sel_C.
+size_t scan_chunk_record_bytes(int B, int L, int H, int N, int C) {
+    return (size_t)B * (((size_t)L + C - 1) / C) * H * C * ((size_t)(N / 2) * 12 + 4);
+}
+
+namespace chunk {
+struct Records {
+    float2* a;
+    uint32_t *v, *g;
+};
+static Records records(void* rec, int B, int L, int H, int N, int C) {
+    const size_t n = (size_t)B * (((size_t)L + C - 1) / C) * H * C;
+    float2* a = static_cast<float2*>(rec);
+    uint32_t* v = reinterpret_cast<uint32_t*>(a + n * (N / 2));
+    return {a, v, v + n * (N / 2)};
+}
+}  // namespace chunk
+
+// The records (scan_chunk_record_bytes bytes) that every pass over the same inputs reads.
+int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
+                        const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
+                        cudaStream_t st) {
+    using namespace chunk;
+    const Records r = records(rec, B, L, H, N, C);
+    DynArgs d;
+    d.v = static_cast<const __nv_bfloat16*>(v);
+    d.gate_raw = static_cast<const __nv_bfloat16*>(gate_raw);
+    d.log_dt_scale = log_dt_scale; d.rope_freqs = rope_freqs;
+    d.rec_a = r.a; d.rec_v = r.v; d.rec_g = r.g;
+    d.dc = dc;
+    d.B = B; d.L = L; d.H = H; d.N = N; d.C = C; d.NC = (L + C - 1) / C; d.pos0 = pos0; d.segs = segs; d.fp32_decay = fp32_decay;
+    const long long tiles = (long long)B * d.NC * (C / kDynTokens);
+    if (tiles > 0x7fffffff || H > 32 * 65535) return CDSSM_ERR_UNSUPPORTED;
+    dynamics_kernel<<<dim3((unsigned)tiles, (H + 31) / 32), 32 * kDynWarps, 0, st>>>(d);
+    return check_launch();
+}
+
+// mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the carries from ws_state,
+// writes y), 2: both in one kernel with the carry handed on inside it (ws_gamma and *ticket zeroed by the caller).
+// status: one int in device memory, set by a bounded wait that ran out (not cleared here).
+int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const float* h0, void* y, float* final_state,
+                    float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
+                    int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st) {
+    using namespace chunk;
+    CUtensorMap tmK, tmQ;
+    if (!make_tile_map(&tmK, k, B, L, H, D, D) || !make_tile_map(&tmQ, mode == 0 ? k : q, B, L, H, D, D)) return CDSSM_ERR_CUDA;
+    Args a;
+    const Records r = records(rec, B, L, H, N, D);
+    a.rec_a = r.a; a.rec_v = r.v; a.rec_g = r.g;
+    a.h0 = h0;
+    a.y = static_cast<__nv_bfloat16*>(y);
+    a.final_state = final_state; a.tail_state = tail_state;
+    a.ws_gamma = ws_gamma; a.ws_state = ws_state; a.status = status; a.ticket = ticket;
+    a.wait_ns = wait_ns ? wait_ns : 400ull * 1000 * 1000;
+    a.withhold = withhold;
+    a.shortcut_scale = shortcut_scale;
+    a.B = B; a.L = L; a.H = H; a.N = N; a.NC = (L + D - 1) / D;
+    if ((long long)B * a.NC * H > 0x7fffffff) return CDSSM_ERR_UNSUPPORTED;
+    const Mode m = mode == 0 ? kLocal : mode == 1 ? kOutput : kFused;
+    if (mode == 0) a.tail_state = nullptr;
+    return D == 128 ? launch_tiles<128>(m, tmK, tmQ, a, st) : launch_tiles<64>(m, tmK, tmQ, a, st);
+}
+
+}  // namespace cdssm

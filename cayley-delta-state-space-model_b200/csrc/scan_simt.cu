@@ -11,8 +11,8 @@
 //   local pass  : per (chunk, head, pair) walk z only -> gamma_c and z_{C-1}  (workspace)
 //   carry pass  : per (batch, head, pair, d) serial over chunks -> s_c in place of z_{C-1}
 //   output pass : per (chunk, head, pair) walk z and r together, read out y
-// The local pass re-reads k, v and the gates (about half of the algorithmic bytes).  scan_wa.cu holds the
-// tensor-core local and output pass for the shapes it supports; the carry pass here serves both.
+// The local pass re-reads k, v and the gates (about half of the algorithmic bytes).  scan_wa.cu and
+// scan_chunk.cu hold the tensor-core kernels for the shapes they take; the carry pass here serves both.
 //
 // Thread mapping: eight lanes own one (chunk, head, pair) unit, each lane D/8 contiguous
 // columns of the two state rows, so a k/q row is fetched with 16-byte loads and a dot product
@@ -462,8 +462,7 @@ scan_carry_kernel(const ScanArgs a) {
                     a.ws_state[u * 2 * D + d] = IO<T>::rnd(sr);       // chunk_states store
                     a.ws_state[u * 2 * D + D + d] = IO<T>::rnd(si);
                 }
-                const float nr = gr[i] * sr - gi[i] * si + lr[i];
-                const float ni = gr[i] * si + gi[i] * sr + li[i];
+                const float nr = carry_re(gr[i], gi[i], sr, si, lr[i]), ni = carry_im(gr[i], gi[i], sr, si, li[i]);
                 sr = nr;
                 si = ni;
                 const float pr = gr[i] * dr - gi[i] * di, pi = gr[i] * di + gi[i] * dr;
@@ -739,24 +738,37 @@ namespace cdssm {
 unsigned long long wait_limit_ns();   // c_abi.cu
 // scan_wa.cu
 bool scan_wa_supported(int D, int N, int C, int H, int dtype);
-size_t scan_wa_record_bytes(int B, int L, int H, int C);
 int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs,
                      void* rec, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
                      cudaStream_t st);
 int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  cudaStream_t st);
+// scan_chunk.cu
+bool scan_chunk_supported(int D, int N, int C, int dtype);
+size_t scan_chunk_record_bytes(int B, int L, int H, int N, int C);
+int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
+                        const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
+                        cudaStream_t st);
+int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const float* h0, void* y, float* final_state,
+                    float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
+                    int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int D, int N, int C) {
-    if (B <= 0 || L <= 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return 0;
+// What the CUDA-core kernels need: status word, chunk decays, chunk states.
+static size_t simt_workspace_bytes(int B, int L, int H, int D, int N, int C) {
     const size_t NC = ((size_t)L + C - 1) / C;
     const size_t units = (size_t)B * NC * H * (N / 2);
-    size_t bytes = 256 + align256(units * 2 * sizeof(float)) + align256(units * 2 * D * sizeof(float));
-    // per-token records of the four-chain tensor-core kernels (the data type is not known here)
-    if (scan_wa_supported(D, N, C, H, CDSSM_BF16)) bytes += align256(scan_wa_record_bytes(B, L, H, C));
+    return 256 + align256(units * 2 * sizeof(float)) + align256(units * 2 * D * sizeof(float));
+}
+
+extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int D, int N, int C) {
+    if (B <= 0 || L <= 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return 0;
+    size_t bytes = simt_workspace_bytes(B, L, H, D, N, C);
+    // per-token records of the tensor-core kernels (the data type is not known here)
+    if (scan_chunk_supported(D, N, C, CDSSM_BF16)) bytes += align256(scan_chunk_record_bytes(B, L, H, N, C));
     return bytes;
 }
 
@@ -767,6 +779,19 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
         return rc;
     if (int rc = check_cuda(cudaStreamSynchronize((cudaStream_t)stream))) return rc;
     return *status_host == 0 ? CDSSM_OK : CDSSM_ERR_TIMEOUT;
+}
+
+// Whether the whole-chunk scan runs as one kernel that hands the carry from chunk to chunk inside it, or as local pass +
+// carry pass + output pass.  One kernel reads k once and computes G once, but a hand-off takes 2 us (flag, carry, rounding,
+// release), so a (batch, head) chain of NC chunks takes 2 NC us whatever the size; the three passes cost a third more work
+// and two launches of which each is as long as one chunk takes.  Measured on B200, us, one kernel / three passes (D 64):
+//     N 4,  H 24, L 2048:  B 4   77 / 82    B 8  126 / 161        N 16, H 24, L 2048: B 4 165 / 175   B 8 251 / 329
+//     N 16, H 24, L 523:   B 1   58 / 73    N 16, H 24, L 16384: B 1 735 / 345     N 2, H 6, L 4096: B 1 109 / 30
+// so: where the chunks that run beside each other cover a hand-off (a chunk's share of a full GPU is per_chunk ns), or the
+// chain is short.
+static bool one_kernel_pays(int B, int H, int NC, int D, int N) {
+    const float per_chunk = D == 64 ? 14.f + 1.7f * N : 40.f + (N > 8 ? 9.f : 5.f) * N;
+    return (float)B * (float)H * per_chunk >= 1800.f || NC <= 4 + N / 2;
 }
 
 static int scan_fused_impl(const void* q, const void* k, const void* v, const void* gate_raw,
@@ -785,11 +810,11 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (((uintptr_t)q | (uintptr_t)k) & 15) return CDSSM_ERR_BAD_ARG;   // 16-byte row loads
     if (N > kMaxStateDim || D > kMaxHeadDim || C > kMaxChunk) return CDSSM_ERR_UNSUPPORTED;
     if (B == 0 || L == 0) return CDSSM_OK;
-    const size_t need = cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
+    const size_t need = (flags & CDSSM_SCAN_FORCE_SIMT) ? simt_workspace_bytes(B, L, H, D, N, C)
+                                                        : cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return CDSSM_ERR_WORKSPACE;
-    // first 256 bytes of the workspace: status word of the tensor-core kernel's bounded waits
+    // first 256 bytes of the workspace: status word of the tensor-core kernel's bounded waits, ticket counter
     int* status = static_cast<int*>(workspace);
-    if (int rc = check_cuda(cudaMemsetAsync(status, 0, sizeof(int), (cudaStream_t)stream))) return rc;
     workspace = static_cast<char*>(workspace) + 256;
     if ((flags & CDSSM_SCAN_EXACT) && (summary_only || segs != 1)) return CDSSM_ERR_UNSUPPORTED;
     ScanArgs a;
@@ -809,10 +834,24 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     a.ws_gamma = static_cast<float*>(workspace);
     a.ws_state = reinterpret_cast<float*>(static_cast<char*>(workspace) +
                                           align256((size_t)a.units * 2 * sizeof(float)));
+    cudaStream_t st = (cudaStream_t)stream;
+    // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 with heads in fours (scan_wa.cu), any other
+    // N <= 16 (scan_chunk.cu).  They read v and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the
+    // contract allows, stay on the CUDA-core kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the
+    // tests to check each tensor-core pass alone.)
+    const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y) & 3) == 0 && !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
+    const bool wa_ok = tensor_ok && tail_state == nullptr && scan_wa_supported(D, N, C, H, dtype);
+    const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
+    if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && !wa_ok) return CDSSM_ERR_UNSUPPORTED;
+    const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
+    const bool one_kernel = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && ((uintptr_t)h0 & 15) == 0 &&
+                            one_kernel_pays(B, H, a.NC, D, N);
+    // (the one-kernel scan keeps its "carry is there" words in the gamma slots)
+    const size_t zero = one_kernel ? 256 + (size_t)a.units * 2 * sizeof(float) : 2 * sizeof(int);
+    if (int rc = check_cuda(cudaMemsetAsync(status, 0, zero, st))) return rc;
     if (flags & CDSSM_SCAN_EXACT) {
         // the recurrent state after the last token is both the "carry" and the tail state
         const int cols = (D + kLanesPerUnit - 1) / kLanesPerUnit;
-        cudaStream_t st = (cudaStream_t)stream;
         float* extra = tail_state;
         if (!a.final_state) { a.final_state = tail_state; extra = nullptr; }
         int rc;
@@ -823,37 +862,30 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                                             cudaMemcpyDeviceToDevice, st));
         return rc;
     }
-    // Warp-autonomous tensor-core passes (scan_wa.cu) for the local and the output pass, with the CUDA-core
-    // carry pass between them: the default wherever the shapes allow.  (Bits 256 / 512 keep the CUDA-core
-    // local / output pass: used by the tests to check each tensor-core pass alone.)
-    // (the tensor-core passes read v and write y as 4-byte pairs: buffers that are only 2-byte aligned, which
-    // the contract allows, stay on the CUDA-core kernels)
-    const bool pair_aligned = ((((uintptr_t)v) | ((uintptr_t)y)) & 3) == 0;
-    const bool wa_ok = tail_state == nullptr && pair_aligned && scan_wa_supported(D, N, C, H, dtype);
-    const bool wa_asked = (flags & CDSSM_SCAN_TENSOR_CORE_WA) != 0;
-    if (!(flags & CDSSM_SCAN_FORCE_SIMT) && (wa_asked || wa_ok)) {
-        if (!wa_ok) return CDSSM_ERR_UNSUPPORTED;
-        cudaStream_t st = (cudaStream_t)stream;
-        const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
-        const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
-        const unsigned long long limit = wait_limit_ns();
-        void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
-        if (int rc = scan_wa_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, a.dc, B, L, H, C, pos0, segs,
-                                      a.fp32_decay, st))
-            return rc;
-        if (a.run_local && tc_local) {
-            if (int rc = scan_wa_pass(false, q, k, rec, a.ws_gamma, a.ws_state, nullptr, status, shortcut_scale, B, L, H,
-                                      D, limit, withhold, st))
-                return rc;
-            a.run_local = 0;
-        }
-        a.run_output = tc_output ? 0 : 1;
-        if (int rc = scan_fused_simt(a, dtype, false, st)) return rc;   // carry pass (+ whatever was kept)
-        if (!tc_output || summary_only) return CDSSM_OK;
-        return scan_wa_pass(true, q, k, rec, a.ws_gamma, a.ws_state, y, status, shortcut_scale, B, L, H, D, limit,
-                            withhold, st);
+    if (!wa_ok && !chunk_ok) return scan_fused_simt(a, dtype, false, st);
+    const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
+    const unsigned long long limit = wait_limit_ns();
+    void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
+    auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
+        if (wa_ok)
+            return scan_wa_pass(mode == 1, q, k, rec, a.ws_gamma, a.ws_state, y, status, shortcut_scale, B, L, H, D, limit,
+                                withhold, st);
+        return scan_chunk_pass(mode, q, k, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
+                               shortcut_scale, B, L, H, D, N, limit, withhold, st);
+    };
+    if (a.run_local) {   // (a summary of the same inputs has left the records in the workspace)
+        const int rc = wa_ok ? scan_wa_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, a.dc, B, L, H, C, pos0, segs, a.fp32_decay, st)
+                             : scan_chunk_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, a.dc, B, L, H, N, C, pos0, segs, a.fp32_decay, st);
+        if (rc) return rc;
     }
-    return scan_fused_simt(a, dtype, false, (cudaStream_t)stream);
+    if (one_kernel) return pass(2);
+    if (a.run_local && tc_local) {
+        if (int rc = pass(0)) return rc;
+        a.run_local = 0;
+    }
+    a.run_output = tc_output ? 0 : 1;
+    if (int rc = scan_fused_simt(a, dtype, false, st)) return rc;   // carry pass (+ whatever was kept)
+    return !tc_output || summary_only ? CDSSM_OK : pass(1);
 }
 
 static int decode_step_impl(float* state, const void* q, const void* k, const void* v,
@@ -984,7 +1016,11 @@ extern "C" int cdssm_b200_scan_fused_fwd_noalloc(const void* q, const void* k, c
     }
     const size_t need = cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
     if (need == 0) return CDSSM_ERR_BAD_ARG;
-    if (need > kNoAllocScratchBytes) return CDSSM_ERR_WORKSPACE;   // beyond the built-in scratch
+    if (need > kNoAllocScratchBytes) {   // beyond the built-in scratch: without the tensor-core kernels' records, if that fits
+        if (simt_workspace_bytes(B, L, H, D, N, C) > kNoAllocScratchBytes || scan_wa_supported(D, N, C, H, dtype))
+            return CDSSM_ERR_WORKSPACE;
+        flags |= CDSSM_SCAN_FORCE_SIMT;
+    }
     int dev = 0;
     if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;
     if (dev < 0 || dev >= kNoAllocMaxDevices) return CDSSM_ERR_UNSUPPORTED;

@@ -33,6 +33,7 @@
 // (W, W0: inclusive / exclusive prefix products of a inside the sub-block.)
 #include "cdssm_common.cuh"
 #include "sm100_ptx.cuh"
+#include "tile_map.cuh"
 
 namespace cdssm {
 using namespace sm100;
@@ -855,35 +856,6 @@ __global__ void __launch_bounds__(256) wa_dynamics_kernel(const DynArgs a) {
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static const EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<EncodeTiledFn>(p);
-        return static_cast<EncodeTiledFn>(nullptr);
-    }();
-    return fn;
-}
-
-// (B, L, H, D) bf16 tensor viewed as 4-D (D, H, L, B); box = 64 columns x 1 head x 32 positions.
-static bool make_tile_map(CUtensorMap* m, const void* base, int B, int L, int H, int D) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return false;
-    const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)L, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)H * D * 2, (cuuint64_t)L * H * D * 2};
-    const cuuint32_t box[4] = {64, 1, (cuuint32_t)kSub, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 #ifdef CDSSM_WA_TRACE
 static int g_grid_override = 0;
 #endif
@@ -916,12 +888,7 @@ bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
     return dtype == CDSSM_BF16 && N == 2 && D == C && (D == 64 || D == 128) && H % 4 == 0;
 }
 
-size_t scan_wa_record_bytes(int B, int L, int H, int C) {
-    const size_t NC = ((size_t)L + C - 1) / C;
-    return (size_t)B * NC * C * H * sizeof(uint4);
-}
-
-// Dynamics pre-pass: fills rec (scan_wa_record_bytes bytes) for both scan passes.
+// Dynamics pre-pass: fills rec (16 bytes per token-head, chunks padded to full length: scan_chunk_record_bytes at N = 2) for both scan passes.
 int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs,
                      void* rec, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
                      cudaStream_t st) {
@@ -946,7 +913,7 @@ int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, flo
                  cudaStream_t st) {
     using namespace wa;
     CUtensorMap tmK, tmQ;
-    if (!make_tile_map(&tmK, k, B, L, H, D) || !make_tile_map(&tmQ, output ? q : k, B, L, H, D)) return CDSSM_ERR_CUDA;
+    if (!make_tile_map(&tmK, k, B, L, H, D, kSub) || !make_tile_map(&tmQ, output ? q : k, B, L, H, D, kSub)) return CDSSM_ERR_CUDA;
     int dev = 0, sms = 0;
     if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;
     if (int rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return rc;
