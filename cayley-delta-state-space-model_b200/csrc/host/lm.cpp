@@ -41,6 +41,13 @@ constexpr double kFinalEps = 1.0 / 16384;   // 2^-14
 constexpr double kGroupEps = 1e-5;
 constexpr int64_t kHeadDim = 64;
 constexpr int64_t kGraphBatch = 32;
+// Prompts beyond this take the CUDA-core scan.  The state that a cache keeps is a product of one bf16-rounded transition a
+// token, so two correct scans, whose outputs differ in single bf16 roundings only, drift apart in it with the square root
+// of the length (12 layers, relative 2-norm of the worst layer's state, any N: 0.011 at 200 tokens, 0.016 at 523, 0.019 at
+// 900, 0.027 at 2000).  Up to this length that stays well inside what bf16 activations give; longer prompts keep the rounding
+// order that caches have always been filled with.
+constexpr int64_t kTensorPrompt = 576;
+constexpr int64_t kScanForceSimt = CDSSM_SCAN_FORCE_SIMT;
 
 const char* kCapsule = "cdssm_lm_plan";
 Plan& plan_of(PyObject* o) {
@@ -92,7 +99,7 @@ void block_sequence(Plan& p, Block& b, const Tensor& x, Tensor& v_first, Cache* 
     const Tensor gates = at::linear(x_conv, b.w_gate, b.b_gate);
     const Tensor Q = at::linear(x_conv, b.w_q).view({B, L, H, kHeadDim});
     ScanOut s = scan_fused(Q, K, V, gates, b.lds, b.rope, p.dyn, H, N, p.chunk, Tensor(), b.shortcut, 0, cache != nullptr,
-                           cache ? 0 : flags, Tensor(), 1);
+                           cache ? (L > kTensorPrompt ? kScanForceSimt : 0) : flags, Tensor(), 1);
     if (cache) cache->state = s.tail;
     const Tensor y = at::linear(s.y.view({B, L, H * N}), b.w_readout);
     // The reference normalises over (channels of the group) x (ALL positions of the sequence) (block.py:216-222), which

@@ -148,6 +148,7 @@ struct DynArgs {
     float2* rec_a;
     uint32_t *rec_v, *rec_g;
     DynConsts dc;
+    int* status;   // cleared here for the passes that follow, or nullptr
     int B, L, H, N, C, NC, pos0, segs, fp32_decay;
 };
 constexpr int kDynTokens = 32, kDynWarps = 8;
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(32 * kDynWarps) dynamics_kernel(const DynArgs 
     __shared__ float2 sa[32][kDynTokens + 1];
     __shared__ uint32_t sv[32][kDynTokens + 1];
     grid_launch_dependents();
+    if (a.status != nullptr && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) *a.status = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, H = a.H, N = a.N, NP = N >> 1;
     const int head0 = blockIdx.y * 32, hd = head0 + lane, heads = min(32, H - head0);
     const int tiles = (a.NC * a.C) / kDynTokens, b = blockIdx.x / tiles, l0 = (blockIdx.x % tiles) * kDynTokens;
@@ -432,7 +434,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         sm.abort_flag = 0;
         fence_barrier_init();
         sm.item = kMode == kFused ? atomicAdd(a.ticket, 1) : (int)blockIdx.x;
-        sm.stop = *reinterpret_cast<volatile int*>(a.status);
+        sm.stop = kMode == kFused ? *reinterpret_cast<volatile int*>(a.status) : 0;
     }
     __syncthreads();
     if ((smem_u32(smem_raw) & 1023u) != 0) {   // the swizzled tiles need 1024-byte alignment
@@ -450,6 +452,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int s = 0; s < G::kSlabs; s++) tma_load_4d(sm.k + s * G::kSlab, &tmK, &sm.full_k, 64 * s, hd, c * kD, b);
     }
 
+    if (kMode == kOutput) grid_dependency_wait();   // the carry pass
     // ---- carry into the chunk: this warp's 32 columns of every state row.  Already there (previous pass), or early if
     // its producer is done; else polled for behind the products that do not need it.
     const float* carry_src = a.ws_state + unit * (size_t)N * kD;
@@ -498,7 +501,8 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         diagonal_of(acc[1][2], acc[1][3], tl, kk[2], kk[3]);
         // the token's dynamics, from the kernel before this one (its launch let this one start early; no __ldg here: loads
         // that claim the data constant may be moved above the wait)
-        grid_dependency_wait();
+        if (kMode != kOutput) grid_dependency_wait();
+        grid_launch_dependents();
         {
             const uint32_t gg = __ldcg(a.rec_g + unit * kD + tid);
             const float2* ra = a.rec_a + unit * (size_t)NP * kD + tid;
@@ -1099,7 +1103,7 @@ static Records records(void* rec, int B, int L, int H, int N, int C) {
 
 // The records (scan_chunk_record_bytes bytes) that every pass over the same inputs reads.
 int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                        const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
+                        int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
                         cudaStream_t st) {
     using namespace chunk;
     const Records r = records(rec, B, L, H, N, C);
@@ -1108,6 +1112,7 @@ int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt
     d.gate_raw = static_cast<const __nv_bfloat16*>(gate_raw);
     d.log_dt_scale = log_dt_scale; d.rope_freqs = rope_freqs;
     d.rec_a = r.a; d.rec_v = r.v; d.rec_g = r.g;
+    d.status = status;
     d.dc = dc;
     d.B = B; d.L = L; d.H = H; d.N = N; d.C = C; d.NC = (L + C - 1) / C; d.pos0 = pos0; d.segs = segs; d.fp32_decay = fp32_decay;
     const long long tiles = (long long)B * d.NC * (C / kDynTokens);

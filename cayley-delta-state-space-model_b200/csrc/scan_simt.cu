@@ -429,6 +429,8 @@ static int launch_recurrent(ScanArgs a, cudaStream_t st) {
 template <typename T>
 __global__ void __launch_bounds__(128)
 scan_carry_kernel(const ScanArgs a) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int NH = a.N >> 1, D = a.D, H = a.H, NC = a.NC;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)a.B * H * NH * D) return;
@@ -497,8 +499,7 @@ static int launch_simt(const ScanArgs& a, cudaStream_t st) {
         if (int rc = check_launch()) return rc;
     }
     const long long th = (long long)a.B * a.H * (a.N / 2) * a.D;
-    scan_carry_kernel<T><<<(unsigned)((th + 127) / 128), 128, 0, st>>>(a);
-    if (int rc = check_launch()) return rc;
+    if (int rc = launch_overlapped(scan_carry_kernel<T>, dim3((unsigned)((th + 127) / 128)), dim3(128), 0, st, a)) return rc;
     if (a.y == nullptr || !a.run_output) return CDSSM_OK;   // summary only, or y comes from another kernel
     scan_walk_kernel<T, kCols, kLanes, true><<<blocks, kSimtThreads, smem, st>>>(a);
     return check_launch();
@@ -739,17 +740,17 @@ unsigned long long wait_limit_ns();   // c_abi.cu
 // scan_wa.cu
 bool scan_wa_supported(int D, int N, int C, int H, int dtype);
 int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs,
-                     void* rec, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
+                     void* rec, int* status, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
                      cudaStream_t st);
 int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, float* ws_gamma, float* ws_state, void* y,
-                 int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
+                 float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  cudaStream_t st);
 // scan_chunk.cu
 bool scan_chunk_supported(int D, int N, int C, int dtype);
 size_t scan_chunk_record_bytes(int B, int L, int H, int N, int C);
 int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                        const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
-                        cudaStream_t st);
+                        int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
+                        int fp32_decay, cudaStream_t st);
 int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const float* h0, void* y, float* final_state,
                     float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
                     int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
@@ -836,19 +837,27 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                                           align256((size_t)a.units * 2 * sizeof(float)));
     cudaStream_t st = (cudaStream_t)stream;
     // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 with heads in fours (scan_wa.cu), any other
-    // N <= 16 (scan_chunk.cu).  They read v and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the
+    // N <= 16 (scan_chunk.cu).  The latter also where N = 2 has few chunks: four launches, of which two walk a chunk in
+    // sub-blocks, take 27 us (D 128: 39) however little there is to do, one kernel and the dynamics before it 14 to 20
+    // (D 64, 216 / 512 / 936 units: 25 / 26 / 36 against 27 / 28 / 32 us; D 128, 160 / 256 / 512: 30 / 32 / 65 against
+    // 41 / 41 / 44).  They read v and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the
     // contract allows, stay on the CUDA-core kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the
     // tests to check each tensor-core pass alone.)
     const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y) & 3) == 0 && !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
-    const bool wa_ok = tensor_ok && tail_state == nullptr && scan_wa_supported(D, N, C, H, dtype);
+    const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, H, dtype) &&
+                       ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || (long long)B * a.NC * H > (D == 64 ? 512 : 256));
     const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
     if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && !wa_ok) return CDSSM_ERR_UNSUPPORTED;
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
     const bool one_kernel = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && ((uintptr_t)h0 & 15) == 0 &&
                             one_kernel_pays(B, H, a.NC, D, N);
-    // (the one-kernel scan keeps its "carry is there" words in the gamma slots)
-    const size_t zero = one_kernel ? 256 + (size_t)a.units * 2 * sizeof(float) : 2 * sizeof(int);
-    if (int rc = check_cuda(cudaMemsetAsync(status, 0, zero, st))) return rc;
+    // Status word, and for the one-kernel scan its ticket counter and its "carry is there" words in the gamma slots; where a
+    // dynamics kernel runs first, that one clears the status.
+    const bool tensor = wa_ok || chunk_ok;
+    if (one_kernel || !tensor || !a.run_local) {
+        const size_t zero = one_kernel ? 256 + (size_t)a.units * 2 * sizeof(float) : sizeof(int);
+        if (int rc = check_cuda(cudaMemsetAsync(status, 0, zero, st))) return rc;
+    }
     if (flags & CDSSM_SCAN_EXACT) {
         // the recurrent state after the last token is both the "carry" and the tail state
         const int cols = (D + kLanesPerUnit - 1) / kLanesPerUnit;
@@ -862,20 +871,23 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                                             cudaMemcpyDeviceToDevice, st));
         return rc;
     }
-    if (!wa_ok && !chunk_ok) return scan_fused_simt(a, dtype, false, st);
+    if (!tensor) return scan_fused_simt(a, dtype, false, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
     void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
-            return scan_wa_pass(mode == 1, q, k, rec, a.ws_gamma, a.ws_state, y, status, shortcut_scale, B, L, H, D, limit,
-                                withhold, st);
+            return scan_wa_pass(mode == 1, q, k, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
+                                limit, withhold, st);
         return scan_chunk_pass(mode, q, k, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
                                shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };
-    if (a.run_local) {   // (a summary of the same inputs has left the records in the workspace)
-        const int rc = wa_ok ? scan_wa_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, a.dc, B, L, H, C, pos0, segs, a.fp32_decay, st)
-                             : scan_chunk_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, a.dc, B, L, H, N, C, pos0, segs, a.fp32_decay, st);
+    // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)
+    if (a.run_local || (flags & CDSSM_SCAN_TENSOR_CORE_WA)) {
+        const int rc = wa_ok ? scan_wa_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, status, a.dc, B, L, H, C, pos0, segs,
+                                                a.fp32_decay, st)
+                             : scan_chunk_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, one_kernel ? nullptr : status, a.dc,
+                                                   B, L, H, N, C, pos0, segs, a.fp32_decay, st);
         if (rc) return rc;
     }
     if (one_kernel) return pass(2);

@@ -75,6 +75,7 @@ struct Args {
     float* ws_gamma;             // (B,NC,H,2): written by the local pass
     float* ws_state;             // (B,NC,H,2,D): local pass writes z_{C-1}; the output pass reads the carry s_c
     __nv_bfloat16* y;
+    float* tail_state;           // (B,H,2,D) or nullptr: the output pass leaves z + r after the last token here
     int* status;
     unsigned long long wait_ns;  // limit of every device-side wait
     int withhold;                // test hook: the producer issues nothing, so the first wait runs out
@@ -255,7 +256,7 @@ __device__ __forceinline__ void producer(Smem<kD, kOutput>& sm, const CUtensorMa
 // with complex right-hand sides only, and the in-block read-out becomes two real-matrix products
 //     sum_{i<t} P[t,i] Gamma[t,i] u_i = W_t sum_{i<t} P[t,i] u^_i   (correction: W0_t, before its step).
 // One pass over the columns does both: per column four shuffles and eight FMAs.  The scaling needs
-// 1 / W_t, so a sub-block whose |W| gets small (strong decay; the zero padding behind the sequence end)
+// 1 / W_t, so a sub-block whose |W| gets small (strong decay)
 // takes the slower walk that builds the decay products explicitly (robust_block).
 // ------------------------------------------------------------------------------------------
 struct Tok {   // per-token quantities of one sub-block step, prepared one step ahead
@@ -272,7 +273,7 @@ struct Tok {   // per-token quantities of one sub-block step, prepared one step 
 // ratios W_t / W_i of the prefix products W_t = a_0 ... a_t, so they are taken relative to the middle of the
 // sub-block, D_t = W_t / W_15: lanes 0-15 hold the suffix product a_{t+1} ... a_15 = 1 / D_t, lanes 16-31 the
 // prefix product a_16 ... a_t = D_t, and neither half leaves the float range unless one half alone decays by
-// more than 1e-30 (then, or with the zero padding behind the sequence end, the explicit walk is taken).
+// more than 1e-30 (then the explicit walk is taken).
 __device__ __forceinline__ Tok prepare(const uint4& rec, int tl) {
     Tok k;
     k.at = {__uint_as_float(rec.x), __uint_as_float(rec.y)};
@@ -471,12 +472,15 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     const uint32_t ktile[2] = {smem_u32(sm.k[0]), smem_u32(sm.k[1])};
     const uint32_t qtile = smem_u32(sm.q);
 
-    const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+    // behind the sequence end a = 1, beta = v = 0: the state stands still
+    const uint4 still4 = make_uint4(0x3f800000u, 0u, 0u, 0u);
     ItemPos cur = item_pos(a, blockIdx.x), nxi = cur;
     Tok tk;
+    grid_dependency_wait();       // records (local pass) / carries (output pass) of the kernel before
+    grid_launch_dependents();
     {
         const bool valid = cur.c * kD + tl < L;
-        const uint4 first = valid ? __ldg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, cur.h0 + J, tl)) : zero4;
+        const uint4 first = valid ? __ldcg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, cur.h0 + J, tl)) : still4;
         tk = prepare(first, tl);
     }
     for (int g = 0; g < NS; g++) {
@@ -504,12 +508,12 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             gam = {1.f, 0.f};
         }
         // ---- fetch the record of step g + 1 (the next item's first sub-block after this item's last)
-        uint4 rec = zero4;
+        uint4 rec = still4;
         if (g + 1 < NS) {
             const ItemPos& np_ = (step + 1 < kSteps) ? cur : nxi;
             const int nsub = (step + 1) % kSteps;
             if (np_.c * kD + nsub * kSub + tl < L)
-                rec = __ldg(a.rec + rec_index(a, kSteps, np_.b, np_.c, nsub, np_.h0 + J, tl));
+                rec = __ldcg(a.rec + rec_index(a, kSteps, np_.b, np_.c, nsub, np_.h0 + J, tl));
         }
         const cplx at = tk.at, vg = tk.vg;
         const float be = tk.be;
@@ -687,9 +691,10 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             }
         }
         WA_STAMP(8);
-        // ---- state update S <- W_31 S + Omega K: not needed after the last sub-block of the output pass
+        // ---- state update S <- W_31 S + Omega K: after the last sub-block of the output pass only for the tail state
         const cplx W31 = tk.W31;
-        if (!kOutput || step + 1 < kSteps) {
+        const bool tail = kOutput && step + 1 == kSteps && a.tail_state != nullptr && cur.c == a.NC - 1;
+        if (!kOutput || step + 1 < kSteps || tail) {
             om[tl] = o.wh.r;
             om[32 + tl] = o.wh.i;
             if (kOutput) {
@@ -746,18 +751,33 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
         WA_STAMP(10);
         if (tl == 0) mbar_arrive(&sm.k_free[st]);
         if (!kOutput && step + 1 == kSteps) {
-            // the carry pass consumes these as the reference's bf16 cum_A[:, -1] / local_h[:, -1]
+            // the carry pass consumes these as the reference's bf16 cum_A[:, -1] / local_h[:, -1]; the reference's zero
+            // padding of a ragged last chunk wipes both (ssd.py:60-67)
+            const float keep = cur.c * kD + kD <= L ? 1.f : 0.f;
             if (!low && np < 2) {
                 float* s = a.ws_state + unit * 2 * kD + (size_t)np * kD;
 #pragma unroll
                 for (int ks = 0; ks < kKs; ks++) {
-                    *reinterpret_cast<float2*>(s + 16 * ks + 2 * tig) = make_float2(bfr(S[ks][0]), bfr(S[ks][1]));
-                    *reinterpret_cast<float2*>(s + 16 * ks + 8 + 2 * tig) = make_float2(bfr(S[ks][2]), bfr(S[ks][3]));
+                    *reinterpret_cast<float2*>(s + 16 * ks + 2 * tig) = make_float2(keep * bfr(S[ks][0]), keep * bfr(S[ks][1]));
+                    *reinterpret_cast<float2*>(s + 16 * ks + 8 + 2 * tig) = make_float2(keep * bfr(S[ks][2]), keep * bfr(S[ks][3]));
                 }
             }
             if (tl == 0) {
-                a.ws_gamma[unit * 2] = bfr(gam.r);
-                a.ws_gamma[unit * 2 + 1] = bfr(gam.i);
+                a.ws_gamma[unit * 2] = keep * bfr(gam.r);
+                a.ws_gamma[unit * 2 + 1] = keep * bfr(gam.i);
+            }
+        }
+        if (tail) {   // z + r: rows n' and n' + 2 sit sixteen lanes apart
+            float* s = a.tail_state + (((size_t)cur.b * H + hd) * 2 + (np & 1)) * kD;
+#pragma unroll
+            for (int ks = 0; ks < kKs; ks++) {
+                float x[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) x[e] = S[ks][e] + __shfl_xor_sync(0xffffffffu, S[ks][e], 16);
+                if (!low && np < 2) {
+                    *reinterpret_cast<float2*>(s + 16 * ks + 2 * tig) = make_float2(x[0], x[1]);
+                    *reinterpret_cast<float2*>(s + 16 * ks + 8 + 2 * tig) = make_float2(x[2], x[3]);
+                }
             }
         }
         if (g + 1 < NS) tk = prepare(rec, tl);
@@ -819,16 +839,18 @@ struct DynArgs {
     uint4* rec;
     DynConsts dc;
     int B, L, H, NB, pos0, segs;   // NB: 32-token blocks per batch row (chunks padded to full length)
+    int* status;                   // cleared here for the passes that follow
     int fp32_decay;                // 0: the transition is rounded to bf16 like the reference's A_bar store
 };
 __global__ void __launch_bounds__(256) wa_dynamics_kernel(const DynArgs a) {
     using T = __nv_bfloat16;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long total = (long long)a.B * a.L * a.H;
+    grid_launch_dependents();
+    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x, total = (uint32_t)a.B * a.L * a.H;   // below 2^32 (host)
+    if (idx == 0) *a.status = 0;
     if (idx >= total) return;
-    const int hd = (int)(idx % a.H);
-    const long long bl = idx / a.H;
-    const int l = (int)(bl % a.L), b = (int)(bl / a.L);
+    const uint32_t bl = idx / (uint32_t)a.H;
+    const int hd = (int)(idx - bl * a.H);
+    const int b = (int)(bl / (uint32_t)a.L), l = (int)(bl - (uint32_t)b * a.L);
     const int H = a.H;
     const T* gr = a.gate_raw + (size_t)bl * (size_t)(7 * H);
     const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
@@ -859,20 +881,18 @@ __global__ void __launch_bounds__(256) wa_dynamics_kernel(const DynArgs a) {
 #ifdef CDSSM_WA_TRACE
 static int g_grid_override = 0;
 #endif
+template <int kD, bool kOutput> struct KernelTag {};
 template <int kD, bool kOutput>
 static int launch_pass(const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, int sms, cudaStream_t st) {
     constexpr int kBlocksPerSm = kOutput ? 2 : (kD == 128 ? 3 : 4);
     const size_t smem = sizeof(Smem<kD, kOutput>);
-    if (int rc = check_cuda(cudaFuncSetAttribute(scan_wa_kernel<kD, kOutput>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem)))
-        return rc;
+    if (int rc = allow_smem<KernelTag<kD, kOutput>>((const void*)scan_wa_kernel<kD, kOutput>, smem)) return rc;
     long long resident = (long long)kBlocksPerSm * sms;
 #ifdef CDSSM_WA_TRACE
     if (g_grid_override > 0) resident = g_grid_override;
 #endif
     const int grid = (int)(a.items < resident ? a.items : resident);
-    scan_wa_kernel<kD, kOutput><<<grid, kThreads, smem, st>>>(tmK, tmQ, a);
-    return check_launch();
+    return launch_overlapped(scan_wa_kernel<kD, kOutput>, dim3(grid), dim3(kThreads), smem, st, tmK, tmQ, a);
 }
 
 }  // namespace wa
@@ -890,9 +910,10 @@ bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
 
 // Dynamics pre-pass: fills rec (16 bytes per token-head, chunks padded to full length: scan_chunk_record_bytes at N = 2) for both scan passes.
 int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs,
-                     void* rec, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
+                     void* rec, int* status, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
                      cudaStream_t st) {
     wa::DynArgs d;
+    d.status = status;
     d.v = static_cast<const __nv_bfloat16*>(v);
     d.gate_raw = static_cast<const __nv_bfloat16*>(gate_raw);
     d.log_dt_scale = log_dt_scale; d.rope_freqs = rope_freqs;
@@ -901,6 +922,7 @@ int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_sc
     d.B = B; d.L = L; d.H = H; d.NB = ((L + C - 1) / C) * (C / wa::kSub); d.pos0 = pos0; d.segs = segs;
     d.fp32_decay = fp32_decay;
     const long long total = (long long)B * L * H;
+    if (total > 0xffffff00LL) return CDSSM_ERR_UNSUPPORTED;
     wa::wa_dynamics_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d);
     return check_launch();
 }
@@ -909,7 +931,7 @@ int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_sc
 // ws_state / ws_gamma for the carry pass); output = true: reads the carries from ws_state, writes y.
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
 int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, float* ws_gamma, float* ws_state, void* y,
-                 int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
+                 float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  cudaStream_t st) {
     using namespace wa;
     CUtensorMap tmK, tmQ;
@@ -921,6 +943,7 @@ int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, flo
     a.rec = static_cast<const uint4*>(rec);
     a.ws_gamma = ws_gamma; a.ws_state = ws_state;
     a.y = static_cast<__nv_bfloat16*>(y);
+    a.tail_state = tail_state;
     a.status = status;
     a.wait_ns = wait_ns ? wait_ns : 400ull * 1000 * 1000;
     a.withhold = withhold;

@@ -187,3 +187,20 @@ def test_float32_transition_option(ops, orc, D, path):
     y0, _ = run_fused(ops, inp, torch.bfloat16, N, D)
     assert not torch.equal(y0, y)
     assert rel_err(to_np(y), wy) < rel_err(to_np(y), wy_ref) or rel_err(wy, wy_ref) < 1e-3
+
+
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("L", [1, 31, 32, 33, 64, 97, 128, 300])
+def test_wa_tail_state(ops, orc, D, L):
+    """The recurrent state after the last token, at lengths around the sub-block and chunk ends."""
+    B, H = 2, 8
+    inp = _inputs(orc, B, H, L, D, seed=L)
+    h0 = np.random.default_rng(2).standard_normal((B, H, N, D)).astype(np.float32)
+    y, fin, tail = run_fused(ops, inp, torch.bfloat16, N, D, h0=h0, flags=ops.TENSOR_CORE_WA, return_tail_state=True)
+    assert ops.scan_fused_status() == 0
+    ys, fs, ts = run_fused(ops, inp, torch.bfloat16, N, D, h0=h0, flags=ops.FORCE_SIMT, return_tail_state=True)
+    y0, f0 = run_fused(ops, inp, torch.bfloat16, N, D, h0=h0, flags=ops.TENSOR_CORE_WA)
+    assert torch.equal(y, y0) and torch.equal(fin, f0)
+    assert rel_err(to_np(y), to_np(ys)) <= BF16_TOL / 2
+    assert np.abs(to_np(fin) - to_np(fs)).max() <= 2e-2 * max(np.abs(to_np(fs)).max(), 1e-3)
+    assert np.abs(to_np(tail) - to_np(ts)).max() <= 1e-2 * np.abs(to_np(ts)).max()
