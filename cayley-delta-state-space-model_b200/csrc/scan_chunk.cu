@@ -136,88 +136,6 @@ struct __align__(1024) Smem {
     }
 };
 
-// ---- dynamics ------------------------------------------------------------------------------------------------
-// dynamics_fused.cu:64-139 and the vp scale of block.py:194-195, every result rounded to bf16 like the reference's stores
-// (the transition optionally not).  The gates lie heads-fastest, the scan wants a head's tokens side by side: a block takes
-// 32 tokens of up to 32 heads, lane = head, and turns its results around in shared memory, so that both sides move whole
-// sectors.  Read where they are used, by the block of one head, each 2-byte gate costs a sector and a slot of the L1 miss
-// queue of its own (seven per token and head): the local pass at B 8, L 2048, H 24, D 64 took 52 us, of which this was 2/3.
-struct DynArgs {
-    const __nv_bfloat16 *v, *gate_raw;
-    const float *log_dt_scale, *rope_freqs;
-    float2* rec_a;
-    uint32_t *rec_v, *rec_g;
-    DynConsts dc;
-    int* status;   // cleared here for the passes that follow, or nullptr
-    int B, L, H, N, C, NC, pos0, segs, fp32_decay;
-};
-constexpr int kDynTokens = 32, kDynWarps = 8;
-__global__ void __launch_bounds__(32 * kDynWarps) dynamics_kernel(const DynArgs a) {
-    using T = __nv_bfloat16;
-    __shared__ float2 sa[32][kDynTokens + 1];
-    __shared__ uint32_t sv[32][kDynTokens + 1];
-    grid_launch_dependents();
-    if (a.status != nullptr && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) *a.status = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, H = a.H, N = a.N, NP = N >> 1;
-    const int head0 = blockIdx.y * 32, hd = head0 + lane, heads = min(32, H - head0);
-    const int tiles = (a.NC * a.C) / kDynTokens, b = blockIdx.x / tiles, l0 = (blockIdx.x % tiles) * kDynTokens;
-    const int c = l0 / a.C, in_chunk = l0 % a.C;
-    constexpr int kPer = kDynTokens / kDynWarps;
-    const bool on = lane < heads;
-    const float lds = on ? a.log_dt_scale[hd] : 0.f, freq = on ? a.rope_freqs[hd] : 0.f;
-    DynShared ds[kPer];
-    float g0[kPer], g1[kPer];
-#pragma unroll
-    for (int i = 0; i < kPer; i++) {
-        const int l = l0 + warp * kPer + i;
-        float x[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        g0[i] = g1[i] = 0.f;
-        if (on && l < a.L) {
-            const T* gr = a.gate_raw + ((size_t)b * a.L + l) * (size_t)((N + 5) * H) + hd;
-            g0[i] = IO<T>::ld(gr);
-            g1[i] = IO<T>::ld(gr + NP * H);
-#pragma unroll
-            for (int s = 0; s < 5; s++) x[s] = IO<T>::ld(gr + (N + s) * H);
-        }
-        const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
-        ds[i] = dyn_shared<true>(g0[i], g1[i], x[0], x[1], x[2], x[3], x[4], lds, freq, pos, a.dc);
-        // behind the sequence end a = 1, beta = v = 0: the state stands still
-        sv[lane][warp * kPer + i] = on && l < a.L ? pack2(ds[i].beta, ds[i].sel_c) : 0u;
-    }
-    const size_t unit0 = ((size_t)b * a.NC + c) * H + head0;
-    __syncthreads();
-    for (int h = warp; h < heads; h += kDynWarps) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sv[h][lane];
-    for (int p = 0; p < NP; p++) {
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < kPer; i++) {
-            const int t = warp * kPer + i, l = l0 + t;
-            float2 at = make_float2(1.f, 0.f);
-            uint32_t vg = 0u;
-            if (on && l < a.L) {
-                const T* gr = a.gate_raw + ((size_t)b * a.L + l) * (size_t)((N + 5) * H) + hd;
-                const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
-                const float ga = p == 0 ? g0[i] : IO<T>::ld(gr + p * H), gw = p == 0 ? g1[i] : IO<T>::ld(gr + (NP + p) * H);
-                const uint32_t vv = *reinterpret_cast<const uint32_t*>(a.v + (((size_t)b * a.L + l) * H + hd) * N + 2 * p);
-                float ar, ai, vp;
-                dyn_pair<true>(ga, gw, freq, pos, ds[i], ar, ai, vp);
-                if (!a.fp32_decay) { ar = bfr(ar); ai = bfr(ai); }
-                vp = bfr(vp);
-                at = make_float2(ar, ai);
-                vg = pack2(bits_lo(vv) * vp, bits_hi(vv) * vp);
-            }
-            sa[lane][t] = at;
-            sv[lane][t] = vg;
-        }
-        __syncthreads();
-        for (int h = warp; h < heads; h += kDynWarps) {
-            const size_t o = ((unit0 + h) * NP + p) * a.C + in_chunk + lane;
-            a.rec_a[o] = sa[h][lane];
-            a.rec_v[o] = sv[h][lane];
-        }
-    }
-}
-
 // ---- fragments ------------------------------------------------------------------------------------------------
 // A (16 tokens x 16 columns, row-major) or, with registers {0,2} / {1,3}, two B fragments (8 tokens each)
 template <uint32_t kSlab>
@@ -1083,43 +1001,8 @@ bool scan_chunk_supported(int D, int N, int C, int dtype) {
     return dtype == CDSSM_BF16 && D == C && (D == 64 || D == 128) && N <= 16;
 }
 
-// Bytes of the per-token records: transition and scaled v per pair, beta and sel_C.
-size_t scan_chunk_record_bytes(int B, int L, int H, int N, int C) {
-    return (size_t)B * (((size_t)L + C - 1) / C) * H * C * ((size_t)(N / 2) * 12 + 4);
-}
-
-namespace chunk {
-struct Records {
-    float2* a;
-    uint32_t *v, *g;
-};
-static Records records(void* rec, int B, int L, int H, int N, int C) {
-    const size_t n = (size_t)B * (((size_t)L + C - 1) / C) * H * C;
-    float2* a = static_cast<float2*>(rec);
-    uint32_t* v = reinterpret_cast<uint32_t*>(a + n * (N / 2));
-    return {a, v, v + n * (N / 2)};
-}
-}  // namespace chunk
-
-// The records (scan_chunk_record_bytes bytes) that every pass over the same inputs reads.
-int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                        int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
-                        cudaStream_t st) {
-    using namespace chunk;
-    const Records r = records(rec, B, L, H, N, C);
-    DynArgs d;
-    d.v = static_cast<const __nv_bfloat16*>(v);
-    d.gate_raw = static_cast<const __nv_bfloat16*>(gate_raw);
-    d.log_dt_scale = log_dt_scale; d.rope_freqs = rope_freqs;
-    d.rec_a = r.a; d.rec_v = r.v; d.rec_g = r.g;
-    d.status = status;
-    d.dc = dc;
-    d.B = B; d.L = L; d.H = H; d.N = N; d.C = C; d.NC = (L + C - 1) / C; d.pos0 = pos0; d.segs = segs; d.fp32_decay = fp32_decay;
-    const long long tiles = (long long)B * d.NC * (C / kDynTokens);
-    if (tiles > 0x7fffffff || H > 32 * 65535) return CDSSM_ERR_UNSUPPORTED;
-    dynamics_kernel<<<dim3((unsigned)tiles, (H + 31) / 32), 32 * kDynWarps, 0, st>>>(d);
-    return check_launch();
-}
+// scan_records.cu
+void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a, uint32_t** v, uint32_t** g);
 
 // mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the carries from ws_state,
 // writes y), 2: both in one kernel with the carry handed on inside it (ws_gamma and *ticket zeroed by the caller).
@@ -1131,8 +1014,10 @@ int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const flo
     CUtensorMap tmK, tmQ;
     if (!make_tile_map(&tmK, k, B, L, H, D, D) || !make_tile_map(&tmQ, mode == 0 ? k : q, B, L, H, D, D)) return CDSSM_ERR_CUDA;
     Args a;
-    const Records r = records(rec, B, L, H, N, D);
-    a.rec_a = r.a; a.rec_v = r.v; a.rec_g = r.g;
+    float2* ra;
+    uint32_t *rv, *rg;
+    scan_record_arrays(rec, B, L, H, N, D, &ra, &rv, &rg);
+    a.rec_a = ra; a.rec_v = rv; a.rec_g = rg;
     a.h0 = h0;
     a.y = static_cast<__nv_bfloat16*>(y);
     a.final_state = final_state; a.tail_state = tail_state;

@@ -1,0 +1,166 @@
+// Per-token records of the tensor-core scans: dynamics (dynamics_fused.cu:64-139) and the vp scale of block.py:194-195, every
+// result rounded to bf16 like the reference's stores (the transition optionally not).
+//
+// The gates lie heads-fastest, the scans want a head's tokens side by side.  A block takes 32 tokens of 8 or 16 heads, reads
+// the gates with the heads across the lanes, and turns its results around in shared memory, so that both sides move whole
+// sectors; a thread has the loads of all its values in flight before the first transcendental.  Bounded by issue slots and the
+// special-function unit (a pair takes some hundred instructions, nine of them special functions).
+// Measured on B200: 393 216 token-heads, N 16: 58 -> 27 us against one pair at a time with two barriers each; N 2, 7.7 -> 7.5,
+// and 2.1 M token-heads 27 -> 26 us against a thread per token-head that wrote its 16-byte record straight to memory.
+#include "cdssm_common.cuh"
+#include <algorithm>
+
+namespace cdssm {
+namespace records {
+
+constexpr int kTokens = 32, kThreads = 256;
+
+struct Args {
+    const __nv_bfloat16 *v, *gate_raw;
+    const float *log_dt_scale, *rope_freqs;
+    uint4* rec;                    // kWa: {a_re, a_im | v pair | beta, sel_C} (B, 32-token blocks, H, 32)
+    float2* rec_a;                 // else: transition (B,NC,H,NP,C)
+    uint32_t *rec_v, *rec_g;       // vp-scaled v (B,NC,H,NP,C); beta and sel_C (B,NC,H,C), bf16 pairs
+    int* status;                   // cleared here for the passes that follow, or nullptr
+    DynConsts dc;
+    int B, L, H, N, C, NC, pos0, segs, fp32_decay, tiles;   // tiles: 32-token tiles per batch row, chunks padded to full length
+};
+
+__device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+// kNP: pair slots (>= N / 2); kHg: heads per block.
+template <int kNP, int kHg, bool kWa>
+__global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
+    using T = __nv_bfloat16;
+    constexpr int kItems = kTokens * kHg / kThreads, kRow = kTokens + 1;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint4* sr = reinterpret_cast<uint4*>(smem);                        // kWa: [head][token]
+    float2* sa = reinterpret_cast<float2*>(smem);                      // else [pair][head][token]
+    uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
+    uint32_t* sg = sv + kNP * kHg * kRow;
+    grid_launch_dependents();
+    if (a.status != nullptr && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) *a.status = 0;
+    const int H = a.H, N = a.N, NP = N >> 1;
+    const int b = (int)(blockIdx.x / (unsigned)a.tiles), tile = (int)(blockIdx.x - (unsigned)b * a.tiles), l0 = tile * kTokens;
+    const int head0 = blockIdx.y * kHg, heads = min(kHg, H - head0);
+    const int head = threadIdx.x & (kHg - 1), hd = head0 + min(head, heads - 1);
+    const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
+    T x[kItems][5], ga[kItems][kNP], gw[kItems][kNP];
+    uint32_t vv[kItems][kNP];
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const int l = min(l0 + (int)(threadIdx.x / kHg) + i * (kThreads / kHg), a.L - 1);
+        const size_t row = (size_t)b * a.L + l;
+        const T* g = a.gate_raw + row * (size_t)((N + 5) * H) + hd;
+        const uint32_t* v = reinterpret_cast<const uint32_t*>(a.v) + (row * H + hd) * NP;
+#pragma unroll
+        for (int s = 0; s < 5; s++) x[i][s] = g[(N + s) * H];
+#pragma unroll
+        for (int p = 0; p < kNP; p++) {
+            const int pp = p < NP ? p : 0;
+            ga[i][p] = g[pp * H];
+            gw[i][p] = g[(NP + pp) * H];
+            vv[i][p] = v[pp];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const int t = (int)(threadIdx.x / kHg) + i * (kThreads / kHg), l = l0 + t;
+        const bool on = l < a.L;                                       // behind the end a = 1, beta = v = 0: the state stands still
+        const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
+        auto f = [](T y) { return __bfloat162float(y); };
+        const DynShared ds = dyn_shared<true>(f(ga[i][0]), f(gw[i][0]), f(x[i][0]), f(x[i][1]), f(x[i][2]), f(x[i][3]), f(x[i][4]),
+                                              lds, freq, pos, a.dc);
+        const uint32_t bs = on ? pack2(ds.beta, ds.sel_c) : 0u;
+        if (!kWa) sg[head * kRow + t] = bs;
+#pragma unroll
+        for (int p = 0; p < kNP; p++) {
+            if (p >= NP) break;
+            float ar, ai, vp;
+            dyn_pair<true>(f(ga[i][p]), f(gw[i][p]), freq, pos, ds, ar, ai, vp);
+            if (!a.fp32_decay) { ar = bfr(ar); ai = bfr(ai); }
+            vp = bfr(vp);
+            const float v0 = __uint_as_float(vv[i][p] << 16), v1 = __uint_as_float(vv[i][p] & 0xffff0000u);
+            const uint32_t vg = on ? pack2(v0 * vp, v1 * vp) : 0u;
+            if (!on) { ar = 1.f; ai = 0.f; }
+            if (kWa) {
+                sr[head * kRow + t] = make_uint4(__float_as_uint(ar), __float_as_uint(ai), vg, bs);
+            } else {
+                sa[(p * kHg + head) * kRow + t] = make_float2(ar, ai);
+                sv[(p * kHg + head) * kRow + t] = vg;
+            }
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (kWa) {
+        for (int h = warp; h < heads; h += kThreads / 32)
+            a.rec[(((size_t)b * a.tiles + tile) * H + head0 + h) * kTokens + lane] = sr[h * kRow + lane];
+    } else {
+        const int c = l0 / a.C, in_chunk = l0 - c * a.C;
+        const size_t unit0 = ((size_t)b * a.NC + c) * H + head0;
+        for (int i = warp; i < heads * NP; i += kThreads / 32) {
+            const int h = i / NP, p = i - h * NP, s = (p * kHg + h) * kRow + lane;
+            const size_t o = ((unit0 + h) * NP + p) * a.C + in_chunk + lane;
+            a.rec_a[o] = sa[s];
+            a.rec_v[o] = sv[s];
+        }
+        for (int h = warp; h < heads; h += kThreads / 32) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sg[h * kRow + lane];
+    }
+}
+
+template <int kNP, int kHg, bool kWa> struct KernelTag {};
+template <int kNP, int kHg, bool kWa>
+static int launch(const Args& a, cudaStream_t st) {
+    const size_t smem = kWa ? (size_t)kHg * (kTokens + 1) * 16 : (size_t)kHg * (kTokens + 1) * (kNP * 12 + 4);
+    if (smem > 48 * 1024)
+        if (int rc = allow_smem<KernelTag<kNP, kHg, kWa>>((const void*)records_kernel<kNP, kHg, kWa>, smem)) return rc;
+    records_kernel<kNP, kHg, kWa><<<dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg), kThreads, smem, st>>>(a);
+    return check_launch();
+}
+// 16 heads fill the sectors of the gate rows; 8 where that leaves fewer lanes empty (24 heads) or more blocks are wanted.
+template <int kNP, bool kWa>
+static int launch_group(const Args& a, cudaStream_t st) {
+    return (a.H + 15) / 16 * 16 > (a.H + 7) / 8 * 8 || (long long)a.B * a.tiles * a.H < 148 * 64 ? launch<kNP, 8, kWa>(a, st)
+                                                                                               : launch<kNP, 16, kWa>(a, st);
+}
+
+}  // namespace records
+
+// Bytes of the records: transition and scaled v per pair, beta and sel_C (both layouts).
+size_t scan_record_bytes(int B, int L, int H, int N, int C) {
+    return (size_t)B * (((size_t)L + C - 1) / C) * H * C * ((size_t)(N / 2) * 12 + 4);
+}
+
+// The three arrays of the layout of scan_chunk.cu inside the record buffer.
+void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a, uint32_t** v, uint32_t** g) {
+    const size_t n = (size_t)B * (((size_t)L + C - 1) / C) * H * C;
+    *a = static_cast<float2*>(rec);
+    *v = reinterpret_cast<uint32_t*>(*a + n * (N / 2));
+    *g = *v + n * (N / 2);
+}
+
+// Fills the records every pass over the same inputs reads.  wa: the layout of scan_wa.cu (N = 2), else of scan_chunk.cu.
+int scan_records(bool wa, const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
+                 int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
+                 cudaStream_t st) {
+    using namespace records;
+    Args a;
+    a.v = static_cast<const __nv_bfloat16*>(v);
+    a.gate_raw = static_cast<const __nv_bfloat16*>(gate_raw);
+    a.log_dt_scale = log_dt_scale; a.rope_freqs = rope_freqs;
+    a.rec = static_cast<uint4*>(rec);
+    scan_record_arrays(rec, B, L, H, N, C, &a.rec_a, &a.rec_v, &a.rec_g);
+    a.status = status;
+    a.dc = dc;
+    a.B = B; a.L = L; a.H = H; a.N = N; a.C = C; a.NC = (L + C - 1) / C; a.pos0 = pos0; a.segs = segs; a.fp32_decay = fp32_decay;
+    a.tiles = a.NC * (C / kTokens);
+    if ((long long)B * a.tiles > 0x7fffffff || H > 8 * 65535) return CDSSM_ERR_UNSUPPORTED;
+    if (wa) return launch_group<1, true>(a, st);
+    if (N <= 2) return launch_group<1, false>(a, st);
+    if (N <= 4) return launch_group<2, false>(a, st);
+    if (N <= 8) return launch_group<4, false>(a, st);
+    return launch_group<8, false>(a, st);
+}
+
+}  // namespace cdssm

@@ -737,20 +737,18 @@ using namespace cdssm;
 
 namespace cdssm {
 unsigned long long wait_limit_ns();   // c_abi.cu
+// scan_records.cu
+size_t scan_record_bytes(int B, int L, int H, int N, int C);
+int scan_records(bool wa, const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
+                 int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
+                 cudaStream_t st);
 // scan_wa.cu
 bool scan_wa_supported(int D, int N, int C, int H, int dtype);
-int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs,
-                     void* rec, int* status, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
-                     cudaStream_t st);
 int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  cudaStream_t st);
 // scan_chunk.cu
 bool scan_chunk_supported(int D, int N, int C, int dtype);
-size_t scan_chunk_record_bytes(int B, int L, int H, int N, int C);
-int scan_chunk_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                        int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
-                        int fp32_decay, cudaStream_t st);
 int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const float* h0, void* y, float* final_state,
                     float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
                     int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
@@ -769,7 +767,7 @@ extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int
     if (B <= 0 || L <= 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return 0;
     size_t bytes = simt_workspace_bytes(B, L, H, D, N, C);
     // per-token records of the tensor-core kernels (the data type is not known here)
-    if (scan_chunk_supported(D, N, C, CDSSM_BF16)) bytes += align256(scan_chunk_record_bytes(B, L, H, N, C));
+    if (scan_chunk_supported(D, N, C, CDSSM_BF16)) bytes += align256(scan_record_bytes(B, L, H, N, C));
     return bytes;
 }
 
@@ -837,15 +835,14 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                                           align256((size_t)a.units * 2 * sizeof(float)));
     cudaStream_t st = (cudaStream_t)stream;
     // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 with heads in fours (scan_wa.cu), any other
-    // N <= 16 (scan_chunk.cu).  The latter also where N = 2 has few chunks: four launches, of which two walk a chunk in
-    // sub-blocks, take 27 us (D 128: 39) however little there is to do, one kernel and the dynamics before it 14 to 20
-    // (D 64, 216 / 512 / 936 units: 25 / 26 / 36 against 27 / 28 / 32 us; D 128, 160 / 256 / 512: 30 / 32 / 65 against
-    // 41 / 41 / 44).  They read v and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the
-    // contract allows, stay on the CUDA-core kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the
-    // tests to check each tensor-core pass alone.)
+    // N <= 16 (scan_chunk.cu).  The latter also for a few chunks of N = 2, which it does in one kernel behind the records'
+    // where scan_wa.cu takes three, two of them walking a chunk in sub-blocks (us, one chunk: 17 / 22 at D 64, 20 / 30 at
+    // D 128; nine chunks of 24 heads of 64: 22 / 20; five and seven chunks of 4 heads of 128: 28 / 31, 29 / 32).  They read v
+    // and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the contract allows, stay on the CUDA-core
+    // kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the tests to check each tensor-core pass alone.)
     const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y) & 3) == 0 && !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
     const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, H, dtype) &&
-                       ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || (long long)B * a.NC * H > (D == 64 ? 512 : 256));
+                       ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > (D == 64 ? 2 : 7) || (long long)B * a.NC * H > (D == 64 ? 512 : 256));
     const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
     if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && !wa_ok) return CDSSM_ERR_UNSUPPORTED;
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
@@ -884,10 +881,8 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     };
     // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)
     if (a.run_local || (flags & CDSSM_SCAN_TENSOR_CORE_WA)) {
-        const int rc = wa_ok ? scan_wa_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, status, a.dc, B, L, H, C, pos0, segs,
-                                                a.fp32_decay, st)
-                             : scan_chunk_dynamics(v, gate_raw, log_dt_scale, rope_freqs, rec, one_kernel ? nullptr : status, a.dc,
-                                                   B, L, H, N, C, pos0, segs, a.fp32_decay, st);
+        const int rc = scan_records(wa_ok, v, gate_raw, log_dt_scale, rope_freqs, rec, one_kernel ? nullptr : status, a.dc, B, L, H,
+                                    N, C, pos0, segs, a.fp32_decay, st);
         if (rc) return rc;
     }
     if (one_kernel) return pass(2);

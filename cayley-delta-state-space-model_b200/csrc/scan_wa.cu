@@ -113,7 +113,7 @@ __device__ __forceinline__ ItemPos item_pos(const Args& a, int item) {
     return p;
 }
 
-// Record of one (token, head): {a_re | a_im | vg_re, vg_im | beta, sel_C}: the transition as two floats (bf16
+// Record of one (token, head), from scan_records.cu: {a_re | a_im | vg_re, vg_im | beta, sel_C}: the transition as two floats (bf16
 // values like the reference's storage unless the caller asked for a float32 transition), the rest as bf16
 // pairs.  Layout (B, blocks of 32 tokens, H, 32): the 32 tokens of a head's
 // sub-block are contiguous, so a warp fetches its step with one 512-byte load.
@@ -828,54 +828,6 @@ scan_wa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------------------------------
-// Dynamics pre-pass: one thread per (token, head), heads fastest (the gate rows are read coalesced).
-// dynamics_fused.cu:64-139 and the vp scale of block.py:194-195, every result rounded to bf16 like the
-// reference's stores.  Both scan passes read the 16-byte records instead of repeating the transcendental
-// chain inside their sequential walks.
-// ------------------------------------------------------------------------------------------
-struct DynArgs {
-    const __nv_bfloat16 *v, *gate_raw;
-    const float *log_dt_scale, *rope_freqs;
-    uint4* rec;
-    DynConsts dc;
-    int B, L, H, NB, pos0, segs;   // NB: 32-token blocks per batch row (chunks padded to full length)
-    int* status;                   // cleared here for the passes that follow
-    int fp32_decay;                // 0: the transition is rounded to bf16 like the reference's A_bar store
-};
-__global__ void __launch_bounds__(256) wa_dynamics_kernel(const DynArgs a) {
-    using T = __nv_bfloat16;
-    grid_launch_dependents();
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x, total = (uint32_t)a.B * a.L * a.H;   // below 2^32 (host)
-    if (idx == 0) *a.status = 0;
-    if (idx >= total) return;
-    const uint32_t bl = idx / (uint32_t)a.H;
-    const int hd = (int)(idx - bl * a.H);
-    const int b = (int)(bl / (uint32_t)a.L), l = (int)(bl - (uint32_t)b * a.L);
-    const int H = a.H;
-    const T* gr = a.gate_raw + (size_t)bl * (size_t)(7 * H);
-    const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
-    const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
-    const float g0 = IO<T>::ld(gr + hd), g1 = IO<T>::ld(gr + H + hd);
-    DynShared ds = dyn_shared<true>(g0, g1, IO<T>::ld(gr + 2 * H + hd), IO<T>::ld(gr + 3 * H + hd),
-                                    IO<T>::ld(gr + 4 * H + hd), IO<T>::ld(gr + 5 * H + hd), IO<T>::ld(gr + 6 * H + hd),
-                                    lds, freq, pos, a.dc);
-    float ar, ai, vp;
-    dyn_pair<true>(g0, g1, freq, pos, ds, ar, ai, vp);
-    vp = bfr(vp);
-    if (!a.fp32_decay) {
-        ar = bfr(ar);
-        ai = bfr(ai);
-    }
-    const __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(a.v + ((size_t)bl * H + hd) * 2);
-    uint4 r;
-    r.x = __float_as_uint(ar);
-    r.y = __float_as_uint(ai);
-    r.z = pack2(__low2float(v2) * vp, __high2float(v2) * vp);
-    r.w = pack2(ds.beta, ds.sel_c);
-    a.rec[(((size_t)b * a.NB + (l >> 5)) * H + hd) * kSub + (l & 31)] = r;
-}
-
-// ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
 #ifdef CDSSM_WA_TRACE
@@ -906,25 +858,6 @@ extern "C" __attribute__((visibility("default"))) int cdssm_b200_wa_trace_read(l
 
 bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
     return dtype == CDSSM_BF16 && N == 2 && D == C && (D == 64 || D == 128) && H % 4 == 0;
-}
-
-// Dynamics pre-pass: fills rec (16 bytes per token-head, chunks padded to full length: scan_chunk_record_bytes at N = 2) for both scan passes.
-int scan_wa_dynamics(const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs,
-                     void* rec, int* status, const DynConsts& dc, int B, int L, int H, int C, int pos0, int segs, int fp32_decay,
-                     cudaStream_t st) {
-    wa::DynArgs d;
-    d.status = status;
-    d.v = static_cast<const __nv_bfloat16*>(v);
-    d.gate_raw = static_cast<const __nv_bfloat16*>(gate_raw);
-    d.log_dt_scale = log_dt_scale; d.rope_freqs = rope_freqs;
-    d.rec = static_cast<uint4*>(rec);
-    d.dc = dc;
-    d.B = B; d.L = L; d.H = H; d.NB = ((L + C - 1) / C) * (C / wa::kSub); d.pos0 = pos0; d.segs = segs;
-    d.fp32_decay = fp32_decay;
-    const long long total = (long long)B * L * H;
-    if (total > 0xffffff00LL) return CDSSM_ERR_UNSUPPORTED;
-    wa::wa_dynamics_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d);
-    return check_launch();
 }
 
 // One pass of the warp-autonomous tensor-core scan over every chunk.  output = false: local pass (fills
