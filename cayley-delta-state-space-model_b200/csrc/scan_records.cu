@@ -38,7 +38,6 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     float2* sa = reinterpret_cast<float2*>(smem);                      // else [pair][head][token]
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
-    grid_launch_dependents();
     if (a.status != nullptr && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) *a.status = 0;
     const int H = a.H, N = a.N, NP = N >> 1;
     const int b = (int)(blockIdx.x / (unsigned)a.tiles), tile = (int)(blockIdx.x - (unsigned)b * a.tiles), l0 = tile * kTokens;
@@ -92,6 +91,7 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
         }
     }
     __syncthreads();
+    grid_launch_dependents();   // (not earlier: blocks that start while these fill the SMs are packed onto the few with room)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (kWa) {
         for (int h = warp; h < heads; h += kThreads / 32)

@@ -40,6 +40,8 @@ struct ScanArgs {
     int run_output;       // 0: stop after the carry pass (another kernel writes y)
     int publish;          // 0: summary only, the carry pass leaves the local results in place
     int fp32_decay;       // 1: the transition a_t keeps float32 precision (the reference stores it as bf16)
+    float4* rec_av;    // (B,NC,H,NP,C): transition and scaled v of a token, or NULL: the walk computes them itself
+    float2* rec_bs;    // (B,NC,H,C): beta and sel_C
     float* ws_gamma;   // (B,NC,H,NP,2)
     float* ws_state;   // (B,NC,H,NP,2,D): z_{C-1} after the local pass, s_c after the carry pass
     DynConsts dc;
@@ -58,51 +60,88 @@ struct ChunkScalars {
     }
 };
 
-// Dynamics of the unit's chunk: lane g handles tokens g, g+8, ...  (dynamics_fused.cu:64-139
-// and the vp scale of block.py:194-195).  Padded positions (l >= L) get a = k = v = beta = 0
-// like the reference's zero padding (ssd.py:60-67).
+// Dynamics of one (token, head): what its pairs share, then pair j (dynamics_fused.cu:64-139 and the vp scale of
+// block.py:194-195).
+template <typename T>
+struct TokenDynamics {
+    const T *gr, *vrow;
+    DynShared ds;
+    float freq, pos;
+    int H, NH, fp32_decay;
+    __device__ __forceinline__ TokenDynamics(const ScanArgs& a, int b, int l, int hd) {
+        H = a.H; NH = a.N >> 1; fp32_decay = a.fp32_decay;
+        const long long bl = (long long)b * a.L + l;
+        gr = static_cast<const T*>(a.gate_raw) + bl * (long long)((a.N + 5) * H) + hd;
+        vrow = static_cast<const T*>(a.v) + (bl * H + hd) * a.N;
+        const T* s5 = gr + a.N * H;
+        freq = a.rope_freqs[hd];
+        pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
+        ds = dyn_shared<IO<T>::kBf16>(IO<T>::ld(gr), IO<T>::ld(gr + NH * H), IO<T>::ld(s5), IO<T>::ld(s5 + H),
+                                      IO<T>::ld(s5 + 2 * H), IO<T>::ld(s5 + 3 * H), IO<T>::ld(s5 + 4 * H),
+                                      a.log_dt_scale[hd], freq, pos, a.dc);
+    }
+    __device__ __forceinline__ float2 beta_sel() const { return make_float2(IO<T>::rnd(ds.beta), IO<T>::rnd(ds.sel_c)); }
+    __device__ __forceinline__ float4 pair(int j) const {
+        float ar, ai, vp;
+        dyn_pair<IO<T>::kBf16>(IO<T>::ld(gr + j * H), IO<T>::ld(gr + (NH + j) * H), freq, pos, ds, ar, ai, vp);
+        if (!fp32_decay) {
+            ar = IO<T>::rnd(ar);
+            ai = IO<T>::rnd(ai);
+        }
+        vp = IO<T>::rnd(vp);
+        return make_float4(ar, ai, IO<T>::rnd(IO<T>::ld(vrow + 2 * j) * vp), IO<T>::rnd(IO<T>::ld(vrow + 2 * j + 1) * vp));
+    }
+};
+
+// The dynamics of every (token, head) before the walks: a warp takes four tokens of eight heads.  Computed by the walks
+// themselves, eight tokens in a row per lane, they were 10 us (float32: 15) of each of the two walks whatever the size.
+template <typename T>
+__global__ void __launch_bounds__(256) simt_records_kernel(const ScanArgs a) {
+    const int lt = threadIdx.x >> 3 & 3, lh = threadIdx.x & 7, warp = threadIdx.x >> 5;
+    const long long tok = (long long)blockIdx.x * 32 + warp * 4 + lt;
+    const int hd = blockIdx.y * 8 + lh;
+    if (tok >= (long long)a.B * a.L || hd >= a.H) return;
+    const int b = (int)(tok / a.L), l = (int)(tok % a.L), c = l / a.C, t = l % a.C, NH = a.N >> 1;
+    const TokenDynamics<T> d(a, b, l, hd);
+    const size_t unit = ((size_t)b * a.NC + c) * a.H + hd;
+    a.rec_bs[unit * a.C + t] = d.beta_sel();
+    for (int j = blockIdx.z; j < NH; j += gridDim.z) a.rec_av[(unit * NH + j) * a.C + t] = d.pair(j);
+    // (at the end: dependents that start while these blocks fill the SMs are packed onto the few with room, and a walk of
+    // 24 blocks of head_dim 128 took 104 us instead of 21)
+    grid_launch_dependents();
+}
+
+// Scalars of the unit's chunk into shared memory: lane g handles tokens g, g+8, ...  Padded positions (l >= L) get
+// a = k = v = beta = 0 like the reference's zero padding (ssd.py:60-67).
 template <typename T, int kLanes>
 __device__ __forceinline__ void stage_dynamics(const ScanArgs& a, ChunkScalars& sm, int ul, int g,
                                                int b, int c, int hd, int j) {
-    const T* gate = static_cast<const T*>(a.gate_raw);
-    const T* vv = static_cast<const T*>(a.v);
-    const int NH = a.N >> 1, H = a.H;
-    const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
-    for (int t = g; t < a.C; t += kLanes) {
-        const int l = c * a.C + t;
-        float ar = 0.f, ai = 0.f, be = 0.f, vr = 0.f, vi = 0.f, sc = 0.f;
-        if (l < a.L) {
-            const long long bl = (long long)b * a.L + l;
-            const T* gr = gate + bl * (long long)((a.N + 5) * H);
-            const T* s5 = gr + a.N * H;
-            const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
-            DynShared ds = dyn_shared<IO<T>::kBf16>(IO<T>::ld(gr + hd), IO<T>::ld(gr + NH * H + hd),
-                                      IO<T>::ld(s5 + hd), IO<T>::ld(s5 + H + hd),
-                                      IO<T>::ld(s5 + 2 * H + hd), IO<T>::ld(s5 + 3 * H + hd),
-                                      IO<T>::ld(s5 + 4 * H + hd), lds, freq, pos, a.dc);
-            float vp;
-            dyn_pair<IO<T>::kBf16>(IO<T>::ld(gr + j * H + hd), IO<T>::ld(gr + (NH + j) * H + hd), freq, pos, ds,
-                     ar, ai, vp);
-            if (!a.fp32_decay) {
-                ar = IO<T>::rnd(ar);
-                ai = IO<T>::rnd(ai);
-            }
-            vp = IO<T>::rnd(vp);
-            be = IO<T>::rnd(ds.beta);
-            sc = IO<T>::rnd(ds.sel_c);
-            const T* vrow = vv + (bl * H + hd) * a.N + 2 * j;
-            vr = IO<T>::rnd(IO<T>::ld(vrow) * vp);
-            vi = IO<T>::rnd(IO<T>::ld(vrow + 1) * vp);
+    const int Lc = min(a.C, a.L - c * a.C), o0 = ul * a.C;
+    const size_t unit = ((size_t)b * a.NC + c) * a.H + hd;
+    auto put = [&](int t, float4 av, float2 bs) {
+        sm.a_re[o0 + t] = av.x; sm.a_im[o0 + t] = av.y; sm.beta[o0 + t] = bs.x;
+        sm.v_re[o0 + t] = av.z; sm.v_im[o0 + t] = av.w; sm.sel_c[o0 + t] = bs.y;
+    };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (a.rec_av != nullptr) {
+        const float4* av = a.rec_av + (unit * (a.N >> 1) + j) * a.C;
+        const float2* bs = a.rec_bs + unit * a.C;
+#pragma unroll 8
+        for (int t = g; t < Lc; t += kLanes) put(t, __ldcg(av + t), __ldcg(bs + t));
+    } else {
+        for (int t = g; t < Lc; t += kLanes) {
+            const TokenDynamics<T> d(a, b, c * a.C + t, hd);
+            put(t, d.pair(j), d.beta_sel());
         }
-        const int o = ul * a.C + t;
-        sm.a_re[o] = ar; sm.a_im[o] = ai; sm.beta[o] = be;
-        sm.v_re[o] = vr; sm.v_im[o] = vi; sm.sel_c[o] = sc;
     }
+    for (int t = Lc + (g - Lc % kLanes + kLanes) % kLanes; t < a.C; t += kLanes) put(t, zero, make_float2(0.f, 0.f));
 }
 
 // kOutput = false: local pass (z only).  kOutput = true: output pass (z, r, read-out).
 template <typename T, int kCols, int kLanes, bool kOutput>
-__global__ void __launch_bounds__(kSimtThreads, kOutput ? (kCols == 16 ? 4 : 6) : 1)
+// (No register cap: at most 6 resident blocks of 80 registers cost the output walk its overlap of a step's eleven sums, float32
+// 61 -> 34 us at 64 units and 173 -> 90 us at head_dim 128, bf16 with a full GPU 380 -> 368 us.)
+__global__ void __launch_bounds__(kSimtThreads, 1)
 scan_walk_kernel(const ScanArgs a) {
     constexpr int kUnits = kSimtThreads / kLanes;       // units per block
     extern __shared__ float smem[];
@@ -119,7 +158,11 @@ scan_walk_kernel(const ScanArgs a) {
     const int b = (int)(u / ((long long)NH * H * a.NC));
     const bool vec = (D == kCols * kLanes);              // rows are 16-byte aligned slices
 
+    // The local walk waits for the records; the output walk is launched when the carry pass, which has waited for the local
+    // one, begins: the records are there, and it waits for the carries only.
+    if (!kOutput) grid_dependency_wait();
     stage_dynamics<T, kLanes>(a, sm, ul, g, b, c, hd, j);
+    if (kOutput) grid_dependency_wait();
     __syncwarp();
 
     const int Lc = min(C, a.L - c * C);                  // valid tokens of this chunk
@@ -430,7 +473,6 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 scan_carry_kernel(const ScanArgs a) {
     grid_dependency_wait();
-    grid_launch_dependents();
     const int NH = a.N >> 1, D = a.D, H = a.H, NC = a.NC;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)a.B * H * NH * D) return;
@@ -473,6 +515,7 @@ scan_carry_kernel(const ScanArgs a) {
             }
         }
     }
+    grid_launch_dependents();
     if (a.final_state) { a.final_state[so] = sr; a.final_state[so + D] = si; }
     if (a.total_decay && d == 0) {
         float* td = a.total_decay + ((long long)b * H + hd) * a.N + 2 * j;
@@ -481,42 +524,40 @@ scan_carry_kernel(const ScanArgs a) {
     }
 }
 
-template <typename T, int kCols, int kLanes>
+template <typename T, int kCols, bool kOutput> struct WalkTag {};
+
+template <typename T, int kCols>
 static int launch_simt(const ScanArgs& a, cudaStream_t st) {
-    constexpr int kUnits = kSimtThreads / kLanes;
+    constexpr int kLanes = kLanesPerUnit, kUnits = kUnitsPerBlock;
     const size_t smem = (size_t)6 * kUnits * a.C * sizeof(float);
     if (smem > 48 * 1024) {   // opt in to more than 48 KB of dynamic shared memory
-        if (int rc = check_cuda(cudaFuncSetAttribute(scan_walk_kernel<T, kCols, kLanes, false>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
-            return rc;
-        if (int rc = check_cuda(cudaFuncSetAttribute(scan_walk_kernel<T, kCols, kLanes, true>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
-            return rc;
+        constexpr size_t kMost = (size_t)6 * kUnits * kMaxChunk * sizeof(float);
+        if (int rc = allow_smem<WalkTag<T, kCols, false>>((const void*)scan_walk_kernel<T, kCols, kLanes, false>, kMost)) return rc;
+        if (int rc = allow_smem<WalkTag<T, kCols, true>>((const void*)scan_walk_kernel<T, kCols, kLanes, true>, kMost)) return rc;
     }
     const unsigned blocks = (unsigned)((a.units + kUnits - 1) / kUnits);
-    if (a.run_local) {
-        scan_walk_kernel<T, kCols, kLanes, false><<<blocks, kSimtThreads, smem, st>>>(a);
+    const bool output = a.y != nullptr && a.run_output;   // else: summary only, or y comes from another kernel
+    if (a.rec_av != nullptr && (a.run_local || output)) {
+        // pairs over the grid as far as one wave goes (what the pairs of a token share is computed again for each)
+        const long long wave = ((long long)a.B * a.L + 31) / 32 * ((a.H + 7) / 8);
+        const int pairs = wave >= 1024 ? 1 : (int)min((long long)(a.N / 2), 1024 / wave);
+        simt_records_kernel<T><<<dim3((unsigned)(((long long)a.B * a.L + 31) / 32), (a.H + 7) / 8, pairs), 256, 0, st>>>(a);
         if (int rc = check_launch()) return rc;
     }
+    if (a.run_local)
+        if (int rc = launch_overlapped(scan_walk_kernel<T, kCols, kLanes, false>, dim3(blocks), dim3(kSimtThreads), smem, st, a)) return rc;
     const long long th = (long long)a.B * a.H * (a.N / 2) * a.D;
     if (int rc = launch_overlapped(scan_carry_kernel<T>, dim3((unsigned)((th + 127) / 128)), dim3(128), 0, st, a)) return rc;
-    if (a.y == nullptr || !a.run_output) return CDSSM_OK;   // summary only, or y comes from another kernel
-    scan_walk_kernel<T, kCols, kLanes, true><<<blocks, kSimtThreads, smem, st>>>(a);
-    return check_launch();
+    if (!output) return CDSSM_OK;
+    return launch_overlapped(scan_walk_kernel<T, kCols, kLanes, true>, dim3(blocks), dim3(kSimtThreads), smem, st, a);
 }
 
-// Column split: D <= 64 -> 8 lanes x 8 columns; D <= 128 -> 8 lanes x 16 columns, or (wide) 16 lanes x 8
-// columns, which halves the state registers per thread and doubles the resident warps - measured
-// slower on B200 (10.8 ms against 8.9 ms at the benchmark size: the per-unit scalar work and the extra
-// shuffle stage cost more than the occupancy gains), so the narrow split is the one used.
-int scan_fused_simt(const ScanArgs& a, int dtype, bool wide, cudaStream_t st) {
+// Column split: D <= 64 -> 8 lanes x 8 columns, D <= 128 -> 8 lanes x 16 columns (16 lanes x 8 columns was slower: 10.8 ms
+// against 8.9 ms at B 16, H 32, L 65536).
+int scan_fused_simt(const ScanArgs& a, int dtype, cudaStream_t st) {
     const int cols = (a.D + kLanesPerUnit - 1) / kLanesPerUnit;
-    if (dtype == CDSSM_BF16) {
-        if (cols <= 8) return launch_simt<__nv_bfloat16, 8, 8>(a, st);
-        return wide ? launch_simt<__nv_bfloat16, 8, 16>(a, st) : launch_simt<__nv_bfloat16, 16, 8>(a, st);
-    }
-    if (cols <= 8) return launch_simt<float, 8, 8>(a, st);
-    return wide ? launch_simt<float, 8, 16>(a, st) : launch_simt<float, 16, 8>(a, st);
+    if (dtype == CDSSM_BF16) return cols <= 8 ? launch_simt<__nv_bfloat16, 8>(a, st) : launch_simt<__nv_bfloat16, 16>(a, st);
+    return cols <= 8 ? launch_simt<float, 8>(a, st) : launch_simt<float, 16>(a, st);
 }
 
 }  // namespace cdssm
@@ -756,19 +797,20 @@ int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const flo
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// What the CUDA-core kernels need: status word, chunk decays, chunk states.
-static size_t simt_workspace_bytes(int B, int L, int H, int D, int N, int C) {
+// What every path needs: status word, chunk decays, chunk states.
+static size_t base_workspace_bytes(int B, int L, int H, int D, int N, int C) {
     const size_t NC = ((size_t)L + C - 1) / C;
     const size_t units = (size_t)B * NC * H * (N / 2);
     return 256 + align256(units * 2 * sizeof(float)) + align256(units * 2 * D * sizeof(float));
 }
+// Per-token records of the CUDA-core walks; never less than those of the tensor-core kernels (scan_record_bytes).
+static size_t simt_record_bytes(int B, int L, int H, int N, int C) {
+    return (size_t)B * (((size_t)L + C - 1) / C) * H * C * ((size_t)(N / 2) * sizeof(float4) + sizeof(float2));
+}
 
 extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int D, int N, int C) {
     if (B <= 0 || L <= 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return 0;
-    size_t bytes = simt_workspace_bytes(B, L, H, D, N, C);
-    // per-token records of the tensor-core kernels (the data type is not known here)
-    if (scan_chunk_supported(D, N, C, CDSSM_BF16)) bytes += align256(scan_record_bytes(B, L, H, N, C));
-    return bytes;
+    return base_workspace_bytes(B, L, H, D, N, C) + align256(simt_record_bytes(B, L, H, N, C));
 }
 
 extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_host, void* stream) {
@@ -799,7 +841,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                            void* workspace, size_t workspace_bytes, float gating_c, float omega_thresh,
                            float adt_delta, float adt_smoothness, float adt_eps, float shortcut_scale,
                            int B, int L, int H, int D, int N, int C, int pos0, int segs, int dtype,
-                           int flags, void* stream) {
+                           int flags, void* stream, bool small_workspace = false) {
     if (summary_only) { q = k; y = nullptr; tail_state = nullptr; }
     if (!q || !k || !v || !gate_raw || !log_dt_scale || !rope_freqs || (!y && !summary_only))
         return CDSSM_ERR_BAD_ARG;
@@ -809,8 +851,9 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (((uintptr_t)q | (uintptr_t)k) & 15) return CDSSM_ERR_BAD_ARG;   // 16-byte row loads
     if (N > kMaxStateDim || D > kMaxHeadDim || C > kMaxChunk) return CDSSM_ERR_UNSUPPORTED;
     if (B == 0 || L == 0) return CDSSM_OK;
-    const size_t need = (flags & CDSSM_SCAN_FORCE_SIMT) ? simt_workspace_bytes(B, L, H, D, N, C)
-                                                        : cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
+    // small_workspace: as many of the records as fit (the walks can do without)
+    const size_t base = base_workspace_bytes(B, L, H, D, N, C);
+    const size_t need = small_workspace ? base : cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return CDSSM_ERR_WORKSPACE;
     // first 256 bytes of the workspace: status word of the tensor-core kernel's bounded waits, ticket counter
     int* status = static_cast<int*>(workspace);
@@ -840,7 +883,8 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     // D 128; nine chunks of 24 heads of 64: 22 / 20; five and seven chunks of 4 heads of 128: 28 / 31, 29 / 32).  They read v
     // and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the contract allows, stay on the CUDA-core
     // kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the tests to check each tensor-core pass alone.)
-    const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y) & 3) == 0 && !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
+    const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y) & 3) == 0 && workspace_bytes - base >= scan_record_bytes(B, L, H, N, C) &&
+                           !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
     const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, H, dtype) &&
                        ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > (D == 64 ? 2 : 7) || (long long)B * a.NC * H > (D == 64 ? 512 : 256));
     const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
@@ -855,7 +899,15 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
         const size_t zero = one_kernel ? 256 + (size_t)a.units * 2 * sizeof(float) : sizeof(int);
         if (int rc = check_cuda(cudaMemsetAsync(status, 0, zero, st))) return rc;
     }
+    void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
+    a.rec_av = nullptr;
+    a.rec_bs = nullptr;
+    if (!tensor && workspace_bytes - base >= simt_record_bytes(B, L, H, N, C)) {
+        a.rec_av = static_cast<float4*>(rec);
+        a.rec_bs = reinterpret_cast<float2*>(a.rec_av + (size_t)a.units * C);
+    }
     if (flags & CDSSM_SCAN_EXACT) {
+        a.rec_av = nullptr;   // (its stages are not the chunks of the records)
         // the recurrent state after the last token is both the "carry" and the tail state
         const int cols = (D + kLanesPerUnit - 1) / kLanesPerUnit;
         float* extra = tail_state;
@@ -868,10 +920,9 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                                             cudaMemcpyDeviceToDevice, st));
         return rc;
     }
-    if (!tensor) return scan_fused_simt(a, dtype, false, st);
+    if (!tensor) return scan_fused_simt(a, dtype, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
-    void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, k, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
@@ -891,7 +942,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
         a.run_local = 0;
     }
     a.run_output = tc_output ? 0 : 1;
-    if (int rc = scan_fused_simt(a, dtype, false, st)) return rc;   // carry pass (+ whatever was kept)
+    if (int rc = scan_fused_simt(a, dtype, st)) return rc;   // carry pass (+ whatever was kept)
     return !tc_output || summary_only ? CDSSM_OK : pass(1);
 }
 
@@ -1021,13 +1072,11 @@ extern "C" int cdssm_b200_scan_fused_fwd_noalloc(const void* q, const void* k, c
                                          adt_smoothness, adt_eps, shortcut_scale, B, L, H, D, N, C, pos0,
                                          dtype, flags, stream);
     }
-    const size_t need = cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
-    if (need == 0) return CDSSM_ERR_BAD_ARG;
-    if (need > kNoAllocScratchBytes) {   // beyond the built-in scratch: without the tensor-core kernels' records, if that fits
-        if (simt_workspace_bytes(B, L, H, D, N, C) > kNoAllocScratchBytes || scan_wa_supported(D, N, C, H, dtype))
-            return CDSSM_ERR_WORKSPACE;
-        flags |= CDSSM_SCAN_FORCE_SIMT;
-    }
+    if (cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C) == 0) return CDSSM_ERR_BAD_ARG;
+    // beyond the built-in scratch?  (the records of the tensor-core kernel of N = 2 are part of it, others only as they fit)
+    size_t need = base_workspace_bytes(B, L, H, D, N, C);
+    if (scan_wa_supported(D, N, C, H, CDSSM_BF16)) need += align256(scan_record_bytes(B, L, H, N, C));
+    if (need > kNoAllocScratchBytes) return CDSSM_ERR_WORKSPACE;
     int dev = 0;
     if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;
     if (dev < 0 || dev >= kNoAllocMaxDevices) return CDSSM_ERR_UNSUPPORTED;
@@ -1040,10 +1089,9 @@ extern "C" int cdssm_b200_scan_fused_fwd_noalloc(const void* q, const void* k, c
     }
     // Nothing in the scratch has to start at zero except the status word, which the scan itself
     // clears on the stream; gamma/state slots are all written by the local pass before they are read.
-    return cdssm_b200_scan_fused_fwd(q, k, v, gate_raw, log_dt_scale, rope_freqs, h0, y, final_state,
-                                     tail_state, scratch, kNoAllocScratchBytes, gating_c,
-                                     omega_thresh, adt_delta, adt_smoothness, adt_eps, shortcut_scale, B, L,
-                                     H, D, N, C, pos0, dtype, flags, stream);
+    return scan_fused_impl(q, k, v, gate_raw, log_dt_scale, rope_freqs, h0, y, final_state, tail_state, nullptr, false,
+                           scratch, kNoAllocScratchBytes, gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps,
+                           shortcut_scale, B, L, H, D, N, C, pos0, 1, dtype, flags, stream, true);
 }
 
 extern "C" int cdssm_b200_scan_fused_noalloc_status(int* status_host, void* stream) {
