@@ -105,13 +105,11 @@ __device__ __forceinline__ void dyn_pair(float alpha_raw, float omega_raw, float
     vp = fminf(sqrtf(fmaxf(1.0f - eff, kEps)), 1.0f);
 }
 
-// s <- gamma s + l, real and imaginary part.  A fixed operation order: the carry pass and the kernel that hands the carry on
-// itself give the same bits, so results do not depend on which of them a length happens to take.
-__device__ __forceinline__ float carry_re(float gr, float gi, float sr, float si, float l) {
-    return __fmaf_rn(gr, sr, __fmaf_rn(-gi, si, l));
-}
-__device__ __forceinline__ float carry_im(float gr, float gi, float sr, float si, float l) {
-    return __fmaf_rn(gr, si, __fmaf_rn(gi, sr, l));
+// Value residual across layers (block.py:167-171): lerp(first, v, w) rounded like the eager operation's output.
+template <typename T>
+__device__ __forceinline__ float value_residual(float first, float v, float w) {
+    const float d = v - first;
+    return IO<T>::rnd(fabsf(w) < 0.5f ? first + w * d : v - d * (1.f - w));
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

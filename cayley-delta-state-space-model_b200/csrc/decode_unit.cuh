@@ -150,12 +150,11 @@ __device__ __forceinline__ void decode_unit(const DecodeUnitArgs& a, long long u
     const float be = IO<T>::rnd(ds.beta), sc = IO<T>::rnd(ds.sel_c);
     const T* vrow = static_cast<const T*>(a.v) + b * a.v_stride + (long long)hd * a.N + 2 * j;
     float v0 = IO<T>::ld(vrow), v1 = IO<T>::ld(vrow + 1);
-    if (a.v_first) {   // value residual across layers (block.py:167-171), rounded like the eager lerp's output
+    if (a.v_first) {
         const T* f = static_cast<const T*>(a.v_first) + b * a.v_first_stride + (long long)hd * a.N + 2 * j;
         const float w = IO<T>::ld(static_cast<const T*>(a.mix) + hd), f0 = IO<T>::ld(f), f1 = IO<T>::ld(f + 1);
-        const float d0 = v0 - f0, d1 = v1 - f1;
-        v0 = IO<T>::rnd(fabsf(w) < 0.5f ? f0 + w * d0 : v0 - d0 * (1.f - w));
-        v1 = IO<T>::rnd(fabsf(w) < 0.5f ? f1 + w * d1 : v1 - d1 * (1.f - w));
+        v0 = value_residual<T>(f0, v0, w);
+        v1 = value_residual<T>(f1, v1, w);
     }
     const float vr = IO<T>::rnd(v0 * vp), vi = IO<T>::rnd(v1 * vp);
 

@@ -88,6 +88,12 @@ Tensor groupnorm_gate(const Tensor& y, const Tensor& gw, const Tensor& gb, const
 Tensor conv1d_silu(const Tensor& x, const Tensor& w, const Tensor& b);
 Tensor conv1d_silu_step(const Tensor& x, const Tensor& hist, const Tensor& w, const Tensor& b);
 
+// ---- library products (gemm.cpp)
+constexpr size_t kGemmWorkspace = 32u << 20;   // what the library is given by default on this architecture
+Tensor gemm_workspace(const Tensor& on);
+void gemm(const Tensor& out, const Tensor& x, const Tensor& w, const Tensor& bias, bool accumulate, const Tensor& workspace);
+Tensor linear(const Tensor& x, const Tensor& w, const Tensor& bias, const Tensor& workspace);
+
 // ---- Python side helpers
 struct Args {   // positional arguments of a METH_FASTCALL function
     PyObject* const* a;

@@ -13,8 +13,8 @@ struct Block {
     Tensor norm_w, w_in, b_in, conv_w, conv_b, w_gate, b_gate, lds, rope, w_q, w_readout, w_out, gn_w, gn_b, D, v_gate, w_qg,
         b_qg;
     double shortcut = 0.0;
-    // views of the input projection's row blocks and of the transposed output projection
-    Tensor w_z, b_z, w_x, b_x, w_k, b_k, w_v, b_v, w_out_t;
+    // views of the input projection's row blocks
+    Tensor w_z, b_z, w_x, b_x, w_k, b_k, w_v, b_v;
     // sigmoid(v_residual_gate) in the activation type, recomputed when the parameter is written
     Tensor mix;
     uint32_t mix_version = 0;
@@ -77,14 +77,15 @@ Tensor norm_gate(const Plan& p, const Block& b, const Tensor& y, const Tensor& z
 struct Cache {
     Tensor state, conv;
 };
-void block_sequence(Plan& p, Block& b, const Tensor& x, Tensor& v_first, Cache* cache, bool per_token, int64_t flags) {
+void block_sequence(Plan& p, Block& b, const Tensor& x, Tensor& v_first, Cache* cache, bool per_token, int64_t flags,
+                    const Tensor& ws) {
     const int64_t B = x.size(0), L = x.size(1), H = p.heads, N = p.N, di = p.d_inner;
     const Tensor xn = rms_norm(x, b.norm_w, p.eps_norm);
     // One product per consumer (row blocks of the in_proj weight): each output is dense, so neither the conv nor the
     // scan has to copy a column slice of a wide projection first.
-    const Tensor z = at::linear(xn, b.w_z, b.b_z), x_gate = at::linear(xn, b.w_x, b.b_x);
-    const Tensor K = at::linear(xn, b.w_k, b.b_k).view({B, L, H, kHeadDim});
-    Tensor V = at::linear(xn, b.w_v, b.b_v).view({B, L, H, N});
+    const Tensor z = linear(xn, b.w_z, b.b_z, ws), x_gate = linear(xn, b.w_x, b.b_x, ws);
+    const Tensor K = linear(xn, b.w_k, b.b_k, ws).view({B, L, H, kHeadDim});
+    Tensor V = linear(xn, b.w_v, b.b_v, ws).view({B, L, H, N});
     if (!v_first.defined()) v_first = V;
     else V = at::lerp(v_first, V, b.residual_mix(V.scalar_type()).view({1, 1, H, 1}));   // value residual (block.py:167-171)
     const Tensor x_conv = conv1d_silu(x_gate, b.conv_w, b.conv_b);
@@ -96,38 +97,38 @@ void block_sequence(Plan& p, Block& b, const Tensor& x, Tensor& v_first, Cache* 
             cache->conv.slice(1, 3 - L, 3).copy_(x_gate);
         }
     }
-    const Tensor gates = at::linear(x_conv, b.w_gate, b.b_gate);
-    const Tensor Q = at::linear(x_conv, b.w_q).view({B, L, H, kHeadDim});
+    const Tensor gates = linear(x_conv, b.w_gate, b.b_gate, ws);
+    const Tensor Q = linear(x_conv, b.w_q, Tensor(), ws).view({B, L, H, kHeadDim});
     ScanOut s = scan_fused(Q, K, V, gates, b.lds, b.rope, p.dyn, H, N, p.chunk, Tensor(), b.shortcut, 0, cache != nullptr,
                            cache ? (L > kTensorPrompt ? kScanForceSimt : 0) : flags, Tensor(), 1);
     if (cache) cache->state = s.tail;
-    const Tensor y = at::linear(s.y.view({B, L, H * N}), b.w_readout);
+    const Tensor y = linear(s.y.view({B, L, H * N}), b.w_readout, Tensor(), ws);
     // The reference normalises over (channels of the group) x (ALL positions of the sequence) (block.py:216-222), which
     // makes its forward non-causal.  A cached decode cannot reproduce that, so with a cache - and in forward() when
     // per_token_group_norm is set - the statistics are taken per token instead.
     const Tensor o = norm_gate(p, b, y, z, x_conv, per_token || cache);
-    x.view({B * L, p.d_model}).addmm_(o.view({B * L, di}), b.w_out_t);   // the residual add rides in the epilogue
+    gemm(x.view({B * L, p.d_model}), o.view({B * L, di}), b.w_out, Tensor(), true, ws);   // the residual add rides in the epilogue
 }
 
 // One block of a one-token step; x (B,1,d) takes the residual sum in place.
 void block_step(Plan& p, Block& b, const Tensor& x, Tensor& v_first, const Tensor& state, const Tensor& conv, int64_t pos,
-                const Tensor& pos_dev) {
+                const Tensor& pos_dev, const Tensor& ws) {
     const int64_t B = x.size(0), H = p.heads, N = p.N, di = p.d_inner;
     const Tensor xn = rms_norm(x.view({B, p.d_model}), b.norm_w, p.eps_norm);
-    const Tensor proj = at::linear(xn, b.w_in, b.b_in);
+    const Tensor proj = linear(xn, b.w_in, b.b_in, ws);
     const Tensor z = proj.slice(1, 0, di).view({B, 1, di}), x_gate = proj.slice(1, di, 2 * di);
     const Tensor K = proj.slice(1, 2 * di, 3 * di).unflatten(1, {H, kHeadDim}), V = proj.slice(1, 3 * di).unflatten(1, {H, N});
     Tensor mix;
     if (!v_first.defined()) v_first = V.contiguous();   // one small copy per step; the kernels read it densely
     else mix = b.residual_mix(V.scalar_type());         // the decode kernel applies the value residual itself
     const Tensor x_conv = conv1d_silu_step(x_gate, conv, b.conv_w, b.conv_b);
-    const Tensor qg = at::linear(x_conv, b.w_qg, b.b_qg);   // one product for Q and the gates; the kernel reads slices
+    const Tensor qg = linear(x_conv, b.w_qg, b.b_qg, ws);   // one product for Q and the gates; the kernel reads slices
     const Tensor Q = qg.slice(1, 0, di).unflatten(1, {H, kHeadDim}), gates = qg.slice(1, di);
     Tensor y = decode_step(state, Q, K, V, gates, b.lds, b.rope, p.dyn, H, N, pos, pos_dev, b.shortcut, Tensor(),
                            mix.defined() ? v_first : Tensor(), mix);
-    y = at::linear(y.view({B, 1, H * N}), b.w_readout);
+    y = linear(y.view({B, 1, H * N}), b.w_readout, Tensor(), ws);
     const Tensor o = norm_gate(p, b, y, z, x_conv.view({B, 1, di}), true);
-    x.view({B, p.d_model}).addmm_(o.view({B, di}), b.w_out_t);
+    gemm(x.view({B, p.d_model}), o.view({B, di}), b.w_out, Tensor(), true, ws);
 }
 
 bool aligned_dense(const Tensor& t, at::ScalarType dt) {
@@ -164,7 +165,9 @@ bool decode_small_batch(Plan& p, const Tensor& x, const std::vector<Cache>& cach
 }
 
 Tensor embed(const Plan& p, const Tensor& ids) { return at::index(p.embedding, {std::optional<Tensor>(ids)}); }
-Tensor head(const Plan& p, const Tensor& x) { return at::linear(rms_norm(x, p.final_norm_w, kFinalEps), p.embedding); }
+Tensor head(const Plan& p, const Tensor& x, const Tensor& ws) {
+    return linear(rms_norm(x, p.final_norm_w, kFinalEps), p.embedding, Tensor(), ws);
+}
 
 struct NoGrad {
     c10::AutoGradMode no_grad{false};
@@ -198,7 +201,6 @@ PyObject* py_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
             b.w_x = rows(b.w_in, di, 2 * di); b.b_x = rows(b.b_in, di, 2 * di);
             b.w_k = rows(b.w_in, 2 * di, 3 * di); b.b_k = rows(b.b_in, 2 * di, 3 * di);
             b.w_v = rows(b.w_in, 3 * di, b.w_in.size(0)); b.b_v = rows(b.b_in, 3 * di, b.b_in.size(0));
-            b.w_out_t = b.w_out.t();
             bool ok = aligned_dense(b.lds, at::kFloat) && aligned_dense(b.rope, at::kFloat);
             for (const Tensor* w : {&b.norm_w, &b.w_in, &b.b_in, &b.conv_w, &b.conv_b, &b.w_qg, &b.b_qg, &b.w_readout, &b.w_out,
                                     &b.gn_w, &b.gn_b, &b.D})
@@ -225,8 +227,9 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const NoGrad ng;
         const c10::cuda::CUDAGuard guard(p.embedding.device());
         Tensor x = embed(p, ids), v_first;
-        for (Block& b : p.blocks) block_sequence(p, b, x, v_first, nullptr, per_token, flags);
-        return wrap(head(p, x));
+        const Tensor ws = gemm_workspace(x);
+        for (Block& b : p.blocks) block_sequence(p, b, x, v_first, nullptr, per_token, flags, ws);
+        return wrap(head(p, x, ws));
     });
 }
 
@@ -240,8 +243,9 @@ PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const NoGrad ng;
         const c10::cuda::CUDAGuard guard(p.embedding.device());
         Tensor x = embed(p, ids), v_first;
+        const Tensor ws = gemm_workspace(x);
         std::vector<Cache> caches(p.blocks.size());
-        for (size_t i = 0; i < p.blocks.size(); i++) block_sequence(p, p.blocks[i], x, v_first, &caches[i], true, 0);
+        for (size_t i = 0; i < p.blocks.size(); i++) block_sequence(p, p.blocks[i], x, v_first, &caches[i], true, 0, ws);
         if (last_only) x = x.slice(1, x.size(1) - 1, x.size(1));
         PyObject* list = PyList_New(2 * (Py_ssize_t)caches.size());
         if (!list) return nullptr;
@@ -249,7 +253,7 @@ PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
             PyList_SET_ITEM(list, 2 * i, wrap(caches[i].state));
             PyList_SET_ITEM(list, 2 * i + 1, wrap(caches[i].conv));
         }
-        PyObject* logits = wrap(head(p, x));
+        PyObject* logits = wrap(head(p, x, ws));
         return Py_BuildValue("(NN)", logits, list);
     });
 }
@@ -281,8 +285,9 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
             if (decode_small_batch(p, x, caches, logits, pos, pos_dev)) return wrap(logits);
         }
         x = x.view({B, 1, p.d_model});
-        for (size_t i = 0; i < layers; i++) block_step(p, p.blocks[i], x, v_first, caches[i].state, caches[i].conv, pos, pos_dev);
-        return wrap(head(p, x.view({B, p.d_model})));
+        const Tensor ws = gemm_workspace(x);
+        for (size_t i = 0; i < layers; i++) block_step(p, p.blocks[i], x, v_first, caches[i].state, caches[i].conv, pos, pos_dev, ws);
+        return wrap(head(p, x.view({B, p.d_model}), ws));
     });
 }
 

@@ -346,6 +346,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     const int tid = threadIdx.x, I = tid >> 5, tl = tid & 31, g = tl >> 2, t4 = tl & 3;
     const int H = a.H, N = a.N, NP = N >> 1, L = a.L;
 
+    if (kMode == kFused) grid_dependency_wait();   // (the records kernel clears the ticket counter)
     if (tid == 0) {
         mbar_init(&sm.full_k, 1);
         mbar_init(&sm.full_q, 1);
@@ -419,7 +420,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         diagonal_of(acc[1][2], acc[1][3], tl, kk[2], kk[3]);
         // the token's dynamics, from the kernel before this one (its launch let this one start early; no __ldg here: loads
         // that claim the data constant may be moved above the wait)
-        if (kMode != kOutput) grid_dependency_wait();
+        if (kMode == kLocal) grid_dependency_wait();
         grid_launch_dependents();
         {
             const uint32_t gg = __ldcg(a.rec_g + unit * kD + tid);
@@ -722,7 +723,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                             a.ws_state[(unit * N + n) * kD + d] = l;
                         } else {
                             const float sr = sm.s_in[2 * p][d], si = sm.s_in[2 * p + 1][d];
-                            const float s = comp ? carry_im(gam.r, gam.i, sr, si, l) : carry_re(gam.r, gam.i, sr, si, l);
+                            const float s = comp ? gam.r * si + gam.i * sr + l : gam.r * sr - gam.i * si + l;
                             if (c + 1 < a.NC) a.ws_state[((unit + H) * N + n) * kD + d] = s;
                             else if (a.final_state) a.final_state[(((size_t)b * H + hd) * N + n) * kD + d] = s;
                         }
@@ -1007,12 +1008,12 @@ void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a
 // mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the carries from ws_state,
 // writes y), 2: both in one kernel with the carry handed on inside it (ws_gamma and *ticket zeroed by the caller).
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
-int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const float* h0, void* y, float* final_state,
+int scan_chunk_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
                     float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
                     int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st) {
     using namespace chunk;
     CUtensorMap tmK, tmQ;
-    if (!make_tile_map(&tmK, k, B, L, H, D, D) || !make_tile_map(&tmQ, mode == 0 ? k : q, B, L, H, D, D)) return CDSSM_ERR_CUDA;
+    if (!make_tile_map(&tmK, k, k_rs, B, L, H, D, D) || !make_tile_map(&tmQ, mode == 0 ? k : q, mode == 0 ? k_rs : q_rs, B, L, H, D, D)) return CDSSM_ERR_CUDA;
     Args a;
     float2* ra;
     uint32_t *rv, *rg;

@@ -21,7 +21,10 @@ struct Args {
     uint4* rec;                    // kWa: {a_re, a_im | v pair | beta, sel_C} (B, 32-token blocks, H, 32)
     float2* rec_a;                 // else: transition (B,NC,H,NP,C)
     uint32_t *rec_v, *rec_g;       // vp-scaled v (B,NC,H,NP,C); beta and sel_C (B,NC,H,C), bf16 pairs
-    int* status;                   // cleared here for the passes that follow, or nullptr
+    const __nv_bfloat16 *v_first, *mix;   // or nullptr: v <- lerp(v_first, v, mix[head])
+    long long v_rs, vf_rs, g_rs;   // elements between token rows
+    int* clear;                    // words cleared here for the passes that follow
+    size_t clear_words;
     DynConsts dc;
     int B, L, H, N, C, NC, pos0, segs, fp32_decay, tiles;   // tiles: 32-token tiles per batch row, chunks padded to full length
 };
@@ -29,7 +32,7 @@ struct Args {
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // kNP: pair slots (>= N / 2); kHg: heads per block.
-template <int kNP, int kHg, bool kWa>
+template <int kNP, int kHg, bool kWa, bool kResidual>
 __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     using T = __nv_bfloat16;
     constexpr int kItems = kTokens * kHg / kThreads, kRow = kTokens + 1;
@@ -38,20 +41,22 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     float2* sa = reinterpret_cast<float2*>(smem);                      // else [pair][head][token]
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
-    if (a.status != nullptr && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) *a.status = 0;
+    for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x; i < a.clear_words;
+         i += (size_t)gridDim.x * gridDim.y * kThreads)
+        a.clear[i] = 0;
     const int H = a.H, N = a.N, NP = N >> 1;
     const int b = (int)(blockIdx.x / (unsigned)a.tiles), tile = (int)(blockIdx.x - (unsigned)b * a.tiles), l0 = tile * kTokens;
     const int head0 = blockIdx.y * kHg, heads = min(kHg, H - head0);
     const int head = threadIdx.x & (kHg - 1), hd = head0 + min(head, heads - 1);
     const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
     T x[kItems][5], ga[kItems][kNP], gw[kItems][kNP];
-    uint32_t vv[kItems][kNP];
+    uint32_t vv[kItems][kNP], vf[kResidual ? kItems : 1][kNP];
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
         const int l = min(l0 + (int)(threadIdx.x / kHg) + i * (kThreads / kHg), a.L - 1);
         const size_t row = (size_t)b * a.L + l;
-        const T* g = a.gate_raw + row * (size_t)((N + 5) * H) + hd;
-        const uint32_t* v = reinterpret_cast<const uint32_t*>(a.v) + (row * H + hd) * NP;
+        const T* g = a.gate_raw + row * a.g_rs + hd;
+        const uint32_t* v = reinterpret_cast<const uint32_t*>(a.v + row * a.v_rs + hd * N);
 #pragma unroll
         for (int s = 0; s < 5; s++) x[i][s] = g[(N + s) * H];
 #pragma unroll
@@ -61,7 +66,13 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
             gw[i][p] = g[(NP + pp) * H];
             vv[i][p] = v[pp];
         }
+        if (kResidual) {
+            const uint32_t* f = reinterpret_cast<const uint32_t*>(a.v_first + row * a.vf_rs + hd * N);
+#pragma unroll
+            for (int p = 0; p < kNP; p++) vf[i][p] = f[p < NP ? p : 0];
+        }
     }
+    const float mix = kResidual ? __bfloat162float(a.mix[hd]) : 0.f;
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
         const int t = (int)(threadIdx.x / kHg) + i * (kThreads / kHg), l = l0 + t;
@@ -79,7 +90,11 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
             dyn_pair<true>(f(ga[i][p]), f(gw[i][p]), freq, pos, ds, ar, ai, vp);
             if (!a.fp32_decay) { ar = bfr(ar); ai = bfr(ai); }
             vp = bfr(vp);
-            const float v0 = __uint_as_float(vv[i][p] << 16), v1 = __uint_as_float(vv[i][p] & 0xffff0000u);
+            float v0 = __uint_as_float(vv[i][p] << 16), v1 = __uint_as_float(vv[i][p] & 0xffff0000u);
+            if (kResidual) {
+                v0 = value_residual<T>(__uint_as_float(vf[i][p] << 16), v0, mix);
+                v1 = value_residual<T>(__uint_as_float(vf[i][p] & 0xffff0000u), v1, mix);
+            }
             const uint32_t vg = on ? pack2(v0 * vp, v1 * vp) : 0u;
             if (!on) { ar = 1.f; ai = 0.f; }
             if (kWa) {
@@ -109,20 +124,21 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     }
 }
 
-template <int kNP, int kHg, bool kWa> struct KernelTag {};
-template <int kNP, int kHg, bool kWa>
+template <int kNP, int kHg, bool kWa, bool kResidual> struct KernelTag {};
+template <int kNP, int kHg, bool kWa, bool kResidual>
 static int launch(const Args& a, cudaStream_t st) {
     const size_t smem = kWa ? (size_t)kHg * (kTokens + 1) * 16 : (size_t)kHg * (kTokens + 1) * (kNP * 12 + 4);
     if (smem > 48 * 1024)
-        if (int rc = allow_smem<KernelTag<kNP, kHg, kWa>>((const void*)records_kernel<kNP, kHg, kWa>, smem)) return rc;
-    records_kernel<kNP, kHg, kWa><<<dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg), kThreads, smem, st>>>(a);
+        if (int rc = allow_smem<KernelTag<kNP, kHg, kWa, kResidual>>((const void*)records_kernel<kNP, kHg, kWa, kResidual>, smem)) return rc;
+    records_kernel<kNP, kHg, kWa, kResidual><<<dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg), kThreads, smem, st>>>(a);
     return check_launch();
 }
 // 16 heads fill the sectors of the gate rows; 8 where that leaves fewer lanes empty (24 heads) or more blocks are wanted.
 template <int kNP, bool kWa>
 static int launch_group(const Args& a, cudaStream_t st) {
-    return (a.H + 15) / 16 * 16 > (a.H + 7) / 8 * 8 || (long long)a.B * a.tiles * a.H < 148 * 64 ? launch<kNP, 8, kWa>(a, st)
-                                                                                               : launch<kNP, 16, kWa>(a, st);
+    const bool eight = (a.H + 15) / 16 * 16 > (a.H + 7) / 8 * 8 || (long long)a.B * a.tiles * a.H < 148 * 64;
+    if (a.v_first) return eight ? launch<kNP, 8, kWa, true>(a, st) : launch<kNP, 16, kWa, true>(a, st);
+    return eight ? launch<kNP, 8, kWa, false>(a, st) : launch<kNP, 16, kWa, false>(a, st);
 }
 
 }  // namespace records
@@ -141,9 +157,10 @@ void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a
 }
 
 // Fills the records every pass over the same inputs reads.  wa: the layout of scan_wa.cu (N = 2), else of scan_chunk.cu.
-int scan_records(bool wa, const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                 int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
-                 cudaStream_t st) {
+int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, long long vf_rs, const void* mix,
+                 const void* gate_raw, long long g_rs, const float* log_dt_scale, const float* rope_freqs, void* rec,
+                 int* clear, size_t clear_words, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
+                 int fp32_decay, cudaStream_t st) {
     using namespace records;
     Args a;
     a.v = static_cast<const __nv_bfloat16*>(v);
@@ -151,7 +168,9 @@ int scan_records(bool wa, const void* v, const void* gate_raw, const float* log_
     a.log_dt_scale = log_dt_scale; a.rope_freqs = rope_freqs;
     a.rec = static_cast<uint4*>(rec);
     scan_record_arrays(rec, B, L, H, N, C, &a.rec_a, &a.rec_v, &a.rec_g);
-    a.status = status;
+    a.v_first = static_cast<const __nv_bfloat16*>(v_first); a.mix = static_cast<const __nv_bfloat16*>(mix);
+    a.v_rs = v_rs; a.vf_rs = vf_rs; a.g_rs = g_rs;
+    a.clear = clear; a.clear_words = clear_words;
     a.dc = dc;
     a.B = B; a.L = L; a.H = H; a.N = N; a.C = C; a.NC = (L + C - 1) / C; a.pos0 = pos0; a.segs = segs; a.fp32_decay = fp32_decay;
     a.tiles = a.NC * (C / kTokens);

@@ -47,6 +47,9 @@ struct ScanArgs {
     DynConsts dc;
     float shortcut_scale;
     int B, L, H, D, N, C, NC, pos0;
+    // elements between the (batch, token) rows of q, k, v, gate_raw and v_first (column slices of wider projections)
+    long long q_rs, k_rs, v_rs, g_rs, vf_rs;
+    const void *v_first, *mix;   // or NULL: v <- lerp(v_first, v, mix[head])
     long long units;   // B*NC*H*NP
 };
 
@@ -64,15 +67,17 @@ struct ChunkScalars {
 // block.py:194-195).
 template <typename T>
 struct TokenDynamics {
-    const T *gr, *vrow;
+    const T *gr, *vrow, *vfirst;
     DynShared ds;
-    float freq, pos;
+    float freq, pos, mix;
     int H, NH, fp32_decay;
     __device__ __forceinline__ TokenDynamics(const ScanArgs& a, int b, int l, int hd) {
         H = a.H; NH = a.N >> 1; fp32_decay = a.fp32_decay;
         const long long bl = (long long)b * a.L + l;
-        gr = static_cast<const T*>(a.gate_raw) + bl * (long long)((a.N + 5) * H) + hd;
-        vrow = static_cast<const T*>(a.v) + (bl * H + hd) * a.N;
+        gr = static_cast<const T*>(a.gate_raw) + bl * a.g_rs + hd;
+        vrow = static_cast<const T*>(a.v) + bl * a.v_rs + (long long)hd * a.N;
+        vfirst = a.v_first ? static_cast<const T*>(a.v_first) + bl * a.vf_rs + (long long)hd * a.N : nullptr;
+        mix = a.v_first ? IO<T>::ld(static_cast<const T*>(a.mix) + hd) : 0.f;
         const T* s5 = gr + a.N * H;
         freq = a.rope_freqs[hd];
         pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
@@ -89,7 +94,12 @@ struct TokenDynamics {
             ai = IO<T>::rnd(ai);
         }
         vp = IO<T>::rnd(vp);
-        return make_float4(ar, ai, IO<T>::rnd(IO<T>::ld(vrow + 2 * j) * vp), IO<T>::rnd(IO<T>::ld(vrow + 2 * j + 1) * vp));
+        float v0 = IO<T>::ld(vrow + 2 * j), v1 = IO<T>::ld(vrow + 2 * j + 1);
+        if (vfirst) {
+            v0 = value_residual<T>(IO<T>::ld(vfirst + 2 * j), v0, mix);
+            v1 = value_residual<T>(IO<T>::ld(vfirst + 2 * j + 1), v1, mix);
+        }
+        return make_float4(ar, ai, IO<T>::rnd(v0 * vp), IO<T>::rnd(v1 * vp));
     }
 };
 
@@ -166,9 +176,8 @@ scan_walk_kernel(const ScanArgs a) {
     __syncwarp();
 
     const int Lc = min(C, a.L - c * C);                  // valid tokens of this chunk
-    const T* kbase = static_cast<const T*>(a.k) + (((long long)b * a.L + (long long)c * C) * H + hd) * D;
-    const T* qbase = static_cast<const T*>(a.q) + (((long long)b * a.L + (long long)c * C) * H + hd) * D;
-    const long long rstride = (long long)H * D;
+    const T* kbase = static_cast<const T*>(a.k) + ((long long)b * a.L + (long long)c * C) * a.k_rs + (long long)hd * D;
+    const T* qbase = static_cast<const T*>(a.q) + ((long long)b * a.L + (long long)c * C) * a.q_rs + (long long)hd * D;
 
     // State columns are held as pairs: every element-wise operation of the step is a packed
     // fp32x2 instruction (Blackwell FFMA2 / FMUL2), which halves the issue slots of a kernel that
@@ -202,8 +211,8 @@ scan_walk_kernel(const ScanArgs a) {
         kraw.get(reinterpret_cast<float*>(kk));
         if (kOutput) qraw.get(reinterpret_cast<float*>(qq));
         if (t + 1 < Lc) {
-            kraw.load(kbase + (long long)(t + 1) * rstride, g, D, vec);
-            if (kOutput) qraw.load(qbase + (long long)(t + 1) * rstride, g, D, vec);
+            kraw.load(kbase + (long long)(t + 1) * a.k_rs, g, D, vec);
+            if (kOutput) qraw.load(qbase + (long long)(t + 1) * a.q_rs, g, D, vec);
         } else {
             kraw.zero();
             if (kOutput) qraw.zero();
@@ -359,7 +368,6 @@ scan_recurrent_kernel(const ScanArgs a) {
     const int hd = (int)((u / NH) % H);
     const int b = (int)(u / ((long long)NH * H));
     const bool vec = (D == kCols * kLanes);
-    const long long rstride = (long long)H * D;
     float2 zr[kP], zi[kP];
     {
         const float* h = a.h0 ? a.h0 + (((long long)b * H + hd) * a.N + 2 * j) * D : nullptr;
@@ -376,8 +384,8 @@ scan_recurrent_kernel(const ScanArgs a) {
         stage_dynamics<T, kLanes>(a, sm, ul, g, b, c, hd, j);
         __syncwarp();
         const int Lc = min(CS, a.L - c * CS);
-        const T* kbase = static_cast<const T*>(a.k) + (((long long)b * a.L + (long long)c * CS) * H + hd) * D;
-        const T* qbase = static_cast<const T*>(a.q) + (((long long)b * a.L + (long long)c * CS) * H + hd) * D;
+        const T* kbase = static_cast<const T*>(a.k) + ((long long)b * a.L + (long long)c * CS) * a.k_rs + (long long)hd * D;
+        const T* qbase = static_cast<const T*>(a.q) + ((long long)b * a.L + (long long)c * CS) * a.q_rs + (long long)hd * D;
         RowSlice<T, kCols> kraw, qraw;
         kraw.load(kbase, g, D, vec);
         qraw.load(qbase, g, D, vec);
@@ -386,8 +394,8 @@ scan_recurrent_kernel(const ScanArgs a) {
             kraw.get(reinterpret_cast<float*>(kk));
             qraw.get(reinterpret_cast<float*>(qq));
             if (t + 1 < Lc) {
-                kraw.load(kbase + (long long)(t + 1) * rstride, g, D, vec);
-                qraw.load(qbase + (long long)(t + 1) * rstride, g, D, vec);
+                kraw.load(kbase + (long long)(t + 1) * a.k_rs, g, D, vec);
+                qraw.load(qbase + (long long)(t + 1) * a.q_rs, g, D, vec);
             }
             const float a_re = sm.a_re[so + t], a_im = sm.a_im[so + t], be = sm.beta[so + t];
             const float vr = sm.v_re[so + t], vi = sm.v_im[so + t];
@@ -506,7 +514,8 @@ scan_carry_kernel(const ScanArgs a) {
                     a.ws_state[u * 2 * D + d] = IO<T>::rnd(sr);       // chunk_states store
                     a.ws_state[u * 2 * D + D + d] = IO<T>::rnd(si);
                 }
-                const float nr = carry_re(gr[i], gi[i], sr, si, lr[i]), ni = carry_im(gr[i], gi[i], sr, si, li[i]);
+                const float nr = gr[i] * sr - gi[i] * si + lr[i];
+                const float ni = gr[i] * si + gi[i] * sr + li[i];
                 sr = nr;
                 si = ni;
                 const float pr = gr[i] * dr - gi[i] * di, pi = gr[i] * di + gi[i] * dr;
@@ -780,17 +789,18 @@ namespace cdssm {
 unsigned long long wait_limit_ns();   // c_abi.cu
 // scan_records.cu
 size_t scan_record_bytes(int B, int L, int H, int N, int C);
-int scan_records(bool wa, const void* v, const void* gate_raw, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                 int* status, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs, int fp32_decay,
-                 cudaStream_t st);
+int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, long long vf_rs, const void* mix,
+                 const void* gate_raw, long long g_rs, const float* log_dt_scale, const float* rope_freqs, void* rec,
+                 int* clear, size_t clear_words, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
+                 int fp32_decay, cudaStream_t st);
 // scan_wa.cu
 bool scan_wa_supported(int D, int N, int C, int H, int dtype);
-int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, float* ws_gamma, float* ws_state, void* y,
+int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  cudaStream_t st);
 // scan_chunk.cu
 bool scan_chunk_supported(int D, int N, int C, int dtype);
-int scan_chunk_pass(int mode, const void* q, const void* k, void* rec, const float* h0, void* y, float* final_state,
+int scan_chunk_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
                     float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
                     int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
 }
@@ -835,20 +845,31 @@ static bool one_kernel_pays(int B, int H, int NC, int D, int N) {
     return (float)B * (float)H * per_chunk >= 1800.f || NC <= 4 + N / 2;
 }
 
+struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual
+    long long q = 0, k = 0, v = 0, gate = 0, v_first = 0;
+    const void *first = nullptr, *mix = nullptr;
+};
+
 static int scan_fused_impl(const void* q, const void* k, const void* v, const void* gate_raw,
                            const float* log_dt_scale, const float* rope_freqs, const float* h0, void* y,
                            float* final_state, float* tail_state, float* total_decay, bool summary_only,
                            void* workspace, size_t workspace_bytes, float gating_c, float omega_thresh,
                            float adt_delta, float adt_smoothness, float adt_eps, float shortcut_scale,
                            int B, int L, int H, int D, int N, int C, int pos0, int segs, int dtype,
-                           int flags, void* stream, bool small_workspace = false) {
+                           int flags, void* stream, bool small_workspace = false, const ScanRows& rows = ScanRows()) {
     if (summary_only) { q = k; y = nullptr; tail_state = nullptr; }
     if (!q || !k || !v || !gate_raw || !log_dt_scale || !rope_freqs || (!y && !summary_only))
         return CDSSM_ERR_BAD_ARG;
     if (segs < 1 || (B > 0 && B % segs)) return CDSSM_ERR_BAD_ARG;
     if (B < 0 || L < 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return CDSSM_ERR_BAD_ARG;
     if (dtype != CDSSM_BF16 && dtype != CDSSM_F32) return CDSSM_ERR_BAD_ARG;
+    const long long es = dtype == CDSSM_F32 ? 4 : 2, hd = (long long)H * D, hn = (long long)H * N, hg = (long long)(N + 5) * H;
+    const long long q_rs = rows.q ? rows.q : hd, k_rs = rows.k ? rows.k : hd, v_rs = rows.v ? rows.v : hn,
+                    g_rs = rows.gate ? rows.gate : hg, vf_rs = rows.v_first ? rows.v_first : hn;
+    if (q_rs < hd || k_rs < hd || v_rs < hn || g_rs < hg || vf_rs < hn || (rows.first != nullptr) != (rows.mix != nullptr))
+        return CDSSM_ERR_BAD_ARG;
     if (((uintptr_t)q | (uintptr_t)k) & 15) return CDSSM_ERR_BAD_ARG;   // 16-byte row loads
+    if ((D == 64 || D == 128) && (((q_rs | k_rs) * es) & 15)) return CDSSM_ERR_BAD_ARG;
     if (N > kMaxStateDim || D > kMaxHeadDim || C > kMaxChunk) return CDSSM_ERR_UNSUPPORTED;
     if (B == 0 || L == 0) return CDSSM_OK;
     // small_workspace: as many of the records as fit (the walks can do without)
@@ -871,6 +892,8 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     a.dc = DynConsts{gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps};
     a.shortcut_scale = shortcut_scale;
     a.B = B; a.L = L; a.H = H; a.D = D; a.N = N; a.C = C; a.pos0 = pos0;
+    a.q_rs = q_rs; a.k_rs = k_rs; a.v_rs = v_rs; a.g_rs = g_rs; a.vf_rs = vf_rs;
+    a.v_first = rows.first; a.mix = rows.mix;
     a.NC = (L + C - 1) / C;
     a.units = (long long)B * a.NC * H * (N / 2);
     a.ws_gamma = static_cast<float*>(workspace);
@@ -883,7 +906,8 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     // D 128; nine chunks of 24 heads of 64: 22 / 20; five and seven chunks of 4 heads of 128: 28 / 31, 29 / 32).  They read v
     // and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the contract allows, stay on the CUDA-core
     // kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the tests to check each tensor-core pass alone.)
-    const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y) & 3) == 0 && workspace_bytes - base >= scan_record_bytes(B, L, H, N, C) &&
+    const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y | (uintptr_t)rows.first | (uintptr_t)(2 * v_rs) |
+                              (uintptr_t)(rows.first ? 2 * vf_rs : 0)) & 3) == 0 && ((q_rs | k_rs) & 7) == 0 && workspace_bytes - base >= scan_record_bytes(B, L, H, N, C) &&
                            !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
     const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, H, dtype) &&
                        ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > (D == 64 ? 2 : 7) || (long long)B * a.NC * H > (D == 64 ? 512 : 256));
@@ -892,13 +916,13 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
     const bool one_kernel = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && ((uintptr_t)h0 & 15) == 0 &&
                             one_kernel_pays(B, H, a.NC, D, N);
-    // Status word, and for the one-kernel scan its ticket counter and its "carry is there" words in the gamma slots; where a
-    // dynamics kernel runs first, that one clears the status.
+    // Status word, and for the one-kernel scan its ticket counter and its "carry is there" words in the gamma slots: cleared
+    // by the records kernel where that runs first.
     const bool tensor = wa_ok || chunk_ok;
-    if (one_kernel || !tensor || !a.run_local) {
-        const size_t zero = one_kernel ? 256 + (size_t)a.units * 2 * sizeof(float) : sizeof(int);
-        if (int rc = check_cuda(cudaMemsetAsync(status, 0, zero, st))) return rc;
-    }
+    const bool fill_records = tensor && (a.run_local || (flags & CDSSM_SCAN_TENSOR_CORE_WA));
+    const size_t clear_words = one_kernel ? 64 + (size_t)a.units * 2 : 1;
+    if (!fill_records)
+        if (int rc = check_cuda(cudaMemsetAsync(status, 0, clear_words * sizeof(int), st))) return rc;
     void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
     a.rec_av = nullptr;
     a.rec_bs = nullptr;
@@ -925,17 +949,16 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     const unsigned long long limit = wait_limit_ns();
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
-            return scan_wa_pass(mode == 1, q, k, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
+            return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
                                 limit, withhold, st);
-        return scan_chunk_pass(mode, q, k, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
+        return scan_chunk_pass(mode, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
                                shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };
     // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)
-    if (a.run_local || (flags & CDSSM_SCAN_TENSOR_CORE_WA)) {
-        const int rc = scan_records(wa_ok, v, gate_raw, log_dt_scale, rope_freqs, rec, one_kernel ? nullptr : status, a.dc, B, L, H,
-                                    N, C, pos0, segs, a.fp32_decay, st);
-        if (rc) return rc;
-    }
+    if (fill_records)
+        if (int rc = scan_records(wa_ok, v, v_rs, rows.first, vf_rs, rows.mix, gate_raw, g_rs, log_dt_scale, rope_freqs, rec, status,
+                                  clear_words, a.dc, B, L, H, N, C, pos0, segs, a.fp32_decay, st))
+            return rc;
     if (one_kernel) return pass(2);
     if (a.run_local && tc_local) {
         if (int rc = pass(0)) return rc;
@@ -1004,6 +1027,23 @@ extern "C" int cdssm_b200_scan_fused_fwd(const void* q, const void* k, const voi
                            nullptr, false, workspace, workspace_bytes, gating_c, omega_thresh, adt_delta,
                            adt_smoothness, adt_eps, shortcut_scale, B, L, H, D, N, C, pos0, 1, dtype, flags,
                            stream);
+}
+
+extern "C" int cdssm_b200_scan_fused_strided_fwd(const void* q, int64_t q_row_stride, const void* k, int64_t k_row_stride,
+                                                 const void* v, int64_t v_row_stride, const void* v_first,
+                                                 int64_t v_first_row_stride, const void* mix, const void* gate_raw,
+                                                 int64_t gate_row_stride, const float* log_dt_scale, const float* rope_freqs,
+                                                 const float* h0, void* y, float* final_state, float* tail_state,
+                                                 void* workspace, size_t workspace_bytes, float gating_c, float omega_thresh,
+                                                 float adt_delta, float adt_smoothness, float adt_eps, float shortcut_scale,
+                                                 int B, int L, int H, int D, int N, int C, int pos0, int dtype, int flags,
+                                                 void* stream) {
+    ScanRows r;
+    r.q = q_row_stride; r.k = k_row_stride; r.v = v_row_stride; r.gate = gate_row_stride;
+    r.first = v_first; r.v_first = v_first_row_stride; r.mix = mix;
+    return scan_fused_impl(q, k, v, gate_raw, log_dt_scale, rope_freqs, h0, y, final_state, tail_state, nullptr, false,
+                           workspace, workspace_bytes, gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps,
+                           shortcut_scale, B, L, H, D, N, C, pos0, 1, dtype, flags, stream, false, r);
 }
 
 extern "C" int cdssm_b200_scan_fused_segmented_fwd(const void* q, const void* k, const void* v,

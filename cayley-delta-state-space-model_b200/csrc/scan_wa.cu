@@ -863,12 +863,12 @@ bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
 // One pass of the warp-autonomous tensor-core scan over every chunk.  output = false: local pass (fills
 // ws_state / ws_gamma for the carry pass); output = true: reads the carries from ws_state, writes y.
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
-int scan_wa_pass(bool output, const void* q, const void* k, const void* rec, float* ws_gamma, float* ws_state, void* y,
+int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  cudaStream_t st) {
     using namespace wa;
     CUtensorMap tmK, tmQ;
-    if (!make_tile_map(&tmK, k, B, L, H, D, kSub) || !make_tile_map(&tmQ, output ? q : k, B, L, H, D, kSub)) return CDSSM_ERR_CUDA;
+    if (!make_tile_map(&tmK, k, k_rs, B, L, H, D, kSub) || !make_tile_map(&tmQ, output ? q : k, output ? q_rs : k_rs, B, L, H, D, kSub)) return CDSSM_ERR_CUDA;
     int dev = 0, sms = 0;
     if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;
     if (int rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return rc;

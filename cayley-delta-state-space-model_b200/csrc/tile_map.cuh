@@ -21,12 +21,13 @@ inline EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// (B, L, H, D) bf16 tensor viewed as 4-D (D, H, L, B); box = 64 columns x 1 head x `rows` positions.
-inline bool make_tile_map(CUtensorMap* m, const void* base, int B, int L, int H, int D, int rows) {
+// (B, L, H, D) bf16 tensor, `stride` elements between tokens, viewed as 4-D (D, H, L, B); box = 64 columns x 1 head x `rows`
+// positions.
+inline bool make_tile_map(CUtensorMap* m, const void* base, long long stride, int B, int L, int H, int D, int rows) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)L, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)H * D * 2, (cuuint64_t)L * H * D * 2};
+    const cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)stride * 2, (cuuint64_t)L * stride * 2};
     const cuuint32_t box[4] = {64, 1, (cuuint32_t)rows, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,

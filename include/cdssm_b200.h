@@ -229,6 +229,20 @@ CDSSM_API int cdssm_b200_scan_fused_fwd(const void* q, const void* k, const void
                               float shortcut_scale, int B, int L, int H, int D, int N, int C,
                               int pos0, int dtype, int flags, void* stream);
 
+/* cdssm_b200_scan_fused_fwd for q, k, v and gate_raw that are column slices of wider per-token projections (*_row_stride
+ * elements between the rows of consecutive tokens, 0: dense; q and k rows 16-byte aligned where D is 64 or 128), and, if
+ * v_first and mix are not NULL, with the value residual of cdssm/models/block.py:167-171 applied on the fly: v <-
+ * lerp(v_first, v, mix[head]) rounded to the storage type (mix (H) = sigmoid(v_residual_gate) in the storage type). */
+CDSSM_API int cdssm_b200_scan_fused_strided_fwd(const void* q, int64_t q_row_stride, const void* k, int64_t k_row_stride,
+                                                const void* v, int64_t v_row_stride, const void* v_first,
+                                                int64_t v_first_row_stride, const void* mix, const void* gate_raw,
+                                                int64_t gate_row_stride, const float* log_dt_scale, const float* rope_freqs,
+                                                const float* h0, void* y, float* final_state, float* tail_state,
+                                                void* workspace, size_t workspace_bytes, float gating_c, float omega_thresh,
+                                                float adt_delta, float adt_smoothness, float adt_eps, float shortcut_scale,
+                                                int B, int L, int H, int D, int N, int C, int pos0, int dtype, int flags,
+                                                void* stream);
+
 /* Sequence segments.  In the reference's semantics the carry between chunks is the diagonal-linear
  * recurrence s <- gamma_c (*) s + l_c (cdssm/csrc/kernels/inter_chunk_scan.cu:73-83) and neither
  * gamma_c nor l_c depends on s, so a chunk-aligned segment is summarised by (total_decay, carry_out):
@@ -279,8 +293,8 @@ CDSSM_API int cdssm_b200_compose_carries(const float* decay, const float* carry_
  * device-wide synchronisation of cudaMalloc).  Same arguments and results as
  * cdssm_b200_scan_fused_fwd without the workspace: the scratch is a 16 MiB array built into the
  * library (cdssm_b200_scan_fused_noalloc_max_bytes()), resident on every GPU that loads it.
- *  - Sizes whose cdssm_b200_scan_fused_workspace_bytes exceeds that limit are refused with
- *    CDSSM_ERR_WORKSPACE; nothing is launched.
+ *  - Sizes whose chunk states (and, for the tensor-core kernel of N = 2, per-token records) exceed that limit are
+ *    refused with CDSSM_ERR_WORKSPACE; nothing is launched.  Other records are used as far as they fit.
  *  - The first call on each device looks up the array's device address (with that device
  *    current); make that first call outside any stream capture.
  *  - No cudaMalloc, cudaFree or other allocating routine is called.
