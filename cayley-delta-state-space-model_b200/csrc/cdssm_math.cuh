@@ -154,4 +154,21 @@ template <> struct Vec8<float> {
     }
 };
 
+template <typename T> struct Raw8;   // the same, kept in storage form until used
+template <> struct Raw8<__nv_bfloat16> {
+    uint4 v;
+    __device__ __forceinline__ void ld(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ void get(float* f) const { unpack8(v, f); }
+};
+template <> struct Raw8<float> {
+    float4 a, b;
+    __device__ __forceinline__ void ld(const float* p) {
+        a = *reinterpret_cast<const float4*>(p);
+        b = *reinterpret_cast<const float4*>(p + 4);
+    }
+    __device__ __forceinline__ void get(float* f) const {
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    }
+};
+
 }  // namespace cdssm

@@ -186,27 +186,26 @@ groupnorm_gate_fwd_kernel(const T* __restrict__ y, const float* __restrict__ sta
     Vec8<T>::st(out + row * di + c, f);
 }
 
-// The same with statistics given, kRows tokens per block: the per-channel parameters are loaded once and the
-// loads of all rows are in flight together.
+// The same with statistics given, kRows tokens per block: the per-channel parameters are loaded once, and the rows' loads are
+// in flight together in storage form (unpacked they held 96 registers, and two blocks per SM left the memory waiting).
+// Measured on B200: 16 384 tokens of 1536 channels MEASURED_GN.
 template <typename T, int kRows>
 __global__ void __launch_bounds__(1024)
 groupnorm_gate_rows_kernel(const T* __restrict__ y, const float* __restrict__ stats, const T* __restrict__ gn_w,
                            const T* __restrict__ gn_b, const T* __restrict__ z, long long z_row_stride,
                            const T* __restrict__ skip, const T* __restrict__ x_conv, T* __restrict__ out,
-                           long long rows, int L, int di, int groups) {
-    const long long r0 = (long long)blockIdx.x * kRows;
-    const int c = threadIdx.x * 8;
+                           int rows, int L, int di, int groups) {
+    const int r0 = blockIdx.x * kRows, c = threadIdx.x * 8;
     const int grp = threadIdx.x / ((di / groups) / 8);
-    float f[kRows][8], zz[kRows][8], xc[kRows][8], mean[kRows], rstd[kRows];
+    Raw8<T> f[kRows], zz[kRows], xc[kRows];
+    float2 st[kRows];
 #pragma unroll
     for (int r = 0; r < kRows; r++) {
-        const long long row = r0 + r < rows ? r0 + r : rows - 1;
-        Vec8<T>::ld(y + row * di + c, f[r]);
-        Vec8<T>::ld(z + row * z_row_stride + c, zz[r]);
-        Vec8<T>::ld(x_conv + row * di + c, xc[r]);
-        const long long b = row / L;
-        mean[r] = stats[2 * (b * groups + grp)];
-        rstd[r] = stats[2 * (b * groups + grp) + 1];
+        const int row = min(r0 + r, rows - 1);
+        f[r].ld(y + (long long)row * di + c);
+        zz[r].ld(z + row * z_row_stride + c);
+        xc[r].ld(x_conv + (long long)row * di + c);
+        st[r] = *reinterpret_cast<const float2*>(stats + 2 * ((long long)(row / L) * groups + grp));
     }
     float gw[8], gb[8], sk[8];
     Vec8<T>::ld(gn_w + c, gw);
@@ -215,13 +214,17 @@ groupnorm_gate_rows_kernel(const T* __restrict__ y, const float* __restrict__ st
 #pragma unroll
     for (int r = 0; r < kRows; r++) {
         if (r0 + r >= rows) break;
+        float a[8], b[8], d[8];
+        f[r].get(a);
+        zz[r].get(b);
+        xc[r].get(d);
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            const float n = IO<T>::rnd((f[r][e] - mean[r]) * rstd[r] * gw[e] + gb[e]);
-            const float g = IO<T>::rnd(siluf_<IO<T>::kBf16>(zz[r][e]));
-            f[r][e] = IO<T>::rnd(n * g) + IO<T>::rnd(sk[e] * xc[r][e]);
+            const float n = IO<T>::rnd((a[e] - st[r].x) * st[r].y * gw[e] + gb[e]);
+            const float s = IO<T>::rnd(siluf_<IO<T>::kBf16>(b[e]));
+            a[e] = IO<T>::rnd(n * s) + IO<T>::rnd(sk[e] * d[e]);
         }
-        Vec8<T>::st(out + (r0 + r) * di + c, f[r]);
+        Vec8<T>::st(out + (long long)(r0 + r) * di + c, a);
     }
 }
 
@@ -352,7 +355,7 @@ extern "C" int cdssm_b200_groupnorm_gate_fwd(const void* y, const float* stats, 
         DISPATCH_DTYPE(dtype, (groupnorm_gate_rows_kernel<T, kRows><<<(unsigned)((rows + kRows - 1) / kRows), di / 8, 0,
                                                                       (cudaStream_t)stream>>>(
                                   (const T*)y, stats, (const T*)gn_weight, (const T*)gn_bias, (const T*)z, z_row_stride,
-                                  (const T*)skip, (const T*)x_conv, (T*)out, rows, L, di, groups)));
+                                  (const T*)skip, (const T*)x_conv, (T*)out, (int)rows, L, di, groups)));
         return check_launch();
     }
     DISPATCH_DTYPE(dtype, (groupnorm_gate_fwd_kernel<T><<<(unsigned)rows, di / 8, 0, (cudaStream_t)stream>>>(

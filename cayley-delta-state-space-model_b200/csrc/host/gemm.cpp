@@ -100,6 +100,18 @@ bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_da
 
 Tensor gemm_workspace(const Tensor& on) { return at::empty({(int64_t)kGemmWorkspace}, on.options().dtype(at::kByte)); }
 
+// bf16: out (rows, M; ldo apart) = x (rows, K; ldx apart) w (M, K)^T [+ bias] [+ out]
+void gemm_raw(int device, void* out, int64_t ldo, const void* x, int64_t ldx, const void* w, const void* bias, int64_t rows, int64_t M,
+              int64_t K, bool accumulate, void* workspace, void* stream) {
+    const Key key{device, M, rows, K, ldx, ldo, bias != nullptr, accumulate};
+    Plan& p = plan_for(key);
+    if (bias) lt_check(cublasLtMatmulDescSetAttribute(p.op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)), "bias");
+    const float one = 1.f, beta = accumulate ? 1.f : 0.f;
+    lt_check(cublasLtMatmul(handle(device), p.op, &one, w, p.a, x, p.b, &beta, out, p.d, out, p.d, &p.algo, workspace,
+                            kGemmWorkspace, static_cast<cudaStream_t>(stream)),
+             "cublasLtMatmul");
+}
+
 // out (rows, M; rows out.stride(0) apart) = x (rows, K; rows x.stride(0) apart) w^T [+ bias] [+ out]; w (M, K) dense.
 void gemm(const Tensor& out, const Tensor& x, const Tensor& w, const Tensor& bias, bool accumulate, const Tensor& workspace) {
     const int64_t rows = x.size(0), K = x.size(1), M = w.size(0);
@@ -112,17 +124,8 @@ void gemm(const Tensor& out, const Tensor& x, const Tensor& w, const Tensor& bia
         else out.copy_(at::linear(x, w, bias));
         return;
     }
-    const Key key{(int)x.device().index(), M, rows, K, x.stride(0), out.stride(0), bias.defined(), accumulate};
-    Plan& p = plan_for(key);
-    if (bias.defined()) {
-        const void* b = bias.const_data_ptr();
-        lt_check(cublasLtMatmulDescSetAttribute(p.op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &b, sizeof(b)), "bias");
-    }
-    const float one = 1.f, beta = accumulate ? 1.f : 0.f;
-    lt_check(cublasLtMatmul(handle(key.device), p.op, &one, w.const_data_ptr(), p.a, x.const_data_ptr(), p.b, &beta, out.data_ptr(),
-                            p.d, out.data_ptr(), p.d, &p.algo, workspace.data_ptr(), kGemmWorkspace,
-                            static_cast<cudaStream_t>(stream_of(x))),
-             "cublasLtMatmul");
+    gemm_raw((int)x.device().index(), out.data_ptr(), out.stride(0), x.const_data_ptr(), x.stride(0), w.const_data_ptr(),
+             bias.defined() ? bias.const_data_ptr() : nullptr, rows, M, K, accumulate, workspace.data_ptr(), stream_of(x));
 }
 
 // x (.., K) w^T [+ bias] as a new tensor (.., M)

@@ -91,6 +91,8 @@ Tensor conv1d_silu_step(const Tensor& x, const Tensor& hist, const Tensor& w, co
 // ---- library products (gemm.cpp)
 constexpr size_t kGemmWorkspace = 32u << 20;   // what the library is given by default on this architecture
 Tensor gemm_workspace(const Tensor& on);
+void gemm_raw(int device, void* out, int64_t ldo, const void* x, int64_t ldx, const void* w, const void* bias, int64_t rows, int64_t M,
+              int64_t K, bool accumulate, void* workspace, void* stream);
 void gemm(const Tensor& out, const Tensor& x, const Tensor& w, const Tensor& bias, bool accumulate, const Tensor& workspace);
 Tensor linear(const Tensor& x, const Tensor& w, const Tensor& bias, const Tensor& workspace);
 

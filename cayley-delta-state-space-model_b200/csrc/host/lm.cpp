@@ -34,7 +34,7 @@ struct Plan {
     Dyn dyn;
     Tensor embedding, final_norm_w;
     std::vector<Block> blocks;
-    bool small_batch_ok = false;   // bf16, dense and 16-byte aligned: what the fused decode kernels read
+    bool dense_bf16 = false;   // every weight bf16, dense and 16-byte aligned: what the kernels read through plain pointers
 };
 
 constexpr double kFinalEps = 1.0 / 16384;   // 2^-14
@@ -110,6 +110,124 @@ void block_sequence(Plan& p, Block& b, const Tensor& x, Tensor& v_first, Cache* 
     gemm(x.view({B * L, p.d_model}), o.view({B * L, di}), b.w_out, Tensor(), true, ws);   // the residual add rides in the epilogue
 }
 
+// The same for bf16 models: every activation of a pass lives in one arena, the kernels are called with pointers and row
+// strides, and a layer's products are two wide ones (z | conv input | K | V and Q | gates) whose column slices the conv, the
+// scan and the gate read in place; the scan applies the value residual.  Tensor by tensor, a layer took 97 us of host time
+// (15 launches, as many allocations and views, nine products) whatever its size.
+struct Arena {
+    char* base;
+    size_t at = 0;
+    void* take(size_t bytes) {
+        void* p = base ? base + at : nullptr;
+        at += (bytes + 255) & ~(size_t)255;
+        return p;
+    }
+};
+struct SequenceBuffers {
+    void *xn, *proj0, *proj, *x_conv, *qg, *y, *y2, *gated, *gemm_ws;
+    float* stats;
+    size_t bytes;
+};
+SequenceBuffers sequence_buffers(const Plan& p, int64_t B, int64_t L, char* base) {
+    Arena a{base};
+    const size_t T = (size_t)(B * L), es = 2, di = p.d_inner, HN = p.heads * p.N, G = (p.N + 5) * p.heads;
+    const size_t pw = (3 * di + HN + 7) & ~(size_t)7, qw = (di + G + 7) & ~(size_t)7;
+    SequenceBuffers s;
+    s.xn = a.take(T * p.d_model * es);
+    s.proj0 = a.take(T * pw * es + 1024);   // layer 0's, kept: its V is every later layer's v_first
+    s.proj = a.take(T * pw * es + 1024);
+    s.x_conv = a.take(T * di * es);
+    s.qg = a.take(T * qw * es + 1024);
+    s.y = a.take(T * HN * es);
+    s.y2 = a.take(T * di * es);
+    s.gated = a.take(T * di * es);
+    s.stats = static_cast<float*>(a.take(sizeof(float) * cdssm_b200_groupnorm_stats_floats((int)B, (int)L, (int)p.groups)));
+    s.gemm_ws = a.take(kGemmWorkspace);
+    s.bytes = a.at;
+    return s;
+}
+
+void run_sequence(Plan& p, const Tensor& x, std::vector<Cache>* caches, bool per_token, int64_t flags, const SequenceBuffers& s) {
+    const int B = (int)x.size(0), L = (int)x.size(1), d = (int)p.d_model, di = (int)p.d_inner, H = (int)p.heads, N = (int)p.N;
+    const int64_t T = (int64_t)B * L;
+    const int HN = H * N, G = (N + 5) * H, dev = (int)x.device().index();
+    const bool long_prompt = caches && L > kTensorPrompt;
+    void* st = stream_of(x);
+    const Workspace ws = workspace(x, cdssm_b200_scan_fused_workspace_bytes(B, L, H, kHeadDim, N, (int)p.chunk));
+    auto product = [&](void* out, int64_t ldo, const void* in, int64_t K, const Tensor& w, const void* bias, bool accumulate) {
+        gemm_raw(dev, out, ldo, in, K, cptr(w), bias, T, w.size(0), K, accumulate, s.gemm_ws, st);
+    };
+    struct Slice { char* p; int64_t stride; };
+    Slice v0{};
+    for (size_t i = 0; i < p.blocks.size(); i++) {
+        Block& b = p.blocks[i];
+        char* proj = static_cast<char*>(i == 0 ? s.proj0 : s.proj);
+        char* qg = static_cast<char*>(s.qg);
+        check(cdssm_b200_rmsnorm_fwd(mptr(x), cptr(b.norm_w), s.xn, T, d, (float)p.eps_norm, CDSSM_BF16, st), "rmsnorm_fwd");
+        Slice z, xg, k, v, q, g;
+        if (!long_prompt) {
+            const int64_t pw = (3 * di + HN + 7) & ~7, qw = (di + G + 7) & ~7;
+            z = {proj, pw}; xg = {proj + 2 * di, pw}; k = {proj + 4 * di, pw}; v = {proj + 6 * di, pw};
+            q = {qg, qw}; g = {qg + 2 * di, qw};
+            product(proj, pw, s.xn, d, b.w_in, cptr(b.b_in), false);
+        } else {   // (one product per consumer, as caches of long prompts have always been filled: see kTensorPrompt)
+            auto dense = [&](int64_t cols_before, int64_t cols) { return Slice{proj + 2 * T * cols_before, cols}; };
+            z = dense(0, di); xg = dense(di, di); k = dense(2 * di, di); v = dense(3 * di, HN);
+            q = {qg, di}; g = {qg + 2 * T * di, G};
+            product(z.p, di, s.xn, d, b.w_z, cptr(b.b_z), false);
+            product(xg.p, di, s.xn, d, b.w_x, cptr(b.b_x), false);
+            product(k.p, di, s.xn, d, b.w_k, cptr(b.b_k), false);
+            product(v.p, HN, s.xn, d, b.w_v, cptr(b.b_v), false);
+        }
+        if (i == 0) v0 = v;
+        Cache* cache = caches ? &(*caches)[i] : nullptr;
+        if (cache) {
+            cache->conv = at::empty({B, 3, di}, x.options());
+            cache->state = empty_f32({B, H, N, kHeadDim}, x);
+        }
+        check(cdssm_b200_conv1d_silu_strided_fwd(xg.p, xg.stride, cptr(b.conv_w), cptr(b.conv_b), s.x_conv,
+                                                 cache ? mptr(cache->conv) : nullptr, B, L, di, CDSSM_BF16, st),
+              "conv1d_silu_fwd");
+        if (!long_prompt) {
+            product(qg, q.stride, s.x_conv, di, b.w_qg, cptr(b.b_qg), false);
+        } else {
+            product(g.p, G, s.x_conv, di, b.w_gate, cptr(b.b_gate), false);
+            product(q.p, di, s.x_conv, di, b.w_q, nullptr, false);
+        }
+        const void* mix = i == 0 ? nullptr : cptr(b.residual_mix(at::kBFloat16));
+        check(cdssm_b200_scan_fused_strided_fwd(q.p, q.stride, k.p, k.stride, v.p, v.stride, i == 0 ? nullptr : v0.p, v0.stride, mix,
+                                                g.p, g.stride, fptr(b.lds), fptr(b.rope), nullptr, s.y, nullptr,
+                                                cache ? fmut(cache->state) : nullptr, ws.ptr, ws.bytes, p.dyn.c[0], p.dyn.c[1],
+                                                p.dyn.c[2], p.dyn.c[3], p.dyn.c[4], (float)b.shortcut, B, L, H, kHeadDim, N,
+                                                (int)p.chunk, 0, CDSSM_BF16,
+                                                (int)(caches ? (long_prompt ? kScanForceSimt : 0) : flags), st),
+              "scan_fused_fwd");
+        product(s.y2, di, s.y, HN, b.w_readout, nullptr, false);
+        const bool token_stats = per_token || caches;   // see block_sequence()
+        if (!token_stats)
+            check(cdssm_b200_groupnorm_stats(s.y2, s.stats, B, L, di, (int)p.groups, (float)kGroupEps, CDSSM_BF16, st), "groupnorm_stats");
+        check(cdssm_b200_groupnorm_gate_fwd(s.y2, token_stats ? nullptr : s.stats, cptr(b.gn_w), cptr(b.gn_b), z.p, z.stride, cptr(b.D),
+                                            s.x_conv, s.gated, B, L, di, (int)p.groups, (float)kGroupEps, CDSSM_BF16, st),
+              "groupnorm_gate_fwd");
+        product(mptr(x), d, s.gated, di, b.w_out, nullptr, true);   // the residual add rides in the epilogue
+    }
+}
+
+// All layers over a sequence; x (B,L,d) is this call's own tensor and takes the residual sums in place.
+void run_blocks(Plan& p, const Tensor& x, std::vector<Cache>* caches, bool per_token, int64_t flags, const Tensor& ws) {
+    if (p.dense_bf16 && x.numel() > 0 && p.d_model % 8 == 0 && (p.heads * p.N) % 8 == 0 && (p.d_inner / p.groups) % 8 == 0 &&
+        p.d_inner <= 8192) {
+        const size_t bytes = sequence_buffers(p, x.size(0), x.size(1), nullptr).bytes;
+        const Tensor arena = at::empty({(int64_t)bytes + 256}, x.options().dtype(at::kByte));
+        char* base = static_cast<char*>(arena.data_ptr());
+        run_sequence(p, x, caches, per_token, flags, sequence_buffers(p, x.size(0), x.size(1), base + (-(uintptr_t)base & 255)));
+        return;
+    }
+    Tensor v_first;
+    for (size_t i = 0; i < p.blocks.size(); i++)
+        block_sequence(p, p.blocks[i], x, v_first, caches ? &(*caches)[i] : nullptr, per_token, flags, ws);
+}
+
 // One block of a one-token step; x (B,1,d) takes the residual sum in place.
 void block_step(Plan& p, Block& b, const Tensor& x, Tensor& v_first, const Tensor& state, const Tensor& conv, int64_t pos,
                 const Tensor& pos_dev, const Tensor& ws) {
@@ -139,7 +257,7 @@ bool aligned_dense(const Tensor& t, at::ScalarType dt) {
 bool decode_small_batch(Plan& p, const Tensor& x, const std::vector<Cache>& caches, const Tensor& logits, int64_t pos,
                         const Tensor& pos_dev) {
     const int64_t B = x.size(0), V = p.embedding.size(0);
-    if (!p.small_batch_ok) return false;
+    if (!p.dense_bf16) return false;
     // replayed from a graph, the library's products are not held up by their launches: see lm_decode_takes()
     if (B > kGraphBatch && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return false;
     const size_t bytes = cdssm_b200_lm_decode_workspace_bytes((int)B, (int)p.d_model, (int)p.N, (int)p.groups, (int)V, CDSSM_BF16);
@@ -205,10 +323,10 @@ PyObject* py_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
             for (const Tensor* w : {&b.norm_w, &b.w_in, &b.b_in, &b.conv_w, &b.conv_b, &b.w_qg, &b.b_qg, &b.w_readout, &b.w_out,
                                     &b.gn_w, &b.gn_b, &b.D})
                 ok = ok && aligned_dense(*w, at::kBFloat16);
-            p->small_batch_ok = (i == 0 || p->small_batch_ok) && ok;
+            p->dense_bf16 = (i == 0 || p->dense_bf16) && ok;
             p->blocks.push_back(std::move(b));
         }
-        p->small_batch_ok = p->small_batch_ok && aligned_dense(p->embedding, at::kBFloat16) &&
+        p->dense_bf16 = p->dense_bf16 && aligned_dense(p->embedding, at::kBFloat16) &&
                             aligned_dense(p->final_norm_w, at::kBFloat16);
         return PyCapsule_New(p.release(), kCapsule, [](PyObject* o) {
             delete static_cast<Plan*>(PyCapsule_GetPointer(o, kCapsule));
@@ -226,9 +344,8 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t flags = in.integer();
         const NoGrad ng;
         const c10::cuda::CUDAGuard guard(p.embedding.device());
-        Tensor x = embed(p, ids), v_first;
-        const Tensor ws = gemm_workspace(x);
-        for (Block& b : p.blocks) block_sequence(p, b, x, v_first, nullptr, per_token, flags, ws);
+        const Tensor x = embed(p, ids), ws = gemm_workspace(x);
+        run_blocks(p, x, nullptr, per_token, flags, ws);
         return wrap(head(p, x, ws));
     });
 }
@@ -242,10 +359,10 @@ PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const bool last_only = in.flag();
         const NoGrad ng;
         const c10::cuda::CUDAGuard guard(p.embedding.device());
-        Tensor x = embed(p, ids), v_first;
+        Tensor x = embed(p, ids);
         const Tensor ws = gemm_workspace(x);
         std::vector<Cache> caches(p.blocks.size());
-        for (size_t i = 0; i < p.blocks.size(); i++) block_sequence(p, p.blocks[i], x, v_first, &caches[i], true, 0, ws);
+        run_blocks(p, x, &caches, true, 0, ws);
         if (last_only) x = x.slice(1, x.size(1) - 1, x.size(1));
         PyObject* list = PyList_New(2 * (Py_ssize_t)caches.size());
         if (!list) return nullptr;
@@ -280,7 +397,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (pos_dev.defined() && (pos_dev.scalar_type() != at::kInt || !pos_dev.is_cuda()))
             throw Error("a tensor position must be an int32 CUDA tensor");
         Tensor x = embed(p, ids).view({B, p.d_model}), v_first;
-        if (p.small_batch_ok) {
+        if (p.dense_bf16) {
             const Tensor logits = at::empty({B, p.embedding.size(0)}, x.options());
             if (decode_small_batch(p, x, caches, logits, pos, pos_dev)) return wrap(logits);
         }

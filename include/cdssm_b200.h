@@ -140,6 +140,11 @@ CDSSM_API int cdssm_b200_exact_correction_fwd(const void* A, const void* K, cons
 CDSSM_API int cdssm_b200_conv1d_silu_fwd(const void* x, const void* weight, const void* bias, void* out,
                                int B, int L, int Dm, int dtype, void* stream);
 
+/* The same for x whose rows are x_row_stride elements apart (a column slice of a projection; 0: dense); hist (B,3,Dm) or NULL
+ * receives the last three inputs of every sequence, zeros before its start (what cdssm_b200_conv1d_silu_step goes on from). */
+CDSSM_API int cdssm_b200_conv1d_silu_strided_fwd(const void* x, int64_t x_row_stride, const void* weight, const void* bias,
+                                                 void* out, void* hist, int B, int L, int Dm, int dtype, void* stream);
+
 /* ---- block glue: the memory-bound steps either side of the scan, one kernel each -------------------- */
 
 /* RMSNorm over the last dimension: out = (x * rsqrt(mean(x^2) + eps)) * weight, rows x d, d a multiple of 8,
