@@ -132,6 +132,15 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&p);
 }
 
+// Rounds two values to the storage type with one conversion instruction.
+template <typename T> __device__ __forceinline__ void rnd2(float& a, float& b) {
+    if (IO<T>::kBf16) {
+        const uint32_t w = pack2(a, b);
+        a = __uint_as_float(w << 16);
+        b = __uint_as_float(w & 0xffff0000u);
+    }
+}
+
 template <typename T> struct Vec8;   // eight consecutive elements
 template <> struct Vec8<__nv_bfloat16> {
     static __device__ __forceinline__ void ld(const __nv_bfloat16* p, float* f) {
@@ -154,7 +163,28 @@ template <> struct Vec8<float> {
     }
 };
 
-template <typename T> struct Raw8;   // the same, kept in storage form until used
+template <typename T> struct Vec4;   // four
+template <> struct Vec4<__nv_bfloat16> {
+    uint2 v;
+    __device__ __forceinline__ void ld(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void get(float* f) const {
+        f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+        f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+    }
+    static __device__ __forceinline__ void st(__nv_bfloat16* p, const float* f) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
+    }
+};
+template <> struct Vec4<float> {
+    float4 v;
+    __device__ __forceinline__ void ld(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void get(float* f) const { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
+    static __device__ __forceinline__ void st(float* p, const float* f) {
+        *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+    }
+};
+
+template <typename T> struct Raw8;   // eight, kept in storage form until used
 template <> struct Raw8<__nv_bfloat16> {
     uint4 v;
     __device__ __forceinline__ void ld(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }

@@ -233,61 +233,76 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, long long x_rs, const T* __restr
     }
 }
 
-// Eight channels per thread, 16-byte accesses, the loads of kStep positions in flight together.  Bounded by memory (one read,
-// one write); kSeg: 32 positions where there are enough of them to fill the GPU, else 8.  Measured on B200, bf16: B 8,
-// L 2048, 1536 channels MEASURED_CONV.
+// Four channels per thread, the loads of the next eight positions in flight while eight are worked on (without that the loads
+// sank to their uses and every position waited for memory).  Bounded by memory latency, then bandwidth (one read, one write).
+// kSeg: 32 positions where that still gives the GPU enough threads, else 8.  Measured on B200, bf16, B 8, L 2048, 1536
+// channels: 30 -> 27 us against a channel per thread, a copy takes 18.5 us.
 template <typename T, int kSeg>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(128)
 conv1d_silu_vec_kernel(const T* __restrict__ x, long long x_rs, const T* __restrict__ w, const T* __restrict__ bias,
                        T* __restrict__ out, T* __restrict__ hist, int L, int Dm) {
     constexpr int kStep = 8;
-    const int d = (blockIdx.x * 64 + threadIdx.x) * 8;
+    const int d = (blockIdx.x * 128 + threadIdx.x) * 4;
     if (d >= Dm) return;
     const int l0 = blockIdx.y * kSeg;
     const T* xb = x + (long long)blockIdx.z * L * x_rs + d;
     T* ob = out + (long long)blockIdx.z * L * Dm + d;
-    float x0[8], x1[8], x2[8], bi[8], wt[4][8];     // wt[i]: taps of channels d + 2 i, d + 2 i + 1
+    float x0[4], x1[4], x2[4], bi[4], wt[4][4];
     auto row = [&](int l, float* f) {
-        if (l >= 0) {
-            Vec8<T>::ld(xb + (long long)l * x_rs, f);
-        } else {
+        Vec4<T> v;
+        v.ld(xb + (long long)max(l, 0) * x_rs);
+        v.get(f);
 #pragma unroll
-            for (int e = 0; e < 8; e++) f[e] = 0.f;
-        }
+        for (int e = 0; e < 4; e++) f[e] = l >= 0 ? f[e] : 0.f;
     };
     row(l0 - 3, x0);
     row(l0 - 2, x1);
     row(l0 - 1, x2);
-    Vec8<T>::ld(bias + d, bi);
+    {
+        Vec4<T> v;
+        v.ld(bias + d);
+        v.get(bi);
 #pragma unroll
-    for (int i = 0; i < 4; i++) Vec8<T>::ld(w + d * 4 + 8 * i, wt[i]);
+        for (int i = 0; i < 4; i++) {
+            v.ld(w + (d + i) * 4);
+            v.get(wt[i]);
+        }
+    }
     const int lend = min(l0 + kSeg, L);
-    for (int l1 = l0; l1 < lend; l1 += kStep) {
-        Raw8<T> r[kStep];
+    Vec4<T> r[kStep];
 #pragma unroll
-        for (int s = 0; s < kStep; s++) r[s].ld(xb + (long long)min(l1 + s, L - 1) * x_rs);
+    for (int s = 0; s < kStep; s++) r[s].ld(xb + (long long)min(l0 + s, L - 1) * x_rs);
+#pragma unroll 1
+    for (int l1 = l0; l1 < lend; l1 += kStep) {
+        Vec4<T> n[kStep];
+        if (kSeg > kStep) {   // the next positions travel while these are worked on
+#pragma unroll
+            for (int s = 0; s < kStep; s++) n[s].ld(xb + (long long)min(l1 + kStep + s, L - 1) * x_rs);
+        }
 #pragma unroll
         for (int s = 0; s < kStep; s++) {
-            if (l1 + s >= lend) break;
-            float x3[8], y[8];
+            float x3[4], y[4];
             r[s].get(x3);
 #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const float* ww = wt[e >> 1] + (e & 1) * 4;
-                const float yv = ww[0] * x0[e] + ww[1] * x1[e] + ww[2] * x2[e] + ww[3] * x3[e] + bi[e];
+            for (int e = 0; e < 4; e++) {
+                const float yv = wt[e][0] * x0[e] + wt[e][1] * x1[e] + wt[e][2] * x2[e] + wt[e][3] * x3[e] + bi[e];
                 y[e] = siluf_<IO<T>::kBf16>(yv);
                 x0[e] = x1[e];
                 x1[e] = x2[e];
                 x2[e] = x3[e];
             }
-            Vec8<T>::st(ob + (long long)(l1 + s) * Dm, y);
+            if (l1 + s < lend) Vec4<T>::st(ob + (long long)(l1 + s) * Dm, y);
+            if (kSeg > kStep) r[s] = n[s];
         }
     }
     if (hist != nullptr && lend == L) {
         T* h = hist + (long long)blockIdx.z * 3 * Dm + d;
-        Vec8<T>::st(h, x0);
-        Vec8<T>::st(h + Dm, x1);
-        Vec8<T>::st(h + 2 * Dm, x2);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            float f[4];
+            row(L - 3 + i, f);
+            Vec4<T>::st(h + (long long)i * Dm, f);
+        }
     }
 }
 
@@ -431,15 +446,15 @@ extern "C" int cdssm_b200_conv1d_silu_strided_fwd(const void* x, int64_t x_row_s
     const size_t es = dtype == CDSSM_F32 ? 4 : 2;
     const uintptr_t all = (uintptr_t)x | (uintptr_t)weight | (uintptr_t)bias | (uintptr_t)out | (uintptr_t)hist |
                           (uintptr_t)(x_row_stride * es);
-    if (Dm % 8 == 0 && (all & 15) == 0) {
-        const int cols = (Dm / 8 + 63) / 64;
+    if (Dm % 4 == 0 && (all & (4 * es - 1)) == 0) {
+        const int cols = (Dm / 4 + 127) / 128;
         const bool many = (long long)cols * ((L + 31) / 32) * B >= 148 * 8;
         const int segs = many ? (L + 31) / 32 : (L + 7) / 8;
         if (segs > 65535) return CDSSM_ERR_UNSUPPORTED;
         const dim3 grid(cols, segs, B);
         DISPATCH_DTYPE(dtype, {
-            if (many) conv1d_silu_vec_kernel<T, 32><<<grid, 64, 0, st>>>((const T*)x, x_row_stride, (const T*)weight, (const T*)bias, (T*)out, (T*)hist, L, Dm);
-            else conv1d_silu_vec_kernel<T, 8><<<grid, 64, 0, st>>>((const T*)x, x_row_stride, (const T*)weight, (const T*)bias, (T*)out, (T*)hist, L, Dm);
+            if (many) conv1d_silu_vec_kernel<T, 32><<<grid, 128, 0, st>>>((const T*)x, x_row_stride, (const T*)weight, (const T*)bias, (T*)out, (T*)hist, L, Dm);
+            else conv1d_silu_vec_kernel<T, 8><<<grid, 128, 0, st>>>((const T*)x, x_row_stride, (const T*)weight, (const T*)bias, (T*)out, (T*)hist, L, Dm);
         });
         return check_launch();
     }
