@@ -246,8 +246,9 @@ __device__ __forceinline__ void scalings(cplx at, cplx vg, int tl, cplx& viw, cp
 }
 
 // Step-by-step walk of pair p over this warp's block, for decays the scaled form cannot hold: state columns over the
-// lanes.  kReadout: walk[t] = {q_t.z_t, W_{t-1} from the block start}, else {g_t carried to the block end}.  The incoming state is rebuilt from
-// the fragments the earlier blocks published for this one.
+// lanes.  First without read-out (walk[t].x = |k_t|^-1 in; out walk[t] = {g_t carried to the block end}, and g_t in place of
+// v_t), later with it (walk[t] = {q_t.z_t, W_{t-1} from the block start}; no sums on the way of the state any more).  The
+// incoming state is rebuilt from the fragments the earlier blocks published for this one.
 template <int kD, int kPairs, Mode kMode, bool kReadout>
 __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I, int tl) {
     using G = Geo<kD, kPairs>;
@@ -261,6 +262,7 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
 #pragma unroll
     for (int i = 0; i < kCols; i++) zr[i] = zi[i] = 0.f;
     for (int J = 0; J < I; J++)
+#pragma unroll 4
         for (int t = 0; t < 32; t++) {
             const int half = t >> 4, r = t & 15, q = (r & 7) >> 1;
             auto value = [&](int col) {
@@ -278,22 +280,27 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
             }
         }
     cplx own = {0.f, 0.f};
+#pragma unroll 2
     for (int t = 0; t < 32; t++) {
         const int row = 32 * I + t;
         const float2 a = sm.dd[p][row], vg = sm.viw[p][row];
-        const float be = sm.beta[row];
-        float k[kCols], kk = 0.f, ur = 0.f, ui = 0.f;
+        float k[kCols];
 #pragma unroll
-        for (int i = 0; i < kCols; i++) {
-            k[i] = column(sm.k, row, tl + 32 * i);
-            kk += k[i] * k[i];
-            ur += zr[i] * k[i];
-            ui += zi[i] * k[i];
+        for (int i = 0; i < kCols; i++) k[i] = column(sm.k, row, tl + 32 * i);
+        cplx gt = {vg.x, vg.y};               // read-out: g_t as the first walk left it
+        if (!kReadout) {
+            const float be = sm.beta[row], n = sm.walk[I][t].x;
+            float ur = 0.f, ui = 0.f;
+#pragma unroll
+            for (int i = 0; i < kCols; i++) {
+                ur += zr[i] * k[i];
+                ui += zi[i] * k[i];
+            }
+            ur = warp_sum(ur); ui = warp_sum(ui);
+            const cplx au = cmul({a.x, a.y}, {n * ur, n * ui});
+            gt = {be * n * (vg.x - au.r), be * n * (vg.y - au.i)};
+            if (tl == t) own = gt;
         }
-        kk = warp_sum(kk); ur = warp_sum(ur); ui = warp_sum(ui);
-        const float n = rsqrtf(kk + kEps);
-        const cplx au = cmul({a.x, a.y}, {n * ur, n * ui});
-        const cplx gt = {be * n * (vg.x - au.r), be * n * (vg.y - au.i)};
 #pragma unroll
         for (int i = 0; i < kCols; i++) {
             const cplx z = cmul({a.x, a.y}, {zr[i], zi[i]});
@@ -310,10 +317,10 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
             }
             yr = warp_sum(yr); yi = warp_sum(yi);
             if (tl == t) own = {yr, yi};
-        } else if (tl == t) {
-            own = gt;
         }
     }
+    __syncwarp();
+    if (!kReadout) sm.viw[p][32 * I + tl] = make_float2(own.r, own.i);
     // g carried to the block end: times a_{t+1} ... a_31; W_{t-1} = a_0 ... a_{t-1}
     const float2 a = sm.dd[p][32 * I + tl];
     cplx S = {a.x, a.y};
@@ -329,6 +336,15 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
     __syncwarp();
     sm.walk[I][tl] = make_float4(own.r, own.i, V.r, V.i);
     __syncwarp();
+}
+
+// s <- gamma s + l in the order in which the carry pass (scan_simt.cu) evaluates it, so that the two ways to hand the carry on
+// give the same bits: chunk-aligned pieces of a sequence compose exactly whichever of them their lengths choose.
+__device__ __forceinline__ float next_re(cplx g, float sr, float si, float l) {
+    return __fadd_rn(__fmaf_rn(g.r, sr, -__fmul_rn(g.i, si)), l);
+}
+__device__ __forceinline__ float next_im(cplx g, float sr, float si, float l) {
+    return __fadd_rn(__fmaf_rn(g.r, si, __fmul_rn(g.i, sr)), l);
 }
 
 // resident blocks per SM the registers are cut for (more blocks spill: N 16, head_dim 64, 5 / 7 / 8 blocks: 279 / 308 / 328 us)
@@ -616,6 +632,11 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll 1
             for (int s = 0; s < kPerTile; s++)   // decays beyond the scaled form: step by step
                 if (sm.bp[2 * q + s][I].slow) {
+                    if (t4 == 0) {
+#pragma unroll
+                        for (int r = 0; r < 4; r++) sm.walk[I][8 * r + g].x = nrm[r];
+                    }
+                    __syncwarp();
                     slow_walk<kD, kPairs, kMode, false>(sm, 2 * q + s, I, tl);
                     if (kPairs == 1 || (t4 >> 1) == s) {
 #pragma unroll
@@ -723,7 +744,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                             a.ws_state[(unit * N + n) * kD + d] = l;
                         } else {
                             const float sr = sm.s_in[2 * p][d], si = sm.s_in[2 * p + 1][d];
-                            const float s = comp ? gam.r * si + gam.i * sr + l : gam.r * sr - gam.i * si + l;
+                            const float s = comp ? next_im(gam, sr, si, l) : next_re(gam, sr, si, l);
                             if (c + 1 < a.NC) a.ws_state[((unit + H) * N + n) * kD + d] = s;
                             else if (a.final_state) a.final_state[(((size_t)b * H + hd) * N + n) * kD + d] = s;
                         }
@@ -926,7 +947,11 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             if (a.shortcut_scale != 0.f) {   // block.py:202-208; v after the vp scale
                 const float qk = mq[r] * nrm[r] * pd[r];
                 const float2 e = sm.viw[p][row], D = sm.dd[p][row];
-                const cplx vg = sm.bp[p][I].slow ? cplx{e.x, e.y} : cmul({e.x, e.y}, {D.x, D.y});
+                cplx vg = cmul({e.x, e.y}, {D.x, D.y});
+                if (sm.bp[p][I].slow) {               // (its v has made room for g)
+                    const uint32_t w = __ldcg(a.rec_v + (unit * (size_t)NP + p) * kD + row);
+                    vg = {bits_lo(w), bits_hi(w)};
+                }
                 yy += a.shortcut_scale * qk * qk * bfr(comp ? vg.i : vg.r);
             }
             if (kPairs > 1 || t4 < 2) sm.y(I, 8 * r + g)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * sm.sel[row]);

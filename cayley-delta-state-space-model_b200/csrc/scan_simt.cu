@@ -833,16 +833,16 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
 }
 
 // Whether the whole-chunk scan runs as one kernel that hands the carry from chunk to chunk inside it, or as local pass +
-// carry pass + output pass.  One kernel reads k once and computes G once, but a hand-off takes 2 us (flag, carry, rounding,
-// release), so a (batch, head) chain of NC chunks takes 2 NC us whatever the size; the three passes cost a third more work
-// and two launches of which each is as long as one chunk takes.  Measured on B200, us, one kernel / three passes (D 64):
-//     N 4,  H 24, L 2048:  B 4   77 / 82    B 8  126 / 161        N 16, H 24, L 2048: B 4 165 / 175   B 8 251 / 329
-//     N 16, H 24, L 523:   B 1   58 / 73    N 16, H 24, L 16384: B 1 735 / 345     N 2, H 6, L 4096: B 1 109 / 30
-// so: where the chunks that run beside each other cover a hand-off (a chunk's share of a full GPU is per_chunk ns), or the
-// chain is short.
+// carry pass + output pass.  One kernel reads k once and forms G once, but a hand-off takes 1.6 to 2 us (flag, carry, rounding,
+// release), so a (batch, head) chain of NC chunks takes that many whatever the size; the three passes cost a third more work.
+// us on B200, fitted to 100 sizes (one kernel / three passes, D 64): N 16, H 24: L 64 21 / 29, L 4096 186 / 130, B 4, L 2048
+// 180 / 168, B 8 220 / 303; N 2, H 6: L 523 23 / 18, L 4096 112 / 23; D 128, N 4, H 24, B 8, L 2048 176 / 257.
 static bool one_kernel_pays(int B, int H, int NC, int D, int N) {
-    const float per_chunk = D == 64 ? 14.f + 1.7f * N : 40.f + (N > 8 ? 9.f : 5.f) * N;
-    return (float)B * (float)H * per_chunk >= 1800.f || NC <= 4 + N / 2;
+    const float units = (float)B * H * NC, n = (float)N;
+    const float per_unit = D == 64 ? 0.0125f + 0.0015f * n : 0.036f + (N > 8 ? 0.0089f : 0.0053f) * n;   // us, full GPU
+    const float one = D == 64 ? 11.f + 0.6f * n : 14.f + n, three = D == 64 ? 16.f + 0.8f * n : 23.f + 1.2f * n;   // alone
+    const float a = one + (1.6f + 0.03f * n) * NC, b = units * per_unit, c = units * per_unit * 1.35f;
+    return (a > b ? a : b) <= (three > c ? three : c);
 }
 
 struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual
