@@ -141,6 +141,26 @@ template <typename T> __device__ __forceinline__ void rnd2(float& a, float& b) {
     }
 }
 
+// Two consecutive elements as one access where `vec` says they are aligned.
+template <typename T> __device__ __forceinline__ float2 ld_pair(const T* p, bool vec) {
+    if (!vec) return make_float2(IO<T>::ld(p), IO<T>::ld(p + 1));
+    if (IO<T>::kBf16) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(p);
+        return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    }
+    return *reinterpret_cast<const float2*>(p);
+}
+template <typename T> __device__ __forceinline__ void st_pair(T* p, bool vec, float a, float b) {
+    if (!vec) {
+        IO<T>::st(p, a);
+        IO<T>::st(p + 1, b);
+    } else if (IO<T>::kBf16) {
+        *reinterpret_cast<uint32_t*>(p) = pack2(a, b);
+    } else {
+        *reinterpret_cast<float2*>(p) = make_float2(a, b);
+    }
+}
+
 template <typename T> struct Vec8;   // eight consecutive elements
 template <> struct Vec8<__nv_bfloat16> {
     static __device__ __forceinline__ void ld(const __nv_bfloat16* p, float* f) {

@@ -3,74 +3,11 @@
 // (lm_decode.cu).
 #pragma once
 #include "cdssm_common.cuh"
+#include "row_slice.cuh"
 
 namespace cdssm {
 
 constexpr int kLanesPerUnit = 8;
-
-template <int kLanes = 8>
-__device__ __forceinline__ float group_sum(float v) {   // sum over the kLanes (8 or 16) lanes of a unit
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    if (kLanes == 16) v += __shfl_xor_sync(0xffffffffu, v, 8);
-    return v;
-}
-
-// Raw (storage-typed) slice of one row: kCols contiguous columns starting at g*kCols.  (Plain loads: kernels that start
-// before their predecessor has finished must not move them above the wait, which __ldg would allow.)
-template <typename T, int kCols> struct RowSlice;
-template <int kCols> struct RowSlice<__nv_bfloat16, kCols> {
-    uint4 v[kCols / 8];
-    __device__ __forceinline__ void load(const __nv_bfloat16* row, int g, int D, bool vec) {
-        if (vec) {
-            const uint4* p = reinterpret_cast<const uint4*>(row + g * kCols);
-#pragma unroll
-            for (int i = 0; i < kCols / 8; i++) v[i] = p[i];
-        } else {
-            unsigned short* s = reinterpret_cast<unsigned short*>(v);
-#pragma unroll
-            for (int i = 0; i < kCols; i++) {
-                const int d = g * kCols + i;
-                s[i] = d < D ? reinterpret_cast<const unsigned short*>(row)[d] : (unsigned short)0;
-            }
-        }
-    }
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int i = 0; i < kCols / 8; i++) v[i] = make_uint4(0, 0, 0, 0);
-    }
-    __device__ __forceinline__ void get(float* f) const {
-#pragma unroll
-        for (int i = 0; i < kCols / 8; i++) unpack8(v[i], f + 8 * i);
-    }
-};
-template <int kCols> struct RowSlice<float, kCols> {
-    float4 v[kCols / 4];
-    __device__ __forceinline__ void load(const float* row, int g, int D, bool vec) {
-        if (vec) {
-            const float4* p = reinterpret_cast<const float4*>(row + g * kCols);
-#pragma unroll
-            for (int i = 0; i < kCols / 4; i++) v[i] = p[i];
-        } else {
-            float* s = reinterpret_cast<float*>(v);
-#pragma unroll
-            for (int i = 0; i < kCols; i++) {
-                const int d = g * kCols + i;
-                s[i] = d < D ? row[d] : 0.f;
-            }
-        }
-    }
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int i = 0; i < kCols / 4; i++) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __device__ __forceinline__ void get(float* f) const {
-        const float* s = reinterpret_cast<const float*>(v);
-#pragma unroll
-        for (int i = 0; i < kCols; i++) f[i] = s[i];
-    }
-};
 
 // x * rsqrt(sum x^2 + 1e-6) over the unit's row, rounded like the reference's K_norm/Q_norm
 // store (normalize_kq.cu:72-79).

@@ -8,11 +8,12 @@
 // Thread mappings differ from the reference's (one block of D threads per (chunk, head) with
 // two block barriers per step):
 //   * the complex pairs of a head never interact (each pair owns two state rows; the erase
-//     uses a per-row dot product), so the sequential kernels run one WARP per
-//     (chunk, head, pair): the per-step reduction is a warp shuffle, no barrier at all;
+//     uses a per-row dot product), so the sequential kernels run a few LANES per
+//     (chunk, head, pair): the per-step reduction is a few shuffles, no barrier at all;
 //   * the dynamics kernel maps consecutive threads to consecutive heads so that every gate
 //     segment is read coalesced.
 #include "cdssm_common.cuh"
+#include "row_slice.cuh"
 
 namespace cdssm {
 
@@ -50,7 +51,33 @@ dynamics_fwd_kernel(const T* __restrict__ gate_raw, const float* __restrict__ lo
 }
 
 // ---------------------------------------------------------------- normalise
-// One warp per row pair (K row and Q row of the same token-head).
+// Eight lanes per row pair (K row and Q row of a token-head) of 64 columns, 16 of 128, one 16-byte access per row and lane;
+// other sizes, and unaligned rows, take a warp each.  Bounded by memory.  Measured on B200, bf16, 98 304 rows of 64: MEASURED_NF.
+template <typename T, int kLanes>
+__global__ void __launch_bounds__(256)
+normalize_kq_fwd_rows_kernel(const T* __restrict__ K, const T* __restrict__ Q, T* __restrict__ Ko, T* __restrict__ Qo, long long rows) {
+    constexpr int kCols = 8, kD = kCols * kLanes;
+    const int g = threadIdx.x % kLanes;
+    long long row = (long long)blockIdx.x * (256 / kLanes) + threadIdx.x / kLanes;
+    const bool on = row < rows;
+    if (!on) row = rows - 1;
+    RowSlice<T, kCols> rk, rq;
+    rk.load(K + row * kD, g, kD, true);
+    rq.load(Q + row * kD, g, kD, true);
+    auto side = [&](const RowSlice<T, kCols>& x, T* out) {
+        float f[kCols], ss = 0.f;
+        x.get(f);
+#pragma unroll
+        for (int i = 0; i < kCols; i++) ss += f[i] * f[i];
+        const float n = rsqrtf(group_sum<kLanes>(ss) + kEps);
+#pragma unroll
+        for (int i = 0; i < kCols; i++) f[i] *= n;
+        if (on) RowSlice<T, kCols>::store(out + row * kD, g, kD, true, f);
+    };
+    side(rk, Ko);
+    side(rq, Qo);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 normalize_kq_fwd_kernel(const T* __restrict__ K, const T* __restrict__ Q, T* __restrict__ Ko,
@@ -75,99 +102,97 @@ normalize_kq_fwd_kernel(const T* __restrict__ K, const T* __restrict__ Q, T* __r
     }
 }
 
-// ---------------------------------------------------------------- intra-chunk scan
-// One warp per (chunk, head, pair).  Lane owns columns lane, lane+32, ... of the pair's two rows.
-template <typename T, bool kInject>
+// ---------------------------------------------------------------- intra-chunk scan and correction
+// kLanes lanes (8 for D <= 64, 16 above) own one (chunk, head, pair), eight contiguous columns of its two state rows each; the
+// next token's inputs are on their way while a step is taken.  Bounded by the states written.  Measured on B200, bf16, 64 chunks
+// of 64, 24 heads, N 16, D 64 (201 MB written): MEASURED_WALK.
+template <typename T, int kLanes, bool kInject>
 __global__ void __launch_bounds__(128)
 chunk_walk_kernel(const T* __restrict__ A, const T* __restrict__ K, const T* __restrict__ V,
                   const T* __restrict__ beta, const T* __restrict__ init,  // correction: carry in
                   T* __restrict__ states,   // local_h or corrections (units,C,H,N,D)
                   T* __restrict__ cum_A,    // intra only
-                  long long units, int C, int H, int D, int N) {
-    const int NH = N >> 1;
-    const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (w >= units * H * NH) return;
-    const int lane = threadIdx.x & 31;
+                  long long units, int C, int H, int D, int N, bool vec) {
+    constexpr int kCols = 8, kP = kCols / 2;
+    const int NH = N >> 1, g = threadIdx.x % kLanes;
+    long long w = (long long)blockIdx.x * (128 / kLanes) + threadIdx.x / kLanes;
+    const bool active = w < units * H * NH;
+    if (!active) w = units * H * NH - 1;                 // keep the lane in the shuffles
     const int j = (int)(w % NH);
     const int hd = (int)((w / NH) % H);
     const long long c = w / ((long long)NH * H);
-    constexpr int kCols = kMaxHeadDim / 32;
-    float zr[kCols], zi[kCols];
+    const long long row0 = c * C * H + hd;
+    const T* Ap = A + row0 * N + 2 * j;
+    const T* Kp = K + row0 * D;
+    const T* Vp = kInject ? V + row0 * N + 2 * j : nullptr;
+    const T* Bp = beta + row0;
+    T* out = states + (row0 * N + 2 * j) * (long long)D;
+    T* cum = kInject ? cum_A + row0 * N + 2 * j : nullptr;
+    float2 zr[kP], zi[kP];
 #pragma unroll
-    for (int i = 0; i < kCols; i++) {
-        zr[i] = 0.f;
-        zi[i] = 0.f;
-        if (!kInject) {
-            const int d = lane + 32 * i;
-            if (d < D) {
-                const T* p = init + ((c * H + hd) * N + 2 * j) * (long long)D + d;
-                zr[i] = IO<T>::ld(p);
-                zi[i] = IO<T>::ld(p + D);
-            }
-        }
+    for (int i = 0; i < kP; i++) zr[i] = zi[i] = make_float2(0.f, 0.f);
+    if (!kInject) {
+        RowSlice<T, kCols> s;
+        const T* p = init + ((c * H + hd) * N + 2 * j) * (long long)D;
+        s.load(p, g, D, vec);
+        s.get(reinterpret_cast<float*>(zr));
+        s.load(p + D, g, D, vec);
+        s.get(reinterpret_cast<float*>(zi));
     }
+    auto store = [&]() {
+        if (!active) return;
+        RowSlice<T, kCols>::store(out, g, D, vec, reinterpret_cast<const float*>(zr));
+        RowSlice<T, kCols>::store(out + D, g, D, vec, reinterpret_cast<const float*>(zi));
+    };
     float cr = 1.f, ci = 0.f;
+    RowSlice<T, kCols> kraw;
+    float a_re, a_im, b, vr = 0.f, vi = 0.f;
+    auto fetch = [&]() {
+        kraw.load(Kp, g, D, vec);
+        a_re = IO<T>::ld(Ap); a_im = IO<T>::ld(Ap + 1);
+        b = IO<T>::ld(Bp);
+        if (kInject) { vr = IO<T>::ld(Vp); vi = IO<T>::ld(Vp + 1); }
+    };
+    fetch();
     for (int t = 0; t < C; t++) {
-        const long long row = (c * C + t) * H + hd;
-        if (!kInject) {  // correction stores the state BEFORE the step (exact_correction.cu:90-94)
-            T* out = states + (row * N + 2 * j) * (long long)D;
-#pragma unroll
-            for (int i = 0; i < kCols; i++) {
-                const int d = lane + 32 * i;
-                if (d < D) {
-                    IO<T>::st(out + d, zr[i]);
-                    IO<T>::st(out + D + d, zi[i]);
-                }
-            }
+        float2 k[kP];
+        kraw.get(reinterpret_cast<float*>(k));
+        const float ar = a_re, ai = a_im, be = b, v0 = vr, v1 = vi;
+        if (t + 1 < C) {
+            Ap += (long long)H * N; Kp += (long long)H * D; Bp += H;
+            if (kInject) Vp += (long long)H * N;
+            fetch();
         }
-        const float a_re = IO<T>::ld(A + row * N + 2 * j), a_im = IO<T>::ld(A + row * N + 2 * j + 1);
-        const float b = IO<T>::ld(beta + row);
-        float kk[kCols], ur = 0.f, ui = 0.f;
+        if (!kInject) store();   // correction stores the state BEFORE the step (exact_correction.cu:90-94)
+        float2 ur2 = make_float2(0.f, 0.f), ui2 = ur2;
 #pragma unroll
-        for (int i = 0; i < kCols; i++) {
-            const int d = lane + 32 * i;
-            kk[i] = d < D ? IO<T>::ld(K + row * D + d) : 0.f;
-            ur += zr[i] * kk[i];
-            ui += zi[i] * kk[i];
+        for (int i = 0; i < kP; i++) {
+            ur2 = __ffma2_rn(zr[i], k[i], ur2);
+            ui2 = __ffma2_rn(zi[i], k[i], ui2);
         }
-        ur = warp_sum(ur);
-        ui = warp_sum(ui);
-        float vr = 0.f, vi = 0.f;
-        if (kInject) {
-            vr = IO<T>::ld(V + row * N + 2 * j);
-            vi = IO<T>::ld(V + row * N + 2 * j + 1);
-        }
+        const float ur = -be * group_sum<kLanes>(ur2.x + ur2.y), ui = -be * group_sum<kLanes>(ui2.x + ui2.y);
+        // z' = a (z + u k) + beta v k
+        const float kr = ar * ur - ai * ui + be * v0, ki = ar * ui + ai * ur + be * v1;
+        const float2 ar2 = make_float2(ar, ar), ai2 = make_float2(ai, ai), ni2 = make_float2(-ai, -ai);
+        const float2 kr2 = make_float2(kr, kr), ki2 = make_float2(ki, ki);
 #pragma unroll
-        for (int i = 0; i < kCols; i++) {
-            float er = zr[i] - b * ur * kk[i];
-            float ei = zi[i] - b * ui * kk[i];
-            float nr = a_re * er - a_im * ei;
-            float ni = a_re * ei + a_im * er;
-            if (kInject) {
-                nr += b * vr * kk[i];
-                ni += b * vi * kk[i];
-            }
-            zr[i] = nr;
-            zi[i] = ni;
+        for (int i = 0; i < kP; i++) {
+            const float2 x = zr[i], y = zi[i];
+            zr[i] = __ffma2_rn(kr2, k[i], __ffma2_rn(ar2, x, __fmul2_rn(ni2, y)));
+            zi[i] = __ffma2_rn(ki2, k[i], __ffma2_rn(ar2, y, __fmul2_rn(ai2, x)));
         }
-        if (kInject) {  // local scan stores the state AFTER the step (intra_chunk_scan.cu:169-173)
-            T* out = states + (row * N + 2 * j) * (long long)D;
-#pragma unroll
-            for (int i = 0; i < kCols; i++) {
-                const int d = lane + 32 * i;
-                if (d < D) {
-                    IO<T>::st(out + d, zr[i]);
-                    IO<T>::st(out + D + d, zi[i]);
-                }
-            }
-            const float nr = a_re * cr - a_im * ci, ni = a_re * ci + a_im * cr;
+        if (kInject) {           // local scan stores the state AFTER the step (intra_chunk_scan.cu:169-173)
+            store();
+            const float nr = ar * cr - ai * ci, ni = ar * ci + ai * cr;
             cr = nr;
             ci = ni;
-            if (lane == 0) {
-                IO<T>::st(cum_A + row * N + 2 * j, cr);
-                IO<T>::st(cum_A + row * N + 2 * j + 1, ci);
+            if (g == 0 && active) {
+                IO<T>::st(cum, cr);
+                IO<T>::st(cum + 1, ci);
             }
+            cum += (long long)H * N;
         }
+        out += (long long)H * N * D;
     }
 }
 
@@ -377,6 +402,18 @@ extern "C" int cdssm_b200_normalize_kq_fwd(const void* K, const void* Q, void* K
                                            int64_t rows, int D, int dtype, void* stream) {
     if (!K || !Q || !K_out || !Q_out || rows < 0 || D <= 0) return CDSSM_ERR_BAD_ARG;
     if (rows == 0) return CDSSM_OK;
+    if (((((uintptr_t)K | (uintptr_t)Q | (uintptr_t)K_out | (uintptr_t)Q_out) & 15) == 0) && (D == 64 || D == 128)) {
+        DISPATCH_DTYPE(dtype, {
+            auto launch = [&](auto kernel, int lanes) {
+                const int per = 256 / lanes;
+                kernel<<<(unsigned)((rows + per - 1) / per), 256, 0, (cudaStream_t)stream>>>((const T*)K, (const T*)Q, (T*)K_out,
+                                                                                             (T*)Q_out, rows);
+            };
+            if (D == 64) launch(normalize_kq_fwd_rows_kernel<T, 8>, 8);
+            else launch(normalize_kq_fwd_rows_kernel<T, 16>, 16);
+        });
+        return check_launch();
+    }
     const unsigned blocks = (unsigned)((rows + 7) / 8);
     DISPATCH_DTYPE(dtype, (normalize_kq_fwd_kernel<T><<<blocks, 256, 0, (cudaStream_t)stream>>>(
                               (const T*)K, (const T*)Q, (T*)K_out, (T*)Q_out, rows, D)));
@@ -397,10 +434,16 @@ extern "C" int cdssm_b200_intra_chunk_scan_fwd(const void* A, const void* K, con
     if (int rc = check_scan_dims(C, H, D, N)) return rc;
     const long long warps = (long long)BNC * H * (N / 2);
     if (warps == 0) return CDSSM_OK;
-    const unsigned blocks = (unsigned)((warps + 3) / 4);
-    DISPATCH_DTYPE(dtype, (chunk_walk_kernel<T, true><<<blocks, 128, 0, (cudaStream_t)stream>>>(
-                              (const T*)A, (const T*)K, (const T*)V, (const T*)beta, nullptr,
-                              (T*)local_h, (T*)cum_A, BNC, C, H, D, N)));
+    const bool aligned = (((uintptr_t)K | (uintptr_t)local_h) & 15) == 0;   // 16-byte pieces of rows
+    DISPATCH_DTYPE(dtype, {
+        auto launch = [&](auto kernel, int lanes) {
+            const int per = 128 / lanes;
+            kernel<<<(unsigned)((warps + per - 1) / per), 128, 0, (cudaStream_t)stream>>>(
+                (const T*)A, (const T*)K, (const T*)V, (const T*)beta, nullptr, (T*)local_h, (T*)cum_A, BNC, C, H, D, N, D == 8 * lanes && aligned);
+        };
+        if (D <= 64) launch(chunk_walk_kernel<T, 8, true>, 8);
+        else launch(chunk_walk_kernel<T, 16, true>, 16);
+    });
     return check_launch();
 }
 
@@ -414,10 +457,16 @@ extern "C" int cdssm_b200_exact_correction_fwd(const void* A, const void* K, con
     const long long units = (long long)B * NC;
     const long long warps = units * H * (N / 2);
     if (warps == 0) return CDSSM_OK;
-    const unsigned blocks = (unsigned)((warps + 3) / 4);
-    DISPATCH_DTYPE(dtype, (chunk_walk_kernel<T, false><<<blocks, 128, 0, (cudaStream_t)stream>>>(
-                              (const T*)A, (const T*)K, nullptr, (const T*)beta,
-                              (const T*)chunk_states, (T*)corrections, nullptr, units, C, H, D, N)));
+    const bool aligned = (((uintptr_t)K | (uintptr_t)chunk_states | (uintptr_t)corrections) & 15) == 0;
+    DISPATCH_DTYPE(dtype, {
+        auto launch = [&](auto kernel, int lanes) {
+            const int per = 128 / lanes;
+            kernel<<<(unsigned)((warps + per - 1) / per), 128, 0, (cudaStream_t)stream>>>(
+                (const T*)A, (const T*)K, nullptr, (const T*)beta, (const T*)chunk_states, (T*)corrections, nullptr, units, C, H, D, N, D == 8 * lanes && aligned);
+        };
+        if (D <= 64) launch(chunk_walk_kernel<T, 8, false>, 8);
+        else launch(chunk_walk_kernel<T, 16, false>, 16);
+    });
     return check_launch();
 }
 
