@@ -7,6 +7,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <array>
 #include <string>
 
 #include "../../../include/cdssm_b200.h"
@@ -159,5 +160,6 @@ PyObject* guarded(F&& fn) {
 inline PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
 
 PyMethodDef* model_methods();   // lm.cpp
+PyMethodDef* train_methods();   // train.cpp
 
 }  // namespace cdssm_host

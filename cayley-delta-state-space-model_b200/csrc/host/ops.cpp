@@ -346,7 +346,7 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_cdssm_host", "Native host path 
 
 PyMODINIT_FUNC PyInit__cdssm_host() {
     PyObject* m = PyModule_Create(&cdssm_host::g_module);
-    if (m && PyModule_AddFunctions(m, cdssm_host::model_methods()) < 0) {
+    if (m && (PyModule_AddFunctions(m, cdssm_host::model_methods()) < 0 || PyModule_AddFunctions(m, cdssm_host::train_methods()) < 0)) {
         Py_DECREF(m);
         return nullptr;
     }

@@ -63,16 +63,7 @@ class CUDAConv1dSiLUOp(Function):
 
     @staticmethod
     def forward(ctx, x: Tensor, weight: Tensor, bias: Tensor) -> Tensor:
-        x = _prep(x, name="x")
-        if weight.shape[-1] != 4:
-            raise CdssmError("Only kernel_size=4 is supported")   # conv1d_silu.cu:241
-        B, L, Dm = x.shape
-        w = _prep(weight.detach().to(x.dtype), name="weight").reshape(Dm, 4)
-        b = _prep(bias.detach().to(x.dtype), name="bias")
-        out = torch.empty_like(x)
-        with torch.cuda.device(x.device):
-            check(_lib.lib().cdssm_b200_conv1d_silu_fwd(_p(x), _p(w), _p(b), _p(out), B, L, Dm,
-                                                        _dtype_code(x), _stream()), "conv1d_silu_fwd")
+        out, x, w, b = _lib.host().conv_fwd(x, weight, bias)
         ctx.save_for_backward(x, w, b)
         ctx.param_meta = (weight.shape, weight.dtype, bias.dtype)
         return out
@@ -80,15 +71,7 @@ class CUDAConv1dSiLUOp(Function):
     @staticmethod
     def backward(ctx, grad_out):
         """(grad_x, grad_weight, grad_bias), as cdssm/ops.py:22-28 (conv1d_silu.cu:94-219)."""
-        x, w, b = ctx.saved_tensors
-        B, L, Dm = x.shape
-        go = _prep(grad_out.to(x.dtype), name="grad_out")
-        gx = torch.empty_like(x)
-        gw = torch.empty(Dm, 4, dtype=torch.float32, device=x.device)
-        gb = torch.empty(Dm, dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
-            check(_lib.lib().cdssm_b200_conv1d_silu_bwd(_p(go), _p(x), _p(w), _p(b), _p(gx), _p(gw), _p(gb), B, L, Dm,
-                                                        _dtype_code(x), _stream()), "conv1d_silu_bwd")
+        gx, gw, gb = _lib.host().conv_bwd(grad_out, *ctx.saved_tensors)
         wshape, wdt, bdt = ctx.param_meta
         return gx, gw.reshape(wshape).to(wdt), gb.to(bdt)
 
@@ -100,43 +83,16 @@ class DynamicsFusedFn(Function):
     def forward(ctx, gate_raw: Tensor, log_dt_scale: Tensor, rope_freqs: Tensor, gating_c: float,
                 omega_thresh: float, adt_delta: float, adt_smoothness: float, adt_eps: float,
                 n_heads: int, state_dim: int):
-        g = _prep(gate_raw, name="gate_raw")
-        B, L, GH = g.shape
-        H, N = int(n_heads), int(state_dim)
-        if GH != (N + 5) * H:
-            raise CdssmError(f"gate_raw last dim {GH} != (state_dim+5)*n_heads = {(N + 5) * H}")
-        lds, rf = _f32(log_dt_scale, "log_dt_scale"), _f32(rope_freqs, "rope_freqs")
-        o = dict(dtype=g.dtype, device=g.device)
-        A = torch.empty(B, L, H, N, **o)
-        vp = torch.empty(B, L, H, N // 2, **o)
-        beta = torch.empty(B, L, H, **o)
-        selc = torch.empty(B, L, H, **o)
-        with torch.cuda.device(g.device):
-            check(_lib.lib().cdssm_b200_dynamics_fwd(
-                _p(g), _p(lds), _p(rf), _p(A), _p(vp), _p(beta), _p(selc), gating_c, omega_thresh,
-                adt_delta, adt_smoothness, adt_eps, B, L, H, N, 0, _dtype_code(g), _stream()),
-                "dynamics_fwd")
+        ctx.args = (gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps, n_heads, state_dim)
+        A, vp, beta, selc, g, lds, rf = _lib.host().dynamics_fwd(gate_raw, log_dt_scale, rope_freqs, *ctx.args)
         ctx.save_for_backward(g, lds, rf)
-        ctx.consts = (gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps)
-        ctx.dims = (B, L, H, N)
         ctx.lds_dtype = log_dt_scale.dtype
         return A, vp, beta, selc
 
     @staticmethod
     def backward(ctx, grad_A_bar, grad_vp_scale, grad_beta, grad_sel_C):
         """(grad_gate_raw, grad_log_dt_scale, None x 8), as cdssm/ops.py:68-81 (dynamics_fused.cu:145-387)."""
-        g, lds, rf = ctx.saved_tensors
-        B, L, H, N = ctx.dims
-        z = lambda t, shape: (torch.zeros(shape, dtype=g.dtype, device=g.device) if t is None
-                              else _prep(t.to(g.dtype), name="upstream gradient"))
-        gA, gvp = z(grad_A_bar, (B, L, H, N)), z(grad_vp_scale, (B, L, H, N // 2))
-        gb, gc = z(grad_beta, (B, L, H)), z(grad_sel_C, (B, L, H))
-        gg = torch.empty_like(g)
-        glds = torch.empty(H, dtype=torch.float32, device=g.device)
-        with torch.cuda.device(g.device):
-            check(_lib.lib().cdssm_b200_dynamics_bwd(
-                _p(gA), _p(gvp), _p(gb), _p(gc), _p(g), _p(lds), _p(rf), _p(gg), _p(glds), *ctx.consts, B, L, H, N, 0,
-                _dtype_code(g), _stream()), "dynamics_bwd")
+        gg, glds = _lib.host().dynamics_bwd(grad_A_bar, grad_vp_scale, grad_beta, grad_sel_C, *ctx.saved_tensors, *ctx.args)
         return (gg, glds.to(ctx.lds_dtype)) + (None,) * 8
 
 
@@ -145,32 +101,14 @@ class NormalizeKQFn(Function):
 
     @staticmethod
     def forward(ctx, K: Tensor, Q: Tensor):
-        K = _prep(K, name="K")
-        Q = _prep(Q, dtype=K.dtype, name="Q")
-        if K.shape != Q.shape:
-            raise CdssmError("K and Q must have the same shape")
-        D = K.shape[-1]
-        Ko, Qo = torch.empty_like(K), torch.empty_like(Q)
-        with torch.cuda.device(K.device):
-            check(_lib.lib().cdssm_b200_normalize_kq_fwd(_p(K), _p(Q), _p(Ko), _p(Qo),
-                                                         K.numel() // D, D, _dtype_code(K), _stream()),
-                  "normalize_kq_fwd")
+        Ko, Qo, K, Q = _lib.host().normalize_fwd(K, Q)
         ctx.save_for_backward(K, Q)
         return Ko, Qo
 
     @staticmethod
     def backward(ctx, grad_K_out, grad_Q_out):
         """(grad_K, grad_Q), as cdssm/ops.py:93-97 (normalize_kq.cu:89-163)."""
-        K, Q = ctx.saved_tensors
-        D = K.shape[-1]
-        z = lambda t: torch.zeros_like(K) if t is None else _prep(t.to(K.dtype), name="upstream gradient")
-        gKo, gQo = z(grad_K_out), z(grad_Q_out)
-        gK, gQ = torch.empty_like(K), torch.empty_like(Q)
-        with torch.cuda.device(K.device):
-            check(_lib.lib().cdssm_b200_normalize_kq_bwd(_p(gKo), _p(gQo), _p(K), _p(Q), _p(gK), _p(gQ),
-                                                         K.numel() // D, D, _dtype_code(K), _stream()),
-                  "normalize_kq_bwd")
-        return gK, gQ
+        return _lib.host().normalize_bwd(grad_K_out, grad_Q_out, *ctx.saved_tensors)
 
 
 class IntraChunkScanFn(Function):
@@ -178,38 +116,15 @@ class IntraChunkScanFn(Function):
 
     @staticmethod
     def forward(ctx, A_flat: Tensor, K_flat: Tensor, V_flat: Tensor, beta_flat: Tensor, state_dim: int):
-        K = _prep(K_flat, name="K_flat")
-        A = _prep(A_flat, dtype=K.dtype, name="A_flat")
-        V = _prep(V_flat, dtype=K.dtype, name="V_flat")
-        be = _prep(beta_flat, dtype=K.dtype, name="beta_flat")
-        BNC, C, H, D = K.shape
-        N = int(state_dim)
-        local_h = torch.empty(BNC, C, H, N, D, dtype=K.dtype, device=K.device)
-        cum_A = torch.empty(BNC, C, H, N, dtype=K.dtype, device=K.device)
-        with torch.cuda.device(K.device):
-            check(_lib.lib().cdssm_b200_intra_chunk_scan_fwd(
-                _p(A), _p(K), _p(V), _p(be), _p(local_h), _p(cum_A), BNC, C, H, D, N,
-                _dtype_code(K), _stream()), "intra_chunk_scan_fwd")
+        local_h, cum_A, A, K, V, be = _lib.host().intra_fwd(A_flat, K_flat, V_flat, beta_flat, state_dim)
         ctx.save_for_backward(A, K, V, be, local_h, cum_A)
-        ctx.state_dim = N
+        ctx.state_dim = int(state_dim)
         return local_h, cum_A
 
     @staticmethod
     def backward(ctx, grad_local_h, grad_cum_A):
         """(grad_A, grad_K, grad_V, grad_beta, None), as cdssm/ops.py:123-135 (intra_chunk_scan.cu:215-553)."""
-        A, K, V, be, local_h, cum_A = ctx.saved_tensors
-        BNC, C, H, D = K.shape
-        N = ctx.state_dim
-        glh = torch.zeros_like(local_h) if grad_local_h is None else _prep(grad_local_h.to(K.dtype), name="grad_local_h")
-        gca = torch.zeros_like(cum_A) if grad_cum_A is None else _prep(grad_cum_A.to(K.dtype), name="grad_cum_A")
-        gA, gV = torch.empty_like(A), torch.empty_like(V)
-        gK = torch.empty(BNC, C, H, D, dtype=torch.float32, device=K.device)
-        gB = torch.empty(BNC, C, H, dtype=torch.float32, device=K.device)
-        with torch.cuda.device(K.device):
-            check(_lib.lib().cdssm_b200_intra_chunk_scan_bwd(
-                _p(glh), _p(gca), _p(A), _p(K), _p(V), _p(be), _p(local_h), _p(cum_A), _p(gA), _p(gK), _p(gV), _p(gB),
-                BNC, C, H, D, N, _dtype_code(K), _stream()), "intra_chunk_scan_bwd")
-        return gA, gK.to(K.dtype), gV, gB.to(be.dtype), None
+        return _lib.host().intra_bwd(grad_local_h, grad_cum_A, *ctx.saved_tensors, ctx.state_dim) + (None,)
 
 
 class InterChunkScanFn(Function):
@@ -217,14 +132,7 @@ class InterChunkScanFn(Function):
 
     @staticmethod
     def forward(ctx, total_A: Tensor, final_local_h: Tensor, state_dim: int) -> Tensor:
-        f = _prep(final_local_h, name="final_local_h")
-        a = _prep(total_A, dtype=f.dtype, name="total_A")
-        B, NC, H, N, D = f.shape
-        out = torch.empty_like(f)
-        with torch.cuda.device(f.device):
-            check(_lib.lib().cdssm_b200_inter_chunk_scan_fwd(_p(a), _p(f), _p(out), B, NC, H, D,
-                                                             int(state_dim), _dtype_code(f), _stream()),
-                  "inter_chunk_scan_fwd")
+        out, a = _lib.host().inter_fwd(total_A, final_local_h, state_dim)
         ctx.save_for_backward(a, out)
         ctx.state_dim = int(state_dim)
         return out
@@ -232,15 +140,7 @@ class InterChunkScanFn(Function):
     @staticmethod
     def backward(ctx, grad_chunk_states):
         """(grad_total_A, grad_final_local_h, None), as cdssm/ops.py:157-163 (inter_chunk_scan.cu:89-196)."""
-        a, states = ctx.saved_tensors
-        B, NC, H, N, D = states.shape
-        g = _prep(grad_chunk_states.to(states.dtype), name="grad_chunk_states")
-        gA, gH = torch.empty_like(a), torch.empty_like(states)
-        with torch.cuda.device(states.device):
-            check(_lib.lib().cdssm_b200_inter_chunk_scan_bwd(_p(g), _p(a), _p(states), _p(gA), _p(gH), B, NC, H, D,
-                                                             ctx.state_dim, _dtype_code(states), _stream()),
-                  "inter_chunk_scan_bwd")
-        return gA, gH, None
+        return _lib.host().inter_bwd(grad_chunk_states, *ctx.saved_tensors, ctx.state_dim) + (None,)
 
 
 # The reference's correction backward kernel adds the upstream gradient of corrections[t] BEFORE it walks step t
@@ -256,38 +156,17 @@ class ExactCorrectionFn(Function):
     @staticmethod
     def forward(ctx, A_chunk: Tensor, K_chunk: Tensor, beta_chunk: Tensor, chunk_states: Tensor,
                 state_dim: int) -> Tensor:
-        K = _prep(K_chunk, name="K_chunk")
-        A = _prep(A_chunk, dtype=K.dtype, name="A_chunk")
-        be = _prep(beta_chunk, dtype=K.dtype, name="beta_chunk")
-        cs = _prep(chunk_states, dtype=K.dtype, name="chunk_states")
-        B, NC, C, H, D = K.shape
-        N = int(state_dim)
-        out = torch.empty(B, NC, C, H, N, D, dtype=K.dtype, device=K.device)
-        with torch.cuda.device(K.device):
-            check(_lib.lib().cdssm_b200_exact_correction_fwd(
-                _p(A), _p(K), _p(be), _p(cs), _p(out), B, NC, C, H, D, N, _dtype_code(K), _stream()),
-                "exact_correction_fwd")
+        out, A, K, be = _lib.host().correction_fwd(A_chunk, K_chunk, beta_chunk, chunk_states, state_dim)
         ctx.save_for_backward(A, K, be, out)
-        ctx.state_dim = N
+        ctx.state_dim = int(state_dim)
         return out
 
     @staticmethod
     def backward(ctx, grad_corrections):
         """(grad_A, grad_K, grad_beta, grad_chunk_states, None), as cdssm/ops.py:188-195
         (exact_correction.cu:169-383)."""
-        A, K, be, corr = ctx.saved_tensors
-        B, NC, C, H, D = K.shape
-        N = ctx.state_dim
-        g = _prep(grad_corrections.to(K.dtype), name="grad_corrections")
-        gA = torch.empty_like(A)
-        gK = torch.empty(B, NC, C, H, D, dtype=torch.float32, device=K.device)
-        gB = torch.empty(B, NC, C, H, dtype=torch.float32, device=K.device)
-        gS = torch.empty(B, NC, H, N, D, dtype=K.dtype, device=K.device)
-        with torch.cuda.device(K.device):
-            check(_lib.lib().cdssm_b200_exact_correction_bwd(
-                _p(g), _p(A), _p(K), _p(be), _p(corr), _p(gA), _p(gK), _p(gB), _p(gS), B, NC, C, H, D, N,
-                0 if EXACT_CORRECTION_TRUE_GRADIENT else 1, _dtype_code(K), _stream()), "exact_correction_bwd")
-        return gA, gK.to(K.dtype), gB.to(be.dtype), gS, None
+        return _lib.host().correction_bwd(grad_corrections, *ctx.saved_tensors, ctx.state_dim,
+                                          0 if EXACT_CORRECTION_TRUE_GRADIENT else 1) + (None,)
 
 
 # ------------------------------------------------------------------------------------------
