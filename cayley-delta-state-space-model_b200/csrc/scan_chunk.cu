@@ -1,6 +1,7 @@
 // The scan on tensor cores: bf16 storage, head_dim D = chunk C in {64, 128}, any even state_dim N <= 16, any head count.
 //
-// One thread block owns one chunk of one head, warp w its 32-token block w.  With g_t the coefficient that the step at
+// One thread block owns one chunk of one head; a warp (head_dim 64 and N > 4: two warps, half of the pairs each) its 32-token
+// block.  With g_t the coefficient that the step at
 // token t adds along k_t (raw keys; n_t = 1/|k_t|, c_t = beta_t n_t^2, W_t = a_0 ... a_t),
 //     local state     z_t = W_t sum_{i<=t} (g_i / W_i) k_i,   g_t = beta_t n_t v_t - c_t W_t sum_{i<t} (g_i / W_i) G[t,i]
 //     correction      r_t = W_t (r_0 - sum_{i<=t} h_i k_i),   h_t = c_t (k_t.r_0) - c_t sum_{i<t} h_i G[t,i]
@@ -9,12 +10,16 @@
 // triangular matrix I + M, M[t,i] = c_t G[t,i], for every complex pair of the head: the pairs are right-hand sides.  So
 //   - G and P are products of the chunk's tiles (mma.sync on ldmatrix fragments of the swizzled TMA tiles, lower triangle
 //     only), computed once per head and chunk whatever N is;
-//   - the two 16 x 16 diagonal blocks of a warp are inverted by substitution, a row per lane, all rows at once and
-//     independent of any state;
+//   - the two 16 x 16 diagonal blocks of 32 tokens are inverted by substitution, a row per lane, all rows at once and
+//     independent of any state (as 8 x 8 halves: seven dependent steps instead of fifteen);
 //   - what is left of the serial chain is three 16-wide products per 32 tokens, passed from warp to warp;
 //   - everything with a right-hand side (cross-block terms, read-outs, K^T g, K r_0, Q r_0) is a product with n = 8
 //     columns {pair 2q: re hi, re lo, im hi, im lo, pair 2q+1: ...}; fp32 values enter as bf16 hi + lo (16 bits), on the
 //     matrix side too, accumulation is fp32.
+// Bounded by the latency of its dependent steps at 15 warps per SM (registers), 46 % of the issue slots busy; a tensor-core
+// generation with tiles of 128 rows has no use for 16-wide products.  Measured on B200, 6144 chunks, D 64, N 16, one kernel:
+// 201 us with one warp per 32 tokens, 178 with two, 162 with the steps of their pairs side by side and the halved inverses
+// (216 chunks, local / output pass: 9.3 / 15.6 -> 6.9 / 10.7 us).
 // The division by W_i only spans a 32-token block, relative to its middle (|W ratio| of 16 tokens >= 1e-30); values cross
 // blocks relative to the block ends, where all factors are plain products.  A (block, pair) that decays further is walked
 // step by step (slow_walk).
@@ -79,7 +84,9 @@ struct Geo {
     static constexpr int kPairs = kPairs_;               // complex pairs held (>= N / 2)
     static constexpr int kTiles = (kPairs + 1) / 2;      // column tiles of two pairs
     static constexpr int kBlocks = kD / 32;              // warps: one per 32-token block
-    static constexpr int kThreads = 32 * kBlocks;
+    static constexpr int kSplit = kD == 64 && kPairs >= 4 ? 2 : 1;   // warps that share the column tiles of a 32-token block
+    static constexpr int kThreads = 32 * kBlocks * kSplit;
+    static constexpr int kOwn = kTiles / kSplit, kOwnPairs = kPairs / kSplit;   // of a warp
     static constexpr int kSlabs = kD / 64, kKs = kD / 16;
     static constexpr uint32_t kSlab = kD * 128;          // bytes of kD rows x 64 bf16 columns
     static constexpr uint32_t kTile = kSlabs * kSlab;
@@ -94,12 +101,18 @@ struct Geo {
 
 struct BlockPair {   // of one 32-token block and pair
     cplx A, R, D31;  // product of a over the block; product of its first half (the scaling's reference); D of the last token
-    int slow, pad;
 };
 
-union Scratch {   // of one warp, until the Q tile arrives in its place
-    float mt[2][16][20];                                 // the diagonal blocks of M, transposed
-    unsigned char t[32][80];                             // rows of the inverses, bf16 hi (32 B) | lo (32 B)
+struct Scratch {   // of one 32-token block, until the Q tile arrives in its place
+    union {
+        struct {                                         // of the two 16 x 16 diagonal blocks of M, 8 x 8 each
+            float tri[4][100];                           // [block, half] diagonal ones: column j, row i at 12 j + i
+            float low[2][68], inv[2][68];                // [block] the one below, the first half's inverse: 8 i + j
+        };
+        unsigned char t[32][80];                         // rows of the inverses, bf16 hi (32 B) | lo (32 B)
+    };
+    uint4 m21[2][32];                                    // for the block's other warp: M between its halves, |k|^-1
+    float nrm[32];
 };
 
 // (head_dim 128 with one pair: 74.2 KB, three blocks per SM)
@@ -118,14 +131,13 @@ struct __align__(1024) Smem {
     BlockPair bp[kPairs][G::kBlocks];
     float s_in[2 * kPairs][kD];                          // carry into the chunk
     __nv_bfloat16 r0[2 * kPairs][kD + 8];                // the same rounded (padded rows: fragment loads hit distinct banks)
-    float4 walk[G::kBlocks][32];                         // slow_walk results
-    __nv_bfloat16 y_[kPairs == 1 ? 1 : G::kBlocks][kPairs == 1 ? 1 : 32][2 * kPairs + 2];
-    // outputs of a warp on their way to one row a lane (with one pair: in place of its walk results)
-    __device__ __forceinline__ __nv_bfloat16* y(int block, int row) {
-        if constexpr (kPairs == 1) return reinterpret_cast<__nv_bfloat16*>(walk[block]) + row * 4;
-        else return y_[block][row];
+    float4 walk[G::kBlocks * G::kSplit][32];             // slow_walk results
+    // outputs of a warp on their way to one row a lane, in place of the carry (in bf16 by then)
+    __device__ __forceinline__ __nv_bfloat16* y(int token) {
+        return reinterpret_cast<__nv_bfloat16*>(s_in) + token * (2 * kPairs + 2);
     }
     uint64_t full_k, full_q;
+    int slow[G::kBlocks];                                // pairs that are walked step by step, a bit each
     int abort_flag, item, stop;
     __device__ __forceinline__ void put(int slot, int tile, int half, int lane, uint2 f) {
         if (kLanes == 32 || lane < 16) frag[slot][tile][half][lane & (kLanes - 1)] = f;
@@ -211,38 +223,48 @@ __device__ __forceinline__ uint2 rhs_frag(float x0, float x1) { return make_uint
 // The scaled unknowns need ratios of the prefix products W_t = a_0 ... a_t only, taken relative to the middle of the
 // block, D_t = W_t / W_15: lanes 0-15 hold the suffix product a_{t+1} ... a_15 = 1 / D_t, lanes 16-31 the prefix product
 // a_16 ... a_t = D_t, and neither half leaves the float range unless one half alone decays by more than 1e-30.
-__device__ __forceinline__ void scalings(cplx at, cplx vg, int tl, cplx& viw, cplx& D, BlockPair& bp) {
+// kW pairs side by side: one alone waits for its shuffles.  at, vg: a_t, v_t in; D, v_t / D out (a and v of a pair outside the
+// range: the walk reads them themselves).  Returns the pairs outside the range, a bit each.
+template <int kW>
+__device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, BlockPair (&bp)[kW]) {
     const bool lo = tl < 16;
-    cplx X = at;
+    cplx X[kW];
+#pragma unroll
+    for (int w = 0; w < kW; w++) X[w] = at[w];
 #pragma unroll
     for (int o = 1; o < 16; o <<= 1) {
-        const cplx other = cshfl(X, lo ? tl + o : tl - o);
-        if (lo ? (tl + o < 16) : (tl - o >= 16)) X = cmul(X, other);
+        const bool on = lo ? (tl + o < 16) : (tl - o >= 16);
+#pragma unroll
+        for (int w = 0; w < kW; w++) {
+            const cplx other = cshfl(X[w], lo ? tl + o : tl - o);
+            if (on) X[w] = cmul(X[w], other);
+        }
     }
-    const cplx R = cshfl(X, 0);                  // a_0 ... a_15
-    cplx E = cshfl(X, tl + 1);                   // first half: exclusive suffix = inclusive suffix of lane t + 1
-    if (tl == 15) E = {1.f, 0.f};
-    if (!lo) E = X;
-    const float m = fmaxf(fabsf(E.r), fabsf(E.i));
-    const bool in_range = m >= 1e-30f && m <= 1e30f;
-    const float sc1 = __fdividef(1.f, m);
-    const cplx En = {E.r * sc1, E.i * sc1};
-    const float q = __fdividef(sc1, En.r * En.r + En.i * En.i);
-    const cplx Einv = {En.r * q, -En.i * q};
-    D = lo ? Einv : E;
-    viw = cmul(vg, lo ? E : Einv);
-    const cplx D31 = cshfl(D, 31);
-    const float mr = fmaxf(fabsf(R.r), fabsf(R.i));
-    const bool fast = __all_sync(0xffffffffu, in_range && mr >= 1e-30f && mr <= 1e30f);
-    bp.A = cmul(D31, R);                         // both factors are plain products of a: valid for any a
-    bp.R = R;
-    bp.D31 = D31;
-    bp.slow = fast ? 0 : 1;
-    if (!fast) {   // the walk reads a and v themselves
-        viw = vg;
-        D = at;
-        bp.R = bp.D31 = {1.f, 0.f};
+    int slow = 0;
+#pragma unroll
+    for (int w = 0; w < kW; w++) {
+        const cplx R = cshfl(X[w], 0);           // a_0 ... a_15
+        cplx E = cshfl(X[w], tl + 1);            // first half: exclusive suffix = inclusive suffix of lane t + 1
+        if (tl == 15) E = {1.f, 0.f};
+        if (!lo) E = X[w];
+        const float m = fmaxf(fabsf(E.r), fabsf(E.i));
+        const bool in_range = m >= 1e-30f && m <= 1e30f;
+        const float sc1 = __fdividef(1.f, m);
+        const cplx En = {E.r * sc1, E.i * sc1};
+        const float q = __fdividef(sc1, En.r * En.r + En.i * En.i);
+        const cplx Einv = {En.r * q, -En.i * q};
+        const cplx D = lo ? Einv : E, v = cmul(vg[w], lo ? E : Einv);
+        const cplx D31 = cshfl(D, 31);
+        const float mr = fmaxf(fabsf(R.r), fabsf(R.i));
+        const bool fast = __all_sync(0xffffffffu, in_range && mr >= 1e-30f && mr <= 1e30f);
+        bp[w].A = cmul(D31, R);                  // both factors are plain products of a: valid for any a
+        bp[w].R = fast ? R : cplx{1.f, 0.f};
+        bp[w].D31 = fast ? D31 : cplx{1.f, 0.f};
+        if (!fast) slow |= 1 << w;
+        at[w] = fast ? D : at[w];
+        vg[w] = fast ? v : vg[w];
     }
+    return slow;
 }
 
 // Step-by-step walk of pair p over this warp's block, for decays the scaled form cannot hold: state columns over the
@@ -250,7 +272,7 @@ __device__ __forceinline__ void scalings(cplx at, cplx vg, int tl, cplx& viw, cp
 // v_t), later with it (walk[t] = {q_t.z_t, W_{t-1} from the block start}; no sums on the way of the state any more).  The
 // incoming state is rebuilt from the fragments the earlier blocks published for this one.
 template <int kD, int kPairs, Mode kMode, bool kReadout>
-__device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I, int tl) {
+__device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I, int W, int tl) {
     using G = Geo<kD, kPairs>;
     constexpr int kCols = kD / 32;
     auto column = [&](const uint8_t* tile, int row, int c) {
@@ -289,7 +311,7 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
         for (int i = 0; i < kCols; i++) k[i] = column(sm.k, row, tl + 32 * i);
         cplx gt = {vg.x, vg.y};               // read-out: g_t as the first walk left it
         if (!kReadout) {
-            const float be = sm.beta[row], n = sm.walk[I][t].x;
+            const float be = sm.beta[row], n = sm.walk[W][t].x;
             float ur = 0.f, ui = 0.f;
 #pragma unroll
             for (int i = 0; i < kCols; i++) {
@@ -334,7 +356,7 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
     if (tl == (kReadout ? 0 : 31)) V = {1.f, 0.f};
     if (!kReadout) own = cmul(V, own);
     __syncwarp();
-    sm.walk[I][tl] = make_float4(own.r, own.i, V.r, V.i);
+    sm.walk[W][tl] = make_float4(own.r, own.i, V.r, V.i);
     __syncwarp();
 }
 
@@ -347,19 +369,22 @@ __device__ __forceinline__ float next_im(cplx g, float sr, float si, float l) {
     return __fadd_rn(__fmaf_rn(g.r, si, __fmul_rn(g.i, sr)), l);
 }
 
-// resident blocks per SM the registers are cut for (more blocks spill: N 16, head_dim 64, 5 / 7 / 8 blocks: 279 / 308 / 328 us)
+// resident blocks per SM the registers are cut for (one more spills: N 16, head_dim 64, 4 / 5 blocks: 178 / 203 us)
 template <int kD, int kPairs>
-constexpr int kMinBlocks = kD == 128 ? (kPairs == 1 ? 3 : 2) : (kPairs <= 2 ? 6 : 5);
+constexpr int kMinBlocks = kD == 128 ? (kPairs == 1 ? 3 : 2) : (kPairs <= 2 ? 6 : 4);
 
 template <int kD, int kPairs, Mode kMode>
 __global__ void __launch_bounds__(Geo<kD, kPairs>::kThreads, kMinBlocks<kD, kPairs>)
 scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const Args a) {
     using G = Geo<kD, kPairs>;
-    constexpr int kBlocks = G::kBlocks, kTiles = G::kTiles, kKs = G::kKs;
+    constexpr int kBlocks = G::kBlocks, kKs = G::kKs;
     constexpr bool kOut = kMode != kLocal, kNeedEnd = kMode != kOutput;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem<kD, kPairs, kMode>& sm = *reinterpret_cast<Smem<kD, kPairs, kMode>*>(smem_raw);
-    const int tid = threadIdx.x, I = tid >> 5, tl = tid & 31, g = tl >> 2, t4 = tl & 3;
+    constexpr int kSplit = G::kSplit, kOwn = G::kOwn;
+    // warp W: 32-token block I, column tiles S * kOwn ... (the warps of a block meet at the tiles and the inverses only)
+    const int tid = threadIdx.x, W = tid >> 5, I = W % kBlocks, S = W / kBlocks, tl = tid & 31, g = tl >> 2, t4 = tl & 3;
+    const int tok = 32 * I + tl;
     const int H = a.H, N = a.N, NP = N >> 1, L = a.L;
 
     if (kMode == kFused) grid_dependency_wait();   // (the records kernel clears the ticket counter)
@@ -395,14 +420,14 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     auto flag_set = [&]() {
         int v;
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(carry_flag) : "memory");
-        return ((v >> I) & 1) != 0;
+        return ((v >> W) & 1) != 0;
     };
     auto load_carry = [&](const float* src) {
         const int col = 32 * I + 4 * (tl & 7);
 #pragma unroll
-        for (int n0 = 0; n0 < 2 * kPairs; n0 += 4) {
-            const int n = n0 + (tl >> 3);
-            if (n < 2 * kPairs) {
+        for (int n0 = 0; n0 < 2 * G::kOwnPairs; n0 += 4) {
+            const int n = 2 * G::kOwnPairs * S + n0 + (tl >> 3);
+            if (n0 + (tl >> 3) < 2 * G::kOwnPairs) {
                 const bool on = src != nullptr && n < N;
                 cp_async16(&sm.s_in[n][col], on ? src + (size_t)n * kD + col : a.ws_state, on);
             }
@@ -416,6 +441,27 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (c == 0) load_carry(a.h0 ? a.h0 + ((size_t)b * H + hd) * N * kD : nullptr);
         else if ((have_carry = __all_sync(0xffffffffu, flag_set()))) load_carry(carry_src);
     }
+    // the token's dynamics, parked where the results will go (padding pairs: identity)
+    const bool first_warp = kSplit == 1 || S == 0, last_warp = kSplit == 1 || S == kSplit - 1;
+    auto load_records = [&]() {
+        if (first_warp) cp_async_small<4>(&sm.beta[tok], a.rec_g + unit * kD + tok);
+        if (last_warp) {
+            const float2* ra = a.rec_a + unit * (size_t)NP * kD + tok;
+            const uint32_t* rv = a.rec_v + unit * (size_t)NP * kD + tok;
+#pragma unroll
+            for (int p = 0; p < kPairs; p++) {
+                if (p < NP) {
+                    cp_async_small<8>(&sm.dd[p][tok], ra + p * kD);
+                    cp_async_small<4>(&sm.viw[p][tok], rv + p * kD);
+                } else {
+                    sm.dd[p][tok] = make_float2(1.f, 0.f);
+                    sm.viw[p][tok] = make_float2(0.f, 0.f);
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    if (kMode != kLocal) load_records();
     const bool k_here = mbar_wait_suspend(&sm.full_k, 0, &sm.abort_flag, a.wait_ns);
     if (!__syncthreads_and(k_here)) {
         if (tid == 0) atomicCAS(a.status, 0, 201);
@@ -429,97 +475,159 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     Split T11, T22, M21;
     Split M[kBlocks > 1 ? kBlocks - 1 : 1][2][2];
     {
-        float acc[2][4][4];
-        gram_block<kD, kPairs, true>(acc, kt, 32 * I, kt, 32 * I, tl, true);
-        float kk[4];
-        diagonal_of(acc[0][0], acc[0][1], tl, kk[0], kk[1]);
-        diagonal_of(acc[1][2], acc[1][3], tl, kk[2], kk[3]);
+        float acc[2][4][4], kk[4];
+        if (first_warp) {
+            gram_block<kD, kPairs, true>(acc, kt, 32 * I, kt, 32 * I, tl, true);
+            diagonal_of(acc[0][0], acc[0][1], tl, kk[0], kk[1]);
+            diagonal_of(acc[1][2], acc[1][3], tl, kk[2], kk[3]);
+        }
         // the token's dynamics, from the kernel before this one (its launch let this one start early; no __ldg here: loads
         // that claim the data constant may be moved above the wait)
         if (kMode == kLocal) grid_dependency_wait();
         grid_launch_dependents();
-        {
-            const uint32_t gg = __ldcg(a.rec_g + unit * kD + tid);
-            const float2* ra = a.rec_a + unit * (size_t)NP * kD + tid;
-            const uint32_t* rv = a.rec_v + unit * (size_t)NP * kD + tid;
-            float2 at[kPairs];
-            uint32_t vg[kPairs];
-#pragma unroll
-            for (int p = 0; p < kPairs; p++) {
-                at[p] = p < NP ? __ldcg(ra + p * kD) : make_float2(1.f, 0.f);
-                vg[p] = p < NP ? __ldcg(rv + p * kD) : 0u;
-            }
-            sm.beta[tid] = bits_lo(gg);
-            sm.sel[tid] = bits_hi(gg);
-#pragma unroll
-            for (int p = 0; p < kPairs; p++) {   // parked where the results will go
-                sm.dd[p][tid] = at[p];
-                sm.viw[p][tid] = make_float2(bits_lo(vg[p]), bits_hi(vg[p]));
-            }
-#pragma unroll 1
-            for (int p = 0; p < kPairs; p++) {
-                const float2 x = sm.dd[p][tid], y = sm.viw[p][tid];
-                cplx viw, D;
-                BlockPair bp;
-                scalings({x.x, x.y}, {y.x, y.y}, tl, viw, D, bp);
-                sm.viw[p][tid] = make_float2(viw.r, viw.i);
-                sm.dd[p][tid] = make_float2(D.r, D.i);
-                if (tl == 0) sm.bp[p][I] = bp;
-            }
+        if (kMode == kLocal) load_records();
+        cp_async_wait_all();
+        if (first_warp) {
+            const uint32_t gg = __float_as_uint(sm.beta[tok]);
+            sm.beta[tok] = bits_lo(gg);
+            sm.sel[tok] = bits_hi(gg);
             __syncwarp();
         }
+        if (last_warp) {
+            constexpr int kW = kPairs < 4 ? kPairs : 4;
+            int slow = 0;
+#pragma unroll 1
+            for (int p0 = 0; p0 < kPairs; p0 += kW) {
+                cplx at[kW], vg[kW];
+                BlockPair bp[kW];
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const float be = sm.beta[32 * I + 8 * r + g];
-            nrm[r] = rsqrtf(kk[r] + kEps);
-            bn[r] = be * nrm[r];
-            cc[r] = bn[r] * nrm[r];
+                for (int w = 0; w < kW; w++) {
+                    const float2 x = sm.dd[p0 + w][tok];
+                    const uint32_t y = __float_as_uint(sm.viw[p0 + w][tok].x);
+                    at[w] = {x.x, x.y};
+                    vg[w] = {bits_lo(y), bits_hi(y)};
+                }
+                slow |= scalings<kW>(at, vg, tl, bp) << p0;
+#pragma unroll
+                for (int w = 0; w < kW; w++) {
+                    sm.viw[p0 + w][tok] = make_float2(vg[w].r, vg[w].i);
+                    sm.dd[p0 + w][tok] = make_float2(at[w].r, at[w].i);
+                    if (tl == 0) sm.bp[p0 + w][I] = bp[w];
+                }
+            }
+            if (tl == 0) sm.slow[I] = slow;
+            __syncwarp();
         }
-        // strictly lower part of the two diagonal 16 x 16 blocks of M, transposed: mt[block][column][row]
-        auto& mt = sm.scr[I].mt;
+        if (first_warp) {
 #pragma unroll
-        for (int m = 0; m < 2; m++)
+            for (int r = 0; r < 4; r++) {
+                const float be = sm.beta[32 * I + 8 * r + g];
+                nrm[r] = rsqrtf(kk[r] + kEps);
+                bn[r] = be * nrm[r];
+                cc[r] = bn[r] * nrm[r];
+            }
+            // M's diagonal 16 x 16 blocks, as 8 x 8: the strictly lower part of two, and the one below
+            auto& sc = sm.scr[I];
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int col = 2 * t4 + e;
+                    sc.tri[2 * m][12 * col + g] = g > col ? cc[2 * m] * acc[m][2 * m][e] : 0.f;
+                    sc.tri[2 * m + 1][12 * col + g] = g > col ? cc[2 * m + 1] * acc[m][2 * m + 1][2 + e] : 0.f;
+                }
+                *reinterpret_cast<float2*>(&sc.low[m][8 * g + 2 * t4]) =
+                    make_float2(cc[2 * m + 1] * acc[m][2 * m][2], cc[2 * m + 1] * acc[m][2 * m][3]);
+            }
 #pragma unroll
             for (int n = 0; n < 2; n++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int row = g + 8 * (e >> 1), col = 8 * n + 2 * t4 + (e & 1);
-                    mt[m][col][row] = row > col ? cc[2 * m + (e >> 1)] * acc[m][2 * m + n][e] : 0.f;
+                for (int e = 0; e < 4; e++) acc[1][n][e] *= cc[2 + (e >> 1)];
+            M21 = split(acc[1][0], acc[1][1]);
+            if (kSplit > 1) {
+                sm.scr[I].m21[0][tl] = make_uint4(M21.hi[0], M21.hi[1], M21.hi[2], M21.hi[3]);
+                sm.scr[I].m21[1][tl] = make_uint4(M21.lo[0], M21.lo[1], M21.lo[2], M21.lo[3]);
+                if (t4 == 0) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) sm.scr[I].nrm[8 * r + g] = nrm[r];
                 }
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) acc[1][n][e] *= cc[2 + (e >> 1)];
-        M21 = split(acc[1][0], acc[1][1]);
-        __syncwarp();
-        // row r of the inverse of I + M (lanes 0-15: first block, 16-31: second): T[r][j] = - sum_{i>j} T[r][i] M[i][j]
-        const int r = tl & 15, blk = tl >> 4;
-        float2 T2[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) T2[j] = make_float2(2 * j == r ? 1.f : 0.f, 2 * j + 1 == r ? 1.f : 0.f);
-#pragma unroll
-        for (int j = 14; j >= 0; j--) {
-            float2 s = make_float2(0.f, 0.f), s2 = s;
-#pragma unroll
-            for (int i4 = (j + 1) / 4; i4 < 4; i4++) {
-                const float4 mm = *reinterpret_cast<const float4*>(&mt[blk][j][4 * i4]);
-                s = __ffma2_rn(T2[2 * i4], make_float2(mm.x, mm.y), s);
-                s2 = __ffma2_rn(T2[2 * i4 + 1], make_float2(mm.z, mm.w), s2);
             }
-            const float sum = (s.x + s.y) + (s2.x + s2.y);
-            if (j & 1) T2[j >> 1].y -= sum;
-            else T2[j >> 1].x -= sum;
-        }
-        __syncwarp();
-        uint32_t* row = reinterpret_cast<uint32_t*>(sm.scr[I].t[tl]);
+            __syncwarp();
+            // A lane has a row of the inverse.  The halves first, T[r][j] = - sum_{i>j} T[r][i] M[i][j]: seven dependent steps
+            // instead of the fifteen of the whole block; then the lower rows' left part, - T_2 M_21 T_1.
+            const int r = tl & 7, half = (tl >> 3) & 1, blk = tl >> 4;
+            float2 T2[4], U[4], X[4];
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) {
-            *reinterpret_cast<uint4*>(row + j) = make_uint4(pair_hi(T2[j].x, T2[j].y), pair_hi(T2[j + 1].x, T2[j + 1].y),
-                                                            pair_hi(T2[j + 2].x, T2[j + 2].y), pair_hi(T2[j + 3].x, T2[j + 3].y));
-            *reinterpret_cast<uint4*>(row + 8 + j) = make_uint4(pair_lo(T2[j].x, T2[j].y), pair_lo(T2[j + 1].x, T2[j + 1].y),
-                                                                pair_lo(T2[j + 2].x, T2[j + 2].y), pair_lo(T2[j + 3].x, T2[j + 3].y));
+            for (int j = 0; j < 4; j++) {
+                T2[j] = make_float2(2 * j == r ? 1.f : 0.f, 2 * j + 1 == r ? 1.f : 0.f);
+                U[j] = X[j] = make_float2(0.f, 0.f);
+            }
+            const float* tri = sc.tri[2 * blk + half];
+#pragma unroll
+            for (int j = 6; j >= 0; j--) {
+                float2 sum = make_float2(0.f, 0.f);
+                const float4 m1 = *reinterpret_cast<const float4*>(tri + 12 * j + 4);
+                if (j < 6) sum = __ffma2_rn(T2[3], make_float2(m1.z, m1.w), sum);
+                else sum.y = T2[3].y * m1.w;
+                if (j < 5) sum = __ffma2_rn(T2[2], make_float2(m1.x, m1.y), sum);
+                if (j < 3) {
+                    const float4 m0 = *reinterpret_cast<const float4*>(tri + 12 * j);
+                    sum = __ffma2_rn(T2[1], make_float2(m0.z, m0.w), sum);
+                    if (j < 1) sum = __ffma2_rn(T2[0], make_float2(m0.x, m0.y), sum);
+                }
+                if (j & 1) T2[j >> 1].y -= sum.x + sum.y;
+                else T2[j >> 1].x -= sum.x + sum.y;
+            }
+            if (half == 0) {
+                float4* inv = reinterpret_cast<float4*>(&sc.inv[blk][8 * r]);
+                inv[0] = make_float4(T2[0].x, T2[0].y, T2[1].x, T2[1].y);
+                inv[1] = make_float4(T2[2].x, T2[2].y, T2[3].x, T2[3].y);
+            }
+            auto add_rows = [&](float2 (&to)[4], const float2 (&by)[4], const float* rows) {   // to += by . rows (8 x 8)
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float4 r0 = *reinterpret_cast<const float4*>(rows + 8 * i), r1 = *reinterpret_cast<const float4*>(rows + 8 * i + 4);
+                    const float f = (i & 1) ? by[i >> 1].y : by[i >> 1].x;
+                    const float2 ff = make_float2(f, f);
+                    to[0] = __ffma2_rn(ff, make_float2(r0.x, r0.y), to[0]);
+                    to[1] = __ffma2_rn(ff, make_float2(r0.z, r0.w), to[1]);
+                    to[2] = __ffma2_rn(ff, make_float2(r1.x, r1.y), to[2]);
+                    to[3] = __ffma2_rn(ff, make_float2(r1.z, r1.w), to[3]);
+                }
+            };
+            add_rows(U, T2, sc.low[blk]);
+            __syncwarp();
+            add_rows(X, U, sc.inv[blk]);
+            float2 R[8];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                R[j] = half == 0 ? T2[j] : make_float2(-X[j].x, -X[j].y);
+                R[4 + j] = half == 0 ? make_float2(0.f, 0.f) : T2[j];
+            }
+            __syncwarp();
+            uint32_t* row = reinterpret_cast<uint32_t*>(sm.scr[I].t[tl]);
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                *reinterpret_cast<uint4*>(row + j) = make_uint4(pair_hi(R[j].x, R[j].y), pair_hi(R[j + 1].x, R[j + 1].y),
+                                                                pair_hi(R[j + 2].x, R[j + 2].y), pair_hi(R[j + 3].x, R[j + 3].y));
+                *reinterpret_cast<uint4*>(row + 8 + j) = make_uint4(pair_lo(R[j].x, R[j].y), pair_lo(R[j + 1].x, R[j + 1].y),
+                                                                    pair_lo(R[j + 2].x, R[j + 2].y), pair_lo(R[j + 3].x, R[j + 3].y));
+            }
+            __syncwarp();
         }
-        __syncwarp();
+        if (kSplit > 1) {
+            __syncthreads();
+            if (!first_warp) {
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    nrm[r] = sm.scr[I].nrm[8 * r + g];
+                    bn[r] = sm.beta[32 * I + 8 * r + g] * nrm[r];
+                    cc[r] = bn[r] * nrm[r];
+                }
+                const uint4 hi = sm.scr[I].m21[0][tl], lo = sm.scr[I].m21[1][tl];
+                M21 = {{hi.x, hi.y, hi.z, hi.w}, {lo.x, lo.y, lo.z, lo.w}};
+            }
+        }
         const uint32_t ts = smem_u32(sm.scr[I].t) + (uint32_t)((tl & 7) + ((tl >> 3) & 1) * 8) * 80u + (uint32_t)(tl >> 4) * 16u;
         ldsm_x4(ts, T11.hi);
         ldsm_x4(ts + 32, T11.lo);
@@ -552,6 +660,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 M[J][m][1] = split(acc[m][2], acc[m][3]);
             }
         }
+    auto tile = [&](int q) { return S * kOwn + q; };
     // x <- (I + M_own)^-1 rhs for one column tile; f: the solution as B fragments of the two 16-token halves
     auto solve = [&](float (&x)[4], uint2 (&f)[2]) {
         float d[4] = {0.f, 0.f, 0.f, 0.f};
@@ -570,9 +679,9 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         f[1] = rhs_frag(x[2], x[3]);
     };
     // sum over the earlier blocks of M times their published fragments, subtracted from the right-hand sides
-    auto subtract_earlier = [&](int J, int slot, float (&x)[kTiles][4]) {
+    auto subtract_earlier = [&](int J, int slot, float (&x)[kOwn][4]) {
 #pragma unroll
-        for (int q = 0; q < kTiles; q++) {
+        for (int q = 0; q < kOwn; q++) {
             float d[2][4];
 #pragma unroll
             for (int m = 0; m < 2; m++)
@@ -580,7 +689,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 for (int e = 0; e < 4; e++) d[m][e] = 0.f;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const uint2 f = sm.get(slot, q, h, tl);
+                const uint2 f = sm.get(slot, tile(q), h, tl);
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
 #pragma unroll
@@ -597,18 +706,19 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     };
     const int comp = t4 & 1;
     // pair of the lane's component / of the fragment column in tile q (with one pair, the second half repeats it unused)
-    auto pair_of = [&](int q) { return kPairs == 1 ? 0 : 2 * q + (t4 >> 1); };
-    auto column_pair = [&](int q) { return kPairs == 1 ? 0 : 2 * q + (g >> 2); };
+    auto pair_of = [&](int q) { return kPairs == 1 ? 0 : 2 * tile(q) + (t4 >> 1); };
+    auto column_pair = [&](int q) { return kPairs == 1 ? 0 : 2 * tile(q) + (g >> 2); };
     constexpr int kPerTile = kPairs == 1 ? 1 : 2;
     // complex factor times the lane's component; `other` is the other component of the same value
     auto rotate = [&](cplx f, float own, float other) { return f.r * own + (comp ? f.i : -f.i) * other; };
 
+    const int slow = sm.slow[I] & (((1 << G::kOwnPairs) - 1) << (G::kOwnPairs * S));   // of this warp's pairs
     // ---- g: the chain over the blocks of the chunk
-    uint2 gf[kTiles][2];                       // own block's g / D
-    float gx[kTiles][4];
+    uint2 gf[kOwn][2];                       // own block's g / D
+    float gx[kOwn][4];
     {
 #pragma unroll
-        for (int q = 0; q < kTiles; q++)
+        for (int q = 0; q < kOwn; q++)
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const float2 e = sm.viw[pair_of(q)][32 * I + 8 * r + g];
@@ -617,40 +727,52 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
         for (int J = 0; J < kBlocks - 1; J++)
             if (J < I) {
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + J), "r"(32 * (kBlocks - J)) : "memory");
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + S * (kBlocks - 1) + J), "r"(32 * (kBlocks - J)) : "memory");
                 subtract_earlier(J, G::slot_g(J, I), gx);
             }
 #pragma unroll
-        for (int q = 0; q < kTiles; q++) solve(gx[q], gf[q]);
+        for (int q = 0; q < kOwn; q++) solve(gx[q], gf[q]);
+        float w[kOwn][4];                      // g carried to the block end
 #pragma unroll
-        for (int q = 0; q < kTiles; q++) {
-            const int p = pair_of(q);
-            float w[4];                        // g carried to the block end
-            const cplx d31 = sm.bp[p][I].D31;
+        for (int q = 0; q < kOwn; q++) {
+            const cplx d31 = sm.bp[pair_of(q)][I].D31;
 #pragma unroll
-            for (int r = 0; r < 4; r++) w[r] = rotate(d31, gx[q][r], __shfl_xor_sync(0xffffffffu, gx[q][r], 1));
+            for (int r = 0; r < 4; r++) w[q][r] = rotate(d31, gx[q][r], __shfl_xor_sync(0xffffffffu, gx[q][r], 1));
+        }
+        if (slow != 0) {                       // decays beyond the scaled form: step by step
+            if (t4 == 0) {
+#pragma unroll
+                for (int r = 0; r < 4; r++) sm.walk[W][8 * r + g].x = nrm[r];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < kOwn; q++)
 #pragma unroll 1
-            for (int s = 0; s < kPerTile; s++)   // decays beyond the scaled form: step by step
-                if (sm.bp[2 * q + s][I].slow) {
-                    if (t4 == 0) {
+                for (int s = 0; s < kPerTile; s++)
+                    if ((slow >> (2 * tile(q) + s)) & 1) {
+                        slow_walk<kD, kPairs, kMode, false>(sm, 2 * tile(q) + s, I, W, tl);
+                        if (kPairs == 1 || (t4 >> 1) == s) {
 #pragma unroll
-                        for (int r = 0; r < 4; r++) sm.walk[I][8 * r + g].x = nrm[r];
-                    }
-                    __syncwarp();
-                    slow_walk<kD, kPairs, kMode, false>(sm, 2 * q + s, I, tl);
-                    if (kPairs == 1 || (t4 >> 1) == s) {
-#pragma unroll
-                        for (int r = 0; r < 4; r++) {
-                            const float4 x = sm.walk[I][8 * r + g];
-                            w[r] = comp ? x.y : x.x;
+                            for (int r = 0; r < 4; r++) {
+                                const float4 x = sm.walk[W][8 * r + g];
+                                w[q][r] = comp ? x.y : x.x;
+                            }
                         }
+                        __syncwarp();
+                        if (t4 == 0) {
+#pragma unroll
+                            for (int r = 0; r < 4; r++) sm.walk[W][8 * r + g].x = nrm[r];
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
-                }
+        }
+        // to every later block's start (times its reference product), and to the chunk end
+#pragma unroll
+        for (int q = 0; q < kOwn; q++) {
+            const int p = pair_of(q);
             float wo[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) wo[r] = __shfl_xor_sync(0xffffffffu, w[r], 1);
-            // to every later block's start (times its reference product), and to the chunk end
+            for (int r = 0; r < 4; r++) wo[r] = __shfl_xor_sync(0xffffffffu, w[q][r], 1);
             cplx f = {1.f, 0.f};
 #pragma unroll
             for (int to = 1; to <= kBlocks; to++) {
@@ -659,24 +781,23 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     if (!end || kNeedEnd || a.tail_state) {
                         const cplx ff = end ? f : cmul(f, sm.bp[p][to < kBlocks ? to : 0].R);
                         const int slot = end ? G::slot_end(I) : G::slot_g(I, to);
-                        sm.put(slot, q, 0, tl, rhs_frag(rotate(ff, w[0], wo[0]), rotate(ff, w[1], wo[1])));
-                        sm.put(slot, q, 1, tl, rhs_frag(rotate(ff, w[2], wo[2]), rotate(ff, w[3], wo[3])));
+                        sm.put(slot, tile(q), 0, tl, rhs_frag(rotate(ff, w[q][0], wo[0]), rotate(ff, w[q][1], wo[1])));
+                        sm.put(slot, tile(q), 1, tl, rhs_frag(rotate(ff, w[q][2], wo[2]), rotate(ff, w[q][3], wo[3])));
                     }
                     if (!end) f = cmul(f, sm.bp[p][to < kBlocks ? to : 0].A);
                 }
             }
         }
-        if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + I), "r"(32 * (kBlocks - I)) : "memory");
-        // (a slow pair takes no part in the scaled read-out)
+        if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + S * (kBlocks - 1) + I), "r"(32 * (kBlocks - I)) : "memory");
+        if (slow != 0) {                       // a slow pair takes no part in the scaled read-out
 #pragma unroll
-        for (int q = 0; q < kTiles; q++)
-            if (sm.bp[2 * q][I].slow | sm.bp[2 * q + kPerTile - 1][I].slow) {
-                const bool mine = sm.bp[pair_of(q)][I].slow;                   // rows: this lane's pair
-                const bool col = sm.bp[column_pair(q)][I].slow;                // fragment: this lane's column
+            for (int q = 0; q < kOwn; q++) {
+                const bool mine = (slow >> pair_of(q)) & 1, col = (slow >> column_pair(q)) & 1;   // this lane's row, fragment column
 #pragma unroll
                 for (int r = 0; r < 4; r++) gx[q][r] = mine ? 0.f : gx[q][r];
                 if (col) gf[q][0] = gf[q][1] = make_uint2(0u, 0u);
             }
+        }
     }
     __syncthreads();
 
@@ -690,7 +811,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int J = 0; J < kBlocks; J++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const uint2 f = sm.get(slot0 + J, q, h, tl);
+                const uint2 f = sm.get(slot0 + J, tile(q), h, tl);
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
                     uint32_t ka[4];
@@ -708,9 +829,9 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 
     // ---- z at the chunk end; the carry
     if (kNeedEnd) {
-        float z[kTiles][2][4];
+        float z[kOwn][2][4];
 #pragma unroll
-        for (int q = 0; q < kTiles; q++) k_transposed(G::slot_end(0), q, z[q]);
+        for (int q = 0; q < kOwn; q++) k_transposed(G::slot_end(0), q, z[q]);
         if (kMode == kFused) {
             if (!have_carry) {
                 const unsigned long long t0 = global_ns();
@@ -726,7 +847,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         }
         const bool whole = Lc == kD;           // the reference's zero padding wipes state and decay (ssd.py:60-67)
 #pragma unroll
-        for (int q = 0; q < kTiles; q++) {
+        for (int q = 0; q < kOwn; q++) {
             const int p = pair_of(q);
             if (p < NP && (kPairs > 1 || t4 < 2)) {
                 cplx gam = chunk_decay(p);
@@ -755,7 +876,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (c + 1 < a.NC && have_carry) {      // release this warp's columns to the next chunk
             __syncwarp();
             int* next = reinterpret_cast<int*>(a.ws_gamma + (unit + H) * (size_t)N);
-            if (tl == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(next), "r"(1 << I) : "memory");
+            if (tl == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(next), "r"(1 << W) : "memory");
         }
     } else {
         cp_async_wait_all();
@@ -763,7 +884,10 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     }
     // r_0: the carry rounded to bf16
 #pragma unroll
-    for (int n = 0; n < 2 * kPairs; n++) sm.r0[n][32 * I + tl] = __float2bfloat16_rn(sm.s_in[n][32 * I + tl]);
+    for (int i = 0; i < 2 * G::kOwnPairs; i++) {
+        const int n = 2 * G::kOwnPairs * S + i;
+        sm.r0[n][tok] = __float2bfloat16_rn(sm.s_in[n][tok]);
+    }
     const bool q_here = mbar_wait_suspend(&sm.full_q, 0, &sm.abort_flag, a.wait_ns);
     if (!__syncthreads_and(q_here && have_carry)) {
         if (tid == 0) atomicCAS(a.status, 0, 202);
@@ -777,11 +901,11 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         return (g & 1) || (kPairs == 1 && g >= 4) ? make_uint2(0u, 0u) : make_uint2(s[0], s[4]);
     };
     // ---- h: right-hand sides c_t k_t.r_0, the same chain
-    float hx[kTiles][4];
+    float hx[kOwn][4];
     {
-        float d[kTiles][2][4];
+        float d[kOwn][2][4];
 #pragma unroll
-        for (int q = 0; q < kTiles; q++)
+        for (int q = 0; q < kOwn; q++)
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -792,43 +916,43 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             ldsm_x4(row_frag<G::kSlab>(kt, 32 * I, ks, tl), ka[0]);
             ldsm_x4(row_frag<G::kSlab>(kt, 32 * I + 16, ks, tl), ka[1]);
 #pragma unroll
-            for (int q = 0; q < kTiles; q++) {
+            for (int q = 0; q < kOwn; q++) {
                 const uint2 f = r0_frag(q, ks);
                 mma_bf16_m16n8k16(d[q][0], ka[0], f.x, f.y);
                 mma_bf16_m16n8k16(d[q][1], ka[1], f.x, f.y);
             }
         }
 #pragma unroll
-        for (int q = 0; q < kTiles; q++)
+        for (int q = 0; q < kOwn; q++)
 #pragma unroll
             for (int r = 0; r < 4; r++) hx[q][r] = cc[r] * d[q][r >> 1][2 * (r & 1)];
 #pragma unroll
         for (int J = 0; J < kBlocks - 1; J++)
             if (J < I) {
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + J), "r"(32 * (kBlocks - J)) : "memory");
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + S * (kBlocks - 1) + J), "r"(32 * (kBlocks - J)) : "memory");
                 subtract_earlier(J, G::slot_h(J), hx);
             }
 #pragma unroll
-        for (int q = 0; q < kTiles; q++) {
+        for (int q = 0; q < kOwn; q++) {
             uint2 f[2];
             solve(hx[q], f);
-            sm.put(G::slot_h(I), q, 0, tl, f[0]);
-            sm.put(G::slot_h(I), q, 1, tl, f[1]);
+            sm.put(G::slot_h(I), tile(q), 0, tl, f[0]);
+            sm.put(G::slot_h(I), tile(q), 1, tl, f[1]);
         }
-        if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + I), "r"(32 * (kBlocks - I)) : "memory");
+        if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + S * (kBlocks - 1) + I), "r"(32 * (kBlocks - I)) : "memory");
         __syncwarp();
     }
 
     // ---- |q|^-1 and q.r_0
-    float mq[4], rho[kTiles][4];
+    float mq[4], rho[kOwn][4];
     {
-        float qd[2][2][4], d[kTiles][2][4];
+        float qd[2][2][4], d[kOwn][2][4];
 #pragma unroll
         for (int m = 0; m < 2; m++)
 #pragma unroll
             for (int e = 0; e < 4; e++) qd[m][0][e] = qd[m][1][e] = 0.f;
 #pragma unroll
-        for (int q = 0; q < kTiles; q++)
+        for (int q = 0; q < kOwn; q++)
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -844,7 +968,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 mma_bf16_m16n8k16(qd[m][1], qa[m], qa[m][1], qa[m][3]);
             }
 #pragma unroll
-            for (int q = 0; q < kTiles; q++) {
+            for (int q = 0; q < kOwn; q++) {
                 const uint2 f = r0_frag(q, ks);
                 mma_bf16_m16n8k16(d[q][0], qa[0], f.x, f.y);
                 mma_bf16_m16n8k16(d[q][1], qa[1], f.x, f.y);
@@ -855,14 +979,14 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
         for (int r = 0; r < 4; r++) mq[r] = rsqrtf(mq[r] + kEps);
 #pragma unroll
-        for (int q = 0; q < kTiles; q++)
+        for (int q = 0; q < kOwn; q++)
 #pragma unroll
             for (int r = 0; r < 4; r++) rho[q][r] = d[q][r >> 1][2 * (r & 1)];
     }
     // ---- read-out: P against the block itself and the earlier ones
-    float oz[kTiles][4], pd[4];
+    float oz[kOwn][4], pd[4];
 #pragma unroll
-    for (int q = 0; q < kTiles; q++)
+    for (int q = 0; q < kOwn; q++)
 #pragma unroll
         for (int r = 0; r < 4; r++) oz[q][r] = 0.f;
 #pragma unroll 1
@@ -885,9 +1009,9 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int h = 0; h < 2; h++) {
             const Split p0 = split(acc[0][2 * h], acc[0][2 * h + 1]), p1 = split(acc[1][2 * h], acc[1][2 * h + 1]);
 #pragma unroll
-            for (int q = 0; q < kTiles; q++) {
-                const uint2 fg = diag ? gf[q][h] : sm.get(G::slot_g(J, I), q, h, tl);
-                const uint2 fh = sm.get(G::slot_h(J), q, h, tl);
+            for (int q = 0; q < kOwn; q++) {
+                const uint2 fg = diag ? gf[q][h] : sm.get(G::slot_g(J, I), tile(q), h, tl);
+                const uint2 fh = sm.get(G::slot_h(J), tile(q), h, tl);
                 float dz[2][4], dh[2][4];
 #pragma unroll
                 for (int m = 0; m < 2; m++)
@@ -907,73 +1031,86 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             }
         }
     }
-#pragma unroll
-    for (int q = 0; q < kTiles; q++) {
-        const int p = pair_of(q);
-        // W_{t-1} = D_{t-1} F, F = (decay up to the block) R; the first token of a block takes the decay itself
+    // W_{t-1} = D_{t-1} F, F = (decay up to the block) R; the first token of a block takes the decay itself
+    auto decay_before = [&](int p) {
         cplx pre = {1.f, 0.f};
 #pragma unroll
         for (int J = 0; J < kBlocks - 1; J++)
             if (J < I) pre = cmul(pre, sm.bp[p][J].A);
-        const cplx F = cmul(pre, sm.bp[p][I].R);
-        float y[4], ho[4];
+        return pre;
+    };
+#pragma unroll
+    for (int q = 0; q < kOwn; q++) {
+        const int p = pair_of(q);
+        const cplx pre = decay_before(p), F = cmul(pre, sm.bp[p][I].R);
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int row = 32 * I + 8 * r + g;
             const float x = oz[q][r] + pd[r] * gx[q][r], xo = __shfl_xor_sync(0xffffffffu, x, 1);
-            ho[r] = __shfl_xor_sync(0xffffffffu, rho[q][r], 1);
+            const float ho = __shfl_xor_sync(0xffffffffu, rho[q][r], 1);
             const float2 D = sm.dd[p][row], D0 = sm.dd[p][row > 0 ? row - 1 : 0];
             const bool first = r == 0 && g == 0;
             const cplx w0 = first ? pre : cmul({D0.x, D0.y}, F);
-            y[r] = rotate({D.x, D.y}, x, xo) + rotate(w0, rho[q][r], ho[r]);
+            oz[q][r] = rotate({D.x, D.y}, x, xo) + rotate(w0, rho[q][r], ho);
         }
+    }
+    if (slow != 0) {
+#pragma unroll
+        for (int q = 0; q < kOwn; q++)
 #pragma unroll 1
-        for (int s = 0; s < kPerTile; s++)
-            if (sm.bp[2 * q + s][I].slow) {
-                slow_walk<kD, kPairs, kMode, true>(sm, 2 * q + s, I, tl);
-                if (kPairs == 1 || (t4 >> 1) == s) {
+            for (int s = 0; s < kPerTile; s++)
+                if ((slow >> (2 * tile(q) + s)) & 1) {
+                    const cplx pre = decay_before(2 * tile(q) + s);
+                    slow_walk<kD, kPairs, kMode, true>(sm, 2 * tile(q) + s, I, W, tl);
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
-                        const float4 x = sm.walk[I][8 * r + g];
-                        y[r] = (comp ? x.y : x.x) + rotate(cmul(pre, {x.z, x.w}), rho[q][r], ho[r]);
+                        const float ho = __shfl_xor_sync(0xffffffffu, rho[q][r], 1);
+                        const float4 x = sm.walk[W][8 * r + g];
+                        if (kPairs == 1 || (t4 >> 1) == s)
+                            oz[q][r] = (comp ? x.y : x.x) + rotate(cmul(pre, {x.z, x.w}), rho[q][r], ho);
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
-            }
+    }
+#pragma unroll
+    for (int q = 0; q < kOwn; q++) {
+        const int p = pair_of(q);
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int row = 32 * I + 8 * r + g;
-            float yy = mq[r] * y[r];
+            float yy = mq[r] * oz[q][r];
             if (a.shortcut_scale != 0.f) {   // block.py:202-208; v after the vp scale
                 const float qk = mq[r] * nrm[r] * pd[r];
                 const float2 e = sm.viw[p][row], D = sm.dd[p][row];
                 cplx vg = cmul({e.x, e.y}, {D.x, D.y});
-                if (sm.bp[p][I].slow) {               // (its v has made room for g)
+                if ((slow >> p) & 1) {               // (its v has made room for g)
                     const uint32_t w = __ldcg(a.rec_v + (unit * (size_t)NP + p) * kD + row);
                     vg = {bits_lo(w), bits_hi(w)};
                 }
                 yy += a.shortcut_scale * qk * qk * bfr(comp ? vg.i : vg.r);
             }
-            if (kPairs > 1 || t4 < 2) sm.y(I, 8 * r + g)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * sm.sel[row]);
+            if (kPairs > 1 || t4 < 2) sm.y(row)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * sm.sel[row]);
         }
     }
     __syncwarp();
-    if (32 * I + tl < Lc) {   // lane = token: its row of N values
-        __nv_bfloat16* yo = a.y + (((size_t)b * L + c * kD + 32 * I + tl) * H + hd) * N;
-        const uint32_t* ys = reinterpret_cast<const uint32_t*>(sm.y(I, tl));
-        if (kPairs >= 4 && N == 2 * kPairs && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0) {
+    if (tok < Lc) {   // lane = token: its row of this warp's values
+        constexpr int kOwnPairs = G::kOwnPairs;
+        __nv_bfloat16* yo = a.y + (((size_t)b * L + c * kD + tok) * H + hd) * N;
+        const uint32_t* ys = reinterpret_cast<const uint32_t*>(sm.y(tok));
+        const int p0 = kOwnPairs * S;
+        if (kOwnPairs >= 4 && N == 2 * kPairs && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0) {
 #pragma unroll
-            for (int i = 0; i < kPairs; i += 4)
-                *reinterpret_cast<uint4*>(yo + 2 * i) = make_uint4(ys[i], ys[i + 1], ys[i + 2], ys[i + 3]);
+            for (int i = 0; i < kOwnPairs; i += 4)
+                *reinterpret_cast<uint4*>(yo + 2 * (p0 + i)) = make_uint4(ys[p0 + i], ys[p0 + i + 1], ys[p0 + i + 2], ys[p0 + i + 3]);
         } else {
-            for (int i = 0; i < NP; i++) reinterpret_cast<uint32_t*>(yo)[i] = ys[i];
+            for (int i = p0; i < min(NP, p0 + kOwnPairs); i++) reinterpret_cast<uint32_t*>(yo)[i] = ys[i];
         }
     }
     // ---- the recurrent state after the last token
     if (a.tail_state && c == a.NC - 1) {
         __syncthreads();   // every block's h is published
 #pragma unroll 1
-        for (int q = 0; q < kTiles; q++) {
+        for (int q = 0; q < kOwn; q++) {
             float z[2][4], h[2][4];
             k_transposed(G::slot_end(0), q, z);
             k_transposed(G::slot_h(0), q, h);

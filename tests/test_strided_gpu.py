@@ -99,7 +99,9 @@ def _by_operators(ops, m, ids, cached):
 @pytest.mark.parametrize("d_model,state_dim", [(256, 2), (512, 6)])
 @pytest.mark.parametrize("B,L", [(1, 1), (3, 2), (2, 70), (2, 576), (1, 577)])   # the last two: both sides of the prompt rule
 def test_lm_sequence_equals_operators(ops, d_model, state_dim, B, L):
-    """bf16 at the same places, other kernels in the scan: 2e-2 is the model-level bound used elsewhere."""
+    """bf16 at the same places, other kernels in the scan: 2e-2 is the model-level bound used elsewhere.  In a state meet k, v,
+    the write gate and the decay, and where the scans' sums differ each of them may round to the next bf16, at most 2^-7 of the
+    value, without averaging out in the largest element: 4 * 2^-7."""
     from cdssm_b200.model import CdssmConfig, CdssmLM
     m = CdssmLM(CdssmConfig(d_model=d_model, n_layers=2, context_length=256, vocab_size=503, state_dim=state_dim), device="cuda", seed=5)
     for i, p in enumerate(m.blocks):
@@ -113,5 +115,5 @@ def test_lm_sequence_equals_operators(ops, d_model, state_dim, B, L):
         assert rel_err(to_np(got), to_np(want)) <= 2e-2
         if cached:
             for c, (tail, conv) in zip(cache["layers"], caches):
-                assert rel_err(to_np(c["state"]), to_np(tail)) <= 2e-2
+                assert rel_err(to_np(c["state"]), to_np(tail)) <= 4 * 2.0 ** -7
                 assert rel_err(to_np(c["conv"]), to_np(conv)) <= 2e-2
