@@ -55,6 +55,7 @@ struct Args {
     unsigned long long wait_ns;  // limit of every device-side wait
     int withhold;                // test hook: nothing is loaded, so the first wait runs out
     float shortcut_scale;
+    int from_chunks;             // kOutput: the carry from the local results of the chunks before (no carry pass has run)
     int B, L, H, N, NC;
 };
 
@@ -412,9 +413,8 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int s = 0; s < G::kSlabs; s++) tma_load_4d(sm.k + s * G::kSlab, &tmK, &sm.full_k, 64 * s, hd, c * kD, b);
     }
 
-    if (kMode == kOutput) grid_dependency_wait();   // the carry pass
-    // ---- carry into the chunk: this warp's 32 columns of every state row.  Already there (previous pass), or early if
-    // its producer is done; else polled for behind the products that do not need it.
+    // ---- carry into the chunk: this warp's 32 columns of its state rows.  Early if its producer is done, else polled for
+    // behind the products that do not need it (kOutput: the previous pass is waited for there).
     const float* carry_src = a.ws_state + unit * (size_t)N * kD;
     int* carry_flag = reinterpret_cast<int*>(a.ws_gamma + unit * (size_t)N);   // a bit per warp
     auto flag_set = [&]() {
@@ -435,9 +435,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         cp_async_commit();
     };
     bool have_carry = true;
-    if (kMode == kOutput) {
-        load_carry(carry_src);
-    } else if (kMode == kFused) {
+    if (kMode == kFused) {
         if (c == 0) load_carry(a.h0 ? a.h0 + ((size_t)b * H + hd) * N * kD : nullptr);
         else if ((have_carry = __all_sync(0xffffffffu, flag_set()))) load_carry(carry_src);
     }
@@ -879,7 +877,74 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             if (tl == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(next), "r"(1 << W) : "memory");
         }
     } else {
-        cp_async_wait_all();
+        grid_dependency_wait();   // the pass before; the records are there: it has waited for them before this launch
+        if (!a.from_chunks) {
+            load_carry(carry_src);
+            cp_async_wait_all();
+        } else {
+            // s <- gamma s + z over the chunks before, in the carry pass's order; lane = column
+            const size_t first = (size_t)b * a.NC * H + hd;
+            float sr[G::kOwnPairs], si[G::kOwnPairs];
+            const float* h0 = a.h0 ? a.h0 + ((size_t)b * H + hd) * N * kD + tok : nullptr;
+            auto row = [&](int i) { return 2 * min(G::kOwnPairs * S + i, NP - 1); };
+#pragma unroll
+            for (int i = 0; i < G::kOwnPairs; i++) {
+                sr[i] = h0 ? h0[row(i) * kD] : 0.f;
+                si[i] = h0 ? h0[(row(i) + 1) * kD] : 0.f;
+            }
+            const int chunks = c + (c + 1 == a.NC && a.final_state ? 1 : 0);
+            constexpr int kBatch = 8 / G::kOwnPairs < 2 ? 2 : 8 / G::kOwnPairs;
+#pragma unroll 1
+            for (int c0 = 0; c0 < chunks; c0 += kBatch) {
+                float l[kBatch][G::kOwnPairs][2];
+                float2 gm[kBatch][G::kOwnPairs];
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    const size_t u = first + (size_t)min(c0 + k, chunks - 1) * H;
+#pragma unroll
+                    for (int i = 0; i < G::kOwnPairs; i++) {
+                        const float* z = a.ws_state + (u * N + row(i)) * kD + tok;
+                        l[k][i][0] = __ldcg(z);
+                        l[k][i][1] = __ldcg(z + kD);
+                        gm[k][i] = __ldcg(reinterpret_cast<const float2*>(a.ws_gamma + u * N + row(i)));
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    if (c0 + k == c) {   // (the last chunk's own step, for the final state)
+#pragma unroll
+                        for (int i = 0; i < G::kOwnPairs; i++) {
+                            sm.s_in[2 * (G::kOwnPairs * S + i)][tok] = sr[i];
+                            sm.s_in[2 * (G::kOwnPairs * S + i) + 1][tok] = si[i];
+                        }
+                    }
+                    if (c0 + k < chunks) {
+#pragma unroll
+                        for (int i = 0; i < G::kOwnPairs; i++) {
+                            const cplx gam = {gm[k][i].x, gm[k][i].y};
+                            const float nr = next_re(gam, sr[i], si[i], l[k][i][0]);
+                            si[i] = next_im(gam, sr[i], si[i], l[k][i][1]);
+                            sr[i] = nr;
+                        }
+                    }
+                }
+            }
+            if (chunks == c) {
+#pragma unroll
+                for (int i = 0; i < G::kOwnPairs; i++) {
+                    sm.s_in[2 * (G::kOwnPairs * S + i)][tok] = sr[i];
+                    sm.s_in[2 * (G::kOwnPairs * S + i) + 1][tok] = si[i];
+                }
+            } else {
+                float* fs = a.final_state + ((size_t)b * H + hd) * N * kD + tok;
+#pragma unroll
+                for (int i = 0; i < G::kOwnPairs; i++)
+                    if (G::kOwnPairs * S + i < NP) {
+                        fs[row(i) * kD] = sr[i];
+                        fs[(row(i) + 1) * kD] = si[i];
+                    }
+            }
+        }
         __syncwarp();
     }
     // r_0: the carry rounded to bf16
@@ -1167,10 +1232,10 @@ bool scan_chunk_supported(int D, int N, int C, int dtype) {
 // scan_records.cu
 void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a, uint32_t** v, uint32_t** g);
 
-// mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the carries from ws_state,
-// writes y), 2: both in one kernel with the carry handed on inside it (ws_gamma and *ticket zeroed by the caller).
+// mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the carries from ws_state, with
+// from_chunks the local results of this call's local pass; writes y, with from_chunks the final state too), 2: both in one kernel with the carry handed on inside it (ws_gamma and *ticket zeroed by the caller).
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
-int scan_chunk_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
+int scan_chunk_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
                     float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
                     int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st) {
     using namespace chunk;
@@ -1187,6 +1252,7 @@ int scan_chunk_pass(int mode, const void* q, long long q_rs, const void* k, long
     a.ws_gamma = ws_gamma; a.ws_state = ws_state; a.status = status; a.ticket = ticket;
     a.wait_ns = wait_ns ? wait_ns : 400ull * 1000 * 1000;
     a.withhold = withhold;
+    a.from_chunks = from_chunks;
     a.shortcut_scale = shortcut_scale;
     a.B = B; a.L = L; a.H = H; a.N = N; a.NC = (L + D - 1) / D;
     if ((long long)B * a.NC * H > 0x7fffffff) return CDSSM_ERR_UNSUPPORTED;

@@ -31,7 +31,7 @@ struct Args {
 
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-// kNP: pair slots (>= N / 2); kHg: heads per block.
+// kNP: pairs per thread, from kNP * blockIdx.z on; kHg: heads per block.
 template <int kNP, int kHg, bool kWa, bool kResidual>
 __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     using T = __nv_bfloat16;
@@ -41,15 +41,15 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     float2* sa = reinterpret_cast<float2*>(smem);                      // else [pair][head][token]
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
-    for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x; i < a.clear_words;
+    for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x; i < a.clear_words && blockIdx.z == 0;
          i += (size_t)gridDim.x * gridDim.y * kThreads)
         a.clear[i] = 0;
-    const int H = a.H, N = a.N, NP = N >> 1;
+    const int H = a.H, N = a.N, NP = N >> 1, p0 = kWa ? 0 : kNP * (int)blockIdx.z, pairs = min(kNP, NP - p0);
     const int b = (int)(blockIdx.x / (unsigned)a.tiles), tile = (int)(blockIdx.x - (unsigned)b * a.tiles), l0 = tile * kTokens;
     const int head0 = blockIdx.y * kHg, heads = min(kHg, H - head0);
     const int head = threadIdx.x & (kHg - 1), hd = head0 + min(head, heads - 1);
     const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
-    T x[kItems][5], ga[kItems][kNP], gw[kItems][kNP];
+    T x[kItems][7], ga[kItems][kNP], gw[kItems][kNP];
     uint32_t vv[kItems][kNP], vf[kResidual ? kItems : 1][kNP];
 #pragma unroll
     for (int i = 0; i < kItems; i++) {
@@ -59,9 +59,11 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
         const uint32_t* v = reinterpret_cast<const uint32_t*>(a.v + row * a.v_rs + hd * N);
 #pragma unroll
         for (int s = 0; s < 5; s++) x[i][s] = g[(N + s) * H];
+        x[i][5] = g[0];             // (the first pair's: part of what the pairs share)
+        x[i][6] = g[NP * H];
 #pragma unroll
         for (int p = 0; p < kNP; p++) {
-            const int pp = p < NP ? p : 0;
+            const int pp = p < pairs ? p0 + p : p0;
             ga[i][p] = g[pp * H];
             gw[i][p] = g[(NP + pp) * H];
             vv[i][p] = v[pp];
@@ -69,7 +71,7 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
         if (kResidual) {
             const uint32_t* f = reinterpret_cast<const uint32_t*>(a.v_first + row * a.vf_rs + hd * N);
 #pragma unroll
-            for (int p = 0; p < kNP; p++) vf[i][p] = f[p < NP ? p : 0];
+            for (int p = 0; p < kNP; p++) vf[i][p] = f[p < pairs ? p0 + p : p0];
         }
     }
     const float mix = kResidual ? __bfloat162float(a.mix[hd]) : 0.f;
@@ -79,13 +81,13 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
         const bool on = l < a.L;                                       // behind the end a = 1, beta = v = 0: the state stands still
         const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
         auto f = [](T y) { return __bfloat162float(y); };
-        const DynShared ds = dyn_shared<true>(f(ga[i][0]), f(gw[i][0]), f(x[i][0]), f(x[i][1]), f(x[i][2]), f(x[i][3]), f(x[i][4]),
+        const DynShared ds = dyn_shared<true>(f(x[i][5]), f(x[i][6]), f(x[i][0]), f(x[i][1]), f(x[i][2]), f(x[i][3]), f(x[i][4]),
                                               lds, freq, pos, a.dc);
         const uint32_t bs = on ? pack2(ds.beta, ds.sel_c) : 0u;
         if (!kWa) sg[head * kRow + t] = bs;
 #pragma unroll
         for (int p = 0; p < kNP; p++) {
-            if (p >= NP) break;
+            if (p >= pairs) break;
             float ar, ai, vp;
             dyn_pair<true>(f(ga[i][p]), f(gw[i][p]), freq, pos, ds, ar, ai, vp);
             if (!a.fp32_decay) { ar = bfr(ar); ai = bfr(ai); }
@@ -114,13 +116,13 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     } else {
         const int c = l0 / a.C, in_chunk = l0 - c * a.C;
         const size_t unit0 = ((size_t)b * a.NC + c) * H + head0;
-        for (int i = warp; i < heads * NP; i += kThreads / 32) {
-            const int h = i / NP, p = i - h * NP, s = (p * kHg + h) * kRow + lane;
-            const size_t o = ((unit0 + h) * NP + p) * a.C + in_chunk + lane;
+        for (int i = warp; i < heads * pairs; i += kThreads / 32) {
+            const int h = i / pairs, p = i - h * pairs, s = (p * kHg + h) * kRow + lane;
+            const size_t o = ((unit0 + h) * NP + p0 + p) * a.C + in_chunk + lane;
             a.rec_a[o] = sa[s];
             a.rec_v[o] = sv[s];
         }
-        for (int h = warp; h < heads; h += kThreads / 32) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sg[h * kRow + lane];
+        for (int h = warp; h < heads && p0 == 0; h += kThreads / 32) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sg[h * kRow + lane];
     }
 }
 
@@ -130,7 +132,8 @@ static int launch(const Args& a, cudaStream_t st) {
     const size_t smem = kWa ? (size_t)kHg * (kTokens + 1) * 16 : (size_t)kHg * (kTokens + 1) * (kNP * 12 + 4);
     if (smem > 48 * 1024)
         if (int rc = allow_smem<KernelTag<kNP, kHg, kWa, kResidual>>((const void*)records_kernel<kNP, kHg, kWa, kResidual>, smem)) return rc;
-    records_kernel<kNP, kHg, kWa, kResidual><<<dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg), kThreads, smem, st>>>(a);
+    records_kernel<kNP, kHg, kWa, kResidual><<<dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg, kWa ? 1 : (a.N / 2 + kNP - 1) / kNP),
+                                               kThreads, smem, st>>>(a);
     return check_launch();
 }
 // 16 heads fill the sectors of the gate rows; 8 where that leaves fewer lanes empty (24 heads) or more blocks are wanted.
@@ -177,6 +180,11 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
     if ((long long)B * a.tiles > 0x7fffffff || H > 8 * 65535) return CDSSM_ERR_UNSUPPORTED;
     if (wa) return launch_group<1, true>(a, st);
     if (N <= 2) return launch_group<1, false>(a, st);
+    // Short inputs: one pair per thread up to two blocks per SM, two up to four; each computes what the pairs share.  us, 24
+    // heads, N 16, all / two / one pair per thread: 523 tokens 5.4 / - / 3.7, 1046 5.6 / 4.6 / 5.9, 2092 7.1 / 7.3 / -.
+    const long long blocks = (long long)B * a.tiles * ((H + 7) / 8);
+    if (blocks * (N / 2) <= 296) return launch_group<1, false>(a, st);
+    if (N > 4 && blocks * ((N / 2 + 1) / 2) <= 592) return launch_group<2, false>(a, st);
     if (N <= 4) return launch_group<2, false>(a, st);
     if (N <= 8) return launch_group<4, false>(a, st);
     return launch_group<8, false>(a, st);

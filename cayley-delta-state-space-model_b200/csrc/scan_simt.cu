@@ -800,7 +800,7 @@ int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long
                  cudaStream_t st);
 // scan_chunk.cu
 bool scan_chunk_supported(int D, int N, int C, int dtype);
-int scan_chunk_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
+int scan_chunk_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
                     float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
                     int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
 }
@@ -832,17 +832,26 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
     return *status_host == 0 ? CDSSM_OK : CDSSM_ERR_TIMEOUT;
 }
 
-// Whether the whole-chunk scan runs as one kernel that hands the carry from chunk to chunk inside it, or as local pass +
-// carry pass + output pass.  One kernel reads k once and forms G once, but a hand-off takes 1.6 to 2 us (flag, carry, rounding,
-// release), so a (batch, head) chain of NC chunks takes that many whatever the size; the three passes cost a third more work.
-// us on B200, fitted to 100 sizes (one kernel / three passes, D 64): N 16, H 24: L 64 21 / 29, L 4096 186 / 130, B 4, L 2048
-// 180 / 168, B 8 220 / 303; N 2, H 6: L 523 23 / 18, L 4096 112 / 23; D 128, N 4, H 24, B 8, L 2048 176 / 257.
+// Whether the output pass of the whole-chunk scan adds the carry up itself from the local results of the chunks before it (else
+// a carry pass runs in between): a read of NC x N rows by every block, in parallel, against a launch and two more trips to
+// memory.  us on B200, carry pass / without (D 64, one sequence): N 16, H 24, 9 chunks 35 / 24, 16 chunks 38 / 27, 32 chunks
+// 43 / 46; N 4, H 6, 9 chunks 14 / 11, 48 chunks 19 / 20; N 2, H 6, 9 chunks 14 / 10.
+static bool few_chunks(int NC, int N) { return NC <= 40 && NC * N <= 400; }
+
+// Whether the whole-chunk scan runs as one kernel that hands the carry from chunk to chunk inside it, or as local pass
+// (+ carry pass) + output pass.  One kernel reads k once and forms G once, but a hand-off takes 2 us and more (flag, carry,
+// rounding, release), so a (batch, head) chain of NC chunks takes that many whatever the size; the passes cost more work.
+// Each form: the larger of its latency and its work on the full GPU, us on B200, fitted to 220 sizes (one kernel / passes, D 64:
+// N 16, B 8, H 12, 29 chunks 122 / 110; N 8, B 4, H 32, 50 chunks 150 / 173; N 2, B 4, H 24, 5 chunks 17 / 13.5, B 16, H 24, 2
+// chunks 18 / 21; D 128, N 4, B 2, H 32, 27 chunks 101 / 135); the choice costs 0.4 % over the better one on average.
 static bool one_kernel_pays(int B, int H, int NC, int D, int N) {
-    const float units = (float)B * H * NC, n = (float)N;
-    const float per_unit = D == 64 ? 0.0125f + 0.0015f * n : 0.036f + (N > 8 ? 0.0089f : 0.0053f) * n;   // us, full GPU
-    const float one = D == 64 ? 11.f + 0.6f * n : 14.f + n, three = D == 64 ? 16.f + 0.8f * n : 23.f + 1.2f * n;   // alone
-    const float a = one + (1.6f + 0.03f * n) * NC, b = units * per_unit, c = units * per_unit * 1.35f;
-    return (a > b ? a : b) <= (three > c ? three : c);
+    const float units = (float)B * H * NC, n = (float)N, c = (float)NC;
+    const bool carry = !few_chunks(NC, N);
+    const float one = D == 64 ? fmaxf(6.7f + (1.96f + 0.1f * n) * c, 6.5f + units * (0.0113f + 0.00118f * n))
+                              : fmaxf(10.7f + (2.6f + 0.033f * n) * c, 9.1f + units * (0.0282f + 0.00665f * n));
+    const float passes = D == 64 ? fmaxf(9.5f + 0.21f * n + 0.173f * c + (carry ? 10.f : 0.f), 7.2f + units * (0.0161f + 0.00161f * n))
+                                 : fmaxf(15.8f + 0.49f * n + (carry ? 1.7f : 0.f), 13.3f + units * (0.0497f + 0.0075f * n));
+    return one <= passes;
 }
 
 struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual
@@ -901,16 +910,17 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                                           align256((size_t)a.units * 2 * sizeof(float)));
     cudaStream_t st = (cudaStream_t)stream;
     // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 with heads in fours (scan_wa.cu), any other
-    // N <= 16 (scan_chunk.cu).  The latter also for a few chunks of N = 2, which it does in one kernel behind the records'
-    // where scan_wa.cu takes three, two of them walking a chunk in sub-blocks (us, one chunk: 17 / 22 at D 64, 20 / 30 at
-    // D 128; nine chunks of 24 heads of 64: 22 / 20; five and seven chunks of 4 heads of 128: 28 / 31, 29 / 32).  They read v
+    // N <= 16 (scan_chunk.cu).  The latter also for N = 2 while the
+    // GPU is not full: its passes do a chunk as a whole where scan_wa.cu walks it in sub-blocks (us, passes / scan_wa.cu, D 64:
+    // 120 chunks 10 / 17, 544 15 / 20, 704 22 / 22, 936 25 / 23; one kernel / scan_wa.cu, up to six chunks in a row: 768 18 / 21,
+    // 1536 28 / 31, 1920 in threes 49 / 37; D 128: 192 21 / 30, 528 39 / 32).  They read v
     // and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the contract allows, stay on the CUDA-core
     // kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the tests to check each tensor-core pass alone.)
     const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y | (uintptr_t)rows.first | (uintptr_t)(2 * v_rs) |
                               (uintptr_t)(rows.first ? 2 * vf_rs : 0)) & 3) == 0 && ((q_rs | k_rs) & 7) == 0 && workspace_bytes - base >= scan_record_bytes(B, L, H, N, C) &&
                            !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
     const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, H, dtype) &&
-                       ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > (D == 64 ? 2 : 7) || (long long)B * a.NC * H > (D == 64 ? 512 : 256));
+                       ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > 40 || (long long)B * a.NC * H > (D == 64 ? (a.NC <= 6 ? 1536 : 640) : 256));
     const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
     if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && !wa_ok) return CDSSM_ERR_UNSUPPORTED;
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
@@ -947,11 +957,13 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (!tensor) return scan_fused_simt(a, dtype, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
+    // (then the output pass has also done all that needs no carry by the time the local pass ends)
+    const int from_chunks = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && few_chunks(a.NC, N) ? 1 : 0;
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
                                 limit, withhold, st);
-        return scan_chunk_pass(mode, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
+        return scan_chunk_pass(mode, from_chunks, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
                                shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };
     // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)
@@ -964,6 +976,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
         if (int rc = pass(0)) return rc;
         a.run_local = 0;
     }
+    if (from_chunks) return pass(1);
     a.run_output = tc_output ? 0 : 1;
     if (int rc = scan_fused_simt(a, dtype, st)) return rc;   // carry pass (+ whatever was kept)
     return !tc_output || summary_only ? CDSSM_OK : pass(1);
