@@ -797,7 +797,7 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
 bool scan_wa_supported(int D, int N, int C, int H, int dtype);
 int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
-                 cudaStream_t st);
+                 int from_chunks, const float* h0, float* final_state, cudaStream_t st);
 // scan_chunk.cu
 bool scan_chunk_supported(int D, int N, int C, int dtype);
 int scan_chunk_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
@@ -957,12 +957,15 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (!tensor) return scan_fused_simt(a, dtype, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
-    // (then the output pass has also done all that needs no carry by the time the local pass ends)
-    const int from_chunks = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && few_chunks(a.NC, N) ? 1 : 0;
+    // (The whole-chunk output pass has also done all that needs no carry by the time the local pass ends.  scan_wa.cu: while its
+    // output pass has a chunk of four heads per block, two blocks per SM; us, carry pass / without: D 64, 936 chunks 24.4 / 21.5,
+    // 3072 42 / 44; D 128, 528 32.3 / 30.5, 1536 61 / 63.)
+    const int from_chunks = (chunk_ok || (wa_ok && (long long)B * a.NC * H <= 4 * 296)) &&
+                            tc_local && tc_output && a.run_local && !summary_only && few_chunks(a.NC, N);
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
-                                limit, withhold, st);
+                                limit, withhold, from_chunks, h0, final_state, st);
         return scan_chunk_pass(mode, from_chunks, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
                                shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };

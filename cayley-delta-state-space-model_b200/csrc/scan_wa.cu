@@ -80,6 +80,9 @@ struct Args {
     unsigned long long wait_ns;  // limit of every device-side wait
     int withhold;                // test hook: the producer issues nothing, so the first wait runs out
     float shortcut_scale;
+    const float* h0;             // output pass, from_chunks: the carry from the local results of the chunks before (no carry
+    float* final_state;          // pass has run), starting from h0; the last chunk's block leaves the final state
+    int from_chunks;
     int B, L, H, NC;
     int HG, items;               // head groups of four; items = B * NC * HG (one chunk of four heads each)
 };
@@ -436,6 +439,65 @@ __device__ __forceinline__ uint32_t split_pack(float x0, float x1, bool low) {
     return __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);   // {r1[31:16], r0[31:16]}
 }
 
+// The carry into a chunk of head hd, rounded: s <- gamma s + z over the chunks before, evaluated as the carry pass does; a lane
+// has kD / 32 columns.  out: its real, then its imaginary row.
+template <int kD>
+__device__ __forceinline__ void carry_from_chunks(const Args& a, const ItemPos& at, int hd, int tl, float* out) {
+    constexpr int kPer = kD / 32, kBatch = kD == 64 ? 8 : 4;
+    const size_t first = (size_t)at.b * a.NC * a.H + hd, so = ((size_t)at.b * a.H + hd) * 2 * kD + tl;
+    float sr[kPer], si[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+        sr[i] = a.h0 ? a.h0[so + 32 * i] : 0.f;
+        si[i] = a.h0 ? a.h0[so + kD + 32 * i] : 0.f;
+    }
+    auto put = [&]() {
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            out[tl + 32 * i] = bfr(sr[i]);
+            out[kD + tl + 32 * i] = bfr(si[i]);
+        }
+    };
+    const int chunks = at.c + (at.c + 1 == a.NC && a.final_state ? 1 : 0);   // (the last chunk's own step, for the final state)
+#pragma unroll 1
+    for (int c0 = 0; c0 < chunks; c0 += kBatch) {
+        float2 gm[kBatch];
+        float l[kBatch][kPer][2];
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) {
+            const size_t u = first + (size_t)min(c0 + k, chunks - 1) * a.H;
+            gm[k] = __ldcg(reinterpret_cast<const float2*>(a.ws_gamma + u * 2));
+#pragma unroll
+            for (int i = 0; i < kPer; i++) {
+                l[k][i][0] = __ldcg(a.ws_state + u * 2 * kD + tl + 32 * i);
+                l[k][i][1] = __ldcg(a.ws_state + u * 2 * kD + kD + tl + 32 * i);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) {
+            if (c0 + k == at.c) put();
+            if (c0 + k < chunks) {
+#pragma unroll
+                for (int i = 0; i < kPer; i++) {
+                    const float nr = __fadd_rn(__fmaf_rn(gm[k].x, sr[i], -__fmul_rn(gm[k].y, si[i])), l[k][i][0]);
+                    si[i] = __fadd_rn(__fmaf_rn(gm[k].x, si[i], __fmul_rn(gm[k].y, sr[i])), l[k][i][1]);
+                    sr[i] = nr;
+                }
+            }
+        }
+    }
+    if (chunks == at.c) {
+        put();
+    } else {
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            a.final_state[so + 32 * i] = sr[i];
+            a.final_state[so + kD + 32 * i] = si[i];
+        }
+    }
+    __syncwarp();
+}
+
 template <int kD, bool kOutput>
 __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     using DM = Dims<kD>;
@@ -496,6 +558,10 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
         const size_t unit = ((size_t)cur.b * a.NC + cur.c) * H + hd;   // workspace slot of this head's chunk
         if (step == 0) {   // states at the chunk start: z = 0, r = the chunk's carry
             const float* s = a.ws_state + unit * 2 * kD + (size_t)(np & 1) * kD;
+            if (kOutput && a.from_chunks) {
+                carry_from_chunks<kD>(a, cur, hd, tl, scr);
+                s = scr + (np & 1) * kD;
+            }
 #pragma unroll
             for (int ks = 0; ks < kKs; ks++) {
                 float2 v0 = make_float2(0.f, 0.f), v1 = v0;
@@ -505,6 +571,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 }
                 S[ks][0] = v0.x; S[ks][1] = v0.y; S[ks][2] = v1.x; S[ks][3] = v1.y;
             }
+            if (kOutput) __syncwarp();     // (scr is used again)
             gam = {1.f, 0.f};
         }
         // ---- fetch the record of step g + 1 (the next item's first sub-block after this item's last)
@@ -861,11 +928,12 @@ bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
 }
 
 // One pass of the warp-autonomous tensor-core scan over every chunk.  output = false: local pass (fills
-// ws_state / ws_gamma for the carry pass); output = true: reads the carries from ws_state, writes y.
+// ws_state / ws_gamma for the carry pass); output = true: reads the carries from ws_state (from_chunks: adds them up from the
+// local pass of this call), writes y.
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
 int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
-                 cudaStream_t st) {
+                 int from_chunks, const float* h0, float* final_state, cudaStream_t st) {
     using namespace wa;
     CUtensorMap tmK, tmQ;
     if (!make_tile_map(&tmK, k, k_rs, B, L, H, D, kSub) || !make_tile_map(&tmQ, output ? q : k, output ? q_rs : k_rs, B, L, H, D, kSub)) return CDSSM_ERR_CUDA;
@@ -880,6 +948,7 @@ int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long
     a.status = status;
     a.wait_ns = wait_ns ? wait_ns : 400ull * 1000 * 1000;
     a.withhold = withhold;
+    a.from_chunks = from_chunks; a.h0 = h0; a.final_state = final_state;
     a.shortcut_scale = shortcut_scale;
     a.B = B; a.L = L; a.H = H; a.NC = (L + D - 1) / D;
     a.HG = H / 4;

@@ -204,3 +204,19 @@ def test_wa_tail_state(ops, orc, D, L):
     assert rel_err(to_np(y), to_np(ys)) <= BF16_TOL / 2
     assert np.abs(to_np(fin) - to_np(fs)).max() <= 2e-2 * max(np.abs(to_np(fs)).max(), 1e-3)
     assert np.abs(to_np(tail) - to_np(ts)).max() <= 1e-2 * np.abs(to_np(ts)).max()
+
+
+@pytest.mark.parametrize("D,NC", [(64, 1), (64, 8), (64, 9), (64, 40), (128, 4), (128, 13)])
+@pytest.mark.parametrize("ragged", [0, 5])
+def test_wa_carry_from_chunks_is_the_carry_pass(ops, orc, D, NC, ragged):
+    """One sequence (the output pass adds the carry up itself) and the same one in a batch of more chunks than that is done for
+    (a carry pass in between): the same bits, at the ends of the batches in which the chunks are read."""
+    H, L = 4, NC * D - ragged
+    inp = _inputs(orc, 1, H, L, D, seed=NC)
+    h0 = np.random.default_rng(3).standard_normal((1, H, N, D)).astype(np.float32)
+    kw = dict(flags=ops.TENSOR_CORE_WA, return_tail_state=True, shortcut_scale=0.3)
+    one = run_fused(ops, inp, torch.bfloat16, N, D, h0=h0, **kw)
+    B = 1184 // (NC * H) + 1
+    many = {k: np.repeat(v, B, 0) if k in ("q", "k", "v", "gate_raw") else v for k, v in inp.items()}
+    for a, b in zip(one, run_fused(ops, many, torch.bfloat16, N, D, h0=np.repeat(h0, B, 0), **kw)):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[0], b[B - 1])
