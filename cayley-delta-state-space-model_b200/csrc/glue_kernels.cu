@@ -11,16 +11,21 @@
 namespace cdssm {
 
 // ---------------------------------------------------------------- RMSNorm
+// The kernels below are launched while their predecessor drains and wait for it before they read anything: between the small
+// products of a short prompt a plain launch cost as much as some of them (12 layers, d 768, 523 tokens: 825 -> 713 us with the conv and
+// the scan's records).  Inputs carry no __restrict__: as read-only data their loads could be moved above that wait.
+
 // One warp per row: out = rnd(rnd(x * rsqrt(mean x^2 + eps)) * w)   (modules.py:50-53)
 template <typename T>
 __global__ void __launch_bounds__(256)
-rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, long long rows, int d,
+rmsnorm_fwd_kernel(const T* x, const T* w, T* __restrict__ out, long long rows, int d,
                    float eps) {
     const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31;
     const T* xr = x + row * d;
     float ss = 0.f;
+    grid_dependency_wait();
     for (int c = lane * 8; c < d; c += 256) {
         float f[8];
         Vec8<T>::ld(xr + c, f);
@@ -43,11 +48,12 @@ rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restri
 // threads instead of one warp's dependent loop.  Same arithmetic; the sum of squares is reduced in a fixed order.
 template <typename T>
 __global__ void __launch_bounds__(256)
-rmsnorm_row_block_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, int d, float eps) {
+rmsnorm_row_block_kernel(const T* x, const T* w, T* __restrict__ out, int d, float eps) {
     const T* xr = x + (long long)blockIdx.x * d;
     T* orow = out + (long long)blockIdx.x * d;
     __shared__ float sh[8];
     float ss = 0.f;
+    grid_dependency_wait();
     for (int c = threadIdx.x * 8; c < d; c += 2048) {
         float f[8];
         Vec8<T>::ld(xr + c, f);
@@ -85,13 +91,14 @@ static int gn_tiles(int L) {
 
 template <typename T>
 __global__ void __launch_bounds__(1024)
-groupnorm_partial_kernel(const T* __restrict__ y, float* __restrict__ partial, int L, int di, int groups, int tiles) {
+groupnorm_partial_kernel(const T* y, float* __restrict__ partial, int L, int di, int groups, int tiles) {
     const int b = blockIdx.x / tiles, tile = blockIdx.x % tiles;
     const int rows = (L + tiles - 1) / tiles;
     const int l0 = tile * rows, l1 = min(L, l0 + rows);
     const int cg = di / groups, tpg = cg / 8;
     const T* base = y + ((long long)b * L) * di + threadIdx.x * 8;
     float s = 0.f, q = 0.f;
+    grid_dependency_wait();
     for (int l = l0; l < l1; l++) {
         float f[8];
         Vec8<T>::ld(base + (long long)l * di, f);
@@ -112,13 +119,14 @@ groupnorm_partial_kernel(const T* __restrict__ y, float* __restrict__ partial, i
 }
 
 __global__ void __launch_bounds__(128)
-groupnorm_finalize_kernel(const float* __restrict__ partial, float* __restrict__ stats, int total, int L, int cg,
+groupnorm_finalize_kernel(const float* partial, float* __restrict__ stats, int total, int L, int cg,
                           int groups, int tiles, float eps) {
     const int i = blockIdx.x * 4 + (threadIdx.x >> 5);     // (batch row, group): one warp each
     if (i >= total) return;
     const int lane = threadIdx.x & 31;
     const int b = i / groups, grp = i % groups;
     double s = 0.0, q = 0.0;
+    grid_dependency_wait();
     for (int t = lane; t < tiles; t += 32) {               // lane-strided, then a fixed shuffle tree: deterministic
         const float* p = partial + (((long long)b * tiles + t) * groups + grp) * 2;
         s += (double)p[0];
@@ -143,15 +151,16 @@ groupnorm_finalize_kernel(const float* __restrict__ partial, float* __restrict__
 // groupnorm_stats_kernel.  out = rnd(rnd(rnd(GN(y)) * rnd(silu(z))) + rnd(D * x_conv))   (block.py:216-224)
 template <typename T>
 __global__ void __launch_bounds__(1024)
-groupnorm_gate_fwd_kernel(const T* __restrict__ y, const float* __restrict__ stats, const T* __restrict__ gn_w,
-                          const T* __restrict__ gn_b, const T* __restrict__ z, long long z_row_stride,
-                          const T* __restrict__ skip, const T* __restrict__ x_conv, T* __restrict__ out, int L,
+groupnorm_gate_fwd_kernel(const T* y, const float* stats, const T* gn_w,
+                          const T* gn_b, const T* z, long long z_row_stride,
+                          const T* skip, const T* x_conv, T* __restrict__ out, int L,
                           int di, int groups, float eps) {
     const long long row = blockIdx.x;
     const int c = threadIdx.x * 8;
     const int cg = di / groups, tpg = cg / 8;          // threads per group
     const int grp = threadIdx.x / tpg;
     float f[8];
+    grid_dependency_wait();
     Vec8<T>::ld(y + row * di + c, f);
     float mean, rstd;
     if (stats == nullptr) {
@@ -192,14 +201,15 @@ groupnorm_gate_fwd_kernel(const T* __restrict__ y, const float* __restrict__ sta
 // rows per block 41.
 template <typename T, int kRows, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads)
-groupnorm_gate_rows_kernel(const T* __restrict__ y, const float* __restrict__ stats, const T* __restrict__ gn_w,
-                           const T* __restrict__ gn_b, const T* __restrict__ z, long long z_row_stride,
-                           const T* __restrict__ skip, const T* __restrict__ x_conv, T* __restrict__ out,
+groupnorm_gate_rows_kernel(const T* y, const float* stats, const T* gn_w,
+                           const T* gn_b, const T* z, long long z_row_stride,
+                           const T* skip, const T* x_conv, T* __restrict__ out,
                            int rows, int L, int di, int groups) {
     const int r0 = blockIdx.x * kRows, c = threadIdx.x * 8;
     const int grp = threadIdx.x / ((di / groups) / 8);
     Raw8<T> f[kRows], zz[kRows], xc[kRows];
     float2 st[kRows];
+    grid_dependency_wait();
 #pragma unroll
     for (int r = 0; r < kRows; r++) {
         const int row = min(r0 + r, rows - 1);
@@ -306,14 +316,12 @@ extern "C" int cdssm_b200_rmsnorm_fwd(const void* x, const void* weight, void* o
     if (d % 8 || !aligned16(x) || !aligned16(weight) || !aligned16(out)) return CDSSM_ERR_UNSUPPORTED;
     if (rows == 0) return CDSSM_OK;
     if (rows <= 2048) {   // one block per row
-        DISPATCH_DTYPE(dtype, (rmsnorm_row_block_kernel<T><<<(unsigned)rows, 256, 0, (cudaStream_t)stream>>>(
-                                  (const T*)x, (const T*)weight, (T*)out, d, eps)));
-        return check_launch();
+        DISPATCH_DTYPE(dtype, return launch_overlapped(rmsnorm_row_block_kernel<T>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream,
+                                                (const T*)x, (const T*)weight, (T*)out, d, eps));
     }
     const unsigned blocks = (unsigned)((rows + 7) / 8);
-    DISPATCH_DTYPE(dtype, (rmsnorm_fwd_kernel<T><<<blocks, 256, 0, (cudaStream_t)stream>>>(
-                              (const T*)x, (const T*)weight, (T*)out, rows, d, eps)));
-    return check_launch();
+    DISPATCH_DTYPE(dtype, return launch_overlapped(rmsnorm_fwd_kernel<T>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream,
+                                                   (const T*)x, (const T*)weight, (T*)out, (long long)rows, d, eps));
 }
 
 static int check_gn(int di, int groups) {
@@ -335,13 +343,13 @@ extern "C" int cdssm_b200_groupnorm_stats(const void* y, float* stats, int B, in
     if (B == 0 || L == 0) return CDSSM_OK;
     const int tiles = gn_tiles(L);
     float* partial = stats + (size_t)B * groups * 2;       // the tiles' sums live behind the results
-    DISPATCH_DTYPE(dtype, (groupnorm_partial_kernel<T><<<(unsigned)(B * tiles), di / 8, 0, (cudaStream_t)stream>>>(
-                              (const T*)y, partial, L, di, groups, tiles)));
-    if (int rc = check_launch()) return rc;
+    int rc = CDSSM_OK;
+    DISPATCH_DTYPE(dtype, rc = launch_overlapped(groupnorm_partial_kernel<T>, dim3((unsigned)(B * tiles)), dim3(di / 8), 0,
+                                                 (cudaStream_t)stream, (const T*)y, partial, L, di, groups, tiles));
+    if (rc) return rc;
     const int total = B * groups;
-    groupnorm_finalize_kernel<<<(unsigned)((total + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
-        partial, stats, total, L, di / groups, groups, tiles, eps);
-    return check_launch();
+    return launch_overlapped(groupnorm_finalize_kernel, dim3((unsigned)((total + 3) / 4)), dim3(128), 0, (cudaStream_t)stream,
+                             partial, stats, total, L, di / groups, groups, tiles, eps);
 }
 
 extern "C" int cdssm_b200_groupnorm_gate_fwd(const void* y, const float* stats, const void* gn_weight,
@@ -362,19 +370,16 @@ extern "C" int cdssm_b200_groupnorm_gate_fwd(const void* y, const float* stats, 
         const unsigned blocks = (unsigned)((rows + kRows - 1) / kRows);
         DISPATCH_DTYPE(dtype, {
             auto launch = [&](auto kernel) {
-                kernel<<<blocks, di / 8, 0, (cudaStream_t)stream>>>((const T*)y, stats, (const T*)gn_weight, (const T*)gn_bias, (const T*)z,
-                                                                    z_row_stride, (const T*)skip, (const T*)x_conv, (T*)out, (int)rows,
-                                                                    L, di, groups);
+                return launch_overlapped(kernel, dim3(blocks), dim3(di / 8), 0, (cudaStream_t)stream, (const T*)y, stats,
+                                         (const T*)gn_weight, (const T*)gn_bias, (const T*)z, (long long)z_row_stride, (const T*)skip,
+                                         (const T*)x_conv, (T*)out, (int)rows, L, di, groups);
             };
-            if (di / 8 <= 256) launch(groupnorm_gate_rows_kernel<T, kRows, 256>);
-            else launch(groupnorm_gate_rows_kernel<T, kRows, 1024>);
+            return di / 8 <= 256 ? launch(groupnorm_gate_rows_kernel<T, kRows, 256>) : launch(groupnorm_gate_rows_kernel<T, kRows, 1024>);
         });
-        return check_launch();
     }
-    DISPATCH_DTYPE(dtype, (groupnorm_gate_fwd_kernel<T><<<(unsigned)rows, di / 8, 0, (cudaStream_t)stream>>>(
-                              (const T*)y, stats, (const T*)gn_weight, (const T*)gn_bias, (const T*)z, z_row_stride,
-                              (const T*)skip, (const T*)x_conv, (T*)out, L, di, groups, eps)));
-    return check_launch();
+    DISPATCH_DTYPE(dtype, return launch_overlapped(groupnorm_gate_fwd_kernel<T>, dim3((unsigned)rows), dim3(di / 8), 0, (cudaStream_t)stream,
+                                            (const T*)y, stats, (const T*)gn_weight, (const T*)gn_bias, (const T*)z, (long long)z_row_stride,
+                                            (const T*)skip, (const T*)x_conv, (T*)out, L, di, groups, eps));
 }
 
 extern "C" int cdssm_b200_conv1d_silu_step(const void* x, int64_t x_row_stride, void* hist, const void* weight,

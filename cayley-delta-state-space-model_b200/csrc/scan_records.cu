@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     float2* sa = reinterpret_cast<float2*>(smem);                      // else [pair][head][token]
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
+    grid_dependency_wait();
     for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x; i < a.clear_words && blockIdx.z == 0;
          i += (size_t)gridDim.x * gridDim.y * kThreads)
         a.clear[i] = 0;
@@ -132,9 +133,9 @@ static int launch(const Args& a, cudaStream_t st) {
     const size_t smem = kWa ? (size_t)kHg * (kTokens + 1) * 16 : (size_t)kHg * (kTokens + 1) * (kNP * 12 + 4);
     if (smem > 48 * 1024)
         if (int rc = allow_smem<KernelTag<kNP, kHg, kWa, kResidual>>((const void*)records_kernel<kNP, kHg, kWa, kResidual>, smem)) return rc;
-    records_kernel<kNP, kHg, kWa, kResidual><<<dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg, kWa ? 1 : (a.N / 2 + kNP - 1) / kNP),
-                                               kThreads, smem, st>>>(a);
-    return check_launch();
+    return launch_overlapped(records_kernel<kNP, kHg, kWa, kResidual>,
+                             dim3((unsigned)(a.B * a.tiles), (a.H + kHg - 1) / kHg, kWa ? 1 : (a.N / 2 + kNP - 1) / kNP), dim3(kThreads),
+                             smem, st, a);
 }
 // 16 heads fill the sectors of the gate rows; 8 where that leaves fewer lanes empty (24 heads) or more blocks are wanted.
 template <int kNP, bool kWa>

@@ -117,3 +117,33 @@ def test_lm_sequence_equals_operators(ops, d_model, state_dim, B, L):
             for c, (tail, conv) in zip(cache["layers"], caches):
                 assert rel_err(to_np(c["state"]), to_np(tail)) <= 4 * 2.0 ** -7
                 assert rel_err(to_np(c["conv"]), to_np(conv)) <= 2e-2
+
+
+@pytest.mark.parametrize("B,L", [(1, 40), (4, 1100)])     # the kernels of short and of long inputs
+def test_kernels_see_what_the_kernel_before_them_wrote(ops, orc, B, L):
+    """They are launched while their predecessor drains: every input is rewritten right before the call, by a kernel that is
+    still running then, and the result has the bits of a call on settled inputs."""
+    H, D, N, di = 4, 64, 4, 512
+    g = torch.Generator(device="cuda").manual_seed(L)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    inp = orc.make_inputs(B, H, L, D, N=N, seed=1, bf16=True)
+    lds, rf = (torch.from_numpy(inp[n]).cuda().float() for n in ("log_dt_scale", "rope_freqs"))
+    calls = {
+        "rms_norm": (lambda x, w: ops.rms_norm(x, w, 1e-5), [rn(B, L, di), rn(di)]),
+        "conv": (lambda x, w, b: ops.CUDAConv1dSiLUOp.apply(x, w, b), [rn(B, L, di), rn(di, 1, 4), rn(di)]),
+        "gate": (lambda y, w, b, z, s, x: ops.groupnorm_gate(y, w, b, z, s, x, 32), [rn(B, L, di), rn(di), rn(di), rn(B, L, di), rn(di), rn(B, L, di)]),
+        "gate, token": (lambda y, w, b, z, s, x: ops.groupnorm_gate(y, w, b, z, s, x, 32, per_token=True),
+                        [rn(B, L, di), rn(di), rn(di), rn(B, L, di), rn(di), rn(B, L, di)]),
+        "scan": (lambda q, k, v, gate: ops.scan_fused(q, k, v, gate, lds, rf, *const_args(inp["consts"]), H, N, D)[0],
+                 [rn(B, L, H, D), rn(B, L, H, D), rn(B, L, H, N), rn(B, L, (N + 5) * H)]),
+    }
+    busy = torch.randn(1 << 24, device="cuda")
+    for name, (call, args) in calls.items():
+        want = call(*args).clone()
+        for late in range(len(args)):
+            work = [a.clone() for a in args]
+            work[late].zero_()
+            torch.cuda.synchronize()
+            busy.mul_(1.0)
+            work[late].copy_(args[late])
+            assert torch.equal(call(*work), want), (name, late)
