@@ -122,6 +122,50 @@ static Tensor rows(const Tensor& t, at::ScalarType dt, int64_t n_rows, int64_t i
     return dense(t, dt, name);
 }
 
+// One long sequence per batch row, cut into S chunk-aligned segments: summaries of all segments, their carries in series, the
+// scan of all segments as a batch on the local results the summaries have left in the workspace.
+std::array<Tensor, 2> scan_fused_long(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gate_, const Tensor& lds_,
+                                      const Tensor& rope_, const Dyn& dyn, int64_t heads, int64_t N, int64_t C, const Tensor& h0_,
+                                      double shortcut, int64_t pos0, int64_t flags, int64_t S) {
+    need_cuda(q_, "q");
+    const int dt = dtype_code(q_);
+    const Tensor q = q_.is_contiguous() ? q_ : q_.contiguous();
+    const Tensor k = dense(k_, q.scalar_type(), "k"), v = dense(v_, q.scalar_type(), "v");
+    const Tensor g = dense(gate_, q.scalar_type(), "gate_raw");
+    const int64_t B = q.size(0), L = q.size(1), H = q.size(2), D = q.size(3), R = B * S, Ls = L / S;
+    if (H != heads || k.sizes() != q.sizes() || v.sizes() != at::IntArrayRef({B, L, H, N}) ||
+        g.sizes() != at::IntArrayRef({B, L, (N + 5) * H}))
+        throw Error("scan_fused_long: inconsistent shapes");
+    const Tensor lds = f32_vector(lds_, "log_dt_scale"), rope = f32_vector(rope_, "rope_freqs");
+    Tensor h0;
+    if (h0_.defined()) {
+        h0 = dense(h0_, at::kFloat, "h0");
+        if (h0.numel() != B * H * N * D) throw Error("h0 must be (B,H,N,D)");
+    }
+    const c10::cuda::CUDAGuard guard(q.device());
+    const Tensor y = empty_like_dims({B, L, H, N}, q), final_state = empty_f32({B, H, N, D}, q);
+    // carries out of and into the segments, the segments' last carries (not handed out), their decays and the whole one
+    const int64_t st_n = (R * H * N * D + 63) & ~63, dc_n = R * H * N;
+    const Tensor scratch = empty_f32({3 * st_n + dc_n + B * H * N}, q);
+    float* carry = fmut(scratch);
+    float *carry_in = carry + st_n, *last = carry_in + st_n, *decay = last + st_n, *total = decay + dc_n;
+    const Workspace ws = workspace(q, cdssm_b200_scan_fused_workspace_bytes((int)R, (int)Ls, (int)H, (int)D, (int)N, (int)C));
+    void* st = stream_of(q);
+    check(cdssm_b200_scan_summary_fwd(cptr(k), cptr(v), cptr(g), fptr(lds), fptr(rope), nullptr, carry, decay, ws.ptr, ws.bytes,
+                                      dyn.c[0], dyn.c[1], dyn.c[2], dyn.c[3], dyn.c[4], (int)R, (int)Ls, (int)H, (int)D, (int)N,
+                                      (int)C, (int)pos0, (int)S, dt, (int)flags & CDSSM_SCAN_FP32_DECAY, st),
+          "scan_summary_fwd");
+    check(cdssm_b200_compose_carries(decay, carry, fptr(h0), carry_in, fmut(final_state), total, (int)B, (int)S, (int)H, (int)D,
+                                     (int)N, S, 1, st),
+          "compose_carries");
+    check(cdssm_b200_scan_fused_segmented_fwd(cptr(q), cptr(k), cptr(v), cptr(g), fptr(lds), fptr(rope), carry_in, mptr(y), last,
+                                              ws.ptr, ws.bytes, dyn.c[0], dyn.c[1], dyn.c[2], dyn.c[3], dyn.c[4], (float)shortcut,
+                                              (int)R, (int)Ls, (int)H, (int)D, (int)N, (int)C, (int)pos0, (int)S, dt,
+                                              (int)flags | CDSSM_SCAN_REUSE_LOCAL, st),
+          "scan_fused_segmented_fwd");
+    return {y, final_state};
+}
+
 Tensor decode_step(const Tensor& state, const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gate_,
                    const Tensor& lds_, const Tensor& rope_, const Dyn& dyn, int64_t heads, int64_t N, int64_t pos,
                    const Tensor& pos_dev, double shortcut, const Tensor& out, const Tensor& v_first_, const Tensor& mix_) {
@@ -275,6 +319,27 @@ PyObject* py_scan_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// scan_fused_long(q, k, v, gate_raw, log_dt_scale, rope_freqs, five dynamics scalars, n_heads, state_dim, chunk_size, h0 or None,
+//                 shortcut_scale, pos0, flags, segments) -> (y, final_state)
+PyObject* py_scan_fused_long(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        Args in{a, n};
+        const Tensor q = in.tensor("q"), k = in.tensor("k"), v = in.tensor("v"), g = in.tensor("gate_raw");
+        const Tensor lds = in.tensor("log_dt_scale"), rope = in.tensor("rope_freqs");
+        const Dyn dyn = in.dyn();
+        const int64_t H = in.integer(), N = in.integer(), C = in.integer();
+        const Tensor h0 = in.tensor_or_none("h0");
+        const double shortcut = in.number();
+        const int64_t pos0 = in.integer(), flags = in.integer(), S = in.integer();
+        const auto o = scan_fused_long(q, k, v, g, lds, rope, dyn, H, N, C, h0, shortcut, pos0, flags, S);
+        PyObject* t = PyTuple_New(2);
+        if (!t) return nullptr;
+        PyTuple_SET_ITEM(t, 0, wrap(o[0]));
+        PyTuple_SET_ITEM(t, 1, wrap(o[1]));
+        return t;
+    });
+}
+
 PyObject* py_rms_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&] {
         Args in{a, n};
@@ -330,6 +395,7 @@ PyObject* py_set_error_type(PyObject*, PyObject* t) {
 PyMethodDef g_methods[] = {
     {"decode_step", FAST(py_decode_step)},
     {"scan_fused", FAST(py_scan_fused)},
+    {"scan_fused_long", FAST(py_scan_fused_long)},
     {"rms_norm", FAST(py_rms_norm)},
     {"groupnorm_gate", FAST(py_groupnorm_gate)},
     {"conv1d_silu_step", FAST(py_conv1d_silu_step)},

@@ -406,6 +406,9 @@ def scan_fused_long(q: Tensor, k: Tensor, v: Tensor, gate_raw: Tensor, log_dt_sc
     seg = lambda t: t.contiguous().view(B * S, Ls, *t.shape[2:])
     consts = (gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps)
     rank, world = sharding.sequence_ranks(sequence_parallel, group)
+    if world == 1 and timings is None and B * L > 0:
+        return _lib.host().scan_fused_long(q, k, v, gate_raw, log_dt_scale, rope_freqs, *consts, n_heads, N, C, h0,
+                                           shortcut_scale, pos0, flags, S)
     if world > 1 and h0 is not None:
         h0 = _prep(h0, dtype=torch.float32, name="h0").clone()
         torch.distributed.broadcast(h0, torch.distributed.get_global_rank(group, 0) if group is not None else 0,
