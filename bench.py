@@ -663,7 +663,7 @@ def main():
                 "gpu_launches": (4 if uses_wa else 3) * args.steps,
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
-                             "kernel": ("the whole step (wa_dynamics + scan_wa local pass + scan_carry + scan_wa output "
+                             "kernel": ("the whole step (records + scan_wa local pass + scan_carry + scan_wa output "
                                         "pass)" if uses_wa else
                                         "the whole step (scan_walk local pass + scan_carry + scan_walk output pass)"),
                              "algorithmic_bytes_per_launch": abytes}}
