@@ -14,12 +14,12 @@
 //     independent of any state (as 8 x 8 halves: seven dependent steps instead of fifteen);
 //   - what is left of the serial chain is three 16-wide products per 32 tokens, passed from warp to warp;
 //   - everything with a right-hand side (cross-block terms, read-outs, K^T g, K r_0, Q r_0) is a product with n = 8
-//     columns {pair 2q: re hi, re lo, im hi, im lo, pair 2q+1: ...}; fp32 values enter as bf16 hi + lo (16 bits), on the
-//     matrix side too, accumulation is fp32.
-// Bounded by the latency of its dependent steps at 15 warps per SM (registers), 46 % of the issue slots busy; a tensor-core
-// generation with tiles of 128 rows has no use for 16-wide products.  Measured on B200, 6144 chunks, D 64, N 16, one kernel:
-// 201 us with one warp per 32 tokens, 178 with two, 162 with the steps of their pairs side by side and the halved inverses
-// (216 chunks, local / output pass: 9.3 / 15.6 -> 6.9 / 10.7 us).
+//     columns {pair 2q: re p1, re p2, im p1, im p2, pair 2q+1: ...} and a second set for p3: a float32 value enters as the
+//     exact sum of three bf16 parts, on the matrix side too; terms below 2^-24 are left out, accumulation is fp32.
+// So the state is as precise as that of a walk in float32 (one chunk: 1.4e-7 of it, the walk 1.1e-7; two parts, 16 bits, left
+// 1.7e-5).  Bounded by issue slots and the latency of its dependent steps at 16 warps per SM (registers); a tensor-core
+// generation with tiles of 128 rows has no use for 16-wide products.  Measured on B200, D 64, N 16, B 8, H 24, 6144 chunks, the
+// whole call: 279 us, 183 with two parts, the walk 540; 216 chunks: 32 us, 26 with two parts, the walk 55.
 // The division by W_i only spans a 32-token block, relative to its middle (|W ratio| of 16 tokens >= 1e-30); values cross
 // blocks relative to the block ends, where all factors are plain products.  A (block, pair) that decays further is walked
 // step by step (slow_walk).
@@ -66,12 +66,10 @@ __device__ __forceinline__ cplx cshfl(cplx v, int src) {
 }
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-// x = hi + lo, hi = x truncated to bf16 and lo the (exact) rest truncated to bf16: 16 significant bits, integer and FMA
-// pipes only.  pair_hi / pair_lo: the two parts of two values; hi_lo: both parts of one value.
+// x = p1 + p2 + p3, each part the next eight significant bits cut off as a bf16: exact, a float has 24.  Integer and FMA pipes
+// only.  pair_hi: the first parts of two values; rest: what is left behind the first part.
 __device__ __forceinline__ uint32_t pair_hi(float x0, float x1) { return __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632); }
 __device__ __forceinline__ float rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
-__device__ __forceinline__ uint32_t pair_lo(float x0, float x1) { return pair_hi(rest(x0), rest(x1)); }
-__device__ __forceinline__ uint32_t hi_lo(float x) { return pair_hi(x, rest(x)); }
 __device__ __forceinline__ uint32_t movmatrix(uint32_t x) {   // 8 x 8 bf16 matrix, one row a quad, transposed
     uint32_t y;
     asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
@@ -79,6 +77,39 @@ __device__ __forceinline__ uint32_t movmatrix(uint32_t x) {   // 8 x 8 bf16 matr
 }
 __device__ __forceinline__ float bits_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ float bits_lo(uint32_t w) { return __uint_as_float(w << 16); }
+
+// A 16 x 16 operand in float32, in the order of two 16 x 8 accumulators, and as A fragments of its three bf16 parts.
+struct Frag { float x[8]; };
+__device__ __forceinline__ Frag frag_of(const float (&n0)[4], const float (&n1)[4]) {
+    return {{n0[0], n0[1], n0[2], n0[3], n1[0], n1[1], n1[2], n1[3]}};
+}
+struct Split { uint32_t p1[4], p2[4], p3[4]; };
+__device__ __forceinline__ Split split(const Frag& f) {
+    Split s;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float r0 = rest(f.x[2 * i]), r1 = rest(f.x[2 * i + 1]);
+        s.p1[i] = pair_hi(f.x[2 * i], f.x[2 * i + 1]);
+        s.p2[i] = pair_hi(r0, r1);
+        s.p3[i] = pair_hi(rest(r0), rest(r1));
+    }
+    return s;
+}
+// B fragments of 16 tokens: ab has columns {p1, p2} of the tile's components, c {p3, 0}.
+struct Rhs { uint2 ab, c; };
+// values of rows g, g + 8 (this lane's complex component)
+__device__ __forceinline__ Rhs rhs_frag(float x0, float x1) {
+    const float r0 = rest(x0), r1 = rest(x1);
+    return {make_uint2(movmatrix(pair_hi(x0, r0)), movmatrix(pair_hi(x1, r1))),
+            make_uint2(movmatrix(pair_hi(rest(r0), 0.f)), movmatrix(pair_hi(rest(r1), 0.f)))};
+}
+// d (+ e) += s f up to 2^-24 of a term; d holds the large terms, e the small ones (may be the same accumulator)
+__device__ __forceinline__ void mma_split(float (&d)[4], float (&e)[4], const Split& s, const Rhs& f) {
+    mma_bf16_m16n8k16(e, s.p3, f.ab.x, f.ab.y);
+    mma_bf16_m16n8k16(e, s.p1, f.c.x, f.c.y);
+    mma_bf16_m16n8k16(d, s.p2, f.ab.x, f.ab.y);
+    mma_bf16_m16n8k16(d, s.p1, f.ab.x, f.ab.y);
+}
 
 template <int kD, int kPairs_>
 struct Geo {
@@ -110,9 +141,9 @@ struct Scratch {   // of one 32-token block, until the Q tile arrives in its pla
             float tri[4][100];                           // [block, half] diagonal ones: column j, row i at 12 j + i
             float low[2][68], inv[2][68];                // [block] the one below, the first half's inverse: 8 i + j
         };
-        unsigned char t[32][80];                         // rows of the inverses, bf16 hi (32 B) | lo (32 B)
+        float t[32][20];                                 // rows of the inverses
     };
-    uint4 m21[2][32];                                    // for the block's other warp: M between its halves, |k|^-1
+    float4 m21[2][32];                                   // for the block's other warp: M between its halves, |k|^-1
     float nrm[32];
 };
 
@@ -120,13 +151,13 @@ struct Scratch {   // of one 32-token block, until the Q tile arrives in its pla
 template <int kD, int kPairs, Mode kMode>
 struct __align__(1024) Smem {
     using G = Geo<kD, kPairs>;
-    static constexpr int kLanes = kPairs == 1 ? 16 : 32; // a single pair fills half of the columns
+    static constexpr int kComps = kPairs == 1 ? 2 : 4;   // complex components of a column tile
     uint8_t k[G::kTile];                                 // swizzled rows = tokens
     union {
         uint8_t q[kMode == kLocal ? 1024 : G::kTile];
         Scratch scr[G::kBlocks];
     };
-    uint2 frag[G::kSlots][G::kTiles][2][kLanes];         // [slot][tile][16-token half][lane]
+    float frag[G::kSlots][G::kTiles][2][16 * kComps];    // [slot][tile][16-token half][component, token]
     float2 viw[kPairs][kD], dd[kPairs][kD];              // v / D, D
     float beta[kD], sel[kD];
     BlockPair bp[kPairs][G::kBlocks];
@@ -140,12 +171,28 @@ struct __align__(1024) Smem {
     uint64_t full_k, full_q;
     int slow[G::kBlocks];                                // pairs that are walked step by step, a bit each
     int abort_flag, item, stop;
-    __device__ __forceinline__ void put(int slot, int tile, int half, int lane, uint2 f) {
-        if (kLanes == 32 || lane < 16) frag[slot][tile][half][lane & (kLanes - 1)] = f;
+    // (the tokens of components 2 and 3 are turned by eight: a store's lanes then hit distinct banks)
+    static __device__ __forceinline__ int at(int comp, int token) { return comp * 16 + (token ^ ((comp >> 1) * 8)); }
+    // values of tokens g, g + 8 of a half, this lane's component
+    __device__ __forceinline__ void put(int slot, int tile, int half, int lane, float x0, float x1) {
+        const int g = lane >> 2, comp = lane & 3;
+        if (kComps == 4 || comp < kComps) {
+            frag[slot][tile][half][at(comp, g)] = x0;
+            frag[slot][tile][half][at(comp, g + 8)] = x1;
+        }
     }
-    __device__ __forceinline__ uint2 get(int slot, int tile, int half, int lane) const {
-        const uint2 f = frag[slot][tile][half][lane & (kLanes - 1)];
-        return kLanes == 32 || lane < 16 ? f : make_uint2(0u, 0u);
+    __device__ __forceinline__ Rhs get(int slot, int tile, int half, int lane) const {
+        const int g = lane >> 2, comp = g >> 1, token = 2 * (lane & 3);
+        Rhs f = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
+        if (kComps == 4 || comp < kComps) {
+            const float2 x0 = *reinterpret_cast<const float2*>(&frag[slot][tile][half][at(comp, token)]);
+            const float2 x1 = *reinterpret_cast<const float2*>(&frag[slot][tile][half][at(comp, token + 8)]);
+            const float2 r0 = make_float2(rest(x0.x), rest(x0.y)), r1 = make_float2(rest(x1.x), rest(x1.y));
+            const bool first = (g & 1) == 0;
+            f.ab = first ? make_uint2(pair_hi(x0.x, x0.y), pair_hi(x1.x, x1.y)) : make_uint2(pair_hi(r0.x, r0.y), pair_hi(r1.x, r1.y));
+            f.c = first ? make_uint2(pair_hi(rest(r0.x), rest(r0.y)), pair_hi(rest(r1.x), rest(r1.y))) : make_uint2(0u, 0u);
+        }
+        return f;
     }
 };
 
@@ -204,22 +251,6 @@ __device__ __forceinline__ void diagonal_of(const float (&n0)[4], const float (&
     d1 = __shfl_sync(0xffffffffu, x1, src);
 }
 
-struct Split { uint32_t hi[4], lo[4]; };   // a 16 x 16 A fragment, bf16 hi + lo
-__device__ __forceinline__ Split split(const float (&n0)[4], const float (&n1)[4]) {
-    Split s;
-    s.hi[0] = pair_hi(n0[0], n0[1]); s.lo[0] = pair_lo(n0[0], n0[1]);
-    s.hi[1] = pair_hi(n0[2], n0[3]); s.lo[1] = pair_lo(n0[2], n0[3]);
-    s.hi[2] = pair_hi(n1[0], n1[1]); s.lo[2] = pair_lo(n1[0], n1[1]);
-    s.hi[3] = pair_hi(n1[2], n1[3]); s.lo[3] = pair_lo(n1[2], n1[3]);
-    return s;
-}
-__device__ __forceinline__ void mma_split(float (&d)[4], const Split& a, uint2 b) {
-    mma_bf16_m16n8k16(d, a.hi, b.x, b.y);
-    mma_bf16_m16n8k16(d, a.lo, b.x, b.y);
-}
-// values of rows g, g + 8 (this lane's complex component) as the B fragment of 16 tokens
-__device__ __forceinline__ uint2 rhs_frag(float x0, float x1) { return make_uint2(movmatrix(hi_lo(x0)), movmatrix(hi_lo(x1))); }
-
 // ---- decay scalings of a 32-token block and pair (lane = token) ---------------------------------------------------
 // The scaled unknowns need ratios of the prefix products W_t = a_0 ... a_t only, taken relative to the middle of the
 // block, D_t = W_t / W_15: lanes 0-15 hold the suffix product a_{t+1} ... a_15 = 1 / D_t, lanes 16-31 the prefix product
@@ -249,12 +280,12 @@ __device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, 
         if (tl == 15) E = {1.f, 0.f};
         if (!lo) E = X[w];
         const float m = fmaxf(fabsf(E.r), fabsf(E.i));
-        const bool in_range = m >= 1e-30f && m <= 1e30f;
-        const float sc1 = __fdividef(1.f, m);
+        const float sc1 = __frcp_rn(m);
         const cplx En = {E.r * sc1, E.i * sc1};
-        const float q = __fdividef(sc1, En.r * En.r + En.i * En.i);
+        const float q = sc1 * __frcp_rn(En.r * En.r + En.i * En.i);
         const cplx Einv = {En.r * q, -En.i * q};
         const cplx D = lo ? Einv : E, v = cmul(vg[w], lo ? E : Einv);
+        const bool in_range = m >= 1e-30f && m <= 1e30f && fabsf(v.r) <= 1e33f && fabsf(v.i) <= 1e33f;   // (false for NaN)
         const cplx D31 = cshfl(D, 31);
         const float mr = fmaxf(fabsf(R.r), fabsf(R.i));
         const bool fast = __all_sync(0xffffffffu, in_range && mr >= 1e-30f && mr <= 1e30f);
@@ -287,14 +318,9 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int I
     for (int J = 0; J < I; J++)
 #pragma unroll 4
         for (int t = 0; t < 32; t++) {
-            const int half = t >> 4, r = t & 15, q = (r & 7) >> 1;
-            auto value = [&](int col) {
-                const uint2 f = sm.get(G::slot_g(J, I), p >> 1, half, col * 4 + q);
-                const uint32_t w = r >= 8 ? f.y : f.x;
-                return (r & 1) ? bits_hi(w) : bits_lo(w);
-            };
-            const int c0 = 4 * (p & 1);
-            const float wr = value(c0) + value(c0 + 1), wi = value(c0 + 2) + value(c0 + 3);
+            const float* f = sm.frag[G::slot_g(J, I)][p >> 1][t >> 4];
+            const int comp = 2 * (p & 1);
+            const float wr = f[sm.at(comp, t & 15)], wi = f[sm.at(comp + 1, t & 15)];
 #pragma unroll
             for (int i = 0; i < kCols; i++) {
                 const float k = column(sm.k, 32 * J + t, tl + 32 * i);
@@ -370,7 +396,8 @@ __device__ __forceinline__ float next_im(cplx g, float sr, float si, float l) {
     return __fadd_rn(__fmaf_rn(g.r, si, __fmul_rn(g.i, sr)), l);
 }
 
-// resident blocks per SM the registers are cut for (one more spills: N 16, head_dim 64, 4 / 5 blocks: 178 / 203 us)
+// resident blocks per SM the registers are cut for (N 16, head_dim 64, 4 / 3 blocks: 285 / 284 us with 6144 chunks, 111 / 119
+// with 1692, where a chain of chunks waits)
 template <int kD, int kPairs>
 constexpr int kMinBlocks = kD == 128 ? (kPairs == 1 ? 3 : 2) : (kPairs <= 2 ? 6 : 4);
 
@@ -470,8 +497,8 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 
     // ---- G: diagonal block, |k|^-1, inverses
     float cc[4], bn[4], nrm[4];               // c_t, beta_t n_t, n_t of rows g, g + 8, g + 16, g + 24
-    Split T11, T22, M21;
-    Split M[kBlocks > 1 ? kBlocks - 1 : 1][2][2];
+    Frag T11, T22, M21;
+    Frag M[kBlocks > 1 ? kBlocks - 1 : 1][2][2];
     {
         float acc[2][4][4], kk[4];
         if (first_warp) {
@@ -541,10 +568,10 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             for (int n = 0; n < 2; n++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) acc[1][n][e] *= cc[2 + (e >> 1)];
-            M21 = split(acc[1][0], acc[1][1]);
+            M21 = frag_of(acc[1][0], acc[1][1]);
             if (kSplit > 1) {
-                sm.scr[I].m21[0][tl] = make_uint4(M21.hi[0], M21.hi[1], M21.hi[2], M21.hi[3]);
-                sm.scr[I].m21[1][tl] = make_uint4(M21.lo[0], M21.lo[1], M21.lo[2], M21.lo[3]);
+                sm.scr[I].m21[0][tl] = make_float4(M21.x[0], M21.x[1], M21.x[2], M21.x[3]);
+                sm.scr[I].m21[1][tl] = make_float4(M21.x[4], M21.x[5], M21.x[6], M21.x[7]);
                 if (t4 == 0) {
 #pragma unroll
                     for (int r = 0; r < 4; r++) sm.scr[I].nrm[8 * r + g] = nrm[r];
@@ -603,14 +630,9 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 R[4 + j] = half == 0 ? make_float2(0.f, 0.f) : T2[j];
             }
             __syncwarp();
-            uint32_t* row = reinterpret_cast<uint32_t*>(sm.scr[I].t[tl]);
+            float4* row = reinterpret_cast<float4*>(sm.scr[I].t[tl]);
 #pragma unroll
-            for (int j = 0; j < 8; j += 4) {
-                *reinterpret_cast<uint4*>(row + j) = make_uint4(pair_hi(R[j].x, R[j].y), pair_hi(R[j + 1].x, R[j + 1].y),
-                                                                pair_hi(R[j + 2].x, R[j + 2].y), pair_hi(R[j + 3].x, R[j + 3].y));
-                *reinterpret_cast<uint4*>(row + 8 + j) = make_uint4(pair_lo(R[j].x, R[j].y), pair_lo(R[j + 1].x, R[j + 1].y),
-                                                                    pair_lo(R[j + 2].x, R[j + 2].y), pair_lo(R[j + 3].x, R[j + 3].y));
-            }
+            for (int j = 0; j < 4; j++) row[j] = make_float4(R[2 * j].x, R[2 * j].y, R[2 * j + 1].x, R[2 * j + 1].y);
             __syncwarp();
         }
         if (kSplit > 1) {
@@ -622,15 +644,22 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     bn[r] = sm.beta[32 * I + 8 * r + g] * nrm[r];
                     cc[r] = bn[r] * nrm[r];
                 }
-                const uint4 hi = sm.scr[I].m21[0][tl], lo = sm.scr[I].m21[1][tl];
-                M21 = {{hi.x, hi.y, hi.z, hi.w}, {lo.x, lo.y, lo.z, lo.w}};
+                const float4 x = sm.scr[I].m21[0][tl], y = sm.scr[I].m21[1][tl];
+                M21 = {{x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w}};
             }
         }
-        const uint32_t ts = smem_u32(sm.scr[I].t) + (uint32_t)((tl & 7) + ((tl >> 3) & 1) * 8) * 80u + (uint32_t)(tl >> 4) * 16u;
-        ldsm_x4(ts, T11.hi);
-        ldsm_x4(ts + 32, T11.lo);
-        ldsm_x4(ts + 16 * 80, T22.hi);
-        ldsm_x4(ts + 16 * 80 + 32, T22.lo);
+        auto half = [&](int r0) {
+            Frag f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 x = *reinterpret_cast<const float2*>(&sm.scr[I].t[r0 + g + 8 * (i & 1)][2 * t4 + 8 * (i >> 1)]);
+                f.x[2 * i] = x.x;
+                f.x[2 * i + 1] = x.y;
+            }
+            return f;
+        };
+        T11 = half(0);
+        T22 = half(16);
     }
     // (block decays of all warps are in shared memory; the scratch has been read: the Q tile comes in its place)
     fence_proxy_async();
@@ -654,51 +683,51 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 for (int n = 0; n < 4; n++)
 #pragma unroll
                     for (int e = 0; e < 4; e++) acc[m][n][e] *= cc[2 * m + (e >> 1)];
-                M[J][m][0] = split(acc[m][0], acc[m][1]);
-                M[J][m][1] = split(acc[m][2], acc[m][3]);
+                M[J][m][0] = frag_of(acc[m][0], acc[m][1]);
+                M[J][m][1] = frag_of(acc[m][2], acc[m][3]);
             }
         }
     auto tile = [&](int q) { return S * kOwn + q; };
-    // x <- (I + M_own)^-1 rhs for one column tile; f: the solution as B fragments of the two 16-token halves
-    auto solve = [&](float (&x)[4], uint2 (&f)[2]) {
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_split(d, T11, rhs_frag(x[0], x[1]));
-        x[0] = d[0] + d[1];
-        x[1] = d[2] + d[3];
-        f[0] = rhs_frag(x[0], x[1]);
-        float e[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_split(e, M21, f[0]);
-        x[2] -= e[0] + e[1];
-        x[3] -= e[2] + e[3];
-        float h[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_split(h, T22, rhs_frag(x[2], x[3]));
-        x[2] = h[0] + h[1];
-        x[3] = h[2] + h[3];
-        f[1] = rhs_frag(x[2], x[3]);
+    // sums of a tile's accumulators: rows g and g + 8, this lane's component
+    auto sum_lo = [](const float (&d)[4], const float (&e)[4]) { return (d[0] + d[1]) + (e[0] + e[1]); };
+    auto sum_hi = [](const float (&d)[4], const float (&e)[4]) { return (d[2] + d[3]) + (e[2] + e[3]); };
+    // x <- (I + M_own)^-1 x, all column tiles
+    auto solve = [&](float (&x)[kOwn][4]) {
+        auto apply = [&](const Frag& f, int from, auto&& use) {
+            const Split s = split(f);
+#pragma unroll
+            for (int q = 0; q < kOwn; q++) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_split(d, e, s, rhs_frag(x[q][from], x[q][from + 1]));
+                use(x[q], sum_lo(d, e), sum_hi(d, e));
+            }
+        };
+        apply(T11, 0, [](float (&v)[4], float lo, float hi) { v[0] = lo; v[1] = hi; });
+        apply(M21, 0, [](float (&v)[4], float lo, float hi) { v[2] -= lo; v[3] -= hi; });
+        apply(T22, 2, [](float (&v)[4], float lo, float hi) { v[2] = lo; v[3] = hi; });
     };
     // sum over the earlier blocks of M times their published fragments, subtracted from the right-hand sides
     auto subtract_earlier = [&](int J, int slot, float (&x)[kOwn][4]) {
 #pragma unroll
-        for (int q = 0; q < kOwn; q++) {
-            float d[2][4];
+        for (int m = 0; m < 2; m++) {
+            float d[kOwn][4], e[kOwn][4];
 #pragma unroll
-            for (int m = 0; m < 2; m++)
+            for (int q = 0; q < kOwn; q++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) d[m][e] = 0.f;
+                for (int i = 0; i < 4; i++) d[q][i] = e[q][i] = 0.f;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const uint2 f = sm.get(slot, tile(q), h, tl);
+            for (int h = 0; h < 2; h++)
 #pragma unroll
-                for (int m = 0; m < 2; m++) {
+                for (int JJ = 0; JJ < kBlocks - 1; JJ++)
+                    if (JJ == J) {
+                        const Split s = split(M[JJ][m][h]);
 #pragma unroll
-                    for (int JJ = 0; JJ < kBlocks - 1; JJ++)
-                        if (JJ == J) mma_split(d[m], M[JJ][m][h], f);
-                }
-            }
+                        for (int q = 0; q < kOwn; q++) mma_split(d[q], e[q], s, sm.get(slot, tile(q), h, tl));
+                    }
 #pragma unroll
-            for (int m = 0; m < 2; m++) {
-                x[q][2 * m] -= d[m][0] + d[m][1];
-                x[q][2 * m + 1] -= d[m][2] + d[m][3];
+            for (int q = 0; q < kOwn; q++) {
+                x[q][2 * m] -= sum_lo(d[q], e[q]);
+                x[q][2 * m + 1] -= sum_hi(d[q], e[q]);
             }
         }
     };
@@ -712,7 +741,6 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 
     const int slow = sm.slow[I] & (((1 << G::kOwnPairs) - 1) << (G::kOwnPairs * S));   // of this warp's pairs
     // ---- g: the chain over the blocks of the chunk
-    uint2 gf[kOwn][2];                       // own block's g / D
     float gx[kOwn][4];
     {
 #pragma unroll
@@ -728,8 +756,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + S * (kBlocks - 1) + J), "r"(32 * (kBlocks - J)) : "memory");
                 subtract_earlier(J, G::slot_g(J, I), gx);
             }
-#pragma unroll
-        for (int q = 0; q < kOwn; q++) solve(gx[q], gf[q]);
+        solve(gx);
         float w[kOwn][4];                      // g carried to the block end
 #pragma unroll
         for (int q = 0; q < kOwn; q++) {
@@ -779,8 +806,8 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     if (!end || kNeedEnd || a.tail_state) {
                         const cplx ff = end ? f : cmul(f, sm.bp[p][to < kBlocks ? to : 0].R);
                         const int slot = end ? G::slot_end(I) : G::slot_g(I, to);
-                        sm.put(slot, tile(q), 0, tl, rhs_frag(rotate(ff, w[q][0], wo[0]), rotate(ff, w[q][1], wo[1])));
-                        sm.put(slot, tile(q), 1, tl, rhs_frag(rotate(ff, w[q][2], wo[2]), rotate(ff, w[q][3], wo[3])));
+                        sm.put(slot, tile(q), 0, tl, rotate(ff, w[q][0], wo[0]), rotate(ff, w[q][1], wo[1]));
+                        sm.put(slot, tile(q), 1, tl, rotate(ff, w[q][2], wo[2]), rotate(ff, w[q][3], wo[3]));
                     }
                     if (!end) f = cmul(f, sm.bp[p][to < kBlocks ? to : 0].A);
                 }
@@ -790,10 +817,9 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (slow != 0) {                       // a slow pair takes no part in the scaled read-out
 #pragma unroll
             for (int q = 0; q < kOwn; q++) {
-                const bool mine = (slow >> pair_of(q)) & 1, col = (slow >> column_pair(q)) & 1;   // this lane's row, fragment column
+                const bool mine = (slow >> pair_of(q)) & 1;
 #pragma unroll
                 for (int r = 0; r < 4; r++) gx[q][r] = mine ? 0.f : gx[q][r];
-                if (col) gf[q][0] = gf[q][1] = make_uint2(0u, 0u);
             }
         }
     }
@@ -809,12 +835,13 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int J = 0; J < kBlocks; J++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const uint2 f = sm.get(slot0 + J, tile(q), h, tl);
+                const Rhs f = sm.get(slot0 + J, tile(q), h, tl);
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
                     uint32_t ka[4];
                     ldsm_x4_trans(col_frag<G::kSlab>(kt, 32 * J + 16 * h, 32 * I + 16 * m, tl), ka);
-                    mma_bf16_m16n8k16(d[m], ka, f.x, f.y);
+                    mma_bf16_m16n8k16(d[m], ka, f.c.x, f.c.y);
+                    mma_bf16_m16n8k16(d[m], ka, f.ab.x, f.ab.y);
                 }
             }
     };
@@ -997,12 +1024,11 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + S * (kBlocks - 1) + J), "r"(32 * (kBlocks - J)) : "memory");
                 subtract_earlier(J, G::slot_h(J), hx);
             }
+        solve(hx);
 #pragma unroll
         for (int q = 0; q < kOwn; q++) {
-            uint2 f[2];
-            solve(hx[q], f);
-            sm.put(G::slot_h(I), tile(q), 0, tl, f[0]);
-            sm.put(G::slot_h(I), tile(q), 1, tl, f[1]);
+            sm.put(G::slot_h(I), tile(q), 0, tl, hx[q][0], hx[q][1]);
+            sm.put(G::slot_h(I), tile(q), 1, tl, hx[q][2], hx[q][3]);
         }
         if (I < kBlocks - 1) asm volatile("bar.arrive %0, %1;" ::"r"(1 + S * (kBlocks - 1) + I), "r"(32 * (kBlocks - I)) : "memory");
         __syncwarp();
@@ -1072,22 +1098,22 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const Split p0 = split(acc[0][2 * h], acc[0][2 * h + 1]), p1 = split(acc[1][2 * h], acc[1][2 * h + 1]);
+            const Split p0 = split(frag_of(acc[0][2 * h], acc[0][2 * h + 1])), p1 = split(frag_of(acc[1][2 * h], acc[1][2 * h + 1]));
 #pragma unroll
             for (int q = 0; q < kOwn; q++) {
-                const uint2 fg = diag ? gf[q][h] : sm.get(G::slot_g(J, I), tile(q), h, tl);
-                const uint2 fh = sm.get(G::slot_h(J), tile(q), h, tl);
+                const Rhs fg = diag ? rhs_frag(gx[q][2 * h], gx[q][2 * h + 1]) : sm.get(G::slot_g(J, I), tile(q), h, tl);
+                const Rhs fh = sm.get(G::slot_h(J), tile(q), h, tl);
                 float dz[2][4], dh[2][4];
 #pragma unroll
                 for (int m = 0; m < 2; m++)
 #pragma unroll
                     for (int e = 0; e < 4; e++) dz[m][e] = dh[m][e] = 0.f;
                 if (!(diag && h == 1)) {
-                    mma_split(dz[0], p0, fg);
-                    mma_split(dh[0], p0, fh);
+                    mma_split(dz[0], dz[0], p0, fg);
+                    mma_split(dh[0], dh[0], p0, fh);
                 }
-                mma_split(dz[1], p1, fg);
-                mma_split(dh[1], p1, fh);
+                mma_split(dz[1], dz[1], p1, fg);
+                mma_split(dh[1], dh[1], p1, fh);
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
                     oz[q][r] += dz[r >> 1][2 * (r & 1)] + dz[r >> 1][2 * (r & 1) + 1];

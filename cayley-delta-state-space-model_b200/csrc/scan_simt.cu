@@ -797,7 +797,7 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
 bool scan_wa_supported(int D, int N, int C, int H, int dtype);
 int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
-                 int from_chunks, const float* h0, float* final_state, cudaStream_t st);
+                 int from_chunks, const float* h0, float* final_state, int parts, cudaStream_t st);
 // scan_chunk.cu
 bool scan_chunk_supported(int D, int N, int C, int dtype);
 int scan_chunk_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
@@ -923,6 +923,8 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
                        ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > 40 || (long long)B * a.NC * H > (D == 64 ? (a.NC <= 6 ? 1536 : 640) : 256));
     const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
     if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && !wa_ok) return CDSSM_ERR_UNSUPPORTED;
+    // (who keeps the state after the last token gets the precision of the CUDA-core walk, which these calls took before)
+    const int wa_parts = tail_state == nullptr || (flags & CDSSM_SCAN_TENSOR_CORE_WA) ? 2 : 3;
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
     const bool one_kernel = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && ((uintptr_t)h0 & 15) == 0 &&
                             one_kernel_pays(B, H, a.NC, D, N);
@@ -965,7 +967,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
-                                limit, withhold, from_chunks, h0, final_state, st);
+                                limit, withhold, from_chunks, h0, final_state, wa_parts, st);
         return scan_chunk_pass(mode, from_chunks, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
                                shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };

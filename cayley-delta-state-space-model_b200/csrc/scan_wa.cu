@@ -438,6 +438,11 @@ __device__ __forceinline__ uint32_t split_pack(float x0, float x1, bool low) {
     const float r1 = x1 - __uint_as_float(__float_as_uint(x1) & m);
     return __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);   // {r1[31:16], r0[31:16]}
 }
+// The pair of what hi + lo leave behind: with it the split is exact (a float has 24 significant bits).
+__device__ __forceinline__ uint32_t third_pack(float x0, float x1) {
+    const float r0 = x0 - __uint_as_float(__float_as_uint(x0) & 0xffff0000u), r1 = x1 - __uint_as_float(__float_as_uint(x1) & 0xffff0000u);
+    return split_pack(r0, r1, true);
+}
 
 // The carry into a chunk of head hd, rounded: s <- gamma s + z over the chunks before, evaluated as the carry pass does; a lane
 // has kD / 32 columns.  out: its real, then its imaginary row.
@@ -498,7 +503,11 @@ __device__ __forceinline__ void carry_from_chunks(const Args& a, const ItemPos& 
     __syncwarp();
 }
 
-template <int kD, bool kOutput>
+// kParts: parts of the split of the state and of the update's coefficients, 2 or 3.  Two carry 16 bits, 1.7e-5 of the state after
+// a chunk, far below the bf16 results; three are exact, 1.5e-7 after a chunk like a walk in float32, for a caller who keeps the
+// float32 state after the last token.  us on B200, two / three parts, D 64: 936 chunks 22 / 25, 6144 74 / 96; a third more on
+// average.
+template <int kD, bool kOutput, int kParts>
 __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     using DM = Dims<kD>;
     using TC = Cols<kOutput>;
@@ -593,6 +602,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             bfrag[ks][0] = split_pack(S[ks][0], S[ks][1], low);
             bfrag[ks][1] = split_pack(S[ks][2], S[ks][3], low);
         }
+        auto third = [&](float x0, float x1) { return low ? 0u : third_pack(x0, x1); };
         WA_STAMP(12);
         float ak[2][4], aq[2][4], qa[2][4], qb[2][4];
 #pragma unroll
@@ -615,6 +625,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 }
 #pragma unroll
                 for (int mt = 0; mt < 2; mt++) {
+                    if (kParts == 3) mma_bf16_m16n8k16(aq[mt], fq[cb][mt], third(S[ks][0], S[ks][1]), third(S[ks][2], S[ks][3]));
                     mma_bf16_m16n8k16(aq[mt], fq[cb][mt], bfrag[ks][0], bfrag[ks][1]);
                     mma_bf16_m16n8k16(qa[mt], fq[cb][mt], fq[cb][mt][0], fq[cb][mt][2]);   // rows x tokens 0-7
                     mma_bf16_m16n8k16(qb[mt], fq[cb][mt], fq[cb][mt][1], fq[cb][mt][3]);   // rows x tokens 8-15
@@ -637,6 +648,11 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 if (ks + 1 < kKs) {
                     ldsm_x4(frag_addr(ktile[st], 0, ks + 1), fa[nb][0]);
                     ldsm_x4(frag_addr(ktile[st], 1, ks + 1), fa[nb][1]);
+                }
+                if (kParts == 3) {
+                    const uint32_t t0 = third(S[ks][0], S[ks][1]), t1 = third(S[ks][2], S[ks][3]);
+                    mma_bf16_m16n8k16(ak[0], fa[cb][0], t0, t1);
+                    mma_bf16_m16n8k16(ak[1], fa[cb][1], t0, t1);
                 }
                 mma_bf16_m16n8k16(ak[0], fa[cb][0], bfrag[ks][0], bfrag[ks][1]);
                 mma_bf16_m16n8k16(ak[1], fa[cb][1], bfrag[ks][0], bfrag[ks][1]);
@@ -770,7 +786,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             }
             __syncwarp();
             // A fragments: row grp (and its duplicate) carries the high parts of omega[n'], row grp + 8 the low parts
-            uint32_t fo[2][4];
+            uint32_t fo[2][4], fo3[2][4];
 #pragma unroll
             for (int kk = 0; kk < 2; kk++) {
                 float2 x0 = make_float2(0.f, 0.f), x1 = x0;
@@ -782,6 +798,9 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 fo[kk][1] = split_pack(x0.x, x0.y, true);
                 fo[kk][2] = split_pack(x1.x, x1.y, false);
                 fo[kk][3] = split_pack(x1.x, x1.y, true);
+                fo3[kk][0] = fo3[kk][2] = 0u;
+                fo3[kk][1] = third_pack(x0.x, x0.y);
+                fo3[kk][3] = third_pack(x1.x, x1.y);
             }
             WA_STAMP(9);
             // decay: complex product with W_31; the other part of the complex row sits eight lanes away
@@ -806,6 +825,10 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 float c0[4] = {S[ks][0], S[ks][1], 0.f, 0.f}, c1[4] = {S[ks][2], S[ks][3], 0.f, 0.f};
 #pragma unroll
                 for (int kk = 0; kk < 2; kk++) {
+                    if (kParts == 3) {
+                        mma_bf16_m16n8k16(c0, fo3[kk], fb[cb][kk][0], fb[cb][kk][1]);
+                        mma_bf16_m16n8k16(c1, fo3[kk], fb[cb][kk][2], fb[cb][kk][3]);
+                    }
                     mma_bf16_m16n8k16(c0, fo[kk], fb[cb][kk][0], fb[cb][kk][1]);
                     mma_bf16_m16n8k16(c1, fo[kk], fb[cb][kk][2], fb[cb][kk][3]);
                 }
@@ -853,7 +876,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     if (code && tl == 0) atomicCAS(a.status, 0, 200 + code);
 }
 
-template <int kD, bool kOutput>
+template <int kD, bool kOutput, int kParts>
 __global__ void __launch_bounds__(kThreads, kOutput ? 2 : (kD == 128 ? 3 : 4))
 scan_wa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -877,7 +900,7 @@ scan_wa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     if (warp < 4) {
-        compute<kD, kOutput>(sm, a);
+        compute<kD, kOutput, kParts>(sm, a);
     } else {
         if (threadIdx.x == 128) {
             prefetch_tmap(&tmK);
@@ -900,18 +923,22 @@ scan_wa_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 #ifdef CDSSM_WA_TRACE
 static int g_grid_override = 0;
 #endif
-template <int kD, bool kOutput> struct KernelTag {};
-template <int kD, bool kOutput>
+template <int kD, bool kOutput, int kParts> struct KernelTag {};
+template <int kD, bool kOutput, int kParts>
 static int launch_pass(const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, int sms, cudaStream_t st) {
     constexpr int kBlocksPerSm = kOutput ? 2 : (kD == 128 ? 3 : 4);
     const size_t smem = sizeof(Smem<kD, kOutput>);
-    if (int rc = allow_smem<KernelTag<kD, kOutput>>((const void*)scan_wa_kernel<kD, kOutput>, smem)) return rc;
+    if (int rc = allow_smem<KernelTag<kD, kOutput, kParts>>((const void*)scan_wa_kernel<kD, kOutput, kParts>, smem)) return rc;
     long long resident = (long long)kBlocksPerSm * sms;
 #ifdef CDSSM_WA_TRACE
     if (g_grid_override > 0) resident = g_grid_override;
 #endif
     const int grid = (int)(a.items < resident ? a.items : resident);
-    return launch_overlapped(scan_wa_kernel<kD, kOutput>, dim3(grid), dim3(kThreads), smem, st, tmK, tmQ, a);
+    return launch_overlapped(scan_wa_kernel<kD, kOutput, kParts>, dim3(grid), dim3(kThreads), smem, st, tmK, tmQ, a);
+}
+template <int kD, int kParts>
+static int launch_parts(bool output, const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, int sms, cudaStream_t st) {
+    return output ? launch_pass<kD, true, kParts>(tmK, tmQ, a, sms, st) : launch_pass<kD, false, kParts>(tmK, tmQ, a, sms, st);
 }
 
 }  // namespace wa
@@ -930,10 +957,10 @@ bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
 // One pass of the warp-autonomous tensor-core scan over every chunk.  output = false: local pass (fills
 // ws_state / ws_gamma for the carry pass); output = true: reads the carries from ws_state (from_chunks: adds them up from the
 // local pass of this call), writes y.
-// status: one int in device memory, set by a bounded wait that ran out (not cleared here).
+// status: one int in device memory, set by a bounded wait that ran out (not cleared here).  parts: see compute().
 int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
-                 int from_chunks, const float* h0, float* final_state, cudaStream_t st) {
+                 int from_chunks, const float* h0, float* final_state, int parts, cudaStream_t st) {
     using namespace wa;
     CUtensorMap tmK, tmQ;
     if (!make_tile_map(&tmK, k, k_rs, B, L, H, D, kSub) || !make_tile_map(&tmQ, output ? q : k, output ? q_rs : k_rs, B, L, H, D, kSub)) return CDSSM_ERR_CUDA;
@@ -955,8 +982,8 @@ int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long
     const long long items = (long long)B * a.NC * a.HG;
     if (items > 0x7fffffff / 8) return CDSSM_ERR_UNSUPPORTED;
     a.items = (int)items;
-    if (D == 128) return output ? launch_pass<128, true>(tmK, tmQ, a, sms, st) : launch_pass<128, false>(tmK, tmQ, a, sms, st);
-    return output ? launch_pass<64, true>(tmK, tmQ, a, sms, st) : launch_pass<64, false>(tmK, tmQ, a, sms, st);
+    if (parts == 3) return D == 128 ? launch_parts<128, 3>(output, tmK, tmQ, a, sms, st) : launch_parts<64, 3>(output, tmK, tmQ, a, sms, st);
+    return D == 128 ? launch_parts<128, 2>(output, tmK, tmQ, a, sms, st) : launch_parts<64, 2>(output, tmK, tmQ, a, sms, st);
 }
 
 }  // namespace cdssm

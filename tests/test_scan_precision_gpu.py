@@ -1,0 +1,54 @@
+"""What the tensor-core scans promise beyond closeness: float32 states where a float32 state is handed out, the same bits for a
+shard or a piece as for the whole, and no token touched by one behind it."""
+import numpy as np
+import pytest
+import torch
+
+from test_scan_gpu import run_fused, unnormalise
+from util import to_dev, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(orc, B, H, L, D, N, seed):
+    inp = unnormalise(orc.make_inputs(B, H, L, D, N=N, seed=seed, bf16=True, context_length=max(L, 2)), np.random.default_rng(seed))
+    inp["q"], inp["k"] = orc.bf16_round(inp["q"]), orc.bf16_round(inp["k"])
+    return inp
+
+
+def _cut(inp, rows=slice(None), tokens=slice(None)):
+    return {k: (v[rows, tokens] if getattr(v, "ndim", 0) >= 3 else v) for k, v in inp.items()}
+
+
+def _state64(ops, inp, N):
+    """The recurrent state after a single chunk in float64, from the package's own (bf16) dynamics."""
+    c = inp["consts"]
+    args = (c["gating_c"], c["omega_thresh"], c["adt_delta"], c["adt_smoothness"], c["adt_eps"])
+    k = to_dev(inp["k"], torch.float64)
+    B, L, H, D = k.shape
+    A, vp, beta, _ = ops.DynamicsFusedFn.apply(to_dev(inp["gate_raw"], torch.bfloat16), to_dev(inp["log_dt_scale"], torch.float32),
+                                               to_dev(inp["rope_freqs"], torch.float32), *args, H, N)
+    v = (to_dev(inp["v"], torch.bfloat16) * vp.repeat_interleave(2, -1)).double()
+    z = torch.zeros(B, H, N, D, dtype=torch.float64, device="cuda")
+    for t in range(L):
+        kn = (k[:, t] / (k[:, t].square().sum(-1, keepdim=True) + 1e-6).sqrt())[:, :, None]
+        b = beta[:, t].double()[..., None, None]
+        z = z - b * (z * kn).sum(-1, keepdim=True) * kn
+        re, im = (A[:, t].double()[..., i::2, None] for i in (0, 1))
+        z = torch.stack([re * z[:, :, 0::2] - im * z[:, :, 1::2], re * z[:, :, 1::2] + im * z[:, :, 0::2]], 3).flatten(2, 3)
+        z = z + b * v[:, t][..., None] * kn
+    return z
+
+
+@pytest.mark.parametrize("H,D,N", [(8, 64, 2), (6, 64, 2), (4, 128, 2), (3, 64, 4), (3, 64, 8), (3, 64, 16), (2, 128, 4), (2, 128, 8),
+                                   (2, 128, 16)])
+def test_tail_state_has_float32_precision(ops, orc, H, D, N):
+    """One chunk: nothing between the inputs and the state is rounded.  A chain of D float32 steps is off by a few times
+    sqrt(D) 2^-24 = 7e-7 of the state at D = 128; products of 16-bit parts left 1.7e-5.  (The median over the heads: where
+    the dynamics of the two sides round one bf16 value differently, a head moves by more.)"""
+    B, L = 6, D - 3
+    inp = _inputs(orc, B, H, L, D, N, seed=D + N)
+    _, _, tail = run_fused(ops, inp, torch.bfloat16, N, D, return_tail_state=True)
+    want = _state64(ops, inp, N)
+    err = (tail.double() - want).flatten(2).norm(dim=-1) / want.flatten(2).norm(dim=-1)
+    assert float(err.median()) <= 2e-6
