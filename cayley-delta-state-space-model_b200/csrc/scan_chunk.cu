@@ -1,4 +1,5 @@
-// The scan on tensor cores: bf16 storage, head_dim D = chunk C in {64, 128}, any even state_dim N <= 16, any head count.
+// The scan on tensor cores: bf16 storage, head_dim D = chunk C in {64, 128}, any even state_dim 2 < N <= 16, any
+// head count.
 //
 // One thread block owns one chunk of one head; a warp (head_dim 64 and N > 4: two warps, half of the pairs each) its 32-token
 // block.  With g_t the coefficient that the step at
@@ -57,6 +58,7 @@ struct Args {
     float shortcut_scale;
     int from_chunks;             // kOutput: the carry from the local results of the chunks before (no carry pass has run)
     int B, L, H, N, NC;
+    int groups;                  // blocks that share a chunk of a head: kPairs pairs each
 };
 
 struct cplx { float r, i; };
@@ -151,13 +153,12 @@ struct Scratch {   // of one 32-token block, until the Q tile arrives in its pla
 template <int kD, int kPairs, Mode kMode>
 struct __align__(1024) Smem {
     using G = Geo<kD, kPairs>;
-    static constexpr int kComps = kPairs == 1 ? 2 : 4;   // complex components of a column tile
     uint8_t k[G::kTile];                                 // swizzled rows = tokens
     union {
         uint8_t q[kMode == kLocal ? 1024 : G::kTile];
         Scratch scr[G::kBlocks];
     };
-    float frag[G::kSlots][G::kTiles][2][16 * kComps];    // [slot][tile][16-token half][component, token]
+    float frag[G::kSlots][G::kTiles][2][64];             // [slot][tile][16-token half][component, token]
     float2 viw[kPairs][kD], dd[kPairs][kD];              // v / D, D
     float beta[kD], sel[kD];
     BlockPair bp[kPairs][G::kBlocks];
@@ -176,23 +177,17 @@ struct __align__(1024) Smem {
     // values of tokens g, g + 8 of a half, this lane's component
     __device__ __forceinline__ void put(int slot, int tile, int half, int lane, float x0, float x1) {
         const int g = lane >> 2, comp = lane & 3;
-        if (kComps == 4 || comp < kComps) {
-            frag[slot][tile][half][at(comp, g)] = x0;
-            frag[slot][tile][half][at(comp, g + 8)] = x1;
-        }
+        frag[slot][tile][half][at(comp, g)] = x0;
+        frag[slot][tile][half][at(comp, g + 8)] = x1;
     }
     __device__ __forceinline__ Rhs get(int slot, int tile, int half, int lane) const {
         const int g = lane >> 2, comp = g >> 1, token = 2 * (lane & 3);
-        Rhs f = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
-        if (kComps == 4 || comp < kComps) {
-            const float2 x0 = *reinterpret_cast<const float2*>(&frag[slot][tile][half][at(comp, token)]);
-            const float2 x1 = *reinterpret_cast<const float2*>(&frag[slot][tile][half][at(comp, token + 8)]);
-            const float2 r0 = make_float2(rest(x0.x), rest(x0.y)), r1 = make_float2(rest(x1.x), rest(x1.y));
-            const bool first = (g & 1) == 0;
-            f.ab = first ? make_uint2(pair_hi(x0.x, x0.y), pair_hi(x1.x, x1.y)) : make_uint2(pair_hi(r0.x, r0.y), pair_hi(r1.x, r1.y));
-            f.c = first ? make_uint2(pair_hi(rest(r0.x), rest(r0.y)), pair_hi(rest(r1.x), rest(r1.y))) : make_uint2(0u, 0u);
-        }
-        return f;
+        const float2 x0 = *reinterpret_cast<const float2*>(&frag[slot][tile][half][at(comp, token)]);
+        const float2 x1 = *reinterpret_cast<const float2*>(&frag[slot][tile][half][at(comp, token + 8)]);
+        const float2 r0 = make_float2(rest(x0.x), rest(x0.y)), r1 = make_float2(rest(x1.x), rest(x1.y));
+        if (g & 1) return {make_uint2(pair_hi(r0.x, r0.y), pair_hi(r1.x, r1.y)), make_uint2(0u, 0u)};
+        return {make_uint2(pair_hi(x0.x, x0.y), pair_hi(x1.x, x1.y)),
+                make_uint2(pair_hi(rest(r0.x), rest(r0.y)), pair_hi(rest(r1.x), rest(r1.y)))};
     }
 };
 
@@ -399,7 +394,7 @@ __device__ __forceinline__ float next_im(cplx g, float sr, float si, float l) {
 // resident blocks per SM the registers are cut for (N 16, head_dim 64, 4 / 3 blocks: 285 / 284 us with 6144 chunks, 111 / 119
 // with 1692, where a chain of chunks waits)
 template <int kD, int kPairs>
-constexpr int kMinBlocks = kD == 128 ? (kPairs == 1 ? 3 : 2) : (kPairs <= 2 ? 6 : 4);
+constexpr int kMinBlocks = kD == 128 ? 2 : (kPairs == 2 ? 6 : 4);
 
 template <int kD, int kPairs, Mode kMode>
 __global__ void __launch_bounds__(Geo<kD, kPairs>::kThreads, kMinBlocks<kD, kPairs>)
@@ -431,7 +426,9 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     }
     if (sm.stop) return;   // an earlier block gave up
     // chunk-major: every block that a block may wait for has an earlier ticket
-    const int item = sm.item, hd = item % H, b = (item / H) % a.B, c = item / (H * a.B);
+    const int group = kD == 128 ? sm.item % a.groups : 0, item = kD == 128 ? sm.item / a.groups : sm.item;
+    const int hd = item % H, b = (item / H) % a.B, c = item / (H * a.B);
+    const int pair0 = group * kPairs, NPB = min(kPairs, NP - pair0);   // the block's pairs
     const size_t unit = ((size_t)b * a.NC + c) * H + hd;       // workspace slot
     const int Lc = min(kD, L - c * kD);
     if (tid == 0 && !a.withhold) {
@@ -442,12 +439,13 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 
     // ---- carry into the chunk: this warp's 32 columns of its state rows.  Early if its producer is done, else polled for
     // behind the products that do not need it (kOutput: the previous pass is waited for there).
-    const float* carry_src = a.ws_state + unit * (size_t)N * kD;
+    const float* carry_src = a.ws_state + (unit * (size_t)N + 2 * pair0) * kD;
+    const int flag_bit = G::kBlocks * kSplit * group + W;
     int* carry_flag = reinterpret_cast<int*>(a.ws_gamma + unit * (size_t)N);   // a bit per warp
     auto flag_set = [&]() {
         int v;
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(carry_flag) : "memory");
-        return ((v >> W) & 1) != 0;
+        return ((v >> flag_bit) & 1) != 0;
     };
     auto load_carry = [&](const float* src) {
         const int col = 32 * I + 4 * (tl & 7);
@@ -455,7 +453,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int n0 = 0; n0 < 2 * G::kOwnPairs; n0 += 4) {
             const int n = 2 * G::kOwnPairs * S + n0 + (tl >> 3);
             if (n0 + (tl >> 3) < 2 * G::kOwnPairs) {
-                const bool on = src != nullptr && n < N;
+                const bool on = src != nullptr && n < 2 * NPB;
                 cp_async16(&sm.s_in[n][col], on ? src + (size_t)n * kD + col : a.ws_state, on);
             }
         }
@@ -463,7 +461,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     };
     bool have_carry = true;
     if (kMode == kFused) {
-        if (c == 0) load_carry(a.h0 ? a.h0 + ((size_t)b * H + hd) * N * kD : nullptr);
+        if (c == 0) load_carry(a.h0 ? a.h0 + (((size_t)b * H + hd) * N + 2 * pair0) * kD : nullptr);
         else if ((have_carry = __all_sync(0xffffffffu, flag_set()))) load_carry(carry_src);
     }
     // the token's dynamics, parked where the results will go (padding pairs: identity)
@@ -471,11 +469,11 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     auto load_records = [&]() {
         if (first_warp) cp_async_small<4>(&sm.beta[tok], a.rec_g + unit * kD + tok);
         if (last_warp) {
-            const float2* ra = a.rec_a + unit * (size_t)NP * kD + tok;
-            const uint32_t* rv = a.rec_v + unit * (size_t)NP * kD + tok;
+            const float2* ra = a.rec_a + (unit * (size_t)NP + pair0) * kD + tok;
+            const uint32_t* rv = a.rec_v + (unit * (size_t)NP + pair0) * kD + tok;
 #pragma unroll
             for (int p = 0; p < kPairs; p++) {
-                if (p < NP) {
+                if (p < NPB) {
                     cp_async_small<8>(&sm.dd[p][tok], ra + p * kD);
                     cp_async_small<4>(&sm.viw[p][tok], rv + p * kD);
                 } else {
@@ -732,10 +730,10 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         }
     };
     const int comp = t4 & 1;
-    // pair of the lane's component / of the fragment column in tile q (with one pair, the second half repeats it unused)
-    auto pair_of = [&](int q) { return kPairs == 1 ? 0 : 2 * tile(q) + (t4 >> 1); };
-    auto column_pair = [&](int q) { return kPairs == 1 ? 0 : 2 * tile(q) + (g >> 2); };
-    constexpr int kPerTile = kPairs == 1 ? 1 : 2;
+    // pair of the lane's component / of the fragment column in tile q
+    auto pair_of = [&](int q) { return 2 * tile(q) + (t4 >> 1); };
+    auto column_pair = [&](int q) { return 2 * tile(q) + (g >> 2); };
+    constexpr int kPerTile = 2;
     // complex factor times the lane's component; `other` is the other component of the same value
     auto rotate = [&](cplx f, float own, float other) { return f.r * own + (comp ? f.i : -f.i) * other; };
 
@@ -748,7 +746,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const float2 e = sm.viw[pair_of(q)][32 * I + 8 * r + g];
-                gx[q][r] = kPairs == 1 && t4 >= 2 ? 0.f : bn[r] * (comp ? e.y : e.x);
+                gx[q][r] = bn[r] * (comp ? e.y : e.x);
             }
 #pragma unroll
         for (int J = 0; J < kBlocks - 1; J++)
@@ -776,7 +774,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 for (int s = 0; s < kPerTile; s++)
                     if ((slow >> (2 * tile(q) + s)) & 1) {
                         slow_walk<kD, kPairs, kMode, false>(sm, 2 * tile(q) + s, I, W, tl);
-                        if (kPairs == 1 || (t4 >> 1) == s) {
+                        if ((t4 >> 1) == s) {
 #pragma unroll
                             for (int r = 0; r < 4; r++) {
                                 const float4 x = sm.walk[W][8 * r + g];
@@ -874,12 +872,12 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
         for (int q = 0; q < kOwn; q++) {
             const int p = pair_of(q);
-            if (p < NP && (kPairs > 1 || t4 < 2)) {
+            if (p < NPB) {
                 cplx gam = chunk_decay(p);
                 gam = whole ? cplx{bfr(gam.r), bfr(gam.i)} : cplx{0.f, 0.f};
                 if (kMode == kLocal && I == 0 && g == 0)
-                    a.ws_gamma[unit * N + 2 * p + comp] = comp ? gam.i : gam.r;
-                const int n = 2 * p + comp;
+                    a.ws_gamma[unit * N + 2 * (pair0 + p) + comp] = comp ? gam.i : gam.r;
+                const int n = 2 * (pair0 + p) + comp;
 #pragma unroll
                 for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -901,7 +899,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (c + 1 < a.NC && have_carry) {      // release this warp's columns to the next chunk
             __syncwarp();
             int* next = reinterpret_cast<int*>(a.ws_gamma + (unit + H) * (size_t)N);
-            if (tl == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(next), "r"(1 << W) : "memory");
+            if (tl == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(next), "r"(1 << flag_bit) : "memory");
         }
     } else {
         grid_dependency_wait();   // the pass before; the records are there: it has waited for them before this launch
@@ -913,7 +911,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             const size_t first = (size_t)b * a.NC * H + hd;
             float sr[G::kOwnPairs], si[G::kOwnPairs];
             const float* h0 = a.h0 ? a.h0 + ((size_t)b * H + hd) * N * kD + tok : nullptr;
-            auto row = [&](int i) { return 2 * min(G::kOwnPairs * S + i, NP - 1); };
+            auto row = [&](int i) { return 2 * (pair0 + min(G::kOwnPairs * S + i, NPB - 1)); };
 #pragma unroll
             for (int i = 0; i < G::kOwnPairs; i++) {
                 sr[i] = h0 ? h0[row(i) * kD] : 0.f;
@@ -966,7 +964,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 float* fs = a.final_state + ((size_t)b * H + hd) * N * kD + tok;
 #pragma unroll
                 for (int i = 0; i < G::kOwnPairs; i++)
-                    if (G::kOwnPairs * S + i < NP) {
+                    if (G::kOwnPairs * S + i < NPB) {
                         fs[row(i) * kD] = sr[i];
                         fs[(row(i) + 1) * kD] = si[i];
                     }
@@ -990,7 +988,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     auto r0_frag = [&](int q, int ks) {
         const int n = 2 * column_pair(q) + ((g >> 1) & 1);
         const uint32_t* s = reinterpret_cast<const uint32_t*>(&sm.r0[n][16 * ks + 2 * t4]);
-        return (g & 1) || (kPairs == 1 && g >= 4) ? make_uint2(0u, 0u) : make_uint2(s[0], s[4]);
+        return (g & 1) ? make_uint2(0u, 0u) : make_uint2(s[0], s[4]);
     };
     // ---- h: right-hand sides c_t k_t.r_0, the same chain
     float hx[kOwn][4];
@@ -1157,7 +1155,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     for (int r = 0; r < 4; r++) {
                         const float ho = __shfl_xor_sync(0xffffffffu, rho[q][r], 1);
                         const float4 x = sm.walk[W][8 * r + g];
-                        if (kPairs == 1 || (t4 >> 1) == s)
+                        if ((t4 >> 1) == s)
                             oz[q][r] = (comp ? x.y : x.x) + rotate(cmul(pre, {x.z, x.w}), rho[q][r], ho);
                     }
                     __syncwarp();
@@ -1175,26 +1173,26 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 const float2 e = sm.viw[p][row], D = sm.dd[p][row];
                 cplx vg = cmul({e.x, e.y}, {D.x, D.y});
                 if ((slow >> p) & 1) {               // (its v has made room for g)
-                    const uint32_t w = __ldcg(a.rec_v + (unit * (size_t)NP + p) * kD + row);
+                    const uint32_t w = __ldcg(a.rec_v + (unit * (size_t)NP + pair0 + p) * kD + row);
                     vg = {bits_lo(w), bits_hi(w)};
                 }
                 yy += a.shortcut_scale * qk * qk * bfr(comp ? vg.i : vg.r);
             }
-            if (kPairs > 1 || t4 < 2) sm.y(row)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * sm.sel[row]);
+            sm.y(row)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * sm.sel[row]);
         }
     }
     __syncwarp();
     if (tok < Lc) {   // lane = token: its row of this warp's values
         constexpr int kOwnPairs = G::kOwnPairs;
-        __nv_bfloat16* yo = a.y + (((size_t)b * L + c * kD + tok) * H + hd) * N;
+        __nv_bfloat16* yo = a.y + (((size_t)b * L + c * kD + tok) * H + hd) * N + 2 * pair0;
         const uint32_t* ys = reinterpret_cast<const uint32_t*>(sm.y(tok));
         const int p0 = kOwnPairs * S;
-        if (kOwnPairs >= 4 && N == 2 * kPairs && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0) {
+        if (kOwnPairs >= 4 && NPB == kPairs && N % 8 == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0) {
 #pragma unroll
             for (int i = 0; i < kOwnPairs; i += 4)
                 *reinterpret_cast<uint4*>(yo + 2 * (p0 + i)) = make_uint4(ys[p0 + i], ys[p0 + i + 1], ys[p0 + i + 2], ys[p0 + i + 3]);
         } else {
-            for (int i = p0; i < min(NP, p0 + kOwnPairs); i++) reinterpret_cast<uint32_t*>(yo)[i] = ys[i];
+            for (int i = p0; i < min(NPB, p0 + kOwnPairs); i++) reinterpret_cast<uint32_t*>(yo)[i] = ys[i];
         }
     }
     // ---- the recurrent state after the last token
@@ -1214,8 +1212,8 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     const int d = 32 * I + 16 * m + 8 * e + g, n = 2 * p + comp;
                     const float r = __bfloat162float(sm.r0[n][d]) - (h[m][2 * e] + h[m][2 * e + 1]);
                     const float o = __shfl_xor_sync(0xffffffffu, r, 1);
-                    if (p < NP && (kPairs > 1 || t4 < 2))
-                        a.tail_state[(((size_t)b * H + hd) * N + n) * kD + d] = z[m][2 * e] + z[m][2 * e + 1] + rotate(w, r, o);
+                    if (p < NPB)
+                        a.tail_state[(((size_t)b * H + hd) * N + 2 * pair0 + n) * kD + d] = z[m][2 * e] + z[m][2 * e + 1] + rotate(w, r, o);
                 }
         }
     }
@@ -1231,7 +1229,7 @@ static int launch_one(const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args
     const size_t smem = sizeof(Smem<kD, kPairs, kMode>);
     static_assert(sizeof(Smem<kD, kPairs, kMode>) <= 227 * 1024, "shared memory");
     if (int rc = allow_smem<KernelTag<kD, kPairs, kMode>>((const void*)scan_chunk_kernel<kD, kPairs, kMode>, smem)) return rc;
-    const long long units = (long long)a.B * a.NC * a.H;
+    const long long units = (long long)a.B * a.NC * a.H * a.groups;
     return launch_overlapped(scan_chunk_kernel<kD, kPairs, kMode>, dim3((unsigned)units), dim3(Geo<kD, kPairs>::kThreads), smem, st,
                              tmK, tmQ, a);
 }
@@ -1243,16 +1241,17 @@ static int launch_mode(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, c
 }
 template <int kD>
 static int launch_tiles(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, const Args& a, cudaStream_t st) {
-    if (a.N <= 2) return launch_mode<kD, 1>(m, tmK, tmQ, a, st);
+    // (head_dim 128, eight pairs in one block: 124 KB, one block per SM, 400 ns a chunk on the full GPU; in two blocks that
+    // both form G and P, 218)
     if (a.N <= 4) return launch_mode<kD, 2>(m, tmK, tmQ, a, st);
-    if (a.N <= 8) return launch_mode<kD, 4>(m, tmK, tmQ, a, st);
-    return launch_mode<kD, 8>(m, tmK, tmQ, a, st);
+    if (kD == 128 || a.N <= 8) return launch_mode<kD, 4>(m, tmK, tmQ, a, st);
+    return launch_mode<64, 8>(m, tmK, tmQ, a, st);
 }
 
 }  // namespace chunk
 
 bool scan_chunk_supported(int D, int N, int C, int dtype) {
-    return dtype == CDSSM_BF16 && D == C && (D == 64 || D == 128) && N <= 16;
+    return dtype == CDSSM_BF16 && D == C && (D == 64 || D == 128) && N > 2 && N <= 16;
 }
 
 // scan_records.cu
@@ -1281,7 +1280,8 @@ int scan_chunk_pass(int mode, int from_chunks, const void* q, long long q_rs, co
     a.from_chunks = from_chunks;
     a.shortcut_scale = shortcut_scale;
     a.B = B; a.L = L; a.H = H; a.N = N; a.NC = (L + D - 1) / D;
-    if ((long long)B * a.NC * H > 0x7fffffff) return CDSSM_ERR_UNSUPPORTED;
+    a.groups = D == 128 && N > 8 ? 2 : 1;
+    if ((long long)B * a.NC * H * a.groups > 0x7fffffff) return CDSSM_ERR_UNSUPPORTED;
     const Mode m = mode == 0 ? kLocal : mode == 1 ? kOutput : kFused;
     if (mode == 0) a.tail_state = nullptr;
     return D == 128 ? launch_tiles<128>(m, tmK, tmQ, a, st) : launch_tiles<64>(m, tmK, tmQ, a, st);

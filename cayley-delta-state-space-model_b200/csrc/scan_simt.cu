@@ -794,7 +794,7 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
                  int* clear, size_t clear_words, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
                  int fp32_decay, cudaStream_t st);
 // scan_wa.cu
-bool scan_wa_supported(int D, int N, int C, int H, int dtype);
+bool scan_wa_supported(int D, int N, int C, int dtype);
 int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  int from_chunks, const float* h0, float* final_state, int parts, cudaStream_t st);
@@ -835,22 +835,27 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
 // Whether the output pass of the whole-chunk scan adds the carry up itself from the local results of the chunks before it (else
 // a carry pass runs in between): a read of NC x N rows by every block, in parallel, against a launch and two more trips to
 // memory.  us on B200, carry pass / without (D 64, one sequence): N 16, H 24, 9 chunks 35 / 24, 16 chunks 38 / 27, 32 chunks
-// 43 / 46; N 4, H 6, 9 chunks 14 / 11, 48 chunks 19 / 20; N 2, H 6, 9 chunks 14 / 10.
+// 43 / 46; N 4, H 6, 9 chunks 14 / 11, 48 chunks 19 / 20.
 static bool few_chunks(int NC, int N) { return NC <= 40 && NC * N <= 400; }
 
 // Whether the whole-chunk scan runs as one kernel that hands the carry from chunk to chunk inside it, or as local pass
-// (+ carry pass) + output pass.  One kernel reads k once and forms G once, but a hand-off takes 2 us and more (flag, carry,
-// rounding, release), so a (batch, head) chain of NC chunks takes that many whatever the size; the passes cost more work.
-// Each form: the larger of its latency and its work on the full GPU, us on B200, fitted to 220 sizes (one kernel / passes, D 64:
-// N 16, B 8, H 12, 29 chunks 122 / 110; N 8, B 4, H 32, 50 chunks 150 / 173; N 2, B 4, H 24, 5 chunks 17 / 13.5, B 16, H 24, 2
-// chunks 18 / 21; D 128, N 4, B 2, H 32, 27 chunks 101 / 135); the choice costs 0.4 % over the better one on average.
+// (+ carry pass) + output pass: the same arithmetic in the same order, so the choice may go by size.  One kernel reads k once
+// and forms G once, but a hand-off takes 2 us and more (flag, carry, rounding, release), so a (batch, head) chain of NC chunks
+// takes that many whatever the size; the passes cost more work.  Each form: the larger of its latency and its work on the full
+// GPU, us on B200, by the number of pairs the kernel holds, fitted to 380 sizes.
+struct FormCost { float one, one_chunk, one_full, one_unit, one_slope, pass, pass_chunk, pass_carry, pass_full, pass_unit; };
 static bool one_kernel_pays(int B, int H, int NC, int D, int N) {
-    const float units = (float)B * H * NC, n = (float)N, c = (float)NC;
-    const bool carry = !few_chunks(NC, N);
-    const float one = D == 64 ? fmaxf(6.7f + (1.96f + 0.1f * n) * c, 6.5f + units * (0.0113f + 0.00118f * n))
-                              : fmaxf(10.7f + (2.6f + 0.033f * n) * c, 9.1f + units * (0.0282f + 0.00665f * n));
-    const float passes = D == 64 ? fmaxf(9.5f + 0.21f * n + 0.173f * c + (carry ? 10.f : 0.f), 7.2f + units * (0.0161f + 0.00161f * n))
-                                 : fmaxf(15.8f + 0.49f * n + (carry ? 1.7f : 0.f), 13.3f + units * (0.0497f + 0.0075f * n));
+    static const FormCost kCost[2][3] = {   // one_slope: work per unit grows with the length of the chains that wait
+        {{8.1f, 2.14f, 10.4f, 0.0185f, 0.f, 11.7f, 0.19f, 10.f, 10.8f, 0.0261f},       // head_dim 64: N 4, 8, 16
+         {8.7f, 2.33f, 11.3f, 0.0238f, 1e-4f, 8.5f, 0.36f, 0.f, 11.8f, 0.0352f},
+         {6.4f, 3.77f, 15.8f, 0.0426f, 1e-4f, 19.1f, 0.44f, 0.f, 15.4f, 0.0577f}},
+        {{16.7f, 1.88f, 17.9f, 0.0616f, 5e-4f, 23.9f, 0.27f, 17.f, 17.9f, 0.0964f},    // head_dim 128: N 4, 8, 16 (two blocks a chunk)
+         {23.6f, 2.31f, 24.9f, 0.102f, 8e-4f, 32.1f, 0.1f, 40.f, 26.5f, 0.1375f},
+         {16.1f, 4.48f, 21.2f, 0.218f, 3e-4f, 11.8f, 5.2f, 7.f, 24.9f, 0.273f}}};
+    const FormCost& f = kCost[D == 128][N <= 4 ? 0 : N <= 8 ? 1 : 2];
+    const float units = (float)B * H * NC, c = (float)NC;
+    const float one = fmaxf(f.one + f.one_chunk * c, f.one_full + units * (f.one_unit + f.one_slope * fminf(c, 100.f)));
+    const float passes = fmaxf(f.pass + f.pass_chunk * c + (few_chunks(NC, N) ? 0.f : f.pass_carry), f.pass_full + units * f.pass_unit);
     return one <= passes;
 }
 
@@ -909,22 +914,18 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     a.ws_state = reinterpret_cast<float*>(static_cast<char*>(workspace) +
                                           align256((size_t)a.units * 2 * sizeof(float)));
     cudaStream_t st = (cudaStream_t)stream;
-    // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 with heads in fours (scan_wa.cu), any other
-    // N <= 16 (scan_chunk.cu).  The latter also for N = 2 while the
-    // GPU is not full: its passes do a chunk as a whole where scan_wa.cu walks it in sub-blocks (us, passes / scan_wa.cu, D 64:
-    // 120 chunks 10 / 17, 544 15 / 20, 704 22 / 22, 936 25 / 23; one kernel / scan_wa.cu, up to six chunks in a row: 768 18 / 21,
-    // 1536 28 / 31, 1920 in threes 49 / 37; D 128: 192 21 / 30, 528 39 / 32).  They read v
+    // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 (scan_wa.cu), any other N <= 16 (scan_chunk.cu).  The
+    // kernel goes by the head's shape and by what is asked for, never by batch or length: a shard of a batch, and chunk-aligned
+    // pieces of a sequence that hand the carry on, give the bits of the whole.  They read v
     // and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the contract allows, stay on the CUDA-core
     // kernels.  (Bits 256 / 512 keep the CUDA-core local / output pass: used by the tests to check each tensor-core pass alone.)
     const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y | (uintptr_t)rows.first | (uintptr_t)(2 * v_rs) |
                               (uintptr_t)(rows.first ? 2 * vf_rs : 0)) & 3) == 0 && ((q_rs | k_rs) & 7) == 0 && workspace_bytes - base >= scan_record_bytes(B, L, H, N, C) &&
                            !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
-    const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, H, dtype) &&
-                       ((flags & CDSSM_SCAN_TENSOR_CORE_WA) || a.NC > 40 || (long long)B * a.NC * H > (D == 64 ? (a.NC <= 6 ? 1536 : 640) : 256));
-    const bool chunk_ok = tensor_ok && !wa_ok && scan_chunk_supported(D, N, C, dtype);
-    if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && !wa_ok) return CDSSM_ERR_UNSUPPORTED;
-    // (who keeps the state after the last token gets the precision of the CUDA-core walk, which these calls took before)
-    const int wa_parts = tail_state == nullptr || (flags & CDSSM_SCAN_TENSOR_CORE_WA) ? 2 : 3;
+    const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, dtype), chunk_ok = tensor_ok && scan_chunk_supported(D, N, C, dtype);
+    if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && (!wa_ok || H % 4)) return CDSSM_ERR_UNSUPPORTED;
+    // (the precision that the CUDA-core walk gave these calls before they came here)
+    const int wa_parts = (H % 4 == 0 && tail_state == nullptr) || (flags & CDSSM_SCAN_TENSOR_CORE_WA) ? 2 : 3;
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
     const bool one_kernel = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && ((uintptr_t)h0 & 15) == 0 &&
                             one_kernel_pays(B, H, a.NC, D, N);
@@ -962,7 +963,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     // (The whole-chunk output pass has also done all that needs no carry by the time the local pass ends.  scan_wa.cu: while its
     // output pass has a chunk of four heads per block, two blocks per SM; us, carry pass / without: D 64, 936 chunks 24.4 / 21.5,
     // 3072 42 / 44; D 128, 528 32.3 / 30.5, 1536 61 / 63.)
-    const int from_chunks = (chunk_ok || (wa_ok && (long long)B * a.NC * H <= 4 * 296)) &&
+    const int from_chunks = (chunk_ok || (wa_ok && (long long)B * a.NC * ((H + 3) / 4) <= 296)) &&
                             tc_local && tc_output && a.run_local && !summary_only && few_chunks(a.NC, N);
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
@@ -1133,7 +1134,7 @@ extern "C" int cdssm_b200_scan_fused_fwd_noalloc(const void* q, const void* k, c
     if (cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C) == 0) return CDSSM_ERR_BAD_ARG;
     // beyond the built-in scratch?  (the records of the tensor-core kernel of N = 2 are part of it, others only as they fit)
     size_t need = base_workspace_bytes(B, L, H, D, N, C);
-    if (scan_wa_supported(D, N, C, H, CDSSM_BF16)) need += align256(scan_record_bytes(B, L, H, N, C));
+    if (scan_wa_supported(D, N, C, CDSSM_BF16) && H % 4 == 0) need += align256(scan_record_bytes(B, L, H, N, C));
     if (need > kNoAllocScratchBytes) return CDSSM_ERR_WORKSPACE;
     int dev = 0;
     if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;

@@ -1,7 +1,8 @@
 // Fused scan with warp-autonomous chains: the Gram blocks of a 32-token sub-block come from the tcgen05
 // tensor cores (TMA-staged bf16 tiles, fp32 accumulators in tensor memory), everything that depends on the
 // running state stays inside the warp that owns the head.
-// Shapes: bf16 storage, state_dim N = 2, head_dim D = chunk C in {64, 128}, H a multiple of 4.
+// Shapes: bf16 storage, state_dim N = 2, head_dim D = chunk C in {64, 128}, any H (a last group of fewer than four heads is
+// filled up with tiles of zeros).
 //
 // A thread block owns the same chunk of FOUR heads and walks it in 32-token sub-blocks; UMMA tile row
 // 32 j + t is token t of head j's sub-block and compute warp j owns head j.  Per sub-block:
@@ -447,7 +448,7 @@ __device__ __forceinline__ uint32_t third_pack(float x0, float x1) {
 // The carry into a chunk of head hd, rounded: s <- gamma s + z over the chunks before, evaluated as the carry pass does; a lane
 // has kD / 32 columns.  out: its real, then its imaginary row.
 template <int kD>
-__device__ __forceinline__ void carry_from_chunks(const Args& a, const ItemPos& at, int hd, int tl, float* out) {
+__device__ __forceinline__ void carry_from_chunks(const Args& a, const ItemPos& at, int hd, int tl, float* out, bool stores) {
     constexpr int kPer = kD / 32, kBatch = kD == 64 ? 8 : 4;
     const size_t first = (size_t)at.b * a.NC * a.H + hd, so = ((size_t)at.b * a.H + hd) * 2 * kD + tl;
     float sr[kPer], si[kPer];
@@ -493,7 +494,7 @@ __device__ __forceinline__ void carry_from_chunks(const Args& a, const ItemPos& 
     }
     if (chunks == at.c) {
         put();
-    } else {
+    } else if (stores) {
 #pragma unroll
         for (int i = 0; i < kPer; i++) {
             a.final_state[so + 32 * i] = sr[i];
@@ -551,7 +552,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     grid_launch_dependents();
     {
         const bool valid = cur.c * kD + tl < L;
-        const uint4 first = valid ? __ldcg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, cur.h0 + J, tl)) : still4;
+        const uint4 first = valid ? __ldcg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, min(cur.h0 + J, H - 1), tl)) : still4;
         tk = prepare(first, tl);
     }
     for (int g = 0; g < NS; g++) {
@@ -562,13 +563,14 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             if (g > 0) cur = nxi;
             nxi = item_pos(a, (int)blockIdx.x + (g / kSteps + 1) * (int)gridDim.x);
         }
-        const int l = cur.c * kD + step * kSub + tl, hd = cur.h0 + J;
-        const bool valid = l < L;
+        // (a group past the last head: the warp reads that head's values beside tiles of zeros and stores nothing)
+        const int l = cur.c * kD + step * kSub + tl, hd = min(cur.h0 + J, H - 1);
+        const bool stores = cur.h0 + J < H, valid = l < L && stores;
         const size_t unit = ((size_t)cur.b * a.NC + cur.c) * H + hd;   // workspace slot of this head's chunk
         if (step == 0) {   // states at the chunk start: z = 0, r = the chunk's carry
             const float* s = a.ws_state + unit * 2 * kD + (size_t)(np & 1) * kD;
             if (kOutput && a.from_chunks) {
-                carry_from_chunks<kD>(a, cur, hd, tl, scr);
+                carry_from_chunks<kD>(a, cur, hd, tl, scr, stores);
                 s = scr + (np & 1) * kD;
             }
 #pragma unroll
@@ -589,7 +591,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             const ItemPos& np_ = (step + 1 < kSteps) ? cur : nxi;
             const int nsub = (step + 1) % kSteps;
             if (np_.c * kD + nsub * kSub + tl < L)
-                rec = __ldcg(a.rec + rec_index(a, kSteps, np_.b, np_.c, nsub, np_.h0 + J, tl));
+                rec = __ldcg(a.rec + rec_index(a, kSteps, np_.b, np_.c, nsub, min(np_.h0 + J, H - 1), tl));
         }
         const cplx at = tk.at, vg = tk.vg;
         const float be = tk.be;
@@ -844,7 +846,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             // the carry pass consumes these as the reference's bf16 cum_A[:, -1] / local_h[:, -1]; the reference's zero
             // padding of a ragged last chunk wipes both (ssd.py:60-67)
             const float keep = cur.c * kD + kD <= L ? 1.f : 0.f;
-            if (!low && np < 2) {
+            if (!low && np < 2 && stores) {
                 float* s = a.ws_state + unit * 2 * kD + (size_t)np * kD;
 #pragma unroll
                 for (int ks = 0; ks < kKs; ks++) {
@@ -852,7 +854,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                     *reinterpret_cast<float2*>(s + 16 * ks + 8 + 2 * tig) = make_float2(keep * bfr(S[ks][2]), keep * bfr(S[ks][3]));
                 }
             }
-            if (tl == 0) {
+            if (tl == 0 && stores) {
                 a.ws_gamma[unit * 2] = keep * bfr(gam.r);
                 a.ws_gamma[unit * 2 + 1] = keep * bfr(gam.i);
             }
@@ -864,7 +866,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 float x[4];
 #pragma unroll
                 for (int e = 0; e < 4; e++) x[e] = S[ks][e] + __shfl_xor_sync(0xffffffffu, S[ks][e], 16);
-                if (!low && np < 2) {
+                if (!low && np < 2 && stores) {
                     *reinterpret_cast<float2*>(s + 16 * ks + 2 * tig) = make_float2(x[0], x[1]);
                     *reinterpret_cast<float2*>(s + 16 * ks + 8 + 2 * tig) = make_float2(x[2], x[3]);
                 }
@@ -950,8 +952,8 @@ extern "C" __attribute__((visibility("default"))) int cdssm_b200_wa_trace_read(l
 }
 #endif
 
-bool scan_wa_supported(int D, int N, int C, int H, int dtype) {
-    return dtype == CDSSM_BF16 && N == 2 && D == C && (D == 64 || D == 128) && H % 4 == 0;
+bool scan_wa_supported(int D, int N, int C, int dtype) {
+    return dtype == CDSSM_BF16 && N == 2 && D == C && (D == 64 || D == 128);
 }
 
 // One pass of the warp-autonomous tensor-core scan over every chunk.  output = false: local pass (fills
@@ -978,7 +980,7 @@ int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long
     a.from_chunks = from_chunks; a.h0 = h0; a.final_state = final_state;
     a.shortcut_scale = shortcut_scale;
     a.B = B; a.L = L; a.H = H; a.NC = (L + D - 1) / D;
-    a.HG = H / 4;
+    a.HG = (H + 3) / 4;
     const long long items = (long long)B * a.NC * a.HG;
     if (items > 0x7fffffff / 8) return CDSSM_ERR_UNSUPPORTED;
     a.items = (int)items;

@@ -52,3 +52,25 @@ def test_tail_state_has_float32_precision(ops, orc, H, D, N):
     want = _state64(ops, inp, N)
     err = (tail.double() - want).flatten(2).norm(dim=-1) / want.flatten(2).norm(dim=-1)
     assert float(err.median()) <= 2e-6
+
+
+@pytest.mark.parametrize("H,D,N", [(8, 64, 2), (6, 64, 2), (4, 128, 2), (8, 64, 4), (8, 64, 16), (4, 128, 8), (4, 128, 16)])
+@pytest.mark.parametrize("tail", [False, True])
+def test_shards_and_pieces_have_the_bits_of_the_whole(ops, orc, H, D, N, tail):
+    """Rows of a batch alone, and chunk-aligned pieces chained through (final_state, pos0), at sizes from one chunk to
+    where the GPU is full: the kernel may not go by batch or length."""
+    B, L = 24, 12 * D - 5
+    inp = _inputs(orc, B, H, L, D, N, seed=H + N)
+    h0 = np.random.default_rng(3).standard_normal((B, H, N, D)).astype(np.float32) * 0.3
+    run = lambda i, h, **kw: run_fused(ops, i, torch.bfloat16, N, D, h0=h, return_tail_state=tail, **kw)
+    whole = run(inp, h0)
+    for rows in (slice(0, 1), slice(7, 10)):
+        part = run(_cut(inp, rows), h0[rows])
+        for w, p in zip(whole, part):
+            assert torch.equal(w[rows], p)
+    cut = 2 * D
+    first = run(_cut(inp, tokens=slice(0, cut)), h0)
+    second = run(_cut(inp, tokens=slice(cut, None)), to_np(first[1]), pos0=cut)
+    assert torch.equal(torch.cat([first[0], second[0]], 1), whole[0])
+    for w, p in zip(whole[1:], second[1:]):
+        assert torch.equal(w, p)
