@@ -61,6 +61,8 @@ struct Args {
     int groups;                  // blocks that share a chunk of a head: kPairs pairs each
 };
 
+#define kNotANumber __int_as_float(0x7fffffff)
+
 struct cplx { float r, i; };
 __device__ __forceinline__ cplx cmul(cplx a, cplx b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
 __device__ __forceinline__ cplx cshfl(cplx v, int src) {
@@ -172,6 +174,7 @@ struct __align__(1024) Smem {
     uint64_t full_k, full_q;
     int slow[G::kBlocks];                                // pairs that are walked step by step, a bit each
     int abort_flag, item, stop;
+    int first_bad;                                       // first token whose key or beta is no number, kD if there is none
     // (the tokens of components 2 and 3 are turned by eight: a store's lanes then hit distinct banks)
     static __device__ __forceinline__ int at(int comp, int token) { return comp * 16 + (token ^ ((comp >> 1) * 8)); }
     // values of tokens g, g + 8 of a half, this lane's component
@@ -396,6 +399,29 @@ __device__ __forceinline__ float next_im(cplx g, float sr, float si, float l) {
 template <int kD, int kPairs>
 constexpr int kMinBlocks = kD == 128 ? 2 : (kPairs == 2 ? 6 : 4);
 
+// A key row or a beta that is infinite or no number makes the state no number from its token on, whatever the pair.  In the
+// products of a block it would reach the tokens before it too (0 x NaN), so its row is emptied and the outputs from it on are set
+// apart at the end.  A finite row whose square overflows has |k|^-1 = 0: it neither erases nor adds.
+template <int kD, int kPairs, Mode kMode>
+__device__ __noinline__ void empty_bad_rows(Smem<kD, kPairs, kMode>& sm, int I, int tl) {
+    using G = Geo<kD, kPairs>;
+    const int row = 32 * I + tl;
+    bool number = fabsf(sm.beta[row]) <= 3e38f;
+    float ss = 0.f;
+    for (int c = 0; c < kD; c++) {
+        const float k = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(sm.k + (c >> 6) * G::kSlab + row * 128)[c & 63]);
+        number = number && fabsf(k) <= 3.4e38f;
+        ss += k * k;
+    }
+    if (!number) atomicMin(&sm.first_bad, row);
+    if (!number || !(ss <= 3.4e38f)) {
+        for (int s = 0; s < G::kSlabs; s++)
+            for (int i = 0; i < 8; i++) *reinterpret_cast<uint4*>(sm.k + s * G::kSlab + row * 128 + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
+        sm.beta[row] = 0.f;
+    }
+    __syncwarp();
+}
+
 template <int kD, int kPairs, Mode kMode>
 __global__ void __launch_bounds__(Geo<kD, kPairs>::kThreads, kMinBlocks<kD, kPairs>)
 scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const Args a) {
@@ -415,6 +441,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         mbar_init(&sm.full_k, 1);
         mbar_init(&sm.full_q, 1);
         sm.abort_flag = 0;
+        sm.first_bad = kD;
         fence_barrier_init();
         sm.item = kMode == kFused ? atomicAdd(a.ticket, 1) : (int)blockIdx.x;
         sm.stop = kMode == kFused ? *reinterpret_cast<volatile int*>(a.status) : 0;
@@ -515,6 +542,15 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             sm.beta[tok] = bits_lo(gg);
             sm.sel[tok] = bits_hi(gg);
             __syncwarp();
+            bool number = fabsf(bits_lo(gg)) <= 3e38f;   // (false for NaN)
+#pragma unroll
+            for (int r = 0; r < 4; r++) number = number && kk[r] <= 3.4e38f;
+            if (!__all_sync(0xffffffffu, number)) {
+                empty_bad_rows<kD, kPairs, kMode>(sm, I, tl);
+                gram_block<kD, kPairs, true>(acc, kt, 32 * I, kt, 32 * I, tl, true);
+                diagonal_of(acc[0][0], acc[0][1], tl, kk[0], kk[1]);
+                diagonal_of(acc[1][2], acc[1][3], tl, kk[2], kk[3]);
+            }
         }
         if (last_warp) {
             constexpr int kW = kPairs < 4 ? kPairs : 4;
@@ -869,6 +905,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             __syncwarp();
         }
         const bool whole = Lc == kD;           // the reference's zero padding wipes state and decay (ssd.py:60-67)
+        const bool bad = sm.first_bad < kD;
 #pragma unroll
         for (int q = 0; q < kOwn; q++) {
             const int p = pair_of(q);
@@ -883,7 +920,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
                         const int d = 32 * I + 16 * m + 8 * e + g;
-                        const float l = whole ? bfr(z[q][m][2 * e] + z[q][m][2 * e + 1]) : 0.f;
+                        const float l = !whole ? 0.f : bad ? kNotANumber : bfr(z[q][m][2 * e] + z[q][m][2 * e + 1]);
                         if (kMode == kLocal) {
                             a.ws_state[(unit * N + n) * kD + d] = l;
                         } else {
@@ -1167,7 +1204,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int row = 32 * I + 8 * r + g;
-            float yy = mq[r] * oz[q][r];
+            float yy = row >= sm.first_bad ? kNotANumber : mq[r] * oz[q][r];
             if (a.shortcut_scale != 0.f) {   // block.py:202-208; v after the vp scale
                 const float qk = mq[r] * nrm[r] * pd[r];
                 const float2 e = sm.viw[p][row], D = sm.dd[p][row];
@@ -1213,7 +1250,8 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     const float r = __bfloat162float(sm.r0[n][d]) - (h[m][2 * e] + h[m][2 * e + 1]);
                     const float o = __shfl_xor_sync(0xffffffffu, r, 1);
                     if (p < NPB)
-                        a.tail_state[(((size_t)b * H + hd) * N + 2 * pair0 + n) * kD + d] = z[m][2 * e] + z[m][2 * e + 1] + rotate(w, r, o);
+                        a.tail_state[(((size_t)b * H + hd) * N + 2 * pair0 + n) * kD + d] =
+                            sm.first_bad < kD ? kNotANumber : z[m][2 * e] + z[m][2 * e + 1] + rotate(w, r, o);
                 }
         }
     }

@@ -372,10 +372,12 @@ __device__ __noinline__ BlockOut robust_block(uint32_t tg, uint32_t tp, int tl, 
             const int i = grp * 8 + e;
             const float cr_ = bnn * cc[i].r, ci_ = bnn * cc[i].i;
             const cplx uw = cshfl(cw, i), ux = cshfl(cx, i);
-            cw.r -= cr_ * uw.r - ci_ * uw.i;
-            cw.i -= cr_ * uw.i + ci_ * uw.r;
-            cx.r -= cr_ * ux.r - ci_ * ux.i;
-            cx.i -= cr_ * ux.i + ci_ * ux.r;
+            if (i < tl) {   // (an unknown that is no number reaches the tokens behind it only)
+                cw.r -= cr_ * uw.r - ci_ * uw.i;
+                cw.i -= cr_ * uw.i + ci_ * uw.r;
+                cx.r -= cr_ * ux.r - ci_ * ux.i;
+                cx.i -= cr_ * ux.i + ci_ * ux.r;
+            }
         }
     }
     BlockOut o;
@@ -403,9 +405,8 @@ __device__ __noinline__ BlockOut robust_block(uint32_t tg, uint32_t tp, int tl, 
                 pd = (i == tl) ? p8[e] : pd;
                 const cplx au = cmul(at, uw);
                 const cplx ee = cmul(cur, cplx{au.r - ux.r, au.i - ux.i});
-                const float pi = on ? p8[e] : 0.f;
-                yin.r += pi * ee.r;
-                yin.i += pi * ee.i;
+                yin.r += on ? p8[e] * ee.r : 0.f;
+                yin.i += on ? p8[e] * ee.i : 0.f;
                 const cplx nx = cmul(cur, ai);
                 cur = {on ? nx.r : cur.r, on ? nx.i : cur.i};
             }

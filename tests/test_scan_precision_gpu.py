@@ -74,3 +74,30 @@ def test_shards_and_pieces_have_the_bits_of_the_whole(ops, orc, H, D, N, tail):
     assert torch.equal(torch.cat([first[0], second[0]], 1), whole[0])
     for w, p in zip(whole[1:], second[1:]):
         assert torch.equal(w, p)
+
+
+@pytest.mark.parametrize("D,N", [(64, 2), (128, 2), (64, 4), (64, 8), (64, 16), (128, 4), (128, 16)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 3e19])
+@pytest.mark.parametrize("what", ["k", "v", "beta", "decay"])
+def test_tokens_before_a_bad_value_do_not_see_it(ops, orc, D, N, value, what):
+    """NaN, infinity and a key whose square overflows, in one token of one head: every other token's output is a number where
+    the walk by steps gives one, and the same.  (At the token itself, components that a complex product joins may differ.)"""
+    B, H, L, t = 1, 3, 2 * D + 40, D + 21
+    inp = _inputs(orc, B, H, L, D, N, seed=N)
+    if what == "k":
+        inp["k"][0, t, 1, 5] = value
+    elif what == "v":
+        inp["v"][0, t, 1, 0] = value
+    else:
+        inp["gate_raw"][0, t, {"beta": (N + 3) * H, "decay": 0}[what] + 1] = value
+    y, fin, tail = run_fused(ops, inp, torch.bfloat16, N, D, return_tail_state=True)
+    ys, fs, ts = run_fused(ops, inp, torch.bfloat16, N, D, return_tail_state=True, flags=ops.FORCE_SIMT)
+    assert ops.scan_fused_status() == 0
+    for a, b in ((y, ys), (fin, fs), (tail, ts)):
+        a, b = to_np(a), to_np(b)
+        if a.shape == tuple(y.shape):
+            a, b = np.delete(a, t, 1), np.delete(b, t, 1)
+        assert np.array_equal(np.isfinite(a), np.isfinite(b))
+        ok = np.isfinite(b)
+        assert np.abs(a[ok] - b[ok]).max() <= 2e-2 * np.abs(b[ok]).max()
+    assert np.isfinite(to_np(y)[0, :t]).all()
