@@ -181,8 +181,9 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
     if ((long long)B * a.tiles > 0x7fffffff || H > 8 * 65535) return CDSSM_ERR_UNSUPPORTED;
     if (wa) return launch_group<1, true>(a, st);
     if (N <= 2) return launch_group<1, false>(a, st);
-    // Short inputs: one pair per thread up to two blocks per SM, two up to four; each computes what the pairs share.  us, 24
-    // heads, N 16, all / two / one pair per thread: 523 tokens 5.4 / - / 3.7, 1046 5.6 / 4.6 / 5.9, 2092 7.1 / 7.3 / -.
+    // Short inputs: one pair per thread up to two blocks per SM, two up to four; each computes what the pairs share.  us of a
+    // whole scan call, 24 heads, N 16, one / two / all pairs per thread: 128 tokens 17.4 / 17.7 / 20.9, 523 30.6 / 31.4 / 32.5,
+    // 1046 37.2 / 37.3 / 40.4, 2092 61.1 / 59.0 / 61.0, 4 x 2092 227 / 214 / 203.
     const long long blocks = (long long)B * a.tiles * ((H + 7) / 8);
     if (blocks * (N / 2) <= 296) return launch_group<1, false>(a, st);
     if (N > 4 && blocks * ((N / 2 + 1) / 2) <= 592) return launch_group<2, false>(a, st);
