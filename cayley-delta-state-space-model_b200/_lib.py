@@ -60,6 +60,7 @@ SIGNATURES = {
     "cdssm_b200_decode_step": (_I, [_P] * 8 + [_F] * 6 + [_I] * 6 + [_P]),
     "cdssm_b200_decode_step_strided": (_I, [_P, _P, _c_int64, _P, _c_int64, _P, _c_int64, _P, _P, _P, _c_int64] + [_P] * 3 + [_F] * 6 + [_I] * 5 + [_P, _I, _P]),
     "cdssm_b200_decode_step_reference": (_I, [_P] * 11 + [_F] * 6 + [_I] * 6 + [_P, _I, _P]),
+    "cdssm_b200_residual_mix": (_I, [_P, _I, _I, _P, _I, _P]),
     "cdssm_b200_lm_decode_workspace_bytes": (_c_size_t, [_I] * 6),
     "cdssm_b200_lm_decode": (_I, [_P, _I] + [_P] * 5 + [_c_size_t] + [_F] * 8 + [_I] * 6 + [_P, _I, _P]),
     "cdssm_b200_decode_step_at": (_I, [_P] * 8 + [_F] * 6 + [_I] * 4 + [_P, _I, _P]),

@@ -10,6 +10,19 @@
 
 namespace cdssm {
 
+// ---------------------------------------------------------------- value-residual weights
+// sigmoid(v_residual_gate) of all layers of a model in the storage type (block.py:167-171): formed in every pass, 2 us of 250 of a
+// decode step, so that nothing has to be kept from one pass for the next.
+constexpr int kMixLayers = 64;
+struct MixGates { const float* of[kMixLayers]; };
+template <typename T>
+__global__ void residual_mix_kernel(const MixGates gates, T* mix, int H) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const float* g = gates.of[blockIdx.x];
+    for (int h = threadIdx.x; h < H; h += blockDim.x) IO<T>::st(mix + (size_t)blockIdx.x * H + h, 1.f / (1.f + expf(-g[h])));
+}
+
 // ---------------------------------------------------------------- RMSNorm
 // The kernels below are launched while their predecessor drains and wait for it before they read anything: between the small
 // products of a short prompt a plain launch cost as much as some of them (12 layers, d 768, 523 tokens: 825 -> 713 us with the conv and
@@ -322,6 +335,21 @@ extern "C" int cdssm_b200_rmsnorm_fwd(const void* x, const void* weight, void* o
     const unsigned blocks = (unsigned)((rows + 7) / 8);
     DISPATCH_DTYPE(dtype, return launch_overlapped(rmsnorm_fwd_kernel<T>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream,
                                                    (const T*)x, (const T*)weight, (T*)out, (long long)rows, d, eps));
+}
+
+extern "C" int cdssm_b200_residual_mix(const float* const* v_gates, int n_layers, int H, void* mix, int dtype, void* stream) {
+    if (!v_gates || !mix || n_layers < 0 || H <= 0) return CDSSM_ERR_BAD_ARG;
+    for (int l0 = 0; l0 < n_layers; l0 += kMixLayers) {
+        MixGates g;
+        const int n = n_layers - l0 < kMixLayers ? n_layers - l0 : kMixLayers;
+        for (int i = 0; i < n; i++)
+            if (!(g.of[i] = v_gates[l0 + i])) return CDSSM_ERR_BAD_ARG;
+        int rc = CDSSM_OK;
+        DISPATCH_DTYPE(dtype, rc = launch_overlapped(residual_mix_kernel<T>, dim3(n), dim3(H < 128 ? H : 128), 0, (cudaStream_t)stream, g,
+                                                     (T*)mix + (size_t)l0 * H, H));
+        if (rc) return rc;
+    }
+    return CDSSM_OK;
 }
 
 static int check_gn(int di, int groups) {

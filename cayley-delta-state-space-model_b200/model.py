@@ -103,12 +103,17 @@ class CdssmBlockParams:
 
 
     def merge_q_and_gate_projections(self):
-        """Q_proj and gate_proj read the same conv output: keep their weights as the two row blocks of ONE matrix,
-        so that a decode step runs one product for both (the separate weights stay available as views)."""
+        """Q_proj and gate_proj read the same conv output: keep their weights as the two row blocks of ONE matrix, so that
+        one product serves both.  The separate weights stay available as views: a write into one is seen, and after an
+        assignment to one each has its own product until this is called again."""
         di = self.w_q.shape[0]
         self.w_qg = torch.cat([self.w_q, self.w_gate]).contiguous()
         self.b_qg = torch.cat([torch.zeros(di, device=self.b_gate.device, dtype=self.b_gate.dtype), self.b_gate])
-        self.w_q, self.w_gate = self.w_qg[:di], self.w_qg[di:]
+        self.w_q, self.w_gate, self.b_gate = self.w_qg[:di], self.w_qg[di:], self.b_qg[di:]
+
+    def residual_mix(self, dtype):
+        """sigmoid(v_residual_gate) in the activation dtype (block.py:167-171)."""
+        return torch.sigmoid(self.v_residual_gate).to(dtype)[None, None, :, None]
 
     # Every assignment to an attribute counts: the model lays its weights out for the native path once per state.
     version = 0
@@ -176,10 +181,11 @@ class CdssmLM:
 
     def _native(self):
         """The model as the native path holds it (csrc/host/lm.cpp: the blocks' layers, one call per pass).  Rebuilt when a
-        weight tensor was replaced; writes into the tensors themselves are seen anyway."""
-        key = (id(self.embedding), id(self.final_norm_w), *[(id(p), p.version) for p in self.blocks])
+        weight tensor was replaced; writes into the tensors and assignments to their ``data`` are seen anyway."""
+        c = self.cfg
+        key = (id(self.embedding), id(self.final_norm_w), c.state_dim, c.chunk_size, c.ssm_norm_groups, c.eps_norm, *c.dyn_consts,
+               *[(id(p), p.version) for p in self.blocks])
         if self._plan is None or self._plan[0] != key:
-            c = self.cfg
             plan = ops._lib.host().lm_plan(c.d_model, c.d_inner, c.n_heads, c.state_dim, c.chunk_size, c.ssm_norm_groups,
                                            c.eps_norm, *c.dyn_consts, self.embedding, self.final_norm_w,
                                            [p.native() for p in self.blocks])

@@ -147,6 +147,10 @@ CDSSM_API int cdssm_b200_conv1d_silu_strided_fwd(const void* x, int64_t x_row_st
 
 /* ---- block glue: the memory-bound steps either side of the scan, one kernel each -------------------- */
 
+/* Weights of the value residual (cdssm/models/block.py:167-171): mix (n_layers,H) = sigmoid(v_gates[layer]) in the storage
+ * type.  v_gates: HOST array of n_layers device pointers to H floats each. */
+CDSSM_API int cdssm_b200_residual_mix(const float* const* v_gates, int n_layers, int H, void* mix, int dtype, void* stream);
+
 /* RMSNorm over the last dimension: out = (x * rsqrt(mean(x^2) + eps)) * weight, rows x d, d a multiple of 8,
  * 16-byte aligned buffers (CDSSM_ERR_UNSUPPORTED otherwise).
  * Replaces RMSNorm.forward, cdssm/models/modules.py:50-53 (four eager kernels). */
