@@ -8,6 +8,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <array>
+#include <mutex>
 #include <string>
 
 #include "../../../include/cdssm_b200.h"
@@ -66,9 +67,11 @@ struct Dyn {   // the five scalars of the dynamics
 };
 
 // The grow-only scratch buffer of a (device, current stream): 256-byte aligned start and usable bytes.
+// While it lives, no other thread launches with that buffer.
 struct Workspace {
     void* ptr;
     size_t bytes;
+    std::unique_lock<std::mutex> hold;
 };
 Workspace workspace(const Tensor& on, size_t bytes);
 void* workspace_if_any(int device);   // start of the buffer of (device, its current stream), or nullptr
@@ -150,12 +153,27 @@ PyObject* guarded(F&& fn) {
         PyObject* t = PyObject_GetAttrString(PyImport_AddModule("torch"), "OutOfMemoryError");
         PyErr_SetString(t ? t : PyExc_RuntimeError, e.what_without_backtrace());
         Py_XDECREF(t);
+    } catch (const c10::IndexError& e) {
+        PyErr_SetString(PyExc_IndexError, e.what_without_backtrace());
+    } catch (const c10::ValueError& e) {
+        PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
+    } catch (const c10::TypeError& e) {
+        PyErr_SetString(PyExc_TypeError, e.what_without_backtrace());
     } catch (const c10::Error& e) {
         PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
     } catch (const std::exception& e) {
         if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
     }
     return nullptr;
+}
+// Runs fn without the interpreter's lock, so that other threads of the program go on while a pass is launched.
+template <typename F>
+auto without_gil(F&& fn) {
+    struct Released {
+        PyThreadState* state = PyEval_SaveThread();
+        ~Released() { PyEval_RestoreThread(state); }
+    } released;
+    return fn();
 }
 inline PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
 

@@ -417,12 +417,12 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t flags = in.integer();
         const NoGrad ng;
         const auto lay = layout_of(p);
-        return wrap([&] {
+        return wrap(without_gil([&] {
             const c10::cuda::CUDAGuard guard(p.embedding.device());
             const Tensor x = embed(p, ids), ws = gemm_workspace(x);
             run_blocks(p, *lay, x, nullptr, per_token, flags, ws);
             return head(p, x, ws);
-        }());
+        }));
     });
 }
 
@@ -436,14 +436,14 @@ PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const NoGrad ng;
         const auto lay = layout_of(p);
         std::vector<Cache> caches(lay->blocks.size());
-        Tensor logits = [&] {
+        Tensor logits = without_gil([&] {
             const c10::cuda::CUDAGuard guard(p.embedding.device());
             Tensor x = embed(p, ids);
             const Tensor ws = gemm_workspace(x);
             run_blocks(p, *lay, x, &caches, true, 0, ws);
             if (last_only) x = x.slice(1, x.size(1) - 1, x.size(1));
             return head(p, x, ws);
-        }();
+        });
         PyObject* list = PyList_New(2 * (Py_ssize_t)caches.size());
         if (!list) return nullptr;
         for (size_t i = 0; i < caches.size(); i++) {
@@ -475,7 +475,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
             throw Error("a tensor position must be an int32 CUDA tensor");
         const NoGrad ng;
         const auto lay = layout_of(p);
-        return wrap([&] {
+        return wrap(without_gil([&] {
             const c10::cuda::CUDAGuard guard(p.embedding.device());
             const int64_t B = ids.size(0);
             Tensor x = embed(p, ids).view({B, p.d_model}), v_first;
@@ -489,7 +489,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
             for (size_t i = 0; i < layers; i++)
                 block_step(p, lay->blocks[i], mixes.at(i), x, v_first, caches[i].state, caches[i].conv, pos, pos_dev, ws);
             return head(p, x.view({B, p.d_model}), ws);
-        }());
+        }));
     });
 }
 

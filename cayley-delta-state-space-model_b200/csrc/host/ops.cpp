@@ -24,32 +24,35 @@ void check(int rc, const char* what) {
 }
 
 namespace {
+struct Buffer {
+    std::mutex launching;   // held while a call's kernels are put on the stream: two threads may share one
+    Tensor memory;
+};
 std::mutex g_ws_mutex;
 // never destroyed: the tensors must not outlive the CUDA context at process exit
-std::map<std::pair<int, void*>, Tensor>& buffers() {
-    static auto* m = new std::map<std::pair<int, void*>, Tensor>();
-    return *m;
-}
-Workspace aligned(const Tensor& buf) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(buf.data_ptr());
-    const size_t off = (size_t)(-p & 255);
-    return {reinterpret_cast<void*>(p + off), (size_t)buf.numel() - off};
+Buffer& buffer_of(const std::pair<int, void*>& key) {
+    static auto* m = new std::map<std::pair<int, void*>, Buffer>();
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    return (*m)[key];
 }
 }  // namespace
 
 Workspace workspace(const Tensor& on, size_t bytes) {
-    const std::pair<int, void*> key{on.device().index(), stream_of(on)};
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    Tensor& buf = buffers()[key];
-    if (!buf.defined() || (size_t)buf.numel() < bytes + 256)
-        buf = at::empty({(int64_t)bytes + 512}, on.options().dtype(at::kByte));
-    return aligned(buf);
+    Buffer& b = buffer_of({on.device().index(), stream_of(on)});
+    std::unique_lock<std::mutex> hold(b.launching);
+    if (!b.memory.defined() || (size_t)b.memory.numel() < bytes + 256)
+        b.memory = at::empty({(int64_t)bytes + 512}, on.options().dtype(at::kByte));
+    const uintptr_t p = reinterpret_cast<uintptr_t>(b.memory.data_ptr());
+    const size_t off = (size_t)(-p & 255);
+    return {reinterpret_cast<void*>(p + off), (size_t)b.memory.numel() - off, std::move(hold)};
 }
 
 void* workspace_if_any(int device) {
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    auto it = buffers().find({device, c10::cuda::getCurrentCUDAStream(device).stream()});
-    return it == buffers().end() ? nullptr : aligned(it->second).ptr;
+    Buffer& b = buffer_of({device, c10::cuda::getCurrentCUDAStream(device).stream()});
+    std::lock_guard<std::mutex> hold(b.launching);
+    if (!b.memory.defined()) return nullptr;
+    const uintptr_t p = reinterpret_cast<uintptr_t>(b.memory.data_ptr());
+    return reinterpret_cast<void*>(p + (size_t)(-p & 255));
 }
 
 ScanOut scan_fused(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gate_, const Tensor& lds_,
@@ -291,7 +294,9 @@ PyObject* py_decode_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
         else pos = in.integer();
         const double shortcut = in.number();
         const Tensor out = in.tensor_or_none("out"), v_first = in.tensor_or_none("v_first"), mix = in.tensor_or_none("mix");
-        return wrap(decode_step(state, q, k, v, g, lds, rope, dyn, H, N, pos, pos_dev, shortcut, out, v_first, mix));
+        return wrap(without_gil([&] {
+            return decode_step(state, q, k, v, g, lds, rope, dyn, H, N, pos, pos_dev, shortcut, out, v_first, mix);
+        }));
     });
 }
 
@@ -309,7 +314,9 @@ PyObject* py_scan_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t flags = in.integer();
         const Tensor out = in.tensor_or_none("out");
         const int64_t segs = in.integer();
-        ScanOut o = scan_fused(q, k, v, g, lds, rope, dyn, H, N, C, h0, shortcut, pos0, tail, flags, out, segs);
+        ScanOut o = without_gil([&] {
+            return scan_fused(q, k, v, g, lds, rope, dyn, H, N, C, h0, shortcut, pos0, tail, flags, out, segs);
+        });
         PyObject* t = PyTuple_New(tail ? 3 : 2);
         if (!t) return nullptr;
         PyTuple_SET_ITEM(t, 0, wrap(o.y));
@@ -331,7 +338,7 @@ PyObject* py_scan_fused_long(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor h0 = in.tensor_or_none("h0");
         const double shortcut = in.number();
         const int64_t pos0 = in.integer(), flags = in.integer(), S = in.integer();
-        const auto o = scan_fused_long(q, k, v, g, lds, rope, dyn, H, N, C, h0, shortcut, pos0, flags, S);
+        const auto o = without_gil([&] { return scan_fused_long(q, k, v, g, lds, rope, dyn, H, N, C, h0, shortcut, pos0, flags, S); });
         PyObject* t = PyTuple_New(2);
         if (!t) return nullptr;
         PyTuple_SET_ITEM(t, 0, wrap(o[0]));
@@ -344,7 +351,8 @@ PyObject* py_rms_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&] {
         Args in{a, n};
         const Tensor x = in.tensor("x"), w = in.tensor("weight");
-        return wrap(rms_norm(x, w, in.number()));
+        const double eps = in.number();
+        return wrap(without_gil([&] { return rms_norm(x, w, eps); }));
     });
 }
 
@@ -355,7 +363,8 @@ PyObject* py_groupnorm_gate(PyObject*, PyObject* const* a, Py_ssize_t n) {
                      sk = in.tensor("skip"), xc = in.tensor("x_conv");
         const int64_t groups = in.integer();
         const double eps = in.number();
-        return wrap(groupnorm_gate(y, gw, gb, z, sk, xc, groups, eps, in.flag()));
+        const bool per_token = in.flag();
+        return wrap(without_gil([&] { return groupnorm_gate(y, gw, gb, z, sk, xc, groups, eps, per_token); }));
     });
 }
 
@@ -363,7 +372,7 @@ PyObject* py_conv1d_silu_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&] {
         Args in{a, n};
         const Tensor x = in.tensor("x"), hist = in.tensor("hist"), w = in.tensor("weight"), b = in.tensor("bias");
-        return wrap(conv1d_silu_step(x, hist, w, b));
+        return wrap(without_gil([&] { return conv1d_silu_step(x, hist, w, b); }));
     });
 }
 
@@ -372,7 +381,8 @@ PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&] {
         Args in{a, n};
         const Tensor on = in.tensor("tensor");
-        const Workspace w = workspace(on, (size_t)in.integer());
+        const size_t bytes = (size_t)in.integer();
+        const Workspace w = without_gil([&] { return workspace(on, bytes); });
         return Py_BuildValue("(Kn)", (unsigned long long)reinterpret_cast<uintptr_t>(w.ptr), (Py_ssize_t)w.bytes);
     });
 }
@@ -381,7 +391,8 @@ PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_workspace_address(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&] {
         Args in{a, n};
-        return PyLong_FromUnsignedLongLong(reinterpret_cast<uintptr_t>(workspace_if_any((int)in.integer())));
+        const int device = (int)in.integer();
+        return PyLong_FromUnsignedLongLong(reinterpret_cast<uintptr_t>(without_gil([&] { return workspace_if_any(device); })));
     });
 }
 

@@ -33,11 +33,13 @@ PyObject* py_conv_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t B = x.size(0), L = x.size(1), Dm = x.size(2);
         const Tensor w = prep(cast(weight.detach(), x.scalar_type()), "weight").reshape({Dm, 4});
         const Tensor b = prep(cast(bias.detach(), x.scalar_type()), "bias");
-        const c10::cuda::CUDAGuard guard(x.device());
-        const Tensor out = at::empty_like(x);
-        check(cdssm_b200_conv1d_silu_fwd(cptr(x), cptr(w), cptr(b), mptr(out), (int)B, (int)L, (int)Dm, dtype_code(x), stream_of(x)),
-              "conv1d_silu_fwd");
-        return tuple_of<4>({out, x, w, b});
+        return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
+            const c10::cuda::CUDAGuard guard(x.device());
+            const Tensor out = at::empty_like(x);
+            check(cdssm_b200_conv1d_silu_fwd(cptr(x), cptr(w), cptr(b), mptr(out), (int)B, (int)L, (int)Dm, dtype_code(x), stream_of(x)),
+                  "conv1d_silu_fwd");
+            return {out, x, w, b};
+        }));
     });
 }
 
@@ -47,13 +49,15 @@ PyObject* py_conv_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Args in{a, n};
         const Tensor g_ = in.tensor("grad_out"), x = in.tensor("x"), w = in.tensor("w"), b = in.tensor("b");
         const Tensor go = prep(cast(g_, x.scalar_type()), "grad_out");
-        const c10::cuda::CUDAGuard guard(x.device());
-        const int64_t Dm = x.size(2);
-        const Tensor gx = at::empty_like(x), gw = empty_f32({Dm, 4}, x), gb = empty_f32({Dm}, x);
-        check(cdssm_b200_conv1d_silu_bwd(cptr(go), cptr(x), cptr(w), cptr(b), mptr(gx), fmut(gw), fmut(gb), (int)x.size(0),
-                                         (int)x.size(1), (int)Dm, dtype_code(x), stream_of(x)),
-              "conv1d_silu_bwd");
-        return tuple_of<3>({gx, gw, gb});
+        return tuple_of<3>(without_gil([&]() -> std::array<Tensor, 3> {
+            const c10::cuda::CUDAGuard guard(x.device());
+            const int64_t Dm = x.size(2);
+            const Tensor gx = at::empty_like(x), gw = empty_f32({Dm, 4}, x), gb = empty_f32({Dm}, x);
+            check(cdssm_b200_conv1d_silu_bwd(cptr(go), cptr(x), cptr(w), cptr(b), mptr(gx), fmut(gw), fmut(gb), (int)x.size(0),
+                                             (int)x.size(1), (int)Dm, dtype_code(x), stream_of(x)),
+                  "conv1d_silu_bwd");
+            return {gx, gw, gb};
+        }));
     });
 }
 
@@ -67,13 +71,15 @@ PyObject* py_dynamics_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (g.size(2) != (N + 5) * H)
             throw Error("gate_raw last dim " + std::to_string(g.size(2)) + " != (state_dim+5)*n_heads = " + std::to_string((N + 5) * H));
         const Tensor lds = f32_vector(lds_, "log_dt_scale"), rope = f32_vector(rope_, "rope_freqs");
-        const c10::cuda::CUDAGuard guard(g.device());
-        const Tensor A = empty_like_dims({B, L, H, N}, g), vp = empty_like_dims({B, L, H, N / 2}, g);
-        const Tensor beta = empty_like_dims({B, L, H}, g), sel = empty_like_dims({B, L, H}, g);
-        check(cdssm_b200_dynamics_fwd(cptr(g), fptr(lds), fptr(rope), mptr(A), mptr(vp), mptr(beta), mptr(sel), d.c[0], d.c[1], d.c[2],
-                                      d.c[3], d.c[4], (int)B, (int)L, (int)H, (int)N, 0, dtype_code(g), stream_of(g)),
-              "dynamics_fwd");
-        return tuple_of<7>({A, vp, beta, sel, g, lds, rope});
+        return tuple_of<7>(without_gil([&]() -> std::array<Tensor, 7> {
+            const c10::cuda::CUDAGuard guard(g.device());
+            const Tensor A = empty_like_dims({B, L, H, N}, g), vp = empty_like_dims({B, L, H, N / 2}, g);
+            const Tensor beta = empty_like_dims({B, L, H}, g), sel = empty_like_dims({B, L, H}, g);
+            check(cdssm_b200_dynamics_fwd(cptr(g), fptr(lds), fptr(rope), mptr(A), mptr(vp), mptr(beta), mptr(sel), d.c[0], d.c[1], d.c[2],
+                                          d.c[3], d.c[4], (int)B, (int)L, (int)H, (int)N, 0, dtype_code(g), stream_of(g)),
+                  "dynamics_fwd");
+            return {A, vp, beta, sel, g, lds, rope};
+        }));
     });
 }
 
@@ -85,14 +91,16 @@ PyObject* py_dynamics_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
                      gc_ = in.tensor_or_none("grad_sel_C"), g = in.tensor("gate"), lds = in.tensor("lds"), rope = in.tensor("rope");
         const Dyn d = in.dyn();
         const int64_t H = in.integer(), N = in.integer(), B = g.size(0), L = g.size(1);
-        const c10::cuda::CUDAGuard guard(g.device());
-        const Tensor gA = grad_or_zeros(gA_, {B, L, H, N}, g), gvp = grad_or_zeros(gvp_, {B, L, H, N / 2}, g);
-        const Tensor gb = grad_or_zeros(gb_, {B, L, H}, g), gc = grad_or_zeros(gc_, {B, L, H}, g);
-        const Tensor gg = at::empty_like(g), gl = empty_f32({H}, g);
-        check(cdssm_b200_dynamics_bwd(cptr(gA), cptr(gvp), cptr(gb), cptr(gc), cptr(g), fptr(lds), fptr(rope), mptr(gg), fmut(gl), d.c[0],
-                                      d.c[1], d.c[2], d.c[3], d.c[4], (int)B, (int)L, (int)H, (int)N, 0, dtype_code(g), stream_of(g)),
-              "dynamics_bwd");
-        return tuple_of<2>({gg, gl});
+        return tuple_of<2>(without_gil([&]() -> std::array<Tensor, 2> {
+            const c10::cuda::CUDAGuard guard(g.device());
+            const Tensor gA = grad_or_zeros(gA_, {B, L, H, N}, g), gvp = grad_or_zeros(gvp_, {B, L, H, N / 2}, g);
+            const Tensor gb = grad_or_zeros(gb_, {B, L, H}, g), gc = grad_or_zeros(gc_, {B, L, H}, g);
+            const Tensor gg = at::empty_like(g), gl = empty_f32({H}, g);
+            check(cdssm_b200_dynamics_bwd(cptr(gA), cptr(gvp), cptr(gb), cptr(gc), cptr(g), fptr(lds), fptr(rope), mptr(gg), fmut(gl), d.c[0],
+                                          d.c[1], d.c[2], d.c[3], d.c[4], (int)B, (int)L, (int)H, (int)N, 0, dtype_code(g), stream_of(g)),
+                  "dynamics_bwd");
+            return {gg, gl};
+        }));
     });
 }
 
@@ -103,11 +111,13 @@ PyObject* py_normalize_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor K = prep(in.tensor("K"), "K"), Q = dense(in.tensor("Q"), K.scalar_type(), "Q");
         if (K.sizes() != Q.sizes()) throw Error("K and Q must have the same shape");
         const int64_t D = K.size(-1);
-        const c10::cuda::CUDAGuard guard(K.device());
-        const Tensor Ko = at::empty_like(K), Qo = at::empty_like(Q);
-        check(cdssm_b200_normalize_kq_fwd(cptr(K), cptr(Q), mptr(Ko), mptr(Qo), K.numel() / D, (int)D, dtype_code(K), stream_of(K)),
-              "normalize_kq_fwd");
-        return tuple_of<4>({Ko, Qo, K, Q});
+        return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
+            const c10::cuda::CUDAGuard guard(K.device());
+            const Tensor Ko = at::empty_like(K), Qo = at::empty_like(Q);
+            check(cdssm_b200_normalize_kq_fwd(cptr(K), cptr(Q), mptr(Ko), mptr(Qo), K.numel() / D, (int)D, dtype_code(K), stream_of(K)),
+                  "normalize_kq_fwd");
+            return {Ko, Qo, K, Q};
+        }));
     });
 }
 
@@ -117,13 +127,15 @@ PyObject* py_normalize_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Args in{a, n};
         const Tensor gk_ = in.tensor_or_none("grad_K_out"), gq_ = in.tensor_or_none("grad_Q_out"), K = in.tensor("K"), Q = in.tensor("Q");
         const int64_t D = K.size(-1);
-        const c10::cuda::CUDAGuard guard(K.device());
-        const Tensor gKo = grad_or_zeros(gk_, K.sizes(), K), gQo = grad_or_zeros(gq_, K.sizes(), K);
-        const Tensor gK = at::empty_like(K), gQ = at::empty_like(Q);
-        check(cdssm_b200_normalize_kq_bwd(cptr(gKo), cptr(gQo), cptr(K), cptr(Q), mptr(gK), mptr(gQ), K.numel() / D, (int)D,
-                                          dtype_code(K), stream_of(K)),
-              "normalize_kq_bwd");
-        return tuple_of<2>({gK, gQ});
+        return tuple_of<2>(without_gil([&]() -> std::array<Tensor, 2> {
+            const c10::cuda::CUDAGuard guard(K.device());
+            const Tensor gKo = grad_or_zeros(gk_, K.sizes(), K), gQo = grad_or_zeros(gq_, K.sizes(), K);
+            const Tensor gK = at::empty_like(K), gQ = at::empty_like(Q);
+            check(cdssm_b200_normalize_kq_bwd(cptr(gKo), cptr(gQo), cptr(K), cptr(Q), mptr(gK), mptr(gQ), K.numel() / D, (int)D,
+                                              dtype_code(K), stream_of(K)),
+                  "normalize_kq_bwd");
+            return {gK, gQ};
+        }));
     });
 }
 
@@ -135,12 +147,14 @@ PyObject* py_intra_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const auto dt = K.scalar_type();
         const Tensor A = dense(A_, dt, "A_flat"), V = dense(V_, dt, "V_flat"), be = dense(b_, dt, "beta_flat");
         const int64_t N = in.integer(), M = K.size(0), C = K.size(1), H = K.size(2), D = K.size(3);
-        const c10::cuda::CUDAGuard guard(K.device());
-        const Tensor h = empty_like_dims({M, C, H, N, D}, K), cum = empty_like_dims({M, C, H, N}, K);
-        check(cdssm_b200_intra_chunk_scan_fwd(cptr(A), cptr(K), cptr(V), cptr(be), mptr(h), mptr(cum), (int)M, (int)C, (int)H, (int)D,
-                                              (int)N, dtype_code(K), stream_of(K)),
-              "intra_chunk_scan_fwd");
-        return tuple_of<6>({h, cum, A, K, V, be});
+        return tuple_of<6>(without_gil([&]() -> std::array<Tensor, 6> {
+            const c10::cuda::CUDAGuard guard(K.device());
+            const Tensor h = empty_like_dims({M, C, H, N, D}, K), cum = empty_like_dims({M, C, H, N}, K);
+            check(cdssm_b200_intra_chunk_scan_fwd(cptr(A), cptr(K), cptr(V), cptr(be), mptr(h), mptr(cum), (int)M, (int)C, (int)H, (int)D,
+                                                  (int)N, dtype_code(K), stream_of(K)),
+                  "intra_chunk_scan_fwd");
+            return {h, cum, A, K, V, be};
+        }));
     });
 }
 
@@ -151,14 +165,16 @@ PyObject* py_intra_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor gh_ = in.tensor_or_none("grad_local_h"), gc_ = in.tensor_or_none("grad_cum_A"), A = in.tensor("A"), K = in.tensor("K"),
                      V = in.tensor("V"), be = in.tensor("beta"), h = in.tensor("local_h"), cum = in.tensor("cum_A");
         const int64_t N = in.integer(), M = K.size(0), C = K.size(1), H = K.size(2), D = K.size(3);
-        const c10::cuda::CUDAGuard guard(K.device());
-        const Tensor gh = grad_or_zeros(gh_, h.sizes(), K), gc = grad_or_zeros(gc_, cum.sizes(), K);
-        const Tensor gA = at::empty_like(A), gV = at::empty_like(V), gK = empty_f32({M, C, H, D}, K), gB = empty_f32({M, C, H}, K);
-        check(cdssm_b200_intra_chunk_scan_bwd(cptr(gh), cptr(gc), cptr(A), cptr(K), cptr(V), cptr(be), cptr(h), cptr(cum), mptr(gA),
-                                              fmut(gK), mptr(gV), fmut(gB), (int)M, (int)C, (int)H, (int)D, (int)N, dtype_code(K),
-                                              stream_of(K)),
-              "intra_chunk_scan_bwd");
-        return tuple_of<4>({gA, cast(gK, K.scalar_type()), gV, cast(gB, K.scalar_type())});
+        return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
+            const c10::cuda::CUDAGuard guard(K.device());
+            const Tensor gh = grad_or_zeros(gh_, h.sizes(), K), gc = grad_or_zeros(gc_, cum.sizes(), K);
+            const Tensor gA = at::empty_like(A), gV = at::empty_like(V), gK = empty_f32({M, C, H, D}, K), gB = empty_f32({M, C, H}, K);
+            check(cdssm_b200_intra_chunk_scan_bwd(cptr(gh), cptr(gc), cptr(A), cptr(K), cptr(V), cptr(be), cptr(h), cptr(cum), mptr(gA),
+                                                  fmut(gK), mptr(gV), fmut(gB), (int)M, (int)C, (int)H, (int)D, (int)N, dtype_code(K),
+                                                  stream_of(K)),
+                  "intra_chunk_scan_bwd");
+            return {gA, cast(gK, K.scalar_type()), gV, cast(gB, K.scalar_type())};
+        }));
     });
 }
 
@@ -168,12 +184,14 @@ PyObject* py_inter_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Args in{a, n};
         const Tensor A_ = in.tensor("total_A"), f = prep(in.tensor("final_local_h"), "final_local_h"), A = dense(A_, f.scalar_type(), "total_A");
         const int64_t N = in.integer();
-        const c10::cuda::CUDAGuard guard(f.device());
-        const Tensor out = at::empty_like(f);
-        check(cdssm_b200_inter_chunk_scan_fwd(cptr(A), cptr(f), mptr(out), (int)f.size(0), (int)f.size(1), (int)f.size(2), (int)f.size(4),
-                                              (int)N, dtype_code(f), stream_of(f)),
-              "inter_chunk_scan_fwd");
-        return tuple_of<2>({out, A});
+        return tuple_of<2>(without_gil([&]() -> std::array<Tensor, 2> {
+            const c10::cuda::CUDAGuard guard(f.device());
+            const Tensor out = at::empty_like(f);
+            check(cdssm_b200_inter_chunk_scan_fwd(cptr(A), cptr(f), mptr(out), (int)f.size(0), (int)f.size(1), (int)f.size(2), (int)f.size(4),
+                                                  (int)N, dtype_code(f), stream_of(f)),
+                  "inter_chunk_scan_fwd");
+            return {out, A};
+        }));
     });
 }
 
@@ -184,12 +202,14 @@ PyObject* py_inter_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor g_ = in.tensor("grad_chunk_states"), A = in.tensor("total_A"), s = in.tensor("chunk_states");
         const int64_t N = in.integer();
         const Tensor g = prep(cast(g_, s.scalar_type()), "grad_chunk_states");
-        const c10::cuda::CUDAGuard guard(s.device());
-        const Tensor gA = at::empty_like(A), gH = at::empty_like(s);
-        check(cdssm_b200_inter_chunk_scan_bwd(cptr(g), cptr(A), cptr(s), mptr(gA), mptr(gH), (int)s.size(0), (int)s.size(1), (int)s.size(2),
-                                              (int)s.size(4), (int)N, dtype_code(s), stream_of(s)),
-              "inter_chunk_scan_bwd");
-        return tuple_of<2>({gA, gH});
+        return tuple_of<2>(without_gil([&]() -> std::array<Tensor, 2> {
+            const c10::cuda::CUDAGuard guard(s.device());
+            const Tensor gA = at::empty_like(A), gH = at::empty_like(s);
+            check(cdssm_b200_inter_chunk_scan_bwd(cptr(g), cptr(A), cptr(s), mptr(gA), mptr(gH), (int)s.size(0), (int)s.size(1), (int)s.size(2),
+                                                  (int)s.size(4), (int)N, dtype_code(s), stream_of(s)),
+                  "inter_chunk_scan_bwd");
+            return {gA, gH};
+        }));
     });
 }
 
@@ -201,12 +221,14 @@ PyObject* py_correction_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const auto dt = K.scalar_type();
         const Tensor A = dense(A_, dt, "A_chunk"), be = dense(b_, dt, "beta_chunk"), s = dense(s_, dt, "chunk_states");
         const int64_t N = in.integer(), B = K.size(0), NC = K.size(1), C = K.size(2), H = K.size(3), D = K.size(4);
-        const c10::cuda::CUDAGuard guard(K.device());
-        const Tensor out = empty_like_dims({B, NC, C, H, N, D}, K);
-        check(cdssm_b200_exact_correction_fwd(cptr(A), cptr(K), cptr(be), cptr(s), mptr(out), (int)B, (int)NC, (int)C, (int)H, (int)D, (int)N,
-                                              dtype_code(K), stream_of(K)),
-              "exact_correction_fwd");
-        return tuple_of<4>({out, A, K, be});
+        return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
+            const c10::cuda::CUDAGuard guard(K.device());
+            const Tensor out = empty_like_dims({B, NC, C, H, N, D}, K);
+            check(cdssm_b200_exact_correction_fwd(cptr(A), cptr(K), cptr(be), cptr(s), mptr(out), (int)B, (int)NC, (int)C, (int)H, (int)D, (int)N,
+                                                  dtype_code(K), stream_of(K)),
+                  "exact_correction_fwd");
+            return {out, A, K, be};
+        }));
     });
 }
 
@@ -217,13 +239,15 @@ PyObject* py_correction_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor g_ = in.tensor("grad_corrections"), A = in.tensor("A"), K = in.tensor("K"), be = in.tensor("beta"), c = in.tensor("corrections");
         const int64_t N = in.integer(), order = in.integer(), B = K.size(0), NC = K.size(1), C = K.size(2), H = K.size(3), D = K.size(4);
         const Tensor g = prep(cast(g_, K.scalar_type()), "grad_corrections");
-        const c10::cuda::CUDAGuard guard(K.device());
-        const Tensor gA = at::empty_like(A), gK = empty_f32({B, NC, C, H, D}, K), gB = empty_f32({B, NC, C, H}, K);
-        const Tensor gS = empty_like_dims({B, NC, H, N, D}, K);
-        check(cdssm_b200_exact_correction_bwd(cptr(g), cptr(A), cptr(K), cptr(be), cptr(c), mptr(gA), fmut(gK), fmut(gB), mptr(gS), (int)B,
-                                              (int)NC, (int)C, (int)H, (int)D, (int)N, (int)order, dtype_code(K), stream_of(K)),
-              "exact_correction_bwd");
-        return tuple_of<4>({gA, cast(gK, K.scalar_type()), cast(gB, K.scalar_type()), gS});
+        return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
+            const c10::cuda::CUDAGuard guard(K.device());
+            const Tensor gA = at::empty_like(A), gK = empty_f32({B, NC, C, H, D}, K), gB = empty_f32({B, NC, C, H}, K);
+            const Tensor gS = empty_like_dims({B, NC, H, N, D}, K);
+            check(cdssm_b200_exact_correction_bwd(cptr(g), cptr(A), cptr(K), cptr(be), cptr(c), mptr(gA), fmut(gK), fmut(gB), mptr(gS), (int)B,
+                                                  (int)NC, (int)C, (int)H, (int)D, (int)N, (int)order, dtype_code(K), stream_of(K)),
+                  "exact_correction_bwd");
+            return {gA, cast(gK, K.scalar_type()), cast(gB, K.scalar_type()), gS};
+        }));
     });
 }
 

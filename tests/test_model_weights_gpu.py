@@ -113,3 +113,31 @@ def test_residual_mix_equals_the_eager_operation(ops, dtype):
                                                 torch.cuda.current_stream().cuda_stream)
     assert rc == 0
     assert torch.equal(out, torch.stack([torch.sigmoid(t).to(dtype) for t in gates]))
+
+
+def test_other_threads_run_during_a_pass(ops):
+    """A native call does not hold the interpreter's lock while it launches a pass: another thread ticks inside it."""
+    import threading
+    import time
+    lm = _model(n_layers=48)
+    ids = torch.randint(0, 503, (1, 40), device="cuda")
+    lm.forward(ids)
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0)
+
+    t = threading.Thread(target=tick)
+    t.start()
+    spans = []
+    for _ in range(20):
+        t0 = time.perf_counter()
+        lm.forward(ids)
+        spans.append((t0, time.perf_counter()))
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    inside = [sum(a < x < b for x in ticks) for a, b in spans]
+    assert sorted(inside)[len(inside) // 2] >= 5, inside      # (one may fall between the call and the clock)

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from test_scan_gpu import run_fused, unnormalise
-from util import to_dev, to_np
+from util import const_args, to_dev, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -101,3 +101,30 @@ def test_tokens_before_a_bad_value_do_not_see_it(ops, orc, D, N, value, what):
         ok = np.isfinite(b)
         assert np.abs(a[ok] - b[ok]).max() <= 2e-2 * np.abs(b[ok]).max()
     assert np.isfinite(to_np(y)[0, :t]).all()
+
+
+def test_two_threads_share_a_stream(ops, orc):
+    """Scans of two sizes from two threads on one stream: each uses the stream's scratch buffer for itself."""
+    import threading
+    sizes = [(2, 4, 700, 64, 2), (1, 3, 300, 64, 16)]
+    calls, want = [], []
+    for B, H, L, D, N in sizes:
+        inp = orc.make_inputs(B, H, L, D, N=N, seed=N, bf16=True)
+        d = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+        args = [d(inp[k]).bfloat16() for k in ("q", "k", "v", "gate_raw")] + [d(inp["log_dt_scale"]), d(inp["rope_freqs"]),
+                                                                             *const_args(inp["consts"]), H, N, D]
+        calls.append(args)
+        want.append(ops.scan_fused(*args, return_tail_state=True))
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        for _ in range(150):
+            got = ops.scan_fused(*calls[i], return_tail_state=True)
+            if not all(torch.equal(a, b) for a, b in zip(got, want[i])):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in (0, 1, 0, 1)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
