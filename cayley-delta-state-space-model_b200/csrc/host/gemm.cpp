@@ -116,8 +116,10 @@ void gemm_raw(int device, void* out, int64_t ldo, const void* x, int64_t ldx, co
 void gemm(const Tensor& out, const Tensor& x, const Tensor& w, const Tensor& bias, bool accumulate, const Tensor& workspace) {
     const int64_t rows = x.size(0), K = x.size(1), M = w.size(0);
     if (rows == 0) return;
-    const bool plain = x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.stride(1) == 1 && w.is_contiguous() &&
-                       out.stride(1) == 1 && (x.stride(0) | out.stride(0) | K) % 8 == 0 && aligned16(x) && aligned16(w) &&
+    const bool fits = w.dim() == 2 && w.size(1) == K && out.size(0) == rows && out.size(1) == M &&
+                      (!bias.defined() || (bias.dim() == 1 && bias.size(0) == M && bias.scalar_type() == w.scalar_type()));
+    const bool plain = fits && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.stride(1) == 1 &&
+                       w.is_contiguous() && out.stride(1) == 1 && (x.stride(0) | out.stride(0) | K) % 8 == 0 && aligned16(x) && aligned16(w) &&
                        aligned16(out) && (!bias.defined() || aligned16(bias));
     if (!plain) {   // float32 models, widths that are no multiple of eight
         if (accumulate) out.add_(at::linear(x, w, bias));

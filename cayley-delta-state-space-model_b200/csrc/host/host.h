@@ -50,6 +50,11 @@ inline Tensor f32_vector(const Tensor& t, const char* name) {
     return t.detach().to(at::kFloat).contiguous();
 }
 
+// (sizes are read by position below: another rank would be taken for a batch of its first dimensions)
+inline void need_dims(const Tensor& t, int64_t n, const char* name) {
+    if (t.dim() != n) throw Error(std::string(name) + " must have " + std::to_string(n) + " dimensions, not " + std::to_string(t.dim()));
+}
+
 inline const void* cptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
 inline void* mptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline const float* fptr(const Tensor& t) { return t.defined() ? static_cast<const float*>(t.const_data_ptr()) : nullptr; }

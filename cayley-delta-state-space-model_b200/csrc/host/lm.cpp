@@ -407,6 +407,11 @@ PyObject* py_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// (B, L) token ids, or an error as the layers' shapes would have given.
+void need_batch(const Tensor& ids) {
+    if (ids.dim() != 2) throw Error("input_ids must be (batch, length)");
+}
+
 // lm_forward(plan, ids, per_token_group_norm, scan_flags) -> logits (B,L,vocab)
 PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -415,6 +420,7 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor ids = in.tensor("input_ids");
         const bool per_token = in.flag();
         const int64_t flags = in.integer();
+        need_batch(ids);
         const NoGrad ng;
         const auto lay = layout_of(p);
         return wrap(without_gil([&] {
@@ -433,6 +439,7 @@ PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Plan& p = plan_of(in.next());
         const Tensor ids = in.tensor("input_ids");
         const bool last_only = in.flag();
+        need_batch(ids);
         const NoGrad ng;
         const auto lay = layout_of(p);
         std::vector<Cache> caches(lay->blocks.size());
@@ -471,6 +478,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
         int64_t pos = 0;
         if (in.at < n && THPVariable_Check(a[in.at])) pos_dev = in.tensor("pos");
         else pos = in.integer();
+        if (ids.dim() != 1) throw Error("token_ids must be (batch)");
         if (pos_dev.defined() && (pos_dev.scalar_type() != at::kInt || !pos_dev.is_cuda()))
             throw Error("a tensor position must be an int32 CUDA tensor");
         const NoGrad ng;

@@ -135,6 +135,7 @@ std::array<Tensor, 2> scan_fused_long(const Tensor& q_, const Tensor& k_, const 
     const Tensor q = q_.is_contiguous() ? q_ : q_.contiguous();
     const Tensor k = dense(k_, q.scalar_type(), "k"), v = dense(v_, q.scalar_type(), "v");
     const Tensor g = dense(gate_, q.scalar_type(), "gate_raw");
+    need_dims(q, 4, "q");
     const int64_t B = q.size(0), L = q.size(1), H = q.size(2), D = q.size(3), R = B * S, Ls = L / S;
     if (H != heads || k.sizes() != q.sizes() || v.sizes() != at::IntArrayRef({B, L, H, N}) ||
         g.sizes() != at::IntArrayRef({B, L, (N + 5) * H}))
@@ -209,6 +210,7 @@ Tensor rms_norm(const Tensor& x_, const Tensor& w_, double eps) {
     need_cuda(x_, "x");
     const Tensor x = x_.is_contiguous() ? x_ : x_.contiguous(), w = dense(w_, x.scalar_type(), "weight");
     const int64_t d = x.size(-1);
+    if (d == 0) throw Error("rms_norm: the last dimension is empty");
     const c10::cuda::CUDAGuard guard(x.device());
     const Tensor out = at::empty_like(x);
     check(cdssm_b200_rmsnorm_fwd(cptr(x), cptr(w), mptr(out), x.numel() / d, (int)d, (float)eps, dtype_code(x), stream_of(x)),
@@ -222,6 +224,7 @@ Tensor groupnorm_gate(const Tensor& y_, const Tensor& gw_, const Tensor& gb_, co
     const Tensor y = y_.is_contiguous() ? y_ : y_.contiguous();
     const auto dt = y.scalar_type();
     const Tensor xc = dense(x_conv, dt, "x_conv");
+    need_dims(y, 3, "y");
     const int64_t B = y.size(0), L = y.size(1), di = y.size(2);
     Tensor z = z_;
     if (!z.is_cuda() || z.scalar_type() != dt || z.sizes() != y.sizes() || z.stride(-1) != 1 ||
@@ -253,6 +256,7 @@ Tensor groupnorm_gate(const Tensor& y_, const Tensor& gw_, const Tensor& gb_, co
 Tensor conv1d_silu(const Tensor& x_, const Tensor& w_, const Tensor& b_) {
     need_cuda(x_, "x");
     const Tensor x = x_.is_contiguous() ? x_ : x_.contiguous();
+    need_dims(x, 3, "x");
     const Tensor w = dense(w_.detach().to(x.scalar_type()), x.scalar_type(), "weight");
     const Tensor b = dense(b_.detach().to(x.scalar_type()), x.scalar_type(), "bias");
     const c10::cuda::CUDAGuard guard(x.device());
@@ -266,6 +270,7 @@ Tensor conv1d_silu(const Tensor& x_, const Tensor& w_, const Tensor& b_) {
 Tensor conv1d_silu_step(const Tensor& x_, const Tensor& hist, const Tensor& w_, const Tensor& b_) {
     const Tensor x = !x_.is_cuda() || x_.stride(-1) != 1 ? x_.contiguous() : x_;
     need_cuda(x, "x");
+    need_dims(x, 2, "x");
     const int64_t B = x.size(0), Dm = x.size(1);
     if (hist.scalar_type() != x.scalar_type() || !hist.is_contiguous() || hist.sizes() != at::IntArrayRef({B, 3, Dm}))
         throw Error("conv1d_silu_step: hist must be a contiguous (B,3,Dm) tensor of the input dtype");

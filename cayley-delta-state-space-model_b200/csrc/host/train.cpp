@@ -30,6 +30,7 @@ PyObject* py_conv_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Args in{a, n};
         const Tensor x = prep(in.tensor("x"), "x"), weight = in.tensor("weight"), bias = in.tensor("bias");
         if (weight.size(-1) != 4) throw Error("Only kernel_size=4 is supported");   // conv1d_silu.cu:241
+        need_dims(x, 3, "x");
         const int64_t B = x.size(0), L = x.size(1), Dm = x.size(2);
         const Tensor w = prep(cast(weight.detach(), x.scalar_type()), "weight").reshape({Dm, 4});
         const Tensor b = prep(cast(bias.detach(), x.scalar_type()), "bias");
@@ -67,6 +68,7 @@ PyObject* py_dynamics_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Args in{a, n};
         const Tensor g = prep(in.tensor("gate_raw"), "gate_raw"), lds_ = in.tensor("log_dt_scale"), rope_ = in.tensor("rope_freqs");
         const Dyn d = in.dyn();
+        need_dims(g, 3, "gate_raw");
         const int64_t H = in.integer(), N = in.integer(), B = g.size(0), L = g.size(1);
         if (g.size(2) != (N + 5) * H)
             throw Error("gate_raw last dim " + std::to_string(g.size(2)) + " != (state_dim+5)*n_heads = " + std::to_string((N + 5) * H));
@@ -111,6 +113,7 @@ PyObject* py_normalize_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor K = prep(in.tensor("K"), "K"), Q = dense(in.tensor("Q"), K.scalar_type(), "Q");
         if (K.sizes() != Q.sizes()) throw Error("K and Q must have the same shape");
         const int64_t D = K.size(-1);
+        if (D == 0) throw Error("K and Q: the last dimension is empty");
         return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
             const c10::cuda::CUDAGuard guard(K.device());
             const Tensor Ko = at::empty_like(K), Qo = at::empty_like(Q);
@@ -146,6 +149,7 @@ PyObject* py_intra_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor A_ = in.tensor("A_flat"), K = prep(in.tensor("K_flat"), "K_flat"), V_ = in.tensor("V_flat"), b_ = in.tensor("beta_flat");
         const auto dt = K.scalar_type();
         const Tensor A = dense(A_, dt, "A_flat"), V = dense(V_, dt, "V_flat"), be = dense(b_, dt, "beta_flat");
+        need_dims(K, 4, "K_flat");
         const int64_t N = in.integer(), M = K.size(0), C = K.size(1), H = K.size(2), D = K.size(3);
         return tuple_of<6>(without_gil([&]() -> std::array<Tensor, 6> {
             const c10::cuda::CUDAGuard guard(K.device());
@@ -183,6 +187,7 @@ PyObject* py_inter_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&] {
         Args in{a, n};
         const Tensor A_ = in.tensor("total_A"), f = prep(in.tensor("final_local_h"), "final_local_h"), A = dense(A_, f.scalar_type(), "total_A");
+        need_dims(f, 5, "final_local_h");
         const int64_t N = in.integer();
         return tuple_of<2>(without_gil([&]() -> std::array<Tensor, 2> {
             const c10::cuda::CUDAGuard guard(f.device());
@@ -220,6 +225,7 @@ PyObject* py_correction_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const Tensor A_ = in.tensor("A_chunk"), K = prep(in.tensor("K_chunk"), "K_chunk"), b_ = in.tensor("beta_chunk"), s_ = in.tensor("chunk_states");
         const auto dt = K.scalar_type();
         const Tensor A = dense(A_, dt, "A_chunk"), be = dense(b_, dt, "beta_chunk"), s = dense(s_, dt, "chunk_states");
+        need_dims(K, 5, "K_chunk");
         const int64_t N = in.integer(), B = K.size(0), NC = K.size(1), C = K.size(2), H = K.size(3), D = K.size(4);
         return tuple_of<4>(without_gil([&]() -> std::array<Tensor, 4> {
             const c10::cuda::CUDAGuard guard(K.device());

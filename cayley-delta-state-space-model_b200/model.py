@@ -192,17 +192,20 @@ class CdssmLM:
             self._plan = (key, plan, self.embedding, self.final_norm_w, list(self.blocks))   # ids stay taken
         return self._plan[1]
 
+    def _ids(self, ids):
+        return ids if isinstance(ids, torch.Tensor) else torch.as_tensor(ids, device=self.device)
+
     # ------------------------------------------------------------------ public API
     @torch.no_grad()
     def forward(self, input_ids, scan_flags=0):
         """Prefill: (B,L) token ids -> (B,L,vocab) logits (cdssm/models/model.py:37-51)."""
-        return ops._lib.host().lm_forward(self._native(), input_ids, self.per_token_group_norm, scan_flags)
+        return ops._lib.host().lm_forward(self._native(), self._ids(input_ids), self.per_token_group_norm, scan_flags)
 
     @torch.no_grad()
     def prefill(self, input_ids, last_only=True):
         """Prefill that also returns the decode cache: per layer the recurrent state after the last
         token (B,H,N,D) fp32 and the last three conv inputs; plus the position counter."""
-        logits, flat = ops._lib.host().lm_prefill(self._native(), input_ids, last_only)
+        logits, flat = ops._lib.host().lm_prefill(self._native(), self._ids(input_ids), last_only)
         layers = [{"state": flat[i], "conv": flat[i + 1]} for i in range(0, len(flat), 2)]
         return logits, {"layers": layers, "pos": input_ids.shape[1]}
 
@@ -214,7 +217,7 @@ class CdssmLM:
         # makes the step graph-replayable (see position())
         name = "pos_dev" if "pos_dev" in cache else "pos"
         flat = [c[n] for c in cache["layers"] for n in ("state", "conv")]
-        logits = ops._lib.host().lm_decode(self._native(), token_ids, flat, cache[name])
+        logits = ops._lib.host().lm_decode(self._native(), self._ids(token_ids), flat, cache[name])
         cache[name] += 1
         return logits
 

@@ -92,3 +92,51 @@ def test_errors_mirror_reference_checks(ops):
     A = torch.zeros(1, 4, 1, 2, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(RuntimeError):                       # intra_chunk_scan.cu:584
         ops.IntraChunkScanFn.apply(A, K, A, A[..., 0], 2)
+
+
+# What has another rank, an empty last dimension or no batch is an error: nothing is launched on sizes read from the wrong places.
+def test_wrong_ranks_are_refused(ops):
+    z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+    f = lambda *s: torch.zeros(*s, device="cuda")
+    dyn = (1.0, 0.1, 0.1, 0.02, 1.0)
+    calls = [
+        lambda: ops.CUDAConv1dSiLUOp.apply(z(2, 8, 16, 3), z(16, 1, 4), z(16)),
+        lambda: ops.CUDAConv1dSiLUOp.apply(z(8, 16), z(16, 1, 4), z(16)),
+        lambda: ops.DynamicsFusedFn.apply(z(2, 8, 7 * 3, 2), f(3), f(3), *dyn, 3, 2),
+        lambda: ops.IntraChunkScanFn.apply(z(2, 8, 3, 2), z(2, 8, 3, 64, 2), z(2, 8, 3, 2), z(2, 8, 3), 2),
+        lambda: ops.InterChunkScanFn.apply(z(2, 4, 3, 2), z(2, 4, 3, 2, 64, 2), 2),
+        lambda: ops.ExactCorrectionFn.apply(z(2, 4, 8, 3, 2), z(2, 4, 8, 3, 64, 2), z(2, 4, 8, 3), z(2, 4, 3, 2, 64), 2),
+        lambda: ops.NormalizeKQFn.apply(z(2, 3, 0), z(2, 3, 0)),
+        lambda: ops.rms_norm(z(2, 0), z(0), 1e-5),
+        lambda: ops.groupnorm_gate(z(2, 4, 64, 2), z(64), z(64), z(2, 4, 64, 2), z(64), z(2, 4, 64, 2), 8),
+        lambda: ops.conv1d_silu_step(z(2, 16, 2), z(2, 3, 16), z(16, 1, 4), z(16)),
+    ]
+    for i, call in enumerate(calls):
+        with pytest.raises((RuntimeError, ValueError, IndexError)):
+            call()
+    torch.cuda.synchronize()
+
+
+def test_wrong_ids_and_weights_are_refused(ops):
+    from cdssm_b200.model import CdssmConfig, CdssmLM
+    lm = CdssmLM(CdssmConfig(d_model=256, n_layers=2, context_length=128, vocab_size=100, state_dim=2), seed=1)
+    ids = torch.zeros(2, 8, dtype=torch.int64, device="cuda")
+    logits, cache = lm.prefill(ids)
+    with pytest.raises((RuntimeError, ValueError)):
+        lm.forward(ids[0])                                 # (L): the batch would be taken for the length
+    with pytest.raises((RuntimeError, ValueError, IndexError)):
+        lm.prefill(ids[None])
+    with pytest.raises((RuntimeError, ValueError)):
+        lm.decode(ids[:, :1], cache)
+    assert torch.isfinite(lm.forward(ids.tolist())).all()  # a list of lists indexes the embedding, as it always did
+    assert torch.isfinite(lm.decode([3, 4], cache)).all()
+    for name, shape in (("w_out", (256, 500)), ("w_readout", (512, 8)), ("w_q", (512, 256))):
+        good = getattr(lm.blocks[1], name)
+        setattr(lm.blocks[1], name, torch.zeros(*shape, device="cuda", dtype=torch.bfloat16))
+        with pytest.raises(RuntimeError):
+            lm.forward(ids)
+        setattr(lm.blocks[1], name, good)
+    odd = CdssmLM(CdssmConfig(d_model=48, n_layers=1, context_length=128, vocab_size=100, state_dim=2), seed=1)   # 96 = 1.5 heads
+    with pytest.raises(RuntimeError):
+        odd.forward(ids)
+    torch.cuda.synchronize()
