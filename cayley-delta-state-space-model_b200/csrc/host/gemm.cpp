@@ -20,15 +20,19 @@ struct Key {
     int device;
     int64_t m, n, k, ldb, ldd;
     int bias, accumulate;
+    int align_w, align_x, align_out, align_bias;   // bytes
+    int reduction;                                 // the program's setting for partial sums of a split product
     bool operator==(const Key& o) const {
         return device == o.device && m == o.m && n == o.n && k == o.k && ldb == o.ldb && ldd == o.ldd && bias == o.bias &&
-               accumulate == o.accumulate;
+               accumulate == o.accumulate && align_w == o.align_w && align_x == o.align_x && align_out == o.align_out &&
+               align_bias == o.align_bias && reduction == o.reduction;
     }
 };
 struct KeyHash {
     size_t operator()(const Key& k) const {
         size_t h = 1469598103934665603ull;
-        for (int64_t v : {(int64_t)k.device, k.m, k.n, k.k, k.ldb, k.ldd, (int64_t)(k.bias * 2 + k.accumulate)})
+        for (int64_t v : {(int64_t)k.device, k.m, k.n, k.k, k.ldb, k.ldd, (int64_t)(k.bias * 8 + k.accumulate * 4 + k.reduction),
+                          (int64_t)k.align_w << 36 | (int64_t)k.align_x << 24 | (int64_t)k.align_out << 12 | k.align_bias})
             h = (h ^ (size_t)v) * 1099511628211ull;
         return h;
     }
@@ -79,6 +83,20 @@ Plan& plan_for(const Key& key) {
     lt_check(cublasLtMatmulPreferenceCreate(&pref), "preference");
     const size_t ws = kGemmWorkspace;
     cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &ws, sizeof(ws));
+    auto prefer = [&](cublasLtMatmulPreferenceAttributes_t attr, uint32_t v) {
+        lt_check(cublasLtMatmulPreferenceSetAttribute(pref, attr, &v, sizeof(v)), "preference");
+    };
+    // (the library takes operands for 256-byte aligned unless it is told)
+    prefer(CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, key.align_w);
+    prefer(CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES, key.align_x);
+    prefer(CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES, key.align_out);
+    prefer(CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES, key.align_out);
+    // torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction, as the framework's own products take it
+    using Reduction = at::CuBLASReductionOption;
+    if (key.reduction == (int)Reduction::DisallowReducedPrecisionAllowSplitK)
+        prefer(CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, CUBLASLT_REDUCTION_SCHEME_COMPUTE_TYPE);
+    if (key.reduction == (int)Reduction::DisallowReducedPrecisionDisallowSplitK)
+        prefer(CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, CUBLASLT_REDUCTION_SCHEME_NONE);
     cublasLtMatmulHeuristicResult_t res;
     int found = 0;
     const cublasStatus_t s = cublasLtMatmulAlgoGetHeuristic(handle(key.device), p->op, p->a, p->b, p->d, p->d, pref, 1, &res, &found);
@@ -94,6 +112,11 @@ Plan& plan_for(const Key& key) {
     return *(t_plans.map[key] = std::move(p));
 }
 
+int alignment(const void* p) {   // of an address, 256 bytes at most
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    return a ? (int)std::min<uintptr_t>(a & -a, 256) : 256;
+}
+
 bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0; }
 
 }  // namespace
@@ -103,7 +126,8 @@ Tensor gemm_workspace(const Tensor& on) { return at::empty({(int64_t)kGemmWorksp
 // bf16: out (rows, M; ldo apart) = x (rows, K; ldx apart) w (M, K)^T [+ bias] [+ out]
 void gemm_raw(int device, void* out, int64_t ldo, const void* x, int64_t ldx, const void* w, const void* bias, int64_t rows, int64_t M,
               int64_t K, bool accumulate, void* workspace, void* stream) {
-    const Key key{device, M, rows, K, ldx, ldo, bias != nullptr, accumulate};
+    const Key key{device, M, rows, K, ldx, ldo, bias != nullptr, accumulate, alignment(w), alignment(x), alignment(out),
+                  bias ? alignment(bias) : 256, (int)at::globalContext().allowBF16ReductionCuBLAS()};
     Plan& p = plan_for(key);
     if (bias) lt_check(cublasLtMatmulDescSetAttribute(p.op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)), "bias");
     const float one = 1.f, beta = accumulate ? 1.f : 0.f;
