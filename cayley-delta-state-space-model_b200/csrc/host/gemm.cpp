@@ -146,7 +146,7 @@ void gemm(const Tensor& out, const Tensor& x, const Tensor& w, const Tensor& bia
                        w.is_contiguous() && out.stride(1) == 1 && (x.stride(0) | out.stride(0) | K) % 8 == 0 && aligned16(x) && aligned16(w) &&
                        aligned16(out) && (!bias.defined() || aligned16(bias));
     if (!plain) {   // float32 models, widths that are no multiple of eight
-        if (accumulate) out.add_(at::linear(x, w, bias));
+        if (accumulate) at::addmm_out(const_cast<Tensor&>(out), out, x, w.t());   // one rounding, as in the epilogue (no bias with it)
         else out.copy_(at::linear(x, w, bias));
         return;
     }
