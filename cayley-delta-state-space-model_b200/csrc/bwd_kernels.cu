@@ -224,9 +224,9 @@ chunk_walk_bwd_kernel(const T* __restrict__ g_saved, const T* __restrict__ g_cum
     int pair = blockIdx.y * slots + ps;
     const bool on = head_on && pair < NP;
     if (pair >= NP) pair = NP - 1;
-    // (row numbers fit 32 bits: the state tensors alone would not fit the memory otherwise; addresses are formed from them at each
-    // access, which takes an instruction or two and no registers in between)
-    const int row_last = (int)((m * C + C - 1) * H + h);
+    // (64 bits: small rows in great number fit the memory; addresses are formed from it at each access, which takes an instruction
+    // or two and no registers in between)
+    const long long row_last = (m * C + C - 1) * H + h;
 
     float2 Gr[kP], Gi[kP];
     cf Gc = {0.f, 0.f};
@@ -235,7 +235,7 @@ chunk_walk_bwd_kernel(const T* __restrict__ g_saved, const T* __restrict__ g_cum
     RowSlice<T, kCols> nk, nzr, nzi, nur, nui;           // the next step's inputs; u: upstream gradient of the saved state
     float2 na, nv = make_float2(0.f, 0.f), nuc = nv, ncp = nv;
     float nbe;
-    auto fetch = [&](int row, bool first) {
+    auto fetch = [&](long long row, bool first) {
         const long long srow = (long long)row * N + 2 * pair, prow = kIntra ? srow - (long long)H * N : srow;
         nk.load(K + (long long)row * D, g, D, vec);
         nbe = IO<T>::ld(beta + row);
@@ -257,7 +257,8 @@ chunk_walk_bwd_kernel(const T* __restrict__ g_saved, const T* __restrict__ g_cum
         }
     };
     fetch(row_last, C == 1);
-    for (int t = C - 1, row = row_last; t >= 0; t--, row -= H) {
+    long long row = row_last;
+    for (int t = C - 1; t >= 0; t--, row -= H) {
         float2 k[kP], zr[kP], zi[kP], gK[kP];
         nk.get(reinterpret_cast<float*>(k));
         nzr.get(reinterpret_cast<float*>(zr));
