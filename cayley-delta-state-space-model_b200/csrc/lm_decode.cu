@@ -10,7 +10,8 @@
 //       5 out-projection  residual sum in place
 //     and the head: final RMSNorm, logits.
 // A kernel is launched while its predecessor drains (programmatic dependent launch) and requests its weight rows, as mma
-// fragments into registers, and the constants of its epilogue BEFORE it waits for the predecessor's results; at most 128
+// fragments into registers, and the constants of its epilogue BEFORE it waits for the predecessor's results (the step's
+// first kernel after: its predecessor is not ours); at most 128
 // registers a thread, so that the blocks of two consecutive kernels are resident together.  The activations of all
 // sequences go through shared memory as the other operand of mma.sync m16n8k16: the weight rows are the 16-row operand,
 // sequences the 8-column one (a tcgen05 tile starts at 128 rows, of which a step of a few sequences could use a
@@ -42,6 +43,7 @@ struct Args {
     float eps_norm, eps_group, eps_final;
     DynConsts dc;
     int B, d, di, H, N, vocab, pos;
+    int first;                  // the step's first kernel: the one before it is the caller's and may write the weights
     const int* pos_dev;
     long long proj_stride, qg_stride;
     const void* ahead[2];       // weights of the kernels behind the next one, requested into the L2 cache
@@ -106,6 +108,7 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
     const int tiles = (p.M + kRows - 1) / kRows, btiles = (a.B + NT * 8 - 1) / (NT * 8), items = tiles * btiles;
     float* red = reinterpret_cast<float*>(smem + (kMode == kHead ? (size_t)NT * 8 * pitch : 0));
     uint4 wr[kAhead][2];
+    if (kMode == kInProj && a.first) grid_dependency_wait();
     if ((int)blockIdx.x < items) fetch_first<MT>(p, (int)blockIdx.x % tiles, wr);
     request_ahead(a);
     bool waited = false;
@@ -455,6 +458,7 @@ extern "C" int cdssm_b200_lm_decode(const cdssm_lm_layer* layers, int n_layers, 
         };
         auto bytes = [](const Product& x) { return (size_t)x.M * x.K * 2; };
         const bool last = l + 1 == n_layers;
+        a.first = l == 0;
         ahead(qg.w, bytes(qg), nullptr, 0);
         if (int rc = launch_batch<2, kInProj>(a, w, in, a.proj, a.proj_stride, 0, st)) return rc;
         ahead(op.w, bytes(op), ro.w, bytes(ro));

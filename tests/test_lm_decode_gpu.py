@@ -1,4 +1,6 @@
 """The small-batch decode kernels against the library-product path of the same model (taken above 128 sequences at these widths)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -43,3 +45,53 @@ def test_small_batch_decode_equals_library_products(ops, d_model, state_dim, bat
                 a, b = c[k].float(), w[k][:n].float()
                 assert (a - b).abs().max() <= 2e-2 * b.abs().max(), k
         assert cache["pos"] == wide["pos"]
+
+
+class _Layer(ctypes.Structure):   # cdssm_lm_layer
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("norm_w", "w_in", "b_in", "conv_w", "conv_b", "w_qg", "b_qg", "log_dt_scale", "rope_freqs",
+                                                "mix", "w_readout", "gn_w", "gn_b", "skip", "w_out")] +
+                [("shortcut_scale", ctypes.c_float), ("state", ctypes.c_void_p), ("conv", ctypes.c_void_p)])
+
+
+def test_step_sees_weights_written_by_the_kernel_before_it(ops):
+    """Through the C ABI nothing stands between the caller's last kernel and the step: a one-token scan step, which lets
+    its successor start at once, writes the first layer's input bias."""
+    from cdssm_b200.model import CdssmConfig, CdssmLM
+    cfg = CdssmConfig(d_model=256, n_layers=2, context_length=256, vocab_size=1000, state_dim=2)
+    lm = CdssmLM(cfg, device="cuda", dtype=torch.bfloat16, seed=3)
+    lib, H, N, B = ops._lib.lib(), cfg.n_heads, 2, 4
+    bias = lm.blocks[0].b_in                                          # 1552 values: y of 97 x (8, 2)
+    rows = bias.numel() // (H * N)
+    rnd = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    q, k, v, g = rnd(rows, H, 64), rnd(rows, H, 64), rnd(rows, H, N), rnd(rows, (N + 5) * H)
+    lds, rope = torch.zeros(H, device="cuda"), torch.full((H,), 0.1, device="cuda")
+    mix = torch.full((2, H), 0.5, device="cuda", dtype=torch.bfloat16)
+    need = lib.cdssm_b200_lm_decode_workspace_bytes(B, 256, N, cfg.ssm_norm_groups, 1000, 0)
+    x0 = rnd(B, 256)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def step(apart):
+        bias.zero_()
+        states = [torch.zeros(B, H, N, 64, device="cuda") for _ in range(2)]
+        convs = [torch.zeros(B, 3, 512, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+        ws, x, logits = torch.empty(need + 256, dtype=torch.uint8, device="cuda"), x0.clone(), rnd(B, 1000)
+        layers = (_Layer * 2)(*[_Layer(*[t.data_ptr() for t in (p.norm_w, p.w_in, p.b_in, p.conv_w, p.conv_b, p.w_qg, p.b_qg,
+                                                                  p.log_dt_scale, p.rope_freqs, mix, p.w_readout, p.gn_w, p.gn_b,
+                                                                  p.D, p.w_out)], 0.2, s.data_ptr(), c.data_ptr())
+                                for p, s, c in zip(lm.blocks, states, convs)])
+        state = torch.ones(rows, H, N, 64, device="cuda")
+        torch.cuda.synchronize()
+        ops.decode_step(state, q, k, v, g, lds, rope, *cfg.dyn_consts, H, N, 5, out=bias[:rows * H * N].view(rows, H, N))
+        if apart:
+            torch.cuda.synchronize()
+        rc = lib.cdssm_b200_lm_decode(ctypes.addressof(layers), 2, x.data_ptr(), lm.final_norm_w.data_ptr(), lm.embedding.data_ptr(),
+                                      logits.data_ptr(), ws.data_ptr() + (-ws.data_ptr()) % 256, need, cfg.eps_norm, 1e-5, 2.0 ** -14,
+                                      *cfg.dyn_consts, B, 256, N, cfg.ssm_norm_groups, 1000, 3, None, 0, stream)
+        assert rc == 0
+        torch.cuda.synchronize()
+        return [logits, x] + states + convs
+
+    want = step(True)
+    assert float(bias.float().abs().max()) > 0.05
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(step(False), want))
