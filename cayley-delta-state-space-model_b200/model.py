@@ -177,7 +177,11 @@ class CdssmLM:
         self.blocks = [CdssmBlockParams(cfg, i, gen, device, dtype) for i in range(cfg.n_layers)]
         self.final_norm_w = torch.ones(cfg.d_model, device=device, dtype=dtype)
         self.per_token_group_norm = False   # False = the reference's sequence-wide GroupNorm statistics
-        self._plan = None
+
+    _plan = None   # of the native path: not part of a copy or a saved model
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_plan"}
 
     def _native(self):
         """The model as the native path holds it (csrc/host/lm.cpp: the blocks' layers, one call per pass).  Rebuilt when a

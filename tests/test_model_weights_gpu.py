@@ -168,3 +168,19 @@ def test_weights_at_any_address(ops, skip, reduced):
     for a, w in zip(got, want):
         a, w = a.float(), w.float()
         assert (a - w).norm() <= 2e-2 * w.norm()
+
+
+def test_used_model_can_be_copied_and_saved(ops, tmp_path):
+    """After a pass too, and a model saved before the native path existed has neither plan nor version."""
+    lm = _model()
+    ids = torch.randint(0, 503, (2, 40), device="cuda")
+    want = lm.forward(ids)
+    torch.save(lm, tmp_path / "lm.pt")
+    for other in (copy.deepcopy(lm), torch.load(tmp_path / "lm.pt", weights_only=False)):
+        assert torch.equal(other.forward(ids), want)
+        for p in other.blocks:
+            p.__dict__.pop("version", None)
+        other.__dict__.pop("_plan")
+        assert torch.equal(other.forward(ids), want)
+        other.blocks[0].w_in.zero_()
+        assert not torch.equal(other.forward(ids), want) and torch.equal(lm.forward(ids), want)
