@@ -46,6 +46,7 @@ SIGNATURES = {
     "cdssm_b200_groupnorm_gate_fwd": (_I, [_P] * 5 + [_c_int64] + [_P] * 3 + [_I] * 4 + [_F, _I, _P]),
     "cdssm_b200_conv1d_silu_step": (_I, [_P, _c_int64, _P, _P, _P, _P, _I, _I, _I, _P]),
     "cdssm_b200_scan_fused_workspace_bytes": (_c_size_t, [_I] * 6),
+    "cdssm_b200_scan_fused_workspace_bytes_for": (_c_size_t, [_I] * 8),
     "cdssm_b200_scan_fused_fwd": (_I, [_P] * 11 + [_c_size_t] + [_F] * 6 + [_I] * 9 + [_P]),
     "cdssm_b200_scan_fused_strided_fwd": (_I, [_P, _c_int64] * 3 + [_P, _c_int64, _P] + [_P, _c_int64] + [_P] * 7 + [_c_size_t] + [_F] * 6 + [_I] * 9 + [_P]),
     "cdssm_b200_scan_summary_fwd": (_I, [_P] * 9 + [_c_size_t] + [_F] * 5 + [_I] * 10 + [_P]),

@@ -250,7 +250,8 @@ void run_sequence(const Plan& p, const Layout& lay, const Mix& mixes, const Tens
     const int64_t T = (int64_t)B * L;
     const int HN = H * N, G = (N + 5) * H, dev = (int)x.device().index();
     void* st = stream_of(x);
-    const Workspace ws = workspace(x, cdssm_b200_scan_fused_workspace_bytes(B, L, H, kHeadDim, N, (int)p.chunk));
+    const int scan_flags = (int)(caches ? (L > kTensorPrompt ? kScanForceSimt : 0) : flags);
+    const Workspace ws = workspace(x, cdssm_b200_scan_fused_workspace_bytes_for(B, L, H, kHeadDim, N, (int)p.chunk, CDSSM_BF16, scan_flags));
     auto product = [&](void* out, int64_t ldo, const void* in, int64_t K, const Tensor& w, const void* bias, bool accumulate) {
         gemm_raw(dev, out, ldo, in, K, cptr(w), bias, T, w.size(0), K, accumulate, s.gemm_ws, st);
     };
@@ -285,7 +286,7 @@ void run_sequence(const Plan& p, const Layout& lay, const Mix& mixes, const Tens
                                                 cache ? fmut(cache->state) : nullptr, ws.ptr, ws.bytes, p.dyn.c[0], p.dyn.c[1],
                                                 p.dyn.c[2], p.dyn.c[3], p.dyn.c[4], (float)b.shortcut, B, L, H, kHeadDim, N,
                                                 (int)p.chunk, 0, CDSSM_BF16,
-                                                (int)(caches ? (L > kTensorPrompt ? kScanForceSimt : 0) : flags), st),
+                                                scan_flags, st),
               "scan_fused_fwd");
         product(s.y2, di, s.y, HN, b.w_readout, nullptr, false);
         const bool token_stats = per_token || caches;   // see block_sequence()

@@ -90,7 +90,9 @@ ScanOut scan_fused(const Tensor& q_, const Tensor& k_, const Tensor& v_, const T
         if (want_tail) o.tail.copy_(o.final_state);
         return o;
     }
-    const Workspace ws = workspace(q, cdssm_b200_scan_fused_workspace_bytes((int)B, (int)L, (int)H, (int)D, (int)N, (int)C));
+    // (a call that reuses a summary's results asks for what the summary asked for: the buffer must not move)
+    const int for_flags = flags & CDSSM_SCAN_REUSE_LOCAL ? 0 : (int)flags;
+    const Workspace ws = workspace(q, cdssm_b200_scan_fused_workspace_bytes_for((int)B, (int)L, (int)H, (int)D, (int)N, (int)C, dt, for_flags));
     void* st = stream_of(q);
     if (segs == 1) {
         check(cdssm_b200_scan_fused_fwd(cptr(q), cptr(k), cptr(v), cptr(g), fptr(lds), fptr(rope), fptr(h0), mptr(o.y),
@@ -153,7 +155,7 @@ std::array<Tensor, 2> scan_fused_long(const Tensor& q_, const Tensor& k_, const 
     const Tensor scratch = empty_f32({3 * st_n + dc_n + B * H * N}, q);
     float* carry = fmut(scratch);
     float *carry_in = carry + st_n, *last = carry_in + st_n, *decay = last + st_n, *total = decay + dc_n;
-    const Workspace ws = workspace(q, cdssm_b200_scan_fused_workspace_bytes((int)R, (int)Ls, (int)H, (int)D, (int)N, (int)C));
+    const Workspace ws = workspace(q, cdssm_b200_scan_fused_workspace_bytes_for((int)R, (int)Ls, (int)H, (int)D, (int)N, (int)C, dt, (int)flags));
     void* st = stream_of(q);
     check(cdssm_b200_scan_summary_fwd(cptr(k), cptr(v), cptr(g), fptr(lds), fptr(rope), nullptr, carry, decay, ws.ptr, ws.bytes,
                                       dyn.c[0], dyn.c[1], dyn.c[2], dyn.c[3], dyn.c[4], (int)R, (int)Ls, (int)H, (int)D, (int)N,

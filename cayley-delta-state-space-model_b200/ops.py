@@ -372,7 +372,9 @@ def scan_summary(k: Tensor, v: Tensor, gate_raw: Tensor, log_dt_scale: Tensor, r
     if B * L == 0:
         return (carry if h0 is None else h0.clone()), decay
     with torch.cuda.device(k.device):
-        ws_ptr, ws_bytes = _workspace(k, scan_fused_workspace_bytes(B, L, H, D, N, C))
+        # (as scan_fused asks for it: a call that reuses the local results must find the buffer as it is)
+        need = _lib.lib().cdssm_b200_scan_fused_workspace_bytes_for(B, L, H, D, N, C, _dtype_code(k), 0)
+        ws_ptr, ws_bytes = _workspace(k, int(need))
         check(_lib.lib().cdssm_b200_scan_summary_fwd(
             _p(k), _p(v), _p(g), _p(lds), _p(rf), _p(h0), _p(carry), _p(decay), ws_ptr, ws_bytes, gating_c,
             omega_thresh, adt_delta, adt_smoothness, adt_eps, B, L, H, D, N, C, int(pos0), int(segs),

@@ -212,6 +212,10 @@ CDSSM_API int cdssm_b200_conv1d_silu_step(const void* x, int64_t x_row_stride, v
 
 /* Bytes of workspace cdssm_b200_scan_fused_fwd needs for these sizes (0 on bad sizes). */
 CDSSM_API size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int D, int N, int C);
+/* The same with room for what the CUDA-core kernels can put to use (they run without it, a tenth slower) where a call of that
+ * dtype and flags takes them.  A segmented call with CDSSM_SCAN_REUSE_LOCAL reads what the summary before it has left: give
+ * both the same buffer. */
+CDSSM_API size_t cdssm_b200_scan_fused_workspace_bytes_for(int B, int L, int H, int D, int N, int C, int dtype, int flags);
 
 /* The whole scan path in one call, nothing of size (B,L,H,N,D) ever stored:
  * dynamics -> L2-normalised q/k -> vp-scaled v -> chunked delta-rule scan in the reference's

@@ -46,6 +46,14 @@ def test_argument_validation_needs_no_gpu(lib):
     n = h.cdssm_b200_scan_fused_workspace_bytes(2, 512, 4, 64, 2, 64)
     assert n >= 2 * 8 * 4 * (2 + 128) * 4
     assert h.cdssm_b200_scan_fused_workspace_bytes(2, 512, 4, 64, 3, 64) == 0      # odd state_dim
+    # what a call needs: decays and states of the chunks, and the records of the tensor-core kernels where those run
+    states = lambda B, L, H, D, N, C: 256 + sum(-(-x // 256) * 256 for x in (B * -(-L // C) * H * N * 4, B * -(-L // C) * H * N * D * 4))
+    ws, more = h.cdssm_b200_scan_fused_workspace_bytes, h.cdssm_b200_scan_fused_workspace_bytes_for
+    assert ws(16, 65536, 32, 128, 2, 128) == states(16, 65536, 32, 128, 2, 128) + 16 * 65536 * 32 * 16
+    assert ws(2, 512, 4, 64, 32, 64) == states(2, 512, 4, 64, 32, 64)
+    assert more(16, 65536, 32, 128, 2, 128, 0, 0) == ws(16, 65536, 32, 128, 2, 128)
+    assert more(2, 512, 4, 64, 2, 64, 1, 0) == states(2, 512, 4, 64, 2, 64) + 2 * 512 * 4 * 24
+    assert more(2, 512, 4, 64, 2, 64, 0, 1) == more(2, 512, 4, 64, 2, 64, 1, 0)
     # null pointers and bad sizes are refused before anything touches CUDA
     null = ctypes.c_void_p(0)
     assert h.cdssm_b200_normalize_kq_fwd(null, null, null, null, 4, 64, 0, null) == -1
