@@ -464,6 +464,11 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int s = 0; s < G::kSlabs; s++) tma_load_4d(sm.k + s * G::kSlab, &tmK, &sm.full_k, 64 * s, hd, c * kD, b);
     }
 
+    // a block that gives up stays until its own copy has landed (or a limit has passed again): the next one has its memory then
+    auto drain = [&](uint64_t* bar) {
+        volatile int never = 0;
+        if (tid == 0 && !a.withhold) mbar_wait_ns(bar, 0, &never, a.wait_ns);
+    };
     // ---- carry into the chunk: this warp's 32 columns of its state rows.  Early if its producer is done, else polled for
     // behind the products that do not need it (kOutput: the previous pass is waited for there).
     const float* carry_src = a.ws_state + (unit * (size_t)N + 2 * pair0) * kD;
@@ -516,6 +521,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     if (!__syncthreads_and(k_here)) {
         if (tid == 0) atomicCAS(a.status, 0, 201);
         cp_async_wait_all();
+        drain(&sm.full_k);
         return;
     }
     const uint32_t kt = smem_u32(sm.k), qt = smem_u32(sm.q);
@@ -1018,6 +1024,7 @@ scan_chunk_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     const bool q_here = mbar_wait_suspend(&sm.full_q, 0, &sm.abort_flag, a.wait_ns);
     if (!__syncthreads_and(q_here && have_carry)) {
         if (tid == 0) atomicCAS(a.status, 0, 202);
+        drain(&sm.full_q);
         return;
     }
 

@@ -35,3 +35,19 @@ def test_scan_waits_run_out_and_the_next_call_is_correct(ops, orc, D):
     assert ops.scan_fused_status() == 0
     wy, _ = oracle_scan(orc, inp, N, D, orc.ROUND_REFERENCE)
     assert rel_err(to_np(y), wy) <= BF16_TOL
+
+
+@pytest.mark.parametrize("D,L", [(64, 69), (64, 3000), (128, 133)])
+def test_whole_chunk_scan_waits_run_out_too(ops, orc, D, L):
+    """Both forms of the whole-chunk scan (a few chunks; a chain of them)."""
+    B, H, N = 1, 3, 4
+    inp = orc.make_inputs(B, H, L, D, N=N, seed=42, bf16=True)
+    old = ops.set_wait_limit_ns(2_000_000)
+    try:
+        run_fused(ops, inp, torch.bfloat16, N, D, flags=ops.TEST_WITHHOLD)
+        assert 200 <= ops.scan_fused_status() < 300
+    finally:
+        ops.set_wait_limit_ns(old)
+    y, _ = run_fused(ops, inp, torch.bfloat16, N, D, strict=True)
+    wy, _ = oracle_scan(orc, inp, N, D, orc.ROUND_REFERENCE)
+    assert rel_err(to_np(y), wy) <= BF16_TOL
