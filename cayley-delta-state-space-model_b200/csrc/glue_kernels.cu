@@ -229,7 +229,8 @@ groupnorm_gate_rows_kernel(const T* y, const float* stats, const T* gn_w,
         f[r].ld(y + (long long)row * di + c);
         zz[r].ld(z + row * z_row_stride + c);
         xc[r].ld(x_conv + (long long)row * di + c);
-        st[r] = *reinterpret_cast<const float2*>(stats + 2 * ((long long)(row / L) * groups + grp));
+        const float* sp = stats + 2 * ((long long)(row / L) * groups + grp);   // (the caller's floats: 4-byte aligned)
+        st[r] = make_float2(sp[0], sp[1]);
     }
     float gw[8], gb[8], sk[8];
     Vec8<T>::ld(gn_w + c, gw);

@@ -66,3 +66,19 @@ def test_conv_step_equals_full_conv(ops, dtype, Dm):
         out = ops.conv1d_silu_step(wide[:, t, :Dm], hist, w, b)
         assert (out.float() - full[:, t].float()).abs().max() <= _tol(dtype) * full.float().abs().max()
     assert torch.equal(hist, x[:, L - 3:])
+
+
+def test_gate_takes_statistics_at_any_float_address(ops):
+    """The statistics are floats of the caller's, not pairs: 4-byte aligned, on the kernel for many rows too."""
+    B, L, di, groups = 2, 2200, 256, 8
+    g = torch.Generator().manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g).cuda().bfloat16()
+    y, z, xc, gw, gb, sk = r(B, L, di), r(B, L, di), r(B, L, di), r(di), r(di), r(di)
+    want = ops.groupnorm_gate(y, gw, gb, z, sk, xc, groups)
+    lib, st = ops._lib.lib(), torch.cuda.current_stream().cuda_stream
+    room = torch.empty(lib.cdssm_b200_groupnorm_stats_floats(B, L, groups) + 1, device="cuda")
+    out = torch.empty_like(y)
+    assert lib.cdssm_b200_groupnorm_stats(y.data_ptr(), room.data_ptr() + 4, B, L, di, groups, 1e-5, 0, st) == 0
+    assert lib.cdssm_b200_groupnorm_gate_fwd(y.data_ptr(), room.data_ptr() + 4, gw.data_ptr(), gb.data_ptr(), z.data_ptr(), di,
+                                             sk.data_ptr(), xc.data_ptr(), out.data_ptr(), B, L, di, groups, 1e-5, 0, st) == 0
+    assert torch.equal(out, want)
