@@ -27,6 +27,7 @@ _P, _I, _F = _c_void_p, _c_int, _c_float
 SIGNATURES = {
     "cdssm_b200_version": (_I, []),
     "cdssm_b200_last_cuda_error": (_I, []),
+    "cdssm_b200_launch_count": (_c_int64, []),
     "cdssm_b200_dynamics_fwd": (_I, [_P] * 7 + [_F] * 5 + [_I] * 6 + [_P]),
     "cdssm_b200_intra_chunk_scan_bwd": (_I, [_P] * 12 + [_I] * 6 + [_P]),
     "cdssm_b200_exact_correction_bwd": (_I, [_P] * 9 + [_I] * 8 + [_P]),

@@ -8,6 +8,10 @@ int& last_cuda_error_ref() {
     static thread_local int e = 0;
     return e;
 }
+std::atomic<long long>& launch_count_ref() {
+    static std::atomic<long long> n{0};
+    return n;
+}
 }  // namespace cdssm
 
 namespace cdssm {
@@ -43,4 +47,5 @@ extern "C" int cdssm_b200_selftest_bounded_wait(int* status_dev, uint64_t limit_
 }
 
 extern "C" int cdssm_b200_version(void) { return 201; }
+extern "C" int64_t cdssm_b200_launch_count(void) { return cdssm::launch_count_ref().load(); }
 extern "C" int cdssm_b200_last_cuda_error(void) { return cdssm::last_cuda_error_ref(); }

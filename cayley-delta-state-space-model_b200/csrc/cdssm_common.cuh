@@ -14,7 +14,13 @@ inline int check_cuda(cudaError_t e) {
     last_cuda_error_ref() = (int)e;
     return CDSSM_ERR_CUDA;
 }
-inline int check_launch() { return check_cuda(cudaGetLastError()); }
+// Kernels this library has launched in this process (cdssm_b200_launch_count).
+std::atomic<long long>& launch_count_ref();
+inline int counted(int rc) {
+    if (rc == CDSSM_OK) launch_count_ref().fetch_add(1, std::memory_order_relaxed);
+    return rc;
+}
+inline int check_launch() { return counted(check_cuda(cudaGetLastError())); }
 
 // Programmatic dependent launch: the kernel may start while its predecessor in the stream drains; it must not touch
 // anything a predecessor writes (nor write anything a predecessor reads) before grid_dependency_wait().
@@ -33,7 +39,7 @@ inline int launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return counted(check_cuda(cudaLaunchKernelEx(&cfg, kernel, P(args)...)));
 }
 
 // Opts a kernel in to `bytes` of dynamic shared memory, once per kernel (Tag) and device.

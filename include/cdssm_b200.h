@@ -41,6 +41,8 @@ extern "C" {
  * on this host thread (0 if none). */
 CDSSM_API int cdssm_b200_version(void);
 CDSSM_API int cdssm_b200_last_cuda_error(void);
+/* Kernels that this library has launched, or put into a graph under capture, in this process. */
+CDSSM_API int64_t cdssm_b200_launch_count(void);
 
 /* Fused dynamics: gate_raw (B,L,(N+5)*H) -> A_bar (B,L,H,N), vp_scale (B,L,H,N/2),
  * beta (B,L,H), sel_C (B,L,H).  log_dt_scale, rope_freqs: (H) float32.  pos0 is added to the
@@ -193,9 +195,10 @@ CDSSM_API int cdssm_b200_conv1d_silu_step(const void* x, int64_t x_row_stride, v
                                       chunk and what decode continues); h0/final_state/tail_state are then
                                       the recurrent state.  One sequential walk per (batch, head, pair). */
 #define CDSSM_SCAN_TENSOR_CORE_WA 128 /* insist on the warp-autonomous tcgen05/TMA passes (Gram blocks on tcgen05,
-                                      state products as warp-level mma; the default whenever bf16, N = 2,
-                                      D = C in {64, 128}, H a multiple of 4 and no tail_state):
-                                      CDSSM_ERR_UNSUPPORTED instead of the CUDA-core kernels otherwise */
+                                      state products as warp-level mma; the default for bf16, N = 2 and
+                                      D = C in {64, 128}), their state products in two bf16 parts also where
+                                      tail_state is asked for (by default three then, which is exact):
+                                      CDSSM_ERR_UNSUPPORTED for other shapes and for H no multiple of 4 */
 
 #define CDSSM_SCAN_KEEP_SIMT_LOCAL 256  /* tests: with the tensor-core passes, keep the CUDA-core LOCAL pass ... */
 #define CDSSM_SCAN_KEEP_SIMT_OUTPUT 512 /* ... or the CUDA-core OUTPUT pass, so that each tensor-core pass is also
@@ -221,9 +224,12 @@ CDSSM_API size_t cdssm_b200_scan_fused_workspace_bytes_for(int B, int L, int H, 
  * dynamics -> L2-normalised q/k -> vp-scaled v -> chunked delta-rule scan in the reference's
  * chunk semantics (local scan from zero per chunk of C tokens, decay-only carry between chunks,
  * correction taken before each step) -> shortcut -> read-out with q -> sel_C gate.
- * Supported: even N <= 32, D <= 128, C <= 256, bf16 or fp32 (CUDA-core kernels, three launches);
- * bf16 with N = 2, D = C in {64, 128}, H a multiple of 4 and no tail_state runs on the tensor cores (tcgen05/TMA
- * local and output pass, four launches).
+ * Supported: even N <= 32, D <= 128, C <= 256, bf16 or fp32: CUDA-core kernels, four launches (records, local pass, carry
+ * pass, output pass), three without room for their records.  bf16 with D = C in {64, 128} and N <= 16 runs on the tensor
+ * cores: N = 2 in local and output pass (tcgen05/TMA), other N in those or in one kernel that hands the carry on inside it;
+ * with the records two to four launches.  The arithmetic of a call goes by H, D, N, C, dtype, flags and whether tail_state is
+ * asked for, not by B or L: rows of a batch alone, and pieces of a sequence chained through final_state and pos0, have the
+ * bits of the whole.
  *   q,k (B,L,H,D) un-normalised; v (B,L,H,N) before the vp scale; gate_raw (B,L,(N+5)*H);
  *   h0 (B,H,N,D) float32 or NULL: carry into the first chunk;
  *   y (B,L,H,N); final_state (B,H,N,D) float32 or NULL: carry after the last chunk;
