@@ -548,12 +548,15 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     // behind the sequence end a = 1, beta = v = 0: the state stands still
     const uint4 still4 = make_uint4(0x3f800000u, 0u, 0u, 0u);
     ItemPos cur = item_pos(a, blockIdx.x), nxi = cur;
+    // (past the last head the warp reads that head's values beside tiles of zeros and stores nothing; with two parts H is a
+    // multiple of four)
+    const int last = H - 1;
     Tok tk;
     grid_dependency_wait();       // records (local pass) / carries (output pass) of the kernel before
     grid_launch_dependents();
     {
         const bool valid = cur.c * kD + tl < L;
-        const uint4 first = valid ? __ldcg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, min(cur.h0 + J, H - 1), tl)) : still4;
+        const uint4 first = valid ? __ldcg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, (kParts == 2 ? cur.h0 + J : min(cur.h0 + J, last)), tl)) : still4;
         tk = prepare(first, tl);
     }
     for (int g = 0; g < NS; g++) {
@@ -564,9 +567,8 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             if (g > 0) cur = nxi;
             nxi = item_pos(a, (int)blockIdx.x + (g / kSteps + 1) * (int)gridDim.x);
         }
-        // (a group past the last head: the warp reads that head's values beside tiles of zeros and stores nothing)
-        const int l = cur.c * kD + step * kSub + tl, hd = min(cur.h0 + J, H - 1);
-        const bool stores = cur.h0 + J < H, valid = l < L && stores;
+        const int l = cur.c * kD + step * kSub + tl, hd = (kParts == 2 ? cur.h0 + J : min(cur.h0 + J, last));
+        const bool stores = kParts == 2 || cur.h0 + J < H, valid = l < L && stores;
         const size_t unit = ((size_t)cur.b * a.NC + cur.c) * H + hd;   // workspace slot of this head's chunk
         if (step == 0) {   // states at the chunk start: z = 0, r = the chunk's carry
             const float* s = a.ws_state + unit * 2 * kD + (size_t)(np & 1) * kD;
@@ -592,7 +594,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             const ItemPos& np_ = (step + 1 < kSteps) ? cur : nxi;
             const int nsub = (step + 1) % kSteps;
             if (np_.c * kD + nsub * kSub + tl < L)
-                rec = __ldcg(a.rec + rec_index(a, kSteps, np_.b, np_.c, nsub, min(np_.h0 + J, H - 1), tl));
+                rec = __ldcg(a.rec + rec_index(a, kSteps, np_.b, np_.c, nsub, (kParts == 2 ? np_.h0 + J : min(np_.h0 + J, last)), tl));
         }
         const cplx at = tk.at, vg = tk.vg;
         const float be = tk.be;

@@ -76,6 +76,25 @@ def test_shards_and_pieces_have_the_bits_of_the_whole(ops, orc, H, D, N, tail):
         assert torch.equal(w, p)
 
 
+@pytest.mark.parametrize("H,D,N", [(8, 64, 2), (8, 64, 4), (3, 64, 16), (4, 128, 4), (2, 128, 16)])
+def test_forms_of_a_kernel_have_the_same_bits(ops, orc, H, D, N):
+    """With a carry pass, without one and with the carry handed on inside one kernel: 60 chunks in a row, the same in pieces
+    of 1, 9 and 50, and beside a batch that fills the GPU."""
+    B, L = 1, 60 * D
+    inp = _inputs(orc, B, H, L, D, N, seed=N + D)
+    run = lambda i, **kw: run_fused(ops, i, torch.bfloat16, N, D, **kw)
+    y, fin = run(inp)
+    ys, h, at = [], None, 0
+    for n in (1, 9, 50):
+        piece, f = run(_cut(inp, tokens=slice(at * D, (at + n) * D)), h0=h, pos0=at * D)
+        ys.append(piece)
+        h, at = to_np(f), at + n
+    assert torch.equal(torch.cat(ys, 1), y) and torch.equal(f, fin)
+    wide = {k: (np.repeat(v, 16, 0) if getattr(v, "ndim", 0) >= 3 else v) for k, v in inp.items()}
+    yw, fw = run(wide)
+    assert torch.equal(yw[:1], y) and torch.equal(yw[15:], y) and torch.equal(fw[7:8], fin)
+
+
 @pytest.mark.parametrize("D,N", [(64, 2), (128, 2), (64, 4), (64, 8), (64, 16), (128, 4), (128, 16)])
 @pytest.mark.parametrize("value", [float("nan"), float("inf"), 3e19])
 @pytest.mark.parametrize("what", ["k", "v", "beta", "decay"])
