@@ -23,8 +23,8 @@ struct Args {
     uint32_t *rec_v, *rec_g;       // vp-scaled v (B,NC,H,NP,C); beta and sel_C (B,NC,H,C), bf16 pairs
     const __nv_bfloat16 *v_first, *mix;   // or nullptr: v <- lerp(v_first, v, mix[head])
     long long v_rs, vf_rs, g_rs;   // elements between token rows
-    int* clear;                    // words cleared here for the passes that follow
-    size_t clear_words;
+    int *clear, *clear2;           // words cleared here for the passes that follow (16-byte aligned; the second: a multiple of four)
+    size_t clear_words, clear2_words;
     DynConsts dc;
     int B, L, H, N, C, NC, pos0, segs, fp32_decay, tiles;   // tiles: 32-token tiles per batch row, chunks padded to full length
 };
@@ -42,9 +42,12 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
     grid_dependency_wait();
-    for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x; i < a.clear_words && blockIdx.z == 0;
-         i += (size_t)gridDim.x * gridDim.y * kThreads)
-        a.clear[i] = 0;
+    if (blockIdx.z == 0) {
+        const size_t first = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x, step = (size_t)gridDim.x * gridDim.y * kThreads;
+        for (size_t i = first; i < a.clear_words / 4; i += step) reinterpret_cast<uint4*>(a.clear)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (first < a.clear_words % 4) a.clear[a.clear_words / 4 * 4 + first] = 0;
+        for (size_t i = first; i < a.clear2_words / 4; i += step) reinterpret_cast<uint4*>(a.clear2)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
     const int H = a.H, N = a.N, NP = N >> 1, p0 = kWa ? 0 : kNP * (int)blockIdx.z, pairs = min(kNP, NP - p0);
     const int b = (int)(blockIdx.x / (unsigned)a.tiles), tile = (int)(blockIdx.x - (unsigned)b * a.tiles), l0 = tile * kTokens;
     const int head0 = blockIdx.y * kHg, heads = min(kHg, H - head0);
@@ -152,7 +155,7 @@ size_t scan_record_bytes(int B, int L, int H, int N, int C) {
     return (size_t)B * (((size_t)L + C - 1) / C) * H * C * ((size_t)(N / 2) * 12 + 4);
 }
 
-// The three arrays of the layout of scan_chunk.cu inside the record buffer.
+// The three arrays of the layout of scan_tile.cu inside the record buffer.
 void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a, uint32_t** v, uint32_t** g) {
     const size_t n = (size_t)B * (((size_t)L + C - 1) / C) * H * C;
     *a = static_cast<float2*>(rec);
@@ -160,10 +163,10 @@ void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a
     *g = *v + n * (N / 2);
 }
 
-// Fills the records every pass over the same inputs reads.  wa: the layout of scan_wa.cu (N = 2), else of scan_chunk.cu.
+// Fills the records every pass over the same inputs reads.  wa: the layout of scan_wa.cu (N = 2), else of scan_tile.cu.
 int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, long long vf_rs, const void* mix,
                  const void* gate_raw, long long g_rs, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                 int* clear, size_t clear_words, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
+                 int* clear, size_t clear_words, int* clear2, size_t clear2_words, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
                  int fp32_decay, cudaStream_t st) {
     using namespace records;
     Args a;
@@ -175,6 +178,7 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
     a.v_first = static_cast<const __nv_bfloat16*>(v_first); a.mix = static_cast<const __nv_bfloat16*>(mix);
     a.v_rs = v_rs; a.vf_rs = vf_rs; a.g_rs = g_rs;
     a.clear = clear; a.clear_words = clear_words;
+    a.clear2 = clear2; a.clear2_words = clear2_words;
     a.dc = dc;
     a.B = B; a.L = L; a.H = H; a.N = N; a.C = C; a.NC = (L + C - 1) / C; a.pos0 = pos0; a.segs = segs; a.fp32_decay = fp32_decay;
     a.tiles = a.NC * (C / kTokens);

@@ -12,7 +12,7 @@
 //   carry pass  : per (batch, head, pair, d) serial over chunks -> s_c in place of z_{C-1}
 //   output pass : per (chunk, head, pair) walk z and r together, read out y
 // The local pass re-reads k, v and the gates (about half of the algorithmic bytes).  scan_wa.cu and
-// scan_chunk.cu hold the tensor-core kernels for the shapes they take; the carry pass here serves both.
+// scan_tile.cu hold the tensor-core kernels for the shapes they take; the carry pass here serves both.
 //
 // Thread mapping: eight lanes own one (chunk, head, pair) unit, each lane D/8 contiguous
 // columns of the two state rows, so a k/q row is fetched with 16-byte loads and a dot product
@@ -791,18 +791,19 @@ unsigned long long wait_limit_ns();   // c_abi.cu
 size_t scan_record_bytes(int B, int L, int H, int N, int C);
 int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, long long vf_rs, const void* mix,
                  const void* gate_raw, long long g_rs, const float* log_dt_scale, const float* rope_freqs, void* rec,
-                 int* clear, size_t clear_words, const DynConsts& dc, int B, int L, int H, int N, int C, int pos0, int segs,
-                 int fp32_decay, cudaStream_t st);
+                 int* clear, size_t clear_words, int* clear2, size_t clear2_words, const DynConsts& dc, int B, int L, int H, int N,
+                 int C, int pos0, int segs, int fp32_decay, cudaStream_t st);
 // scan_wa.cu
 bool scan_wa_supported(int D, int N, int C, int dtype);
 int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long long k_rs, const void* rec, float* ws_gamma, float* ws_state, void* y,
                  float* tail_state, int* status, float shortcut_scale, int B, int L, int H, int D, unsigned long long wait_ns, int withhold,
                  int from_chunks, const float* h0, float* final_state, int parts, cudaStream_t st);
-// scan_chunk.cu
-bool scan_chunk_supported(int D, int N, int C, int dtype);
-int scan_chunk_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y, float* final_state,
-                    float* tail_state, float* ws_gamma, float* ws_state, int* status, int* ticket, float shortcut_scale, int B,
-                    int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
+// scan_tile.cu
+bool scan_tile_supported(int D, int N, int C, int dtype);
+size_t scan_tile_extra_bytes(int B, int L, int H, int D, int N);
+int scan_tile_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
+                   float* final_state, float* tail_state, float* ws_gamma, float* ws_state, void* extra, int* status, int* ticket,
+                   float shortcut_scale, int B, int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -818,10 +819,17 @@ static size_t simt_record_bytes(int B, int L, int H, int N, int C) {
     return (size_t)B * (((size_t)L + C - 1) / C) * H * C * ((size_t)(N / 2) * sizeof(float4) + sizeof(float2));
 }
 
+// What a call cannot do without: the tensor-core scans' records beside the base.
+static size_t least_workspace_bytes(int B, int L, int H, int D, int N, int C) {
+    size_t bytes = base_workspace_bytes(B, L, H, D, N, C);
+    if (scan_wa_supported(D, N, C, CDSSM_BF16) || scan_tile_supported(D, N, C, CDSSM_BF16)) bytes += align256(scan_record_bytes(B, L, H, N, C));
+    return bytes;
+}
+
 extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int D, int N, int C) {
     if (B <= 0 || L <= 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return 0;
-    size_t bytes = base_workspace_bytes(B, L, H, D, N, C);
-    if (scan_wa_supported(D, N, C, CDSSM_BF16) || scan_chunk_supported(D, N, C, CDSSM_BF16)) bytes += align256(scan_record_bytes(B, L, H, N, C));
+    size_t bytes = least_workspace_bytes(B, L, H, D, N, C);
+    if (scan_tile_supported(D, N, C, CDSSM_BF16)) bytes += scan_tile_extra_bytes(B, L, H, D, N);
     return bytes;
 }
 // With room for the CUDA-core walks' records where those kernels run: a tenth faster (8 bytes more per token-head and 8 per pair
@@ -829,8 +837,9 @@ extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int
 extern "C" size_t cdssm_b200_scan_fused_workspace_bytes_for(int B, int L, int H, int D, int N, int C, int dtype, int flags) {
     const size_t least = cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
     if (least == 0 || (flags & CDSSM_SCAN_EXACT)) return least;
-    const bool tensor = !(flags & CDSSM_SCAN_FORCE_SIMT) && (scan_wa_supported(D, N, C, dtype) || scan_chunk_supported(D, N, C, dtype));
-    return tensor ? least : base_workspace_bytes(B, L, H, D, N, C) + align256(simt_record_bytes(B, L, H, N, C));
+    const bool tensor = !(flags & CDSSM_SCAN_FORCE_SIMT) && (scan_wa_supported(D, N, C, dtype) || scan_tile_supported(D, N, C, dtype));
+    return tensor ? least : std::max(least_workspace_bytes(B, L, H, D, N, C),
+                                     base_workspace_bytes(B, L, H, D, N, C) + align256(simt_record_bytes(B, L, H, N, C)));
 }
 
 extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_host, void* stream) {
@@ -842,31 +851,22 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
     return *status_host == 0 ? CDSSM_OK : CDSSM_ERR_TIMEOUT;
 }
 
-// Whether the output pass of the whole-chunk scan adds the carry up itself from the local results of the chunks before it (else
-// a carry pass runs in between): a read of NC x N rows by every block, in parallel, against a launch and two more trips to
-// memory.  us on B200, carry pass / without (D 64, one sequence): N 16, H 24, 9 chunks 35 / 24, 16 chunks 38 / 27, 32 chunks
-// 43 / 46; N 4, H 6, 9 chunks 14 / 11, 48 chunks 19 / 20.
-static bool few_chunks(int NC, int N) { return NC <= 40 && NC * N <= 400; }
+// Whether scan_wa.cu's output pass adds the carry up itself from the local results of the chunks before it (else a carry pass runs
+// in between): while it has a chunk of four heads per block, two blocks per SM.  us on B200, carry pass / without: D 64, 936 chunks
+// 24.4 / 21.5, 3072 42 / 44; D 128, 528 32.3 / 30.5, 1536 61 / 63.
+static bool carry_in_output(int B, int NC, int H) { return (long long)B * NC * ((H + 3) / 4) <= 296 && NC <= 40; }
 
-// Whether the whole-chunk scan runs as one kernel that hands the carry from chunk to chunk inside it, or as local pass
-// (+ carry pass) + output pass: the same arithmetic in the same order, so the choice may go by size.  One kernel reads k once
-// and forms G once, but a hand-off takes 2 us and more (flag, carry, rounding, release), so a (batch, head) chain of NC chunks
-// takes that many whatever the size; the passes cost more work.  Each form: the larger of its latency and its work on the full
-// GPU, us on B200, by the number of pairs the kernel holds, fitted to 380 sizes.
-struct FormCost { float one, one_chunk, one_full, one_unit, one_slope, pass, pass_chunk, pass_carry, pass_full, pass_unit; };
-static bool one_kernel_pays(int B, int H, int NC, int D, int N) {
-    static const FormCost kCost[2][3] = {   // one_slope: work per unit grows with the length of the chains that wait
-        {{8.1f, 2.14f, 10.4f, 0.0185f, 0.f, 11.7f, 0.19f, 10.f, 10.8f, 0.0261f},       // head_dim 64: N 4, 8, 16
-         {8.7f, 2.33f, 11.3f, 0.0238f, 1e-4f, 8.5f, 0.36f, 0.f, 11.8f, 0.0352f},
-         {6.4f, 3.77f, 15.8f, 0.0426f, 1e-4f, 19.1f, 0.44f, 0.f, 15.4f, 0.0577f}},
-        {{16.7f, 1.88f, 17.9f, 0.0616f, 5e-4f, 23.9f, 0.27f, 17.f, 17.9f, 0.0964f},    // head_dim 128: N 4, 8, 16 (two blocks a chunk)
-         {23.6f, 2.31f, 24.9f, 0.102f, 8e-4f, 32.1f, 0.1f, 40.f, 26.5f, 0.1375f},
-         {16.1f, 4.48f, 21.2f, 0.218f, 3e-4f, 11.8f, 5.2f, 7.f, 24.9f, 0.273f}}};
-    const FormCost& f = kCost[D == 128][N <= 4 ? 0 : N <= 8 ? 1 : 2];
-    const float units = (float)B * H * NC, c = (float)NC;
-    const float one = fmaxf(f.one + f.one_chunk * c, f.one_full + units * (f.one_unit + f.one_slope * fminf(c, 100.f)));
-    const float passes = fmaxf(f.pass + f.pass_chunk * c + (few_chunks(NC, N) ? 0.f : f.pass_carry), f.pass_full + units * f.pass_unit);
-    return one <= passes;
+// Whether the whole-chunk scan (scan_tile.cu) hands the carry on inside one kernel, or runs as local pass, carry pass and output
+// pass: the same arithmetic in the same order, so this choice may go by size.  One kernel forms G once and reads k once, but its
+// blocks add up the chunks between theirs and the last finished one, as many as there are blocks on a sequence: too many when few
+// tiles beside each other fill the GPU (head_dim 64: 592 blocks for N <= 4, else 296).  us on B200, one kernel / passes: N 4, 12
+// tiles 91 / 82, 24 tiles 163 / 160, 48 tiles 61 / 67; N 8, 6 tiles 63 / 78, 12 tiles 77 / 95, 24 tiles 139 / 176; N 16, 6 tiles
+// 122 / 112, 12 tiles 104 / 120, 24 tiles 163 / 188; N 16, 12 tiles, 9 chunks 30 / 43; head_dim 128, N 4, 4 tiles 49 / 59, N 16,
+// 24 tiles 146 / 178.
+static bool hands_carry_on(int B, int H, int NC, int D, int N) {
+    if (D == 128 || NC <= 28) return true;
+    const long long tiles = (long long)B * ((H + 1) / 2);
+    return N <= 4 ? tiles * 22 >= 592 : N <= 8 || tiles * 28 >= 296;
 }
 
 struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual
@@ -898,7 +898,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (B == 0 || L == 0) return CDSSM_OK;
     // small_workspace: as many of the records as fit (the walks can do without)
     const size_t base = base_workspace_bytes(B, L, H, D, N, C);
-    const size_t need = small_workspace ? base : cdssm_b200_scan_fused_workspace_bytes(B, L, H, D, N, C);
+    const size_t need = small_workspace ? base : least_workspace_bytes(B, L, H, D, N, C);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return CDSSM_ERR_WORKSPACE;
     // first 256 bytes of the workspace: status word of the tensor-core kernel's bounded waits, ticket counter
     int* status = static_cast<int*>(workspace);
@@ -924,7 +924,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     a.ws_state = reinterpret_cast<float*>(static_cast<char*>(workspace) +
                                           align256((size_t)a.units * 2 * sizeof(float)));
     cudaStream_t st = (cudaStream_t)stream;
-    // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 (scan_wa.cu), any other N <= 16 (scan_chunk.cu).  The
+    // Tensor-core kernels for bf16, chunk = head_dim in {64, 128}: N = 2 (scan_wa.cu), any other N <= 16 (scan_tile.cu).  The
     // kernel goes by the head's shape and by what is asked for, never by batch or length: a shard of a batch, and chunk-aligned
     // pieces of a sequence that hand the carry on, give the bits of the whole.  They read v
     // and write y as 4-byte pairs: buffers that are only 2-byte aligned, which the contract allows, stay on the CUDA-core
@@ -932,21 +932,24 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     const bool tensor_ok = (((uintptr_t)v | (uintptr_t)y | (uintptr_t)rows.first | (uintptr_t)(2 * v_rs) |
                               (uintptr_t)(rows.first ? 2 * vf_rs : 0)) & 3) == 0 && ((q_rs | k_rs) & 7) == 0 && workspace_bytes - base >= scan_record_bytes(B, L, H, N, C) &&
                            !(flags & (CDSSM_SCAN_EXACT | CDSSM_SCAN_FORCE_SIMT));
-    const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, dtype), chunk_ok = tensor_ok && scan_chunk_supported(D, N, C, dtype);
+    const bool wa_ok = tensor_ok && scan_wa_supported(D, N, C, dtype), tile_ok = tensor_ok && scan_tile_supported(D, N, C, dtype);
     if ((flags & CDSSM_SCAN_TENSOR_CORE_WA) && !(flags & CDSSM_SCAN_FORCE_SIMT) && (!wa_ok || H % 4)) return CDSSM_ERR_UNSUPPORTED;
     // (the precision that the CUDA-core walk gave these calls before they came here)
     const int wa_parts = (H % 4 == 0 && tail_state == nullptr) || (flags & CDSSM_SCAN_TENSOR_CORE_WA) ? 2 : 3;
     const bool tc_local = !(flags & CDSSM_SCAN_KEEP_SIMT_LOCAL), tc_output = !(flags & CDSSM_SCAN_KEEP_SIMT_OUTPUT);
-    const bool one_kernel = chunk_ok && tc_local && tc_output && a.run_local && !summary_only && ((uintptr_t)h0 & 15) == 0 &&
-                            one_kernel_pays(B, H, a.NC, D, N);
-    // Status word, and for the one-kernel scan its ticket counter and its "carry is there" words in the gamma slots: cleared
-    // by the records kernel where that runs first.
-    const bool tensor = wa_ok || chunk_ok;
+    // The whole-chunk scan hands the carry on inside one kernel where the scratch has room for the words that do it; else local,
+    // carry and output pass: the same arithmetic in the same order, so this choice may go by size.
+    const size_t records = align256(scan_record_bytes(B, L, H, N, C));
+    const bool one_kernel = tile_ok && tc_local && tc_output && a.run_local && !summary_only && hands_carry_on(B, H, a.NC, D, N) &&
+                            workspace_bytes - base >= records + scan_tile_extra_bytes(B, L, H, D, N);
+    // Status word; for the one-kernel scan everything from there through the chunk states, and the carries: cleared by the records
+    // kernel where that runs first.
+    const bool tensor = wa_ok || tile_ok;
     const bool fill_records = tensor && (a.run_local || (flags & CDSSM_SCAN_TENSOR_CORE_WA));
-    const size_t clear_words = one_kernel ? 64 + (size_t)a.units * 2 : 1;
-    if (!fill_records)
-        if (int rc = check_cuda(cudaMemsetAsync(status, 0, clear_words * sizeof(int), st))) return rc;
     void* rec = reinterpret_cast<char*>(a.ws_state) + align256((size_t)a.units * 2 * D * sizeof(float));
+    void* extra = static_cast<char*>(rec) + records;
+    if (!fill_records)
+        if (int rc = check_cuda(cudaMemsetAsync(status, 0, sizeof(int), st))) return rc;
     a.rec_av = nullptr;
     a.rec_bs = nullptr;
     if (!tensor && workspace_bytes - base >= simt_record_bytes(B, L, H, N, C)) {
@@ -970,22 +973,20 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (!tensor) return scan_fused_simt(a, dtype, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
-    // (The whole-chunk output pass has also done all that needs no carry by the time the local pass ends.  scan_wa.cu: while its
-    // output pass has a chunk of four heads per block, two blocks per SM; us, carry pass / without: D 64, 936 chunks 24.4 / 21.5,
-    // 3072 42 / 44; D 128, 528 32.3 / 30.5, 1536 61 / 63.)
-    const int from_chunks = (chunk_ok || (wa_ok && (long long)B * a.NC * ((H + 3) / 4) <= 296)) &&
-                            tc_local && tc_output && a.run_local && !summary_only && few_chunks(a.NC, N);
+    const int from_chunks = wa_ok && carry_in_output(B, a.NC, H) && tc_local && tc_output && a.run_local && !summary_only;
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
                                 limit, withhold, from_chunks, h0, final_state, wa_parts, st);
-        return scan_chunk_pass(mode, from_chunks, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, status, status + 1,
-                               shortcut_scale, B, L, H, D, N, limit, withhold, st);
+        return scan_tile_pass(mode, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, one_kernel ? extra : nullptr,
+                              status, status + 1, shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };
     // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)
     if (fill_records)
         if (int rc = scan_records(wa_ok, v, v_rs, rows.first, vf_rs, rows.mix, gate_raw, g_rs, log_dt_scale, rope_freqs, rec, status,
-                                  clear_words, a.dc, B, L, H, N, C, pos0, segs, a.fp32_decay, st))
+                                  one_kernel ? ((char*)rec - (char*)status) / sizeof(int) : 1, static_cast<int*>(extra),
+                                  one_kernel ? scan_tile_extra_bytes(B, L, H, D, N) / sizeof(int) : 0, a.dc, B, L, H, N, C, pos0, segs,
+                                  a.fp32_decay, st))
             return rc;
     if (one_kernel) return pass(2);
     if (a.run_local && tc_local) {

@@ -239,6 +239,28 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* r) {
                  : "r"(taddr)
                  : "memory");
 }
+// 16 rows x 32 columns in the accumulator layout of the warp-level mma: x[4 n + e] = row g (+ 8 for e >= 2), column 8 n + 2 t4
+// (+ 1 for odd e), with g = lane / 4, t4 = lane % 4.  taddr's lane: a multiple of 16 inside the warp's 32.  Not waited for:
+// tmem_ld_wait() comes before the values are used.
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, float (&x)[16]) {
+    uint32_t* u = reinterpret_cast<uint32_t*>(x);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+        : "r"(taddr)
+        : "memory");
+}
+// Waits for every tensor-memory load of the warp; the values pass through, so no use of them moves above it.
+__device__ __forceinline__ void tmem_ld_wait(float (&x)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile(""
+                 : "+f"(x[0]), "+f"(x[1]), "+f"(x[2]), "+f"(x[3]), "+f"(x[4]), "+f"(x[5]), "+f"(x[6]), "+f"(x[7]), "+f"(x[8]),
+                   "+f"(x[9]), "+f"(x[10]), "+f"(x[11]), "+f"(x[12]), "+f"(x[13]), "+f"(x[14]), "+f"(x[15])
+                 :
+                 : "memory");
+}
 // Bounded wait with the limit as an argument (nanoseconds of the global timer).
 __device__ __forceinline__ bool mbar_wait_ns(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                              uint64_t limit_ns) {

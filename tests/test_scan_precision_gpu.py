@@ -122,6 +122,35 @@ def test_tokens_before_a_bad_value_do_not_see_it(ops, orc, D, N, value, what):
     assert np.isfinite(to_np(y)[0, :t]).all()
 
 
+@pytest.mark.parametrize("B,H,NC,D,N", [(1, 3, 5, 64, 4), (2, 5, 3, 64, 16), (24, 8, 40, 64, 6), (1, 1, 29, 64, 16), (3, 2, 4, 128, 8), (2, 3, 2, 128, 16)])
+def test_scratch_without_room_for_the_carries_gives_the_same_bits(ops, orc, B, H, NC, D, N):
+    """The whole-chunk scan hands the carry on inside one kernel where the scratch has room for the words that do it, else between
+    three: full and partly filled column tiles, an odd last head, two blocks a chunk, more chunks back than a warp asks for at once."""
+    import ctypes
+    import cdssm_b200
+    lib = cdssm_b200._lib.lib()
+    L = NC * D - 3
+    inp = _inputs(orc, B, H, L, D, N, seed=N)
+    bf = lambda x: to_dev(x, torch.bfloat16)
+    f = lambda x: to_dev(x, torch.float32)
+    h0 = f(np.random.default_rng(5).standard_normal((B, H, N, D)).astype(np.float32))
+    t = [bf(inp[k]) for k in ("q", "k", "v", "gate_raw")] + [f(inp["log_dt_scale"]), f(inp["rope_freqs"]), h0]
+    full = ops.scan_fused_workspace_bytes(B, L, H, D, N, D)
+    least = full - B * NC * H * (N // 2) * D * 8
+    results = []
+    for room in (full, least):
+        ws = torch.full((room + 256,), 0xa5, dtype=torch.uint8, device="cuda")
+        out = [torch.full((B, L, H, N), 3.0, device="cuda", dtype=torch.bfloat16), torch.full((B, H, N, D), 3.0, device="cuda"),
+               torch.full((B, H, N, D), 3.0, device="cuda")]
+        args = [x.data_ptr() for x in t + out] + [ws.data_ptr() + (-ws.data_ptr()) % 256, room]
+        args += [ctypes.c_float(c) for c in const_args(inp["consts"])] + [ctypes.c_float(0.25), B, L, H, D, N, D, 0, 0, 0]
+        assert lib.cdssm_b200_scan_fused_fwd(*args, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        results.append(out)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 def test_two_threads_share_a_stream(ops, orc):
     """Scans of two sizes from two threads on one stream: each uses the stream's scratch buffer for itself."""
     import threading
