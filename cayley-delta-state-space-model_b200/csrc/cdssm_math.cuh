@@ -141,6 +141,35 @@ template <typename T> __device__ __forceinline__ void rnd2(float& a, float& b) {
     }
 }
 
+// Pairs, for the kernels that are bound by issue slots beside memory: two values an instruction, in float32 or, where the values are
+// bf16 already and the result is rounded to it, in bf16 (one rounding, as of the float32 result).
+__device__ __forceinline__ float2 unpack2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ __nv_bfloat162 as_bf16x2(uint32_t w) { return *reinterpret_cast<__nv_bfloat162*>(&w); }
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    __nv_bfloat162 p = __hmul2_rn(as_bf16x2(a), as_bf16x2(b));
+    return *reinterpret_cast<uint32_t*>(&p);
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    __nv_bfloat162 p = __hadd2_rn(as_bf16x2(a), as_bf16x2(b));
+    return *reinterpret_cast<uint32_t*>(&p);
+}
+// x / (1 + 2^(-x log2 e)); what the approximations flush to zero is nothing beside one, or below every quotient that is kept.
+__device__ __forceinline__ float2 silu2(float2 x) {
+    const float2 t = __fmul2_rn(x, make_float2(-1.44269504f, -1.44269504f));
+    float2 e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
+    const float2 d = __fadd2_rn(e, make_float2(1.f, 1.f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
+    return __fmul2_rn(x, r);
+}
+// Two channels of GroupNorm, gate and skip: rnd(rnd(rnd(GN(f)) rnd(silu(z))) + rnd(skip x)), bf16 pairs
+__device__ __forceinline__ uint32_t gate_pair(float2 f, float mean, float rstd, float2 gw, float2 gb, uint32_t z, uint32_t skip, uint32_t x) {
+    const float2 n = __ffma2_rn(__fmul2_rn(__fadd2_rn(f, make_float2(-mean, -mean)), make_float2(rstd, rstd)), gw, gb), s = silu2(unpack2(z));
+    return add_bf16x2(mul_bf16x2(pack2(n.x, n.y), pack2(s.x, s.y)), mul_bf16x2(skip, x));
+}
+
 // Two consecutive elements as one access where `vec` says they are aligned.
 template <typename T> __device__ __forceinline__ float2 ld_pair(const T* p, bool vec) {
     if (!vec) return make_float2(IO<T>::ld(p), IO<T>::ld(p + 1));

@@ -199,19 +199,27 @@ groupnorm_gate_fwd_kernel(const T* y, const float* stats, const T* gn_w,
     Vec8<T>::ld(z + row * z_row_stride + c, zz);
     Vec8<T>::ld(skip + c, sk);
     Vec8<T>::ld(x_conv + row * di + c, xc);
+    if constexpr (IO<T>::kBf16) {
+        uint32_t o[4];
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const float n = IO<T>::rnd((f[e] - mean) * rstd * gw[e] + gb[e]);
-        const float g = IO<T>::rnd(siluf_<IO<T>::kBf16>(zz[e]));
-        f[e] = IO<T>::rnd(n * g) + IO<T>::rnd(sk[e] * xc[e]);
+        for (int i = 0; i < 4; i++)
+            o[i] = gate_pair(make_float2(f[2 * i], f[2 * i + 1]), mean, rstd, make_float2(gw[2 * i], gw[2 * i + 1]),
+                             make_float2(gb[2 * i], gb[2 * i + 1]), pack2(zz[2 * i], zz[2 * i + 1]), pack2(sk[2 * i], sk[2 * i + 1]),
+                             pack2(xc[2 * i], xc[2 * i + 1]));
+        *reinterpret_cast<uint4*>(out + row * di + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; e++) f[e] = ((f[e] - mean) * rstd * gw[e] + gb[e]) * siluf_<false>(zz[e]) + sk[e] * xc[e];
+        Vec8<T>::st(out + row * di + c, f);
     }
-    Vec8<T>::st(out + row * di + c, f);
 }
 
 // The same with statistics given, kRows tokens per block: the per-channel parameters are loaded once, and the rows' loads are
 // in flight together in storage form (unpacked they held 96 registers, and few blocks per SM left the memory waiting).
 // Measured on B200, bf16, 16 384 tokens of 1536 channels: 57 -> 37 us, twice what a copy of half the bytes takes (18.5 us); four
-// rows per block 41.
+// rows per block 41.  Bound by issue slots beside memory (602 instructions a warp for 16 values a lane): with values and products in pairs
+// (gate_pair) read-out, statistics and this take 60 instead of 65 us.  Read-out and gate in one kernel, the read-out formed twice on
+// the tensor cores instead of stored: 65 to 72.
 template <typename T, int kRows, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads)
 groupnorm_gate_rows_kernel(const T* y, const float* stats, const T* gn_w,
@@ -239,23 +247,27 @@ groupnorm_gate_rows_kernel(const T* y, const float* stats, const T* gn_w,
 #pragma unroll
     for (int r = 0; r < kRows; r++) {
         if (r0 + r >= rows) break;
-        float a[8], b[8], d[8];
+        float a[8];
         f[r].get(a);
-        zz[r].get(b);
-        xc[r].get(d);
+        if constexpr (IO<T>::kBf16) {
+            const uint32_t z4[4] = {zz[r].v.x, zz[r].v.y, zz[r].v.z, zz[r].v.w}, x4[4] = {xc[r].v.x, xc[r].v.y, xc[r].v.z, xc[r].v.w};
+            uint32_t o[4];
 #pragma unroll
-        for (int e = 0; e < 8; e += 2) {   // in pairs: one conversion instruction rounds two values
-            float n0 = (a[e] - st[r].x) * st[r].y * gw[e] + gb[e], n1 = (a[e + 1] - st[r].x) * st[r].y * gw[e + 1] + gb[e + 1];
-            float s0 = siluf_<IO<T>::kBf16>(b[e]), s1 = siluf_<IO<T>::kBf16>(b[e + 1]);
-            rnd2<T>(n0, n1);
-            rnd2<T>(s0, s1);
-            float p0 = n0 * s0, p1 = n1 * s1, q0 = sk[e] * d[e], q1 = sk[e + 1] * d[e + 1];
-            rnd2<T>(p0, p1);
-            rnd2<T>(q0, q1);
-            a[e] = p0 + q0;
-            a[e + 1] = p1 + q1;
+            for (int i = 0; i < 4; i++)
+                o[i] = gate_pair(make_float2(a[2 * i], a[2 * i + 1]), st[r].x, st[r].y, make_float2(gw[2 * i], gw[2 * i + 1]),
+                                 make_float2(gb[2 * i], gb[2 * i + 1]), z4[i], pack2(sk[2 * i], sk[2 * i + 1]), x4[i]);
+            *reinterpret_cast<uint4*>(out + (long long)(r0 + r) * di + c) = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+            float b[8], d[8];
+            zz[r].get(b);
+            xc[r].get(d);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float n = (a[e] - st[r].x) * st[r].y * gw[e] + gb[e];
+                a[e] = n * siluf_<false>(b[e]) + sk[e] * d[e];
+            }
+            Vec8<T>::st(out + (long long)(r0 + r) * di + c, a);
         }
-        Vec8<T>::st(out + (long long)(r0 + r) * di + c, a);
     }
 }
 
