@@ -21,6 +21,7 @@
 // The dynamics of a chunk are computed once per unit into shared memory before the walk.
 #include "cdssm_common.cuh"
 #include "decode_unit.cuh"
+#include "sm100_ptx.cuh"
 #include <atomic>
 
 namespace cdssm {
@@ -148,7 +149,9 @@ __device__ __forceinline__ void stage_dynamics(const ScanArgs& a, ChunkScalars& 
 }
 
 // kOutput = false: local pass (z only).  kOutput = true: output pass (z, r, read-out).
-template <typename T, int kCols, int kLanes, bool kOutput>
+// kRing: rows that travel ahead of the step that uses them, as asynchronous copies to shared memory (a lane reads only what it has
+// copied itself: no barrier).  0: the next row only, in registers.  A step of a short walk takes less time than a row does to come.
+template <typename T, int kCols, int kLanes, bool kOutput, int kRing>
 // (No register cap: at most 6 resident blocks of 80 registers cost the output walk its overlap of a step's eleven sums, float32
 // 61 -> 34 us at 64 units and 173 -> 90 us at head_dim 128, bf16 with a full GPU 380 -> 368 us.)
 __global__ void __launch_bounds__(kSimtThreads, 1)
@@ -199,8 +202,34 @@ scan_walk_kernel(const ScanArgs a) {
     float cr = 1.f, ci = 0.f;
 
     RowSlice<T, kCols> kraw, qraw;
-    kraw.load(kbase, g, D, vec);
-    if (kOutput) qraw.load(qbase, g, D, vec);
+    constexpr int kPieces = kCols * (int)sizeof(T) / 16, kRows = kOutput ? 2 : 1;   // 16-byte pieces of a lane's slice; rows a token
+    uint4* ring = reinterpret_cast<uint4*>(smem + 6 * kUnits * C) + threadIdx.x;
+    auto piece = [&](int t, int row, int p) { return ring + (((t % kRing) * kRows + row) * kPieces + p) * kSimtThreads; };
+    auto fetch = [&](int t) {
+        const int row = min(t, Lc - 1);
+#pragma unroll
+        for (int p = 0; p < kPieces; p++) {
+            sm100::cp_async16(piece(t, 0, p), kbase + (long long)row * a.k_rs + g * kCols + p * (16 / (int)sizeof(T)), t < Lc);
+            if (kOutput) sm100::cp_async16(piece(t, 1, p), qbase + (long long)row * a.q_rs + g * kCols + p * (16 / (int)sizeof(T)), t < Lc);
+        }
+        sm100::cp_async_commit();
+    };
+    auto take = [&](int t) {   // row t, requested kRing - 1 requests ago
+        sm100::cp_async_wait_group<kRing - 2 < 0 ? 0 : kRing - 2>();
+#pragma unroll
+        for (int p = 0; p < kPieces; p++) {
+            *(reinterpret_cast<uint4*>(&kraw) + p) = *piece(t, 0, p);
+            if (kOutput) *(reinterpret_cast<uint4*>(&qraw) + p) = *piece(t, 1, p);
+        }
+    };
+    if constexpr (kRing > 0) {
+#pragma unroll 1
+        for (int t = 0; t < kRing - 1; t++) fetch(t);
+        take(0);
+    } else {
+        kraw.load(kbase, g, D, vec);
+        if (kOutput) qraw.load(qbase, g, D, vec);
+    }
     const int so = ul * C;
     // The four units of a warp may sit in different chunks (a full one and the ragged last one):
     // every lane walks the warp's longest chunk so that the shuffles stay warp-wide; beyond its
@@ -210,7 +239,10 @@ scan_walk_kernel(const ScanArgs a) {
         float2 kk[kP], qq[kP];
         kraw.get(reinterpret_cast<float*>(kk));
         if (kOutput) qraw.get(reinterpret_cast<float*>(qq));
-        if (t + 1 < Lc) {
+        if constexpr (kRing > 0) {
+            fetch(t + kRing - 1);
+            take(t + 1);
+        } else if (t + 1 < Lc) {
             kraw.load(kbase + (long long)(t + 1) * a.k_rs, g, D, vec);
             if (kOutput) qraw.load(qbase + (long long)(t + 1) * a.q_rs, g, D, vec);
         } else {
@@ -533,19 +565,35 @@ scan_carry_kernel(const ScanArgs a) {
     }
 }
 
-template <typename T, int kCols, bool kOutput> struct WalkTag {};
+// Whether the walks' rows travel ahead through shared memory: while there is a block per SM at most; more blocks hide each other's
+// waits and want the shared memory.  us of a call on B200, next row in registers / ring of eight: float32, D 64, 64 units 49.3 / 45.8,
+// 768 52.4 / 49.7, 1536 57.0 / 50.0, 6144 98 / 129; D 128, 1024 units 154 / 135, 4096 236 / 291; bf16, D 64, 240 units 52.5 / 46.9,
+// 3072 69.3 / 65.8, 6144 92.3 / 93.6.
+static bool walk_with_ring(const ScanArgs& a, int cols, int es, unsigned blocks) {
+    return blocks <= 148 && a.D == cols * kLanesPerUnit && a.C <= a.D && ((a.k_rs | a.q_rs) * es) % 16 == 0;
+}
+
+template <typename T, int kCols, bool kOutput, int kRing> struct WalkTag {};
+
+template <typename T, int kCols, bool kOutput, int kRing>
+static int launch_walk(const ScanArgs& a, unsigned blocks, cudaStream_t st) {
+    constexpr int kRows = kOutput ? 2 : 1;
+    constexpr size_t ring = (size_t)kRing * kRows * kCols * sizeof(T) * kSimtThreads;
+    const size_t scalars = (size_t)6 * kUnitsPerBlock * sizeof(float);
+    const size_t smem = scalars * a.C + ring;
+    if (smem > 48 * 1024) {   // opt in to more than 48 KB of dynamic shared memory
+        const size_t most = kRing ? scalars * kCols * kLanesPerUnit + ring : scalars * kMaxChunk;   // (with a ring: C <= D)
+        if (int rc = allow_smem<WalkTag<T, kCols, kOutput, kRing>>((const void*)scan_walk_kernel<T, kCols, kLanesPerUnit, kOutput, kRing>, most)) return rc;
+    }
+    return launch_overlapped(scan_walk_kernel<T, kCols, kLanesPerUnit, kOutput, kRing>, dim3(blocks), dim3(kSimtThreads), smem, st, a);
+}
 
 template <typename T, int kCols>
 static int launch_simt(const ScanArgs& a, cudaStream_t st) {
-    constexpr int kLanes = kLanesPerUnit, kUnits = kUnitsPerBlock;
-    const size_t smem = (size_t)6 * kUnits * a.C * sizeof(float);
-    if (smem > 48 * 1024) {   // opt in to more than 48 KB of dynamic shared memory
-        constexpr size_t kMost = (size_t)6 * kUnits * kMaxChunk * sizeof(float);
-        if (int rc = allow_smem<WalkTag<T, kCols, false>>((const void*)scan_walk_kernel<T, kCols, kLanes, false>, kMost)) return rc;
-        if (int rc = allow_smem<WalkTag<T, kCols, true>>((const void*)scan_walk_kernel<T, kCols, kLanes, true>, kMost)) return rc;
-    }
+    constexpr int kUnits = kUnitsPerBlock, kRing = 8;
     const unsigned blocks = (unsigned)((a.units + kUnits - 1) / kUnits);
     const bool output = a.y != nullptr && a.run_output;   // else: summary only, or y comes from another kernel
+    const bool ring = walk_with_ring(a, kCols, (int)sizeof(T), blocks);
     if (a.rec_av != nullptr && (a.run_local || output)) {
         // pairs over the grid as far as one wave goes (what the pairs of a token share is computed again for each)
         const long long wave = ((long long)a.B * a.L + 31) / 32 * ((a.H + 7) / 8);
@@ -554,11 +602,11 @@ static int launch_simt(const ScanArgs& a, cudaStream_t st) {
         if (int rc = check_launch()) return rc;
     }
     if (a.run_local)
-        if (int rc = launch_overlapped(scan_walk_kernel<T, kCols, kLanes, false>, dim3(blocks), dim3(kSimtThreads), smem, st, a)) return rc;
+        if (int rc = ring ? launch_walk<T, kCols, false, kRing>(a, blocks, st) : launch_walk<T, kCols, false, 0>(a, blocks, st)) return rc;
     const long long th = (long long)a.B * a.H * (a.N / 2) * a.D;
     if (int rc = launch_overlapped(scan_carry_kernel<T>, dim3((unsigned)((th + 127) / 128)), dim3(128), 0, st, a)) return rc;
     if (!output) return CDSSM_OK;
-    return launch_overlapped(scan_walk_kernel<T, kCols, kLanes, true>, dim3(blocks), dim3(kSimtThreads), smem, st, a);
+    return ring ? launch_walk<T, kCols, true, kRing>(a, blocks, st) : launch_walk<T, kCols, true, 0>(a, blocks, st);
 }
 
 // Column split: D <= 64 -> 8 lanes x 8 columns, D <= 128 -> 8 lanes x 16 columns (16 lanes x 8 columns was slower: 10.8 ms
