@@ -42,8 +42,10 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
     grid_dependency_wait();
-    if (blockIdx.z == 0) {
-        const size_t first = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x, step = (size_t)gridDim.x * gridDim.y * kThreads;
+    const size_t first = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x, step = (size_t)gridDim.x * gridDim.y * kThreads;
+    if (kWa) {   // a few words
+        for (size_t i = first; i < a.clear_words; i += step) a.clear[i] = 0;
+    } else if (blockIdx.z == 0) {
         for (size_t i = first; i < a.clear_words / 4; i += step) reinterpret_cast<uint4*>(a.clear)[i] = make_uint4(0u, 0u, 0u, 0u);
         if (first < a.clear_words % 4) a.clear[a.clear_words / 4 * 4 + first] = 0;
         for (size_t i = first; i < a.clear2_words / 4; i += step) reinterpret_cast<uint4*>(a.clear2)[i] = make_uint4(0u, 0u, 0u, 0u);
