@@ -138,10 +138,12 @@ __device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, 
     return slow;
 }
 
-// Factor that takes block `from`'s scaled sums into block `to`'s frame (to = blocks: the chunk end), blocks counted in the
-// chunk, bp at the chunk's first block: decay behind `from`'s middle, over the blocks in between, up to `to`'s middle.
-__device__ __forceinline__ cplx frame(const BlockPair* bp, int from, int to, int blocks) {
-    cplx f = bp[from].D31;
+// What takes block `from`'s sums, carried to its end, into block `to`'s frame (to = blocks: the chunk end), blocks counted in the
+// chunk, bp at the chunk's first block: the decay over the blocks in between and up to `to`'s middle.  To its end a block's scaled
+// sums (up to 1e30) are carried by D31 (down to 1e-30), and by that alone: its product with the later block's R (1e-30 as well) would
+// be zero in float32 where the value is of order one.
+__device__ __forceinline__ cplx behind(const BlockPair* bp, int from, int to, int blocks) {
+    cplx f = {1.f, 0.f};
     for (int j = from + 1; j < to; j++) f = cmul(f, bp[j].A);
     return to < blocks ? cmul(f, bp[to].R) : f;
 }
@@ -320,11 +322,11 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int r
 #pragma unroll
     for (int i = 0; i < kCols; i++) zr[i] = zi[i] = 0.f;
     for (int J = 0; J < I; J++) {
-        const cplx F = frame(bp, J, I, G::kBlocks);   // (this block's own reference product is one)
+        const cplx D31 = bp[J].D31, F = behind(bp, J, I, G::kBlocks);   // (this block's own reference product is one)
         const float* gr = sm.vec[kG] + 2 * p * G::kRow + row0 + 32 * J;
 #pragma unroll 4
         for (int t = 0; t < 32; t++) {
-            const cplx w = cmul(F, {gr[t] + gr[G::kPart + t], gr[G::kRow + t] + gr[G::kRow + G::kPart + t]});
+            const cplx w = cmul(F, cmul(D31, {gr[t] + gr[G::kPart + t], gr[G::kRow + t] + gr[G::kRow + G::kPart + t]}));
 #pragma unroll
             for (int i = 0; i < kCols; i++) {
                 const float k = column(sm.k, row0 + 32 * J + t, tl + 32 * i);
@@ -770,6 +772,11 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     // complex factor times the lane's component; `other` is the other component of the same value
     auto rotate = [&](cplx f, float own, float other) { return f.r * own + (comp ? f.i : -f.i) * other; };
     auto other_of = [](float x) { return __shfl_xor_sync(0xffffffffu, x, 1); };
+    // block J's scaled sum times D31, then times f (behind()), this lane's component
+    auto carried = [&](cplx d31, cplx f, float own) {
+        const float other = other_of(own), i = comp ? d31.i : -d31.i;
+        return rotate(f, d31.r * own + i * other, d31.r * other - i * own);
+    };
 
     // x <- (I + M_own)^-1 x, all column tiles; published as vector v
     auto solve = [&](int v, float (&x)[kOwn][4]) {
@@ -892,9 +899,10 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 times(M[J], One(), kG, J, &s[0][0]);
 #pragma unroll
                 for (int q = 0; q < kOwn; q++) {
-                    const cplx F = frame(&sm.bp[pair_of(q)][row0 / 32], J, I, kBlocks);
+                    const BlockPair* bp = &sm.bp[pair_of(q)][row0 / 32];
+                    const cplx D31 = bp[J].D31, F = behind(bp, J, I, kBlocks);
 #pragma unroll
-                    for (int r = 0; r < 4; r++) gx[q][r] -= cc[r] * rotate(F, s[q][r], other_of(s[q][r]));
+                    for (int r = 0; r < 4; r++) gx[q][r] -= cc[r] * carried(D31, F, s[q][r]);
                 }
             }
         solve(kG, gx);
@@ -966,13 +974,13 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 }
 #pragma unroll
             for (int q = 0; q < kOwn; q++) {
-                cplx F = {1.f, 0.f};
-                if (v == kG) F = frame(&sm.bp[pair_of(q)][row0 / 32], J, kBlocks, kBlocks);
+                const BlockPair* bp = &sm.bp[pair_of(q)][row0 / 32];
+                const cplx D31 = bp[J].D31, F = behind(bp, J, kBlocks, kBlocks);
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
                     const float x0 = sum_lo(d[q][m][0], d[q][m][1]), x1 = sum_hi(d[q][m][0], d[q][m][1]);
-                    z[q][m][0] += v == kG ? rotate(F, x0, other_of(x0)) : x0;
-                    z[q][m][1] += v == kG ? rotate(F, x1, other_of(x1)) : x1;
+                    z[q][m][0] += v == kG ? carried(D31, F, x0) : x0;
+                    z[q][m][1] += v == kG ? carried(D31, F, x1) : x1;
                 }
             }
         }
@@ -1269,11 +1277,15 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         times(x, Two(), kG, J, &s[0][0][0]);
 #pragma unroll
         for (int q = 0; q < kOwn; q++) {
-            cplx F = {1.f, 0.f};
-            if (!diag) F = frame(&sm.bp[pair_of(q)][row0 / 32], J, I, kBlocks);
+            cplx D31 = {1.f, 0.f}, F = {1.f, 0.f};
+            if (!diag) {
+                const BlockPair* bp = &sm.bp[pair_of(q)][row0 / 32];
+                D31 = bp[J].D31;
+                F = behind(bp, J, I, kBlocks);
+            }
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                oz[q][r] += rotate(F, s[0][q][r], other_of(s[0][q][r]));
+                oz[q][r] += carried(D31, F, s[0][q][r]);
                 rho[q][r] -= s[1][q][r];
             }
         }

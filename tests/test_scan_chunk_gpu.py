@@ -75,3 +75,36 @@ def test_chunk_scan_strong_decay(ops, orc, D, N, alpha_gate):
     assert rel_err(to_np(y), to_np(ys)) <= BF16_TOL / 2
     _close(fin, fs, 2e-2)
     _close(tail, ts, 2e-2)
+
+
+@pytest.mark.parametrize("keep", [0, KEEP_SIMT_LOCAL, KEEP_SIMT_OUTPUT])
+@pytest.mark.parametrize("D,N", [(64, 4), (64, 16), (128, 4), (128, 16)])
+@pytest.mark.parametrize("decay", ["every token", "two tokens"])
+def test_chunk_scan_decay_on_both_sides_of_a_block_boundary(ops, orc, D, N, decay, keep):
+    """A strong decay in the second half of a 32-token block and another in the first half of the next, each inside the range of the
+    scaled unknowns (1e-30), their product far below the smallest float32: what one block hands to the next is of order one all the same.
+    Each output against the walk: both round y twice, four times 2^-8 of the larger of itself and the typical output."""
+    B, H, L = 2, 4, 4 * D - 3
+    inp = _inputs(orc, B, H, L, D, N, seed=5)
+    NH, r = N // 2, slice((N + 4) * H, None)
+    inp["rope_freqs"], inp["log_dt_scale"] = np.zeros(H, np.float32), np.zeros(H, np.float32)
+    inp["consts"] = orc.derive_constants(2048)
+    g = inp["gate_raw"].copy()
+    if decay == "every token":                   # 0.02 each
+        g[..., :NH * H], g[..., NH * H:2 * NH * H], g[..., (N + 2) * H:(N + 3) * H] = 4.0, 0.0, 1.0
+        g[..., r] = np.random.default_rng(6).uniform(0.7, 0.9, g[..., r].shape)
+    else:                                        # 1e-19 once, ordinary ones beside it
+        at = (np.arange(L) % 64 == 18) | (np.arange(L) % 64 == 44)
+        g[..., r] -= 2.0
+        g[:, at, :NH * H], g[:, at, NH * H:2 * NH * H], g[:, at, (N + 2) * H:(N + 3) * H] = 2.0625, 0.0, 0.0
+        g[:, at, r] = 8.0
+    inp["gate_raw"] = orc.bf16_round(g)
+    A, *_ = orc.dynamics(inp["gate_raw"], inp["log_dt_scale"], inp["rope_freqs"], inp["consts"], H, N, round_bf16=orc.ROUND_INPUTS)
+    size = np.log10(np.hypot(A[..., 0::2], A[..., 1::2]))[:, :2 * 32].reshape(B, 4, 16, H, NH).sum(2)   # of the first half blocks
+    assert size.min() > -29.0 and np.median(size[:, 1] + size[:, 2]) < -40.0
+    y, fin, tail = run_fused(ops, inp, torch.bfloat16, N, D, flags=keep, return_tail_state=True, shortcut_scale=0.3)
+    assert ops.scan_fused_status() == 0
+    ys, fs, ts = run_fused(ops, inp, torch.bfloat16, N, D, flags=ops.FORCE_SIMT, return_tail_state=True, shortcut_scale=0.3)
+    for a, b in ((y, ys), (fin, fs), (tail, ts)):
+        a, b = to_np(a), to_np(b)
+        assert (np.abs(a - b) <= 2.0 ** -6 * np.maximum(np.abs(b), np.sqrt(np.square(b).mean()))).all()
