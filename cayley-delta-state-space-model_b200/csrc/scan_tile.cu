@@ -15,9 +15,11 @@
 //     (as 8 x 8 halves: seven dependent steps instead of fifteen);
 //   - what is left of the serial chain is three 16-wide products per 32 tokens, passed from warp to warp;
 //   - everything with a right-hand side is a warp-level tf32 product with n = 8 columns {re hi, re lo, im hi, im lo} of two
-//     pairs; a float32 operand enters as hi + lo, 11 significant bits each, on the matrix side too.  G and P go in as they
-//     come from tensor memory: an instruction's split costs two operations a value (three bf16 parts: five and a half, and as
-//     many products).  One chunk's state is off by no more than that of a walk in float32 (test_scan_precision_gpu.py).
+//     pairs; a float32 operand enters as hi + lo, 11 significant bits each, on the matrix side too, hi rounded to nearest: the sum
+//     is the value to half an ulp (root mean square).  G and P go in as they come from tensor memory: an instruction's split costs
+//     three operations a value (three bf16 parts: five and a half, and as many products).  State after one chunk against float64,
+//     median, D 64 / 128: 1.6e-7 / 1.8e-7 of it; three bf16 parts 1.6e-7 / 1.9e-7, the walk in float32 1.5e-7 / 1.8e-7, hi cut off
+//     instead of rounded 2.5e-7 / 2.4e-7 (test_scan_precision_gpu.py).
 // The division by W_i only spans a 32-token block, relative to its middle (|W ratio| of 16 tokens >= 1e-30); between blocks
 // all factors are plain products, applied to the sums over a block.  A (block, pair) that decays further is walked step by
 // step (slow_walk).
@@ -80,7 +82,9 @@ __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2
 __device__ __forceinline__ float bits_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ float bits_lo(uint32_t w) { return __uint_as_float(w << 16); }
 
-// 1 / x for normal x in 1e-30 ... 1e30: the approximation and one Newton step, no branch for the values outside.
+// 1 / x for normal x in 1e-30 ... 1e30: the approximation and one Newton step, no branch for the values outside.  Its remainder is
+// squared by the step (2^-44), so the result is the nearest float but where two are as near to 2^-20 of their distance; __frcp_rn
+// gave states off by the same three digits and took 3 % of the call.
 __device__ __forceinline__ float reciprocal(float x) {
     const float r = __fdividef(1.f, x);
     return fmaf(r, fmaf(-x, r, 1.f), r);
@@ -184,8 +188,10 @@ __device__ __forceinline__ uint64_t carry_word(float r, float i) {
 __device__ __forceinline__ uint32_t bf16_pair(cplx x) { return pack2(x.r, x.i); }
 __device__ __forceinline__ cplx pair_of_word(uint32_t w) { return {bits_lo(~w), bits_hi(~w)}; }
 
-// The leading 11 significant bits, what a tf32 operand holds; the rest fits another one (to 2^-22 of x).
-__device__ __forceinline__ float tf32_hi(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
+// The nearest value of 11 significant bits, what a tf32 operand holds.  The rest, 12 bits and a sign, goes into another one, which
+// drops its last bit: an ulp of x in one value of four, to either side.  (Cut off instead of rounded, the rest had 13 bits and lost
+// up to three ulps, always to the same side.)
+__device__ __forceinline__ float tf32_hi(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
 
 // One k-step of eight columns: x in accumulator order (row g: columns 2 t4, 2 t4 + 1; row g + 8), b the two tokens' values of
 // this lane's column.  kFirst: d = x b, else d += x b.

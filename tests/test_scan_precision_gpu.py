@@ -43,15 +43,20 @@ def _state64(ops, inp, N):
 @pytest.mark.parametrize("H,D,N", [(8, 64, 2), (6, 64, 2), (4, 128, 2), (3, 64, 4), (3, 64, 8), (3, 64, 16), (2, 128, 4), (2, 128, 8),
                                    (2, 128, 16)])
 def test_tail_state_has_float32_precision(ops, orc, H, D, N):
-    """One chunk: nothing between the inputs and the state is rounded.  A chain of D float32 steps is off by a few times
-    sqrt(D) 2^-24 = 7e-7 of the state at D = 128; products of 16-bit parts left 1.7e-5.  (The median over the heads: where
-    the dynamics of the two sides round one bf16 value differently, a head moves by more.)"""
-    B, L = 6, D - 3
+    """One chunk: nothing between the inputs and the state is rounded, so the state is as near to float64 as the walk's, which is all
+    float32.  Measured, times 1e-7 of the state, D 64 / 128: N > 2 1.6 / 1.8, N 2 1.8 / 2.0, the walk 1.2 to 2.1 / 2.0 to 2.2; three bf16
+    parts for N > 2 1.7 / 2.3, operands of 22 bits cut off instead of rounded 2.4 / 2.5, products of 16-bit parts 170.  The bound: 3.7
+    roundings.  (The median over heads and pairs: where the dynamics of the two sides round one bf16 value differently, a head moves
+    by more.)"""
+    B, L = 24, D - 3
     inp = _inputs(orc, B, H, L, D, N, seed=D + N)
-    _, _, tail = run_fused(ops, inp, torch.bfloat16, N, D, return_tail_state=True)
-    want = _state64(ops, inp, N)
-    err = (tail.double() - want).flatten(2).norm(dim=-1) / want.flatten(2).norm(dim=-1)
-    assert float(err.median()) <= 2e-6
+    want = _state64(ops, inp, N).view(B, H, N // 2, 2 * D)
+    err = []
+    for flags in (0, ops.FORCE_SIMT):
+        tail = run_fused(ops, inp, torch.bfloat16, N, D, return_tail_state=True, flags=flags)[2]
+        off = (tail.double().view(B, H, N // 2, 2 * D) - want).norm(dim=-1) / want.norm(dim=-1)
+        err.append(float(off.median()))
+    assert err[0] <= 3.7 * 2.0 ** -24 and err[0] <= 1.6 * err[1]
 
 
 @pytest.mark.parametrize("H,D,N", [(8, 64, 2), (6, 64, 2), (4, 128, 2), (8, 64, 4), (8, 64, 16), (4, 128, 8), (4, 128, 16)])
