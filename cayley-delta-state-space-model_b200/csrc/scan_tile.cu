@@ -536,7 +536,8 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     };
     // A block that gives up stays until its own copies and products have landed (or a limit has passed again): the next one has
     // its memory then.
-    bool g_issued = false, p_issued = false;   // (warp 0)
+    int g_issued = 0;                          // (warp 0) products G: a second one where key rows have been emptied
+    bool p_issued = false;
     auto give_up = [&](int code, bool q_loaded) {
         cp_async_wait_all();
         if (W == 0) {
@@ -545,7 +546,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 int never = 0;
                 if (!a.withhold) mbar_wait_ns(&sm.full_k, 0, &never, a.wait_ns);
                 if (q_loaded && !a.withhold) mbar_wait_ns(&sm.full_q, 0, &never, a.wait_ns);
-                if (g_issued) mbar_wait_ns(&sm.mma_g, sm.bad_rows ? 1 : 0, &never, a.wait_ns);
+                if (g_issued) mbar_wait_ns(&sm.mma_g, g_issued - 1, &never, a.wait_ns);
                 if (p_issued) mbar_wait_ns(&sm.mma_p, 0, &never, a.wait_ns);
             }
             __syncwarp();
@@ -556,7 +557,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     };
 
     bool ok = wait(&sm.full_k, 0);
-    if (W == 0 && ok) { gram(kt, &sm.mma_g); g_issued = true; }
+    if (W == 0 && ok) { gram(kt, &sm.mma_g); g_issued = 1; }
     // the token's dynamics, from the kernel before this one (its launch let this one start early; no __ldg here: loads
     // that claim the data constant may be moved above the wait)
     if (early) grid_dependency_wait();
@@ -607,7 +608,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         bool number = fabsf(bits_lo(sm.bs[tok])) <= 3e38f;   // (false for NaN)
 #pragma unroll
         for (int r = 0; r < 4; r++) number = number && kk[r] <= 3.4e38f;
-        if (!__all_sync(0xffffffffu, number)) {
+        if (ok && !__all_sync(0xffffffffu, number)) {   // (not from tensor memory that nothing has been written to)
             const uint32_t bad = __ballot_sync(0xffffffffu, empty_bad_rows<kD, kPairs, kMode>(sm, tok, hs));
 #pragma unroll
             for (int m = 0; m < 2; m++)
@@ -739,7 +740,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     tc_fence_after();
     if (kOut && tid == 0 && !a.withhold) load_tile(sm.q, &tmQ, &sm.full_q);
     if (sm.bad_rows) {   // G without the emptied rows
-        if (W == 0) gram(kt, &sm.mma_g);
+        if (W == 0) { gram(kt, &sm.mma_g); g_issued = 2; }
         ok = wait(&sm.mma_g, 1);
         tc_fence_after();
     }

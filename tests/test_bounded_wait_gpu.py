@@ -51,3 +51,26 @@ def test_whole_chunk_scan_waits_run_out_too(ops, orc, D, L):
     y, _ = run_fused(ops, inp, torch.bfloat16, N, D, strict=True)
     wy, _ = oracle_scan(orc, inp, N, D, orc.ROUND_REFERENCE)
     assert rel_err(to_np(y), wy) <= BF16_TOL
+
+
+@pytest.mark.parametrize("D,N", [(64, 16), (64, 8), (128, 16)])
+@pytest.mark.parametrize("keep", [256, 512])
+def test_halves_of_the_whole_chunk_scan_give_up_too(ops, orc, D, N, keep):
+    """Its output pass (256: the local results come from the walk) and its local pass (512), two warps or two blocks to a chunk; the
+    next call finds the tensor memory free, with a key that is no number among its rows."""
+    B, H, L = 2, 5, 3 * D + 7
+    inp = orc.make_inputs(B, H, L, D, N=N, seed=43, bf16=True)
+    old = ops.set_wait_limit_ns(2_000_000)
+    try:
+        run_fused(ops, inp, torch.bfloat16, N, D, flags=ops.TEST_WITHHOLD | keep)
+        assert 200 <= ops.scan_fused_status() < 300
+    finally:
+        ops.set_wait_limit_ns(old)
+    inp["k"][1, D + 3, 2, 7] = np.nan
+    y, _ = run_fused(ops, inp, torch.bfloat16, N, D, strict=True, flags=keep)
+    y = to_np(y)
+    assert np.isnan(y[1, D + 3:, 2]).all()
+    inp["k"][1, D + 3:, 2] = inp["k"][1, D + 2, 2]
+    wy, _ = oracle_scan(orc, inp, N, D, orc.ROUND_FP32_STATE)
+    y[1, D + 3:, 2] = wy[1, D + 3:, 2]
+    assert rel_err(y, wy) <= BF16_TOL
