@@ -849,7 +849,7 @@ int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long
 // scan_tile.cu
 bool scan_tile_supported(int D, int N, int C, int dtype);
 size_t scan_tile_extra_bytes(int B, int L, int H, int D, int N);
-int scan_tile_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
+int scan_tile_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
                    float* final_state, float* tail_state, float* ws_gamma, float* ws_state, void* extra, int* status, int* ticket,
                    float shortcut_scale, int B, int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st);
 }
@@ -904,17 +904,32 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
 // 24.4 / 21.5, 3072 42 / 44; D 128, 528 32.3 / 30.5, 1536 61 / 63.
 static bool carry_in_output(int B, int NC, int H) { return (long long)B * NC * ((H + 3) / 4) <= 296 && NC <= 40; }
 
+// Tiles of the whole-chunk scan beside each other: a head (head_dim 128) or two (64) of a sequence.
+static long long scan_tiles(int B, int H, int D) { return (long long)B * (D == 128 ? H : (H + 1) / 2); }
+
+// Whether the output pass of the whole-chunk scan, where it is not one kernel, adds the carry up itself: a read of NC x N rows by every
+// block, in parallel, against a launch and two more trips to memory.  us of a call on B200, carry pass / without, one sequence: 4 heads
+// of 64, N 4 9 chunks 18.1 / 15.3, 25 20.1 / 18.2, 40 21.1 / 22.7; N 16 2 chunks 26.0 / 20.2, 16 29.4 / 28.8, 25 30.9 / 34.8; 24 heads,
+// N 8 9 chunks 24.0 / 22.1, 16 28.1 / 29.3; N 16 9 31.0 / 31.9; 24 heads of 128, N 8 9 chunks 99.8 / 72.6, 25 84.7 / 89.8.
+static bool few_chunks(int B, int H, int NC, int D, int N) {
+    return NC <= 10 || (scan_tiles(B, H, D) * NC <= 64 && NC * N <= 260);
+}
+
 // Whether the whole-chunk scan (scan_tile.cu) hands the carry on inside one kernel, or runs as local pass, carry pass and output
 // pass: the same arithmetic in the same order, so this choice may go by size.  One kernel forms G once and reads k once, but its
-// blocks add up the chunks between theirs and the last finished one, as many as there are blocks on a sequence: too many when few
-// tiles beside each other fill the GPU (head_dim 64: 592 blocks for N <= 4, else 296).  us on B200, one kernel / passes: N 4, 12
-// tiles 91 / 82, 24 tiles 163 / 160, 48 tiles 61 / 67; N 8, 6 tiles 63 / 78, 12 tiles 77 / 95, 24 tiles 139 / 176; N 16, 6 tiles
-// 122 / 112, 12 tiles 104 / 120, 24 tiles 163 / 188; N 16, 12 tiles, 9 chunks 30 / 43; head_dim 128, N 4, 4 tiles 49 / 59, N 16,
-// 24 tiles 146 / 178.
+// blocks add up the chunks between theirs and the last finished one, as many as there are blocks on a sequence.  That is too much for
+// head_dim 64 (592 blocks at a time for N <= 4, else 296), when few tiles beside each other fill the GPU with long sequences.  Time of
+// one kernel over that of the passes on B200, at these numbers of chunks:
+//   N 4:  1 tile 256: 0.96, 400: 1.07, 1024: 1.5; 6 tiles 96: 0.84, 180: 1.0, 512: 1.2; 12 tiles 64: 0.95, 96: 1.0, 256: 1.2; 24 tiles
+//         44: 0.91, 64: 1.04, 256: 1.2; 48 tiles 32: 0.92, 60: 1.05; 96 tiles 128: 1.04; 192 tiles 128: 0.94
+//   N 8:  1 tile 180: 0.95, 1024: 1.2; 2 tiles and more 512: 0.92 to 0.97
+//   N 16: 1 tile 96: 0.8, 256: 1.03, 1024: 1.6; 2 tiles 180: 1.0, 512: 1.1; 4 tiles 256: 0.94, 1024: 1.03; 96 tiles 0.8
+// (head_dim 128: 0.65 to 1.0, up to 1.1 with N 16 beyond 200 chunks.)
 static bool hands_carry_on(int B, int H, int NC, int D, int N) {
-    if (D == 128 || NC <= 28) return true;
-    const long long tiles = (long long)B * ((H + 1) / 2);
-    return N <= 4 ? tiles * 22 >= 592 : N <= 8 || tiles * 28 >= 296;
+    if (D == 128 || NC <= 45) return true;
+    const long long tiles = scan_tiles(B, H, D);
+    if (N > 4) return tiles > 2 || NC <= 180 * tiles;
+    return tiles >= 96 || (NC <= 300 && tiles * NC <= 1100);
 }
 
 struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual
@@ -1021,12 +1036,12 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (!tensor) return scan_fused_simt(a, dtype, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
-    const int from_chunks = wa_ok && carry_in_output(B, a.NC, H) && tc_local && tc_output && a.run_local && !summary_only;
+    const int from_chunks = (wa_ok ? carry_in_output(B, a.NC, H) : few_chunks(B, H, a.NC, D, N)) && tc_local && tc_output && a.run_local && !summary_only;
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,
                                 limit, withhold, from_chunks, h0, final_state, wa_parts, st);
-        return scan_tile_pass(mode, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, one_kernel ? extra : nullptr,
+        return scan_tile_pass(mode, from_chunks, q, q_rs, k, k_rs, rec, h0, y, final_state, tail_state, a.ws_gamma, a.ws_state, one_kernel ? extra : nullptr,
                               status, status + 1, shortcut_scale, B, L, H, D, N, limit, withhold, st);
     };
     // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)

@@ -28,7 +28,8 @@
 // (chunk, batch, head) work in chunk-major order from a ticket counter, leave their chunk's (gamma, z) for others as soon as they
 // have it, then look back for the nearest chunk whose carry-out is known and add up the chunks in between, in the order of the
 // sequence: the bits do not depend on how far anybody had come.  kLocal / kOutput are the two halves with the carry pass of
-// scan_simt.cu between them (summaries, callers with little scratch, few long sequences: hands_carry_on() there).
+// scan_simt.cu between them (summaries, callers with little scratch, few long sequences: hands_carry_on() there); while there are
+// few chunks the output pass adds them up itself instead, having done all that needs no carry by the time the local pass ends.
 //
 // Bounded by issue slots (45 % of them busy at 16 warps per SM) and by the chain of barriers and products through a chunk.  us of a
 // whole call on B200, before (a block per chunk and head, Gram blocks and three bf16 parts on the warp-level mma, carry behind a
@@ -68,6 +69,7 @@ struct Args {
     int B, L, H, N, NC;
     int HG;                      // tiles beside each other: ceil(H / heads of a tile) x blocks that share a tile (kPairs pairs each)
     int groups;
+    int from_chunks;             // kOutput: the carry from the local results of the chunks before (no carry pass has run)
     int fixed;                   // kFused: blocks have the tiles of their own numbers, not of tickets
 };
 
@@ -1164,17 +1166,70 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
     } else {
         grid_dependency_wait();   // the pass before; the records are there: it has waited for them before this launch
+        float sr[kOwnPairs], si[kOwnPairs];
 #pragma unroll
         for (int i = 0; i < kOwnPairs; i++) {
-            const int p = kOwnPairs * S + i;
-            float sr = 0.f, si = 0.f;
-            if (i < own_pairs) {
-                const float* s = state_at(a.ws_state, unit, i);
-                sr = __ldcg(s);
-                si = __ldcg(s + kD);
+            sr[i] = si[i] = 0.f;
+            if (i < own_pairs && (!a.from_chunks || a.h0)) {
+                const float* s = a.from_chunks ? state_at(a.h0, (size_t)b * H + hd, i) : state_at(a.ws_state, unit, i);
+                sr[i] = __ldcg(s);
+                si[i] = __ldcg(s + kD);
             }
-            sm.r0[hs][2 * p][col] = __float2bfloat16_rn(sr);
-            sm.r0[hs][2 * p + 1][col] = __float2bfloat16_rn(si);
+        }
+        auto into_chunk = [&]() {
+#pragma unroll
+            for (int i = 0; i < kOwnPairs; i++) {
+                const int p = kOwnPairs * S + i;
+                sm.r0[hs][2 * p][col] = __float2bfloat16_rn(sr[i]);
+                sm.r0[hs][2 * p + 1][col] = __float2bfloat16_rn(si[i]);
+            }
+        };
+        if (a.from_chunks) {      // s <- gamma s + z over the chunks before, in the carry pass's order
+            // (the last chunk's own step too, where the final state is wanted)
+            const int chunks = c + (c + 1 == a.NC && a.final_state ? 1 : 0);
+            constexpr int kBatch = 8 / kOwnPairs;
+#pragma unroll 1
+            for (int c0 = 0; c0 < chunks; c0 += kBatch) {
+                float l[kBatch][kOwnPairs][2];
+                float2 gm[kBatch][kOwnPairs];
+#pragma unroll
+                for (int k = 0; k < kBatch; k++)
+#pragma unroll
+                    for (int i = 0; i < kOwnPairs; i++)
+                        if (i < own_pairs) {
+                            const size_t u = ((size_t)b * a.NC + min(c0 + k, chunks - 1)) * H + hd;
+                            const float* z = state_at(a.ws_state, u, i);
+                            l[k][i][0] = __ldcg(z);
+                            l[k][i][1] = __ldcg(z + kD);
+                            gm[k][i] = __ldcg(reinterpret_cast<const float2*>(a.ws_gamma + u * N + 2 * (pair0 + kOwnPairs * S + i)));
+                        }
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    if (c0 + k >= chunks) break;
+                    if (c0 + k == c) into_chunk();
+#pragma unroll
+                    for (int i = 0; i < kOwnPairs; i++)
+                        if (i < own_pairs) {
+                            const cplx gam = {gm[k][i].x, gm[k][i].y};
+                            const float nr = next_re(gam, sr[i], si[i], l[k][i][0]);
+                            si[i] = next_im(gam, sr[i], si[i], l[k][i][1]);
+                            sr[i] = nr;
+                        }
+                }
+            }
+            if (chunks > c) {
+#pragma unroll
+                for (int i = 0; i < kOwnPairs; i++)
+                    if (i < own_pairs) {
+                        float* to = a.final_state + (((size_t)b * H + hd) * N + 2 * (pair0 + kOwnPairs * S + i)) * kD + col;
+                        to[0] = sr[i];
+                        to[kD] = si[i];
+                    }
+            } else {
+                into_chunk();
+            }
+        } else {
+            into_chunk();
         }
         __syncthreads();
     }
@@ -1446,11 +1501,11 @@ size_t scan_tile_extra_bytes(int B, int L, int H, int D, int N) {
 // scan_records.cu
 void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a, uint32_t** v, uint32_t** g);
 
-// mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the rounded carries from ws_state,
-// writes y), 2: both in one kernel with the carry handed on inside it (extra: scan_tile_extra_bytes() of scratch; it, ws_gamma,
+// mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the rounded carries from ws_state, with
+// from_chunks the local results of this call's local pass; writes y, with from_chunks the final state too), 2: both in one kernel with the carry handed on inside it (extra: scan_tile_extra_bytes() of scratch; it, ws_gamma,
 // ws_state and *ticket zeroed by the caller).
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
-int scan_tile_pass(int mode, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
+int scan_tile_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
                    float* final_state, float* tail_state, float* ws_gamma, float* ws_state, void* extra, int* status, int* ticket,
                    float shortcut_scale, int B, int L, int H, int D, int N, unsigned long long wait_ns, int withhold, cudaStream_t st) {
     using namespace tile;
@@ -1470,6 +1525,7 @@ int scan_tile_pass(int mode, const void* q, long long q_rs, const void* k, long 
     a.carries = static_cast<uint64_t*>(extra);
     a.wait_ns = wait_ns ? wait_ns : 400ull * 1000 * 1000;
     a.withhold = withhold;
+    a.from_chunks = from_chunks;
     a.shortcut_scale = shortcut_scale;
     a.B = B; a.L = L; a.H = H; a.N = N; a.NC = (L + D - 1) / D;
     a.groups = groups_of(D, N);

@@ -127,10 +127,12 @@ def test_tokens_before_a_bad_value_do_not_see_it(ops, orc, D, N, value, what):
     assert np.isfinite(to_np(y)[0, :t]).all()
 
 
-@pytest.mark.parametrize("B,H,NC,D,N", [(1, 3, 5, 64, 4), (2, 5, 3, 64, 16), (24, 8, 40, 64, 6), (1, 1, 29, 64, 16), (3, 2, 4, 128, 8), (2, 3, 2, 128, 16)])
-def test_scratch_without_room_for_the_carries_gives_the_same_bits(ops, orc, B, H, NC, D, N):
+@pytest.mark.parametrize("B,H,NC,D,N,few", [(1, 3, 5, 64, 4, 2), (2, 5, 3, 64, 16, 2), (24, 8, 40, 64, 6, 3), (1, 1, 29, 64, 16, 3), (3, 2, 4, 128, 8, 2),
+                                            (2, 3, 2, 128, 16, 2), (1, 2, 60, 64, 8, 3), (1, 1, 70, 128, 4, 3), (1, 3, 26, 64, 10, 2), (1, 5, 1, 64, 12, 2)])
+def test_scratch_without_room_for_the_carries_gives_the_same_bits(ops, orc, B, H, NC, D, N, few):
     """The whole-chunk scan hands the carry on inside one kernel where the scratch has room for the words that do it, else between
-    three: full and partly filled column tiles, an odd last head, two blocks a chunk, more chunks back than a warp asks for at once."""
+    two, with a carry pass in between where there are many chunks: full and partly filled column tiles, an odd last head, two blocks
+    a chunk, more chunks back than a warp asks for at once."""
     import ctypes
     import cdssm_b200
     lib = cdssm_b200._lib.lib()
@@ -149,7 +151,10 @@ def test_scratch_without_room_for_the_carries_gives_the_same_bits(ops, orc, B, H
                torch.full((B, H, N, D), 3.0, device="cuda")]
         args = [x.data_ptr() for x in t + out] + [ws.data_ptr() + (-ws.data_ptr()) % 256, room]
         args += [ctypes.c_float(c) for c in const_args(inp["consts"])] + [ctypes.c_float(0.25), B, L, H, D, N, D, 0, 0, 0]
+        before = lib.cdssm_b200_launch_count()
         assert lib.cdssm_b200_scan_fused_fwd(*args, torch.cuda.current_stream().cuda_stream) == 0
+        passes = lib.cdssm_b200_launch_count() - before - 1   # (behind the records)
+        assert passes == (1 if room == full else few)
         torch.cuda.synchronize()
         results.append(out)
     for a, b in zip(*results):
