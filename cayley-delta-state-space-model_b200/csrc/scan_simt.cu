@@ -908,28 +908,29 @@ static bool carry_in_output(int B, int NC, int H) { return (long long)B * NC * (
 static long long scan_tiles(int B, int H, int D) { return (long long)B * (D == 128 ? H : (H + 1) / 2); }
 
 // Whether the output pass of the whole-chunk scan, where it is not one kernel, adds the carry up itself: a read of NC x N rows by every
-// block, in parallel, against a launch and two more trips to memory.  us of a call on B200, carry pass / without, one sequence: 4 heads
-// of 64, N 4 9 chunks 18.1 / 15.3, 25 20.1 / 18.2, 40 21.1 / 22.7; N 16 2 chunks 26.0 / 20.2, 16 29.4 / 28.8, 25 30.9 / 34.8; 24 heads,
-// N 8 9 chunks 24.0 / 22.1, 16 28.1 / 29.3; N 16 9 31.0 / 31.9; 24 heads of 128, N 8 9 chunks 99.8 / 72.6, 25 84.7 / 89.8.
+// block, in parallel, against a launch and two more trips to memory.  us of a call on B200, carry pass / without, by tiles beside each
+// other, D 64: N 4, 2 tiles, 9 chunks 16.8 / 14.3, 25 18.4 / 17.0, 32 19.3 / 20.7; 12 tiles 9 18.5 / 17.9, 25 26.0 / 26.4; N 8, 2 tiles,
+// 16 chunks 20.5 / 19.3, 25 22.2 / 22.1; 12 tiles 9 21.7 / 21.0, 16 27.0 / 28.7; N 16, 1 tile, 2 chunks 23.5 / 19.5, 9 24.8 / 23.9, 16
+// 25.2 / 27.3; 12 tiles 9 27.5 / 29.1.  D 128, N 8, 4 tiles, 9 chunks 28.8 / 26.2, 25 32.2 / 35.4.
 static bool few_chunks(int B, int H, int NC, int D, int N) {
-    return NC <= 10 || (scan_tiles(B, H, D) * NC <= 64 && NC * N <= 260);
+    return NC * N <= 130 && NC <= (scan_tiles(B, H, D) <= 6 ? 20 : 10);
 }
 
 // Whether the whole-chunk scan (scan_tile.cu) hands the carry on inside one kernel, or runs as local pass, carry pass and output
 // pass: the same arithmetic in the same order, so this choice may go by size.  One kernel forms G once and reads k once, but its
 // blocks add up the chunks between theirs and the last finished one, as many as there are blocks on a sequence.  That is too much for
-// head_dim 64 (592 blocks at a time for N <= 4, else 296), when few tiles beside each other fill the GPU with long sequences.  Time of
-// one kernel over that of the passes on B200, at these numbers of chunks:
-//   N 4:  1 tile 256: 0.96, 400: 1.07, 1024: 1.5; 6 tiles 96: 0.84, 180: 1.0, 512: 1.2; 12 tiles 64: 0.95, 96: 1.0, 256: 1.2; 24 tiles
-//         44: 0.91, 64: 1.04, 256: 1.2; 48 tiles 32: 0.92, 60: 1.05; 96 tiles 128: 1.04; 192 tiles 128: 0.94
-//   N 8:  1 tile 180: 0.95, 1024: 1.2; 2 tiles and more 512: 0.92 to 0.97
-//   N 16: 1 tile 96: 0.8, 256: 1.03, 1024: 1.6; 2 tiles 180: 1.0, 512: 1.1; 4 tiles 256: 0.94, 1024: 1.03; 96 tiles 0.8
-// (head_dim 128: 0.65 to 1.0, up to 1.1 with N 16 beyond 200 chunks.)
+// head_dim 64 (592 blocks at a time for N <= 4, else 296) when few tiles beside each other fill the GPU with long sequences.  us of a
+// call on B200, one kernel / passes, by tiles beside each other:
+//   N 4:  1 tile, 64 chunks 21.3 / 22.8, 96 26.3 / 25.2, 512 112 / 75; 12 tiles 64 43.5 / 45.2, 96 59.3 / 58.5, 256 159 / 142; 48 tiles 64
+//         123 / 125, 128 245 / 236; 96 tiles 128 449 / 446; 192 tiles 64 361 / 439
+//   N 8:  1 tile, 96 chunks 29.8 / 29.5, 256 65 / 51; 2 tiles 96 34.8 / 35.9, 128 42 / 39, 512 121 / 124; 6 tiles 256 104 / 137
+//   N 16: 1 tile, 25 chunks 25.4 / 26.9, 45 32.1 / 29.9, 256 109 / 62; 4 tiles 25 27.8 / 28.4, 64 47.5 / 42.0, 512 255 / 256; 6 tiles 64 57 / 62,
+//         512 384 / 376; 12 tiles 256 337 / 338; 48 tiles 64 286 / 318
 static bool hands_carry_on(int B, int H, int NC, int D, int N) {
-    if (D == 128 || NC <= 45) return true;
+    if (D == 128) return true;
     const long long tiles = scan_tiles(B, H, D);
-    if (N > 4) return tiles > 2 || NC <= 180 * tiles;
-    return tiles >= 96 || (NC <= 300 && tiles * NC <= 1100);
+    if (N <= 4) return NC <= 90 || tiles >= 96;
+    return N <= 8 ? NC <= 110 || tiles >= 2 : NC <= 30 || tiles >= 5;
 }
 
 struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual
