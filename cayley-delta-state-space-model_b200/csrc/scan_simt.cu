@@ -848,6 +848,7 @@ int scan_wa_pass(bool output, const void* q, long long q_rs, const void* k, long
                  int from_chunks, const float* h0, float* final_state, int parts, cudaStream_t st);
 // scan_tile.cu
 bool scan_tile_supported(int D, int N, int C, int dtype);
+size_t scan_tile_words(int B, int L, int H, int D, int N);
 size_t scan_tile_extra_bytes(int B, int L, int H, int D, int N);
 int scan_tile_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
                    float* final_state, float* tail_state, float* ws_gamma, float* ws_state, void* extra, int* status, int* ticket,
@@ -1006,7 +1007,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     const size_t records = align256(scan_record_bytes(B, L, H, N, C));
     const bool one_kernel = tile_ok && tc_local && tc_output && a.run_local && !summary_only && hands_carry_on(B, H, a.NC, D, N) &&
                             workspace_bytes - base >= records + scan_tile_extra_bytes(B, L, H, D, N);
-    // Status word; for the one-kernel scan everything from there through the chunk states, and the carries: cleared by the records
+    // Status word; for the one-kernel scan everything from there through the chunks' words, and the carries: cleared by the records
     // kernel where that runs first.
     const bool tensor = wa_ok || tile_ok;
     const bool fill_records = tensor && (a.run_local || (flags & CDSSM_SCAN_TENSOR_CORE_WA));
@@ -1048,7 +1049,7 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     // (a summary of the same inputs has left the records in the workspace, in the order of the kernels that sizes alone choose)
     if (fill_records)
         if (int rc = scan_records(wa_ok, v, v_rs, rows.first, vf_rs, rows.mix, gate_raw, g_rs, log_dt_scale, rope_freqs, rec, status,
-                                  one_kernel ? ((char*)rec - (char*)status) / sizeof(int) : 1, static_cast<int*>(extra),
+                                  one_kernel ? 64 + scan_tile_words(B, L, H, D, N) : 1, static_cast<int*>(extra),
                                   one_kernel ? scan_tile_extra_bytes(B, L, H, D, N) / sizeof(int) : 0, a.dc, B, L, H, N, C, pos0, segs,
                                   a.fp32_decay, st))
             return rc;

@@ -1504,7 +1504,15 @@ static int tiles_of(int H, int D, int N) { return D == 128 ? H * groups_of(D, N)
 bool scan_tile_supported(int D, int N, int C, int dtype) {
     return dtype == CDSSM_BF16 && D == C && (D == 64 || D == 128) && N > 2 && N <= 16;
 }
-// Bytes of the carries that the one-kernel form hands on (beside the words in the places of the chunk decays and states).
+// Words of the chunks' gammas and states that the one-kernel form hands on, in the places of the chunk decays and states; the gammas
+// before the states (from a multiple of 64 words on).
+static size_t gamma_words(int B, int L, int H, int D, int N) {
+    return ((size_t)B * (((size_t)L + D - 1) / D) * H * (N / 2) + 63) & ~(size_t)63;
+}
+size_t scan_tile_words(int B, int L, int H, int D, int N) {
+    return gamma_words(B, L, H, D, N) + (size_t)B * (((size_t)L + D - 1) / D) * H * (N / 2) * D;
+}
+// Bytes of the carries that it hands on beside them.
 size_t scan_tile_extra_bytes(int B, int L, int H, int D, int N) {
     return (size_t)B * (((size_t)L + D - 1) / D) * H * (N / 2) * D * sizeof(uint64_t);
 }
@@ -1513,8 +1521,9 @@ size_t scan_tile_extra_bytes(int B, int L, int H, int D, int N) {
 void scan_record_arrays(void* rec, int B, int L, int H, int N, int C, float2** a, uint32_t** v, uint32_t** g);
 
 // mode 0: local pass (fills ws_gamma / ws_state for the carry pass), 1: output pass (reads the rounded carries from ws_state, with
-// from_chunks the local results of this call's local pass; writes y, with from_chunks the final state too), 2: both in one kernel with the carry handed on inside it (extra: scan_tile_extra_bytes() of scratch; it, ws_gamma,
-// ws_state and *ticket zeroed by the caller).
+// from_chunks the local results of this call's local pass; writes y, with from_chunks the final state too), 2: both in one kernel
+// with the carry handed on inside it (extra: scan_tile_extra_bytes() of scratch; it, scan_tile_words() words from ws_gamma on and
+// *ticket zeroed by the caller).
 // status: one int in device memory, set by a bounded wait that ran out (not cleared here).
 int scan_tile_pass(int mode, int from_chunks, const void* q, long long q_rs, const void* k, long long k_rs, void* rec, const float* h0, void* y,
                    float* final_state, float* tail_state, float* ws_gamma, float* ws_state, void* extra, int* status, int* ticket,
@@ -1532,7 +1541,7 @@ int scan_tile_pass(int mode, int from_chunks, const void* q, long long q_rs, con
     a.final_state = final_state; a.tail_state = mode == 0 ? nullptr : tail_state;
     a.ws_gamma = ws_gamma; a.ws_state = ws_state; a.status = status; a.ticket = ticket;
     a.gammas = reinterpret_cast<uint32_t*>(ws_gamma);
-    a.chunks = reinterpret_cast<uint32_t*>(ws_state);
+    a.chunks = a.gammas + gamma_words(B, L, H, D, N);
     a.carries = static_cast<uint64_t*>(extra);
     a.wait_ns = wait_ns ? wait_ns : 400ull * 1000 * 1000;
     a.withhold = withhold;

@@ -156,6 +156,11 @@ def test_scratch_without_room_for_the_carries_gives_the_same_bits(ops, orc, B, H
         passes = lib.cdssm_b200_launch_count() - before - 1   # (behind the records)
         assert passes == (1 if room == full else few)
         torch.cuda.synchronize()
+        # (one kernel: a word per gamma and per column of a state, where the passes keep two floats; nothing else is cleared)
+        units, up = B * NC * H * (N // 2), lambda n: -(-n // 256) * 256
+        at = (-ws.data_ptr()) % 256 + 256
+        unused = ws[at + up(4 * units) + 4 * units * D:at + up(8 * units) + up(8 * units * D)]
+        assert room < full or bool((unused == 0xa5).all())
         results.append(out)
     for a, b in zip(*results):
         assert torch.equal(a, b)
