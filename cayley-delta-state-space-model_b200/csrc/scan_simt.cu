@@ -875,10 +875,30 @@ static size_t least_workspace_bytes(int B, int L, int H, int D, int N, int C) {
     return bytes;
 }
 
+// Tiles of the whole-chunk scan beside each other: a head (head_dim 128) or two (64) of a sequence.
+static long long scan_tiles(int B, int H, int D) { return (long long)B * (D == 128 ? H : (H + 1) / 2); }
+
+// Whether the whole-chunk scan (scan_tile.cu) hands the carry on inside one kernel, or runs as local pass, carry pass and output
+// pass: the same arithmetic in the same order, so this choice may go by size.  One kernel forms G once and reads k once, but its
+// blocks add up the chunks between theirs and the last finished one, as many as there are blocks on a sequence.  That is too much for
+// head_dim 64 (592 blocks at a time for N <= 4, else 296) when few tiles beside each other fill the GPU with long sequences.  us of a
+// call on B200, one kernel / passes, by tiles beside each other:
+//   N 4:  1 tile, 64 chunks 21.3 / 22.8, 96 26.3 / 25.2, 512 112 / 75; 12 tiles 64 43.5 / 45.2, 96 59.3 / 58.5, 256 159 / 142; 48 tiles 64
+//         123 / 125, 128 245 / 236; 96 tiles 128 449 / 446; 192 tiles 64 361 / 439
+//   N 8:  1 tile, 96 chunks 29.8 / 29.5, 256 65 / 51; 2 tiles 96 34.8 / 35.9, 128 42 / 39, 512 121 / 124; 6 tiles 256 104 / 137
+//   N 16: 1 tile, 25 chunks 25.4 / 26.9, 45 32.1 / 29.9, 256 109 / 62; 4 tiles 25 27.8 / 28.4, 64 47.5 / 42.0, 512 255 / 256; 6 tiles 64 57 / 62,
+//         512 384 / 376; 12 tiles 256 337 / 338; 48 tiles 64 286 / 318
+static bool hands_carry_on(int B, int H, int NC, int D, int N) {
+    if (D == 128) return true;
+    const long long tiles = scan_tiles(B, H, D);
+    if (N <= 4) return NC <= 90 || tiles >= 96;
+    return N <= 8 ? NC <= 110 || tiles >= 2 : NC <= 30 || tiles >= 5;
+}
+
 extern "C" size_t cdssm_b200_scan_fused_workspace_bytes(int B, int L, int H, int D, int N, int C) {
     if (B <= 0 || L <= 0 || H <= 0 || D <= 0 || N <= 0 || (N & 1) || C <= 0) return 0;
     size_t bytes = least_workspace_bytes(B, L, H, D, N, C);
-    if (scan_tile_supported(D, N, C, CDSSM_BF16)) bytes += scan_tile_extra_bytes(B, L, H, D, N);
+    if (scan_tile_supported(D, N, C, CDSSM_BF16) && hands_carry_on(B, H, (L + C - 1) / C, D, N)) bytes += scan_tile_extra_bytes(B, L, H, D, N);
     return bytes;
 }
 // With room for the CUDA-core walks' records where those kernels run: a tenth faster (8 bytes more per token-head and 8 per pair
@@ -905,9 +925,6 @@ extern "C" int cdssm_b200_scan_fused_status(const void* workspace, int* status_h
 // 24.4 / 21.5, 3072 42 / 44; D 128, 528 32.3 / 30.5, 1536 61 / 63.
 static bool carry_in_output(int B, int NC, int H) { return (long long)B * NC * ((H + 3) / 4) <= 296 && NC <= 40; }
 
-// Tiles of the whole-chunk scan beside each other: a head (head_dim 128) or two (64) of a sequence.
-static long long scan_tiles(int B, int H, int D) { return (long long)B * (D == 128 ? H : (H + 1) / 2); }
-
 // Whether the output pass of the whole-chunk scan, where it is not one kernel, adds the carry up itself: a read of NC x N rows by every
 // block, in parallel, against a launch and two more trips to memory.  us of a call on B200, carry pass / without, by tiles beside each
 // other, D 64: N 4, 2 tiles, 9 chunks 16.8 / 14.3, 25 18.4 / 17.0, 32 19.3 / 20.7; 12 tiles 9 18.5 / 17.9, 25 26.0 / 26.4; N 8, 2 tiles,
@@ -915,23 +932,6 @@ static long long scan_tiles(int B, int H, int D) { return (long long)B * (D == 1
 // 25.2 / 27.3; 12 tiles 9 27.5 / 29.1.  D 128, N 8, 4 tiles, 9 chunks 28.8 / 26.2, 25 32.2 / 35.4.
 static bool few_chunks(int B, int H, int NC, int D, int N) {
     return NC * N <= 130 && NC <= (scan_tiles(B, H, D) <= 6 ? 20 : 10);
-}
-
-// Whether the whole-chunk scan (scan_tile.cu) hands the carry on inside one kernel, or runs as local pass, carry pass and output
-// pass: the same arithmetic in the same order, so this choice may go by size.  One kernel forms G once and reads k once, but its
-// blocks add up the chunks between theirs and the last finished one, as many as there are blocks on a sequence.  That is too much for
-// head_dim 64 (592 blocks at a time for N <= 4, else 296) when few tiles beside each other fill the GPU with long sequences.  us of a
-// call on B200, one kernel / passes, by tiles beside each other:
-//   N 4:  1 tile, 64 chunks 21.3 / 22.8, 96 26.3 / 25.2, 512 112 / 75; 12 tiles 64 43.5 / 45.2, 96 59.3 / 58.5, 256 159 / 142; 48 tiles 64
-//         123 / 125, 128 245 / 236; 96 tiles 128 449 / 446; 192 tiles 64 361 / 439
-//   N 8:  1 tile, 96 chunks 29.8 / 29.5, 256 65 / 51; 2 tiles 96 34.8 / 35.9, 128 42 / 39, 512 121 / 124; 6 tiles 256 104 / 137
-//   N 16: 1 tile, 25 chunks 25.4 / 26.9, 45 32.1 / 29.9, 256 109 / 62; 4 tiles 25 27.8 / 28.4, 64 47.5 / 42.0, 512 255 / 256; 6 tiles 64 57 / 62,
-//         512 384 / 376; 12 tiles 256 337 / 338; 48 tiles 64 286 / 318
-static bool hands_carry_on(int B, int H, int NC, int D, int N) {
-    if (D == 128) return true;
-    const long long tiles = scan_tiles(B, H, D);
-    if (N <= 4) return NC <= 90 || tiles >= 96;
-    return N <= 8 ? NC <= 110 || tiles >= 2 : NC <= 30 || tiles >= 5;
 }
 
 struct ScanRows {   // elements between (batch, token) rows, 0: dense; and the value residual

@@ -54,6 +54,11 @@ def test_argument_validation_needs_no_gpu(lib):
     assert more(16, 65536, 32, 128, 2, 128, 0, 0) == ws(16, 65536, 32, 128, 2, 128)
     assert more(2, 512, 4, 64, 2, 64, 1, 0) == states(2, 512, 4, 64, 2, 64) + 2 * 512 * 4 * 24
     assert more(2, 512, 4, 64, 2, 64, 0, 1) == more(2, 512, 4, 64, 2, 64, 1, 0)
+    # ... and where those hand the carry on inside one kernel, 8 bytes per chunk, pair and column (not where they run in passes)
+    records = lambda B, L, H, D, N: -(-B * -(-L // D) * H * D * (6 * N + 4) // 256) * 256
+    for B, L, H, D, N, handed_on in [(8, 2048, 24, 64, 16, 1), (1, 523, 3, 64, 4, 1), (2, 5000, 5, 128, 6, 1), (1, 65536, 12, 64, 4, 0), (1, 4000, 2, 64, 16, 0)]:
+        carries = handed_on * B * -(-L // D) * H * N // 2 * D * 8
+        assert ws(B, L, H, D, N, D) == states(B, L, H, D, N, D) + records(B, L, H, D, N) + carries
     # null pointers and bad sizes are refused before anything touches CUDA
     null = ctypes.c_void_p(0)
     assert h.cdssm_b200_normalize_kq_fwd(null, null, null, null, 4, 64, 0, null) == -1
