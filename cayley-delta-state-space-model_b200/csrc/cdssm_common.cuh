@@ -42,6 +42,13 @@ inline int launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t
     return counted(check_cuda(cudaLaunchKernelEx(&cfg, kernel, P(args)...)));
 }
 
+// Multiprocessors of the current device.
+inline int sm_count(int& sms) {
+    int dev = 0;
+    if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;
+    return check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+}
+
 // Opts a kernel in to `bytes` of dynamic shared memory, once per kernel (Tag) and device.
 template <typename Tag>
 inline int allow_smem(const void* kernel, size_t bytes) {

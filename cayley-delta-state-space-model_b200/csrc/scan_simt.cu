@@ -204,7 +204,7 @@ scan_walk_kernel(const ScanArgs a) {
     RowSlice<T, kCols> kraw, qraw;
     constexpr int kPieces = kCols * (int)sizeof(T) / 16, kRows = kOutput ? 2 : 1;   // 16-byte pieces of a lane's slice; rows a token
     uint4* ring = reinterpret_cast<uint4*>(smem + 6 * kUnits * C) + threadIdx.x;
-    auto piece = [&](int t, int row, int p) { return ring + (((t % kRing) * kRows + row) * kPieces + p) * kSimtThreads; };
+    auto piece = [&](int t, int row, int p) { return ring + (((t % (kRing > 0 ? kRing : 1)) * kRows + row) * kPieces + p) * kSimtThreads; };
     auto fetch = [&](int t) {
         const int row = min(t, Lc - 1);
 #pragma unroll
@@ -569,8 +569,8 @@ scan_carry_kernel(const ScanArgs a) {
 // waits and want the shared memory.  us of a call on B200, next row in registers / ring of eight: float32, D 64, 64 units 49.3 / 45.8,
 // 768 52.4 / 49.7, 1536 57.0 / 50.0, 6144 98 / 129; D 128, 1024 units 154 / 135, 4096 236 / 291; bf16, D 64, 240 units 52.5 / 46.9,
 // 3072 69.3 / 65.8, 6144 92.3 / 93.6.
-static bool walk_with_ring(const ScanArgs& a, int cols, int es, unsigned blocks) {
-    return blocks <= 148 && a.D == cols * kLanesPerUnit && a.C <= a.D && ((a.k_rs | a.q_rs) * es) % 16 == 0;
+static bool walk_with_ring(const ScanArgs& a, int cols, int es, unsigned blocks, int sms) {
+    return blocks <= (unsigned)sms && a.D == cols * kLanesPerUnit && a.C <= a.D && ((a.k_rs | a.q_rs) * es) % 16 == 0;
 }
 
 template <typename T, int kCols, bool kOutput, int kRing> struct WalkTag {};
@@ -593,7 +593,9 @@ static int launch_simt(const ScanArgs& a, cudaStream_t st) {
     constexpr int kUnits = kUnitsPerBlock, kRing = 8;
     const unsigned blocks = (unsigned)((a.units + kUnits - 1) / kUnits);
     const bool output = a.y != nullptr && a.run_output;   // else: summary only, or y comes from another kernel
-    const bool ring = walk_with_ring(a, kCols, (int)sizeof(T), blocks);
+    int sms = 0;
+    if (int rc = sm_count(sms)) return rc;
+    const bool ring = walk_with_ring(a, kCols, (int)sizeof(T), blocks, sms);
     if (a.rec_av != nullptr && (a.run_local || output)) {
         // pairs over the grid as far as one wave goes (what the pairs of a token share is computed again for each)
         const long long wave = ((long long)a.B * a.L + 31) / 32 * ((a.H + 7) / 8);
