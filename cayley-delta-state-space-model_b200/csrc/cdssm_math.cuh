@@ -153,7 +153,8 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
     __nv_bfloat162 p = __hadd2_rn(as_bf16x2(a), as_bf16x2(b));
     return *reinterpret_cast<uint32_t*>(&p);
 }
-// x / (1 + 2^(-x log2 e)); what the approximations flush to zero is nothing beside one, or below every quotient that is kept.
+// x / (1 + 2^(-x log2 e)).  What the exponential flushes to zero is nothing beside one; the reciprocal flushes below x = -87.3, where the
+// result (-1e-36 and nearer to zero) becomes zero, as it did with __fdividef.
 __device__ __forceinline__ float2 silu2(float2 x) {
     const float2 t = __fmul2_rn(x, make_float2(-1.44269504f, -1.44269504f));
     float2 e, r;

@@ -33,8 +33,9 @@
 //
 // Bounded by issue slots (45 % of them busy at 16 warps per SM) and by the chain of barriers and products through a chunk.  us of a
 // whole call on B200, before (a block per chunk and head, Gram blocks and three bf16 parts on the warp-level mma, carry behind a
-// fence and a flag) / now: D 64, B 8, L 2048, H 24, N 16 281 / 246, N 8 176 / 166, N 4 129 / 117; one sequence of 523, N 16
-// 33.6 / 30.1, N 4 20 / 15.7; D 128, 4 x 2048, H 32, N 8 241 / 164, 4 x 4096, H 12, N 4 147 / 93.
+// fence and a flag) / now: D 64, B 8, L 2048, H 24, N 16 291 / 245, N 8 171 / 157, N 4 136 / 121; one sequence of 523, N 16
+// 36.7 / 32.5, N 4 22.8 / 20.6; D 128, 4 x 2048, H 12, N 4 76 / 51, 2 x 1000, H 32, N 8 73 / 53, 4000 tokens, H 12, N 16 144 / 81.
+// One or two chunks of D 64, N 8, gain nothing: 2 x 41 tokens, H 16 11.5 / 12.9.
 //
 // Reference semantics (intra_chunk_scan.cu:100-195, exact_correction.cu:89-150): z starts at zero at the chunk start, r
 // from the bf16-rounded carry, the correction is read before its step.
@@ -60,7 +61,7 @@ struct Args {
     float *final_state, *tail_state;
     float* ws_gamma;             // (B,NC,H,NP,2): chunk decays (kLocal)
     float* ws_state;             // (B,NC,H,NP,2,D): z_{C-1} (kLocal), rounded carry into the chunk (kOutput)
-    uint32_t *gammas, *chunks;   // (B,NC,H,NP) gamma, (B,NC,H,NP,D) z of a chunk: words (scan_common.cuh) of bf16 pairs
+    uint32_t *gammas, *chunks;   // (B,NC,H,NP) gamma, (B,NC,H,NP,D) z of a chunk: words (put_word32()) of bf16 pairs
     uint64_t* carries;           // (B,NC,H,NP,D): carry out of a chunk (kFused: all three zeroed by the records kernel)
     int *status, *ticket;
     unsigned long long wait_ns;  // limit of every device-side wait
@@ -260,7 +261,7 @@ struct Scratch {   // of one 32-token block, until the Q tile arrives in its pla
     float nrm[32];
 };
 
-// (head_dim 128 with one pair: 75.0 KB, three blocks per SM)
+// (resident blocks per SM: kMinBlocks below)
 template <int kD, int kPairs, Mode kMode>
 struct __align__(1024) Smem {
     using G = Geo<kD, kPairs>;
@@ -462,8 +463,8 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         if (tid == 0) atomicCAS(a.status, 0, 399);
         return;
     }
-    // The records kernel clears the ticket counter.  Where all blocks are resident together they need no tickets, and start on
-    // their tiles while it is still at work (8 layers of 2 x 41 tokens, N 8: 404 us with tickets, 376 without).
+    // The records kernel clears the ticket counter.  While there is a block per SM at most the blocks need no tickets (launch_one()),
+    // and start on their tiles while it is still at work (8 layers of 2 x 41 tokens, N 8: 404 us with tickets, 376 without).
     const bool early = kMode == kLocal || (kMode == kFused && a.fixed);
     if (kMode == kFused && !early) grid_dependency_wait();
     if (tid == 0) {
@@ -1476,10 +1477,12 @@ static int launch_one(const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, c
     if (int rc = allow_smem<KernelTag<kD, kPairs, kMode>>((const void*)scan_tile_kernel<kD, kPairs, kMode>, smem)) return rc;
     const long long items = (long long)a.B * a.NC * a.HG;
     if (items > 0x7fffffff) return CDSSM_ERR_UNSUPPORTED;
-    int dev = 0, sms = 0;
-    if (int rc = check_cuda(cudaGetDevice(&dev))) return rc;
-    if (int rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return rc;
-    a.fixed = items <= sms;      // (one block per SM, whatever else is resident there)
+    int sms = 0;
+    if (int rc = sm_count(sms)) return rc;
+    // Blocks wait for those with smaller numbers, which start first: blocks start in the order of their numbers.  No document says
+    // so, hence one block per SM at most: should other streams' kernels hold back an earlier one, the waiting blocks have at most one
+    // of two or more places of an SM, and a wait that lasts ends with the status word set.
+    a.fixed = items <= sms;
     return launch_overlapped(scan_tile_kernel<kD, kPairs, kMode>, dim3((unsigned)items), dim3(Geo<kD, kPairs>::kThreads), smem, st,
                              tmK, tmQ, a);
 }
