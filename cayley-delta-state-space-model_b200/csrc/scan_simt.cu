@@ -1,5 +1,5 @@
 // Fused CD-SSM scan on CUDA cores (the general path: any even N <= 32, D <= 128, C <= 256,
-// bf16 or fp32 storage).
+// bf16 or fp32 storage).  scan_short.cu has the same walk for few units of head_dim 64 and 128.
 //
 // Reference chunk semantics (cdssm/models/ssd.py:56-111 over intra_chunk_scan.cu:100-195,
 // inter_chunk_scan.cu:52-84, exact_correction.cu:89-150), per head and complex pair:
@@ -21,6 +21,7 @@
 // The dynamics of a chunk are computed once per unit into shared memory before the walk.
 #include "cdssm_common.cuh"
 #include "decode_unit.cuh"
+#include "scan_args.cuh"
 #include "sm100_ptx.cuh"
 #include <atomic>
 
@@ -29,30 +30,6 @@ namespace cdssm {
 constexpr int kUnitsPerBlock = 16;
 constexpr int kSimtThreads = kLanesPerUnit * kUnitsPerBlock;   // 128
 constexpr int kMaxChunk = 256;
-
-struct ScanArgs {
-    const void *q, *k, *v, *gate_raw;
-    const float *log_dt_scale, *rope_freqs, *h0;
-    void* y;
-    float *final_state, *tail_state;
-    float* total_decay;   // (B,H,N) or NULL: product over the chunks of the (rounded) chunk decays
-    int segs;             // batch rows are `segs` consecutive segments of longer sequences
-    int run_local;        // 0: the workspace already holds this input's local pass
-    int run_output;       // 0: stop after the carry pass (another kernel writes y)
-    int publish;          // 0: summary only, the carry pass leaves the local results in place
-    int fp32_decay;       // 1: the transition a_t keeps float32 precision (the reference stores it as bf16)
-    float4* rec_av;    // (B,NC,H,NP,C): transition and scaled v of a token, or NULL: the walk computes them itself
-    float2* rec_bs;    // (B,NC,H,C): beta and sel_C
-    float* ws_gamma;   // (B,NC,H,NP,2)
-    float* ws_state;   // (B,NC,H,NP,2,D): z_{C-1} after the local pass, s_c after the carry pass
-    DynConsts dc;
-    float shortcut_scale;
-    int B, L, H, D, N, C, NC, pos0;
-    // elements between the (batch, token) rows of q, k, v, gate_raw and v_first (column slices of wider projections)
-    long long q_rs, k_rs, v_rs, g_rs, vf_rs;
-    const void *v_first, *mix;   // or NULL: v <- lerp(v_first, v, mix[head])
-    long long units;   // B*NC*H*NP
-};
 
 // Shared-memory staging of one chunk's per-token scalars for the 16 units of a block.
 struct ChunkScalars {
@@ -64,51 +41,12 @@ struct ChunkScalars {
     }
 };
 
-// Dynamics of one (token, head): what its pairs share, then pair j (dynamics_fused.cu:64-139 and the vp scale of
-// block.py:194-195).
-template <typename T>
-struct TokenDynamics {
-    const T *gr, *vrow, *vfirst;
-    DynShared ds;
-    float freq, pos, mix;
-    int H, NH, fp32_decay;
-    __device__ __forceinline__ TokenDynamics(const ScanArgs& a, int b, int l, int hd) {
-        H = a.H; NH = a.N >> 1; fp32_decay = a.fp32_decay;
-        const long long bl = (long long)b * a.L + l;
-        gr = static_cast<const T*>(a.gate_raw) + bl * a.g_rs + hd;
-        vrow = static_cast<const T*>(a.v) + bl * a.v_rs + (long long)hd * a.N;
-        vfirst = a.v_first ? static_cast<const T*>(a.v_first) + bl * a.vf_rs + (long long)hd * a.N : nullptr;
-        mix = a.v_first ? IO<T>::ld(static_cast<const T*>(a.mix) + hd) : 0.f;
-        const T* s5 = gr + a.N * H;
-        freq = a.rope_freqs[hd];
-        pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
-        ds = dyn_shared<IO<T>::kBf16>(IO<T>::ld(gr), IO<T>::ld(gr + NH * H), IO<T>::ld(s5), IO<T>::ld(s5 + H),
-                                      IO<T>::ld(s5 + 2 * H), IO<T>::ld(s5 + 3 * H), IO<T>::ld(s5 + 4 * H),
-                                      a.log_dt_scale[hd], freq, pos, a.dc);
-    }
-    __device__ __forceinline__ float2 beta_sel() const { return make_float2(IO<T>::rnd(ds.beta), IO<T>::rnd(ds.sel_c)); }
-    __device__ __forceinline__ float4 pair(int j) const {
-        float ar, ai, vp;
-        dyn_pair<IO<T>::kBf16>(IO<T>::ld(gr + j * H), IO<T>::ld(gr + (NH + j) * H), freq, pos, ds, ar, ai, vp);
-        if (!fp32_decay) {
-            ar = IO<T>::rnd(ar);
-            ai = IO<T>::rnd(ai);
-        }
-        vp = IO<T>::rnd(vp);
-        float v0 = IO<T>::ld(vrow + 2 * j), v1 = IO<T>::ld(vrow + 2 * j + 1);
-        if (vfirst) {
-            v0 = value_residual<T>(IO<T>::ld(vfirst + 2 * j), v0, mix);
-            v1 = value_residual<T>(IO<T>::ld(vfirst + 2 * j + 1), v1, mix);
-        }
-        return make_float4(ar, ai, IO<T>::rnd(v0 * vp), IO<T>::rnd(v1 * vp));
-    }
-};
-
 // The dynamics of every (token, head) before the walks: a warp takes four tokens of eight heads.  Computed by the walks
 // themselves, eight tokens in a row per lane, they were 10 us (float32: 15) of each of the two walks whatever the size.
 template <typename T>
-__global__ void __launch_bounds__(256) simt_records_kernel(const ScanArgs a) {
+__global__ void __launch_bounds__(256) simt_records_kernel(const ScanArgs a, const bool early) {
     const int lt = threadIdx.x >> 3 & 3, lh = threadIdx.x & 7, warp = threadIdx.x >> 5;
+    if (early) grid_launch_dependents();
     const long long tok = (long long)blockIdx.x * 32 + warp * 4 + lt;
     const int hd = blockIdx.y * 8 + lh;
     if (tok >= (long long)a.B * a.L || hd >= a.H) return;
@@ -117,9 +55,9 @@ __global__ void __launch_bounds__(256) simt_records_kernel(const ScanArgs a) {
     const size_t unit = ((size_t)b * a.NC + c) * a.H + hd;
     a.rec_bs[unit * a.C + t] = d.beta_sel();
     for (int j = blockIdx.z; j < NH; j += gridDim.z) a.rec_av[(unit * NH + j) * a.C + t] = d.pair(j);
-    // (at the end: dependents that start while these blocks fill the SMs are packed onto the few with room, and a walk of
+    // (at the end where these blocks fill the SMs: dependents that start meanwhile are packed onto the few with room, and a walk of
     // 24 blocks of head_dim 128 took 104 us instead of 21)
-    grid_launch_dependents();
+    if (!early) grid_launch_dependents();
 }
 
 // Scalars of the unit's chunk into shared memory: lane g handles tokens g, g+8, ...  Padded positions (l >= L) get
@@ -595,19 +533,31 @@ static int launch_simt(const ScanArgs& a, cudaStream_t st) {
     const bool output = a.y != nullptr && a.run_output;   // else: summary only, or y comes from another kernel
     int sms = 0;
     if (int rc = sm_count(sms)) return rc;
+    constexpr int dtype = IO<T>::kBf16 ? CDSSM_BF16 : CDSSM_F32;
+    const bool short_walk = scan_short_takes(a, dtype, sms);
     const bool ring = walk_with_ring(a, kCols, (int)sizeof(T), blocks, sms);
     if (a.rec_av != nullptr && (a.run_local || output)) {
         // pairs over the grid as far as one wave goes (what the pairs of a token share is computed again for each)
         const long long wave = ((long long)a.B * a.L + 31) / 32 * ((a.H + 7) / 8);
         const int pairs = wave >= 1024 ? 1 : (int)min((long long)(a.N / 2), 1024 / wave);
-        simt_records_kernel<T><<<dim3((unsigned)(((long long)a.B * a.L + 31) / 32), (a.H + 7) / 8, pairs), 256, 0, st>>>(a);
+        const bool early = short_walk && wave * pairs <= sms;   // (the walk has rows to fetch and norms to form meanwhile)
+        simt_records_kernel<T><<<dim3((unsigned)(((long long)a.B * a.L + 31) / 32), (a.H + 7) / 8, pairs), 256, 0, st>>>(a, early);
         if (int rc = check_launch()) return rc;
     }
-    if (a.run_local)
-        if (int rc = ring ? launch_walk<T, kCols, false, kRing>(a, blocks, st) : launch_walk<T, kCols, false, 0>(a, blocks, st)) return rc;
-    const long long th = (long long)a.B * a.H * (a.N / 2) * a.D;
-    if (int rc = launch_overlapped(scan_carry_kernel<T>, dim3((unsigned)((th + 127) / 128)), dim3(128), 0, st, a)) return rc;
+    if (a.run_local) {
+        if (int rc = short_walk ? scan_short_pass(false, a, dtype, 0, st)
+                     : ring     ? launch_walk<T, kCols, false, kRing>(a, blocks, st)
+                                : launch_walk<T, kCols, false, 0>(a, blocks, st))
+            return rc;
+    }
+    // (the short walk adds a few chunks up itself, instead of a launch and two more trips to memory)
+    const bool from_chunks = short_walk && output && a.run_local && a.publish && !a.total_decay && a.NC <= 12;
+    if (!from_chunks) {
+        const long long th = (long long)a.B * a.H * (a.N / 2) * a.D;
+        if (int rc = launch_overlapped(scan_carry_kernel<T>, dim3((unsigned)((th + 127) / 128)), dim3(128), 0, st, a)) return rc;
+    }
     if (!output) return CDSSM_OK;
+    if (short_walk) return scan_short_pass(true, a, dtype, from_chunks, st);
     return ring ? launch_walk<T, kCols, true, kRing>(a, blocks, st) : launch_walk<T, kCols, true, 0>(a, blocks, st);
 }
 
