@@ -34,10 +34,19 @@ template <> struct IO<float> {
     static __device__ __forceinline__ float rnd(float x) { return x; }
 };
 
-template <bool kFast> __device__ __forceinline__ float exp_(float x) { return kFast ? __expf(x) : expf(x); }
-template <bool kFast> __device__ __forceinline__ float log_(float x) { return kFast ? __logf(x) : logf(x); }
-template <bool kFast> __device__ __forceinline__ float pow_(float x, float y) { return kFast ? __powf(x, y) : powf(x, y); }
-template <bool kFast> __device__ __forceinline__ float div_(float a, float b) { return kFast ? __fdividef(a, b) : a / b; }
+// kFast, from the special-function unit: e^x = 2^(x log2 e), ln x = ln 2 log2 x, x^y = 2^(y log2 x), a / b = a (1 / b).  The intrinsics
+// (__expf, __logf, __powf, __fdividef) give the same bits wherever neither an argument nor a result is subnormal, and take up to five
+// more instructions each for those: an exponential that small is added to one here, logarithms are of 1 + e^x or of at least
+// 1e-8, divisors are 1 + e^x or sums of positive terms.  (The power itself may be subnormal: no flush there.)
+__device__ __forceinline__ float sfu_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float sfu_exp2_sub(float x) { float r; asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float sfu_log2(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float sfu_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+
+template <bool kFast> __device__ __forceinline__ float exp_(float x) { return kFast ? sfu_exp2(__fmul_rn(x, 1.44269504f)) : expf(x); }
+template <bool kFast> __device__ __forceinline__ float log_(float x) { return kFast ? __fmul_rn(sfu_log2(x), 0.693147181f) : logf(x); }
+template <bool kFast> __device__ __forceinline__ float pow_(float x, float y) { return kFast ? sfu_exp2_sub(__fmul_rn(y, sfu_log2(x))) : powf(x, y); }
+template <bool kFast> __device__ __forceinline__ float div_(float a, float b) { return kFast ? __fmul_rn(a, sfu_rcp(b)) : a / b; }
 
 template <bool kFast> __device__ __forceinline__ float sigmoidf_(float x) {
     return div_<kFast>(1.0f, 1.0f + exp_<kFast>(-x));
@@ -53,6 +62,8 @@ struct DynConsts {
     float gating_c, omega_thresh, adt_delta, adt_smoothness, adt_eps;
 };
 
+// Which products and sums go together is said, not left to the compiler: kernels that form the dynamics on their own (records, walks,
+// one-token steps, the operator) and versions of one for other sizes have the same bits.
 // Per-(token, head) quantities shared by all complex pairs of the head.
 struct DynShared {
     float dt, cr, beta, sel_c;   // cr = gating_c * sigmoid(r_gate)
@@ -68,14 +79,14 @@ __device__ __forceinline__ DynShared dyn_shared(float alpha0_raw, float omega0_r
     DynShared o;
     float r_gate = sigmoidf_<kFast>(r_raw);
     float alpha0 = softplusf_<kFast>(alpha0_raw);
-    float w0 = fabsf(omega0_raw + pos * freq);
+    float w0 = fabsf(__fadd_rn(omega0_raw, __fmul_rn(pos, freq)));
     float dt_scale = softplusf_<kFast>(log_dt_scale);
     float dt_raw = div_<kFast>(dt_scale, alpha0 + w0 + c.adt_eps);
     float dt_max = div_<kFast>(2.0f - c.adt_delta, alpha0 + c.adt_eps);
     float blend = sigmoidf_<kFast>(div_<kFast>(c.omega_thresh - w0, c.adt_smoothness));
     float dt_cap = fminf(dt_raw, dt_max);
-    o.dt = blend * dt_cap + (1.0f - blend) * dt_raw + softplusf_<kFast>(sel_dt);
-    o.cr = c.gating_c * r_gate;
+    o.dt = __fadd_rn(__fmaf_rn(blend, dt_cap, __fmul_rn(1.0f - blend, dt_raw)), softplusf_<kFast>(sel_dt));
+    o.cr = __fmul_rn(c.gating_c, r_gate);
     o.beta = sigmoidf_<kFast>(beta_raw) * sigmoidf_<kFast>(sel_B);
     o.sel_c = sigmoidf_<kFast>(sel_C);
     return o;
@@ -88,20 +99,21 @@ template <bool kFast>
 __device__ __forceinline__ void dyn_pair(float alpha_raw, float omega_raw, float freq, float pos,
                                          const DynShared& s, float& a_re, float& a_im, float& vp) {
     float alpha = fmaxf(softplusf_<kFast>(alpha_raw), 0.0f);
-    float omega = omega_raw + pos * freq;
-    float tau = s.dt * 0.5f, ta = tau * alpha, tw = tau * omega;
-    float nr = 1.0f - ta, ni = tw, dr = 1.0f + ta, di = -tw;
-    float denom = __fmaf_rn(dr, dr, di * di) + kEps;
-    float inv_d = __fdiv_rn(1.0f, denom);
-    float mu_re = (nr * dr + ni * di) * inv_d;
-    float mu_im = (ni * dr - nr * di) * inv_d;
-    float numer = __fmaf_rn(1.0f - ta, 1.0f - ta, tw * tw);
-    float den2 = __fmaf_rn(1.0f + ta, 1.0f + ta, tw * tw);
+    float omega = __fadd_rn(omega_raw, __fmul_rn(pos, freq));
+    const float tau = s.dt * 0.5f, tw = __fmul_rn(tau, omega), tw2 = __fmul_rn(tw, tw);
+    const float nr = __fmaf_rn(-tau, alpha, 1.0f), dr = __fmaf_rn(tau, alpha, 1.0f);
+    const float ni = tw, di = -tw;
+    const float denom = __fadd_rn(__fmaf_rn(dr, dr, tw2), kEps);
+    float inv_d = __frcp_rn(denom);
+    const float mu_re = __fmul_rn(__fmaf_rn(nr, dr, __fmul_rn(ni, di)), inv_d);
+    const float mu_im = __fmul_rn(__fmaf_rn(ni, dr, -__fmul_rn(nr, di)), inv_d);
+    const float numer = __fmaf_rn(nr, nr, tw2);
+    const float den2 = __fmaf_rn(dr, dr, tw2);
     float eig = fmaxf(div_<kFast>(numer, den2 + kEps), 1e-8f);
-    float scale = pow_<kFast>(eig, (s.cr - 1.0f) / 2.0f);
+    float scale = pow_<kFast>(eig, __fadd_rn(s.cr, -1.0f) * 0.5f);
     a_re = mu_re * scale;
     a_im = -mu_im * scale;
-    float eff = pow_<kFast>(eig, s.cr);
+    float eff = kFast ? sfu_exp2(__fmul_rn(s.cr, sfu_log2(eig))) : powf(eig, s.cr);   // (nothing beside one where it is flushed)
     vp = fminf(sqrtf(fmaxf(1.0f - eff, kEps)), 1.0f);
 }
 

@@ -5,6 +5,8 @@
 // the gates with the heads across the lanes, and turns its results around in shared memory, so that both sides move whole
 // sectors; a thread has the loads of all its values in flight before the first transcendental.  Bounded by issue slots and the
 // special-function unit (a pair takes some hundred instructions, nine of them special functions).
+// Instructions a pair at N 16: 209 -> 160 without divisions by what is known before and without the special functions' ways for subnormal
+// numbers (cdssm_math.cuh), 31.7 -> 26.3 us cold; N 2 328 -> 287 a token-head.
 // Measured on B200: 393 216 token-heads, N 16: 58 -> 27 us against one pair at a time with two barriers each; N 2, 7.7 -> 7.5,
 // and 2.1 M token-heads 27 -> 26 us against a thread per token-head that wrote its 16-byte record straight to memory.
 #include "cdssm_common.cuh"
@@ -27,13 +29,19 @@ struct Args {
     size_t clear_words, clear2_words;
     DynConsts dc;
     int B, L, H, N, C, NC, pos0, segs, fp32_decay, tiles;   // tiles: 32-token tiles per batch row, chunks padded to full length
+    uint32_t tiles_inv;            // 2^32 / tiles, rounded up (at least two tiles): a division is twenty instructions of every thread
 };
 
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+// (Resident blocks that the registers are cut for.  Left to itself the compiler takes 32 registers for one or two pairs and has loads wait
+// for each other: 3 x 777 tokens of 24 heads, N 2, 27.3 us a scan, so 26.5; 12 layers of a 16-token-a-head draw 660, 622.)
+template <int kNP, int kHg, bool kResidual>
+constexpr int kMinBlocks = kHg == 16 ? 2 : kNP <= 2 ? 5 : kNP == 8 && kResidual ? 3 : 4;
+
 // kNP: pairs per thread, from kNP * blockIdx.z on; kHg: heads per block.
 template <int kNP, int kHg, bool kWa, bool kResidual>
-__global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
+__global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual>) records_kernel(const Args a) {
     using T = __nv_bfloat16;
     constexpr int kItems = kTokens * kHg / kThreads, kRow = kTokens + 1;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -44,14 +52,20 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     grid_dependency_wait();
     const size_t first = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x, step = (size_t)gridDim.x * gridDim.y * kThreads;
     if (kWa) {   // a few words
+#pragma unroll 1
         for (size_t i = first; i < a.clear_words; i += step) a.clear[i] = 0;
     } else if (blockIdx.z == 0) {
+#pragma unroll 1
         for (size_t i = first; i < a.clear_words / 4; i += step) reinterpret_cast<uint4*>(a.clear)[i] = make_uint4(0u, 0u, 0u, 0u);
         if (first < a.clear_words % 4) a.clear[a.clear_words / 4 * 4 + first] = 0;
+#pragma unroll 1
         for (size_t i = first; i < a.clear2_words / 4; i += step) reinterpret_cast<uint4*>(a.clear2)[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     const int H = a.H, N = a.N, NP = N >> 1, p0 = kWa ? 0 : kNP * (int)blockIdx.z, pairs = min(kNP, NP - p0);
-    const int b = (int)(blockIdx.x / (unsigned)a.tiles), tile = (int)(blockIdx.x - (unsigned)b * a.tiles), l0 = tile * kTokens;
+    uint32_t row_of = __umulhi(blockIdx.x, a.tiles_inv);   // (the quotient, or one more)
+    if (row_of * (uint32_t)a.tiles > blockIdx.x) row_of--;
+    const int b = (int)row_of, tile = (int)(blockIdx.x - row_of * (uint32_t)a.tiles), l0 = tile * kTokens;
+    const int before = a.pos0 + (a.segs > 1 ? (b % a.segs) * a.L : 0);   // position of the row's first token
     const int head0 = blockIdx.y * kHg, heads = min(kHg, H - head0);
     const int head = threadIdx.x & (kHg - 1), hd = head0 + min(head, heads - 1);
     const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
@@ -85,7 +99,7 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     for (int i = 0; i < kItems; i++) {
         const int t = (int)(threadIdx.x / kHg) + i * (kThreads / kHg), l = l0 + t;
         const bool on = l < a.L;                                       // behind the end a = 1, beta = v = 0: the state stands still
-        const float pos = (float)(l + a.pos0 + (b % a.segs) * a.L);
+        const float pos = (float)(l + before);
         auto f = [](T y) { return __bfloat162float(y); };
         const DynShared ds = dyn_shared<true>(f(x[i][5]), f(x[i][6]), f(x[i][0]), f(x[i][1]), f(x[i][2]), f(x[i][3]), f(x[i][4]),
                                               lds, freq, pos, a.dc);
@@ -117,17 +131,35 @@ __global__ void __launch_bounds__(kThreads) records_kernel(const Args a) {
     grid_launch_dependents();   // (not earlier: blocks that start while these fill the SMs are packed onto the few with room)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (kWa) {
+#pragma unroll 1
         for (int h = warp; h < heads; h += kThreads / 32)
             a.rec[(((size_t)b * a.tiles + tile) * H + head0 + h) * kTokens + lane] = sr[h * kRow + lane];
     } else {
-        const int c = l0 / a.C, in_chunk = l0 - c * a.C;
+        const int c = l0 >> (a.C == 64 ? 6 : 7), in_chunk = l0 & (a.C - 1);
         const size_t unit0 = ((size_t)b * a.NC + c) * H + head0;
-        for (int i = warp; i < heads * pairs; i += kThreads / 32) {
-            const int h = i / pairs, p = i - h * pairs, s = (p * kHg + h) * kRow + lane;
-            const size_t o = ((unit0 + h) * NP + p0 + p) * a.C + in_chunk + lane;
-            a.rec_a[o] = sa[s];
-            a.rec_v[o] = sv[s];
+        if constexpr (kNP >= 4) {   // a warp has a head and its pairs: no division an item
+#pragma unroll 1
+            for (int h = warp; h < heads; h += kThreads / 32) {
+                const size_t o = ((unit0 + h) * NP + p0) * a.C + in_chunk + lane;
+                const float2* fa = sa + h * kRow + lane;
+                const uint32_t* fv = sv + h * kRow + lane;
+#pragma unroll
+                for (int p = 0; p < kNP; p++) {
+                    if (p >= pairs) break;
+                    a.rec_a[o + p * a.C] = fa[p * kHg * kRow];
+                    a.rec_v[o + p * a.C] = fv[p * kHg * kRow];
+                }
+            }
+        } else {                    // (12 layers of a 523-token prompt, two pairs a thread: 796 us, 823 in the other order)
+#pragma unroll 1
+            for (int i = warp; i < heads * pairs; i += kThreads / 32) {
+                const int h = i / pairs, p = i - h * pairs, s = (p * kHg + h) * kRow + lane;
+                const size_t o = ((unit0 + h) * NP + p0 + p) * a.C + in_chunk + lane;
+                a.rec_a[o] = sa[s];
+                a.rec_v[o] = sv[s];
+            }
         }
+#pragma unroll 1
         for (int h = warp; h < heads && p0 == 0; h += kThreads / 32) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sg[h * kRow + lane];
     }
 }
@@ -184,6 +216,7 @@ int scan_records(bool wa, const void* v, long long v_rs, const void* v_first, lo
     a.dc = dc;
     a.B = B; a.L = L; a.H = H; a.N = N; a.C = C; a.NC = (L + C - 1) / C; a.pos0 = pos0; a.segs = segs; a.fp32_decay = fp32_decay;
     a.tiles = a.NC * (C / kTokens);
+    a.tiles_inv = (uint32_t)(((1ull << 32) + a.tiles - 1) / a.tiles);
     if ((long long)B * a.tiles > 0x7fffffff || H > 8 * 65535) return CDSSM_ERR_UNSUPPORTED;
     if (wa) return launch_group<1, true>(a, st);
     if (N <= 2) return launch_group<1, false>(a, st);
