@@ -77,7 +77,10 @@ struct Args {
 #define kNotANumber __int_as_float(0x7fffffff)
 
 struct cplx { float r, i; };
-__device__ __forceinline__ cplx cmul(cplx a, cplx b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
+// (Which products and sums go together is said here and below, not left to the compiler: the versions of the kernel have the same bits.)
+__device__ __forceinline__ cplx cmul(cplx a, cplx b) {
+    return {__fmaf_rn(a.r, b.r, -__fmul_rn(a.i, b.i)), __fmaf_rn(a.r, b.i, __fmul_rn(a.i, b.r))};
+}
 __device__ __forceinline__ cplx cshfl(cplx v, int src) {
     return {__shfl_sync(0xffffffffu, v.r, src), __shfl_sync(0xffffffffu, v.i, src)};
 }
@@ -128,7 +131,7 @@ __device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, 
         const float m = fmaxf(fabsf(E.r), fabsf(E.i));
         const float sc1 = reciprocal(m);
         const cplx En = {E.r * sc1, E.i * sc1};
-        const float q = sc1 * reciprocal(En.r * En.r + En.i * En.i);
+        const float q = sc1 * reciprocal(__fmaf_rn(En.r, En.r, __fmul_rn(En.i, En.i)));
         const cplx Einv = {En.r * q, -En.i * q};
         const cplx D = lo ? Einv : E, v = cmul(vg[w], lo ? E : Einv);
         const bool in_range = m >= 1e-30f && m <= 1e30f && fabsf(v.r) <= 1e33f && fabsf(v.i) <= 1e33f;   // (false for NaN)
@@ -230,14 +233,16 @@ __device__ __forceinline__ void mma_split(float (&d)[4], float (&e)[4], const Sp
     mma_tf32<kFirst>(e, s.lo[0], s.lo[1], s.lo[2], s.lo[3], b);
 }
 
-template <int kD, int kPairs_>
+// kWide: a warp per column tile of a 32-token block, for calls that have an SM per tile: half the chain, half the code
+template <int kD, int kPairs_, bool kWide = false>
 struct Geo {
     static constexpr int kPairs = kPairs_;               // complex pairs held (>= N / 2)
     static constexpr int kComps = 2 * kPairs;
     static constexpr int kHeads = 128 / kD;              // of a tile
     static constexpr int kBlocks = kD / 32;              // 32-token blocks of a chunk
     static constexpr int kTiles = (kPairs + 1) / 2;      // column tiles of two pairs
-    static constexpr int kSplit = kPairs >= 8 || (kD == 64 && kPairs >= 4) ? 2 : 1;   // warps that share the column tiles of a 32-token block
+    static constexpr int kNarrow = kPairs >= 8 || (kD == 64 && kPairs >= 4) ? 2 : 1;
+    static constexpr int kSplit = kWide ? kTiles : kNarrow;   // warps that share the column tiles of a 32-token block
     static constexpr int kThreads = 128 * kSplit;
     static constexpr int kOwn = kTiles / kSplit, kOwnPairs = kPairs / kSplit;   // of a warp
     static constexpr int kSlabs = kD / 64, kKs = kD / 16;
@@ -262,9 +267,9 @@ struct Scratch {   // of one 32-token block, until the Q tile arrives in its pla
 };
 
 // (resident blocks per SM: kMinBlocks below)
-template <int kD, int kPairs, Mode kMode>
+template <int kD, int kPairs, Mode kMode, bool kWide>
 struct __align__(1024) Smem {
-    using G = Geo<kD, kPairs>;
+    using G = Geo<kD, kPairs, kWide>;
     uint8_t k[G::kTile];                                 // swizzled rows = tokens
     union {
         uint8_t q[kMode == kLocal ? 1024 : G::kTile];
@@ -319,9 +324,9 @@ __device__ __forceinline__ void diagonal_of(const float* n0, const float* n1, in
 // hold: state columns over the lanes.  First without read-out (walk[t].x = |k_t|^-1 in; out walk[t] = {g_t carried to the block
 // end}, and g_t in place of v_t), later with it (walk[t] = {q_t.z_t, W_{t-1} from the block start}; no sums on the way of the
 // state any more).  The incoming state is rebuilt from what the earlier blocks published.
-template <int kD, int kPairs, Mode kMode, bool kReadout>
-__device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int row0, int I, int W, int tl) {
-    using G = Geo<kD, kPairs>;
+template <int kD, int kPairs, Mode kMode, bool kWide, bool kReadout>
+__device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode, kWide>& sm, int p, int row0, int I, int W, int tl) {
+    using G = Geo<kD, kPairs, kWide>;
     constexpr int kCols = kD / 32;
     auto column = [&](const uint8_t* tile, int row, int c) {
         const int piece = (c & 63) >> 3;
@@ -419,9 +424,9 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode>& sm, int p, int r
 // products of a block it would reach the tokens before it too (0 x NaN), so its row is emptied and the outputs from it on are set
 // apart at the end.  A finite row whose square overflows has |k|^-1 = 0: it neither erases nor adds.  Returns whether this
 // lane's row is emptied.
-template <int kD, int kPairs, Mode kMode>
-__device__ __noinline__ bool empty_bad_rows(Smem<kD, kPairs, kMode>& sm, int row, int head) {
-    using G = Geo<kD, kPairs>;
+template <int kD, int kPairs, Mode kMode, bool kWide>
+__device__ __noinline__ bool empty_bad_rows(Smem<kD, kPairs, kMode, kWide>& sm, int row, int head) {
+    using G = Geo<kD, kPairs, kWide>;
     bool number = fabsf(bits_lo(sm.bs[row])) <= 3e38f;
     float ss = 0.f;
     for (int c = 0; c < kD; c++) {
@@ -441,18 +446,50 @@ __device__ __noinline__ bool empty_bad_rows(Smem<kD, kPairs, kMode>& sm, int row
     return empty;
 }
 
-// resident blocks per SM the registers are cut for
-template <int kD, int kPairs>
-constexpr int kMinBlocks = kPairs >= 4 || kD == 128 ? 2 : 4;
+// A block runs most of its code once, 100 to 200 KB of straight line, more than an SM's instruction cache: a warp of a call with a block per
+// SM spent 44 % of its stalls on waiting for instructions, of a full GPU 13 %.  So what comes at several places, or seldom, is a function
+// or a loop: with that and kWide, us before / now: D 64, 523 tokens, H 24, N 16 32.0 / 29.8; B 8, L 2048, H 24, N 4 120 / 112, N 16 245 / 229;
+// D 128, 1000 tokens, H 12, N 8 24.5 / 21.4; 12 layers of a 523-token prompt 801 / 750.  (Not faster: the records' loads as a function with a
+// loop, or one turn of the look-back for carries and states alike.)
+__device__ __noinline__ bool wait_longer(uint64_t* bar, uint32_t parity, int* abort_flag, unsigned long long limit) {
+    return mbar_wait_suspend(bar, parity, abort_flag, limit);
+}
 
-template <int kD, int kPairs, Mode kMode>
-__global__ void __launch_bounds__(Geo<kD, kPairs>::kThreads, kMinBlocks<kD, kPairs>)
-scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const Args a) {
-    using G = Geo<kD, kPairs>;
+// A block that gives up stays until its own copies and products have landed (or a limit has passed again): the next one has
+// its memory then.  (g_issued, p_issued: warp 0's)
+template <typename Smem>
+__device__ __noinline__ void leave(Smem& sm, const Args& a, int code, bool q_loaded, int g_issued, bool p_issued, uint32_t tmem) {
+    const int W = threadIdx.x >> 5;
+    cp_async_wait_all();
+    if (W == 0) {
+        if ((threadIdx.x & 31) == 0) {
+            atomicCAS(a.status, 0, code);
+            int never = 0;
+            if (!a.withhold) mbar_wait_ns(&sm.full_k, 0, &never, a.wait_ns);
+            if (q_loaded && !a.withhold) mbar_wait_ns(&sm.full_q, 0, &never, a.wait_ns);
+            if (g_issued) mbar_wait_ns(&sm.mma_g, g_issued - 1, &never, a.wait_ns);
+            if (p_issued) mbar_wait_ns(&sm.mma_p, 0, &never, a.wait_ns);
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (W == 0) tmem_dealloc(tmem, 128);
+}
+
+// resident blocks per SM the registers are cut for
+template <int kD, int kPairs, bool kWide = false>
+constexpr int kMinBlocks = kWide ? 1 : kPairs >= 4 || kD == 128 ? 2 : 4;
+
+template <int kD, int kPairs, Mode kMode, bool kWide>
+__global__ void __launch_bounds__(Geo<kD, kPairs, kWide>::kThreads, kMinBlocks<kD, kPairs, kWide>)
+scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ Args a) {
+    using G = Geo<kD, kPairs, kWide>;
     constexpr int kBlocks = G::kBlocks, kKs = G::kKs, kSplit = G::kSplit, kOwn = G::kOwn, kOwnPairs = G::kOwnPairs;
     constexpr bool kOut = kMode != kLocal, kNeedEnd = kMode != kOutput;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    Smem<kD, kPairs, kMode>& sm = *reinterpret_cast<Smem<kD, kPairs, kMode>*>(smem_raw);
+    using S_ = Smem<kD, kPairs, kMode, kWide>;
+    S_& sm = *reinterpret_cast<S_*>(smem_raw);
     // warp W: 32-token block W4 of the tile, column tiles S * kOwn ... (the warps of a block meet at the tiles and the inverses only)
     const int tid = threadIdx.x, W = tid >> 5, W4 = W & 3, S = W >> 2, tl = tid & 31, g = tl >> 2, t4 = tl & 3;
     const int hs = W4 / kBlocks, I = W4 % kBlocks, row0 = hs * kD;   // head of the tile, block of the chunk, the chunk's first row
@@ -499,10 +536,11 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     };
     if (tid == 0 && !a.withhold) load_tile(sm.k, &tmK, &sm.full_k);
     // the token's dynamics, parked where the results will go (padding: identity)
-    // (two warps: fewer pairs beside the inverses)
+    // (two warps: fewer pairs beside the inverses; four: none)
     const bool first_warp = kSplit == 1 || S == 0;
-    constexpr int kFirstPairs = kSplit == 1 ? kPairs : kPairs == 4 ? 1 : 3;
-    const int p_lo = first_warp ? 0 : kFirstPairs, p_hi = first_warp ? kFirstPairs : kPairs;
+    constexpr int kFirstPairs = kSplit == 1 ? kPairs : kSplit == 4 ? 0 : kPairs == 4 ? 1 : 3;
+    constexpr int kOtherPairs = kSplit == 4 ? 3 : kPairs - kFirstPairs;
+    const int p_lo = first_warp ? 0 : kFirstPairs + (S - 1) * kOtherPairs, p_hi = first_warp ? kFirstPairs : min(kPairs, p_lo + kOtherPairs);
     auto load_records = [&]() {
         const size_t t = (size_t)(tok - row0);
         if (first_warp) {
@@ -546,29 +584,11 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         umma_commit_elect(bar);
     };
     auto wait = [&](uint64_t* bar, uint32_t parity) {
-        return __all_sync(0xffffffffu, mbar_wait_suspend(bar, parity, &sm.abort_flag, a.wait_ns));
+        return __all_sync(0xffffffffu, mbar_try_wait_nohint(bar, parity) || wait_longer(bar, parity, &sm.abort_flag, a.wait_ns));
     };
-    // A block that gives up stays until its own copies and products have landed (or a limit has passed again): the next one has
-    // its memory then.
     int g_issued = 0;                          // (warp 0) products G: a second one where key rows have been emptied
     bool p_issued = false;
-    auto give_up = [&](int code, bool q_loaded) {
-        cp_async_wait_all();
-        if (W == 0) {
-            if (tl == 0) {
-                atomicCAS(a.status, 0, code);
-                int never = 0;
-                if (!a.withhold) mbar_wait_ns(&sm.full_k, 0, &never, a.wait_ns);
-                if (q_loaded && !a.withhold) mbar_wait_ns(&sm.full_q, 0, &never, a.wait_ns);
-                if (g_issued) mbar_wait_ns(&sm.mma_g, g_issued - 1, &never, a.wait_ns);
-                if (p_issued) mbar_wait_ns(&sm.mma_p, 0, &never, a.wait_ns);
-            }
-            __syncwarp();
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (W == 0) tmem_dealloc(tmem, 128);
-    };
+    auto give_up = [&](int code, bool q_loaded) { leave(sm, a, code, q_loaded, g_issued, p_issued, tmem); };
 
     bool ok = wait(&sm.full_k, 0);
     if (W == 0 && ok) { gram(kt, &sm.mma_g); g_issued = 1; }
@@ -585,23 +605,31 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             BlockPair bp[kW];
 #pragma unroll
             for (int w = 0; w < kW; w++) {
-                const float2 x = sm.dd[p0 + w][tok];
-                const uint32_t y = __float_as_uint(sm.viw[p0 + w][tok].x);
+                const int p = min(p0 + w, p_hi - 1);   // (a warp's last three may be two: it forms one twice)
+                const float2 x = sm.dd[p][tok];
+                const uint32_t y = __float_as_uint(sm.viw[p][tok].x);
                 at[w] = {x.x, x.y};
                 vg[w] = {bits_lo(y), bits_hi(y)};
             }
-            const int slow = scalings<kW>(at, vg, tl, bp) << p0;
+            const int slow = (scalings<kW>(at, vg, tl, bp) << p0) & ((1 << p_hi) - 1);
 #pragma unroll
             for (int w = 0; w < kW; w++) {
+                if (p0 + w >= p_hi) break;
                 sm.viw[p0 + w][tok] = make_float2(vg[w].r, vg[w].i);
                 sm.dd[p0 + w][tok] = make_float2(at[w].r, at[w].i);
                 if (tl == 0) sm.bp[p0 + w][W4] = bp[w];
             }
             return slow;
         };
-        int slow;
-        if constexpr (kSplit == 1) slow = some(std::integral_constant<int, kPairs>(), 0);
-        else slow = first_warp ? some(std::integral_constant<int, kFirstPairs>(), 0) : some(std::integral_constant<int, kPairs - kFirstPairs>(), kFirstPairs);
+        int slow = 0;
+        if constexpr (kSplit == 1) {
+            slow = some(std::integral_constant<int, kPairs>(), 0);
+        } else if constexpr (kPairs == 8) {    // (three at a time, whoever has how many)
+#pragma unroll 1
+            for (int p0 = p_lo; p0 < p_hi; p0 += 3) slow |= some(std::integral_constant<int, 3>(), p0);
+        } else {
+            slow = first_warp ? some(std::integral_constant<int, kFirstPairs>(), 0) : some(std::integral_constant<int, kOtherPairs>(), kFirstPairs);
+        }
         if (tl == 0) sm.slow[S][W4] = slow;
         __syncwarp();
     }
@@ -623,7 +651,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll
         for (int r = 0; r < 4; r++) number = number && kk[r] <= 3.4e38f;
         if (ok && !__all_sync(0xffffffffu, number)) {   // (not from tensor memory that nothing has been written to)
-            const uint32_t bad = __ballot_sync(0xffffffffu, empty_bad_rows<kD, kPairs, kMode>(sm, tok, hs));
+            const uint32_t bad = __ballot_sync(0xffffffffu, empty_bad_rows<kD, kPairs, kMode, kWide>(sm, tok, hs));
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -791,12 +819,12 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     auto sum_lo = [](const float (&d)[4], const float (&e)[4]) { return (d[0] + d[1]) + (e[0] + e[1]); };
     auto sum_hi = [](const float (&d)[4], const float (&e)[4]) { return (d[2] + d[3]) + (e[2] + e[3]); };
     // complex factor times the lane's component; `other` is the other component of the same value
-    auto rotate = [&](cplx f, float own, float other) { return f.r * own + (comp ? f.i : -f.i) * other; };
+    auto rotate = [&](cplx f, float own, float other) { return __fmaf_rn(f.r, own, __fmul_rn(comp ? f.i : -f.i, other)); };
     auto other_of = [](float x) { return __shfl_xor_sync(0xffffffffu, x, 1); };
     // block J's scaled sum times D31, then times f (behind()), this lane's component
     auto carried = [&](cplx d31, cplx f, float own) {
         const float other = other_of(own), i = comp ? d31.i : -d31.i;
-        return rotate(f, d31.r * own + i * other, d31.r * other - i * own);
+        return rotate(f, __fmaf_rn(d31.r, own, __fmul_rn(i, other)), __fmaf_rn(d31.r, other, -__fmul_rn(i, own)));
     };
 
     // x <- (I + M_own)^-1 x, all column tiles; published as vector v
@@ -846,7 +874,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     auto times = [&](const float (&x)[2][16], auto kVectors, int v, int J, float* out) {
         constexpr int kV = decltype(kVectors)::value;
         // (accumulators of their own for the lo parts where there are few chains of products beside each other)
-        constexpr bool kApart = kV * kOwn < 4;
+        constexpr bool kApart = kV * (G::kTiles / G::kNarrow) < 4;   // (the same sums, and so the same bits, however many warps share the tiles)
         float d[kV][kOwn][2][4], e[kApart ? kV : 1][kOwn][2][4];
 #pragma unroll
         for (int n = 0; n < 4; n++) {
@@ -901,7 +929,10 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         __syncwarp();
     };
 
-    const int slow = (sm.slow[0][W4] | sm.slow[kSplit - 1][W4]) & (((1 << kOwnPairs) - 1) << (kOwnPairs * S));   // of this warp's pairs
+    int slow = 0;                              // of this warp's pairs
+#pragma unroll
+    for (int i = 0; i < kSplit; i++) slow |= sm.slow[i][W4];
+    slow &= ((1 << kOwnPairs) - 1) << (kOwnPairs * S);
     // ---- g: the chain over the blocks of the chunk
     float gx[kOwn][4];
     {
@@ -910,7 +941,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const float2 e = sm.viw[pair_of(q)][base + 8 * r + g];
-                gx[q][r] = bn[r] * (comp ? e.y : e.x);
+                gx[q][r] = __fmul_rn(bn[r], comp ? e.y : e.x);
             }
 #pragma unroll
         for (int J = 0; J < kEarlier; J++)
@@ -923,7 +954,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                     const BlockPair* bp = &sm.bp[pair_of(q)][row0 / 32];
                     const cplx D31 = bp[J].D31, F = behind(bp, J, I, kBlocks);
 #pragma unroll
-                    for (int r = 0; r < 4; r++) gx[q][r] -= cc[r] * carried(D31, F, s[q][r]);
+                    for (int r = 0; r < 4; r++) gx[q][r] = __fmaf_rn(-cc[r], carried(D31, F, s[q][r]), gx[q][r]);
                 }
             }
         solve(kG, gx);
@@ -939,7 +970,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll 1
                 for (int s = 0; s < 2; s++)
                     if ((slow >> (2 * tile(q) + s)) & 1) {
-                        slow_walk<kD, kPairs, kMode, false>(sm, 2 * tile(q) + s, row0, I, W, tl);
+                        slow_walk<kD, kPairs, kMode, kWide, false>(sm, 2 * tile(q) + s, row0, I, W, tl);
                         if ((t4 >> 1) == s) {
 #pragma unroll
                             for (int r = 0; r < 4; r++) {
@@ -1302,7 +1333,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll
         for (int q = 0; q < kOwn; q++)
 #pragma unroll
-            for (int r = 0; r < 4; r++) hx[q][r] *= cc[r];
+            for (int r = 0; r < 4; r++) hx[q][r] = __fmul_rn(hx[q][r], cc[r]);
 #pragma unroll
         for (int J = 0; J < kEarlier; J++)
             if (J < I) {
@@ -1312,7 +1343,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll
                 for (int q = 0; q < kOwn; q++)
 #pragma unroll
-                    for (int r = 0; r < 4; r++) hx[q][r] -= cc[r] * s[q][r];
+                    for (int r = 0; r < 4; r++) hx[q][r] = __fmaf_rn(-cc[r], s[q][r], hx[q][r]);
             }
         solve(kH, hx);
         chain_pass();
@@ -1379,7 +1410,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int row = base + 8 * r + g;
-            const float x = oz[q][r] + pd[r] * gx[q][r], xo = other_of(x), ho = other_of(rho[q][r]);
+            const float x = __fmaf_rn(pd[r], gx[q][r], oz[q][r]), xo = other_of(x), ho = other_of(rho[q][r]);
             const float2 D = sm.dd[p][row], D0 = sm.dd[p][row > 0 ? row - 1 : 0];
             const bool first = r == 0 && g == 0;
             const cplx w0 = first ? pre : cmul({D0.x, D0.y}, F);
@@ -1393,7 +1424,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             for (int s = 0; s < 2; s++)
                 if ((slow >> (2 * tile(q) + s)) & 1) {
                     const cplx pre = decay_before(2 * tile(q) + s);
-                    slow_walk<kD, kPairs, kMode, true>(sm, 2 * tile(q) + s, row0, I, W, tl);
+                    slow_walk<kD, kPairs, kMode, kWide, true>(sm, 2 * tile(q) + s, row0, I, W, tl);
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
                         const float ho = other_of(rho[q][r]);
@@ -1410,7 +1441,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int row = base + 8 * r + g;
-            float yy = row - row0 >= sm.first_bad[hs] ? kNotANumber : mq[r] * oz[q][r];
+            float yy = row - row0 >= sm.first_bad[hs] ? kNotANumber : __fmul_rn(mq[r], oz[q][r]);
             if (a.shortcut_scale != 0.f) {   // block.py:202-208; v after the vp scale
                 const float qk = mq[r] * nrm[r] * pd[r];
                 const float2 e = sm.viw[p][row], D = sm.dd[p][row];
@@ -1419,7 +1450,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                     const uint32_t w = __ldcg(a.rec_v + (unit * (size_t)NP + pair0 + p) * kD + row - row0);
                     vg = {bits_lo(w), bits_hi(w)};
                 }
-                yy += a.shortcut_scale * qk * qk * bfr(comp ? vg.i : vg.r);
+                yy = __fmaf_rn(a.shortcut_scale * qk * qk, bfr(comp ? vg.i : vg.r), yy);
             }
             sm.y(row)[2 * p + comp] = __float2bfloat16_rn(bfr(yy) * bits_hi(sm.bs[row]));
         }
@@ -1467,14 +1498,19 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
-template <int kD, int kPairs, Mode kMode> struct KernelTag {};
+template <int kD, int kPairs, Mode kMode, bool kWide> struct KernelTag {};
 
-template <int kD, int kPairs, Mode kMode>
-static int launch_one(const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, cudaStream_t st) {
-    const size_t smem = sizeof(Smem<kD, kPairs, kMode>);
-    static_assert(sizeof(Smem<kD, kPairs, kMode>) <= (227 * 1024 + 1024) / kMinBlocks<kD, kPairs> - 1024, "shared memory");
-    static_assert(kMinBlocks<kD, kPairs> <= 4, "tensor memory: 128 columns a block");
-    if (int rc = allow_smem<KernelTag<kD, kPairs, kMode>>((const void*)scan_tile_kernel<kD, kPairs, kMode>, smem)) return rc;
+template <int kD, int kPairs, Mode kMode, bool kWide = false>
+static int launch_one(const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, long long items, cudaStream_t st) {
+    const size_t smem = sizeof(Smem<kD, kPairs, kMode, kWide>);
+    static_assert(sizeof(Smem<kD, kPairs, kMode, kWide>) <= (227 * 1024 + 1024) / kMinBlocks<kD, kPairs, kWide> - 1024, "shared memory");
+    static_assert(kMinBlocks<kD, kPairs, kWide> <= 4, "tensor memory: 128 columns a block");
+    if (int rc = allow_smem<KernelTag<kD, kPairs, kMode, kWide>>((const void*)scan_tile_kernel<kD, kPairs, kMode, kWide>, smem)) return rc;
+    return launch_overlapped(scan_tile_kernel<kD, kPairs, kMode, kWide>, dim3((unsigned)items), dim3(Geo<kD, kPairs, kWide>::kThreads), smem, st,
+                             tmK, tmQ, a);
+}
+template <int kD, int kPairs>
+static int launch_mode(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, cudaStream_t st) {
     const long long items = (long long)a.B * a.NC * a.HG;
     if (items > 0x7fffffff) return CDSSM_ERR_UNSUPPORTED;
     int sms = 0;
@@ -1483,14 +1519,11 @@ static int launch_one(const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, c
     // so, hence one block per SM at most: should other streams' kernels hold back an earlier one, the waiting blocks have at most one
     // of two or more places of an SM, and a wait that lasts ends with the status word set.
     a.fixed = items <= sms;
-    return launch_overlapped(scan_tile_kernel<kD, kPairs, kMode>, dim3((unsigned)items), dim3(Geo<kD, kPairs>::kThreads), smem, st,
-                             tmK, tmQ, a);
-}
-template <int kD, int kPairs>
-static int launch_mode(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, cudaStream_t st) {
-    if (m == kLocal) return launch_one<kD, kPairs, kLocal>(tmK, tmQ, a, st);
-    if (m == kOutput) return launch_one<kD, kPairs, kOutput>(tmK, tmQ, a, st);
-    return launch_one<kD, kPairs, kFused>(tmK, tmQ, a, st);
+    if (m == kLocal) return launch_one<kD, kPairs, kLocal>(tmK, tmQ, a, items, st);
+    if (m == kOutput) return launch_one<kD, kPairs, kOutput>(tmK, tmQ, a, items, st);
+    if constexpr (Geo<kD, kPairs>::kOwn > 1)
+        if (a.fixed) return launch_one<kD, kPairs, kFused, true>(tmK, tmQ, a, items, st);
+    return launch_one<kD, kPairs, kFused>(tmK, tmQ, a, items, st);
 }
 template <int kD>
 static int launch_pairs(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, Args& a, cudaStream_t st) {
