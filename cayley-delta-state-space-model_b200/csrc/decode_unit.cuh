@@ -37,22 +37,32 @@ struct DecodeUnitArgs {
 };
 
 // Unit u of this thread's group of eight lanes; the whole warp calls together (units past the end take part in the
-// shuffles and write nothing).
-template <typename T, int kCols>
-__device__ __forceinline__ void decode_unit(const DecodeUnitArgs& a, long long u) {
+// shuffles and write nothing).  ready() comes before the first read of q and the gates: state, k and v are on their way by then.
+// A step of a few units is a chain of trips to memory and of the dynamics' special functions: places in 32 bits (four divisions in 64
+// took longer than a trip to the L2 cache).
+template <typename T, int kCols, typename Ready>
+__device__ __forceinline__ void decode_unit(const DecodeUnitArgs& a, long long u, Ready ready) {
     const int g = threadIdx.x % kLanesPerUnit;
     const bool active = u < a.units;
     if (!active) u = a.units - 1;
     const int NH = a.N >> 1, D = a.D, H = a.H;
-    const int j = (int)(u % NH);
-    const int hd = (int)((u / NH) % H);
-    const long long b = u / ((long long)NH * H);
+    int j, hd;
+    long long b;
+    if (a.units <= 0xffffffffll) {
+        const unsigned n = (unsigned)u / (unsigned)NH, m = n / (unsigned)H;
+        j = (int)((unsigned)u - n * (unsigned)NH);
+        hd = (int)(n - m * (unsigned)H);
+        b = m;
+    } else {
+        j = (int)(u % NH);
+        hd = (int)((u / NH) % H);
+        b = u / ((long long)NH * H);
+    }
     const bool vec = (D == kCols * kLanesPerUnit);
     const long long bh = b * H + hd;
 
     RowSlice<T, kCols> kraw, qraw;
     kraw.load(static_cast<const T*>(a.k) + b * a.k_stride + (long long)hd * D, g, D, vec);
-    qraw.load(static_cast<const T*>(a.q) + b * a.q_stride + (long long)hd * D, g, D, vec);
     float* st = a.state + (bh * a.N + 2 * j) * D;
     float zr[kCols], zi[kCols];
     if (vec) {
@@ -71,27 +81,33 @@ __device__ __forceinline__ void decode_unit(const DecodeUnitArgs& a, long long u
             zi[i] = d < D ? st[D + d] : 0.f;
         }
     }
+    const T* vrow = static_cast<const T*>(a.v) + b * a.v_stride + (long long)hd * a.N + 2 * j;
+    float v0 = IO<T>::ld(vrow), v1 = IO<T>::ld(vrow + 1), f0 = 0.f, f1 = 0.f, mix = 0.f;
+    if (a.v_first) {
+        const T* f = static_cast<const T*>(a.v_first) + b * a.v_first_stride + (long long)hd * a.N + 2 * j;
+        mix = IO<T>::ld(static_cast<const T*>(a.mix) + hd);
+        f0 = IO<T>::ld(f);
+        f1 = IO<T>::ld(f + 1);
+    }
+    const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd], pos = (float)a.pos;
+    ready();
+    qraw.load(static_cast<const T*>(a.q) + b * a.q_stride + (long long)hd * D, g, D, vec);
     // dynamics (every lane of the unit computes the same scalars; dynamics_fused.cu:64-139)
     const T* gr = static_cast<const T*>(a.gate) + b * a.gate_stride;
     const T* s5 = gr + a.N * H;
-    const float freq = a.rope_freqs[hd], pos = (float)a.pos;
     DynShared ds = dyn_shared<IO<T>::kBf16>(IO<T>::ld(gr + hd), IO<T>::ld(gr + NH * H + hd), IO<T>::ld(s5 + hd),
                               IO<T>::ld(s5 + H + hd), IO<T>::ld(s5 + 2 * H + hd),
                               IO<T>::ld(s5 + 3 * H + hd), IO<T>::ld(s5 + 4 * H + hd),
-                              a.log_dt_scale[hd], freq, pos, a.dc);
+                              lds, freq, pos, a.dc);
     float a_re, a_im, vp;
     dyn_pair<IO<T>::kBf16>(IO<T>::ld(gr + j * H + hd), IO<T>::ld(gr + (NH + j) * H + hd), freq, pos, ds, a_re, a_im, vp);
     a_re = IO<T>::rnd(a_re);
     a_im = IO<T>::rnd(a_im);
     vp = IO<T>::rnd(vp);
     const float be = IO<T>::rnd(ds.beta), sc = IO<T>::rnd(ds.sel_c);
-    const T* vrow = static_cast<const T*>(a.v) + b * a.v_stride + (long long)hd * a.N + 2 * j;
-    float v0 = IO<T>::ld(vrow), v1 = IO<T>::ld(vrow + 1);
     if (a.v_first) {
-        const T* f = static_cast<const T*>(a.v_first) + b * a.v_first_stride + (long long)hd * a.N + 2 * j;
-        const float w = IO<T>::ld(static_cast<const T*>(a.mix) + hd), f0 = IO<T>::ld(f), f1 = IO<T>::ld(f + 1);
-        v0 = value_residual<T>(f0, v0, w);
-        v1 = value_residual<T>(f1, v1, w);
+        v0 = value_residual<T>(f0, v0, mix);
+        v1 = value_residual<T>(f1, v1, mix);
     }
     const float vr = IO<T>::rnd(v0 * vp), vi = IO<T>::rnd(v1 * vp);
 

@@ -74,6 +74,7 @@ struct Product {
     const bf16* x;            // (B, x_stride)
     long long x_stride;
     int M, K;
+    int apart;                // the partial sums have shared memory of their own, beside the activations
 };
 
 // Weight rows of work item `item` to registers: rows g and g + 8 of the warp's fragment, columns 8 t .. 8 t + 7 of the
@@ -106,10 +107,18 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
     const int pitch = x_pitch(p.K), kblocks = (p.K + 31) / 32;
     const int mine = warp < MT * KW ? (kblocks - kp + KW - 1) / KW : 0;
     const int tiles = (p.M + kRows - 1) / kRows, btiles = (a.B + NT * 8 - 1) / (NT * 8), items = tiles * btiles;
-    float* red = reinterpret_cast<float*>(smem + (kMode == kHead ? (size_t)NT * 8 * pitch : 0));
+    float* red = reinterpret_cast<float*>(smem + (kMode == kHead || p.apart ? (size_t)NT * 8 * pitch : 0));
     uint4 wr[kAhead][2];
     if (kMode == kInProj && a.first) grid_dependency_wait();
     if ((int)blockIdx.x < items) fetch_first<MT>(p, (int)blockIdx.x % tiles, wr);
+    constexpr int kNormAhead = 3;   // 256-column pieces of the norm's weights that are there before the activations are
+    uint4 nwr[kNormAhead];
+    const bf16* nw = kMode == kHead ? a.final_norm_w : (const bf16*)w.norm_w;
+    if (kNorm) {
+#pragma unroll
+        for (int i = 0; i < kNormAhead; i++)
+            if (lane * 8 + 256 * i < p.K) nwr[i] = __ldg(reinterpret_cast<const uint4*>(nw + lane * 8 + 256 * i));
+    }
     request_ahead(a);
     bool waited = false;
     int staged = -1;      // batch tile whose activations are in shared memory
@@ -189,7 +198,6 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
             sm100::cp_async_wait_all();
             __syncwarp();
             if (kNorm) {
-                const bf16* nw = kMode == kHead ? a.final_norm_w : (const bf16*)w.norm_w;
                 const float eps = kMode == kHead ? a.eps_final : a.eps_norm;
                 for (int b = warp; b < nb; b += kWarps) {
                     bf16* xs = reinterpret_cast<bf16*>(smem + (size_t)b * pitch);
@@ -201,14 +209,18 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
                         for (int e = 0; e < 8; e++) ss += f[e] * f[e];
                     }
                     const float rms = rsqrtf(warp_sum(ss) / (float)p.K + eps);
-                    for (int c = lane * 8; c < p.K; c += 256) {
+                    auto scale = [&](int c, const uint4& weights) {
                         float f[8], n[8];
                         Vec8<bf16>::ld(xs + c, f);
-                        unpack8(__ldg(reinterpret_cast<const uint4*>(nw + c)), n);
+                        unpack8(weights, n);
 #pragma unroll
                         for (int e = 0; e < 8; e++) f[e] = IO<bf16>::rnd(f[e] * rms) * n[e];
                         Vec8<bf16>::st(xs + c, f);
-                    }
+                    };
+#pragma unroll
+                    for (int i = 0; i < kNormAhead; i++)
+                        if (lane * 8 + 256 * i < p.K) scale(lane * 8 + 256 * i, nwr[i]);
+                    for (int c = lane * 8 + 256 * kNormAhead; c < p.K; c += 256) scale(c, __ldg(reinterpret_cast<const uint4*>(nw + c)));
                 }
             }
             staged = b0;
@@ -239,7 +251,7 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
         }
         if (kMode == kHead && item + (int)gridDim.x < items)   // the next item's weights travel during the epilogue
             fetch_first<MT>(p, (item + gridDim.x) % tiles, wr);
-        if (kMode != kHead) __syncthreads();   // the sums take the place of the activations
+        if (kMode != kHead && !p.apart) __syncthreads();   // the sums take the place of the activations
         if (warp < MT * KW) {
             float* mr = red + (size_t)kp * NT * 8 * kRP;
 #pragma unroll
@@ -312,8 +324,7 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
 // The recurrent step of a layer: eight lanes per (sequence, head, pair).
 __global__ void __launch_bounds__(128) lm_step_kernel(const Args a, const cdssm_lm_layer w) {
     request_ahead(a);
-    grid_dependency_wait();
-    grid_launch_dependents();
+    // (the state is the step's before, k and v are two kernels back: the one before this has waited for both)
     DecodeUnitArgs u;
     u.state = (float*)w.state;
     u.q = a.qg; u.q_stride = a.qg_stride;
@@ -329,21 +340,26 @@ __global__ void __launch_bounds__(128) lm_step_kernel(const Args a, const cdssm_
     u.H = a.H; u.D = 64; u.N = a.N;
     u.pos = a.pos_dev ? *a.pos_dev : a.pos;
     u.units = (long long)a.B * a.H * (a.N / 2);
-    decode_unit<bf16, 8>(u, (long long)blockIdx.x * 16 + threadIdx.x / 8);
+    decode_unit<bf16, 8>(u, (long long)blockIdx.x * 16 + threadIdx.x / 8, [] {
+        grid_dependency_wait();
+        grid_launch_dependents();
+    });
 }
 
 template <int NT, int MT, bool kHeadMode>
-static size_t smem_bytes(int K) {
+static size_t smem_bytes(int K, bool apart = false) {
     const size_t xs = (size_t)NT * 8 * x_pitch(K), red = sizeof(float) * NT * 8 * (kWarps / MT) * (16 * MT + 4);
-    return kHeadMode ? xs + red : (xs > red ? xs : red);
+    return kHeadMode || apart ? xs + red : (xs > red ? xs : red);
 }
 
 template <int NT, int MT, Mode kMode> struct KernelTag {};
 
 template <int NT, int MT, Mode kMode>
-static int launch(const Args& a, const cdssm_lm_layer& w, const Product& p, bf16* out, long long out_stride, int max_blocks,
+static int launch(const Args& a, const cdssm_lm_layer& w, const Product& product, bf16* out, long long out_stride, int max_blocks,
                   cudaStream_t st) {
-    const size_t smem = smem_bytes<NT, MT, kMode == kHead>(p.K);
+    Product p = product;
+    p.apart = smem_bytes<NT, MT, false>(p.K, true) <= kSmemMost / 2 - 1024;   // (a block of the next kernel has room beside it)
+    const size_t smem = smem_bytes<NT, MT, kMode == kHead>(p.K, p.apart);
     if (smem > 48 * 1024)
         if (int rc = allow_smem<KernelTag<NT, MT, kMode>>((const void*)lm_product_kernel<NT, MT, kMode>, kSmemMost)) return rc;
     const int items = ((p.M + 16 * MT - 1) / (16 * MT)) * ((a.B + NT * 8 - 1) / (NT * 8));
@@ -448,10 +464,10 @@ extern "C" int cdssm_b200_lm_decode(const cdssm_lm_layer* layers, int n_layers, 
         a.proj = at(l == 0 ? off.proj0 : off.proj);
         a.v_first = l == 0 ? nullptr : at(off.proj0) + 3 * di;
         if (l > 0 && !w.mix) return CDSSM_ERR_BAD_ARG;
-        const Product in = {(const bf16*)w.w_in, a.x, d_model, 3 * di + H * N, d_model};
-        const Product qg = {(const bf16*)w.w_qg, a.x_conv, di, di + G, di};
-        const Product ro = {(const bf16*)w.w_readout, a.y, (long long)H * N, di, H * N};
-        const Product op = {(const bf16*)w.w_out, a.gated, di, d_model, di};
+        const Product in = {(const bf16*)w.w_in, a.x, d_model, 3 * di + H * N, d_model, 0};
+        const Product qg = {(const bf16*)w.w_qg, a.x_conv, di, di + G, di, 0};
+        const Product ro = {(const bf16*)w.w_readout, a.y, (long long)H * N, di, H * N, 0};
+        const Product op = {(const bf16*)w.w_out, a.gated, di, d_model, di, 0};
         auto ahead = [&](const void* w0, size_t b0, const void* w1, size_t b1) {
             a.ahead[0] = w0; a.ahead_bytes[0] = w0 ? (unsigned)b0 & ~15u : 0;
             a.ahead[1] = w1; a.ahead_bytes[1] = w1 ? (unsigned)b1 & ~15u : 0;
@@ -477,6 +493,6 @@ extern "C" int cdssm_b200_lm_decode(const cdssm_lm_layer* layers, int n_layers, 
         if (rc) return rc;
         if (int rc2 = launch_batch<1, kOutProj>(a, w, op, a.x, d_model, 0, st)) return rc2;
     }
-    const Product head = {(const bf16*)head_w, a.x, d_model, vocab, d_model};
+    const Product head = {(const bf16*)head_w, a.x, d_model, vocab, d_model, 0};
     return launch_batch<2, kHead>(a, layers[0], head, (bf16*)logits, vocab, 2 * sms, st);
 }

@@ -610,7 +610,7 @@ decode_step_kernel(const DecodeArgs a) {
     u.H = a.H; u.D = a.D; u.N = a.N;
     u.pos = a.pos_dev ? *a.pos_dev : a.pos;
     u.units = a.units;
-    decode_unit<T, kCols>(u, (long long)blockIdx.x * kUnitsPerBlock + threadIdx.x / kLanesPerUnit);
+    decode_unit<T, kCols>(u, (long long)blockIdx.x * kUnitsPerBlock + threadIdx.x / kLanesPerUnit, [] {});
 }
 
 // The decode step that reproduces the reference's CHUNKED scan token by token (its outputs beyond the first
