@@ -60,6 +60,7 @@ struct __align__(1024) Smem {
     float scr[4][32 * 12];                         // per warp: kappa[4], rho[4] of token t at 12 t (transposition)
     float qs[4][32];                               // per warp: |q_t|^2
     float om[4][4 * 32];                           // per warp: omega[n'][t]
+    float next[kOutput ? 4 : 1][kOutput ? 2 * kD : 4];   // per warp: the carry into the next item's chunk, on its way
     uint64_t full_k[2], full_q, mma_g, mma_p, taken, q_free, k_free[2], drain;
     uint32_t tmem_base;
     int abort_flag;
@@ -505,6 +506,15 @@ __device__ __forceinline__ void carry_from_chunks(const Args& a, const ItemPos& 
     __syncwarp();
 }
 
+// The carry into an item's chunk, asked for an item ahead: a trip to memory of the two to four sub-blocks that an item has.
+template <int kD>
+__device__ __forceinline__ void ask_for_carry(float* to, const Args& a, const ItemPos& at, int hd, int tl) {
+    const float* from = a.ws_state + (((size_t)at.b * a.NC + at.c) * a.H + hd) * 2 * kD;
+#pragma unroll
+    for (int i = 0; i < kD / 64; i++) cp_async16(to + 128 * i + 4 * tl, from + 128 * i + 4 * tl, true);
+    cp_async_commit();
+}
+
 // kParts: parts of the split of the state and of the update's coefficients, 2 or 3.  Two carry 16 bits, 1.7e-5 of the state after
 // a chunk, far below the bf16 results; three are exact, 1.5e-7 after a chunk like a walk in float32, for a caller who keeps the
 // float32 state after the last token.  us on B200, two / three parts, D 64: 936 chunks 22 / 25, 6144 74 / 96; a third more on
@@ -554,6 +564,8 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
     Tok tk;
     grid_dependency_wait();       // records (local pass) / carries (output pass) of the kernel before
     grid_launch_dependents();
+    if constexpr (kOutput)
+        if (!a.from_chunks) ask_for_carry<kD>(sm.next[J], a, cur, kParts == 2 ? cur.h0 + J : min(cur.h0 + J, last), tl);
     {
         const bool valid = cur.c * kD + tl < L;
         const uint4 first = valid ? __ldcg(a.rec + rec_index(a, kSteps, cur.b, cur.c, 0, (kParts == 2 ? cur.h0 + J : min(cur.h0 + J, last)), tl)) : still4;
@@ -575,6 +587,10 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             if (kOutput && a.from_chunks) {
                 carry_from_chunks<kD>(a, cur, hd, tl, scr, stores);
                 s = scr + (np & 1) * kD;
+            } else if (kOutput) {
+                cp_async_wait_all();
+                __syncwarp();
+                s = sm.next[kOutput ? J : 0] + (np & 1) * kD;
             }
 #pragma unroll
             for (int ks = 0; ks < kKs; ks++) {
@@ -585,7 +601,9 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
                 }
                 S[ks][0] = v0.x; S[ks][1] = v0.y; S[ks][2] = v1.x; S[ks][3] = v1.y;
             }
-            if (kOutput) __syncwarp();     // (scr is used again)
+            if (kOutput) __syncwarp();     // (scr and next are used again)
+            if constexpr (kOutput)
+                if (!a.from_chunks && g + kSteps < NS) ask_for_carry<kD>(sm.next[J], a, nxi, kParts == 2 ? nxi.h0 + J : min(nxi.h0 + J, last), tl);
             gam = {1.f, 0.f};
         }
         // ---- fetch the record of step g + 1 (the next item's first sub-block after this item's last)
@@ -643,7 +661,7 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
         }
         if (!wait(&sm.full_k[st], ph2)) { code = 11; break; }
         if (!kOutput) WA_STAMP(1);
-        {
+        if (kOutput || step > 0) {   // (the local state is zero at the chunk's start)
             uint32_t fa[2][2][4];
             ldsm_x4(frag_addr(ktile[st], 0, 0), fa[0][0]);
             ldsm_x4(frag_addr(ktile[st], 1, 0), fa[0][1]);
@@ -810,13 +828,16 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
             WA_STAMP(9);
             // decay: complex product with W_31; the other part of the complex row sits eight lanes away
             const float wr = W31.r, wi = (np & 1) ? W31.i : -W31.i;
+            // (nothing to decay at the chunk's start; a decay that is no number makes the state none.  128: the test costs as much)
+            if (kOutput || kD == 128 || step > 0 || !(fabsf(W31.r) + fabsf(W31.i) <= 3e38f)) {
 #pragma unroll
-            for (int ks = 0; ks < kKs; ks++)
+                for (int ks = 0; ks < kKs; ks++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const float other = __shfl_xor_sync(0xffffffffu, S[ks][e], 8);
-                    S[ks][e] = wr * S[ks][e] + wi * other;
-                }
+                    for (int e = 0; e < 4; e++) {
+                        const float other = __shfl_xor_sync(0xffffffffu, S[ks][e], 8);
+                        S[ks][e] = wr * S[ks][e] + wi * other;
+                    }
+            }
             uint32_t fb[2][2][4];
             ldsm_x4_trans(frag_addr(ktile[st], 0, 0), fb[0][0]);
             ldsm_x4_trans(frag_addr(ktile[st], 1, 0), fb[0][1]);
