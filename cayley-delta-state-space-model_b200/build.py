@@ -81,7 +81,7 @@ def build(force=False, verbose=False):
     if force or host_procs or _stale(host_path(), host_objs):
         from torch.utils import cpp_extension as ext
         cmd = ["g++", "-shared", "-o", host_path()] + host_objs + [f"-L{p}" for p in ext.library_paths(device_type="cuda")]
-        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-lcublasLt", f"-L{PKG_DIR}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"]
+        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcublasLt", f"-L{PKG_DIR}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"]
         if verbose:
             print(" ".join(cmd))
         subprocess.check_call(cmd)

@@ -3,6 +3,7 @@
 // its Python-side checks took 29 us around a 4 us kernel).  The kernels stay behind the C ABI of libcdssm_b200.so.
 #pragma once
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -62,9 +63,13 @@ inline float* fmut(const Tensor& t) { return t.defined() ? static_cast<float*>(t
 
 inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
-inline Tensor empty_like_dims(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options()); }
+// Outputs straight from the framework's CUDA allocator: by way of the dispatcher an allocation took 0.4 us more, of the 4.5 that a one-token
+// step's call takes.
+inline Tensor empty_like_dims(at::IntArrayRef sizes, const Tensor& like) {
+    return at::detail::empty_cuda(sizes, like.scalar_type(), like.device(), std::nullopt);
+}
 inline Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) {
-    return at::empty(sizes, like.options().dtype(at::kFloat));
+    return at::detail::empty_cuda(sizes, at::kFloat, like.device(), std::nullopt);
 }
 
 struct Dyn {   // the five scalars of the dynamics
