@@ -380,12 +380,12 @@ static int launch_batch(const Args& a, const cdssm_lm_layer& w, const Product& p
 }
 
 // us per step on B200, these kernels / the library's products with this library's glue kernels (issued natively; in
-// brackets replayed from a CUDA graph), 12 layers, N 2, vocabulary 32000 (d 512: 8 layers, N 16; d 256: 4 layers):
-//     d 256    B 16:  73 / 305  (64 / 95)    B 32:  93 / 311  (86 / 97)     B 128: 165 / 301 (156 / 103)
-//     d 512    B 16: 164 / 573 (154 / 233)   B 32: 213 / 575 (201 / 239)    B 128: 477 / 613 (462 / 275)
-//     d 768    B 1:  229 / 864 (214 / 400)   B 16: 253 / 836 (237 / 378)    B 32:  352 / 878 (334 / 378)
+// brackets, as the second figure, from before the loads ahead of the wait, replayed from a CUDA graph), 12 layers, N 2, vocabulary 32000 (d 512: 8 layers, N 16; d 256: 4 layers):
+//     d 256    B 16:  74 / 305  (64 / 95)    B 32:  95 / 311  (86 / 97)     B 128: 165 / 301 (156 / 103)
+//     d 512    B 16: 154 / 573 (154 / 233)   B 32: 217 / 575 (201 / 239)    B 128: 472 / 613 (462 / 275)
+//     d 768    B 1:  203 / 864 (214 / 400)   B 16: 240 / 836 (237 / 378)    B 32:  354 / 878 (334 / 378)
 //              B 64: 522 / 852 (501 / 380)   B 96: 726 / 856 (706 / 390)
-//     d 1024   B 16: 315 / 916 (304 / 420)   B 32: 434 / 836 (416 / 417)    B 64:  758 / 872 (740 / 415)
+//     d 1024   B 16: 306 / 916 (304 / 420)   B 32: 434 / 836 (416 / 417)    B 64:  758 / 872 (740 / 415)
 // Issued call by call the library path is bounded by the host that issues its 112 launches, and these kernels win until the
 // activations every block reads (B x d) weigh more; inside a captured graph the line is at 32 sequences (the caller's check).
 static bool lm_decode_takes(int B, int d, int di, int H, int N, int groups) {

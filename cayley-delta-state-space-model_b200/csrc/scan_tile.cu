@@ -33,9 +33,9 @@
 //
 // Bounded by issue slots (45 % of them busy at 16 warps per SM) and by the chain of barriers and products through a chunk.  us of a
 // whole call on B200, before (a block per chunk and head, Gram blocks and three bf16 parts on the warp-level mma, carry behind a
-// fence and a flag) / now: D 64, B 8, L 2048, H 24, N 16 291 / 245, N 8 171 / 157, N 4 136 / 121; one sequence of 523, N 16
-// 36.7 / 32.5, N 4 22.8 / 20.6; D 128, 4 x 2048, H 12, N 4 76 / 51, 2 x 1000, H 32, N 8 73 / 53, 4000 tokens, H 12, N 16 144 / 81.
-// One or two chunks of D 64, N 8, gain nothing: 2 x 41 tokens, H 16 11.5 / 12.9.
+// fence and a flag) / now: D 64, B 8, L 2048, H 24, N 16 291 / 229, N 8 171 / 151, N 4 136 / 113; one sequence of 523, N 16
+// 36.7 / 29.8, N 4 22.8 / 19.0; D 128, 4 x 2048, H 12, N 4 76 / 49, 2 x 1000, H 32, N 8 73 / 51, 4000 tokens, H 12, N 16 144 / 74.
+// One or two chunks of D 64, N 8, gain nothing: 2 x 41 tokens, H 16 11.5 / 12.3.
 //
 // Reference semantics (intra_chunk_scan.cu:100-195, exact_correction.cu:89-150): z starts at zero at the chunk start, r
 // from the bf16-rounded carry, the correction is read before its step.
