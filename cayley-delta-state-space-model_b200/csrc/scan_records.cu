@@ -34,14 +34,14 @@ struct Args {
 
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-// (Resident blocks that the registers are cut for.  Left to itself the compiler takes 32 registers for one or two pairs and has loads wait
-// for each other: 3 x 777 tokens of 24 heads, N 2, 27.3 us a scan, so 26.5; 12 layers of a 16-token-a-head draw 660, 622.)
-template <int kNP, int kHg, bool kResidual>
-constexpr int kMinBlocks = kHg == 16 ? 2 : kNP <= 2 ? 5 : kNP == 8 && kResidual ? 3 : 4;
+// (Resident blocks that the registers are cut for.  Left to itself the compiler takes 32 registers for the N = 2 form and has loads wait
+// for each other: 3 x 777 tokens of 24 heads 27.3 us a scan, so 26.5.)
+template <int kNP, int kHg, bool kResidual, bool kWa>
+constexpr int kMinBlocks = kHg == 16 ? 2 : kNP <= 2 ? (kWa ? 5 : 1) : kNP == 8 && kResidual ? 3 : 4;
 
 // kNP: pairs per thread, from kNP * blockIdx.z on; kHg: heads per block.
 template <int kNP, int kHg, bool kWa, bool kResidual>
-__global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual>) records_kernel(const Args a) {
+__global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>) records_kernel(const Args a) {
     using T = __nv_bfloat16;
     constexpr int kItems = kTokens * kHg / kThreads, kRow = kTokens + 1;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -52,20 +52,26 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual>) rec
     grid_dependency_wait();
     const size_t first = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x, step = (size_t)gridDim.x * gridDim.y * kThreads;
     if (kWa) {   // a few words
-#pragma unroll 1
         for (size_t i = first; i < a.clear_words; i += step) a.clear[i] = 0;
     } else if (blockIdx.z == 0) {
-#pragma unroll 1
         for (size_t i = first; i < a.clear_words / 4; i += step) reinterpret_cast<uint4*>(a.clear)[i] = make_uint4(0u, 0u, 0u, 0u);
         if (first < a.clear_words % 4) a.clear[a.clear_words / 4 * 4 + first] = 0;
-#pragma unroll 1
         for (size_t i = first; i < a.clear2_words / 4; i += step) reinterpret_cast<uint4*>(a.clear2)[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     const int H = a.H, N = a.N, NP = N >> 1, p0 = kWa ? 0 : kNP * (int)blockIdx.z, pairs = min(kNP, NP - p0);
-    uint32_t row_of = __umulhi(blockIdx.x, a.tiles_inv);   // (the quotient, or one more)
-    if (row_of * (uint32_t)a.tiles > blockIdx.x) row_of--;
+    // (One or two pairs a thread are for short inputs, a layer's scan of which takes 15 us whatever these instructions: with the quick
+    // division and cut registers 8 layers of 300 tokens, N 4, took 403 us, without 387; 12 of 60, N 8, 545 / 536.)
+    constexpr bool kQuick = kWa || kNP >= 4;
+    uint32_t row_of;
+    if (kQuick) {
+        row_of = __umulhi(blockIdx.x, a.tiles_inv);   // (the quotient, or one more)
+        if (row_of * (uint32_t)a.tiles > blockIdx.x) row_of--;
+    } else {
+        row_of = blockIdx.x / (unsigned)a.tiles;
+    }
     const int b = (int)row_of, tile = (int)(blockIdx.x - row_of * (uint32_t)a.tiles), l0 = tile * kTokens;
-    const int before = a.pos0 + (a.segs > 1 ? (b % a.segs) * a.L : 0);   // position of the row's first token
+    // position of the row's first token
+    const int before = a.pos0 + (kQuick ? (a.segs > 1 ? (b % a.segs) * a.L : 0) : (b % a.segs) * a.L);
     const int head0 = blockIdx.y * kHg, heads = min(kHg, H - head0);
     const int head = threadIdx.x & (kHg - 1), hd = head0 + min(head, heads - 1);
     const float lds = a.log_dt_scale[hd], freq = a.rope_freqs[hd];
@@ -135,7 +141,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual>) rec
         for (int h = warp; h < heads; h += kThreads / 32)
             a.rec[(((size_t)b * a.tiles + tile) * H + head0 + h) * kTokens + lane] = sr[h * kRow + lane];
     } else {
-        const int c = l0 >> (a.C == 64 ? 6 : 7), in_chunk = l0 & (a.C - 1);
+        const int c = kQuick ? l0 >> (a.C == 64 ? 6 : 7) : l0 / a.C, in_chunk = l0 - c * a.C;
         const size_t unit0 = ((size_t)b * a.NC + c) * H + head0;
         if constexpr (kNP >= 4) {   // a warp has a head and its pairs: no division an item
 #pragma unroll 1
@@ -151,7 +157,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual>) rec
                 }
             }
         } else {                    // (12 layers of a 523-token prompt, two pairs a thread: 796 us, 823 in the other order)
-#pragma unroll 1
             for (int i = warp; i < heads * pairs; i += kThreads / 32) {
                 const int h = i / pairs, p = i - h * pairs, s = (p * kHg + h) * kRow + lane;
                 const size_t o = ((unit0 + h) * NP + p0 + p) * a.C + in_chunk + lane;
@@ -159,7 +164,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual>) rec
                 a.rec_v[o] = sv[s];
             }
         }
-#pragma unroll 1
         for (int h = warp; h < heads && p0 == 0; h += kThreads / 32) a.rec_g[(unit0 + h) * a.C + in_chunk + lane] = sg[h * kRow + lane];
     }
 }
