@@ -899,7 +899,10 @@ __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
         if (g + 1 < NS) tk = prepare(rec, tl);
         WA_STAMP(11);
     }
-    if (code && tl == 0) atomicCAS(a.status, 0, 200 + code);
+    if (code) {
+        if (kOutput) cp_async_wait_all();   // (a carry may be on its way)
+        if (tl == 0) atomicCAS(a.status, 0, 200 + code);
+    }
 }
 
 template <int kD, bool kOutput, int kParts>
