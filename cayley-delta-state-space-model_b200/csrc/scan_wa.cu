@@ -517,7 +517,7 @@ __device__ __forceinline__ void ask_for_carry(float* to, const Args& a, const It
 
 // kParts: parts of the split of the state and of the update's coefficients, 2 or 3.  Two carry 16 bits, 1.7e-5 of the state after
 // a chunk, far below the bf16 results; three are exact, 1.5e-7 after a chunk like a walk in float32, for a caller who keeps the
-// float32 state after the last token.  us on B200, two / three parts, D 64: 936 chunks 22 / 25, 6144 74 / 96; a third more on
+// float32 state after the last token.  us on B200, two / three parts, D 64: 936 chunks 21 / 24, 6144 70 / 85; a quarter more on
 // average.
 template <int kD, bool kOutput, int kParts>
 __device__ __forceinline__ void compute(Smem<kD, kOutput>& sm, const Args& a) {
