@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>
         const bool on = l < a.L;                                       // behind the end a = 1, beta = v = 0: the state stands still
         const float pos = (float)(l + before);
         auto f = [](T y) { return __bfloat162float(y); };
-        const DynShared ds = dyn_shared<true>(f(x[i][5]), f(x[i][6]), f(x[i][0]), f(x[i][1]), f(x[i][2]), f(x[i][3]), f(x[i][4]),
+        const DynShared ds = dyn_shared<true, kWa>(f(x[i][5]), f(x[i][6]), f(x[i][0]), f(x[i][1]), f(x[i][2]), f(x[i][3]), f(x[i][4]),
                                               lds, freq, pos, a.dc);
         const uint32_t bs = on ? pack2(ds.beta, ds.sel_c) : 0u;
         if (!kWa) sg[head * kRow + t] = bs;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>
         for (int p = 0; p < kNP; p++) {
             if (p >= pairs) break;
             float ar, ai, vp;
-            dyn_pair<true>(f(ga[i][p]), f(gw[i][p]), freq, pos, ds, ar, ai, vp);
+            dyn_pair<true, kWa>(f(ga[i][p]), f(gw[i][p]), freq, pos, ds, ar, ai, vp);
             if (!a.fp32_decay) { ar = bfr(ar); ai = bfr(ai); }
             vp = bfr(vp);
             float v0 = __uint_as_float(vv[i][p] << 16), v1 = __uint_as_float(vv[i][p] & 0xffff0000u);
