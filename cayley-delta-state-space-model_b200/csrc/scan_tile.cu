@@ -77,7 +77,8 @@ struct Args {
 #define kNotANumber __int_as_float(0x7fffffff)
 
 struct cplx { float r, i; };
-// (Which products and sums go together is said here and below, not left to the compiler: the versions of the kernel have the same bits.)
+// (Which products and sums go together is said here and below, not left to the compiler: the versions of the kernel have the same bits.
+// cmul(a, b) and cmul(b, a) differ in the last bit of the imaginary part.)
 __device__ __forceinline__ cplx cmul(cplx a, cplx b) {
     return {__fmaf_rn(a.r, b.r, -__fmul_rn(a.i, b.i)), __fmaf_rn(a.r, b.i, __fmul_rn(a.i, b.r))};
 }
@@ -106,7 +107,8 @@ struct BlockPair {   // of one 32-token block and pair
 // a_16 ... a_t = D_t, and neither half leaves the float range unless one half alone decays by more than 1e-30.
 // kW pairs side by side: one alone waits for its shuffles.  at, vg: a_t, v_t in; D, v_t / D out (a and v of a pair outside the
 // range: the walk reads them themselves).  Returns the pairs outside the range, a bit each.
-template <int kW>
+// kSwap: the factors of the prefix products the other way round, for the bits of the pair that a first warp has alone (kD 64, four pairs).
+template <int kW, bool kSwap>
 __device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, BlockPair (&bp)[kW]) {
     const bool lo = tl < 16;
     cplx X[kW];
@@ -118,7 +120,7 @@ __device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, 
 #pragma unroll
         for (int w = 0; w < kW; w++) {
             const cplx other = cshfl(X[w], lo ? tl + o : tl - o);
-            if (on) X[w] = cmul(X[w], other);
+            if (on) X[w] = kSwap ? cmul(other, X[w]) : cmul(X[w], other);
         }
     }
     int slow = 0;
@@ -154,8 +156,8 @@ __device__ __forceinline__ int scalings(cplx (&at)[kW], cplx (&vg)[kW], int tl, 
 // be zero in float32 where the value is of order one.
 __device__ __forceinline__ cplx behind(const BlockPair* bp, int from, int to, int blocks) {
     cplx f = {1.f, 0.f};
-    for (int j = from + 1; j < to; j++) f = cmul(f, bp[j].A);
-    return to < blocks ? cmul(f, bp[to].R) : f;
+    for (int j = from + 1; j < to; j++) f = cmul(bp[j].A, f);
+    return to < blocks ? cmul(bp[to].R, f) : f;
 }
 
 // s <- gamma s + l in the order in which the carry pass (scan_simt.cu) evaluates it, so that the two ways to hand the carry on
@@ -384,7 +386,7 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode, kWide>& sm, int p
         }
 #pragma unroll
         for (int i = 0; i < kCols; i++) {
-            const cplx z = cmul({a.x, a.y}, {zr[i], zi[i]});
+            const cplx z = cmul({zr[i], zi[i]}, {a.x, a.y});
             zr[i] = z.r + gt.r * k[i];
             zi[i] = z.i + gt.i * k[i];
         }
@@ -410,7 +412,7 @@ __device__ __noinline__ void slow_walk(Smem<kD, kPairs, kMode, kWide>& sm, int p
     for (int o = 1; o < 32; o <<= 1) {
         const int from = kReadout ? tl - o : tl + o;
         const cplx other = cshfl(S, from);
-        if (from >= 0 && from < 32) S = cmul(S, other);
+        if (from >= 0 && from < 32) S = cmul(other, S);
     }
     cplx V = cshfl(S, kReadout ? tl - 1 : tl + 1);
     if (tl == (kReadout ? 0 : 31)) V = {1.f, 0.f};
@@ -611,7 +613,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
                 at[w] = {x.x, x.y};
                 vg[w] = {bits_lo(y), bits_hi(y)};
             }
-            const int slow = (scalings<kW>(at, vg, tl, bp) << p0) & ((1 << p_hi) - 1);
+            const int slow = (scalings<kW, kD == 64 && kPairs == 4 && kW == 1>(at, vg, tl, bp) << p0) & ((1 << p_hi) - 1);
 #pragma unroll
             for (int w = 0; w < kW; w++) {
                 if (p0 + w >= p_hi) break;
@@ -1041,7 +1043,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         const BlockPair* bp = &sm.bp[p][row0 / 32];
         cplx w = bp[0].A;
 #pragma unroll
-        for (int J = 1; J < kBlocks; J++) w = cmul(w, bp[J].A);
+        for (int J = 1; J < kBlocks; J++) w = cmul(bp[J].A, w);
         return w;
     };
 
@@ -1400,21 +1402,21 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         cplx pre = {1.f, 0.f};
 #pragma unroll
         for (int J = 0; J < kEarlier; J++)
-            if (J < I) pre = cmul(pre, sm.bp[p][row0 / 32 + J].A);
+            if (J < I) pre = cmul(sm.bp[p][row0 / 32 + J].A, pre);
         return pre;
     };
 #pragma unroll
     for (int q = 0; q < kOwn; q++) {
         const int p = pair_of(q);
-        const cplx pre = decay_before(p), F = cmul(pre, sm.bp[p][W4].R);
+        const cplx pre = decay_before(p), F = cmul(sm.bp[p][W4].R, pre);
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int row = base + 8 * r + g;
             const float x = __fmaf_rn(pd[r], gx[q][r], oz[q][r]), xo = other_of(x), ho = other_of(rho[q][r]);
             const float2 D = sm.dd[p][row], D0 = sm.dd[p][row > 0 ? row - 1 : 0];
             const bool first = r == 0 && g == 0;
-            const cplx w0 = first ? pre : cmul({D0.x, D0.y}, F);
-            oz[q][r] = rotate({D.x, D.y}, x, xo) + rotate(w0, rho[q][r], ho);
+            const cplx w0 = first ? pre : cmul(F, {D0.x, D0.y});
+            oz[q][r] = rotate({D.x, D.y}, x, xo) + __fmaf_rn(comp ? w0.i : -w0.i, ho, __fmul_rn(w0.r, rho[q][r]));
         }
     }
     if (slow != 0) {

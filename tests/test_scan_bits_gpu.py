@@ -13,8 +13,18 @@ pytestmark = pytest.mark.gpu
 
 # (H, L, D, N): CRC-32 of y and of the state after the last token.  Gates as a model meets them; "wild": decays that leave the range of a
 # block's scaled unknowns, so that pairs of it are walked.
-MODEL = {(8, 500, 64, 2): (3704699172, 2960037014), (4, 700, 128, 2): (1125811291, 434316177)}
-WILD = {(8, 500, 64, 2): (1628976053, 3590081624), (4, 700, 128, 2): (4044209766, 648969707)}
+MODEL = {(8, 500, 64, 2): (3704699172, 2960037014), (4, 700, 128, 2): (1125811291, 434316177),
+         (5, 381, 64, 4): (2027905606, 1066116165), (24, 1000, 64, 6): (2352845244, 254133680),
+         (3, 381, 64, 8): (1354727775, 2107887923), (24, 1277, 64, 12): (1203873897, 415273592),
+         (8, 523, 64, 16): (4094638131, 2880548728), (3, 765, 128, 4): (575050562, 3904660780),
+         (12, 1000, 128, 6): (143255022, 802764237), (2, 765, 128, 8): (535030354, 2139756516),
+         (24, 1500, 128, 16): (2966473696, 1151683306)}
+WILD = {(8, 500, 64, 2): (1628976053, 3590081624), (4, 700, 128, 2): (4044209766, 648969707),
+        (5, 381, 64, 4): (4013498383, 172472818), (24, 1000, 64, 6): (1437431076, 3742570834),
+        (3, 381, 64, 8): (566478194, 676250229), (24, 1277, 64, 12): (3864467463, 195932802),
+        (8, 523, 64, 16): (1137290871, 1282402986), (3, 765, 128, 4): (76320381, 709193589),
+        (12, 1000, 128, 6): (784751710, 2207710518), (2, 765, 128, 8): (1275000913, 2199383906),
+        (24, 1500, 128, 16): (2169433470, 2795242774)}
 
 
 def _inputs(H, L, D, N, wild):
