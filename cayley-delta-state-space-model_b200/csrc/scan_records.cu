@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>
     float2* sa = reinterpret_cast<float2*>(smem);                      // else [pair][head][token]
     uint32_t* sv = reinterpret_cast<uint32_t*>(sa + kNP * kHg * kRow);
     uint32_t* sg = sv + kNP * kHg * kRow;
+    __shared__ int old_ticket;   // (read by nobody: the wait for it is what counts)
     grid_dependency_wait();
     const size_t first = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kThreads + threadIdx.x, step = (size_t)gridDim.x * gridDim.y * kThreads;
     if (kWa) {   // a few words
@@ -58,6 +59,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>
         if (first < a.clear_words % 4) a.clear[a.clear_words / 4 * 4 + first] = 0;
         for (size_t i = first; i < a.clear2_words / 4; i += step) reinterpret_cast<uint4*>(a.clear2)[i] = make_uint4(0u, 0u, 0u, 0u);
     }
+    // The whole-chunk scan's wide blocks draw tickets from clear[1] before this kernel is done (scan_tile.cu): the word is zero in the L2 cache
+    // when the exchange is back, and nothing else of this launch touches it afterwards (the store above is the same thread's).
+    const bool clears_ticket = !kWa && first == 0 && blockIdx.z == 0 && a.clear_words > 1;
+    int ticket = 0;
+    if (clears_ticket) ticket = atomicExch(a.clear + 1, 0);
     const int H = a.H, N = a.N, NP = N >> 1, p0 = kWa ? 0 : kNP * (int)blockIdx.z, pairs = min(kNP, NP - p0);
     // (One or two pairs a thread are for short inputs, a layer's scan of which takes 15 us whatever these instructions: with the quick
     // division and cut registers 8 layers of 300 tokens, N 4, took 403 us, without 387; 12 of 60, N 8, 545 / 536.)
@@ -133,6 +139,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>
             }
         }
     }
+    if (clears_ticket) *reinterpret_cast<volatile int*>(&old_ticket) = ticket;   // (it is back)
     __syncthreads();
     grid_launch_dependents();   // (not earlier: blocks that start while these fill the SMs are packed onto the few with room)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -71,7 +71,7 @@ struct Args {
     int HG;                      // tiles beside each other: ceil(H / heads of a tile) x blocks that share a tile (kPairs pairs each)
     int groups;
     int from_chunks;             // kOutput: the carry from the local results of the chunks before (no carry pass has run)
-    int fixed;                   // kFused: blocks have the tiles of their own numbers, not of tickets
+    int fixed;                   // kFused: a block per SM at most: narrow blocks have the tiles of their own numbers, not of tickets
 };
 
 #define kNotANumber __int_as_float(0x7fffffff)
@@ -502,8 +502,11 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         if (tid == 0) atomicCAS(a.status, 0, 399);
         return;
     }
-    // The records kernel clears the ticket counter.  While there is a block per SM at most the blocks need no tickets (launch_one()),
-    // and start on their tiles while it is still at work (8 layers of 2 x 41 tokens, N 8: 404 us with tickets, 376 without).
+    // The records kernel clears the ticket counter.  While there is a block per SM at most the blocks start on their tiles while it is still at
+    // work (8 layers of 2 x 41 tokens, N 8: 404 us, 376 so).  Narrow ones need no tickets then (launch_mode()).  Wide ones do, an SM has
+    // room for one, and draw them before the records are there: the exchange that clears the counter has come back to its block before that
+    // block lets this kernel start, and the additions here take place at the same word of the L2 cache.  It costs 0.1 to 0.5 us
+    // of a call (523 tokens, H 24, N 16 29.6 -> 30.1; D 128, 1000 tokens, H 12, N 8 21.4 -> 21.5), the narrow form 30.9 and 23.7.
     const bool early = kMode == kLocal || (kMode == kFused && a.fixed);
     if (kMode == kFused && !early) grid_dependency_wait();
     if (tid == 0) {
@@ -515,9 +518,8 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         sm.bad_rows = 0;
         sm.first_bad[0] = sm.first_bad[1] = kD;
         fence_barrier_init();
-        const bool drawn = kMode == kFused && !early;
-        sm.item = drawn ? atomicAdd(a.ticket, 1) : (int)blockIdx.x;
-        sm.stop = drawn ? *reinterpret_cast<volatile int*>(a.status) : 0;
+        sm.item = kMode == kFused && (kWide || !early) ? atomicAdd(a.ticket, 1) : (int)blockIdx.x;
+        sm.stop = kMode == kFused && !early ? *reinterpret_cast<volatile int*>(a.status) : 0;
     }
     __syncthreads();
     if (sm.stop) return;   // an earlier block gave up
@@ -1519,7 +1521,8 @@ static int launch_mode(Mode m, const CUtensorMap& tmK, const CUtensorMap& tmQ, A
     if (int rc = sm_count(sms)) return rc;
     // Blocks wait for those with smaller numbers, which start first: blocks start in the order of their numbers.  No document says
     // so, hence one block per SM at most: should other streams' kernels hold back an earlier one, the waiting blocks have at most one
-    // of two or more places of an SM, and a wait that lasts ends with the status word set.
+    // of two or more places of an SM, and a wait that lasts ends with the status word set.  A wide block has an SM to itself, two calls on two
+    // streams would have no place left, so wide blocks draw tickets: whatever a block waits for is done or running.
     a.fixed = items <= sms;
     if (m == kLocal) return launch_one<kD, kPairs, kLocal>(tmK, tmQ, a, items, st);
     if (m == kOutput) return launch_one<kD, kPairs, kOutput>(tmK, tmQ, a, items, st);

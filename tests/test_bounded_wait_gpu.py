@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from test_scan_gpu import oracle_scan, run_fused
-from util import BF16_TOL, rel_err, to_np
+from util import BF16_TOL, const_args, rel_err, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +74,42 @@ def test_halves_of_the_whole_chunk_scan_give_up_too(ops, orc, D, N, keep):
     wy, _ = oracle_scan(orc, inp, N, D, orc.ROUND_FP32_STATE)
     y[1, D + 3:, 2] = wy[1, D + 3:, 2]
     assert rel_err(y, wy) <= BF16_TOL
+
+
+@pytest.mark.parametrize("D,N,H,L", [(64, 16, 24, 523), (64, 12, 3, 69), (128, 8, 12, 1000), (128, 16, 2, 133)])
+def test_wide_blocks_give_up_too(ops, orc, D, N, H, L):
+    """The form with a warp per column tile (a block per SM at most), with tickets."""
+    inp = orc.make_inputs(1, H, L, D, N=N, seed=44, bf16=True)
+    old = ops.set_wait_limit_ns(2_000_000)
+    try:
+        run_fused(ops, inp, torch.bfloat16, N, D, flags=ops.TEST_WITHHOLD)
+        assert 200 <= ops.scan_fused_status() < 300
+    finally:
+        ops.set_wait_limit_ns(old)
+    y, _ = run_fused(ops, inp, torch.bfloat16, N, D, strict=True)
+    wy, _ = oracle_scan(orc, inp, N, D, orc.ROUND_REFERENCE)
+    assert rel_err(to_np(y), wy) <= BF16_TOL
+
+
+@pytest.mark.parametrize("D,N,H,L", [(64, 16, 24, 523), (64, 10, 24, 700), (128, 8, 12, 1400)])
+def test_wide_blocks_of_two_streams_share_the_gpu(ops, orc, D, N, H, L):
+    """Two calls whose blocks fill an SM each and are together more than there are SMs: a block that waits for another must find it done or
+    running whichever call's blocks started first."""
+    inp = orc.make_inputs(1, H, L, D, N=N, seed=45, bf16=True)
+    d = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    args = [d(inp[k]).bfloat16() for k in ("q", "k", "v", "gate_raw")] + [d(inp["log_dt_scale"]), d(inp["rope_freqs"]), *const_args(inp["consts"]),
+                                                                         H, N, D]
+    want = ops.scan_fused(*args)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = [[], []]
+    for i in range(40):
+        for s, out in zip(streams, got):
+            with torch.cuda.stream(s):
+                out.append(ops.scan_fused(*args))
+                if i % 10 == 9:
+                    assert ops.scan_fused_status() == 0
+    torch.cuda.synchronize()
+    for out in got:
+        for y, fin in out:
+            assert torch.equal(y, want[0]) and torch.equal(fin, want[1])
