@@ -526,6 +526,14 @@ static int launch_walk(const ScanArgs& a, unsigned blocks, cudaStream_t st) {
     return launch_overlapped(scan_walk_kernel<T, kCols, kLanesPerUnit, kOutput, kRing>, dim3(blocks), dim3(kSimtThreads), smem, st, a);
 }
 
+// Whether a state that the call leaves lies where h0 does (a caller who carries one buffer on).  The carry pass reads and writes an element in one
+// thread; where the output pass adds the carry up itself, every chunk's block reads h0 and the last chunk's writes.
+static bool writes_into_h0(const ScanArgs& a) {
+    const uintptr_t bytes = (uintptr_t)a.B * a.H * a.N * a.D * sizeof(float), h0 = (uintptr_t)a.h0;
+    auto meets = [&](const float* out) { return out != nullptr && (uintptr_t)out < h0 + bytes && h0 < (uintptr_t)out + bytes; };
+    return h0 != 0 && (meets(a.final_state) || meets(a.tail_state));
+}
+
 template <typename T, int kCols>
 static int launch_simt(const ScanArgs& a, cudaStream_t st) {
     constexpr int kUnits = kUnitsPerBlock, kRing = 8;
@@ -551,7 +559,7 @@ static int launch_simt(const ScanArgs& a, cudaStream_t st) {
             return rc;
     }
     // (the short walk adds a few chunks up itself, instead of a launch and two more trips to memory)
-    const bool from_chunks = short_walk && output && a.run_local && a.publish && !a.total_decay && a.NC <= 12;
+    const bool from_chunks = short_walk && output && a.run_local && a.publish && !a.total_decay && a.NC <= 12 && !writes_into_h0(a);
     if (!from_chunks) {
         const long long th = (long long)a.B * a.H * (a.N / 2) * a.D;
         if (int rc = launch_overlapped(scan_carry_kernel<T>, dim3((unsigned)((th + 127) / 128)), dim3(128), 0, st, a)) return rc;
@@ -990,7 +998,8 @@ static int scan_fused_impl(const void* q, const void* k, const void* v, const vo
     if (!tensor) return scan_fused_simt(a, dtype, st);
     const int withhold = (flags & CDSSM_SCAN_TEST_WITHHOLD) ? 1 : 0;
     const unsigned long long limit = wait_limit_ns();
-    const int from_chunks = (wa_ok ? carry_in_output(B, a.NC, H) : few_chunks(B, H, a.NC, D, N)) && tc_local && tc_output && a.run_local && !summary_only;
+    const int from_chunks = (wa_ok ? carry_in_output(B, a.NC, H) : few_chunks(B, H, a.NC, D, N)) && tc_local && tc_output && a.run_local && !summary_only &&
+                            !writes_into_h0(a);
     auto pass = [&](int mode) {   // 0: local, 1: output, 2: both in one kernel
         if (wa_ok)
             return scan_wa_pass(mode == 1, q, q_rs, k, k_rs, rec, a.ws_gamma, a.ws_state, y, tail_state, status, shortcut_scale, B, L, H, D,

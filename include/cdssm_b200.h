@@ -234,7 +234,7 @@ CDSSM_API size_t cdssm_b200_scan_fused_workspace_bytes_for(int B, int L, int H, 
  *   h0 (B,H,N,D) float32 or NULL: carry into the first chunk;
  *   y (B,L,H,N); final_state (B,H,N,D) float32 or NULL: carry after the last chunk;
  *   tail_state (B,H,N,D) float32 or NULL: the recurrent state after token L-1 (what the
- *   one-token decode step continues from);
+ *   one-token decode step continues from); either may be h0's own buffer;
  *   workspace: at least cdssm_b200_scan_fused_workspace_bytes bytes, 256-byte aligned.
  * With h0 = NULL and shortcut handled as in cdssm/models/block.py:202-211 this equals
  * DynamicsFusedFn + NormalizeKQFn + SSDChunkwiseScan + the read-out of the reference block.

@@ -11,15 +11,15 @@ from util import const_args, to_dev
 pytestmark = pytest.mark.gpu
 
 
-def _call(lib, t, outs, consts, dims, dt, rows=None, room=None):
-    """The scan through the C ABI on the CUDA cores; t: q, k, v, gates, log_dt_scale, rope_freqs, h0."""
+def _call(lib, t, outs, consts, dims, dt, room=None, flags=1):
+    """The scan through the C ABI, by default on the CUDA cores; t: q, k, v, gates, log_dt_scale, rope_freqs, h0."""
     B, L, H, D, N, C = dims
     if room is None:
-        room = lib.cdssm_b200_scan_fused_workspace_bytes_for(B, L, H, D, N, C, dt, 1)
+        room = lib.cdssm_b200_scan_fused_workspace_bytes_for(B, L, H, D, N, C, dt, flags)
     ws = torch.full((room + 256,), 0x5a, dtype=torch.uint8, device="cuda")
     ptr = lambda x: ctypes.c_void_p(0 if x is None else x.data_ptr())
     args = [ptr(x) for x in t + outs] + [ctypes.c_void_p(ws.data_ptr() + (-ws.data_ptr()) % 256), ctypes.c_size_t(room)]
-    args += [ctypes.c_float(c) for c in consts] + [ctypes.c_float(0.25), B, L, H, D, N, C, 3, dt, 1]
+    args += [ctypes.c_float(c) for c in consts] + [ctypes.c_float(0.25), B, L, H, D, N, C, 3, dt, flags]
     assert lib.cdssm_b200_scan_fused_fwd(*args, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     torch.cuda.synchronize()
 
@@ -75,3 +75,31 @@ def test_nothing_is_written_beside_the_outputs(ops, orc, dtype):
     _call(lib, t + [None], want, const_args(inp["consts"]), (B, L, H, D, N, C), dt)
     for b, n, w in zip(bufs, sizes, want):
         assert bool((b[:5] == 7).all()) and bool((b[5 + n:] == 7).all()) and torch.equal(b[5:5 + n], w)
+
+
+@pytest.mark.parametrize("dtype,H,L,D,N,flags,little", [
+    (torch.float32, 3, 50, 64, 2, 0, False), (torch.float32, 4, 128, 64, 6, 0, False), (torch.float32, 2, 64 * 12, 64, 2, 0, False),
+    (torch.float32, 2, 300, 128, 2, 0, False), (torch.bfloat16, 2, 500, 64, 4, 1, False),
+    (torch.bfloat16, 8, 300, 64, 2, 0, False), (torch.bfloat16, 3, 300, 128, 2, 0, False),    # N = 2 on the tensor cores
+    (torch.bfloat16, 3, 300, 64, 8, 0, True), (torch.bfloat16, 2, 300, 128, 4, 0, True),      # whole chunks, two kernels
+    (torch.bfloat16, 6, 500, 64, 16, 0, False)])                                              # and one
+@pytest.mark.parametrize("which", [1, 2])
+def test_states_may_take_the_place_of_h0(ops, orc, dtype, H, L, D, N, flags, little, which):
+    """final_state or tail_state in h0's buffer: no block reads what another has written over, whoever adds the carry up."""
+    import cdssm_b200
+    lib = cdssm_b200._lib.lib()
+    B, dt = 2, 1 if dtype == torch.float32 else 0
+    inp = unnormalise(orc.make_inputs(B, H, L, D, N=N, seed=L + N, context_length=L), np.random.default_rng(L))
+    state = to_dev(np.random.default_rng(N).standard_normal((B, H, N, D)).astype(np.float32) * 0.3, torch.float32)
+    t = [to_dev(inp[n], dtype) for n in ("q", "k", "v", "gate_raw")] + [to_dev(inp[n], torch.float32) for n in ("log_dt_scale", "rope_freqs")]
+    room = lib.cdssm_b200_scan_fused_workspace_bytes_for(B, L, H, D, N, D, dt, flags)
+    room -= B * -(-L // D) * H * (N // 2) * D * 8 if little else 0   # (words that hand the carry on)
+    outs = lambda: [torch.full((B, L, H, N), 3.0, device="cuda", dtype=dtype)] + [torch.full((B, H, N, D), 3.0, device="cuda") for _ in range(2)]
+    want = outs()
+    _call(lib, t + [state], want, const_args(inp["consts"]), (B, L, H, D, N, D), dt, room=room, flags=flags)
+    for _ in range(10):
+        got = outs()
+        got[which] = state.clone()
+        _call(lib, t + [got[which]], got, const_args(inp["consts"]), (B, L, H, D, N, D), dt, room=room, flags=flags)
+        for w, g in zip(want, got):
+            assert torch.equal(w, g)
