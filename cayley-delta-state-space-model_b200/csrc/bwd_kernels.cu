@@ -69,7 +69,7 @@ dynamics_bwd_kernel(const T* __restrict__ gA, const T* __restrict__ gvp, const T
             const float e_raw = num2 * iden;
             const bool e_free = e_raw > 1e-8f;                            // the clamp passes the gradient through
             const float e = fmaxf(e_raw, 1e-8f), le = log_<kFast>(e);
-            const float scale = exp_<kFast>(x * le), eff = exp_<kFast>(cr * le);
+            const float scale = exp_alone<kFast>(x * le), eff = exp_alone<kFast>(cr * le);
             const float vp2 = 1.0f - eff;
             const float uA_re = IO<T>::ld(gA + idx * N + 2 * j), uA_im = IO<T>::ld(gA + idx * N + 2 * j + 1);
             const float uvp = IO<T>::ld(gvp + idx * NH + j);

@@ -3,8 +3,8 @@
 // The formulas restate the reference's (cdssm/csrc/include/common.cuh:82-91 for the
 // activations, cdssm/csrc/include/cayley_math.cuh:51-99 for the Cayley map,
 // cdssm/csrc/kernels/dynamics_fused.cu:64-139 for the gate pipeline).  The reference is built
-// with --use_fast_math, so its expf/logf/powf and '/' are the fast intrinsics; the bfloat16
-// instantiations here call those intrinsics explicitly (kFast) and their outputs agree with
+// with --use_fast_math, so its expf/logf/powf and '/' come from the special-function unit; the
+// bfloat16 instantiations here take theirs from it too (kFast), and their outputs agree with
 // the reference's bit for bit almost everywhere.  The float32 instantiations use the accurate
 // library functions instead, to stay within 1e-4 of an fp32 restatement over long sequences.
 #pragma once
@@ -34,16 +34,18 @@ template <> struct IO<float> {
     static __device__ __forceinline__ float rnd(float x) { return x; }
 };
 
-// kFast, from the special-function unit: e^x = 2^(x log2 e), ln x = ln 2 log2 x, x^y = 2^(y log2 x), a / b = a (1 / b).  The intrinsics
-// (__expf, __logf, __powf, __fdividef) give the same bits wherever neither an argument nor a result is subnormal, and take up to five
-// more instructions each for those: an exponential that small is added to one here, logarithms are of 1 + e^x or of at least
-// 1e-8, divisors are 1 + e^x or sums of positive terms.  (The power itself may be subnormal: no flush there.)
+// kFast, from the special-function unit by the identities e^x = 2^(x log2 e), ln x = ln 2 log2 x, x^y = 2^(y log2 x) and a / b = a (1 / b).  The
+// instructions are good to 2^-22 (PTX ISA); .ftz takes subnormal numbers for zero.  That is harmless where an exponential is added to one, a
+// logarithm is of 1 + e^x or of at least 1e-8, a divisor is 1 + e^x, a sum of positive terms or the caller's adt_smoothness.  Powers stand alone: no
+// flush there (sfu_exp2_sub).  Against float64 over the range of the gates: test_scan_bits_gpu.py.
 __device__ __forceinline__ float sfu_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float sfu_exp2_sub(float x) { float r; asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float sfu_log2(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float sfu_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 
+// (of terms beside one)
 template <bool kFast> __device__ __forceinline__ float exp_(float x) { return kFast ? sfu_exp2(__fmul_rn(x, 1.44269504f)) : expf(x); }
+template <bool kFast> __device__ __forceinline__ float exp_alone(float x) { return kFast ? sfu_exp2_sub(__fmul_rn(x, 1.44269504f)) : expf(x); }
 template <bool kFast> __device__ __forceinline__ float log_(float x) { return kFast ? __fmul_rn(sfu_log2(x), 0.693147181f) : logf(x); }
 template <bool kFast> __device__ __forceinline__ float pow_(float x, float y) { return kFast ? sfu_exp2_sub(__fmul_rn(y, sfu_log2(x))) : powf(x, y); }
 template <bool kFast> __device__ __forceinline__ float div_(float a, float b) { return kFast ? __fmul_rn(a, sfu_rcp(b)) : a / b; }
@@ -174,7 +176,7 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
     return *reinterpret_cast<uint32_t*>(&p);
 }
 // x / (1 + 2^(-x log2 e)).  What the exponential flushes to zero is nothing beside one; the reciprocal flushes below x = -87.3, where the
-// result (-1e-36 and nearer to zero) becomes zero, as it did with __fdividef.
+// result (-1e-36 and nearer to zero) becomes zero.
 __device__ __forceinline__ float2 silu2(float2 x) {
     const float2 t = __fmul2_rn(x, make_float2(-1.44269504f, -1.44269504f));
     float2 e, r;

@@ -30,6 +30,27 @@ def test_dynamics_backward(ops, orc, dtype, tol, B, H, L, N):
     assert np.abs(to_np(lds.grad) - wl).max() <= tol * max(np.abs(wl).max(), 1e-6)
 
 
+def test_dynamics_backward_through_a_subnormal_power(ops):
+    """A strong gate (scale = |mu|^(c r - 1) below 1.2e-38) and a gradient that brings it back: bf16 as float32, nothing taken for zero.  The
+    bound: a bf16 rounding of the result and ten bits of a power of 1e-42."""
+    B, L, H, N, c = 4, 2048, 4, 2, (60.0, 2.0 ** -3.5, 0.125, 0.018, 1.0)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    gate = torch.randn(B, L, (N + 5) * H, generator=g, device="cuda")
+    gate[..., (N + 4) * H:] += 4.0                                   # (r near one)
+    gate, lds, rf = gate.bfloat16(), 0.5 * torch.randn(H, generator=g, device="cuda"), torch.zeros(H, device="cuda")
+    grads = []
+    for dtype in (torch.float32, torch.bfloat16):
+        x = gate.to(dtype).requires_grad_(True)
+        A = ops.DynamicsFusedFn.apply(x, lds, rf, *c, H, N)[0]
+        grads.append(torch.autograd.grad(A, x, torch.full_like(A, 2.0 ** 120))[0].float()[..., :H])   # (alpha's)
+        if dtype == torch.float32:
+            power = A.detach().abs().amax(-1)
+    at = (power > 1e-42) & (power < 1e-38) & (grads[0].abs() > 1e-8)
+    assert int(at.sum()) > 200
+    off = (grads[1] - grads[0]).abs()[at] / grads[0].abs()[at]
+    assert float(off.median()) <= 2.0 ** -8 and float((off > 2.0 ** -6).float().mean()) <= 0.05
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("rows,D", [(37, 64), (5, 128), (9, 40)])
 def test_normalize_backward(ops, orc, dtype, tol, rows, D):
