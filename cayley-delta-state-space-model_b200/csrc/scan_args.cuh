@@ -68,6 +68,21 @@ struct TokenDynamics {
     }
 };
 
+// The walks' sums and products whose grouping is said, not left to the compiler: either walk may run, by size, and has the bits of the other.
+// x y - z w, x y + z w, the second product rounded
+__device__ __forceinline__ float msub(float x, float y, float z, float w) { return __fmaf_rn(x, y, -__fmul_rn(z, w)); }
+__device__ __forceinline__ float madd(float x, float y, float z, float w) { return __fmaf_rn(x, y, __fmul_rn(z, w)); }
+// s <- gamma s + l
+__device__ __forceinline__ float next_re(float2 g, float sr, float si, float l) { return __fadd_rn(msub(g.x, sr, g.y, si), l); }
+__device__ __forceinline__ float next_im(float2 g, float sr, float si, float l) { return __fadd_rn(madd(g.x, si, g.y, sr), l); }
+// read-out before the norms: (r.q + a_re (z.q)_re -+ a_im (z.q)_im) + K (k.q)
+__device__ __forceinline__ float read_re(float rq, float are, float aim, float zqr, float zqi, float K, float kq) {
+    return __fmaf_rn(K, kq, __fmaf_rn(-aim, zqi, __fmaf_rn(are, zqr, rq)));
+}
+__device__ __forceinline__ float read_im(float rq, float are, float aim, float zqr, float zqi, float K, float kq) {
+    return __fmaf_rn(K, kq, __fmaf_rn(aim, zqr, __fmaf_rn(are, zqi, rq)));
+}
+
 // scan_short.cu: the walk's local and output pass for few units, bit for bit.  from_chunks: no carry pass has run, the output pass adds up
 // the chunks before its own (and writes the final state).
 bool scan_short_takes(const ScanArgs& a, int dtype, int sms);

@@ -29,16 +29,6 @@ struct Geo {
     static constexpr int kBytes = kRows + kScal + kPart + kCoef;
 };
 
-// s <- gamma s + l as the carry pass evaluates it
-__device__ __forceinline__ float next_re(float2 g, float sr, float si, float l) {
-    return __fadd_rn(__fmaf_rn(g.x, sr, -__fmul_rn(g.y, si)), l);
-}
-__device__ __forceinline__ float next_im(float2 g, float sr, float si, float l) {
-    return __fadd_rn(__fmaf_rn(g.x, si, __fmul_rn(g.y, sr)), l);
-}
-// x y - z w, x y + z w, the second product rounded: as the compiler contracts them in scan_simt.cu
-__device__ __forceinline__ float msub(float x, float y, float z, float w) { return __fmaf_rn(x, y, -__fmul_rn(z, w)); }
-__device__ __forceinline__ float madd(float x, float y, float z, float w) { return __fmaf_rn(x, y, __fmul_rn(z, w)); }
 // the order of a butterfly over eight lanes
 __device__ __forceinline__ float tree(const float (&p)[8]) { return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])); }
 
@@ -387,8 +377,8 @@ __global__ void __launch_bounds__(64, 1) scan_short_kernel(const __grid_constant
                     const float* t1 = sc + 12 * tt;
                     const float kq = t1[6], iq = t1[7];
                     // correction is read BEFORE its step (exact_correction.cu:90-94), the local state after
-                    float yr = __fmul_rn(iq, __fmaf_rn(K.x, kq, __fmaf_rn(-t1[1], zqi, __fmaf_rn(t1[0], zqr, rqr))));
-                    float yi = __fmul_rn(iq, __fmaf_rn(K.y, kq, __fmaf_rn(t1[1], zqr, __fmaf_rn(t1[0], zqi, rqi))));
+                    float yr = __fmul_rn(iq, read_re(rqr, t1[0], t1[1], zqr, zqi, K.x, kq));
+                    float yi = __fmul_rn(iq, read_im(rqi, t1[0], t1[1], zqr, zqi, K.y, kq));
                     if (a.shortcut_scale != 0.f) {   // block.py:202-208: sum_d shortcut[s,d] q[d] = (q^.k^)^2 v[s]
                         const float qk = __fmul_rn(__fmul_rn(iq, t1[8]), kq), f = __fmul_rn(__fmul_rn(a.shortcut_scale, qk), qk);
                         yr = __fmaf_rn(f, t1[4], yr);

@@ -229,9 +229,9 @@ scan_walk_kernel(const ScanArgs a) {
         const float ik = rsqrtf(skk + kEps);
         const float bik = be * ik, bik2 = bik * ik;
         // z' = a (z - beta (z.k^) k^) + beta v k^ = a z + Kz k
-        const float czr = bik2 * zkr, czi = bik2 * zki;
-        const float Kzr = bik * vr - (a_re * czr - a_im * czi);
-        const float Kzi = bik * vi - (a_re * czi + a_im * czr);
+        const float czr = __fmul_rn(bik2, zkr), czi = __fmul_rn(bik2, zki);
+        const float Kzr = __fmaf_rn(bik, vr, -msub(a_re, czr, a_im, czi));
+        const float Kzi = __fmaf_rn(bik, vi, -madd(a_re, czi, a_im, czr));
         const float2 are2 = make_float2(a_re, a_re), aim2 = make_float2(a_im, a_im), nim2 = make_float2(-a_im, -a_im);
         {
             const float2 kzr2 = make_float2(Kzr, Kzr), kzi2 = make_float2(Kzi, Kzi);
@@ -242,17 +242,17 @@ scan_walk_kernel(const ScanArgs a) {
                 zi[i] = __ffma2_rn(kzi2, kk[i], __ffma2_rn(are2, y, __fmul2_rn(aim2, x)));
             }
         }
-        const float ncr = a_re * cr - a_im * ci, nci = a_re * ci + a_im * cr;
+        const float ncr = msub(a_re, cr, a_im, ci), nci = madd(a_re, ci, a_im, cr);
         cr = ncr;
         ci = nci;
         if (kOutput) {
             const float iq = rsqrtf(sqq + kEps);
             // correction is read BEFORE its step (exact_correction.cu:90-94), the local state after
-            float yr = iq * (rqr + a_re * zqr - a_im * zqi + Kzr * kq);
-            float yi = iq * (rqi + a_re * zqi + a_im * zqr + Kzi * kq);
+            float yr = __fmul_rn(iq, read_re(rqr, a_re, a_im, zqr, zqi, Kzr, kq));
+            float yi = __fmul_rn(iq, read_im(rqi, a_re, a_im, zqr, zqi, Kzi, kq));
             // r' = a (r - beta (r.k^) k^) = a r + Kr k
-            const float crr = bik2 * rkr, cri = bik2 * rki;
-            const float Krr = -(a_re * crr - a_im * cri), Kri = -(a_re * cri + a_im * crr);
+            const float crr = __fmul_rn(bik2, rkr), cri = __fmul_rn(bik2, rki);
+            const float Krr = -msub(a_re, crr, a_im, cri), Kri = -madd(a_re, cri, a_im, crr);
             const float2 krr2 = make_float2(Krr, Krr), kri2 = make_float2(Kri, Kri);
 #pragma unroll
             for (int i = 0; i < kP; i++) {
@@ -261,10 +261,9 @@ scan_walk_kernel(const ScanArgs a) {
                 ri[i] = __ffma2_rn(kri2, kk[i], __ffma2_rn(are2, y, __fmul2_rn(aim2, x)));
             }
             if (a.shortcut_scale != 0.f) {   // block.py:202-208: sum_d shortcut[s,d] q[d] = (q^.k^)^2 v[s]
-                const float qk = iq * ik * kq;
-                const float f = a.shortcut_scale * qk * qk;
-                yr += f * vr;
-                yi += f * vi;
+                const float qk = __fmul_rn(__fmul_rn(iq, ik), kq), f = __fmul_rn(__fmul_rn(a.shortcut_scale, qk), qk);
+                yr = __fmaf_rn(f, vr, yr);
+                yi = __fmaf_rn(f, vi, yi);
             }
             if (g == 0) {   // v slots of this step are consumed: reuse them to stage y
                 const float sc = sm.sel_c[so + t];
@@ -484,11 +483,11 @@ scan_carry_kernel(const ScanArgs a) {
                     a.ws_state[u * 2 * D + d] = IO<T>::rnd(sr);       // chunk_states store
                     a.ws_state[u * 2 * D + D + d] = IO<T>::rnd(si);
                 }
-                const float nr = gr[i] * sr - gi[i] * si + lr[i];
-                const float ni = gr[i] * si + gi[i] * sr + li[i];
+                const float2 gm = make_float2(gr[i], gi[i]);
+                const float nr = next_re(gm, sr, si, lr[i]);
+                si = next_im(gm, sr, si, li[i]);
                 sr = nr;
-                si = ni;
-                const float pr = gr[i] * dr - gi[i] * di, pi = gr[i] * di + gi[i] * dr;
+                const float pr = msub(gm.x, dr, gm.y, di), pi = madd(gm.x, di, gm.y, dr);
                 dr = pr;
                 di = pi;
             }

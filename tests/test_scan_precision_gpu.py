@@ -169,16 +169,18 @@ def test_scratch_without_room_for_the_carries_gives_the_same_bits(ops, orc, B, H
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("L,D,N,C", [(317, 64, 4, 64), (5, 64, 2, 64), (129, 64, 2, 32), (260, 128, 2, 128)])
 def test_rows_that_travel_ahead_change_no_bit(ops, orc, dtype, L, D, N, C):
-    """The CUDA-core walk takes its rows ahead through shared memory while every SM has a block at most, and one row ahead in
-    registers beyond: fewer tokens than rows travel ahead, ragged and short chunks, a short chunk first and a longer one behind."""
+    """The CUDA-core walk takes its rows ahead through shared memory while every SM has a block at most (1 500 units), and one row ahead in
+    registers beyond (few units: scan_short.cu): fewer tokens than rows travel ahead, ragged and short chunks, a short chunk first and a longer
+    one behind."""
     inp = _inputs(orc, 1, 3, L, D, N, seed=L)
     inp["q"], inp["k"] = inp["q"] * 0.7, inp["k"] * 1.3
     few = run_fused(ops, inp, dtype, N, C, return_tail_state=True, flags=ops.FORCE_SIMT)
-    times = 148 * 16 // (-(-L // C) * 3 * (N // 2)) + 1
-    wide = {k: (np.repeat(v, times, 0) if getattr(v, "ndim", 0) >= 3 else v) for k, v in inp.items()}
-    many = run_fused(ops, wide, dtype, N, C, return_tail_state=True, flags=ops.FORCE_SIMT)
-    for f, m in zip(few, many):
-        assert torch.equal(m[:1], f) and torch.equal(m[-1:], f)
+    units = -(-L // C) * 3 * (N // 2)
+    for times in (1500 // units, 148 * 16 // units + 1):
+        wide = {k: (np.repeat(v, times, 0) if getattr(v, "ndim", 0) >= 3 else v) for k, v in inp.items()}
+        many = run_fused(ops, wide, dtype, N, C, return_tail_state=True, flags=ops.FORCE_SIMT)
+        for f, m in zip(few, many):
+            assert torch.equal(m[:1], f) and torch.equal(m[-1:], f)
 
 
 def test_two_threads_share_a_stream(ops, orc):

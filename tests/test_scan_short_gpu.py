@@ -61,6 +61,28 @@ def test_few_units_have_the_bits_of_many(ops, orc, dtype, H, L, D, N, C, records
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,segments,NC,D,N", [(2, 3, 2, 64, 4), (1, 2, 13, 64, 2), (2, 4, 1, 128, 2)])
+@pytest.mark.parametrize("decay", [0, 4096])
+def test_segments_of_few_units_have_the_bits_of_many(ops, orc, dtype, H, segments, NC, D, N, decay):
+    """Summaries, and scans on the local results that they have left, with positions by segment and with decays in float32: the walk for few
+    units, the one whose rows travel ahead, and the one of many."""
+    L = segments * NC * D
+    inp = unnormalise(orc.make_inputs(1, H, L, D, N=N, seed=L + N, context_length=L), np.random.default_rng(L))
+    one = [to_dev(inp[n], dtype) for n in ("q", "k", "v", "gate_raw")]
+    both = [to_dev(inp[n], torch.float32) for n in ("log_dt_scale", "rope_freqs")]
+    state = to_dev(np.random.default_rng(N).standard_normal((1, H, N, D)).astype(np.float32) * 0.3, torch.float32)
+    units = segments * NC * H * (N // 2)
+    got = []
+    for B in (1, 1500 // units, 148 * 20 // units + 1):
+        wide = lambda x: x.expand(B, *x.shape[1:]).contiguous()
+        got.append(ops.scan_fused_long(*[wide(x) for x in one], *both, *const_args(inp["consts"]), H, N, D, wide(state), segments=segments,
+                                       shortcut_scale=0.25, pos0=5, flags=ops.FORCE_SIMT | decay))
+    for few, ring, many in zip(*got):
+        for x in (ring, many):
+            assert torch.equal(few[0], x[0]) and torch.equal(few[0], x[-1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_nothing_is_written_beside_the_outputs(ops, orc, dtype):
     import cdssm_b200
     lib = cdssm_b200._lib.lib()
