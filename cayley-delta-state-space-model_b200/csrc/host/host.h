@@ -4,6 +4,7 @@
 #pragma once
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -64,13 +65,15 @@ inline float* fmut(const Tensor& t) { return t.defined() ? static_cast<float*>(t
 inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
 // Outputs straight from the framework's CUDA allocator: by way of the dispatcher an allocation took 0.4 us more, of the 4.5 that a one-token
-// step's call takes.
-inline Tensor empty_like_dims(at::IntArrayRef sizes, const Tensor& like) {
-    return at::detail::empty_cuda(sizes, like.scalar_type(), like.device(), std::nullopt);
+// step's call takes.  Not where somebody looks on (dispatch modes and transforms are keys beside the default ones) or wants memory filled
+// (deterministic algorithms).
+inline Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType dt, const Tensor& like) {
+    const bool watched = !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty();
+    if (watched || at::globalContext().deterministicAlgorithms()) return at::empty(sizes, like.options().dtype(dt));
+    return at::detail::empty_cuda(sizes, dt, like.device(), std::nullopt);
 }
-inline Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) {
-    return at::detail::empty_cuda(sizes, at::kFloat, like.device(), std::nullopt);
-}
+inline Tensor empty_like_dims(at::IntArrayRef sizes, const Tensor& like) { return empty_cuda(sizes, like.scalar_type(), like); }
+inline Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) { return empty_cuda(sizes, at::kFloat, like); }
 
 struct Dyn {   // the five scalars of the dynamics
     float c[5];

@@ -140,3 +140,32 @@ def test_wrong_ids_and_weights_are_refused(ops):
     with pytest.raises(RuntimeError):
         odd.forward(ids)
     torch.cuda.synchronize()
+
+
+def _step_args(ops, B=2, H=3, N=4, D=64):
+    from cdssm_b200.model import CdssmConfig
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    c = CdssmConfig(d_model=128, n_layers=1, context_length=64, vocab_size=64, state_dim=N)
+    consts = (c.gating_c, c.omega_thresh, c.adt_delta, c.adt_smoothness, c.adt_eps)
+    return (r(B, H, D), r(B, H, D), r(B, H, N), r(B, (N + 5) * H), r(H).float(), torch.ones(H, device="cuda"), *consts, H, N)
+
+
+def test_outputs_are_seen_by_dispatch_modes(ops):
+    """An output's allocation passes the dispatcher where somebody looks on (memory trackers, loggers)."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchDispatchMode):
+        names = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(func.name())
+            return func(*args, **(kwargs or {}))
+
+    args = _step_args(ops)
+    state = torch.zeros(2, 3, 4, 64, device="cuda")
+    want = ops.decode_step(state.clone(), *args, 5)
+    with Seen() as seen:
+        y = ops.decode_step(state, *args, 5)
+    assert any(n.startswith("aten::empty") for n in seen.names)
+    assert torch.equal(y, want)
