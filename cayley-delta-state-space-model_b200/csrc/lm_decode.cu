@@ -111,7 +111,8 @@ lm_product_kernel(const Args a, const cdssm_lm_layer w, const Product p, bf16* c
     uint4 wr[kAhead][2];
     if (kMode == kInProj && a.first) grid_dependency_wait();
     if ((int)blockIdx.x < items) fetch_first<MT>(p, (int)blockIdx.x % tiles, wr);
-    constexpr int kNormAhead = 3;   // 256-column pieces of the norm's weights that are there before the activations are
+    constexpr int kNormAhead = 3;   // 256-column pieces of the norm's weights that are there before the activations are; wider rows load the rest
+                                    // afterwards (more of them would be registers of every width's kernel)
     uint4 nwr[kNormAhead];
     const bf16* nw = kMode == kHead ? a.final_norm_w : (const bf16*)w.norm_w;
     if (kNorm) {
@@ -379,15 +380,15 @@ static int launch_batch(const Args& a, const cdssm_lm_layer& w, const Product& p
     return launch<1, MT, kMode>(a, w, p, out, out_stride, max_blocks, st);
 }
 
-// us per step on B200, these kernels / the library's products with this library's glue kernels (issued natively; in
-// brackets, as the second figure, from before the loads ahead of the wait, replayed from a CUDA graph), 12 layers, N 2, vocabulary 32000 (d 512: 8 layers, N 16; d 256: 4 layers):
-//     d 256    B 16:  74 / 305  (64 / 95)    B 32:  95 / 311  (86 / 97)     B 128: 165 / 301 (156 / 103)
-//     d 512    B 16: 154 / 573 (154 / 233)   B 32: 217 / 575 (201 / 239)    B 128: 472 / 613 (462 / 275)
-//     d 768    B 1:  203 / 864 (214 / 400)   B 16: 240 / 836 (237 / 378)    B 32:  354 / 878 (334 / 378)
-//              B 64: 522 / 852 (501 / 380)   B 96: 726 / 856 (706 / 390)
-//     d 1024   B 16: 306 / 916 (304 / 420)   B 32: 434 / 836 (416 / 417)    B 64:  758 / 872 (740 / 415)
-// Issued call by call the library path is bounded by the host that issues its 112 launches, and these kernels win until the
-// activations every block reads (B x d) weigh more; inside a captured graph the line is at 32 sequences (the caller's check).
+// us per step on B200, these kernels / the library's products with this library's glue kernels, issued natively (in brackets replayed from a
+// CUDA graph), all of one build; 12 layers, N 2, vocabulary 32000 (d 512: 8 layers, N 16; d 256: 4 layers):
+//     d 256    B 16:  70 / 219  (63 / 86)     B 32:  94 / 223  (86 / 94)     B 128: 162 / 226 (154 / 101)
+//     d 512    B 16: 151 / 490 (140 / 233)    B 32: 212 / 459 (199 / 240)    B 128: 469 / 411 (445 / 274)
+//     d 768    B 1:  207 / 596 (203 / 396)    B 16: 239 / 587 (226 / 374)    B 32:  349 / 602 (329 / 335)    B 64: 502 / 595 (480 / 335)
+//     d 1024   B 16: 300 / 604 (279 / 416)    B 32: 444 / 612 (426 / 415)    B 64:  748 / 605 (728 / 411)
+// Issued call by call the library path is bounded by the host that issues its 112 launches (300 to 920 us on a slower host than this one), and
+// these kernels win until the activations every block reads (B x d) weigh more: d 512, B 128 and d 1024, B 64 are ahead with the slower host only.
+// Inside a captured graph the line is at 32 sequences (the caller's check).
 static bool lm_decode_takes(int B, int d, int di, int H, int N, int groups) {
     // 16-byte pieces of every row; a read-out item is one normalisation group of one to four 16-row fragments
     if (d % 32 || (H * N) % 8 || di % groups) return false;

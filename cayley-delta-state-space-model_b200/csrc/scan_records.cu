@@ -66,7 +66,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kNP, kHg, kResidual, kWa>
     if (clears_ticket) ticket = atomicExch(a.clear + 1, 0);
     const int H = a.H, N = a.N, NP = N >> 1, p0 = kWa ? 0 : kNP * (int)blockIdx.z, pairs = min(kNP, NP - p0);
     // (One or two pairs a thread are for short inputs, a layer's scan of which takes 15 us whatever these instructions: with the quick
-    // division and cut registers 8 layers of 300 tokens, N 4, took 403 us, without 387; 12 of 60, N 8, 545 / 536.)
+    // division and cut registers the kernel alone took 3.7 us instead of 4.3, but 8 layers of 300 tokens, N 4, 403 us, without 387; 12 of 60,
+    // N 8, 545 / 536.  Why is not shown; the moment at which the next kernel's blocks start moves with these instructions.)
     constexpr bool kQuick = kWa || kNP >= 4;
     uint32_t row_of;
     if (kQuick) {

@@ -34,7 +34,7 @@
 // Bounded by issue slots (45 % of them busy at 16 warps per SM) and by the chain of barriers and products through a chunk.  us of a
 // whole call on B200, before (a block per chunk and head, Gram blocks and three bf16 parts on the warp-level mma, carry behind a
 // fence and a flag) / now: D 64, B 8, L 2048, H 24, N 16 291 / 229, N 8 171 / 151, N 4 136 / 113; one sequence of 523, N 16
-// 36.7 / 29.8, N 4 22.8 / 19.0; D 128, 4 x 2048, H 12, N 4 76 / 49, 2 x 1000, H 32, N 8 73 / 51, 4000 tokens, H 12, N 16 144 / 74.
+// 36.7 / 30.1, N 4 22.8 / 19.0; D 128, 4 x 2048, H 12, N 4 76 / 49, 2 x 1000, H 32, N 8 73 / 51, 4000 tokens, H 12, N 16 144 / 74.
 // One or two chunks of D 64, N 8, gain nothing: 2 x 41 tokens, H 16 11.5 / 12.3.
 //
 // Reference semantics (intra_chunk_scan.cu:100-195, exact_correction.cu:89-150): z starts at zero at the chunk start, r
@@ -450,8 +450,8 @@ __device__ __noinline__ bool empty_bad_rows(Smem<kD, kPairs, kMode, kWide>& sm, 
 
 // A block runs most of its code once, 100 to 200 KB of straight line, more than an SM's instruction cache: a warp of a call with a block per
 // SM spent 44 % of its stalls on waiting for instructions, of a full GPU 13 %.  So what comes at several places, or seldom, is a function
-// or a loop: with that and kWide, us before / now: D 64, 523 tokens, H 24, N 16 32.0 / 29.8; B 8, L 2048, H 24, N 4 120 / 112, N 16 245 / 229;
-// D 128, 1000 tokens, H 12, N 8 24.5 / 21.4; 12 layers of a 523-token prompt 801 / 750.  (Not faster: the records' loads as a function with a
+// or a loop: with that and kWide, us before / now: D 64, 523 tokens, H 24, N 16 32.0 / 30.1; B 8, L 2048, H 24, N 4 120 / 112, N 16 245 / 229;
+// D 128, 1000 tokens, H 12, N 8 24.5 / 21.5; 12 layers of a 523-token prompt 801 / 751.  (Not faster: the records' loads as a function with a
 // loop, or one turn of the look-back for carries and states alike.)
 __device__ __noinline__ bool wait_longer(uint64_t* bar, uint32_t parity, int* abort_flag, unsigned long long limit) {
     return mbar_wait_suspend(bar, parity, abort_flag, limit);

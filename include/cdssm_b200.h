@@ -225,7 +225,7 @@ CDSSM_API size_t cdssm_b200_scan_fused_workspace_bytes_for(int B, int L, int H, 
  * chunk semantics (local scan from zero per chunk of C tokens, decay-only carry between chunks,
  * correction taken before each step) -> shortcut -> read-out with q -> sel_C gate.
  * Supported: even N <= 32, D <= 128, C <= 256, bf16 or fp32: CUDA-core kernels, four launches (records, local pass, carry
- * pass, output pass), three without room for their records.  bf16 with D = C in {64, 128} and N <= 16 runs on the tensor
+ * pass, output pass), one less without room for their records and one less where few chunks of few units need no carry pass.  bf16 with D = C in {64, 128} and N <= 16 runs on the tensor
  * cores: N = 2 in local and output pass (tcgen05/TMA), other N in those or in one kernel that hands the carry on inside it;
  * with the records two to four launches.  The arithmetic of a call goes by H, D, N, C, dtype, flags and whether tail_state is
  * asked for, not by B or L: rows of a batch alone, and pieces of a sequence chained through final_state and pos0, have the
