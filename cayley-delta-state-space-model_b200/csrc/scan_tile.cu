@@ -1449,7 +1449,7 @@ scan_tile_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
             if (a.shortcut_scale != 0.f) {   // block.py:202-208; v after the vp scale
                 const float qk = mq[r] * nrm[r] * pd[r];
                 const float2 e = sm.viw[p][row], D = sm.dd[p][row];
-                cplx vg = cmul({e.x, e.y}, {D.x, D.y});
+                cplx vg = cmul({D.x, D.y}, {e.x, e.y});
                 if (((slow >> p) & 1) && p < NPB && head_on) {   // (its v has made room for g)
                     const uint32_t w = __ldcg(a.rec_v + (unit * (size_t)NP + pair0 + p) * kD + row - row0);
                     vg = {bits_lo(w), bits_hi(w)};

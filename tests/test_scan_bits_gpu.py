@@ -26,6 +26,8 @@ WILD = {(8, 500, 64, 2): (1628976053, 3590081624), (4, 700, 128, 2): (4044209766
         (12, 1000, 128, 6): (784751710, 2207710518), (2, 765, 128, 8): (1275000913, 2199383906),
         (24, 1500, 128, 16): (2169433470, 2795242774)}
 
+HUGE = {(5, 165, 64, 4): (566075848, 419627732), (3, 200, 64, 16): (2090349564, 2479583917), (2, 300, 128, 8): (605016733, 4188771241)}
+
 
 def _inputs(H, L, D, N, wild):
     r = np.random.default_rng(H + L + D + N)
@@ -42,8 +44,10 @@ def _inputs(H, L, D, N, wild):
                 rope_freqs=(2048.0 ** (-np.arange(H) / H)).astype(np.float32)), 0.1 * normal(2, H, N, D)
 
 
-def bits(ops, orc, H, L, D, N, wild):
+def bits(ops, orc, H, L, D, N, wild, huge=False):
     inp, h0 = _inputs(H, L, D, N, wild)
+    if huge:   # (the real part; what is left of the imaginary one beside it is the last bit's)
+        inp["v"][0, 29, :, 0] = inp["v"][1, L // 2, :, N - 2] = 3e19
     inp["consts"] = orc.derive_constants(2048)
     y, _, tail = run_fused(ops, inp, torch.bfloat16, N, D, h0=h0, pos0=4 * D, shortcut_scale=0.25, return_tail_state=True)
     return tuple(zlib.crc32(t.contiguous().view(torch.uint8).cpu().numpy().tobytes()) for t in (y, tail))
@@ -53,6 +57,11 @@ def bits(ops, orc, H, L, D, N, wild):
 @pytest.mark.parametrize("wild", [False, True])
 def test_order_of_evaluation_is_kept(ops, orc, H, L, D, N, wild):
     assert bits(ops, orc, H, L, D, N, wild) == (WILD if wild else MODEL)[H, L, D, N]
+
+
+@pytest.mark.parametrize("H,L,D,N", list(HUGE))
+def test_order_of_evaluation_beside_a_huge_value(ops, orc, H, L, D, N):
+    assert bits(ops, orc, H, L, D, N, False, True) == HUGE[H, L, D, N]
 
 
 def _transition(g, lds, freq, pos, c, off_alpha=0.0, off_tau=0.0, off_ta=0.0, off_tw=0.0):
